@@ -63,8 +63,14 @@ std::tuple<Tensor, Tensor> flash_attn_fwd(const Tensor& q, const Tensor& k, cons
   const int64_t qs[3] = {q.stride(0), q.stride(1), q.stride(2)};
   const int64_t ks[3] = {k.stride(0), k.stride(1), k.stride(2)};
   const int64_t vs[3] = {v.stride(0), v.stride(1), v.stride(2)};
+  // few row tiles: the keys are split over work items, whose shares a second kernel combines
+  const int64_t splits = slapo::flash_fwd_splits(B, H, Sq, Sk);
+  Tensor scratch;
+  if (splits > 1)
+    scratch = at::empty({splits * B * H * Sq * (D + 2)}, q.options().dtype(at::kFloat));
   int rc = slapo::launch_flash_fwd(
       q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
+      splits > 1 ? scratch.data_ptr<float>() : nullptr,
       opt_f32(kbias, "key bias"), opt_f32(rel, "relative bias"), B, H, Sq, Sk, D, qs, ks, vs,
       static_cast<float>(scale), causal ? 1 : 0, static_cast<float>(p_drop), unpack_rng(rng),
       q.scalar_type() == at::kBFloat16, slapo_status_ptr(q.get_device()),
@@ -81,31 +87,27 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> flash_attn_bwd(
   TORCH_CHECK(dout.is_contiguous() && o.is_contiguous(), "dout and out must be contiguous");
   c10::cuda::CUDAGuard guard(q.device());
   const int B = q.size(0), Sq = q.size(1), H = q.size(2), D = q.size(3), Sk = k.size(1);
-  // dQ: one fp32 partial per 128-key tile, written with plain stores and summed by the
-  // conversion kernel (no zero fill, no atomics); beyond 16 key tiles, or 4 GB of partials,
-  // a single zero-filled accumulator that the key tiles reduce into
-  const int64_t n_kt = (Sk + 127) / 128;
-  const int64_t dq_elems = static_cast<int64_t>(B) * Sq * H * D;
-  const bool sliced = n_kt <= 16 && n_kt * dq_elems * 4 <= (int64_t(4) << 30);
-  const int n_slices = sliced ? static_cast<int>(n_kt) : 1;
-  Tensor dq_accum = sliced ? at::empty({n_kt, B, Sq, H, D}, q.options().dtype(at::kFloat))
-                           : at::zeros({B, Sq, H, D}, q.options().dtype(at::kFloat));
   // packed_qkv: q, k, v are the slices [..., 0/1/2, :] of one [B, S, H, 3, D]
   // projection output; the gradients are written into one tensor of that
   // layout so that autograd needs no concatenation
-  Tensor dk, dv, dqkv;
-  int64_t dkv_stride = D;
+  Tensor dq, dk, dv, dqkv;
+  int64_t row_stride = D;
   if (packed_qkv) {
     TORCH_CHECK(Sq == Sk, "packed QKV needs equal query and key lengths");
     dqkv = at::empty({B, Sq, H, 3, D}, q.options());
+    dq = dqkv.select(3, 0);
     dk = dqkv.select(3, 1);
     dv = dqkv.select(3, 2);
-    dkv_stride = 3 * D;
+    row_stride = 3 * D;
   } else {
+    dq = at::empty({B, Sq, H, D}, q.options());
     dk = at::empty({B, Sk, H, D}, q.options());
     dv = at::empty({B, Sk, H, D}, q.options());
   }
-  Tensor delta = at::empty({B, H, Sq}, q.options().dtype(at::kFloat));
+  const bool has_bias = kbias.has_value() && kbias->defined();
+  const slapo::FlashBwdScratch sizes =
+      slapo::flash_bwd_scratch(B, H, Sq, Sk, has_bias, static_cast<float>(p_drop));
+  Tensor scratch = at::empty({sizes.total()}, q.options().dtype(at::kFloat));
   Tensor drel;
   const bool has_rel = rel.has_value() && rel->defined();
   if (has_rel) drel = at::zeros_like(*rel);
@@ -115,25 +117,15 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> flash_attn_bwd(
   const int64_t vs[3] = {v.stride(0), v.stride(1), v.stride(2)};
   int rc = slapo::launch_flash_bwd(
       q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), dout.data_ptr(),
-      lse.data_ptr<float>(), delta.data_ptr<float>(), dq_accum.data_ptr<float>(),
-      sliced ? dq_elems : 0, dk.data_ptr(), dv.data_ptr(), dkv_stride, opt_f32(kbias, "key bias"), opt_f32(rel, "relative bias"),
+      lse.data_ptr<float>(), scratch.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(),
+      dv.data_ptr(), row_stride, row_stride, opt_f32(kbias, "key bias"),
+      opt_f32(rel, "relative bias"),
       has_rel ? drel.data_ptr<float>() : nullptr, B, H, Sq, Sk, D, qs, ks, vs,
       static_cast<float>(scale), causal ? 1 : 0, static_cast<float>(p_drop), unpack_rng(rng),
       q.scalar_type() == at::kBFloat16, slapo_status_ptr(q.get_device()),
       at::cuda::getCurrentCUDAStream().stream());
   TORCH_CHECK(rc == 0, "flash_attn_bwd: launch refused (code ", rc, ")");
-  const bool bf16 = q.scalar_type() == at::kBFloat16;
-  const int64_t rows = static_cast<int64_t>(B) * Sq * H;
-  auto stream = at::cuda::getCurrentCUDAStream().stream();
-  if (packed_qkv) {
-    // dq is slice 0 of the packed gradient: rows of D values, 3 D apart
-    slapo::launch_flash_dq_convert(dq_accum.data_ptr<float>(), dqkv.data_ptr(), rows, D, 3 * D,
-                                   bf16, n_slices, dq_elems, Sq, Sk, H, causal ? 1 : 0, stream);
-    return {dqkv, dk, dv, drel};
-  }
-  Tensor dq = at::empty({B, Sq, H, D}, q.options());
-  slapo::launch_flash_dq_convert(dq_accum.data_ptr<float>(), dq.data_ptr(), rows, D, D, bf16,
-                                 n_slices, dq_elems, Sq, Sk, H, causal ? 1 : 0, stream);
+  if (packed_qkv) return {dqkv, dk, dv, drel};
   return {dq, dk, dv, drel};
 }
 

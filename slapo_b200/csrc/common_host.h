@@ -37,20 +37,30 @@ void launch_ln_bwd(const void* gy, const void* gz, const void* zin, const void* 
 namespace slapo {
 // Flash attention on [B, S, H, D] tensors (D contiguous, a multiple of 8 up to 128);
 // *_strides = element strides of (B, S, H).  Return 0 on success.
+int flash_fwd_splits(int B, int H, int Sq, int Sk);
 int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float* lse,
+                     float* scratch,
                      const float* kbias, const float* rel, int B, int H, int Sq, int Sk, int D,
                      const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
                      float scale, int causal, float p_drop, PhiloxArgs rng, bool bf16, int* status,
                      cudaStream_t stream);
+// Scratch of the backward pass, in floats: row statistics, padded key bias and, with dropout,
+// keep bits.  `pairs`: (batch, head) pairs per launch (the keep bits of all of them would
+// grow with B H Sq Sk).
+struct FlashBwdScratch {
+  int64_t stats, bias, keep;
+  int pairs;
+  int64_t total() const { return stats + bias + keep; }
+};
+FlashBwdScratch flash_bwd_scratch(int B, int H, int Sq, int Sk, bool key_bias, float p_drop);
+// dq_row_stride / dkv_row_stride: elements between consecutive (b, s, head) rows of the outputs
 int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
-                     const float* lse, float* delta, float* dq_accum, int64_t dq_slice_stride,
-                     void* dk, void* dv, int64_t dkv_row_stride, const float* kbias, const float* rel, float* drel,
-                     int B, int H, int Sq, int Sk, int D, const int64_t* q_strides, const int64_t* k_strides,
-                     const int64_t* v_strides, float scale, int causal, float p_drop,
-                     PhiloxArgs rng, bool bf16, int* status, cudaStream_t stream);
-void launch_flash_dq_convert(const float* acc, void* out, int64_t rows, int D,
-                             int64_t out_row_stride, bool bf16, int n_slices, int64_t slice_stride,
-                             int Sq, int Sk, int H, int causal, cudaStream_t stream);
+                     const float* lse, float* scratch, void* dq, void* dk, void* dv,
+                     int64_t dq_row_stride, int64_t dkv_row_stride, const float* kbias,
+                     const float* rel, float* drel, int B, int H, int Sq, int Sk, int D,
+                     const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
+                     float scale, int causal, float p_drop, PhiloxArgs rng, bool bf16, int* status,
+                     cudaStream_t stream);
 void launch_flash_dropout_mask(uint8_t* mask, int B, int H, int Sq, int Sk, float p_drop,
                                PhiloxArgs rng, cudaStream_t stream);
 }  // namespace slapo

@@ -4,21 +4,24 @@
 // (so q/k/v slices of a fused QKV projection are read in place through 4-D
 // TMA maps - no .contiguous() copies).  D is 64 or 128.
 //
-// One CTA handles 128 query rows of one (batch, head) and walks over the keys
-// in tiles of 128:
-//   warp 0    TMA: Q once, then a 2-deep K ring and a V buffer
-//   warp 1    tcgen05.mma:  S = Q K^T  (fp32, 128 TMEM columns)
-//                           O_j = P_j V_j  (fp32, double-buffered, D columns each)
-//   warps 2-5 one query row per thread: read S from TMEM, online softmax in
-//             the exp2 domain (scale, additive key bias, relative-position
-//             bias, causal mask, Philox dropout), write P as bf16/fp16 into
-//             swizzled shared memory for the second MMA, fold the per-tile O_j
-//             into a register accumulator with the running rescale.
-// The next S tile is issued before the previous P V product so the tensor
-// core works while the softmax warps fold; for D = 64 two CTAs share an SM.
-#include "common.cuh"
+// Persistent CTAs (D = 64: two per SM with 256 of the 512 TMEM columns each; D = 128: one) walk
+// over work items of 128 query rows of one (batch, head); for each they stream the keys in tiles of 128:
+//   warp 0    TMA: Q, K ring, V ring (runs ahead over tiles and over work items)
+//   warp 1    tcgen05.mma:  S = Q K^T       (fp32, 128 TMEM columns)
+//                           O += P V        (P read from TMEM, fp32 accumulator in TMEM)
+//   warps 2-5 one query row per thread: the row's 128 scores in registers, online softmax in
+//             the exp2 domain, P back to TMEM as bf16 / fp16.
+// The running maximum that P and O are scaled by is only raised when a row's maximum has grown
+// by more than 2^8: until then P simply exceeds 1 (it keeps its relative precision), and O
+// stays where it is.  When it is raised, the warp scales its O rows in TMEM.
+// P has columns of its own: S of the next tile is computed while the softmax warps work on this
+// one.
+//
+// What bounds it: the special-function unit (one exp2 per score, 1024 cycles per 128 x 128 tile
+// and SM) next to the issue slots of the softmax warps.  One thread per whole row needs no
+// exchange between warps; for D = 64 two independent CTAs fill each other's waits.
+#include "flash_common.cuh"
 #include "kernels.h"
-#include "tc05.cuh"
 
 #include <mutex>
 
@@ -28,6 +31,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+void ensure_cuda_context();   // gemm.cu
 
 bool make_tmap_bshd(CUtensorMap* out, const void* base, uint64_t B, uint64_t S, uint64_t H,
                     uint64_t D, uint64_t stride_b, uint64_t stride_s, uint64_t stride_h,
@@ -42,6 +47,7 @@ bool make_tmap_bshd(CUtensorMap* out, const void* base, uint64_t B, uint64_t S, 
       fn = reinterpret_cast<EncodeTiledFn>(ptr);
   });
   if (fn == nullptr) return false;
+  ensure_cuda_context();
   cuuint64_t dims[4] = {D, H, S, B};
   cuuint64_t strides[3] = {stride_h * 2, stride_s * 2, stride_b * 2};
   cuuint32_t box[4] = {64, 1, box_s, 1};
@@ -54,14 +60,20 @@ bool make_tmap_bshd(CUtensorMap* out, const void* base, uint64_t B, uint64_t S, 
 }
 
 // ------------------------------------------------------------------------ //
-constexpr int kBlockM = 128;   // query rows per CTA
+constexpr int kBlockM = 128;   // query rows per work item
 constexpr int kBlockN = 128;   // keys per tile
-constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kRaise = 8.f;  // growth of a row maximum (log2) that makes O be rescaled
 
 struct FlashFwdParams {
   int B, H, Sq, Sk;
   int Dr;              // the tensors' head dimension (<= the kernel's tile width D, % 8 == 0):
                        // TMA zero-fills columns Dr .. D - 1 of every Q / K / V tile
+  int k_steps;         // ceil(Dr / 16): steps of the Q K^T contraction
+  TileWalk walk;
+  int splits;          // work items per row tile: each takes tiles_per_split of the key tiles
+  int tiles_per_split;
+  float* part_o;       // splits > 1: [splits][B H Sq][Dr] unnormalised outputs and
+  float2* part_ml;     // [splits][B H Sq] (maximum in the log2 domain, sum), see combine kernel
   void* O;             // [B, Sq, H, Dr] contiguous
   float* lse;          // [B, H, Sq] natural-log sum-exp of the scaled scores
   const float* kbias;  // [B, Sk] additive key bias or nullptr
@@ -71,92 +83,72 @@ struct FlashFwdParams {
   float p_drop;        // effective probability thr7 / 128
   uint32_t thr7;
   PhiloxArgs rng;
-  int out_bf16;
   uint32_t idesc_qk, idesc_pv;
   int* status;
 };
 
-__device__ __forceinline__ uint32_t pack_pair(float a, float b, int bf16) {
-  if (bf16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-  __half2 v = __floats2half2_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
+template <int D>
+struct FwdSmem {
+  static constexpr int kTile = 128 * D * 2;          // one [128 x D] 16-bit tile
+  static constexpr int kStages = 2;                  // K and V rings
+  static constexpr int kCtas = D == 64 ? 2 : 1;      // per SM: shared memory and TMEM columns
+  static constexpr int kK = kTile;
+  static constexpr int kV = kK + kStages * kTile;
+  static constexpr int kBias = kV + kStages * kTile; // [4 warps][2][128] floats
+  static constexpr int kBars = kBias + 4 * 2 * 128 * 4;
+  static constexpr int kTotal = kBars + 20 * 8 + 1024;
+};
 
-__device__ __forceinline__ void softmax_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-
-// additive (log2-domain) score terms and masking for 32 consecutive keys
-template <bool kFirstPass>
-__device__ __forceinline__ void score_chunk(const uint32_t (&raw)[32], float (&v)[32], int row,
-                                            int key0, const FlashFwdParams& p,
-                                            const float* kb_tile, const float* rel_row,
-                                            int key_limit, int col_in_tile) {
-#pragma unroll
-  for (int t = 0; t < 32; ++t) {
-    const int key = key0 + t;
-    float s = __uint_as_float(raw[t]) * p.scale_log2;
-    if (kb_tile != nullptr) s += kb_tile[col_in_tile + t];
-    if (rel_row != nullptr) s += rel_row[key] * kLog2e;
-    v[t] = key < key_limit ? s : -INFINITY;
-  }
-}
-
-// kPlain: no key bias, no relative bias, not causal, Sk a multiple of 128 and a positive
-// scale - the row maximum is then taken on the raw scores and every probability is one
-// fused multiply-add plus one exp2.
-template <int D, bool kPlain>
+// kGeneral: key bias, relative bias, causal mask, a ragged last key tile or a scale <= 0;
+// without any of them the kernel takes row maxima on the raw scores and every probability is
+// one fused multiply-add plus one exp2.
+template <int D, bool kGeneral, typename T>
 __global__ void __launch_bounds__(192, D == 64 ? 2 : 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const FlashFwdParams p) {
-  constexpr int kTileBytes = 128 * D * 2;   // one [128 x D] 16-bit tile
+  using L = FwdSmem<D>;
+  constexpr int kTileBytes = L::kTile;
+  constexpr int kStages = L::kStages;
   constexpr int kBlkBytes = 128 * 128;      // one [128 rows x 64 cols] swizzled block
   constexpr int kDBlocks = D / 64;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* s_q = smem;
-  uint8_t* s_k = s_q + kTileBytes;          // 2 stages
-  uint8_t* s_v = s_k + 2 * kTileBytes;
-  uint8_t* s_p = s_v + kTileBytes;          // [128 x 128] 16-bit = 2 blocks
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_p + 2 * kBlkBytes);
+  uint8_t* s_k = smem + L::kK;
+  uint8_t* s_v = smem + L::kV;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
   uint64_t* q_full = bars;            // 1
-  uint64_t* k_full = bars + 1;        // 2
-  uint64_t* k_empty = bars + 3;       // 2
-  uint64_t* v_full = bars + 5;
-  uint64_t* v_empty = bars + 6;
-  uint64_t* s_full = bars + 7;
-  uint64_t* p_full = bars + 8;
-  uint64_t* o_full = bars + 9;        // 2
-  uint64_t* o_empty = bars + 11;      // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+  uint64_t* q_empty = bars + 1;       // 1
+  uint64_t* k_full = bars + 2;        // 2
+  uint64_t* k_empty = bars + 4;       // 2
+  uint64_t* v_full = bars + 6;        // 2
+  uint64_t* v_empty = bars + 8;       // 2
+  uint64_t* s_full = bars + 10;       // S of a tile is in tensor memory
+  uint64_t* s_free = bars + 11;       // ... and has been read out of it
+  uint64_t* p_full = bars + 12;       // P of a tile is in tensor memory
+  uint64_t* pv_done = bars + 13;      // O includes a tile
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* kb_tile = reinterpret_cast<float*>(bars + 16);  // 128 floats
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q0 = blockIdx.x * kBlockM;
-  const int head = blockIdx.y, batch = blockIdx.z;
   const int diag = p.Sk - p.Sq;  // key j visible to query i iff j <= i + diag (causal)
-  int n_tiles = (p.Sk + kBlockN - 1) / kBlockN;
-  if (p.causal) {
-    const int last_key = min(p.Sk, q0 + kBlockM + diag);
-    n_tiles = max(1, min(n_tiles, (last_key + kBlockN - 1) / kBlockN));
-  }
   constexpr uint32_t kTmemCols = D == 64 ? 256 : 512;
+  constexpr uint32_t kColP = 128, kColO = 192;    // S: 0
 
   if (threadIdx.x == 0) {
     tc::mbar_init(q_full, 1);
+    tc::mbar_init(q_empty, 1);
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&k_full[i], 1);
       tc::mbar_init(&k_empty[i], 1);
-      tc::mbar_init(&o_full[i], 1);
-      tc::mbar_init(&o_empty[i], 4);
+      tc::mbar_init(&v_full[i], 1);
+      tc::mbar_init(&v_empty[i], 1);
     }
-    tc::mbar_init(v_full, 1);
-    tc::mbar_init(v_empty, 1);
     tc::mbar_init(s_full, 1);
+    tc::mbar_init(s_free, 4);
     tc::mbar_init(p_full, 4);
+    tc::mbar_init(pv_done, 1);
     *abort_flag = 0;
     tc::fence_barrier_init();
   }
@@ -168,233 +160,324 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s = tmem_base;
-  const uint32_t tmem_o = tmem_base + 128;
+  const int items = p.walk.items() * p.splits;
+  // row tile, (batch, head) and key tiles [j0, j0 + n) of a work item
+  auto item_at = [&](int item, int& tile, int& bh, int& j0) {
+    const int unit = p.splits == 1 ? item : item / p.splits;
+    p.walk.at(unit, tile, bh);
+    int n = (p.Sk + kBlockN - 1) / kBlockN;
+    if (p.causal) {
+      const int last_key = min(p.Sk, tile * kBlockM + kBlockM + diag);
+      n = max(1, min(n, (last_key + kBlockN - 1) / kBlockN));
+    }
+    j0 = 0;
+    if (p.splits > 1) {     // (one row tile per head: every split has at least one key tile)
+      j0 = (item - unit * p.splits) * p.tiles_per_split;
+      n = min(p.tiles_per_split, n - j0);
+    }
+    return n;
+  };
 
   if (warp == 0) {
     if (lane == 0) {
       tc::tma_prefetch_desc(&tm_q);
       tc::tma_prefetch_desc(&tm_k);
       tc::tma_prefetch_desc(&tm_v);
-      tc::mbar_arrive_expect_tx(q_full, kTileBytes);
-#pragma unroll
-      for (int d = 0; d < kDBlocks; ++d)
-        tc::tma_load_4d(s_q + d * kBlkBytes, &tm_q, q_full, d * 64, head, q0, batch);
       bool ok = true;
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int st = j & 1;
-        if (!tc::mbar_wait(&k_empty[st], ((j >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
-        tc::mbar_arrive_expect_tx(&k_full[st], kTileBytes);
+      int t = 0, w = 0;
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++w) {
+        int tile, bh, j0;
+        const int n = item_at(item, tile, bh, j0);
+        const int batch = bh / p.H, head = bh - batch * p.H;
+        if (!tc::mbar_wait(q_empty, (w & 1) ^ 1, abort_flag)) { ok = false; break; }
+        tc::mbar_arrive_expect_tx(q_full, kTileBytes);
 #pragma unroll
         for (int d = 0; d < kDBlocks; ++d)
-          tc::tma_load_4d(s_k + st * kTileBytes + d * kBlkBytes, &tm_k, &k_full[st], d * 64, head,
-                          j * kBlockN, batch);
-        if (!tc::mbar_wait(v_empty, (j & 1) ^ 1, abort_flag)) { ok = false; break; }
-        tc::mbar_arrive_expect_tx(v_full, kTileBytes);
+          tc::tma_load_4d(s_q + d * kBlkBytes, &tm_q, q_full, d * 64, head, tile * kBlockM, batch);
+        for (int j = 0; j < n; ++j, ++t) {
+          const int st = t % kStages;
+          const uint32_t ph = (t / kStages) & 1;
+          if (!tc::mbar_wait(&k_empty[st], ph ^ 1, abort_flag)) { ok = false; break; }
+          tc::mbar_arrive_expect_tx(&k_full[st], kTileBytes);
 #pragma unroll
-        for (int d = 0; d < kDBlocks; ++d)
-          tc::tma_load_4d(s_v + d * kBlkBytes, &tm_v, v_full, d * 64, head, j * kBlockN, batch);
+          for (int d = 0; d < kDBlocks; ++d)
+            tc::tma_load_4d(s_k + st * kTileBytes + d * kBlkBytes, &tm_k, &k_full[st], d * 64, head,
+                            (j0 + j) * kBlockN, batch);
+          if (!tc::mbar_wait(&v_empty[st], ph ^ 1, abort_flag)) { ok = false; break; }
+          tc::mbar_arrive_expect_tx(&v_full[st], kTileBytes);
+#pragma unroll
+          for (int d = 0; d < kDBlocks; ++d)
+            tc::tma_load_4d(s_v + st * kTileBytes + d * kBlkBytes, &tm_v, &v_full[st], d * 64, head,
+                            (j0 + j) * kBlockN, batch);
+        }
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      bool ok = tc::mbar_wait(q_full, 0, abort_flag);
       const uint32_t q_addr = tc::smem_u32(s_q);
-      const uint32_t v_addr = tc::smem_u32(s_v);
-      const uint32_t p_addr = tc::smem_u32(s_p);
-      auto issue_qk = [&](int j) -> bool {
-        const int st = j & 1;
-        if (!tc::mbar_wait(&k_full[st], (j >> 1) & 1, abort_flag)) return false;
+      // S of tile t (the w-th item's; `last`: its last one)
+      auto issue_qk = [&](int t, int w, bool first, bool last) -> bool {
+        const int st = t % kStages;
+        if (first && !tc::mbar_wait(q_full, w & 1, abort_flag)) return false;
+        if (!tc::mbar_wait(&k_full[st], (t / kStages) & 1, abort_flag)) return false;
         tc::fence_after_sync();
         const uint32_t k_addr = tc::smem_u32(s_k + st * kTileBytes);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * kBlkBytes + (kk & 3) * 32;
-          tc::umma_f16(tmem_s, tc::smem_desc(q_addr + off, 16, 1024),
-                       tc::smem_desc(k_addr + off, 16, 1024), p.idesc_qk, kk != 0 ? 1u : 0u);
+          if (kk < p.k_steps) {
+            const uint32_t off = (kk >> 2) * kBlkBytes + (kk & 3) * 32;
+            tc::umma_f16(tmem_base, tc::smem_desc(q_addr + off, 16, 1024),
+                         tc::smem_desc(k_addr + off, 16, 1024), p.idesc_qk, kk != 0 ? 1u : 0u);
+          }
         }
         tc::umma_commit(s_full);
         tc::umma_commit(&k_empty[st]);
+        if (last) tc::umma_commit(q_empty);
         return true;
       };
-      if (ok) ok = issue_qk(0);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        // P_j written (hence S_j fully read): S may be overwritten by the next tile
-        if (!tc::mbar_wait(p_full, j & 1, abort_flag)) { ok = false; break; }
-        tc::fence_after_sync();
-        if (j + 1 < n_tiles && !issue_qk(j + 1)) { ok = false; break; }
-        const int ob = j & 1;
-        if (!tc::mbar_wait(&o_empty[ob], ((j >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
-        if (!tc::mbar_wait(v_full, j & 1, abort_flag)) { ok = false; break; }
-        tc::fence_after_sync();
-#pragma unroll
-        for (int kk = 0; kk < kBlockN / 16; ++kk) {
-          const uint64_t a_desc =
-              tc::smem_desc(p_addr + (kk >> 2) * kBlkBytes + (kk & 3) * 32, 16, 1024);
-          const uint64_t b_desc = tc::smem_desc(v_addr + kk * 2048, kBlkBytes, 1024);
-          tc::umma_f16(tmem_o + ob * D, a_desc, b_desc, p.idesc_pv, kk != 0 ? 1u : 0u);
+      bool ok = true;
+      int t = 0, w = 0;
+      int item = blockIdx.x;
+      int n = 0;
+      if (item < items) {
+        int tile, bh, j0;
+        n = item_at(item, tile, bh, j0);
+        ok = issue_qk(0, 0, true, n == 1);
+      }
+      while (item < items && ok) {
+        const int next_item = item + gridDim.x;
+        int next_n = 0;
+        if (next_item < items) {
+          int tile, bh, j0;
+          next_n = item_at(next_item, tile, bh, j0);
         }
-        tc::umma_commit(&o_full[ob]);
-        tc::umma_commit(v_empty);
+        for (int j = 0; j < n; ++j, ++t) {
+          auto issue_next = [&]() -> bool {
+            if (j + 1 < n) return issue_qk(t + 1, w, false, j + 2 == n);
+            if (next_n > 0) return issue_qk(t + 1, w + 1, true, next_n == 1);
+            return true;
+          };
+          // S has been read out: the next tile's goes in its place under this one's softmax
+          if (!tc::mbar_wait(s_free, t & 1, abort_flag) || !issue_next()) { ok = false; break; }
+          const int st = t % kStages;
+          if (!tc::mbar_wait(&v_full[st], (t / kStages) & 1, abort_flag) ||
+              !tc::mbar_wait(p_full, t & 1, abort_flag)) { ok = false; break; }
+          tc::fence_after_sync();
+          const uint32_t v_addr = tc::smem_u32(s_v + st * kTileBytes);
+#pragma unroll
+          for (int kk = 0; kk < kBlockN / 16; ++kk)
+            tc::umma_f16_ts(tmem_base + kColO, tmem_base + kColP + kk * 8,
+                            tc::smem_desc(v_addr + kk * 2048, kBlkBytes, 1024), p.idesc_pv,
+                            (j | kk) != 0 ? 1u : 0u);
+          tc::umma_commit(pv_done);
+          tc::umma_commit(&v_empty[st]);
+        }
+        item = next_item;
+        n = next_n;
+        ++w;
       }
     }
   } else {
     // ------------------------------ softmax warps ------------------------------
     const int quarter = warp & 3;
     const int row_in_tile = quarter * 32 + lane;
-    const int row = q0 + row_in_tile;
-    const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
-    const int sm_tid = (warp - 2) * 32 + lane;
+    const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    float* kb_buf = reinterpret_cast<float*>(smem + L::kBias) + (warp - 2) * 256;
     uint64_t seed = 0, offset = 0;
     if (p.p_drop > 0.f) philox_unpack(p.rng, seed, offset);
     const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
     const int sk16 = (p.Sk + 15) >> 4;
-    const uint64_t drop_row_base =
-        (static_cast<uint64_t>(batch * p.H + head) * p.Sq + min(row, p.Sq - 1)) * sk16;
-    const float* rel_row = nullptr;
-    if (p.rel != nullptr)
-      rel_row = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + (p.Sq - 1) - min(row, p.Sq - 1);
-    float o_acc[D];
-#pragma unroll
-    for (int d = 0; d < D; ++d) o_acc[d] = 0.f;
-    float m_run = -INFINITY, l_run = 0.f, alpha_fold = 1.f;
+    // scores are brought to the log2 domain before the maximum only where something is added
+    // to them (or the scale would turn the maximum around)
+    const bool biased = kGeneral && (p.kbias != nullptr || p.rel != nullptr || !(p.scale_log2 > 0.f));
+    const float sc = biased ? 1.f : p.scale_log2;
     bool ok = true;
-
-    auto fold = [&](int jt) -> bool {
-      const int ob = jt & 1;
-      if (!tc::mbar_wait_warp(&o_full[ob], (jt >> 1) & 1, abort_flag)) return false;
-      tc::fence_after_sync();
-#pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t r[32];
-        tc::tmem_ld_x32(tmem_o + ob * D + c * 32 + lane_sel, r);
-        tc::tmem_ld_wait();
-#pragma unroll
-        for (int t = 0; t < 32; ++t)
-          o_acc[c * 32 + t] = o_acc[c * 32 + t] * alpha_fold + __uint_as_float(r[t]);
-      }
-      tc::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&o_empty[ob]);
-      return true;
-    };
-
-    for (int j = 0; j < n_tiles && ok; ++j) {
-      const int k0 = j * kBlockN;
-      if (p.kbias != nullptr) {
-        softmax_bar_sync();  // previous tile's readers are done
-        const int key = k0 + sm_tid;
-        kb_tile[sm_tid] = key < p.Sk ? p.kbias[static_cast<int64_t>(batch) * p.Sk + key] * kLog2e : 0.f;
-        softmax_bar_sync();
-      }
-      if (!tc::mbar_wait_warp(s_full, j & 1, abort_flag)) { ok = false; break; }
-      tc::fence_after_sync();
+    int t = 0;
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+      int tile, bh, j0;
+      const int n = item_at(item, tile, bh, j0);
+      const int batch = bh / p.H, head = bh - batch * p.H;
+      const int row = tile * kBlockM + row_in_tile;
+      const uint64_t drop_row_base =
+          (static_cast<uint64_t>(bh) * p.Sq + min(row, p.Sq - 1)) * sk16;
+      const float* rel_row = nullptr;
+      if (kGeneral && p.rel != nullptr)
+        rel_row = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + (p.Sq - 1) -
+                  min(row, p.Sq - 1);
       int key_limit = p.Sk;
       if (p.causal) key_limit = min(key_limit, row + diag + 1);
-      const float* kb = p.kbias != nullptr ? kb_tile : nullptr;
-      // pass 1: row maximum
-      float mm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // 4 chains for ILP
-#pragma unroll 1
-      for (int c = 0; c < kBlockN / 32; ++c) {
-        uint32_t raw[32];
-        tc::tmem_ld_x32(tmem_s + c * 32 + lane_sel, raw);
-        tc::tmem_ld_wait();
-        if constexpr (kPlain) {
-#pragma unroll
-          for (int t = 0; t < 32; ++t) mm[t & 3] = fmaxf(mm[t & 3], __uint_as_float(raw[t]));
-        } else {
-          float v[32];
-          score_chunk<true>(raw, v, row, k0 + c * 32, p, kb, rel_row, key_limit, c * 32);
-#pragma unroll
-          for (int t = 0; t < 32; ++t) mm[t & 3] = fmaxf(mm[t & 3], v[t]);
-        }
-      }
-      float m_tile = fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3]));
-      if constexpr (kPlain) m_tile *= p.scale_log2;
-      const float m_new = fmaxf(m_run, m_tile);
-      const float m_use = m_new == -INFINITY ? 0.f : m_new;
-      const float alpha = m_run == -INFINITY ? 0.f : exp2f(m_run - m_use);
-      // the P buffer is single: the previous P V product must have retired
-      // before it is overwritten (the fold below consumes the same phase)
-      if (j > 0 && !tc::mbar_wait_warp(&o_full[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag)) {
-        ok = false;
-        break;
-      }
-      // pass 2: probabilities, row sum, dropout, P -> shared memory
-      float ll[4] = {0.f, 0.f, 0.f, 0.f};
-      uint8_t* p_row = s_p + row_in_tile * 128;
-#pragma unroll 1
-      for (int c = 0; c < kBlockN / 32; ++c) {
-        uint32_t raw[32];
-        float v[32];
-        tc::tmem_ld_x32(tmem_s + c * 32 + lane_sel, raw);
-        tc::tmem_ld_wait();
-        if constexpr (kPlain) {
-#pragma unroll
-          for (int t = 0; t < 32; ++t) {
-            v[t] = exp2f(fmaf(__uint_as_float(raw[t]), p.scale_log2, -m_use));
-            ll[t & 3] += v[t];
+      float m_ref = -INFINITY;
+      uint64_t l2 = 0;      // two fp32 partial row sums
+      for (int j = 0; j < n; ++j, ++t) {
+        const int k0 = (j0 + j) * kBlockN;
+        const float* kb = nullptr;
+        if (kGeneral && p.kbias != nullptr) {
+          // this warp's copy of the tile's key bias (two buffers: the readers of the one
+          // before the last are done once every lane has passed the __syncwarp in between)
+          float* dst = kb_buf + (t & 1) * 128;
+          for (int i = lane; i < kBlockN; i += 32) {
+            const int key = k0 + i;
+            dst[i] = key < p.Sk ? p.kbias[static_cast<int64_t>(batch) * p.Sk + key] * kLog2e : 0.f;
           }
-        } else {
-          score_chunk<false>(raw, v, row, k0 + c * 32, p, kb, rel_row, key_limit, c * 32);
+          __syncwarp();
+          kb = dst;
+        }
+        if (!tc::mbar_wait_warp(s_full, t & 1, abort_flag)) { ok = false; break; }
+        tc::fence_after_sync();
+        uint32_t raw[4][32];
 #pragma unroll
-          for (int t = 0; t < 32; ++t) {
-            v[t] = exp2f(v[t] - m_use);
-            ll[t & 3] += v[t];
+        for (int c = 0; c < 4; ++c) tc::tmem_ld_x32(tmem_row + c * 32, raw[c]);
+        tc::tmem_ld_wait();
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(s_free);
+        if constexpr (kGeneral) {
+          if (biased) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                float s = __uint_as_float(raw[c][i]) * p.scale_log2;
+                if (kb != nullptr) s += kb[c * 32 + i];
+                if (rel_row != nullptr)
+                  s = fmaf(rel_row[min(k0 + c * 32 + i, p.Sk - 1)], kLog2e, s);
+                raw[c][i] = __float_as_uint(s);
+              }
+          }
+          const int first_limit = p.causal ? min(p.Sk, tile * kBlockM + quarter * 32 + diag + 1) : p.Sk;
+          if (k0 + kBlockN > first_limit) {     // some lane of the warp masks something
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (k0 + c * 32 + i >= key_limit) raw[c][i] = 0xff800000u;   // -inf
           }
         }
-        uint32_t pk[16];
+        float mm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // 4 chains for ILP
 #pragma unroll
-        for (int i = 0; i < 16; ++i) pk[i] = pack_pair(v[2 * i], v[2 * i + 1], p.out_bf16);
-        if (p.p_drop > 0.f) {
-          // dropped probabilities are cleared in the packed 16-bit pairs
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint4 kw = philox_keep16(seed, offset,
-                                           drop_row_base + ((k0 + c * 32 + h * 16) >> 4), add4);
-            const uint32_t w[4] = {kw.x, kw.y, kw.z, kw.w};
+          for (int i = 0; i < 32; i += 2)
+            mm[c] = fmaxf(mm[c], fmaxf(__uint_as_float(raw[c][i]), __uint_as_float(raw[c][i + 1])));
+        const float m_tile = fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3])) * sc;
+        // P of the tile before has been read (and O includes it)
+        if (t > 0 && !tc::mbar_wait_warp(pv_done, (t - 1) & 1, abort_flag)) { ok = false; break; }
+        if (j == 0) {
+          m_ref = m_tile;
+        } else if (__any_sync(0xffffffffu, m_tile > m_ref + kRaise)) {
+          const float m_new = fmaxf(m_ref, m_tile);
+          const float alpha = m_ref == -INFINITY ? 0.f : exp2f(m_ref - m_new);
+          const uint64_t alpha2 = f2_pack(alpha, alpha);
+          tc::fence_after_sync();
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              pk[h * 8 + i * 2 + 0] &= keep_mask_pair(w[i], 0);
-              pk[h * 8 + i * 2 + 1] &= keep_mask_pair(w[i], 1);
+          for (int c = 0; c < D / 16; ++c) {
+            uint32_t o[16];
+            tc::tmem_ld_x16(tmem_row + kColO + c * 16, o);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tc::tmem_st_x16(tmem_row + kColO + c * 16, o);
+          }
+          l2 = f2_mul(l2, alpha2);
+          m_ref = m_new;
+        }
+        const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+        const uint64_t sc2 = f2_pack(sc, sc), nm2 = f2_pack(-m_use, -m_use);
+        if (j == 0) l2 = 0;
+        uint64_t la = l2, lb = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const uint64_t x = f2_fma(
+                f2_pack(__uint_as_float(raw[c][2 * i]), __uint_as_float(raw[c][2 * i + 1])), sc2, nm2);
+            float a, b;
+            f2_unpack(x, a, b);
+            a = exp2f(a);
+            b = exp2f(b);
+            if (i & 1) lb = f2_add(lb, f2_pack(a, b));
+            else la = f2_add(la, f2_pack(a, b));
+            pk[i] = pack16<T>(a, b);
+          }
+          if (p.p_drop > 0.f) {
+            // dropped probabilities are cleared in the packed 16-bit pairs
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const uint4 kw = philox_keep16(seed, offset,
+                                             drop_row_base + ((k0 + c * 32 + h * 16) >> 4), add4);
+              const uint32_t wd[4] = {kw.x, kw.y, kw.z, kw.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                pk[h * 8 + i * 2 + 0] &= keep_mask_pair(wd[i], 0);
+                pk[h * 8 + i * 2 + 1] &= keep_mask_pair(wd[i], 1);
+              }
+            }
+          }
+          tc::tmem_st_x16(tmem_row + kColP + c * 16, pk);
+        }
+        l2 = f2_add(la, lb);
+        tc::tmem_st_wait();
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(p_full);
+      }
+      if (!ok) break;
+      // O of this item (the next item's first P V product waits for this warp's next P)
+      if (!tc::mbar_wait_warp(pv_done, (t - 1) & 1, abort_flag)) { ok = false; break; }
+      tc::fence_after_sync();
+      float l_run, l_hi;
+      f2_unpack(l2, l_run, l_hi);
+      l_run += l_hi;
+      if (p.splits > 1) {
+        // this split's share: unnormalised output, maximum and sum
+        const int split = item - item / p.splits * p.splits;
+        const int64_t at = (static_cast<int64_t>(split) * p.B * p.H + bh) * p.Sq + min(row, p.Sq - 1);
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t o[32];
+          tc::tmem_ld_x32(tmem_row + kColO + c * 32, o);
+          tc::tmem_ld_wait();
+          if (row < p.Sq) {
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+              if (c * 32 + g * 4 < p.Dr)
+                *reinterpret_cast<uint4*>(p.part_o + at * p.Dr + c * 32 + g * 4) =
+                    make_uint4(o[4 * g], o[4 * g + 1], o[4 * g + 2], o[4 * g + 3]);
+          }
+        }
+        tc::fence_before_sync();
+        if (row < p.Sq) p.part_ml[at] = make_float2(m_ref, l_run);
+        continue;
+      }
+      const float inv = l_run > 0.f ? 1.f / (l_run * (1.f - p.p_drop)) : 0.f;
+      uint8_t* dst = static_cast<uint8_t*>(p.O) +
+                     ((static_cast<int64_t>(batch) * p.Sq + min(row, p.Sq - 1)) * p.H + head) * p.Dr * 2;
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t o[32];
+        tc::tmem_ld_x32(tmem_row + kColO + c * 32, o);
+        tc::tmem_ld_wait();
+        if (row < p.Sq) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            if (c * 32 + g * 8 < p.Dr) {     // padded columns are not part of the output
+              uint32_t v[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                v[i] = pack16<T>(__uint_as_float(o[g * 8 + 2 * i]) * inv,
+                                 __uint_as_float(o[g * 8 + 2 * i + 1]) * inv);
+              *reinterpret_cast<uint4*>(dst + (c * 32 + g * 8) * 2) = make_uint4(v[0], v[1], v[2], v[3]);
             }
           }
         }
-        // keys [c*32, c*32+32) of this row: block (c >> 1), 16-byte chunks (c & 1) * 4 + g
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const int chunk = (c & 1) * 4 + g;
-          *reinterpret_cast<uint4*>(p_row + (c >> 1) * kBlkBytes +
-                                    ((chunk ^ (row_in_tile & 7)) << 4)) =
-              make_uint4(pk[g * 4], pk[g * 4 + 1], pk[g * 4 + 2], pk[g * 4 + 3]);
-        }
       }
-      tc::fence_before_sync();   // S reads are complete
-      tc::fence_proxy_async();   // P stores visible to the tensor core
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(p_full);
-      l_run = l_run * alpha + ((ll[0] + ll[1]) + (ll[2] + ll[3]));
-      if (j > 0) ok = fold(j - 1);
-      alpha_fold = alpha;
-      m_run = m_new;
-    }
-    if (ok) ok = fold(n_tiles - 1);
-    if (ok && row < p.Sq) {
-      const float inv = l_run > 0.f ? 1.f / (l_run * (1.f - p.p_drop)) : 0.f;
-      uint8_t* dst = static_cast<uint8_t*>(p.O) +
-                     ((static_cast<int64_t>(batch) * p.Sq + row) * p.H + head) * p.Dr * 2;
-#pragma unroll
-      for (int g = 0; g < D / 8; ++g) {
-        if (g * 8 >= p.Dr) break;     // padded columns (zero) are not part of the output
-        uint4 pk = make_uint4(pack_pair(o_acc[g * 8 + 0] * inv, o_acc[g * 8 + 1] * inv, p.out_bf16),
-                              pack_pair(o_acc[g * 8 + 2] * inv, o_acc[g * 8 + 3] * inv, p.out_bf16),
-                              pack_pair(o_acc[g * 8 + 4] * inv, o_acc[g * 8 + 5] * inv, p.out_bf16),
-                              pack_pair(o_acc[g * 8 + 6] * inv, o_acc[g * 8 + 7] * inv, p.out_bf16));
-        *reinterpret_cast<uint4*>(dst + g * 16) = pk;
+      tc::fence_before_sync();
+      if (row < p.Sq) {
+        const float m_nat = (m_ref == -INFINITY ? 0.f : m_ref) * 0.6931471805599453f;
+        p.lse[static_cast<int64_t>(bh) * p.Sq + row] = l_run > 0.f ? m_nat + logf(l_run) : -INFINITY;
       }
-      const float m_nat = (m_run == -INFINITY ? 0.f : m_run) * 0.6931471805599453f;
-      p.lse[(static_cast<int64_t>(batch) * p.H + head) * p.Sq + row] =
-          l_run > 0.f ? m_nat + logf(l_run) : -INFINITY;
     }
   }
 
@@ -405,6 +488,42 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem_base, kTmemCols);
   }
+}
+
+// Output and log-sum-exp of rows whose keys were split over work items: one warp per row, lanes
+// along d (8 per thread for the 16 lanes that D = 128 needs, the other half idle).
+template <typename T>
+__global__ void __launch_bounds__(128) flash_combine_kernel(
+    const float* __restrict__ part_o, const float2* __restrict__ part_ml, T* __restrict__ out,
+    float* __restrict__ lse, int splits, int rows, int H, int Sq, int Dr, float keep_prob) {
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= rows) return;       // r = (b * H + h) * Sq + i
+  float m = -INFINITY;
+  for (int s = 0; s < splits; ++s) m = fmaxf(m, part_ml[static_cast<int64_t>(s) * rows + r].x);
+  const float m_use = m == -INFINITY ? 0.f : m;
+  float l = 0.f, v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  const int d = lane * 8;
+  for (int s = 0; s < splits; ++s) {
+    const int64_t at = static_cast<int64_t>(s) * rows + r;
+    const float2 ml = part_ml[at];
+    const float w = exp2f(ml.x - m_use);      // 0 for a split without a visible key
+    l += w * ml.y;
+    if (d < Dr) {
+      float x[8];
+      Vec8<float>::load(part_o + at * Dr + d, x);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] += w * x[k];
+    }
+  }
+  if (d < Dr) {
+    const float inv = l > 0.f ? 1.f / (l * keep_prob) : 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] *= inv;
+    const int i = r % Sq, bh = r / Sq;
+    const int h = bh % H, b = bh / H;
+    Vec8<T>::store(out + ((static_cast<int64_t>(b) * Sq + i) * H + h) * Dr + d, v);
+  }
+  if (lane == 0) lse[r] = l > 0.f ? m_use * 0.6931471805599453f + logf(l) : -INFINITY;
 }
 
 // Dropout keep-mask exactly as the attention kernels draw it (testing aid).
@@ -432,11 +551,12 @@ void launch_flash_dropout_mask(uint8_t* mask, int B, int H, int Sq, int Sk, floa
   flash_dropout_mask_kernel<<<sm_count() * 4, 256, 0, stream>>>(mask, B, H, Sq, Sk, p_drop, rng);
 }
 
-template <int D, bool kPlain>
+template <int D, bool kGeneral, typename T>
 static int launch_fwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                         const FlashFwdParams& p, cudaStream_t stream) {
-  constexpr int kSmem = 4 * 128 * D * 2 + 2 * 128 * 128 + 16 * 8 + 128 * 4 + 1024;
-  auto kernel = flash_fwd_kernel<D, kPlain>;
+  constexpr int kSmem = FwdSmem<D>::kTotal;
+  static_assert(FwdSmem<D>::kCtas * (kSmem + 1024) <= 228 * 1024, "flash forward: shared memory");
+  auto kernel = flash_fwd_kernel<D, kGeneral, T>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
@@ -444,13 +564,29 @@ static int launch_fwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
       return 3;
     configured = true;
   }
-  dim3 grid((p.Sq + kBlockM - 1) / kBlockM, p.H, p.B);
+  const int64_t items = static_cast<int64_t>(p.walk.row_tiles) * p.walk.nbh * p.splits;
+  const int64_t cap = FwdSmem<D>::kCtas * sm_count();
   count_launch();
-  kernel<<<grid, 192, kSmem, stream>>>(tq, tk, tv, p);
+  kernel<<<static_cast<int>(items < cap ? items : cap), 192, kSmem, stream>>>(tq, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
+// Work items per row tile.  One row tile per (batch, head) - generation, short queries - and
+// fewer of them than half the resident CTAs (two per SM): the keys are split so that the CTAs
+// are used, down to one key tile per item.
+int flash_fwd_splits(int B, int H, int Sq, int Sk) {
+  const int tiles = (Sk + kBlockN - 1) / kBlockN;
+  const int64_t bh = static_cast<int64_t>(B) * H, cap = 2 * sm_count();
+  if (Sq > kBlockM || bh <= 0 || 2 * bh > cap || tiles < 2) return 1;
+  int64_t s = cap / bh;
+  if (s > tiles) s = tiles;
+  const int per = static_cast<int>((tiles + s - 1) / s);
+  return (tiles + per - 1) / per;     // no empty split
+}
+
+// `scratch`: flash_fwd_splits() * B * H * Sq * (D + 2) floats, or null with a single split
 int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float* lse,
+                     float* scratch,
                      const float* kbias, const float* rel, int B, int H, int Sq, int Sk, int D,
                      const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
                      float scale, int causal, float p_drop, PhiloxArgs rng, bool bf16, int* status,
@@ -466,19 +602,49 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float
     return 2;
   FlashFwdParams p;
   p.B = B; p.H = H; p.Sq = Sq; p.Sk = Sk; p.Dr = D; p.O = o; p.lse = lse; p.kbias = kbias; p.rel = rel;
+  p.k_steps = (D + 15) / 16;
+  p.walk.row_tiles = (Sq + kBlockM - 1) / kBlockM;
+  p.walk.bh0 = 0; p.walk.nbh = B * H; p.walk.H = H;
+  p.walk.by_cost = causal ? 2 : 0;
+  p.splits = scratch != nullptr ? flash_fwd_splits(B, H, Sq, Sk) : 1;
+  const int key_tiles = (Sk + kBlockN - 1) / kBlockN;
+  p.tiles_per_split = (key_tiles + p.splits - 1) / p.splits;
+  const int64_t rows = static_cast<int64_t>(B) * H * Sq;
+  p.part_o = scratch;
+  p.part_ml = reinterpret_cast<float2*>(scratch + (p.splits > 1 ? p.splits * rows * D : 0));
   p.scale_log2 = scale * kLog2e; p.causal = causal; p.rng = rng;
   // the dropout probability is quantised to a multiple of 1/128 (see philox_keep16)
   p.thr7 = dropout_thr7(p_drop);
   p.p_drop = p.thr7 / 128.f;
-  p.out_bf16 = bf16 ? 1 : 0; p.status = status;
+  p.status = status;
   p.idesc_qk = tc::instr_desc_f16(128, 128, bf16 ? 1 : 0, false, false);
-  p.idesc_pv = tc::instr_desc_f16(128, Dt, bf16 ? 1 : 0, false, true);
-  const bool plain = kbias == nullptr && rel == nullptr && !causal && Sk % kBlockN == 0 && scale > 0.f;
-  if (Dt == 64)
-    return plain ? launch_fwd_d<64, true>(tq, tk, tv, p, stream)
-                 : launch_fwd_d<64, false>(tq, tk, tv, p, stream);
-  return plain ? launch_fwd_d<128, true>(tq, tk, tv, p, stream)
-               : launch_fwd_d<128, false>(tq, tk, tv, p, stream);
+  // only the columns that exist (a multiple of 16) take part in P V
+  p.idesc_pv = tc::instr_desc_f16(128, p.k_steps * 16, bf16 ? 1 : 0, false, true);
+  const bool general = kbias != nullptr || rel != nullptr || causal || Sk % kBlockN != 0 || !(scale > 0.f);
+  int rc;
+#define FLASH_FWD_CASE(D_, T_)                                            \
+  rc = general ? launch_fwd_d<D_, true, T_>(tq, tk, tv, p, stream)        \
+               : launch_fwd_d<D_, false, T_>(tq, tk, tv, p, stream)
+  if (Dt == 64) {
+    if (bf16) FLASH_FWD_CASE(64, __nv_bfloat16);
+    else FLASH_FWD_CASE(64, __half);
+  } else {
+    if (bf16) FLASH_FWD_CASE(128, __nv_bfloat16);
+    else FLASH_FWD_CASE(128, __half);
+  }
+#undef FLASH_FWD_CASE
+  if (rc != 0 || p.splits == 1) return rc;
+  count_launch();
+  const unsigned blocks = static_cast<unsigned>((rows + 3) / 4);
+  if (bf16)
+    flash_combine_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>(
+        p.part_o, p.part_ml, static_cast<__nv_bfloat16*>(o), lse, p.splits, static_cast<int>(rows),
+        H, Sq, D, 1.f - p.p_drop);
+  else
+    flash_combine_kernel<__half><<<blocks, 128, 0, stream>>>(
+        p.part_o, p.part_ml, static_cast<__half*>(o), lse, p.splits, static_cast<int>(rows), H, Sq,
+        D, 1.f - p.p_drop);
+  return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
 }  // namespace slapo

@@ -1,175 +1,223 @@
 // Flash attention backward on tcgen05 / TMEM (sm_100a).
 //
-// One CTA owns 128 keys of one (batch, head) and walks over the query tiles
-// (128 rows) that can see them.  Per query tile:
-//   tensor core   S  = Q K^T            dP = dO V^T                (fp32 in TMEM)
-//   128 threads   p  = exp2(s - lse),   ds = p * (dp - delta)      (one query row each,
-//                 Philox dropout replayed), P and scale*dS written as 16-bit
-//                 tiles into swizzled shared memory
-//   tensor core   dV += P^T dO          dK += dS^T Q               (TMEM accumulators
-//                 dQ_tile = dS K                                    over all query tiles)
-//   128 threads   dQ_tile -> fp32 partial of this key tile (plain 16-byte stores; the
-//                 conversion kernel sums the partials), or, for very long key sequences,
-//                 a shared fp32 accumulator (vector red.add)
-// The same shared-memory bytes serve as K-major and M/N-major operands: only
-// the descriptors differ, nothing is transposed.  delta = rowsum(dO * O) comes
-// from a small pre-pass; the fp32 dQ accumulator is converted by the caller.
-#include "common.cuh"
+// Two passes of one kernel, each with the same shape as the forward: a work item keeps a
+// 128-row tile of two tensors (X1, X2) in shared memory, streams 128-row tiles of two others
+// (Y1, Y2) and accumulates in tensor memory - nothing is added up between work items.
+//
+//   pass      rows      X1  X2   streams   Y1  Y2     accumulators
+//   dQ        queries   Q   dO   keys      K   V      dQ += dS K
+//   dK / dV   keys      K   V    queries   Q   dO     dK += dS^T Q     dV += P^T dO
+//
+// Per tile, with rows on the TMEM lanes:
+//   tensor core   S = X1 Y1^T ,  dP = X2 Y2^T                       (fp32 in TMEM)
+//   8 warps       p = exp2(s - lse) ;  ds = p * (dp - delta)        (a row and half the columns
+//                 per thread; dropout replayed), P and dS written back to TMEM as 16 bit
+//   tensor core   accumulators += dS Y1 , P Y2                      (A operand from TMEM)
+// P and dS never pass through shared memory, and no transpose is needed: the two passes form
+// S with its rows where they want them.
+//
+// The order of the products keeps the tensor core and the softmax warps apart:
+//   tensor   ... P Y2 (t)   S (t+1)      dS Y1 (t)   dP (t+1) ...
+//   softmax      dS (t)          P (t+1)          dS (t+1)
+// CTAs are persistent; the loads and the first S of the next work item run under the last tile of
+// this one, and its accumulators are read out after the first P of the next.
+//
+// A single pass (5 products per tile instead of 7) has to add up dQ over the key tiles: one fp32
+// partial of dQ per key tile written and read again was most of its time (BERT-large, 32 x 512
+// tokens x 16 heads of 64: 268 MB each way).  Bound now: exp2 (1024 cycles per tile and pass) and
+// the issue slots of the softmax warps.
+//
+// With dropout the dQ pass draws the keep decisions (16 keys of a query row per Philox call, as
+// in the forward) and leaves them as one bit each, [B H][key / 32][query] words, for the dK / dV
+// pass, whose lanes are keys.
+#include "flash_common.cuh"
 #include "kernels.h"
-#include "tc05.cuh"
 
 namespace slapo {
 
-constexpr float kLog2eB = 1.4426950408889634f;
-
 struct FlashBwdParams {
-  int B, H, Sq, Sk;
-  int Dr;               // the tensors' head dimension (<= the tile width D, % 8 == 0)
-  const float* lse;     // [B, H, Sq]
-  const float* delta;   // [B, H, Sq]
-  float* dq_accum;      // [B, Sq, H, Dr] fp32, zero-initialised (dq_slice_stride == 0), or one
-                        // such partial per 128-key tile, written with plain stores
-  int64_t dq_slice_stride;
-  void* dK;             // rows (b, key, head) spaced dkv_row_stride elements apart
-  void* dV;
-  int64_t dkv_row_stride;  // D for contiguous [B, Sk, H, D]; 3 D inside a packed QKV gradient
-  const float* kbias;   // [B, Sk] or nullptr
-  const float* rel;     // [H, Sq + Sk - 1] or nullptr
-  float* drel;          // same shape fp32 accumulator or nullptr
-  float scale, scale_log2;
+  int Sq, Sk, H;
+  int Dr;                 // the tensors' head dimension (<= the tile width D, % 8 == 0)
+  int k_steps;            // ceil(Dr / 16)
+  int Rq, Rk;             // Sq and Sk rounded up to 128
+  TileWalk walk;
+  const float* nlse;      // [B H][Rq]  -log2(e) * lse ; -inf for rows without any key (and padding)
+  const float* ndelta;    // [B H][Rq]  -rowsum(dO O) * keep probability ; 0 in the padding
+  const float* kb2;       // [B][Rk] log2(e) * key bias, 0 in the padding, or nullptr
+  uint32_t* keep;         // [B H of this launch][Rk / 32][Rq] keep bits (dropout), or nullptr
+  const float* rel;       // [H, Sq + Sk - 1] or nullptr
+  float* drel;            // same shape fp32 accumulator or nullptr
+  void* out1;             // dQ or dK: rows (b, s, head) spaced row_stride elements apart
+  void* out2;             // dV
+  int64_t row_stride1, row_stride2;
+  float scale, scale_log2, inv_keep;
   int causal;
-  float p_drop;         // effective probability thr7 / 128
-  uint32_t thr7;
+  uint32_t thr7;          // dropout: keep a draw >= thr7 of 128 ; 0 = no dropout
   PhiloxArgs rng;
-  int bf16;
-  uint32_t idesc_s, idesc_dvk, idesc_dq;
+  uint32_t idesc_s, idesc_acc;
   int* status;
 };
 
-__device__ __forceinline__ uint32_t pack_pair_b(float a, float b, int bf16) {
-  if (bf16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-  __half2 v = __floats2half2_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c),
-               "f"(d)
-               : "memory");
-}
-
-// delta[b, h, i] = sum_d dO[b, i, h, d] * O[b, i, h, d]   (both contiguous [B, Sq, H, Dr]).
-// D / 8 lanes share a row (16-byte loads), D = Dr rounded up to 64 or 128, so a warp covers
-// 256 / D rows; lanes beyond Dr / 8 contribute zero.
+// Row statistics in the layout the kernels read, one launch:
+//   nlse   [B H][Rq]  -log2(e) * lse
+//   ndelta [B H][Rq]  -keep_prob * sum_d dO[b, i, h, d] * O[b, i, h, d]
+// dO and O are contiguous [B, Sq, H, Dr].  A block takes 32 query rows of one batch entry and
+// 8 heads: lanes along d while reading (16-byte loads), then the sums pass through shared
+// memory so that the stores run along the rows.
 template <typename T>
-__global__ void flash_bwd_delta_kernel(const T* __restrict__ dout, const T* __restrict__ out,
-                                       float* __restrict__ delta, int B, int H, int Sq, int D,
-                                       int Dr) {
-  const int lanes_per_row = D >> 3;              // 8 (D = 64) or 16 (D = 128)
-  const int rows_per_warp = 32 / lanes_per_row;
-  const int warps_per_block = blockDim.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int64_t warp_id = static_cast<int64_t>(blockIdx.x) * warps_per_block + (threadIdx.x >> 5);
-  const int64_t row = warp_id * rows_per_warp + lane / lanes_per_row;
-  const int64_t rows = static_cast<int64_t>(B) * Sq * H;
-  float s = 0.f;
-  const int d = (lane % lanes_per_row) * 8;
-  if (row < rows && d < Dr) {
-    float a[8], b[8];
-    Vec8<T>::load(dout + row * Dr + d, a);
-    Vec8<T>::load(out + row * Dr + d, b);
+__global__ void __launch_bounds__(256) flash_bwd_stats_kernel(
+    const T* __restrict__ dout, const T* __restrict__ out, const float* __restrict__ lse,
+    float* __restrict__ nlse, float* __restrict__ ndelta, int H, int Sq, int Rq, int Dr, int lanes,
+    float keep_prob) {
+  __shared__ float sums[8][33];
+  const int i0 = blockIdx.x * 32, h0 = blockIdx.y * 8, b = blockIdx.z;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rows_per_warp = 32 / lanes;        // `lanes` (8 or 16) threads share a row of Dr
+  const int d = (lane % lanes) * 8;
+  for (int r = warp * rows_per_warp + lane / lanes; r < 256; r += 8 * rows_per_warp) {
+    const int i = i0 + (r >> 3), h = h0 + (r & 7);    // neighbouring heads are contiguous
+    float s = 0.f;
+    if (i < Sq && h < H && d < Dr) {
+      const int64_t at = ((static_cast<int64_t>(b) * Sq + i) * H + h) * Dr + d;
+      float x[8], y[8];
+      Vec8<T>::load(dout + at, x);
+      Vec8<T>::load(out + at, y);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) s += a[k] * b[k];
+      for (int k = 0; k < 8; ++k) s += x[k] * y[k];
+    }
+    for (int o = lanes >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane % lanes == 0) sums[r & 7][r >> 3] = s;
   }
-  for (int o = lanes_per_row >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (row < rows && lane % lanes_per_row == 0) {
-    const int h = static_cast<int>(row % H);
-    const int64_t bi = row / H;
-    const int i = static_cast<int>(bi % Sq);
-    const int b = static_cast<int>(bi / Sq);
-    delta[(static_cast<int64_t>(b) * H + h) * Sq + i] = s;
+  __syncthreads();
+  const int h = h0 + warp, i = i0 + lane;
+  if (h < H && i < Rq) {
+    const int64_t bh = static_cast<int64_t>(b) * H + h;
+    float nl = -INFINITY;
+    if (i < Sq) {
+      const float l = lse[bh * Sq + i];
+      nl = l == -INFINITY ? -INFINITY : -l * kLog2e;
+    }
+    nlse[bh * Rq + i] = nl;
+    ndelta[bh * Rq + i] = i < Sq ? -sums[warp][lane] * keep_prob : 0.f;
   }
 }
 
-// 10 warps: TMA, MMA and 8 softmax warps.  Softmax warps w and w + 4 share a quarter of the
-// TMEM lanes (query rows) and split the 128 key columns (and later the D output columns)
-// in halves, so every scheduler of the SM has two of them to interleave.
-// kPlain: no key bias / relative bias, not causal, Sq and Sk multiples of 128.
-template <int D, bool kPlain>
+// kb2 [B][Rk] = log2(e) * key bias, padded with zeros
+__global__ void __launch_bounds__(256) flash_bwd_bias_kernel(const float* __restrict__ kbias,
+                                                             float* __restrict__ kb2, int Sk,
+                                                             int Rk) {
+  const int key = blockIdx.x * 256 + threadIdx.x, b = blockIdx.y;
+  if (key < Rk)
+    kb2[static_cast<int64_t>(b) * Rk + key] =
+        key < Sk ? kbias[static_cast<int64_t>(b) * Sk + key] * kLog2e : 0.f;
+}
+
+template <int D, bool kKeys>
+struct BwdSmem {
+  static constexpr int kTile = 128 * D * 2;
+  static constexpr int kStages = D == 64 ? 3 : 2;
+  // per stage: Y1, Y2 and the column vectors: nlse, ndelta (512 B each) and four rows of keep
+  // bits (2 KB) for the dK / dV pass, the key bias (512 B) for the dQ pass
+  static constexpr int kVec = kKeys ? 1024 + 2048 : 1024;
+  static constexpr int kY = 2 * kTile;
+  static constexpr int kVecs = kY + kStages * 2 * kTile;
+  static constexpr int kDrel = kVecs + kStages * kVec;       // [8 warps][64] floats
+  static constexpr int kBars = kDrel + (kKeys ? 8 * 64 * 4 : 0);
+  static constexpr int kTotal = kBars + 24 * 8 + 1024;
+};
+
+// 10 warps: TMA, MMA and 8 softmax warps; warps w and w + 4 share a quarter of the TMEM lanes
+// (rows) and split the tile's columns in halves.
+// kKeys: the dK / dV pass.  kGeneral: key bias, relative bias, causal mask or ragged lengths.
+template <int D, bool kKeys, bool kGeneral, typename T>
 __global__ void __launch_bounds__(320, 1)
-flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ CUtensorMap tm_x2,
+                 const __grid_constant__ CUtensorMap tm_y1, const __grid_constant__ CUtensorMap tm_y2,
                  const FlashBwdParams p) {
-  constexpr int kTileBytes = 128 * D * 2;
+  using L = BwdSmem<D, kKeys>;
+  constexpr int kTileBytes = L::kTile;
   constexpr int kBlkBytes = 128 * 128;
   constexpr int kDBlocks = D / 64;
-  constexpr int kStages = D == 64 ? 2 : 1;
-  // D = 64: two P / dS buffers, so that the softmax warps write the tiles of query block j + 1
-  // while the tensor core still reads those of block j (dV, dK, dQ); D = 128 has no room
-  constexpr int kPB = D == 64 ? 2 : 1;
+  constexpr int kStages = L::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* s_k = smem;
-  uint8_t* s_v = s_k + kTileBytes;
-  uint8_t* s_q = s_v + kTileBytes;                  // kStages
-  uint8_t* s_do = s_q + kStages * kTileBytes;       // kStages
-  uint8_t* s_p = s_do + kStages * kTileBytes;       // kPB buffers of [P: 2 blocks | dS: 2 blocks]
-  uint8_t* s_ds = s_p + 2 * kBlkBytes;
-  constexpr int kPdsBytes = 4 * kBlkBytes;          // distance between the P / dS buffers
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_p + kPB * kPdsBytes);
-  uint64_t* kv_full = bars;            // 1
-  uint64_t* qdo_full = bars + 1;       // kStages (<= 2)
-  uint64_t* qdo_empty = bars + 3;      // kStages
-  uint64_t* sdp_full = bars + 5;
-  uint64_t* pds_full = bars + 6;       // 4 arrivals
-  uint64_t* dq_full = bars + 7;
-  uint64_t* dq_empty = bars + 8;       // 4 arrivals
-  uint64_t* acc_full = bars + 9;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  uint8_t* s_x1 = smem;
+  uint8_t* s_x2 = smem + kTileBytes;
+  uint8_t* s_y = smem + L::kY;            // [stage][Y1 | Y2]
+  uint8_t* s_vec = smem + L::kVecs;       // [stage][kVec]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
+  uint64_t* x1_full = bars;
+  uint64_t* x1_empty = bars + 1;
+  uint64_t* x2_full = bars + 2;
+  uint64_t* x2_empty = bars + 3;
+  uint64_t* y_full = bars + 4;      // kStages (<= 3)
+  uint64_t* y_empty = bars + 7;     // kStages
+  uint64_t* s_full = bars + 10;
+  uint64_t* p_ready = bars + 11;    // 8 warps: S has been read (and P written over it)
+  uint64_t* dp_full = bars + 12;
+  uint64_t* ds_ready = bars + 13;   // 8 warps: dS written over dP
+  uint64_t* acc_full = bars + 14;
+  uint64_t* acc_free = bars + 15;   // 8 warps
+  uint64_t* a1_done = bars + 16;    // the tensor core has read dS / P of a tile
+  uint64_t* a2_done = bars + 17;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* kb_tile = reinterpret_cast<float*>(bars + 12);  // 128 floats
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * 128;
-  const int head = blockIdx.y, batch = blockIdx.z;
   const int diag = p.Sk - p.Sq;
-  const int q_tiles = (p.Sq + 127) / 128;
-  int i_begin = 0;
-  if (p.causal) i_begin = max(0, (n0 - diag) / 128);
-  i_begin = min(i_begin, q_tiles);
-  const int n_iter = q_tiles - i_begin;
-
   constexpr uint32_t kTmemCols = 512;
-  constexpr uint32_t kColS = 0, kColDP = 128, kColDV = 256, kColDK = 256 + D;
-  constexpr uint32_t kColDQ = D == 64 ? 384 : 0;  // D = 128: dQ reuses the S columns
+  constexpr uint32_t kColS = 0, kColDP = 128, kColA1 = 256, kColA2 = 256 + D;
+  // P and dS get columns of their own where 512 suffice; for D = 128 the dK / dV pass writes them
+  // over S and dP (each warp over the half it has read: halves start 64 columns apart).
+  // Products of one thread run in order for ONE accumulator only: a product that overwrites the
+  // A operand of the one before it has to wait for that one's completion.
+  constexpr bool kOver = kKeys && D == 128;
+  constexpr uint32_t kColP = kOver ? kColS : 384, kColDS = kOver ? kColDP : (kKeys ? 448 : 256 + D);
+  constexpr uint32_t kHalf = kOver ? 64 : 32;    // columns from one half of P / dS to the other
+  const int items = p.walk.items();
+  const bool drop = p.thr7 != 0;
+
+  // first streamed tile of a row tile, and how many (at least one: a row tile that nothing
+  // reaches still has its zeros written)
+  auto tiles_of = [&](int tile, int& first) {
+    int n;
+    if constexpr (kKeys) {
+      const int q_tiles = p.Rq >> 7;
+      first = 0;
+      if (p.causal) first = min(max(0, (tile * 128 - diag) / 128), q_tiles - 1);
+      n = q_tiles - first;
+    } else {
+      first = 0;
+      n = p.Rk >> 7;
+      if (p.causal) n = max(1, min(n, (min(p.Sk, tile * 128 + 128 + diag) + 127) / 128));
+    }
+    return n;
+  };
 
   if (threadIdx.x == 0) {
-    tc::mbar_init(kv_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      tc::mbar_init(&qdo_full[s], 1);
-      tc::mbar_init(&qdo_empty[s], 1);
+    tc::mbar_init(x1_full, 1);
+    tc::mbar_init(x1_empty, 1);
+    tc::mbar_init(x2_full, 1);
+    tc::mbar_init(x2_empty, 1);
+    for (int s = 0; s < 3; ++s) {
+      tc::mbar_init(&y_full[s], 1);
+      tc::mbar_init(&y_empty[s], 1);
     }
-    tc::mbar_init(sdp_full, 1);
-    tc::mbar_init(pds_full, 8);
-    tc::mbar_init(dq_full, 1);
-    tc::mbar_init(dq_empty, 8);
+    tc::mbar_init(s_full, 1);
+    tc::mbar_init(p_ready, 8);
+    tc::mbar_init(dp_full, 1);
+    tc::mbar_init(ds_ready, 8);
     tc::mbar_init(acc_full, 1);
+    tc::mbar_init(acc_free, 8);
+    tc::mbar_init(a1_done, 1);
+    tc::mbar_init(a2_done, 1);
     *abort_flag = 0;
     tc::fence_barrier_init();
   }
   if (warp == 1) {
     tc::tmem_alloc(tmem_slot, kTmemCols);
     tc::tmem_relinquish();
-  }
-  if (warp >= 2 && warp < 6) {
-    const int t = (warp - 2) * 32 + lane;
-    const int key = n0 + t;
-    kb_tile[t] = (p.kbias != nullptr && key < p.Sk)
-                     ? p.kbias[static_cast<int64_t>(batch) * p.Sk + key] * kLog2eB : 0.f;
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -178,298 +226,467 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
   if (warp == 0) {
     if (lane == 0) {
-      tc::tma_prefetch_desc(&tm_q);
-      tc::tma_prefetch_desc(&tm_do);
-      tc::mbar_arrive_expect_tx(kv_full, 2 * kTileBytes);
-#pragma unroll
-      for (int d = 0; d < kDBlocks; ++d) {
-        tc::tma_load_4d(s_k + d * kBlkBytes, &tm_k, kv_full, d * 64, head, n0, batch);
-        tc::tma_load_4d(s_v + d * kBlkBytes, &tm_v, kv_full, d * 64, head, n0, batch);
-      }
+      tc::tma_prefetch_desc(&tm_x1);
+      tc::tma_prefetch_desc(&tm_x2);
+      tc::tma_prefetch_desc(&tm_y1);
+      tc::tma_prefetch_desc(&tm_y2);
+      const uint32_t vec_bytes = kKeys ? 1024u + (drop ? 2048u : 0u) : (p.kb2 != nullptr ? 512u : 0u);
       bool ok = true;
-      for (int it = 0; it < n_iter && ok; ++it) {
-        const int st = it % kStages;
-        const uint32_t ph = (it / kStages) & 1;
-        if (!tc::mbar_wait(&qdo_empty[st], ph ^ 1, abort_flag)) { ok = false; break; }
-        tc::mbar_arrive_expect_tx(&qdo_full[st], 2 * kTileBytes);
-        const int m0 = (i_begin + it) * 128;
+      int t = 0, w = 0;
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++w) {
+        int tile, bhl, first;
+        p.walk.at(item, tile, bhl);
+        const int bh = p.walk.bh0 + bhl;
+        const int batch = bh / p.H, head = bh - batch * p.H;
+        const int n = tiles_of(tile, first);
+        auto load_y = [&](int j) -> bool {
+          const int st = t % kStages;
+          const uint32_t ph = ((t / kStages) & 1) ^ 1;
+          if (!tc::mbar_wait(&y_empty[st], ph, abort_flag)) return false;
+          // (the stage's column vectors were read before ds_ready, which y_empty follows)
+          tc::mbar_arrive_expect_tx(&y_full[st], 2 * kTileBytes + vec_bytes);
+          const int s0 = (first + j) * 128;
+          uint8_t* y = s_y + st * 2 * kTileBytes;
 #pragma unroll
-        for (int d = 0; d < kDBlocks; ++d) {
-          tc::tma_load_4d(s_q + st * kTileBytes + d * kBlkBytes, &tm_q, &qdo_full[st], d * 64, head,
-                          m0, batch);
-          tc::tma_load_4d(s_do + st * kTileBytes + d * kBlkBytes, &tm_do, &qdo_full[st], d * 64,
-                          head, m0, batch);
-        }
+          for (int d = 0; d < kDBlocks; ++d)
+            tc::tma_load_4d(y + d * kBlkBytes, &tm_y1, &y_full[st], d * 64, head, s0, batch);
+#pragma unroll
+          for (int d = 0; d < kDBlocks; ++d)
+            tc::tma_load_4d(y + kTileBytes + d * kBlkBytes, &tm_y2, &y_full[st], d * 64, head, s0,
+                            batch);
+          uint8_t* v = s_vec + st * L::kVec;
+          if constexpr (kKeys) {
+            tc::bulk_load(v, p.nlse + static_cast<int64_t>(bh) * p.Rq + s0, 512, &y_full[st]);
+            tc::bulk_load(v + 512, p.ndelta + static_cast<int64_t>(bh) * p.Rq + s0, 512, &y_full[st]);
+            if (drop)
+#pragma unroll
+              for (int r = 0; r < 4; ++r)
+                tc::bulk_load(v + 1024 + r * 512,
+                              p.keep + (static_cast<int64_t>(bhl) * (p.Rk >> 5) + tile * 4 + r) * p.Rq + s0,
+                              512, &y_full[st]);
+          } else {
+            if (vec_bytes != 0)
+              tc::bulk_load(v, p.kb2 + static_cast<int64_t>(batch) * p.Rk + s0, 512, &y_full[st]);
+          }
+          return true;
+        };
+        if (!tc::mbar_wait(x1_empty, (w & 1) ^ 1, abort_flag)) { ok = false; break; }
+        tc::mbar_arrive_expect_tx(x1_full, kTileBytes);
+#pragma unroll
+        for (int d = 0; d < kDBlocks; ++d)
+          tc::tma_load_4d(s_x1 + d * kBlkBytes, &tm_x1, x1_full, d * 64, head, tile * 128, batch);
+        if (!load_y(0)) { ok = false; break; }
+        ++t;
+        if (!tc::mbar_wait(x2_empty, (w & 1) ^ 1, abort_flag)) { ok = false; break; }
+        tc::mbar_arrive_expect_tx(x2_full, kTileBytes);
+#pragma unroll
+        for (int d = 0; d < kDBlocks; ++d)
+          tc::tma_load_4d(s_x2 + d * kBlkBytes, &tm_x2, x2_full, d * 64, head, tile * 128, batch);
+        for (int j = 1; j < n; ++j, ++t)
+          if (!load_y(j)) { ok = false; break; }
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      bool ok = tc::mbar_wait(kv_full, 0, abort_flag);
-      const uint32_t k_addr = tc::smem_u32(s_k), v_addr = tc::smem_u32(s_v);
-      const uint32_t p_addr = tc::smem_u32(s_p), ds_addr = tc::smem_u32(s_ds);
-      auto issue_s_dp = [&](int it) -> bool {
-        const int st = it % kStages;
-        if (!tc::mbar_wait(&qdo_full[st], (it / kStages) & 1, abort_flag)) return false;
-        if (D == 128 && it > 0 && !tc::mbar_wait(dq_empty, (it - 1) & 1, abort_flag)) return false;
+      const uint32_t x1_addr = tc::smem_u32(s_x1), x2_addr = tc::smem_u32(s_x2);
+      // S / dP of tile t, which belongs to this CTA's w-th item
+      auto scores = [&](uint32_t col, uint32_t a_addr, uint32_t b_addr) {
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+          if (kk < p.k_steps) {
+            const uint32_t off = (kk >> 2) * kBlkBytes + (kk & 3) * 32;
+            tc::umma_f16(tmem_base + col, tc::smem_desc(a_addr + off, 16, 1024),
+                         tc::smem_desc(b_addr + off, 16, 1024), p.idesc_s, kk != 0 ? 1u : 0u);
+          }
+        }
+      };
+      // accumulator += [128 rows x 128 streamed] 16-bit tile in TMEM times Y
+      auto accumulate = [&](uint32_t col, uint32_t a_col, uint32_t y_addr, bool fresh) {
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          tc::umma_f16_ts(tmem_base + col, tmem_base + a_col + (kk >> 2) * kHalf + (kk & 3) * 8,
+                          tc::smem_desc(y_addr + kk * 2048, kBlkBytes, 1024), p.idesc_acc,
+                          (fresh && kk == 0) ? 0u : 1u);
+      };
+      auto issue_s = [&](int t, int w, bool first, bool last) -> bool {
+        const int st = t % kStages;
+        if (first && !tc::mbar_wait(x1_full, w & 1, abort_flag)) return false;
+        if (!tc::mbar_wait(&y_full[st], (t / kStages) & 1, abort_flag)) return false;
         tc::fence_after_sync();
-        const uint32_t q_addr = tc::smem_u32(s_q + st * kTileBytes);
-        const uint32_t do_addr = tc::smem_u32(s_do + st * kTileBytes);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * kBlkBytes + (kk & 3) * 32;
-          tc::umma_f16(tmem_base + kColS, tc::smem_desc(q_addr + off, 16, 1024),
-                       tc::smem_desc(k_addr + off, 16, 1024), p.idesc_s, kk != 0 ? 1u : 0u);
-        }
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * kBlkBytes + (kk & 3) * 32;
-          tc::umma_f16(tmem_base + kColDP, tc::smem_desc(do_addr + off, 16, 1024),
-                       tc::smem_desc(v_addr + off, 16, 1024), p.idesc_s, kk != 0 ? 1u : 0u);
-        }
-        tc::umma_commit(sdp_full);
+        scores(kColS, x1_addr, tc::smem_u32(s_y + st * 2 * kTileBytes));
+        tc::umma_commit(s_full);
+        if (last) tc::umma_commit(x1_empty);
         return true;
       };
-      if (ok && n_iter > 0) ok = issue_s_dp(0);
-      for (int it = 0; it < n_iter && ok; ++it) {
-        const int st = it % kStages;
-        if (!tc::mbar_wait(pds_full, it & 1, abort_flag)) { ok = false; break; }
+      auto issue_dp = [&](int t, int w, bool first, bool last) -> bool {
+        const int st = t % kStages;
+        if (first && !tc::mbar_wait(x2_full, w & 1, abort_flag)) return false;
         tc::fence_after_sync();
-        if constexpr (kPB == 2) {
-          // S / dP of the next query block first: the softmax warps have taken block `it` out
-          // of tensor memory, and their work on block it + 1 then runs under the three
-          // products of block `it` below (which read the other P / dS buffer)
-          if (it + 1 < n_iter && !issue_s_dp(it + 1)) { ok = false; break; }
+        scores(kColDP, x2_addr, tc::smem_u32(s_y + st * 2 * kTileBytes + kTileBytes));
+        tc::umma_commit(dp_full);
+        if (last) tc::umma_commit(x2_empty);
+        return true;
+      };
+      auto n_of = [&](int item) {
+        if (item >= items) return 0;
+        int tile, bhl, first;
+        p.walk.at(item, tile, bhl);
+        return tiles_of(tile, first);
+      };
+      bool ok = true;
+      int t = 0, w = 0, item = blockIdx.x;
+      int n = n_of(item);
+      if (n > 0) ok = issue_s(0, 0, true, n == 1) && issue_dp(0, 0, true, n == 1);
+      while (item < items && ok) {
+        const int next_item = item + gridDim.x;
+        const int next_n = n_of(next_item);
+        for (int j = 0; j < n; ++j, ++t) {
+          const int st = t % kStages;
+          const uint32_t y_addr = tc::smem_u32(s_y + st * 2 * kTileBytes);
+          const bool same = j + 1 < n, more = same || next_n > 0;
+          const bool next_last = same ? j + 2 == n : next_n == 1;
+          if (!tc::mbar_wait(p_ready, t & 1, abort_flag)) { ok = false; break; }
+          if constexpr (kKeys) {
+            // the accumulators of the item before have been read out
+            if (j == 0 && !tc::mbar_wait(acc_free, (w & 1) ^ 1, abort_flag)) { ok = false; break; }
+            tc::fence_after_sync();
+            accumulate(kColA2, kColP, y_addr + kTileBytes, j == 0);
+            tc::umma_commit(a2_done);
+            if (kOver && more && !tc::mbar_wait(a2_done, t & 1, abort_flag)) { ok = false; break; }
+          }
+          if (more && !issue_s(t + 1, same ? w : w + 1, !same, next_last)) { ok = false; break; }
+          if (!tc::mbar_wait(ds_ready, t & 1, abort_flag)) { ok = false; break; }
+          if constexpr (!kKeys) {
+            if (j == 0 && !tc::mbar_wait(acc_free, (w & 1) ^ 1, abort_flag)) { ok = false; break; }
+          }
+          tc::fence_after_sync();
+          accumulate(kColA1, kColDS, y_addr, j == 0);
+          tc::umma_commit(a1_done);
+          tc::umma_commit(&y_empty[st]);
+          if (j + 1 == n) tc::umma_commit(acc_full);
+          if (kOver && more && !tc::mbar_wait(a1_done, t & 1, abort_flag)) { ok = false; break; }
+          if (more && !issue_dp(t + 1, same ? w : w + 1, !same, next_last)) { ok = false; break; }
         }
-        if (D == 64 && it > 0 && !tc::mbar_wait(dq_empty, (it - 1) & 1, abort_flag)) { ok = false; break; }
-        tc::fence_after_sync();
-        const uint32_t q_addr = tc::smem_u32(s_q + st * kTileBytes);
-        const uint32_t do_addr = tc::smem_u32(s_do + st * kTileBytes);
-        const uint32_t pb_addr = p_addr + (it % kPB) * kPdsBytes;
-        const uint32_t dsb_addr = ds_addr + (it % kPB) * kPdsBytes;
-        // dV += P^T dO ; dK += dS^T Q : A = [q rows x keys] read M-major (M = keys, K = q rows),
-        // B = [q rows x D] read N-major.  16 query rows per instruction.
-#pragma unroll
-        for (int kk = 0; kk < 128 / 16; ++kk) {
-          const uint64_t b_do = tc::smem_desc(do_addr + kk * 2048, kBlkBytes, 1024);
-          const uint64_t b_q = tc::smem_desc(q_addr + kk * 2048, kBlkBytes, 1024);
-          const uint64_t a_p = tc::smem_desc(pb_addr + kk * 2048, kBlkBytes, 1024);
-          const uint64_t a_ds = tc::smem_desc(dsb_addr + kk * 2048, kBlkBytes, 1024);
-          const uint32_t accum = (it | kk) != 0 ? 1u : 0u;
-          tc::umma_f16(tmem_base + kColDV, a_p, b_do, p.idesc_dvk, accum);
-          tc::umma_f16(tmem_base + kColDK, a_ds, b_q, p.idesc_dvk, accum);
-        }
-        // dQ_tile = dS K : A = dS K-major (M = q rows, K = keys), B = K read N-major
-#pragma unroll
-        for (int kk = 0; kk < 128 / 16; ++kk) {
-          const uint64_t a_ds =
-              tc::smem_desc(dsb_addr + (kk >> 2) * kBlkBytes + (kk & 3) * 32, 16, 1024);
-          const uint64_t b_k = tc::smem_desc(k_addr + kk * 2048, kBlkBytes, 1024);
-          tc::umma_f16(tmem_base + kColDQ, a_ds, b_k, p.idesc_dq, kk != 0 ? 1u : 0u);
-        }
-        tc::umma_commit(dq_full);
-        tc::umma_commit(&qdo_empty[st]);
-        if constexpr (kPB == 1) {
-          if (it + 1 < n_iter && !issue_s_dp(it + 1)) { ok = false; break; }
-        }
+        item = next_item;
+        n = next_n;
+        ++w;
       }
-      if (ok) tc::umma_commit(acc_full);
     }
   } else {
+    // ------------------------------ softmax warps ------------------------------
     const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;   // which 64 of the 128 key columns / which output half
+    const int half = (warp - 2) >> 2;   // which 64 of the tile's 128 columns
     const int r_in = quarter * 32 + lane;
-    const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     uint64_t seed = 0, offset = 0;
-    if (p.p_drop > 0.f) philox_unpack(p.rng, seed, offset);
+    if (!kKeys && drop) philox_unpack(p.rng, seed, offset);
     const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
-    const float keep_prob = 1.f - p.p_drop;
-    const float inv_keep = 1.f / keep_prob;
+    const int sk16 = (p.Sk + 15) >> 4;
     // dS is formed without the factors scale and 1 / keep_prob; they are applied once to
     // dQ and dK (and 1 / keep_prob to dV) when those leave TMEM
-    const float out_scale = p.scale * inv_keep;
-    const int sk16 = (p.Sk + 15) >> 4;
-    bool ok = true;
-    // dQ tile of query block `j`: out of tensor memory into this key tile's fp32 partial.
-    // Reductions into one accumulator run at the rate of the L2 atomic units; each key tile
-    // stores into its own partial instead (the conversion kernel adds them up).
-    auto dq_readout = [&](int j) -> bool {
-      if (!tc::mbar_wait_warp(dq_full, j & 1, abort_flag)) return false;
+    const float out_scale = p.scale * p.inv_keep;
+    const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
+
+    // accumulators of work item `item` out of tensor memory
+    auto read_out = [&](int item) {
+      int tile, bhl;
+      p.walk.at(item, tile, bhl);
+      const int bh = p.walk.bh0 + bhl;
+      const int batch = bh / p.H, head = bh - batch * p.H;
+      const int row = tile * 128 + r_in;
+      const int rows = kKeys ? p.Sk : p.Sq;
+      // dK / dV pass: the first four warps write dV, the others dK; dQ pass: half the columns each
+      const bool second = kKeys && half == 0;
+      const float f = second ? p.inv_keep : out_scale;
+      const int64_t at = (static_cast<int64_t>(batch) * rows + min(row, rows - 1)) * p.H + head;
+      T* dst = second ? static_cast<T*>(p.out2) + at * p.row_stride2
+                      : static_cast<T*>(p.out1) + at * p.row_stride1;
+      const int c0 = kKeys ? 0 : half * (D / 2);
+      const uint32_t col = second ? kColA2 : kColA1;
       tc::fence_after_sync();
-      const int row = (i_begin + j) * 128 + r_in;
-      const bool row_ok = row < p.Sq;
-      const bool dq_sliced = p.dq_slice_stride != 0;
-      float* dq_dst = p.dq_accum + static_cast<int64_t>(blockIdx.x) * p.dq_slice_stride +
-                      ((static_cast<int64_t>(batch) * p.Sq + min(row, p.Sq - 1)) * p.H + head) * p.Dr;
 #pragma unroll
-      for (int cc = 0; cc < D / 64; ++cc) {
-        const int c = half * (D / 64) + cc;   // this warp's share of the D columns
+      for (int c = 0; c < (kKeys ? D : D / 2); c += 32) {
         uint32_t r[32];
-        tc::tmem_ld_x32(tmem_base + kColDQ + c * 32 + lane_sel, r);
+        tc::tmem_ld_x32(tmem_row + col + c0 + c, r);
         tc::tmem_ld_wait();
-        if (row_ok) {
+        if (row < rows) {
 #pragma unroll
-          for (int g = 0; g < 8; ++g) {
-            if (c * 32 + g * 4 >= p.Dr) break;
-            const float4 val = make_float4(__uint_as_float(r[g * 4]) * out_scale,
-                                           __uint_as_float(r[g * 4 + 1]) * out_scale,
-                                           __uint_as_float(r[g * 4 + 2]) * out_scale,
-                                           __uint_as_float(r[g * 4 + 3]) * out_scale);
-            if (dq_sliced) *reinterpret_cast<float4*>(dq_dst + c * 32 + g * 4) = val;
-            else red_add_v4(dq_dst + c * 32 + g * 4, val.x, val.y, val.z, val.w);
+          for (int g = 0; g < 4; ++g) {
+            if (c0 + c + g * 8 < p.Dr) {
+              uint32_t v[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                v[i] = pack16<T>(__uint_as_float(r[g * 8 + 2 * i]) * f,
+                                 __uint_as_float(r[g * 8 + 2 * i + 1]) * f);
+              *reinterpret_cast<uint4*>(dst + c0 + c + g * 8) = make_uint4(v[0], v[1], v[2], v[3]);
+            }
           }
         }
       }
       tc::fence_before_sync();
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(dq_empty);
-      return true;
+      if (lane == 0) tc::mbar_arrive(acc_free);
     };
-    for (int it = 0; it < n_iter && ok; ++it) {
-      const int row = (i_begin + it) * 128 + r_in;
-      const bool row_ok = row < p.Sq;
-      const int64_t stat_idx = (static_cast<int64_t>(batch) * p.H + head) * p.Sq + min(row, p.Sq - 1);
-      const float lse2 = row_ok ? p.lse[stat_idx] * kLog2eB : -INFINITY;
-      const float delta = row_ok ? p.delta[stat_idx] * keep_prob : 0.f;
-      const uint64_t drop_row_base = static_cast<uint64_t>(stat_idx) * sk16;
-      const float* rel_row = nullptr;
-      float* drel_row = nullptr;
-      if (p.rel != nullptr) {
-        const int64_t base = static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + (p.Sq - 1) - min(row, p.Sq - 1);
-        rel_row = p.rel + base;
-        if (p.drel != nullptr) drel_row = p.drel + base;
+
+    // per-row scalars of a work item: the dQ pass's statistics, the dK / dV pass's key bias
+    auto row_scalars = [&](int item, float& a, float& b) {
+      a = 0.f;
+      b = 0.f;
+      if (item >= items) return;
+      int tile, bhl;
+      p.walk.at(item, tile, bhl);
+      const int bh = p.walk.bh0 + bhl;
+      if constexpr (kKeys) {
+        if (kGeneral && p.kb2 != nullptr)
+          a = p.kb2[static_cast<int64_t>(bh / p.H) * p.Rk + tile * 128 + r_in];
+      } else {
+        a = p.nlse[static_cast<int64_t>(bh) * p.Rq + tile * 128 + r_in];
+        b = p.ndelta[static_cast<int64_t>(bh) * p.Rq + tile * 128 + r_in];
       }
-      int key_limit = p.Sk;
-      if (p.causal) key_limit = min(key_limit, row + diag + 1);
-      if (!row_ok || lse2 == -INFINITY) key_limit = 0;
-      if (!tc::mbar_wait_warp(sdp_full, it & 1, abort_flag)) { ok = false; break; }
-      tc::fence_after_sync();
-      uint8_t* p_row = s_p + (it % kPB) * kPdsBytes + r_in * 128;
-      uint8_t* ds_row = s_ds + (it % kPB) * kPdsBytes + r_in * 128;
-#pragma unroll 1
-      for (int c = 2 * half; c < 2 * half + 2; ++c) {
-        uint32_t s_raw[32], dp_raw[32];
-        tc::tmem_ld_x32(tmem_base + kColS + c * 32 + lane_sel, s_raw);
-        tc::tmem_ld_x32(tmem_base + kColDP + c * 32 + lane_sel, dp_raw);
-        tc::tmem_ld_wait();
-        float pv[32], dsv[32];
-        if constexpr (kPlain) {
+    };
+
+    bool ok = true;
+    int t = 0, w = 0, prev_item = -1;
+    float rs_a, rs_b;
+    row_scalars(blockIdx.x, rs_a, rs_b);
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++w) {
+      int tile, bhl, first;
+      p.walk.at(item, tile, bhl);
+      const int bh = p.walk.bh0 + bhl;
+      const int head = bh % p.H;
+      const int row = tile * 128 + r_in;
+      const int n = tiles_of(tile, first);
+      const float row_a = rs_a, row_b = rs_b;
+      row_scalars(item + gridDim.x, rs_a, rs_b);      // under this item's work
+      const uint64_t ra2 = f2_pack(row_a, row_a), rb2 = f2_pack(row_b, row_b);
+      for (int j = 0; j < n; ++j, ++t) {
+        const int st = t % kStages;
+        const int col0 = (first + j) * 128 + half * 64;     // this thread's first column
+        const uint8_t* vec = s_vec + st * L::kVec;
+        // ---- dropout decisions of this row and the thread's 64 keys (dQ pass) ----
+        uint32_t keep16[4][4];
+        if (!kKeys && drop) {
+          const uint64_t base = (static_cast<uint64_t>(bh) * p.Sq + min(row, p.Sq - 1)) * sk16 + (col0 >> 4);
+          uint32_t bits[2];
 #pragma unroll
-          for (int t = 0; t < 32; ++t)
-            pv[t] = exp2f(fmaf(__uint_as_float(s_raw[t]), p.scale_log2, -lse2));
-        } else {
+          for (int g = 0; g < 4; ++g) {
+            const uint4 kw = philox_keep16(seed, offset, base + g, add4);
+            keep16[g][0] = kw.x; keep16[g][1] = kw.y; keep16[g][2] = kw.z; keep16[g][3] = kw.w;
+            uint32_t m = 0;
 #pragma unroll
-          for (int t = 0; t < 32; ++t) {
-            const int key = n0 + c * 32 + t;
-            float s2 = __uint_as_float(s_raw[t]) * p.scale_log2 + kb_tile[c * 32 + t];
-            if (rel_row != nullptr) s2 += rel_row[key] * kLog2eB;
-            pv[t] = key < key_limit ? exp2f(s2 - lse2) : 0.f;
+            for (int i = 0; i < 4; ++i)     // bit 7 of the four bytes, gathered by one multiply
+              m |= ((((keep16[g][i] >> 7) & 0x01010101u) * 0x01020408u) >> 24) << (4 * i);
+            if (g & 1) bits[g >> 1] |= m << 16;
+            else bits[g >> 1] = m;
+          }
+          uint32_t* dst = p.keep + (static_cast<int64_t>(bhl) * (p.Rk >> 5) + (col0 >> 5)) * p.Rq + row;
+          dst[0] = bits[0];
+          dst[p.Rq] = bits[1];
+        }
+        // ---- P ----
+        if (!tc::mbar_wait_warp(s_full, t & 1, abort_flag)) { ok = false; break; }
+        // (complete since before s_full; waiting on it makes the column vectors visible)
+        if (!tc::mbar_wait_warp(&y_full[st], (t / kStages) & 1, abort_flag)) { ok = false; break; }
+        tc::fence_after_sync();
+        float pr[64];
+        {
+          uint32_t s0[32], s1[32];
+          tc::tmem_ld_x32(tmem_row + kColS + half * 64, s0);
+          tc::tmem_ld_x32(tmem_row + kColS + half * 64 + 32, s1);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            pr[i] = __uint_as_float(s0[i]);
+            pr[32 + i] = __uint_as_float(s1[i]);
           }
         }
-        if (p.p_drop > 0.f) {
+        if constexpr (!kKeys) {
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(p_ready);
+        }
+        {
+          const float4* cv = reinterpret_cast<const float4*>(vec) + half * 16;
+          const bool cols = kKeys || (kGeneral && p.kb2 != nullptr);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint4 kw = philox_keep16(seed, offset,
-                                           drop_row_base + ((n0 + c * 32 + h * 16) >> 4), add4);
-            const uint32_t w[4] = {kw.x, kw.y, kw.z, kw.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const int e = h * 16 + i * 4 + j;
-                const float pr = pv[e];
-                // kept probability (zero where dropped); dS / keep_prob = P (mask dP - delta')
-                const float pm = __uint_as_float(__float_as_uint(pr) & keep_mask_full(w[i], j));
-                dsv[e] = fmaf(pm, __uint_as_float(dp_raw[e]), -pr * delta);
-                pv[e] = pm;
+          for (int i = 0; i < 64; i += 4) {
+            uint64_t x0 = f2_pack(pr[i], pr[i + 1]), x1 = f2_pack(pr[i + 2], pr[i + 3]);
+            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (cols) c = cv[i >> 2];
+            if constexpr (kKeys) {
+              x0 = f2_fma(x0, sc2, f2_pack(c.x, c.y));
+              x1 = f2_fma(x1, sc2, f2_pack(c.z, c.w));
+              if (kGeneral) {
+                x0 = f2_add(x0, ra2);
+                x1 = f2_add(x1, ra2);
+              }
+            } else {
+              x0 = f2_fma(x0, sc2, ra2);
+              x1 = f2_fma(x1, sc2, ra2);
+              if (kGeneral && cols) {
+                x0 = f2_add(x0, f2_pack(c.x, c.y));
+                x1 = f2_add(x1, f2_pack(c.z, c.w));
               }
             }
-          }
-        } else {
-#pragma unroll
-          for (int t = 0; t < 32; ++t) dsv[t] = pv[t] * (__uint_as_float(dp_raw[t]) - delta);
-        }
-        if (drel_row != nullptr) {
-#pragma unroll
-          for (int t = 0; t < 32; ++t) {
-            const int key = n0 + c * 32 + t;
-            if (key < key_limit && dsv[t] != 0.f) atomicAdd(drel_row + key, dsv[t] * inv_keep);
+            f2_unpack(x0, pr[i], pr[i + 1]);
+            f2_unpack(x1, pr[i + 2], pr[i + 3]);
           }
         }
+        if constexpr (kGeneral) {
+          if (p.rel != nullptr) {
+            const float* rel = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + p.Sq - 1;
+            if constexpr (kKeys) {
+              const int key = min(row, p.Sk - 1);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const int chunk = (c & 1) * 4 + g;
-          const int off = (c >> 1) * kBlkBytes + ((chunk ^ (r_in & 7)) << 4);
-          uint4 pk = make_uint4(pack_pair_b(pv[g * 8 + 0], pv[g * 8 + 1], p.bf16),
-                                pack_pair_b(pv[g * 8 + 2], pv[g * 8 + 3], p.bf16),
-                                pack_pair_b(pv[g * 8 + 4], pv[g * 8 + 5], p.bf16),
-                                pack_pair_b(pv[g * 8 + 6], pv[g * 8 + 7], p.bf16));
-          *reinterpret_cast<uint4*>(p_row + off) = pk;
-          uint4 dk = make_uint4(pack_pair_b(dsv[g * 8 + 0], dsv[g * 8 + 1], p.bf16),
-                                pack_pair_b(dsv[g * 8 + 2], dsv[g * 8 + 3], p.bf16),
-                                pack_pair_b(dsv[g * 8 + 4], dsv[g * 8 + 5], p.bf16),
-                                pack_pair_b(dsv[g * 8 + 6], dsv[g * 8 + 7], p.bf16));
-          *reinterpret_cast<uint4*>(ds_row + off) = dk;
-        }
-      }
-      tc::fence_before_sync();
-      tc::fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(pds_full);
-      if constexpr (kPB == 2) {
-        // with two P / dS buffers the tensor core is already on S / dP of block it + 1: take
-        // the dQ tile of the PREVIOUS block out now, the one of this block after the next
-        // block's softmax gradient
-        if (it > 0 && !dq_readout(it - 1)) { ok = false; break; }
-      } else {
-        if (!dq_readout(it)) { ok = false; break; }
-      }
-    }
-    if constexpr (kPB == 2) {
-      if (ok && n_iter > 0) ok = dq_readout(n_iter - 1);
-    }
-    // dK / dV of this key tile: thread = key row
-    if (ok && n_iter > 0) ok = tc::mbar_wait_warp(acc_full, 0, abort_flag);
-    tc::fence_after_sync();
-    const int key = n0 + r_in;
-    // tcgen05.ld is warp-collective: every lane takes part, only the stores
-    // are predicated on the key being in range
-    if (ok) {
-      const int key_c = min(key, p.Sk - 1);
-      uint8_t* dk_dst = static_cast<uint8_t*>(p.dK) +
-                        ((static_cast<int64_t>(batch) * p.Sk + key_c) * p.H + head) * p.dkv_row_stride * 2;
-      uint8_t* dv_dst = static_cast<uint8_t*>(p.dV) +
-                        ((static_cast<int64_t>(batch) * p.Sk + key_c) * p.H + head) * p.dkv_row_stride * 2;
-      {
-        // the first four softmax warps write dV, the other four dK
-        const int which = half;
-        uint8_t* dst = which == 0 ? dv_dst : dk_dst;
-        const uint32_t col = which == 0 ? kColDV : kColDK;
-        const float f = which == 0 ? inv_keep : out_scale;
+              for (int i = 0; i < 64; ++i)
+                pr[i] = fmaf(rel[key - min(col0 + i, p.Sq - 1)], kLog2e, pr[i]);
+            } else {
+              const int query = min(row, p.Sq - 1);
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t r[32];
-          if (n_iter > 0) {
-            tc::tmem_ld_x32(tmem_base + col + c * 32 + lane_sel, r);
-            tc::tmem_ld_wait();
+              for (int i = 0; i < 64; ++i)
+                pr[i] = fmaf(rel[min(col0 + i, p.Sk - 1) - query], kLog2e, pr[i]);
+            }
+          }
+          if constexpr (kKeys) {
+            // key `row` is seen by queries >= row - diag (queries beyond Sq have nlse = -inf)
+            if (p.causal && col0 + diag < tile * 128 + quarter * 32 + 31) {
+#pragma unroll
+              for (int i = 0; i < 64; ++i)
+                if (col0 + i + diag < row) pr[i] = -INFINITY;
+            }
           } else {
+            const int limit = p.causal ? min(p.Sk, row + diag + 1) : p.Sk;
+            const int first_limit = p.causal ? min(p.Sk, tile * 128 + quarter * 32 + diag + 1) : p.Sk;
+            if (col0 + 64 > first_limit) {
 #pragma unroll
-            for (int t = 0; t < 32; ++t) r[t] = 0u;
-          }
-          if (key < p.Sk) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              if (c * 32 + g * 8 >= p.Dr) break;
-              uint4 pk = make_uint4(
-                  pack_pair_b(__uint_as_float(r[g * 8 + 0]) * f, __uint_as_float(r[g * 8 + 1]) * f, p.bf16),
-                  pack_pair_b(__uint_as_float(r[g * 8 + 2]) * f, __uint_as_float(r[g * 8 + 3]) * f, p.bf16),
-                  pack_pair_b(__uint_as_float(r[g * 8 + 4]) * f, __uint_as_float(r[g * 8 + 5]) * f, p.bf16),
-                  pack_pair_b(__uint_as_float(r[g * 8 + 6]) * f, __uint_as_float(r[g * 8 + 7]) * f, p.bf16));
-              *reinterpret_cast<uint4*>(dst + (c * 32 + g * 8) * 2) = pk;
+              for (int i = 0; i < 64; ++i)
+                if (col0 + i >= limit) pr[i] = -INFINITY;
             }
           }
         }
+#pragma unroll
+        for (int i = 0; i < 64; ++i) pr[i] = exp2f(pr[i]);
+        const uint4* kw4 = reinterpret_cast<const uint4*>(vec + 1024 + quarter * 512) + half * 16;
+        const uint32_t lane_bit = 1u << lane;
+        if constexpr (kKeys) {
+          if (!kOver && t > 0 && !tc::mbar_wait_warp(a2_done, (t - 1) & 1, abort_flag)) {
+            ok = false;
+            break;
+          }
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            uint32_t pk[16];
+            if (drop) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const uint4 k = kw4[c * 8 + i];
+                const float* v = pr + c * 32 + i * 4;
+                pk[2 * i] = pack16<T>((k.x & lane_bit) ? v[0] : 0.f, (k.y & lane_bit) ? v[1] : 0.f);
+                pk[2 * i + 1] = pack16<T>((k.z & lane_bit) ? v[2] : 0.f, (k.w & lane_bit) ? v[3] : 0.f);
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) pk[i] = pack16<T>(pr[c * 32 + 2 * i], pr[c * 32 + 2 * i + 1]);
+            }
+            tc::tmem_st_x16(tmem_row + kColP + half * kHalf + c * 16, pk);
+          }
+          tc::tmem_st_wait();
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(p_ready);
+        }
+        // ---- the item before this one leaves tensor memory ----
+        if (j == 0 && prev_item >= 0) {
+          if (!tc::mbar_wait_warp(acc_full, (w - 1) & 1, abort_flag)) { ok = false; break; }
+          read_out(prev_item);
+        }
+        // ---- dS ----
+        if (!tc::mbar_wait_warp(dp_full, t & 1, abort_flag)) { ok = false; break; }
+        if (!kOver && t > 0 && !tc::mbar_wait_warp(a1_done, (t - 1) & 1, abort_flag)) { ok = false; break; }
+        tc::fence_after_sync();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t d[32];
+          tc::tmem_ld_x32(tmem_row + kColDP + half * 64 + c * 32, d);
+          tc::tmem_ld_wait();
+          if (drop) {
+            if constexpr (kKeys) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const uint4 k = kw4[c * 8 + i];
+                d[4 * i] = (k.x & lane_bit) ? d[4 * i] : 0u;
+                d[4 * i + 1] = (k.y & lane_bit) ? d[4 * i + 1] : 0u;
+                d[4 * i + 2] = (k.z & lane_bit) ? d[4 * i + 2] : 0u;
+                d[4 * i + 3] = (k.w & lane_bit) ? d[4 * i + 3] : 0u;
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                d[i] &= keep_mask_full(keep16[c * 2 + (i >> 4)][(i >> 2) & 3], i & 3);
+            }
+          }
+          const float4* nd = reinterpret_cast<const float4*>(vec + 512) + half * 16 + c * 8;
+          float ds[32];
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            uint64_t x0 = f2_pack(__uint_as_float(d[i]), __uint_as_float(d[i + 1]));
+            uint64_t x1 = f2_pack(__uint_as_float(d[i + 2]), __uint_as_float(d[i + 3]));
+            if constexpr (kKeys) {
+              const float4 dl = nd[i >> 2];
+              x0 = f2_add(x0, f2_pack(dl.x, dl.y));
+              x1 = f2_add(x1, f2_pack(dl.z, dl.w));
+            } else {
+              x0 = f2_add(x0, rb2);
+              x1 = f2_add(x1, rb2);
+            }
+            const float* v = pr + c * 32 + i;
+            x0 = f2_mul(x0, f2_pack(v[0], v[1]));
+            x1 = f2_mul(x1, f2_pack(v[2], v[3]));
+            f2_unpack(x0, ds[i], ds[i + 1]);
+            f2_unpack(x1, ds[i + 2], ds[i + 3]);
+          }
+          if constexpr (kKeys && kGeneral) {
+            if (p.drel != nullptr) {
+              // Sums along the diagonals key - query = const: the running sum moves one lane up
+              // (next key) with every column (next query), so that it stays on its diagonal;
+              // what leaves at lane 31 is collected and added to the result 32 at a time.
+              float* buf = reinterpret_cast<float*>(smem + L::kDrel) + (warp - 2) * 64;
+              float* out = p.drel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1);
+              const int key0 = tile * 128 + quarter * 32, q0 = col0 + c * 32;
+              const int last = p.Sq + p.Sk - 2;
+              float acc = 0.f;
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                // padding: keys beyond Sk have a P (their rows go nowhere else), queries have none
+                if (row < p.Sk) acc += ds[i];
+                acc = __shfl_sync(0xffffffffu, acc, (lane + 31) & 31);
+                if (lane == 0) {
+                  buf[i] = acc;               // diagonal key0 + 31 - (q0 + i)
+                  acc = 0.f;
+                }
+              }
+              __syncwarp();
+              const int at = key0 + 31 - (q0 + lane) + p.Sq - 1;
+              if (at >= 0 && at <= last) atomicAdd(out + at, buf[lane] * p.inv_keep);
+              const int rest = key0 + lane - (q0 + 32) + p.Sq - 1;     // still under way in the lanes
+              if (lane > 0 && rest >= 0 && rest <= last) atomicAdd(out + rest, acc * p.inv_keep);
+              __syncwarp();
+            }
+          }
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) pk[i] = pack16<T>(ds[2 * i], ds[2 * i + 1]);
+          tc::tmem_st_x16(tmem_row + kColDS + half * kHalf + c * 16, pk);
+        }
+        tc::tmem_st_wait();
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(ds_ready);
       }
+      prev_item = item;
     }
+    if (ok && prev_item >= 0 && tc::mbar_wait_warp(acc_full, (w - 1) & 1, abort_flag))
+      read_out(prev_item);
   }
 
   tc::fence_before_sync();
@@ -481,68 +698,12 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   }
 }
 
-// dq (16-bit, rows spaced out_row_stride elements apart) <- sum of the fp32 partials (contiguous
-// rows of D, one partial per 128-key tile, slice_stride elements apart; a single accumulator
-// when n_slices == 1): the conversion that closes the backward pass; 8 values per thread,
-// 16-byte stores.  Under a causal mask key tile kt holds rows of query tiles >= first_q(kt)
-// only (the others were never written and are skipped).
-template <typename T>
-__global__ void __launch_bounds__(256) flash_dq_convert_kernel(
-    const float* __restrict__ acc, T* __restrict__ out, int64_t rows, int D, int64_t out_row_stride,
-    int n_slices, int64_t slice_stride, int Sq, int Sk, int H, int causal) {
-  const int vecs_per_row = D >> 3;
-  const int64_t n_vec = rows * vecs_per_row;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  const int diag = Sk - Sq;
-  const int q_tiles = (Sq + 127) / 128;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_vec;
-       i += stride) {
-    const int64_t row = i / vecs_per_row;
-    const int d = static_cast<int>(i - row * vecs_per_row) * 8;
-    const int q_tile = static_cast<int>((row / H) % Sq) >> 7;
-    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int kt = 0; kt < n_slices; ++kt) {
-      if (causal && n_slices > 1) {
-        int first_q = (kt * 128 - diag) / 128;
-        first_q = first_q < 0 ? 0 : (first_q > q_tiles ? q_tiles : first_q);
-        if (q_tile < first_q) break;      // later key tiles start even later
-      }
-      float part[8];
-      Vec8<float>::load(acc + kt * slice_stride + row * D + d, part);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] += part[j];
-    }
-    Vec8<T>::store(out + row * out_row_stride + d, v);
-  }
-}
-
-void launch_flash_dq_convert(const float* acc, void* out, int64_t rows, int D,
-                             int64_t out_row_stride, bool bf16, int n_slices, int64_t slice_stride,
-                             int Sq, int Sk, int H, int causal, cudaStream_t stream) {
-  const int64_t n_vec = rows * (D >> 3);
-  if (n_vec == 0) return;
-  int64_t blocks = (n_vec + 255) / 256;
-  const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
-  if (blocks > cap) blocks = cap;
-  count_launch();
-  if (bf16)
-    flash_dq_convert_kernel<__nv_bfloat16><<<static_cast<int>(blocks), 256, 0, stream>>>(
-        acc, static_cast<__nv_bfloat16*>(out), rows, D, out_row_stride, n_slices, slice_stride, Sq,
-        Sk, H, causal);
-  else
-    flash_dq_convert_kernel<__half><<<static_cast<int>(blocks), 256, 0, stream>>>(
-        acc, static_cast<__half*>(out), rows, D, out_row_stride, n_slices, slice_stride, Sq, Sk, H,
-        causal);
-}
-
-template <int D, bool kPlain>
-static int launch_bwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                        const CUtensorMap& tdo, const FlashBwdParams& p, cudaStream_t stream) {
-  constexpr int kStages = D == 64 ? 2 : 1;
-  constexpr int kPB = D == 64 ? 2 : 1;
-  constexpr int kSmem = (2 + 2 * kStages) * 128 * D * 2 + kPB * 4 * 128 * 128 + 12 * 8 + 128 * 4 + 1024;
+template <int D, bool kKeys, bool kGeneral, typename T>
+static int launch_bwd_d(const CUtensorMap& x1, const CUtensorMap& x2, const CUtensorMap& y1,
+                        const CUtensorMap& y2, const FlashBwdParams& p, cudaStream_t stream) {
+  constexpr int kSmem = BwdSmem<D, kKeys>::kTotal;
   static_assert(kSmem <= 227 * 1024, "flash backward: shared memory over the per-CTA limit");
-  auto kernel = flash_bwd_kernel<D, kPlain>;
+  auto kernel = flash_bwd_kernel<D, kKeys, kGeneral, T>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
@@ -550,35 +711,55 @@ static int launch_bwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
       return 3;
     configured = true;
   }
-  dim3 grid((p.Sk + 127) / 128, p.H, p.B);
+  const int64_t items = static_cast<int64_t>(p.walk.row_tiles) * p.walk.nbh;
+  const int64_t cap = sm_count();
   count_launch();
-  kernel<<<grid, 320, kSmem, stream>>>(tq, tk, tv, tdo, p);
+  kernel<<<static_cast<int>(items < cap ? items : cap), 320, kSmem, stream>>>(x1, x2, y1, y2, p);
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
-int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
-                     const float* lse, float* delta, float* dq_accum, int64_t dq_slice_stride,
-                     void* dk, void* dv, int64_t dkv_row_stride, const float* kbias, const float* rel, float* drel,
-                     int B, int H, int Sq, int Sk, int D, const int64_t* q_strides, const int64_t* k_strides,
-                     const int64_t* v_strides, float scale, int causal, float p_drop,
-                     PhiloxArgs rng, bool bf16, int* status, cudaStream_t stream) {
-  if (D < 8 || D > 128 || D % 8 != 0) return 1;
-  const int Dt = D <= 64 ? 64 : 128;     // tile width; columns D .. Dt - 1 are zero-filled by TMA
-  // pre-pass: delta (o and dout are contiguous [B, Sq, H, D])
-  {
-    const int64_t rows = static_cast<int64_t>(B) * Sq * H;
-    const int wpb = 8;
-    const int64_t rows_per_block = static_cast<int64_t>(wpb) * (256 / Dt);
-    const unsigned blocks = static_cast<unsigned>((rows + rows_per_block - 1) / rows_per_block);
-    count_launch();
-    if (bf16)
-      flash_bwd_delta_kernel<__nv_bfloat16><<<blocks, wpb * 32, 0, stream>>>(
-          static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), delta, B, H,
-          Sq, Dt, D);
-    else
-      flash_bwd_delta_kernel<__half><<<blocks, wpb * 32, 0, stream>>>(
-          static_cast<const __half*>(dout), static_cast<const __half*>(o), delta, B, H, Sq, Dt, D);
+template <bool kKeys>
+static int launch_bwd_pass(const CUtensorMap& x1, const CUtensorMap& x2, const CUtensorMap& y1,
+                           const CUtensorMap& y2, const FlashBwdParams& p, bool general, bool bf16,
+                           cudaStream_t stream) {
+#define FLASH_BWD_CASE(D_, T_)                                                            \
+  return general ? launch_bwd_d<D_, kKeys, true, T_>(x1, x2, y1, y2, p, stream)           \
+                 : launch_bwd_d<D_, kKeys, false, T_>(x1, x2, y1, y2, p, stream)
+  if (p.Dr <= 64) {
+    if (bf16) FLASH_BWD_CASE(64, __nv_bfloat16);
+    FLASH_BWD_CASE(64, __half);
   }
+  if (bf16) FLASH_BWD_CASE(128, __nv_bfloat16);
+  FLASH_BWD_CASE(128, __half);
+#undef FLASH_BWD_CASE
+}
+
+static int round128(int n) { return (n + 127) / 128 * 128; }
+
+FlashBwdScratch flash_bwd_scratch(int B, int H, int Sq, int Sk, bool key_bias, float p_drop) {
+  FlashBwdScratch s;
+  const int64_t rq = round128(Sq), rk = round128(Sk), bh = static_cast<int64_t>(B) * H;
+  s.stats = 2 * bh * rq;
+  s.bias = key_bias ? B * rk : 0;
+  // keep bits of as many (batch, head) pairs at a time as fit 1 GB (at least one)
+  const int64_t words = rk / 32 * rq;
+  int64_t pairs = words > 0 ? (int64_t(1) << 28) / words : bh;
+  if (pairs < 1) pairs = 1;
+  if (pairs > bh) pairs = bh;
+  const bool drop = dropout_thr7(p_drop) != 0;
+  s.pairs = static_cast<int>(drop ? pairs : bh);
+  s.keep = drop ? s.pairs * words : 0;
+  return s;
+}
+
+int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
+                     const float* lse, float* scratch, void* dq, void* dk, void* dv,
+                     int64_t dq_row_stride, int64_t dkv_row_stride, const float* kbias,
+                     const float* rel, float* drel, int B, int H, int Sq, int Sk, int D,
+                     const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
+                     float scale, int causal, float p_drop, PhiloxArgs rng, bool bf16, int* status,
+                     cudaStream_t stream) {
+  if (D < 8 || D > 128 || D % 8 != 0) return 1;
   CUtensorMap tq, tk, tv, tdo;
   const int64_t do_strides[3] = {static_cast<int64_t>(Sq) * H * D, static_cast<int64_t>(H) * D, D};
   if (!make_tmap_bshd(&tq, q, B, Sq, H, D, q_strides[0], q_strides[1], q_strides[2], 128, bf16) ||
@@ -586,24 +767,63 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o,
       !make_tmap_bshd(&tv, v, B, Sk, H, D, v_strides[0], v_strides[1], v_strides[2], 128, bf16) ||
       !make_tmap_bshd(&tdo, dout, B, Sq, H, D, do_strides[0], do_strides[1], do_strides[2], 128, bf16))
     return 2;
+  const FlashBwdScratch sizes = flash_bwd_scratch(B, H, Sq, Sk, kbias != nullptr, p_drop);
   FlashBwdParams p;
-  p.B = B; p.H = H; p.Sq = Sq; p.Sk = Sk; p.Dr = D; p.lse = lse; p.delta = delta; p.dq_accum = dq_accum;
-  p.dq_slice_stride = dq_slice_stride;
-  p.dK = dk; p.dV = dv; p.dkv_row_stride = dkv_row_stride; p.kbias = kbias; p.rel = rel; p.drel = drel; p.scale = scale;
-  p.scale_log2 = scale * kLog2eB; p.causal = causal; p.rng = rng;
+  p.Sq = Sq; p.Sk = Sk; p.H = H; p.Dr = D;
+  p.k_steps = (D + 15) / 16;
+  p.Rq = round128(Sq); p.Rk = round128(Sk);
   p.thr7 = dropout_thr7(p_drop);   // same quantisation as the forward kernel
-  p.p_drop = p.thr7 / 128.f;
-  p.bf16 = bf16 ? 1 : 0; p.status = status;
-  const int f = bf16 ? 1 : 0;
-  p.idesc_s = tc::instr_desc_f16(128, 128, f, false, false);   // S, dP
-  p.idesc_dvk = tc::instr_desc_f16(128, Dt, f, true, true);     // dV, dK
-  p.idesc_dq = tc::instr_desc_f16(128, Dt, f, false, true);     // dQ
-  const bool plain = kbias == nullptr && rel == nullptr && !causal && Sk % 128 == 0 && Sq % 128 == 0;
-  if (Dt == 64)
-    return plain ? launch_bwd_d<64, true>(tq, tk, tv, tdo, p, stream)
-                 : launch_bwd_d<64, false>(tq, tk, tv, tdo, p, stream);
-  return plain ? launch_bwd_d<128, true>(tq, tk, tv, tdo, p, stream)
-               : launch_bwd_d<128, false>(tq, tk, tv, tdo, p, stream);
+  const float keep_prob = 1.f - p.thr7 / 128.f;
+  // scratch: nlse | ndelta | key bias | keep bits, each a multiple of 128 words
+  float* nlse = scratch;
+  float* ndelta = nlse + sizes.stats / 2;
+  float* kb2 = ndelta + sizes.stats / 2;
+  p.nlse = nlse; p.ndelta = ndelta;
+  p.kb2 = kbias != nullptr ? kb2 : nullptr;
+  p.keep = p.thr7 != 0 ? reinterpret_cast<uint32_t*>(kb2 + sizes.bias) : nullptr;
+  p.rel = rel; p.drel = drel;
+  p.scale = scale; p.scale_log2 = scale * kLog2e; p.inv_keep = 1.f / keep_prob;
+  p.causal = causal; p.rng = rng; p.status = status;
+  p.idesc_s = tc::instr_desc_f16(128, 128, bf16 ? 1 : 0, false, false);
+  p.idesc_acc = tc::instr_desc_f16(128, p.k_steps * 16, bf16 ? 1 : 0, false, true);
+  {
+    const int lanes = D <= 64 ? 8 : 16;
+    const dim3 grid((p.Rq + 31) / 32, (H + 7) / 8, B);
+    count_launch();
+    if (bf16)
+      flash_bwd_stats_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(
+          static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), lse, nlse,
+          ndelta, H, Sq, p.Rq, D, lanes, keep_prob);
+    else
+      flash_bwd_stats_kernel<__half><<<grid, 256, 0, stream>>>(
+          static_cast<const __half*>(dout), static_cast<const __half*>(o), lse, nlse, ndelta, H, Sq,
+          p.Rq, D, lanes, keep_prob);
+  }
+  if (kbias != nullptr) {
+    count_launch();
+    flash_bwd_bias_kernel<<<dim3((p.Rk + 255) / 256, B), 256, 0, stream>>>(kbias, kb2, Sk, p.Rk);
+  }
+  const bool general = kbias != nullptr || rel != nullptr || causal || Sk % 128 != 0;
+  p.walk.H = H;
+  const int bh = B * H;
+  for (int at = 0; at < bh; at += sizes.pairs) {
+    p.walk.bh0 = at;
+    p.walk.nbh = bh - at < sizes.pairs ? bh - at : sizes.pairs;
+    // dQ first: with dropout it leaves the keep bits that the dK / dV pass reads
+    p.walk.row_tiles = p.Rq / 128;
+    p.walk.by_cost = causal ? 2 : 0;
+    p.out1 = dq; p.row_stride1 = dq_row_stride;
+    p.out2 = nullptr; p.row_stride2 = 0;
+    int rc = launch_bwd_pass<false>(tq, tdo, tk, tv, p, general, bf16, stream);
+    if (rc != 0) return rc;
+    p.walk.row_tiles = p.Rk / 128;
+    p.walk.by_cost = causal ? 1 : 0;
+    p.out1 = dk; p.row_stride1 = dkv_row_stride;
+    p.out2 = dv; p.row_stride2 = dkv_row_stride;
+    rc = launch_bwd_pass<true>(tk, tv, tq, tdo, p, general, bf16, stream);
+    if (rc != 0) return rc;
+  }
+  return 0;
 }
 
 }  // namespace slapo

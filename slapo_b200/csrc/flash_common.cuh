@@ -1,0 +1,67 @@
+// Device helpers shared by the flash-attention forward and backward kernels: packed fp32
+// arithmetic, 16-bit packing by type, exp2 on the special-function unit.
+#pragma once
+#include "common.cuh"
+#include "tc05.cuh"
+
+namespace slapo {
+
+constexpr float kLog2e = 1.4426950408889634f;
+
+// two fp32 values in one 64-bit register: sm_100 issues an FMA / add / multiply on both at once
+__device__ __forceinline__ uint64_t f2_pack(float a, float b) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ void f2_unpack(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+template <typename T> __device__ __forceinline__ uint32_t pack16(float a, float b);
+template <> __device__ __forceinline__ uint32_t pack16<__nv_bfloat16>(float a, float b) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+template <> __device__ __forceinline__ uint32_t pack16<__half>(float a, float b) {
+  __half2 v = __floats2half2_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+
+// Row tiles of 128 of all (batch, head) pairs, walked by a persistent grid.  Under a causal
+// mask the tiles differ in cost: they are ordered by cost, heaviest first, over all heads.
+// Otherwise the tiles of one head are neighbours, so that the tensors they share stay in L2.
+struct TileWalk {
+  int row_tiles;     // per (batch, head)
+  int bh0, nbh;      // range of (batch, head) pairs of this launch
+  int H;
+  int by_cost;       // 0 = head-major, 1 = first tile heaviest, 2 = last tile heaviest
+  __device__ __forceinline__ int items() const { return row_tiles * nbh; }
+  __device__ __forceinline__ void at(int item, int& tile, int& bh_local) const {
+    if (by_cost == 0) {
+      bh_local = item / row_tiles;
+      tile = item - bh_local * row_tiles;
+    } else {
+      tile = item / nbh;
+      bh_local = item - tile * nbh;
+      if (by_cost == 2) tile = row_tiles - 1 - tile;
+    }
+  }
+};
+
+}  // namespace slapo

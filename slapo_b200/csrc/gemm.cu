@@ -46,11 +46,22 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
+// A thread that has not yet made a CUDA call of its own (autograd's device thread whose first node
+// is one of ours) has no current context, and encoding a tensor map without one crashes in the
+// driver.  Setting the device makes its primary context current (allowed during stream capture).
+void ensure_cuda_context() {
+  static thread_local bool ready = false;
+  if (ready) return;
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) ready = true;
+}
+
 bool make_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer,
                   uint64_t row_stride_elems, uint32_t box_inner, uint32_t box_outer,
                   int elem_bytes, bool is_bf16) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return false;
+  ensure_cuda_context();
   cuuint64_t dims[2] = {inner, outer};
   cuuint64_t strides[1] = {row_stride_elems * static_cast<uint64_t>(elem_bytes)};
   cuuint32_t box[2] = {box_inner, box_outer};

@@ -1,0 +1,101 @@
+"""Flash attention at the edges of its paths against a 64-bit restatement: work items beyond one
+wave of the persistent grid, a single key tile, ragged and unequal lengths, keys split over work
+items, row maxima that grow along the keys, relative bias and dropout on the general path.
+
+Tolerance: P, dS and the results are rounded to 16 bits once each, an independent relative error of
+up to 2^-9 (bf16) or 2^-12 (fp16) per value; the 2-norm of a result's error stays below four times
+that."""
+import pytest
+import torch
+
+from slapo_b200.ops import functional as NF
+from slapo_b200.ops import native
+from slapo_b200.ops.flash_attn import dropout_keep_mask, effective_dropout_p
+
+pytestmark = pytest.mark.gpu
+
+BF, FP = torch.bfloat16, torch.float16
+TOL = {BF: 4 * 2.0 ** -9, FP: 4 * 2.0 ** -12}
+
+
+def _reference(q, k, v, bias, causal, scale, table, mask, p):
+    q, k, v = (t.detach().double().requires_grad_(True) for t in (q, k, v))
+    s = torch.einsum("bqhd,bkhd->bhqk", q, k) * scale
+    sq, sk = s.shape[-2:]
+    if table is not None:
+        table = table.detach().double().requires_grad_(True)
+        pos = torch.arange(sk, device="cuda")[None] - (torch.arange(sq, device="cuda")[:, None]
+                                                       + sk - sq)
+        s = s + table[NF.t5_relative_position_bucket(pos, not causal, 32, 128)].permute(2, 0, 1)
+    if bias is not None:
+        s = s + bias.double()[:, None, None]
+    if causal:
+        ahead = torch.ones(sq, sk, dtype=torch.bool, device="cuda").triu(sk - sq + 1)
+        s = s.masked_fill(ahead, float("-inf"))
+    pr = torch.softmax(s, -1).nan_to_num(nan=0.0)      # rows without a key give zeros
+    if mask is not None:
+        pr = pr * mask.double() / (1 - p)
+    return torch.einsum("bhqk,bkhd->bqhd", pr, v), q, k, v, table
+
+
+# batch, sq, sk, heads, dim, dtype, then: c causal, k key padding, r relative table, g growing
+# scores; dropout probability
+CASES = [
+    (2, 512, 512, 40, 64, BF, "", 0.0),        # more row tiles than resident CTAs
+    (1, 1024, 1024, 40, 128, FP, "", 0.0),
+    (2, 640, 640, 30, 128, BF, "c", 0.1),
+    (2, 300, 300, 3, 64, BF, "c", 0.0),
+    (2, 200, 333, 3, 80, BF, "k", 0.0),
+    (2, 333, 200, 3, 80, FP, "ck", 0.0),       # early queries see no key
+    (2, 200, 333, 3, 64, BF, "c", 0.0),
+    (3, 520, 520, 50, 64, FP, "k", 0.1),
+    (300, 130, 130, 2, 64, BF, "", 0.1),
+    (2, 256, 256, 4, 64, BF, "r", 0.0),
+    (2, 200, 200, 4, 64, BF, "ckr", 0.1),
+    (1, 300, 300, 4, 128, BF, "r", 0.1),
+    (2, 1024, 1024, 4, 64, BF, "g", 0.0),      # row maxima raised many times
+    (2, 1024, 1024, 4, 128, FP, "cg", 0.1),
+    (1, 1, 1000, 4, 128, BF, "c", 0.0),        # keys split over work items
+    (3, 5, 700, 4, 64, BF, "ck", 0.0),
+    (2, 100, 1500, 8, 80, FP, "g", 0.1),
+    (8, 1, 1500, 16, 128, BF, "c", 0.0),
+    (1, 48, 2048, 4, 40, BF, "cr", 0.1),
+    (1, 1, 1, 1, 8, BF, "", 0.0),
+    (2, 129, 1, 2, 64, BF, "", 0.0),
+]
+
+
+@pytest.mark.parametrize("b,sq,sk,h,d,dtype,how,p", CASES)
+def test_flash_attention_paths(b, sq, sk, h, d, dtype, how, p):
+    torch.manual_seed(b + sq + sk + h + d)
+    q = torch.randn(b, sq, h, d, device="cuda", dtype=dtype, requires_grad=True)
+    k = torch.randn(b, sk, h, d, device="cuda", dtype=dtype)
+    if "g" in how:
+        k = (k * torch.linspace(0.2, 6, sk, device="cuda")[None, :, None, None]).to(dtype)
+    k.requires_grad_(True)
+    v = torch.randn(b, sk, h, d, device="cuda", dtype=dtype, requires_grad=True)
+    bias = None
+    if "k" in how:
+        # at least half of the keys are real: with a handful dS = P (dP - delta) cancels, and its
+        # error, 2^-9 P (|dP| + |delta|), is bounded against the terms but not against dS
+        real = torch.randint((sk + 1) // 2, sk + 1, (b, 1), device="cuda")
+        bias = torch.where(torch.arange(sk, device="cuda")[None] < real, 0.0, -10000.0)
+    table = (torch.randn(32, h, device="cuda") * 0.5).requires_grad_(True) if "r" in how else None
+    causal = "c" in how
+    torch.cuda.manual_seed(5)
+    mask = dropout_keep_mask(b, h, sq, sk, p) if p else None
+    out = NF.flash_attention(q, k, v, key_padding_bias=bias, causal=causal, dropout_p=p,
+                             rel_bias_table=table, rel_bidirectional=not causal)
+    g = torch.randn_like(out)
+    out.backward(g)
+    assert native.ops().device_status() == 0, "a bounded wait inside a kernel ran out"
+    want, *leaves = _reference(q, k, v, bias, causal, d ** -0.5, table, mask,
+                               effective_dropout_p(p))
+    want.backward(g.double())
+    got = [("out", out, want.detach())] + [
+        (name, x.grad, y.grad) for name, x, y in zip(("dq", "dk", "dv", "dtable"),
+                                                     (q, k, v, table), leaves) if x is not None]
+    for name, x, y in got:
+        # (with a single key dS is a difference of equal numbers: measured against unit scale)
+        err = ((x.double() - y).norm() / y.norm().clamp(min=0.05 * y.numel() ** 0.5)).item()
+        assert err < TOL[dtype], f"{name}: {err:.2e}"
