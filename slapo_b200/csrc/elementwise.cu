@@ -20,10 +20,21 @@ int64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
 // Four independent 16-byte loads per thread are issued before any of them is used: with
 // 2048 resident threads per SM a single load each leaves too few bytes in flight to cover the
 // HBM latency at full bandwidth.
-template <typename T>
+template <int kAct, typename T>
+__device__ __forceinline__ float act_value(float x) {
+  if constexpr (sizeof(T) == 2) return act_fwd16<kAct>(x);
+  else return act_fwd(x, kAct);
+}
+template <int kAct, typename T>
+__device__ __forceinline__ float act_slope(float x) {
+  if constexpr (sizeof(T) == 2) return act_grad16<kAct>(x);
+  else return act_grad(x, kAct);
+}
+
+template <int kAct, typename T>
 __global__ void __launch_bounds__(256) bias_act_fwd_kernel(
     const T* __restrict__ x, const T* __restrict__ bias, T* __restrict__ y, int64_t n_vec,
-    int cols, int act) {
+    int cols) {
   constexpr int kUnroll = 4;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int vpr = cols / kVec;  // vectors per row
@@ -50,7 +61,7 @@ __global__ void __launch_bounds__(256) bias_act_fwd_kernel(
         for (int k = 0; k < 8; ++k) v[u][k] += b[k];
       }
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[u][k] = act_fwd(v[u][k], act);
+      for (int k = 0; k < 8; ++k) v[u][k] = act_value<kAct, T>(v[u][k]);
       Vec8<T>::store(y + (i + u * stride) * kVec, v[u]);
     }
   }
@@ -66,7 +77,7 @@ __global__ void __launch_bounds__(256) bias_act_fwd_kernel(
     cv += step;
     if (cv >= vpr) cv -= vpr;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = act_fwd(v[k], act);
+    for (int k = 0; k < 8; ++k) v[k] = act_value<kAct, T>(v[k]);
     Vec8<T>::store(y + i * kVec, v);
   }
 }
@@ -95,11 +106,10 @@ __device__ __forceinline__ void slab_reduce_store(float acc[8], float* partial, 
   }
 }
 
-template <typename T>
+template <int kAct, typename T>
 __global__ void __launch_bounds__(256) bias_act_bwd_kernel(
     const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ bias,
-    T* __restrict__ dx, float* __restrict__ partial, int rows, int cols, int rows_per_chunk,
-    int act) {
+    T* __restrict__ dx, float* __restrict__ partial, int rows, int cols, int rows_per_chunk) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * 256 + lane * 8;
   const bool col_ok = col + 8 <= cols;
@@ -117,7 +127,7 @@ __global__ void __launch_bounds__(256) bias_act_bwd_kernel(
       Vec8<T>::load(x + e, v);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        g[k] *= act_grad(v[k] + b[k], act);
+        g[k] *= act_slope<kAct, T>(v[k] + b[k]);
         acc[k] += g[k];
       }
       Vec8<T>::store(dx + e, g);
@@ -299,13 +309,21 @@ int colsum_chunks(int rows, int cols) {
     default: { using T = float; __VA_ARGS__; break; }                \
   }
 
+#define DISPATCH_ACT(act, ...)                                       \
+  switch (act) {                                                     \
+    case 0: { constexpr int kAct = 0; __VA_ARGS__; break; }          \
+    case 1: { constexpr int kAct = 1; __VA_ARGS__; break; }          \
+    default: { constexpr int kAct = 2; __VA_ARGS__; break; }         \
+  }
+
 void launch_bias_act_fwd(const void* x, const void* bias, void* y, int64_t rows, int cols,
                          int act, int dtype, cudaStream_t stream) {
   const int64_t n_vec = rows * cols / kVec;
   if (n_vec == 0) return;
   count_launch();
-  DISPATCH_DTYPE(dtype, (bias_act_fwd_kernel<T><<<flat_grid(n_vec), 256, 0, stream>>>(
-      static_cast<const T*>(x), static_cast<const T*>(bias), static_cast<T*>(y), n_vec, cols, act)));
+  DISPATCH_DTYPE(dtype, DISPATCH_ACT(act, (bias_act_fwd_kernel<kAct, T>
+      <<<flat_grid(n_vec), 256, 0, stream>>>(
+          static_cast<const T*>(x), static_cast<const T*>(bias), static_cast<T*>(y), n_vec, cols))));
 }
 
 void launch_colsum_finalize(const float* partial, void* out, int chunks, int cols, int dtype,
@@ -324,9 +342,9 @@ void launch_bias_act_bwd(const void* dy, const void* x, const void* bias, void* 
   dim3 grid((cols + 255) / 256, chunks);
   float* part = dbias != nullptr ? partial : nullptr;
   count_launch();
-  DISPATCH_DTYPE(dtype, (bias_act_bwd_kernel<T><<<grid, 256, 0, stream>>>(
+  DISPATCH_DTYPE(dtype, DISPATCH_ACT(act, (bias_act_bwd_kernel<kAct, T><<<grid, 256, 0, stream>>>(
       static_cast<const T*>(dy), static_cast<const T*>(x), static_cast<const T*>(bias),
-      static_cast<T*>(dx), part, rows, cols, rows_per_chunk, act)));
+      static_cast<T*>(dx), part, rows, cols, rows_per_chunk))));
   if (dbias != nullptr) launch_colsum_finalize(partial, dbias, chunks, cols, dtype, stream);
 }
 
