@@ -138,6 +138,45 @@ Tensor flash_attn_dropout_mask(int64_t B, int64_t H, int64_t Sq, int64_t Sk, dou
   return mask;
 }
 
+// the caches of one layer grown by new tokens: ([B, past + n, H, D] contiguous) k and v
+std::tuple<Tensor, Tensor> kv_append(const Tensor& past_k, const Tensor& past_v, const Tensor& k,
+                                     const Tensor& v) {
+  const Tensor* past[2] = {&past_k, &past_v};
+  const Tensor* fresh[2] = {&k, &v};
+  Tensor out[2];
+  c10::cuda::CUDAGuard guard(k.device());
+  const int64_t B = k.size(0), n = k.size(1), H = k.size(2), D = k.size(3), len = past_k.size(1);
+  const int64_t e = k.element_size();
+  TORCH_CHECK(D * e % 16 == 0, "kv_append: heads must be a multiple of 16 bytes");
+  const void* past_ptr[2];
+  const void* fresh_ptr[2];
+  void* out_ptr[2];
+  int64_t strides[2][3];
+  for (int i = 0; i < 2; ++i) {
+    const Tensor &p = *past[i], &f = *fresh[i];
+    TORCH_CHECK(p.is_cuda() && f.is_cuda() && p.dim() == 4 && f.dim() == 4 &&
+                    p.get_device() == k.get_device() && f.get_device() == k.get_device() &&
+                    p.scalar_type() == k.scalar_type() && f.scalar_type() == k.scalar_type(),
+                "kv_append: four [B, S, H, D] CUDA tensors of one type and device required");
+    TORCH_CHECK(p.size(0) == B && p.size(1) == len && p.size(2) == H && p.size(3) == D &&
+                    f.sizes() == k.sizes(), "kv_append: sizes differ");
+    TORCH_CHECK(p.is_contiguous() && f.stride(3) == 1, "kv_append: contiguous cache and heads required");
+    for (int d = 0; d < 3; ++d) {
+      strides[i][d] = f.stride(d) * e;
+      TORCH_CHECK(strides[i][d] % 16 == 0, "kv_append: strides must be multiples of 16 bytes");
+    }
+    out[i] = at::empty({B, len + n, H, D}, k.options());
+    past_ptr[i] = p.data_ptr();
+    fresh_ptr[i] = f.data_ptr();
+    out_ptr[i] = out[i].data_ptr();
+    TORCH_CHECK((reinterpret_cast<uintptr_t>(past_ptr[i]) | reinterpret_cast<uintptr_t>(fresh_ptr[i])) %
+                        16 == 0, "kv_append: data must be 16-byte aligned");
+  }
+  slapo::launch_kv_append(past_ptr, fresh_ptr, out_ptr, B, len, n, H, D * e, strides,
+                          at::cuda::getCurrentCUDAStream().stream());
+  return {out[0], out[1]};
+}
+
 }  // namespace
 
 void register_attn_ops(torch::Library& m) {
@@ -145,6 +184,7 @@ void register_attn_ops(torch::Library& m) {
         &flash_attn_fwd);
   m.def("flash_attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor? kbias, Tensor? rel, bool causal, float scale, float p_drop, Tensor? rng, bool packed_qkv) -> (Tensor, Tensor, Tensor, Tensor)",
         &flash_attn_bwd);
+  m.def("kv_append(Tensor past_k, Tensor past_v, Tensor k, Tensor v) -> (Tensor, Tensor)", &kv_append);
   m.def("flash_attn_dropout_mask(int B, int H, int Sq, int Sk, float p_drop, Tensor rng) -> Tensor",
         &flash_attn_dropout_mask);
 }

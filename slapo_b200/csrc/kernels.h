@@ -47,6 +47,13 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
                  int K, int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act,
                  float* workspace, int* status, cudaStream_t stream);
 
+// out[i] = cache past[i] ([B, past_len, H, head_bytes] contiguous) followed along the tokens by
+// fresh[i] ([B, new_len, H, head_bytes], strides of B / token / head in bytes), i = k, v.
+// Everything 16-byte aligned.
+void launch_kv_append(const void* const past[2], const void* const fresh[2], void* const out[2],
+                      int64_t B, int64_t past_len, int64_t new_len, int64_t H, int64_t head_bytes,
+                      const int64_t (&fresh_strides)[2][3], cudaStream_t stream);
+
 // Cross entropy in two steps (per-row statistics, then gradient); see loss.cu.
 void launch_ce_stats(const void* logits, const int64_t* labels, float* stats, int rows, int cols,
                      int64_t row_stride, int vocab_start, int64_t ignore_index, int dtype,

@@ -192,8 +192,7 @@ class FlashAttention(nn.Module):
             k = self.reshape_for_scores(self.key(hidden_states))
             v = self.reshape_for_scores(self.value(hidden_states))
         if past is not None:
-            k = torch.cat((past[0], k), dim=1)
-            v = torch.cat((past[1], v), dim=1)
+            k, v = NF.append_kv(past[0], past[1], k, v)
         present = (k, v) if use_cache else None
         ctx = self.attn_op(q, k, v, attention_mask, self.attn_pdrop if self.training else 0.0)
         ctx = ctx.reshape(ctx.shape[:-2] + (-1,))
