@@ -203,6 +203,8 @@ class LinearWithDropout(LinearWithSyncFunc):
         self.p = p
 
     def forward(self, x):
+        if self.p == 0.0 or not self.training:
+            return self.matmul_sync(x, self.bias)      # nothing to drop: bias in the GEMM epilogue
         return NF.bias_dropout(self.matmul_sync(x), self.bias, self.p, self.training)
 
     def extra_repr(self):
