@@ -294,6 +294,7 @@ void register_gemm_ops(torch::Library& m);
 void register_attn_ops(torch::Library& m);
 void register_comm_ops(torch::Library& m);
 void register_loss_ops(torch::Library& m);
+void register_autograd_ops(torch::Library& m);
 
 TORCH_LIBRARY(slapo_b200, m) {
   m.def("philox_reserve(int increment) -> Tensor", &philox_reserve);
@@ -321,4 +322,5 @@ TORCH_LIBRARY(slapo_b200, m) {
   register_attn_ops(m);
   register_comm_ops(m);
   register_loss_ops(m);
+  register_autograd_ops(m);
 }

@@ -32,51 +32,6 @@ def native_supported(q, k, v) -> bool:
     return native.available()
 
 
-class _FlashAttnFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, key_bias, rel, causal, scale, p):
-        rng = native.ops().philox_reserve(q.shape[0] * q.shape[2] * q.shape[1] * k.shape[1]) \
-            if p > 0 else None
-        out, lse = native.ops().flash_attn_fwd(q, k, v, key_bias, rel, causal, scale, p, rng)
-        ctx.save_for_backward(q, k, v, out, lse, key_bias, rel)
-        ctx.cfg = (causal, scale, p, rng)
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        q, k, v, out, lse, key_bias, rel = ctx.saved_tensors
-        causal, scale, p, rng = ctx.cfg
-        dq, dk, dv, drel = native.ops().flash_attn_bwd(
-            dout.contiguous(), q, k, v, out, lse, key_bias, rel, causal, scale, p, rng, False)
-        return dq, dk, dv, None, (drel if rel is not None else None), None, None, None
-
-
-class _FlashAttnPackedFn(torch.autograd.Function):
-    """Same kernels on a packed projection output ``[B, S, H, 3, D]``: q, k, v
-    are read in place through strided views and the three gradients are
-    written into one tensor of the packed layout (no slicing copies, no
-    concatenation in autograd)."""
-
-    @staticmethod
-    def forward(ctx, qkv, key_bias, rel, causal, scale, p):
-        q, k, v = qkv[..., 0, :], qkv[..., 1, :], qkv[..., 2, :]
-        rng = native.ops().philox_reserve(q.shape[0] * q.shape[2] * q.shape[1] * k.shape[1]) \
-            if p > 0 else None
-        out, lse = native.ops().flash_attn_fwd(q, k, v, key_bias, rel, causal, scale, p, rng)
-        ctx.save_for_backward(qkv, out, lse, key_bias, rel)
-        ctx.cfg = (causal, scale, p, rng)
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        qkv, out, lse, key_bias, rel = ctx.saved_tensors
-        causal, scale, p, rng = ctx.cfg
-        q, k, v = qkv[..., 0, :], qkv[..., 1, :], qkv[..., 2, :]
-        dqkv, _, _, drel = native.ops().flash_attn_bwd(
-            dout.contiguous(), q, k, v, out, lse, key_bias, rel, causal, scale, p, rng, True)
-        return dqkv, None, (drel if rel is not None else None), None, None, None
-
-
 def relative_bias_by_distance(table, sq, sk, bidirectional, max_distance):
     """``[num_buckets, H]`` table -> ``[H, sq + sk - 1]`` bias per (key - query)."""
     from .functional import t5_relative_position_bucket
@@ -94,7 +49,7 @@ def flash_attention_native(q, k, v, key_bias, causal, scale, p, rel_table, rel_b
     rel = None
     if rel_table is not None:
         rel = relative_bias_by_distance(rel_table, q.shape[1], k.shape[1], rel_bidir, rel_maxd)
-    return _FlashAttnFn.apply(q, k, v, key_bias, rel, bool(causal), float(scale), float(p))
+    return native.ops().flash(q, k, v, key_bias, rel, bool(causal), float(scale), float(p))
 
 
 def flash_attention_qkvpacked(qkv, key_bias=None, causal=False, scale=None, p=0.0,
@@ -106,7 +61,7 @@ def flash_attention_qkvpacked(qkv, key_bias=None, causal=False, scale=None, p=0.
     rel = None
     if rel_table is not None:
         rel = relative_bias_by_distance(rel_table, qkv.shape[1], qkv.shape[1], rel_bidir, rel_maxd)
-    return _FlashAttnPackedFn.apply(qkv, key_bias, rel, bool(causal), float(scale), float(p))
+    return native.ops().flash(qkv, None, None, key_bias, rel, bool(causal), float(scale), float(p))
 
 
 def packed_supported(qkv) -> bool:

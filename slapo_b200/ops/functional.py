@@ -57,26 +57,10 @@ def _act_code(act):
     return {"gelu": 0, "relu": 2}.get(act, 1)
 
 
-class _BiasActFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, bias, act):
-        ctx.act = act
-        ctx.has_bias = bias is not None
-        ctx.save_for_backward(x, bias)
-        return native.ops().bias_act_fwd(x.contiguous(), bias, _act_code(act))
-
-    @staticmethod
-    def backward(ctx, grad):
-        x, bias = ctx.saved_tensors
-        dx, dbias = native.ops().bias_act_bwd(grad.contiguous(), x.contiguous(), bias,
-                                              _act_code(ctx.act))
-        return dx, (dbias if ctx.has_bias else None), None
-
-
 def bias_act(x, bias, act: str = "gelu"):
     """``act(x + bias)``; act in gelu (erf) / gelu_new (tanh) / relu."""
     if _native_ok(x) and x.shape[-1] % 8 == 0:
-        return _BiasActFn.apply(x, bias, act)
+        return native.ops().bias_act(x, bias, _act_code(act))
     return _act_ref(x + bias if bias is not None else x, act)
 
 
@@ -98,14 +82,6 @@ def gemm_supported(x, weight) -> bool:
             and x.numel() > 0 and _native_ok(x))
 
 
-def _rows(t):
-    """``t`` as a 2-D matrix with contiguous rows whose stride TMA accepts."""
-    t2 = t.reshape(-1, t.shape[-1])
-    if t2.stride(1) != 1 or t2.stride(0) % 8 or t2.data_ptr() % 16:
-        t2 = t2.contiguous()
-    return t2
-
-
 def gemm(a, b, bias=None, act=-1, a_mn=False, b_mn=False, out=None, pre_act=None, split_k=False):
     """``act(A B^T + bias)`` on this library's tcgen05 kernels (CTA pairs where the problem
     has a pair tile).  ``a_mn`` / ``b_mn``: the operand is stored ``[K, M]`` / ``[K, N]``."""
@@ -115,70 +91,6 @@ def gemm(a, b, bias=None, act=-1, a_mn=False, b_mn=False, out=None, pre_act=None
 _RELU = 2
 
 
-class _LinearFn(torch.autograd.Function):
-    """``y = x W^T + b`` (optionally ``relu`` of it): three GEMMs of this library, none of them
-    transposing an operand in memory.  The bias rides in the forward GEMM's epilogue and so
-    does ReLU, whose derivative the backward reads off the output (``y > 0``).  GeLU is NOT
-    fused: the four epilogue warps of a tcgen05 GEMM have a fraction of the SM's FP32 issue
-    rate, and an erf per element made the GEMM 2.5 x slower than running
-    :func:`bias_act` over the output afterwards."""
-
-    @staticmethod
-    def forward(ctx, x, weight, bias, act):
-        x2 = _rows(x)
-        y = gemm(x2, weight, bias, act)
-        ctx.act, ctx.has_bias = act, bias is not None
-        ctx.save_for_backward(x2, weight, y if act >= 0 else None)
-        ctx.x_shape = x.shape
-        return y.view(tuple(x.shape[:-1]) + (weight.shape[0],))
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2, weight, y = ctx.saved_tensors
-        dy2 = _rows(dy)
-        dbias = None
-        if ctx.act >= 0:
-            # relu'(z) = (y > 0): the saved output stands in for the pre-activation
-            dy2, dbias = native.ops().act_bwd_colsum(dy2.contiguous(), y, ctx.act)
-        elif ctx.has_bias and ctx.needs_input_grad[2]:
-            dbias = native.ops().colsum(dy2)
-        dx = dw = None
-        if ctx.needs_input_grad[0]:
-            # dX = dZ W:  B = W [N, K] read N-major (its rows are the contraction)
-            dx = gemm(dy2, weight, b_mn=True).view(ctx.x_shape)
-        if ctx.needs_input_grad[1]:
-            # dW = dZ^T X:  A = dZ [T, N] read M-major, B = X [T, K] read N-major; few tiles and a
-            # long contraction, hence split-K
-            dw = gemm(dy2, x2, a_mn=True, b_mn=True, split_k=True)
-        return dx, dw, (dbias if ctx.has_bias else None), None
-
-
-class _LinearTFn(torch.autograd.Function):
-    """``y = x W + b`` with ``W`` stored ``[in, out]`` (GPT-2's ``Conv1D``): the same three
-    GEMMs with the operand roles read the other way round, again without a transpose in memory."""
-
-    @staticmethod
-    def forward(ctx, x, weight, bias):
-        x2 = _rows(x)
-        y = gemm(x2, weight, bias, b_mn=True)            # B = W [K, N] read N-major
-        ctx.has_bias = bias is not None
-        ctx.save_for_backward(x2, weight)
-        ctx.x_shape = x.shape
-        return y.view(tuple(x.shape[:-1]) + (weight.shape[1],))
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2, weight = ctx.saved_tensors
-        dy2 = _rows(dy)
-        dbias = native.ops().colsum(dy2) if ctx.has_bias and ctx.needs_input_grad[2] else None
-        dx = dw = None
-        if ctx.needs_input_grad[0]:
-            dx = gemm(dy2, weight).view(ctx.x_shape)      # dX = dY W^T: B = W [in, out] K-major
-        if ctx.needs_input_grad[1]:
-            dw = gemm(x2, dy2, a_mn=True, b_mn=True, split_k=True)    # dW = X^T dY
-        return dx, dw, dbias
-
-
 def linear_t(x, weight, bias=None):
     """``x @ weight + bias`` for a weight stored ``[in_features, out_features]``."""
     if (torch.is_tensor(x) and x.is_cuda and x.dtype in (torch.bfloat16, torch.float16)
@@ -186,7 +98,7 @@ def linear_t(x, weight, bias=None):
             and weight.shape[0] % 8 == 0 and weight.shape[1] % 8 == 0 and weight.stride(0) % 8 == 0
             and x.numel() > 0 and os.environ.get("SLAPO_B200_LIBRARY_GEMM", "0") != "1"
             and _native_ok(x)):
-        return _LinearTFn.apply(x, weight, bias)
+        return native.ops().linear(x, weight, bias, -1, True)
     out = torch.matmul(x, weight)
     return out if bias is None else out + bias
 
@@ -197,8 +109,11 @@ def linear(x, weight, bias=None, act=None):
     else PyTorch."""
     if gemm_supported(x, weight):
         if act is None or act == "relu":
-            return _LinearFn.apply(x, weight, bias, -1 if act is None else _RELU)
-        return bias_act(_LinearFn.apply(x, weight, None, -1), bias, act)
+            return native.ops().linear(x, weight, bias, -1 if act is None else _RELU, False)
+        # GeLU is NOT fused: the epilogue warps of a tcgen05 GEMM have a fraction of the SM's
+        # FP32 issue rate, and an erf per element made the GEMM 2.5 x slower than running
+        # bias_act over the output afterwards
+        return bias_act(native.ops().linear(x, weight, None, -1, False), bias, act)
     out = F.linear(x, weight, bias)
     return out if act is None else _act_ref(out, act)
 
@@ -213,34 +128,10 @@ def effective_dropout_p(p: float) -> float:
     return min(max(int(p * 128.0 + 0.5), 0), 127) / 128.0
 
 
-def _philox_reserve(numel):
-    """Reserve Philox offsets on the current CUDA generator (so masks follow
-    torch's RNG state: manual_seed, fork_rng, checkpoint replay).  Returns the
-    opaque CPU int64[4] state the kernels take; valid under graph capture."""
-    return native.ops().philox_reserve(int(numel))
-
-
-class _BiasDropoutAddFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, bias, residual, p):
-        rng = _philox_reserve(x.numel())
-        ctx.p, ctx.rng = p, rng
-        ctx.has_bias, ctx.has_res = bias is not None, residual is not None
-        return native.ops().bias_dropout_add_fwd(
-            x.contiguous(), bias, residual.contiguous() if residual is not None else None,
-            p, rng)
-
-    @staticmethod
-    def backward(ctx, grad):
-        grad = grad.contiguous()
-        dx, dbias = native.ops().bias_dropout_add_bwd(grad, ctx.p, ctx.rng, ctx.has_bias)
-        return dx, (dbias if ctx.has_bias else None), (grad if ctx.has_res else None), None
-
-
 def bias_dropout_add(x, bias, residual, p: float, training: bool = True):
     """``dropout(x + bias, p) + residual`` (bias / residual may be None)."""
     if _native_ok(x) and training and p > 0.0 and x.shape[-1] % 8 == 0:
-        return _BiasDropoutAddFn.apply(x, bias, residual, p)
+        return native.ops().bias_dropout_add(x, bias, residual, p)
     out = x + bias if bias is not None else x
     out = F.dropout(out, p, training)
     return out + residual if residual is not None else out
@@ -252,64 +143,18 @@ def bias_dropout(x, bias, p: float, training: bool = True):
 
 # ---------------------------------------------------------------------- #
 # normalisation
-class _LayerNormFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, bias, eps, rms):
-        shape = x.shape
-        x2 = x.contiguous().view(-1, shape[-1])
-        y, mean, rstd = native.ops().layer_norm_fwd(x2, weight, bias, eps, rms)
-        ctx.save_for_backward(x2, weight, mean, rstd)
-        ctx.rms, ctx.has_bias, ctx.shape = rms, bias is not None, shape
-        return y.view(shape)
-
-    @staticmethod
-    def backward(ctx, grad):
-        x2, weight, mean, rstd = ctx.saved_tensors
-        g2 = grad.contiguous().view(-1, ctx.shape[-1])
-        dx, dw, db = native.ops().layer_norm_bwd(g2, x2, weight, mean, rstd, ctx.rms)
-        return dx.view(ctx.shape), dw, (db if ctx.has_bias else None), None, None
-
-
 def layer_norm(x, weight, bias, eps: float = 1e-5):
     if _native_ok(x) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 16384:
-        return _LayerNormFn.apply(x, weight, bias, eps, False)
+        return native.ops().norm(x, weight, bias, eps, False)
     return F.layer_norm(x, (x.shape[-1],), weight, bias, eps)
 
 
 def rms_norm(x, weight, eps: float = 1e-6):
     """T5-style RMS norm: no mean subtraction, no bias, fp32 statistics."""
     if _native_ok(x) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 16384:
-        return _LayerNormFn.apply(x, weight, None, eps, True)
+        return native.ops().norm(x, weight, None, eps, True)
     var = x.float().pow(2).mean(-1, keepdim=True)
     return (x.float() * torch.rsqrt(var + eps)).to(x.dtype) * weight
-
-
-class _DropoutAddLayerNormFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, bias, residual, weight, ln_bias, p, eps, training):
-        shape = x.shape
-        cols = shape[-1]
-        x2 = x.contiguous().view(-1, cols)
-        r2 = residual.contiguous().view(-1, cols)
-        p_eff = p if training else 0.0
-        rng = _philox_reserve(x.numel()) if p_eff > 0 else None
-        y, z, mean, rstd = native.ops().dropout_add_ln_fwd(
-            x2, bias, r2, weight, ln_bias, p_eff, eps, rng)
-        ctx.save_for_backward(z, weight, mean, rstd)
-        ctx.p, ctx.rng = p_eff, rng
-        ctx.has_bias, ctx.shape = bias is not None, shape
-        return y.view(shape), z.view(shape)
-
-    @staticmethod
-    def backward(ctx, gy, gz):
-        z, weight, mean, rstd = ctx.saved_tensors
-        cols = ctx.shape[-1]
-        gy2 = gy.contiguous().view(-1, cols)
-        gz2 = gz.contiguous().view(-1, cols) if gz is not None else None
-        dx, dres, dw, db, dbias = native.ops().dropout_add_ln_bwd(
-            gy2, gz2, z, weight, mean, rstd, ctx.p, ctx.rng, ctx.has_bias)
-        return (dx.view(ctx.shape), (dbias if ctx.has_bias else None), dres.view(ctx.shape),
-                dw, db, None, None, None)
 
 
 def dropout_add_layer_norm(x, bias, residual, weight, ln_bias, p: float, eps: float,
@@ -319,7 +164,8 @@ def dropout_add_layer_norm(x, bias, residual, weight, ln_bias, p: float, eps: fl
     ``z`` is returned because a pre-LN block needs it as the next residual; a
     post-LN block (BERT) just drops it."""
     if _native_ok(x) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 16384:
-        return _DropoutAddLayerNormFn.apply(x, bias, residual, weight, ln_bias, p, eps, training)
+        return native.ops().dropout_add_norm(x, bias, residual, weight, ln_bias,
+                                             p if training else 0.0, eps)
     z = x + bias if bias is not None else x
     z = F.dropout(z, p, training) + residual
     return F.layer_norm(z, (z.shape[-1],), weight, ln_bias, eps), z
