@@ -177,6 +177,36 @@ std::tuple<Tensor, Tensor> kv_append(const Tensor& past_k, const Tensor& past_v,
   return {out[0], out[1]};
 }
 
+// T5's table [buckets, H] by distance, and its gradient (see rel_bias.cu)
+int rel_dtype(const Tensor& t) {
+  return t.scalar_type() == at::kBFloat16 ? 0 : (t.scalar_type() == at::kHalf ? 1 : 2);
+}
+
+Tensor rel_bias_fwd(const Tensor& table, const Tensor& buckets) {
+  TORCH_CHECK(table.is_cuda() && table.dim() == 2 && table.is_contiguous() &&
+                  (rel_dtype(table) < 2 || table.scalar_type() == at::kFloat),
+              "rel_bias: a contiguous [buckets, H] CUDA table of fp32, bf16 or fp16 required");
+  TORCH_CHECK(buckets.is_cuda() && buckets.dim() == 1 && buckets.is_contiguous() &&
+                  buckets.scalar_type() == at::kLong, "rel_bias: int64 buckets required");
+  c10::cuda::CUDAGuard guard(table.device());
+  const int n = static_cast<int>(buckets.numel()), H = static_cast<int>(table.size(1));
+  Tensor out = at::empty({H, n}, table.options().dtype(at::kFloat));
+  slapo::launch_rel_bias_fwd(table.data_ptr(), buckets.data_ptr<int64_t>(), out.data_ptr<float>(), n, H,
+                             rel_dtype(table), at::cuda::getCurrentCUDAStream().stream());
+  return out;
+}
+
+Tensor rel_bias_bwd(const Tensor& grad, const Tensor& buckets, const Tensor& table) {
+  TORCH_CHECK(grad.is_cuda() && grad.is_contiguous() && grad.scalar_type() == at::kFloat);
+  c10::cuda::CUDAGuard guard(table.device());
+  Tensor dtable = at::empty(table.sizes(), table.options());
+  slapo::launch_rel_bias_bwd(grad.data_ptr<float>(), buckets.data_ptr<int64_t>(), dtable.data_ptr(),
+                             static_cast<int>(buckets.numel()), static_cast<int>(table.size(1)),
+                             static_cast<int>(table.size(0)), rel_dtype(table),
+                             at::cuda::getCurrentCUDAStream().stream());
+  return dtable;
+}
+
 }  // namespace
 
 void register_attn_ops(torch::Library& m) {
@@ -185,6 +215,8 @@ void register_attn_ops(torch::Library& m) {
   m.def("flash_attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor? kbias, Tensor? rel, bool causal, float scale, float p_drop, Tensor? rng, bool packed_qkv) -> (Tensor, Tensor, Tensor, Tensor)",
         &flash_attn_bwd);
   m.def("kv_append(Tensor past_k, Tensor past_v, Tensor k, Tensor v) -> (Tensor, Tensor)", &kv_append);
+  m.def("rel_bias_fwd(Tensor table, Tensor buckets) -> Tensor", &rel_bias_fwd);
+  m.def("rel_bias_bwd(Tensor grad, Tensor buckets, Tensor table) -> Tensor", &rel_bias_bwd);
   m.def("flash_attn_dropout_mask(int B, int H, int Sq, int Sk, float p_drop, Tensor rng) -> Tensor",
         &flash_attn_dropout_mask);
 }

@@ -272,6 +272,21 @@ struct FlashFn : public Function<FlashFn> {
   }
 };
 
+// T5's relative-position table by distance: [buckets, H] -> [H, n] fp32
+struct RelBiasFn : public Function<RelBiasFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& table, const Tensor& buckets) {
+    Tensor t = table.contiguous();
+    ctx->save_for_backward({t, buckets});
+    static auto f = op<Tensor(const Tensor&, const Tensor&)>("slapo_b200::rel_bias_fwd");
+    return f.call(t, buckets);
+  }
+  static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    static auto f = op<Tensor(const Tensor&, const Tensor&, const Tensor&)>("slapo_b200::rel_bias_bwd");
+    return {f.call(grads[0].contiguous(), s[1], s[0]), Tensor()};
+  }
+};
+
 // ------------------------------------------------------------------------ //
 Tensor linear(const Tensor& x, const Tensor& weight, const optional<Tensor>& bias, int64_t act,
               bool transposed) {
@@ -299,6 +314,8 @@ Tensor flash(const Tensor& q, const optional<Tensor>& k, const optional<Tensor>&
   return FlashFn::apply(q, k, v, key_bias, rel, causal, scale, p);
 }
 
+Tensor rel_bias(const Tensor& table, const Tensor& buckets) { return RelBiasFn::apply(table, buckets); }
+
 }  // namespace
 
 void register_autograd_ops(torch::Library& m) {
@@ -309,6 +326,7 @@ void register_autograd_ops(torch::Library& m) {
   m.def("norm(Tensor x, Tensor weight, Tensor? bias, float eps, bool rms) -> Tensor", &norm);
   m.def("dropout_add_norm(Tensor x, Tensor? bias, Tensor residual, Tensor weight, Tensor? ln_bias, float p, float eps) -> (Tensor, Tensor)",
         &dropout_add_norm);
+  m.def("rel_bias(Tensor table, Tensor buckets) -> Tensor", &rel_bias);
   m.def("flash(Tensor q, Tensor? k, Tensor? v, Tensor? key_bias, Tensor? rel, bool causal, float scale, float p) -> Tensor",
         &flash);
 }

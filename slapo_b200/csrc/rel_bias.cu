@@ -1,0 +1,60 @@
+// T5's relative-position table [buckets, H] as a bias by distance [H, n], and its gradient.
+//
+// Both are latency-bound (n is a few thousand): one launch each, where indexing the table with
+// torch operators took a cast, a gather and a transposing copy, and its gradient an index-add
+// that serialises on the few rows of the table (85 us at 1023 distances x 16 heads).
+#include "common.cuh"
+#include "kernels.h"
+
+namespace slapo {
+
+template <typename T>
+__global__ void __launch_bounds__(256) rel_bias_fwd_kernel(const T* __restrict__ table,
+                                                           const int64_t* __restrict__ buckets,
+                                                           float* __restrict__ out, int n, int H) {
+  const int d = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y;
+  if (d < n)
+    out[static_cast<int64_t>(h) * n + d] = static_cast<float>(table[buckets[d] * H + h]);
+}
+
+// one block per head; each warp sums the distances of one bucket at a time (fp32, fixed order)
+template <typename T>
+__global__ void __launch_bounds__(256) rel_bias_bwd_kernel(const float* __restrict__ grad,
+                                                           const int64_t* __restrict__ buckets,
+                                                           T* __restrict__ dtable, int n, int H,
+                                                           int n_buckets) {
+  const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float* g = grad + static_cast<int64_t>(h) * n;
+  for (int b = warp; b < n_buckets; b += 8) {
+    float s = 0.f;
+    for (int d = lane; d < n; d += 32)
+      if (buckets[d] == b) s += g[d];
+    s = warp_sum(s);
+    if (lane == 0) dtable[static_cast<int64_t>(b) * H + h] = static_cast<T>(s);
+  }
+}
+
+#define DISPATCH_DTYPE(dtype, ...)                                   \
+  switch (dtype) {                                                   \
+    case 0: { using T = __nv_bfloat16; __VA_ARGS__; break; }         \
+    case 1: { using T = __half; __VA_ARGS__; break; }                \
+    default: { using T = float; __VA_ARGS__; break; }                \
+  }
+
+void launch_rel_bias_fwd(const void* table, const int64_t* buckets, float* out, int n, int H,
+                         int dtype, cudaStream_t stream) {
+  if (n == 0 || H == 0) return;
+  count_launch();
+  DISPATCH_DTYPE(dtype, (rel_bias_fwd_kernel<T><<<dim3((n + 255) / 256, H), 256, 0, stream>>>(
+      static_cast<const T*>(table), buckets, out, n, H)));
+}
+
+void launch_rel_bias_bwd(const float* grad, const int64_t* buckets, void* dtable, int n, int H,
+                         int n_buckets, int dtype, cudaStream_t stream) {
+  if (H == 0 || n_buckets == 0) return;
+  count_launch();
+  DISPATCH_DTYPE(dtype, (rel_bias_bwd_kernel<T><<<H, 256, 0, stream>>>(
+      grad, buckets, static_cast<T*>(dtable), n, H, n_buckets)));
+}
+
+}  // namespace slapo

@@ -32,13 +32,20 @@ def native_supported(q, k, v) -> bool:
     return native.available()
 
 
-def relative_bias_by_distance(table, sq, sk, bidirectional, max_distance):
-    """``[num_buckets, H]`` table -> ``[H, sq + sk - 1]`` bias per (key - query)."""
+def _distance_buckets(device, sq, sk, n_buckets, bidirectional, max_distance):
+    """Bucket of every distance key - query, ``[sq + sk - 1]`` int64."""
     from .functional import t5_relative_position_bucket
 
     # query i sits at absolute position i + (sk - sq); distance = key - that
-    dist = torch.arange(-(sq - 1), sk, device=table.device) - (sk - sq)
-    buckets = t5_relative_position_bucket(dist, bidirectional, table.shape[0], max_distance)
+    dist = torch.arange(-(sq - 1), sk, device=device) - (sk - sq)
+    return t5_relative_position_bucket(dist, bidirectional, n_buckets, max_distance)
+
+
+def relative_bias_by_distance(table, sq, sk, bidirectional, max_distance):
+    """``[num_buckets, H]`` table -> ``[H, sq + sk - 1]`` bias per (key - query)."""
+    buckets = _distance_buckets(table.device, sq, sk, table.shape[0], bidirectional, max_distance)
+    if table.dtype in (torch.bfloat16, torch.float16, torch.float32) and native.available():
+        return native.ops().rel_bias(table, buckets)
     return table.float()[buckets].t().contiguous()
 
 
