@@ -338,15 +338,15 @@ static int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const Ge
 
 // Returns 0 on success; >0 = host-side refusal (bad shape / alignment / driver).
 int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
-                int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act, int* status,
-                cudaStream_t stream) {
+                int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act, int bn,
+                int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (N % 8 || K % 8 || lda % 8 || ldb % 8 || ldc % 8) return 1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) |
        reinterpret_cast<uintptr_t>(C)) & 15)
     return 1;
   if (a_mn && M % 8) return 1;
-  const int BN = N > 128 ? 256 : (N > 64 ? 128 : 64);
+  const int BN = bn != 0 ? bn : (N > 128 ? 256 : (N > 64 ? 128 : 64));
   CUtensorMap ta, tb;
   bool ok;
   // K-major: [rows, K] -> inner K, outer rows, box 64 x rows_per_tile

@@ -455,13 +455,42 @@ int gemm2_splits(int M, int N, int K, int bn) {
   return (num_kb + per - 1) / per;     // no empty split
 }
 
+// Small products are one wave of few tiles, whatever the tile: the launch, the first loads and
+// the epilogue of ONE tile are what they take, and narrow tiles have less of all three and put
+// more SMs on the weights.  Measured per call (us, B in L2; wide = the tile that large products
+// use, 256 x 256 per pair or, up to 128 rows, 128 x 256):
+//     M x N x K             128 x 64   256 x 128 pair   wide
+//     8 x 2048 x 2048         12.9           -          14.5
+//     200 x 3072 x 768         8.0          9.4         12.0
+//     512 x 1024 x 1024        8.6         10.4         13.3
+//     768 x 768 x 64           4.4          7.1          9.2
+//     384 x 4096 x 1024       14.4         10.8         13.7
+//     2048 x 1024 x 4096      43.0         23.1         27.5
+//     1024 x 3072 x 1024      20.1         14.9         13.9
+// So: tiles of 64 columns while they fit one wave of CTAs and the contraction is short (a narrow
+// tile pays more per step of it: 18.3 against 17.6 us at 200 x 768 x 3072), pairs of 128 columns
+// while those fit one wave of pairs, wide tiles beyond.  Up to 128 rows there is no pair tile: the
+// narrowest of 64 / 128 / 256 columns that fits one wave.
+GemmTile gemm_tile(int M, int N, int K) {
+  const int sms = sm_count();
+  const int64_t rows = (M + PBM - 1) / PBM, pair_rows = (M + 2 * PBM - 1) / (2 * PBM);
+  if (M <= PBM) {
+    if (rows * ((N + 63) / 64) <= sms) return {false, 64};
+    if (rows * ((N + 127) / 128) <= sms) return {false, 128};
+    return {false, 0};
+  }
+  if (K <= 2048 && rows * ((N + 63) / 64) <= sms) return {false, 64};
+  if (pair_rows * ((N + 127) / 128) <= sms / 2) return {true, 128};
+  return {true, 0};
+}
+
 // C = act(A B^T + bias) on CTA pairs.  `workspace`: scratch for split-K, gemm2_splits() * M * N
 // floats of any contents, or null (no split).
 // Returns 0 on success; >0 = refused on the host (shape / alignment / driver), 5 = too small
 // for a pair tile (use launch_gemm).
 int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bias, int M, int N,
                  int K, int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act,
-                 float* workspace, int* status, cudaStream_t stream) {
+                 int bn, float* workspace, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (N % 8 || K % 8 || lda % 8 || ldb % 8 || ldc % 8) return 1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) |
@@ -469,7 +498,7 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
     return 1;
   if (a_mn && M % 8) return 1;
   if (M <= PBM || N <= 64) return 5;
-  const int BN = N > 128 ? 256 : 128;
+  const int BN = bn != 0 ? bn : (N > 128 ? 256 : 128);
   CUtensorMap ta, tb;
   bool ok = a_mn ? cached_tmap_2d(&ta, A, M, K, lda, PBK, bf16)
                  : cached_tmap_2d(&ta, A, K, M, lda, PBM, bf16);

@@ -84,14 +84,17 @@ Tensor gemm_out(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& b
   const bool bf16 = a.scalar_type() == at::kBFloat16;
   auto stream = at::cuda::getCurrentCUDAStream().stream();
   int rc = 5;
-  if (impl != 1) {
+  const int splits = split_k && impl != 1 ? slapo::gemm2_splits(M, N, K, N > 128 ? 256 : 128) : 1;
+  // a second output and several pairs per tile exist on the pair kernel's default tile only
+  slapo::GemmTile tile{impl != 1, 0};
+  if (impl == 0 && splits == 1 && c2 == nullptr) tile = slapo::gemm_tile(M, N, K);
+  if (tile.pair) {
     float* ws = nullptr;
-    const int splits = split_k ? slapo::gemm2_splits(M, N, K, N > 128 ? 256 : 128) : 1;
     if (splits > 1) ws = split_scratch(dev, static_cast<int64_t>(splits) * M * N).data_ptr<float>();
     rc = slapo::launch_gemm2(a.data_ptr(), b.data_ptr(), c.data_ptr(), c2, bias_ptr, M, N, K,
                              static_cast<int>(a.stride(0)), static_cast<int>(b.stride(0)),
                              static_cast<int>(c.stride(0)), a_mn, b_mn, bf16,
-                             static_cast<int>(act), ws,
+                             static_cast<int>(act), tile.bn, ws,
                              status_word(dev).data_ptr<int>(), stream);
     TORCH_CHECK(impl != 2 || rc == 0, "gemm: the CTA-pair kernel refused the launch (code ", rc, ")");
   }
@@ -100,7 +103,7 @@ Tensor gemm_out(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& b
     rc = slapo::launch_gemm(a.data_ptr(), b.data_ptr(), c.data_ptr(), bias_ptr, M, N, K,
                             static_cast<int>(a.stride(0)), static_cast<int>(b.stride(0)),
                             static_cast<int>(c.stride(0)), a_mn, b_mn, bf16, static_cast<int>(act),
-                            status_word(dev).data_ptr<int>(), stream);
+                            tile.pair ? 0 : tile.bn, status_word(dev).data_ptr<int>(), stream);
   }
   TORCH_CHECK(rc == 0, "gemm: launch refused (code ", rc,
               "): sizes must be multiples of 8 and pointers 16-byte aligned");

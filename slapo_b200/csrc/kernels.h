@@ -35,17 +35,21 @@ void launch_fused_adamw(void* param, const void* grad, float* master, float* exp
 // C[M,N] = act(A B^T + bias); a_mn / b_mn select M/N-major operands (see gemm.cu).
 // Returns 0 on success, >0 when the launch was refused on the host.
 int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
-                int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act, int* status,
-                cudaStream_t stream);
+                int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act, int bn,
+                int* status, cudaStream_t stream);
 
 // The same product on CTA pairs (gemm2.cu): 256 x 256 tiles shared by two SMs, optional second
 // output `C2` (the value before the activation), optional split-K through `workspace`
 // (gemm2_splits() * M * N floats of scratch).  Returns 5 when
 // the problem is smaller than one pair tile (use launch_gemm).
 int gemm2_splits(int M, int N, int K, int bn);
+// Tile for a product: CTA pairs or single CTAs, and the tile's columns (`bn` of the launchers;
+// there 0 = the widest that N fills).
+struct GemmTile { bool pair; int bn; };
+GemmTile gemm_tile(int M, int N, int K);
 int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bias, int M, int N,
                  int K, int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act,
-                 float* workspace, int* status, cudaStream_t stream);
+                 int bn, float* workspace, int* status, cudaStream_t stream);
 
 // out[i] = cache past[i] ([B, past_len, H, head_bytes] contiguous) followed along the tokens by
 // fresh[i] ([B, new_len, H, head_bytes], strides of B / token / head in bytes), i = k, v.
