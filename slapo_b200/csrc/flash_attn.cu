@@ -20,6 +20,11 @@
 // What bounds it: the special-function unit (one exp2 per score, 1024 cycles per 128 x 128 tile
 // and SM) next to the issue slots of the softmax warps.  One thread per whole row needs no
 // exchange between warps; for D = 64 two independent CTAs fill each other's waits.
+// Measured (one kernel, before: P through shared memory, O folded in registers, one work item per
+// CTA -> now): 32 x 512 x 16 heads of 64, p 0.1: 125 -> 107 us; 4 x 2048 x 16 x 128 causal: 299 ->
+// 127 us; 4 x 1000 x 32 x 80 causal with key bias: 180 -> 147 us; 8 x 512 x 16 x 64 with T5's bias,
+// key bias and p 0.1: 67 -> 73 us (per-element bias loads); 1 query x 1501 keys x 8 x 16 x 128,
+// keys split: 53 -> 31 + 3 us.
 #include "flash_common.cuh"
 #include "kernels.h"
 
