@@ -17,8 +17,9 @@
 // S with its rows where they want them.
 //
 // The order of the products keeps the tensor core and the softmax warps apart:
-//   tensor   ... P Y2 (t)   S (t+1)      dS Y1 (t)   dP (t+1) ...
+//   tensor   ... S (t+1)   P Y2 (t)      dP (t+1)   dS Y1 (t) ...
 //   softmax      dS (t)          P (t+1)          dS (t+1)
+// (D = 128: each pair the other way round).
 // CTAs are persistent; the loads and the first S of the next work item run under the last tile of
 // this one, and its accumulators are read out after the first P of the next.
 //
@@ -28,7 +29,7 @@
 // exp2, pack, TMEM store, barrier, product); exp2 alone needs 1024 cycles per tile and pass.  Twice
 // the softmax warps on half the columns each changed nothing (181 -> 185 and 144 -> 153 us).
 // Measured (all kernels of the backward, before -> now): 32 x 512 x 16 heads of 64, p 0.1: 360 ->
-// 338 us; 4 x 2048 x 16 x 128 causal: 655 -> 395 us; 4 x 1000 x 32 x 80 causal: 345 -> 226 us.
+// 317 us; 4 x 2048 x 16 x 128 causal: 655 -> 395 us; 4 x 1000 x 32 x 80 causal: 345 -> 226 us.
 //
 // With dropout the dQ pass draws the keep decisions (16 keys of a query row per Philox call, as
 // in the forward) and leaves them as one bit each, [B H][key / 32][query] words, for the dK / dV
@@ -178,6 +179,12 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
   constexpr bool kOver = kKeys && D == 128;
   constexpr uint32_t kColP = kOver ? kColS : 384, kColDS = kOver ? kColDP : (kKeys ? 448 : 256 + D);
   constexpr uint32_t kHalf = kOver ? 64 : 32;    // columns from one half of P / dS to the other
+  // With columns of their own, the next tile's S and dP need only that the softmax warps have read
+  // this tile's, and those warps wait for them: they go before the accumulating products.  That
+  // took the passes at D = 64 from 181 + 144 to 165 + 138 us (32 x 512 x 16 heads, p 0.1); at
+  // D = 128 the products are twice as long and two stages leave the loads less slack, and the dQ
+  // pass lost (170 -> 183 us at 4 x 2048 x 16, causal).
+  constexpr bool kFirst = D == 64;
   const int items = p.walk.items();
   const bool drop = p.thr7 != 0;
 
@@ -349,6 +356,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
           const bool same = j + 1 < n, more = same || next_n > 0;
           const bool next_last = same ? j + 2 == n : next_n == 1;
           if (!tc::mbar_wait(p_ready, t & 1, abort_flag)) { ok = false; break; }
+          const int next_w = same ? w : w + 1;
+          if (kFirst && more && !issue_s(t + 1, next_w, !same, next_last)) { ok = false; break; }
           if constexpr (kKeys) {
             // the accumulators of the item before have been read out
             if (j == 0 && !tc::mbar_wait(acc_free, (w & 1) ^ 1, abort_flag)) { ok = false; break; }
@@ -357,8 +366,9 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
             tc::umma_commit(a2_done);
             if (kOver && more && !tc::mbar_wait(a2_done, t & 1, abort_flag)) { ok = false; break; }
           }
-          if (more && !issue_s(t + 1, same ? w : w + 1, !same, next_last)) { ok = false; break; }
+          if (!kFirst && more && !issue_s(t + 1, next_w, !same, next_last)) { ok = false; break; }
           if (!tc::mbar_wait(ds_ready, t & 1, abort_flag)) { ok = false; break; }
+          if (kFirst && more && !issue_dp(t + 1, next_w, !same, next_last)) { ok = false; break; }
           if constexpr (!kKeys) {
             if (j == 0 && !tc::mbar_wait(acc_free, (w & 1) ^ 1, abort_flag)) { ok = false; break; }
           }
@@ -368,7 +378,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
           tc::umma_commit(&y_empty[st]);
           if (j + 1 == n) tc::umma_commit(acc_full);
           if (kOver && more && !tc::mbar_wait(a1_done, t & 1, abort_flag)) { ok = false; break; }
-          if (more && !issue_dp(t + 1, same ? w : w + 1, !same, next_last)) { ok = false; break; }
+          if (!kFirst && more && !issue_dp(t + 1, next_w, !same, next_last)) { ok = false; break; }
         }
         item = next_item;
         n = next_n;
