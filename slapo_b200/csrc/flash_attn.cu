@@ -367,13 +367,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const float m_tile = fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3])) * sc;
         // P of the tile before has been read (and O includes it)
         if (t > 0 && !tc::mbar_wait_warp(pv_done, (t - 1) & 1, abort_flag)) { ok = false; break; }
+        tc::fence_after_sync();
         if (j == 0) {
           m_ref = m_tile;
         } else if (__any_sync(0xffffffffu, m_tile > m_ref + kRaise)) {
           const float m_new = fmaxf(m_ref, m_tile);
           const float alpha = m_ref == -INFINITY ? 0.f : exp2f(m_ref - m_new);
           const uint64_t alpha2 = f2_pack(alpha, alpha);
-          tc::fence_after_sync();
 #pragma unroll
           for (int c = 0; c < D / 16; ++c) {
             uint32_t o[16];

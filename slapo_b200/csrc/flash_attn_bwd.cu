@@ -586,6 +586,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
             ok = false;
             break;
           }
+          tc::fence_after_sync();
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             uint32_t pk[16];
