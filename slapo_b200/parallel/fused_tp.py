@@ -100,6 +100,13 @@ def _debug_check(ctx, epoch, a_ptrs, b_ptrs, M, N, K, lda, ldb, dtype, gather, s
             raise ValueError("chunk flag pad is too small")
 
 
+def _rows(x):
+    """``[T, K]`` with contiguous rows whose stride and start TMA accepts."""
+    if x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
+        return x.contiguous()
+    return x
+
+
 def _wgrad(dy, x):
     """``dW = dY^T X`` on this library's split-K GEMM (both operands read as stored: ``dY``
     M-major, ``X`` N-major); tensors the kernel cannot address go to PyTorch."""
@@ -529,7 +536,7 @@ class _ColLinearARBwd(torch.autograd.Function):
         ctx.save_for_backward(x, w)
         ctx.has_bias = bias is not None
         if NF.gemm_supported(x, w):
-            return NF.gemm(NF._rows(x), w, bias)
+            return NF.gemm(_rows(x), w, bias)
         return torch.nn.functional.linear(x, w, bias)
 
     @staticmethod
