@@ -272,20 +272,32 @@ struct FlashFn : public Function<FlashFn> {
   }
 };
 
-// T5's relative-position table by distance: [buckets, H] -> [H, n] fp32
+// T5's relative-position table by distance, [buckets, H] -> [H, n] fp32, and the sum over the
+// distances of each bucket: linear maps, each the other's derivative (of any order).
 struct RelBiasFn : public Function<RelBiasFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& table, const Tensor& buckets) {
-    Tensor t = table.contiguous();
-    ctx->save_for_backward({t, buckets});
-    static auto f = op<Tensor(const Tensor&, const Tensor&)>("slapo_b200::rel_bias_fwd");
-    return f.call(t, buckets);
+  static Tensor forward(AutogradContext* ctx, const Tensor& table, const Tensor& buckets);
+  static tensor_list backward(AutogradContext* ctx, tensor_list grads);
+};
+struct RelBiasSumFn : public Function<RelBiasSumFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& grad, const Tensor& buckets,
+                        const Tensor& table) {
+    ctx->save_for_backward({buckets});
+    static auto f = op<Tensor(const Tensor&, const Tensor&, const Tensor&)>("slapo_b200::rel_bias_bwd");
+    return f.call(grad.contiguous(), buckets, table);
   }
   static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
-    const variable_list s = ctx->get_saved_variables();
-    static auto f = op<Tensor(const Tensor&, const Tensor&, const Tensor&)>("slapo_b200::rel_bias_bwd");
-    return {f.call(grads[0].contiguous(), s[1], s[0]), Tensor()};
+    return {RelBiasFn::apply(grads[0], ctx->get_saved_variables()[0]), Tensor(), Tensor()};
   }
 };
+Tensor RelBiasFn::forward(AutogradContext* ctx, const Tensor& table, const Tensor& buckets) {
+  ctx->save_for_backward({table, buckets});
+  static auto f = op<Tensor(const Tensor&, const Tensor&)>("slapo_b200::rel_bias_fwd");
+  return f.call(table.contiguous(), buckets);
+}
+tensor_list RelBiasFn::backward(AutogradContext* ctx, tensor_list grads) {
+  const variable_list s = ctx->get_saved_variables();
+  return {RelBiasSumFn::apply(grads[0], s[1], s[0].detach()), Tensor()};
+}
 
 // ------------------------------------------------------------------------ //
 Tensor linear(const Tensor& x, const Tensor& weight, const optional<Tensor>& bias, int64_t act,

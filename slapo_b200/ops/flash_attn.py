@@ -1,11 +1,11 @@
 """Python binding of the tcgen05 flash-attention kernels.
 
 ``flash_attention_native`` is differentiable in q, k, v and in the T5
-relative-position table.  The table ``[num_buckets, H]`` is expanded with
-plain (differentiable) torch indexing into a per-distance bias ``[H, Sq + Sk -
-1]`` - entry ``(key - query) + Sq - 1`` - which the kernels add in-line, so the
-``[H, Sq, Sk]`` bias matrix is never materialised and the table gradient flows
-back through that small gather.
+relative-position table.  The table ``[num_buckets, H]`` is expanded into a
+per-distance bias ``[H, Sq + Sk - 1]`` - entry ``(key - query) + Sq - 1`` -
+which the kernels add in-line, so the ``[H, Sq, Sk]`` bias matrix is never
+materialised and the table gradient flows back through that small gather (a
+kernel per direction; tables that those do not take are indexed with torch).
 """
 from __future__ import annotations
 
@@ -41,10 +41,19 @@ def _distance_buckets(device, sq, sk, n_buckets, bidirectional, max_distance):
     return t5_relative_position_bucket(dist, bidirectional, n_buckets, max_distance)
 
 
+def _table_supported(table) -> bool:
+    """A plain CUDA table outside of functorch and forward-mode transforms; others are indexed."""
+    from .functional import _transformed
+
+    return (type(table) in (torch.Tensor, torch.nn.Parameter) and table.is_cuda and table.dim() == 2
+            and table.dtype in (torch.bfloat16, torch.float16, torch.float32)
+            and native.available() and not _transformed((table,)))
+
+
 def relative_bias_by_distance(table, sq, sk, bidirectional, max_distance):
     """``[num_buckets, H]`` table -> ``[H, sq + sk - 1]`` bias per (key - query)."""
     buckets = _distance_buckets(table.device, sq, sk, table.shape[0], bidirectional, max_distance)
-    if table.dtype in (torch.bfloat16, torch.float16, torch.float32) and native.available():
+    if _table_supported(table):
         return native.ops().rel_bias(table, buckets)
     return table.float()[buckets].t().contiguous()
 

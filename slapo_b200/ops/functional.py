@@ -229,6 +229,12 @@ def attention_reference(q, k, v, key_padding_bias=None, causal=False, scale=None
     return out.transpose(1, 2).to(q.dtype)
 
 
+def _transformed(tensors):
+    """Whether a functorch transform or forward-mode differentiation is at work on them."""
+    return torch.autograd.forward_ad._current_level >= 0 or any(
+        torch._C._functorch.is_functorch_wrapped_tensor(t) for t in tensors)
+
+
 def _append_supported(past_k, past_v, k, v):
     """The four tensors as one launch takes them: plain CUDA tensors outside of autograd and of
     functorch / forward-mode transforms, one type, contiguous caches, 16-byte aligned heads."""
@@ -237,8 +243,7 @@ def _append_supported(past_k, past_v, k, v):
         return False
     if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
         return False
-    if torch.autograd.forward_ad._current_level >= 0 or any(
-            torch._C._functorch.is_functorch_wrapped_tensor(t) for t in tensors):
+    if _transformed(tensors):
         return False
     e = k.element_size()
     if k.dtype not in (torch.bfloat16, torch.float16, torch.float32) or any(

@@ -81,6 +81,30 @@ def test_relative_bias(dtype, buckets, heads, sq, sk):
     assert ((table.grad.double() - want).norm() / want.norm()).item() < eps
 
 
+def test_relative_bias_under_transforms():
+    """What indexing the table could do: second derivatives, forward mode, vmap."""
+    sq, sk = 20, 33
+    table = torch.randn(32, 3, device="cuda", requires_grad=True)
+
+    def by_indexing(t):
+        dist = torch.arange(-(sq - 1), sk, device="cuda") - (sk - sq)
+        return t.float()[NF.t5_relative_position_bucket(dist, True, 32, 128)].t()
+
+    def bias(t):
+        return relative_bias_by_distance(t, sq, sk, True, 128)
+
+    grads = []
+    for fn in (bias, by_indexing):
+        (g,) = torch.autograd.grad((fn(table) ** 3).sum(), table, create_graph=True)
+        grads.append(torch.autograd.grad((g ** 2).sum(), table)[0])
+    torch.testing.assert_close(*grads)
+    v = torch.randn_like(table)
+    for got, want in zip(torch.func.jvp(bias, (table.detach(),), (v,)),
+                         torch.func.jvp(by_indexing, (table.detach(),), (v,))):
+        assert torch.equal(got, want)
+    assert torch.equal(torch.vmap(bias)(torch.stack([v, -v])), torch.stack([bias(v), bias(-v)]))
+
+
 @pytest.mark.parametrize("dtype", [BF, FP])
 def test_gelu_extremes(dtype):
     big = 60000.0 if dtype == FP else 1e30

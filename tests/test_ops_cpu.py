@@ -125,3 +125,17 @@ def test_print_survives_tracing_and_prints_runtime_values():
         out = sch.mod(torch.zeros(2, 4))
     assert "y has shape torch.Size([2, 4])" in buf.getvalue()
     torch.testing.assert_close(out, (model.lin(torch.zeros(2, 4)) + 1) * 2)
+
+
+def test_relative_bias_of_a_table_on_the_cpu():
+    """The kernels are for CUDA tables: one on the CPU is indexed, also where they are loaded."""
+    from slapo_b200.ops.flash_attn import relative_bias_by_distance
+    from slapo_b200.ops.functional import t5_relative_position_bucket
+
+    table = torch.randn(8, 3, requires_grad=True)
+    out = relative_bias_by_distance(table, 5, 7, False, 16)
+    dist = torch.arange(-4, 7) - 2
+    at = t5_relative_position_bucket(dist, False, 8, 16)
+    torch.testing.assert_close(out, table.detach()[at].t())
+    out.sum().backward()
+    torch.testing.assert_close(table.grad, torch.bincount(at, minlength=8).float()[:, None].expand(8, 3))
