@@ -182,24 +182,38 @@ int rel_dtype(const Tensor& t) {
   return t.scalar_type() == at::kBFloat16 ? 0 : (t.scalar_type() == at::kHalf ? 1 : 2);
 }
 
-Tensor rel_bias_fwd(const Tensor& table, const Tensor& buckets) {
+// (indexes outside of the table are the kernels' to check)
+void check_rel(const Tensor& table, const Tensor& buckets) {
   TORCH_CHECK(table.is_cuda() && table.dim() == 2 && table.is_contiguous() &&
                   (rel_dtype(table) < 2 || table.scalar_type() == at::kFloat),
               "rel_bias: a contiguous [buckets, H] CUDA table of fp32, bf16 or fp16 required");
   TORCH_CHECK(buckets.is_cuda() && buckets.dim() == 1 && buckets.is_contiguous() &&
-                  buckets.scalar_type() == at::kLong, "rel_bias: int64 buckets required");
+                  buckets.scalar_type() == at::kLong && buckets.get_device() == table.get_device(),
+              "rel_bias: contiguous int64 buckets on the table's device required");
+  TORCH_CHECK(table.size(0) <= INT_MAX && table.size(1) <= 65535 && buckets.numel() <= INT_MAX - 256,
+              "rel_bias: table or distances too large");
+}
+
+Tensor rel_bias_fwd(const Tensor& table, const Tensor& buckets) {
+  check_rel(table, buckets);
   c10::cuda::CUDAGuard guard(table.device());
   const int n = static_cast<int>(buckets.numel()), H = static_cast<int>(table.size(1));
   Tensor out = at::empty({H, n}, table.options().dtype(at::kFloat));
   slapo::launch_rel_bias_fwd(table.data_ptr(), buckets.data_ptr<int64_t>(), out.data_ptr<float>(), n, H,
-                             rel_dtype(table), at::cuda::getCurrentCUDAStream().stream());
+                             static_cast<int>(table.size(0)), rel_dtype(table),
+                             at::cuda::getCurrentCUDAStream().stream());
   return out;
 }
 
+// `table`: only its sizes and type
 Tensor rel_bias_bwd(const Tensor& grad, const Tensor& buckets, const Tensor& table) {
-  TORCH_CHECK(grad.is_cuda() && grad.is_contiguous() && grad.scalar_type() == at::kFloat);
+  Tensor dtable = at::empty(table.sizes(), table.options(), at::MemoryFormat::Contiguous);
+  check_rel(dtable, buckets);
+  TORCH_CHECK(grad.is_cuda() && grad.is_contiguous() && grad.scalar_type() == at::kFloat &&
+                  grad.get_device() == table.get_device() && grad.dim() == 2 &&
+                  grad.size(0) == table.size(1) && grad.size(1) == buckets.numel(),
+              "rel_bias: a contiguous fp32 [H, distances] gradient on the table's device required");
   c10::cuda::CUDAGuard guard(table.device());
-  Tensor dtable = at::empty(table.sizes(), table.options());
   slapo::launch_rel_bias_bwd(grad.data_ptr<float>(), buckets.data_ptr<int64_t>(), dtable.data_ptr(),
                              static_cast<int>(buckets.numel()), static_cast<int>(table.size(1)),
                              static_cast<int>(table.size(0)), rel_dtype(table),

@@ -60,7 +60,7 @@ void launch_kv_append(const void* const past[2], const void* const fresh[2], voi
 
 // out[h, d] = table[buckets[d], h] (fp32) and dtable[b, h] = sum of grad[h, d] over buckets[d] == b
 void launch_rel_bias_fwd(const void* table, const int64_t* buckets, float* out, int n, int H,
-                         int dtype, cudaStream_t stream);
+                         int n_buckets, int dtype, cudaStream_t stream);
 void launch_rel_bias_bwd(const float* grad, const int64_t* buckets, void* dtable, int n, int H,
                          int n_buckets, int dtype, cudaStream_t stream);
 

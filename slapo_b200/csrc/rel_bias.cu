@@ -8,13 +8,23 @@
 
 namespace slapo {
 
+// Row of the table that an index names: negative ones count from the end, as in torch; -1 for an
+// index outside of the table, which reads nothing and gives NaN.
+__device__ __forceinline__ int64_t rel_row_of(int64_t index, int n_buckets) {
+  if (index < 0) index += n_buckets;
+  return index >= 0 && index < n_buckets ? index : -1;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) rel_bias_fwd_kernel(const T* __restrict__ table,
                                                            const int64_t* __restrict__ buckets,
-                                                           float* __restrict__ out, int n, int H) {
+                                                           float* __restrict__ out, int n, int H,
+                                                           int n_buckets) {
   const int d = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y;
-  if (d < n)
-    out[static_cast<int64_t>(h) * n + d] = static_cast<float>(table[buckets[d] * H + h]);
+  if (d >= n) return;
+  const int64_t row = rel_row_of(buckets[d], n_buckets);
+  out[static_cast<int64_t>(h) * n + d] =
+      row >= 0 ? static_cast<float>(table[row * H + h]) : __int_as_float(0x7fc00000);
 }
 
 // one block per head; each warp sums the distances of one bucket at a time (fp32, fixed order)
@@ -28,7 +38,7 @@ __global__ void __launch_bounds__(256) rel_bias_bwd_kernel(const float* __restri
   for (int b = warp; b < n_buckets; b += 8) {
     float s = 0.f;
     for (int d = lane; d < n; d += 32)
-      if (buckets[d] == b) s += g[d];
+      if (rel_row_of(buckets[d], n_buckets) == b) s += g[d];
     s = warp_sum(s);
     if (lane == 0) dtable[static_cast<int64_t>(b) * H + h] = static_cast<T>(s);
   }
@@ -42,11 +52,11 @@ __global__ void __launch_bounds__(256) rel_bias_bwd_kernel(const float* __restri
   }
 
 void launch_rel_bias_fwd(const void* table, const int64_t* buckets, float* out, int n, int H,
-                         int dtype, cudaStream_t stream) {
+                         int n_buckets, int dtype, cudaStream_t stream) {
   if (n == 0 || H == 0) return;
   count_launch();
   DISPATCH_DTYPE(dtype, (rel_bias_fwd_kernel<T><<<dim3((n + 255) / 256, H), 256, 0, stream>>>(
-      static_cast<const T*>(table), buckets, out, n, H)));
+      static_cast<const T*>(table), buckets, out, n, H, n_buckets)));
 }
 
 void launch_rel_bias_bwd(const float* grad, const int64_t* buckets, void* dtable, int n, int H,

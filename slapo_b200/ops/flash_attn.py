@@ -53,7 +53,8 @@ def _table_supported(table) -> bool:
 def relative_bias_by_distance(table, sq, sk, bidirectional, max_distance):
     """``[num_buckets, H]`` table -> ``[H, sq + sk - 1]`` bias per (key - query)."""
     buckets = _distance_buckets(table.device, sq, sk, table.shape[0], bidirectional, max_distance)
-    if _table_supported(table):
+    # (parameters that order the buckets otherwise can index outside of the table: torch's to report)
+    if _table_supported(table) and max_distance > table.shape[0] // (4 if bidirectional else 2):
         return native.ops().rel_bias(table, buckets)
     return table.float()[buckets].t().contiguous()
 

@@ -105,6 +105,36 @@ def test_relative_bias_under_transforms():
     assert torch.equal(torch.vmap(bias)(torch.stack([v, -v])), torch.stack([bias(v), bias(-v)]))
 
 
+def test_relative_bias_refuses_what_does_not_fit():
+    ops = native.ops()
+    table = torch.randn(8, 3, device="cuda")
+    at = torch.arange(5, device="cuda")
+    grad = torch.randn(3, 5, device="cuda")
+    for args in ((table, at.int()), (table, at.cpu()), (table, at[None]), (table.double(), at),
+                 (table.t(), at), (table[0], at)):
+        with pytest.raises(RuntimeError):
+            ops.rel_bias_fwd(*args)
+    for args in ((grad, at.int(), table), (grad, at.cpu(), table), (grad[:, :4], at, table),
+                 (grad[:2], at, table), (grad.t(), at, table), (grad.half(), at, table),
+                 (grad[0], at, table), (grad, at, table.double()), (grad, at, table[0]),
+                 (grad, at[:4], table), (grad.cpu(), at, table)):
+        with pytest.raises(RuntimeError):
+            ops.rel_bias_bwd(*args)
+
+
+def test_relative_bias_indexes_outside_of_the_table():
+    """Negative ones count from the end; what lies outside is not read: NaN, and no gradient."""
+    ops = native.ops()
+    table = torch.randn(4, 2, device="cuda")
+    at = torch.tensor([-1, 3, 4, -5, 0, 1 << 40], device="cuda")
+    out = ops.rel_bias_fwd(table, at)
+    assert torch.equal(out[:, [0, 1, 4]], table.t()[:, [3, 3, 0]])
+    assert out[:, [2, 3, 5]].isnan().all()
+    grad = torch.ones(2, 6, device="cuda")
+    want = torch.tensor([1.0, 0, 0, 2], device="cuda")[:, None].expand(4, 2)
+    assert torch.equal(ops.rel_bias_bwd(grad, at, table), want)
+
+
 @pytest.mark.parametrize("dtype", [BF, FP])
 def test_gelu_extremes(dtype):
     big = 60000.0 if dtype == FP else 1e30
