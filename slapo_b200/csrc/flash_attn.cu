@@ -11,9 +11,11 @@
 //                           O += P V        (P read from TMEM, fp32 accumulator in TMEM)
 //   warps 2-5 one query row per thread: the row's 128 scores in registers, online softmax in
 //             the exp2 domain, P back to TMEM as bf16 / fp16.
-// The running maximum that P and O are scaled by is only raised when a row's maximum has grown
-// by more than 2^8: until then P simply exceeds 1 (it keeps its relative precision), and O
-// stays where it is.  When it is raised, the warp scales its O rows in TMEM.
+// P and O are scaled by the running row maximum: when that of any of a warp's rows has grown, the
+// warp scales its O rows in TMEM.  (Raising it only after a growth of 2^8 saves 2 - 9 % of the
+// forward - 32 x 512 x 16 x 64, p 0.1: 113 against 117 us, 4 x 2048 x 16 x 128: 186 against 205 - but
+// then the probabilities that count lie anywhere in their binade instead of at or just below 1,
+// and the result's rounding error grows by up to 5 %: 0.00230 against 0.00220 at 512 keys, bf16.)
 // P has columns of its own: S of the next tile is computed while the softmax warps work on this
 // one.
 //
@@ -67,7 +69,6 @@ bool make_tmap_bshd(CUtensorMap* out, const void* base, uint64_t B, uint64_t S, 
 // ------------------------------------------------------------------------ //
 constexpr int kBlockM = 128;   // query rows per work item
 constexpr int kBlockN = 128;   // keys per tile
-constexpr float kRaise = 8.f;  // growth of a row maximum (log2) that makes O be rescaled
 
 struct FlashFwdParams {
   int B, H, Sq, Sk;
@@ -370,7 +371,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         tc::fence_after_sync();
         if (j == 0) {
           m_ref = m_tile;
-        } else if (__any_sync(0xffffffffu, m_tile > m_ref + kRaise)) {
+        } else if (__any_sync(0xffffffffu, m_tile > m_ref)) {
           const float m_new = fmaxf(m_ref, m_tile);
           const float alpha = m_ref == -INFINITY ? 0.f : exp2f(m_ref - m_new);
           const uint64_t alpha2 = f2_pack(alpha, alpha);

@@ -99,3 +99,39 @@ def test_flash_attention_paths(b, sq, sk, h, d, dtype, how, p):
         # (with a single key dS is a difference of equal numbers: measured against unit scale)
         err = ((x.double() - y).norm() / y.norm().clamp(min=0.05 * y.numel() ** 0.5)).item()
         assert err < TOL[dtype], f"{name}: {err:.2e}"
+
+
+def _rounded_as_the_running_maximum_says(q, k, v, scale, dtype, tile=128):
+    """64-bit attention with one rounding of P, scaled by the row maximum of the keys up to and
+    including its tile, and one of the result: what the order of an online softmax gives."""
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) * scale
+    v = v.double().transpose(1, 2)
+    m = torch.full(s.shape[:-1], float("-inf"), device=s.device, dtype=s.dtype)
+    o, l = torch.zeros_like(q.double().transpose(1, 2)), torch.zeros_like(m)
+    for at in range(0, s.shape[-1], tile):
+        part = s[..., at:at + tile]
+        new = torch.maximum(m, part.amax(-1))
+        p = torch.exp(part - new[..., None])
+        shrink = torch.exp(m - new)
+        o = o * shrink[..., None] + p.to(dtype).double() @ v[..., at:at + tile, :]
+        l = l * shrink + p.sum(-1)
+        m = new
+    return (o / l[..., None]).to(dtype).transpose(1, 2)
+
+
+@pytest.mark.parametrize("sk,d,dtype,grow", [(512, 64, BF, False), (1024, 128, BF, False),
+                                             (512, 64, FP, False), (1024, 64, BF, True)])
+def test_forward_rounds_no_more_than_an_online_softmax(sk, d, dtype, grow):
+    """P scaled by an older maximum lies anywhere in its binade and is rounded more coarsely where
+    it counts (5 % of the result's error at 512 keys); half a million results put the two errors'
+    ratio within 0.3 %."""
+    torch.manual_seed(sk + d)
+    q, k, v = (torch.randn(4, n, 4, d, device="cuda", dtype=dtype) for n in (512, sk, sk))
+    if grow:
+        k = (k * torch.linspace(0.5, 2, sk, device="cuda")[None, :, None, None]).to(dtype)
+    scale = d ** -0.5
+    want = _reference(q, k, v, None, False, scale, None, None, 0.0)[0].detach()
+    got = NF.flash_attention(q, k, v)
+    err = [((x.double() - want).norm() / want.norm()).item()
+           for x in (got, _rounded_as_the_running_maximum_says(q, k, v, scale, dtype))]
+    assert err[0] < 1.01 * err[1], err
