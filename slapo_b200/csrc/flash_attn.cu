@@ -22,11 +22,15 @@
 // What bounds it: the special-function unit (one exp2 per score, 1024 cycles per 128 x 128 tile
 // and SM) next to the issue slots of the softmax warps.  One thread per whole row needs no
 // exchange between warps; for D = 64 two independent CTAs fill each other's waits.
-// Measured (one kernel, before: P through shared memory, O folded in registers, one work item per
-// CTA -> now): 32 x 512 x 16 heads of 64, p 0.1: 125 -> 107 us; 4 x 2048 x 16 x 128 causal: 299 ->
-// 127 us; 4 x 1000 x 32 x 80 causal with key bias: 180 -> 147 us; 8 x 512 x 16 x 64 with T5's bias,
-// key bias and p 0.1: 67 -> 73 us (per-element bias loads); 1 query x 1501 keys x 8 x 16 x 128,
-// keys split: 53 -> 31 + 3 us.
+// Measured (L2 flushed; P through shared memory, O folded in registers, one work item per CTA ->
+// now): 32 x 512 x 16 heads of 64, p 0.1: 126 -> 114 us; 4 x 2048 x 16 x 128 causal: 302 -> 137 us; 4 x
+// 1000 x 32 x 80 causal with key bias: 180 -> 105 us; 8 x 512 x 16 x 64 with T5's bias, key bias and p
+// 0.1: 66 -> 47 us; 1 query x 1500 keys x 8 x 16 x 128, keys split: 54 -> 33 us with the combine kernel.
+//
+// Biases are added from shared memory, which asynchronous copies fill a tile ahead: a warp's 32
+// queries see 159 distances in a tile of 128 keys, against 128 loads per query.  Fetched by each
+// thread as it needed them they stood in the tile's chain: 73 -> 36 us with T5's bias, 65 -> 35 us
+// with a key bias (8 x 512 x 16 x 64).
 #include "flash_common.cuh"
 #include "kernels.h"
 
@@ -100,8 +104,11 @@ struct FwdSmem {
   static constexpr int kCtas = D == 64 ? 2 : 1;      // per SM: shared memory and TMEM columns
   static constexpr int kK = kTile;
   static constexpr int kV = kK + kStages * kTile;
-  static constexpr int kBias = kV + kStages * kTile; // [4 warps][2][128] floats
-  static constexpr int kBars = kBias + 4 * 2 * 128 * 4;
+  // per softmax warp, twice (this tile's and the next one's): the tile's 128 key biases and the
+  // relative bias of the 32 + 128 - 1 distances between its queries and the tile's keys
+  static constexpr int kBiasFloats = 128 + 160;
+  static constexpr int kBias = kV + kStages * kTile;
+  static constexpr int kBars = kBias + 4 * 2 * kBiasFloats * 4;
   static constexpr int kTotal = kBars + 20 * 8 + 1024;
 };
 
@@ -288,7 +295,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const int quarter = warp & 3;
     const int row_in_tile = quarter * 32 + lane;
     const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    float* kb_buf = reinterpret_cast<float*>(smem + L::kBias) + (warp - 2) * 256;
+    float* bias_buf = reinterpret_cast<float*>(smem + L::kBias) + (warp - 2) * 2 * L::kBiasFloats;
     uint64_t seed = 0, offset = 0;
     if (p.p_drop > 0.f) philox_unpack(p.rng, seed, offset);
     const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
@@ -297,8 +304,32 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // to them (or the scale would turn the maximum around)
     const bool biased = kGeneral && (p.kbias != nullptr || p.rel != nullptr || !(p.scale_log2 > 0.f));
     const float sc = biased ? 1.f : p.scale_log2;
+    // Biases of key tile `jt` of a work item on their way into buffer `buf`: copied a tile ahead,
+    // element by element (rows start anywhere).  What lies outside of the tensors is masked later.
+    auto fetch_bias = [&](int tile, int bh, int jt, int buf) {
+      float* dst = bias_buf + buf * L::kBiasFloats;
+      const int batch = bh / p.H, head = bh - batch * p.H, k0 = jt * kBlockN;
+      if (p.kbias != nullptr) {
+        const float* src = p.kbias + static_cast<int64_t>(batch) * p.Sk;
+#pragma unroll
+        for (int i = lane; i < 128; i += 32) cp_async4(dst + i, src + min(k0 + i, p.Sk - 1));
+      }
+      if (p.rel != nullptr) {
+        // key - query from that of the warp's last row and the first key on
+        const float* src = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + p.Sq - 1;
+        const int d0 = k0 - (tile * kBlockM + quarter * 32 + 31);
+#pragma unroll
+        for (int i = lane; i < 160; i += 32)
+          cp_async4(dst + 128 + i, src + max(1 - p.Sq, min(d0 + i, p.Sk - 1)));
+      }
+    };
     bool ok = true;
     int t = 0;
+    if (biased && static_cast<int>(blockIdx.x) < items) {
+      int tile, bh, j0;
+      item_at(blockIdx.x, tile, bh, j0);
+      fetch_bias(tile, bh, j0, 0);
+    }
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
       int tile, bh, j0;
       const int n = item_at(item, tile, bh, j0);
@@ -306,27 +337,29 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int row = tile * kBlockM + row_in_tile;
       const uint64_t drop_row_base =
           (static_cast<uint64_t>(bh) * p.Sq + min(row, p.Sq - 1)) * sk16;
-      const float* rel_row = nullptr;
-      if (kGeneral && p.rel != nullptr)
-        rel_row = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + (p.Sq - 1) -
-                  min(row, p.Sq - 1);
       int key_limit = p.Sk;
       if (p.causal) key_limit = min(key_limit, row + diag + 1);
       float m_ref = -INFINITY;
       uint64_t l2 = 0;      // two fp32 partial row sums
       for (int j = 0; j < n; ++j, ++t) {
         const int k0 = (j0 + j) * kBlockN;
-        const float* kb = nullptr;
-        if (kGeneral && p.kbias != nullptr) {
-          // this warp's copy of the tile's key bias (two buffers: the readers of the one
-          // before the last are done once every lane has passed the __syncwarp in between)
-          float* dst = kb_buf + (t & 1) * 128;
-          for (int i = lane; i < kBlockN; i += 32) {
-            const int key = k0 + i;
-            dst[i] = key < p.Sk ? p.kbias[static_cast<int64_t>(batch) * p.Sk + key] * kLog2e : 0.f;
+        const float* bias = bias_buf + (t & 1) * L::kBiasFloats;
+        if (kGeneral && biased) {
+          cp_async_wait();
+          if (p.kbias != nullptr) {
+#pragma unroll
+            for (int i = lane; i < 128; i += 32)      // (the elements that this lane copied)
+              bias_buf[(t & 1) * L::kBiasFloats + i] *= kLog2e;
           }
+          // this tile's biases are visible to the warp, and the other buffer's readers are done
           __syncwarp();
-          kb = dst;
+          if (j + 1 < n) {
+            fetch_bias(tile, bh, j0 + j + 1, (t + 1) & 1);
+          } else if (item + static_cast<int>(gridDim.x) < items) {
+            int next_tile, next_bh, next_j0;
+            item_at(item + gridDim.x, next_tile, next_bh, next_j0);
+            fetch_bias(next_tile, next_bh, next_j0, (t + 1) & 1);
+          }
         }
         if (!tc::mbar_wait_warp(s_full, t & 1, abort_flag)) { ok = false; break; }
         tc::fence_after_sync();
@@ -339,16 +372,28 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (lane == 0) tc::mbar_arrive(s_free);
         if constexpr (kGeneral) {
           if (biased) {
+            const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2);
+            const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
+            const bool key_bias = p.kbias != nullptr;
 #pragma unroll
             for (int c = 0; c < 4; ++c)
 #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                float s = __uint_as_float(raw[c][i]) * p.scale_log2;
-                if (kb != nullptr) s += kb[c * 32 + i];
-                if (rel_row != nullptr)
-                  s = fmaf(rel_row[min(k0 + c * 32 + i, p.Sk - 1)], kLog2e, s);
-                raw[c][i] = __float_as_uint(s);
+              for (int i = 0; i < 32; i += 4) {
+                float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (key_bias) b = *reinterpret_cast<const float4*>(bias + c * 32 + i);
+                f2_store(raw[c] + i, f2_fma(f2_load(raw[c] + i), scale2, f2_pack(b.x, b.y)));
+                f2_store(raw[c] + i + 2, f2_fma(f2_load(raw[c] + i + 2), scale2, f2_pack(b.z, b.w)));
               }
+            if (p.rel != nullptr) {
+              // neighbouring lanes (queries) read neighbouring words
+              const float* rel = bias + 128 + 31 - lane;
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int i = 0; i < 32; i += 2)
+                  f2_store(raw[c] + i, f2_fma(f2_pack(rel[c * 32 + i], rel[c * 32 + i + 1]), log2e2,
+                                              f2_load(raw[c] + i)));
+            }
           }
           const int first_limit = p.causal ? min(p.Sk, tile * kBlockM + quarter * 32 + diag + 1) : p.Sk;
           if (k0 + kBlockN > first_limit) {     // some lane of the warp masks something
@@ -485,6 +530,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         p.lse[static_cast<int64_t>(bh) * p.Sq + row] = l_run > 0.f ? m_nat + logf(l_run) : -INFINITY;
       }
     }
+    if (kGeneral) cp_async_wait();      // (a give-up leaves copies under way)
   }
 
   tc::fence_before_sync();

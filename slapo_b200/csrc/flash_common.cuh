@@ -33,6 +33,25 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
   return d;
 }
 
+// two neighbouring words of a row of scores as one such pair
+__device__ __forceinline__ uint64_t f2_load(const uint32_t* r) {
+  return f2_pack(__uint_as_float(r[0]), __uint_as_float(r[1]));
+}
+__device__ __forceinline__ void f2_store(uint32_t* r, uint64_t v) {
+  float a, b;
+  f2_unpack(v, a, b);
+  r[0] = __float_as_uint(a);
+  r[1] = __float_as_uint(b);
+}
+
+// a 4-byte copy from global to shared memory that runs on its own, and the wait for all of a
+// thread's copies
+__device__ __forceinline__ void cp_async4(float* smem_dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(tc::smem_u32(smem_dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 template <typename T> __device__ __forceinline__ uint32_t pack16(float a, float b);
 template <> __device__ __forceinline__ uint32_t pack16<__nv_bfloat16>(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);

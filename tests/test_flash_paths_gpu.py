@@ -53,6 +53,10 @@ CASES = [
     (2, 256, 256, 4, 64, BF, "r", 0.0),
     (2, 200, 200, 4, 64, BF, "ckr", 0.1),
     (1, 300, 300, 4, 128, BF, "r", 0.1),
+    (2, 130, 333, 3, 64, BF, "kr", 0.0),       # biases of ragged tiles and unequal lengths
+    (1, 333, 130, 2, 80, FP, "r", 0.0),
+    (20, 200, 300, 12, 64, FP, "kr", 0.0),     # ... of the next work item, fetched ahead
+    (12, 260, 140, 9, 128, BF, "kr", 0.1),
     (2, 1024, 1024, 4, 64, BF, "g", 0.0),      # row maxima raised many times
     (2, 1024, 1024, 4, 128, FP, "cg", 0.1),
     (1, 1, 1000, 4, 128, BF, "c", 0.0),        # keys split over work items
