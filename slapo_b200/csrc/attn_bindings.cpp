@@ -64,7 +64,7 @@ std::tuple<Tensor, Tensor> flash_attn_fwd(const Tensor& q, const Tensor& k, cons
   const int64_t ks[3] = {k.stride(0), k.stride(1), k.stride(2)};
   const int64_t vs[3] = {v.stride(0), v.stride(1), v.stride(2)};
   // few row tiles: the keys are split over work items, whose shares a second kernel combines
-  const int64_t splits = slapo::flash_fwd_splits(B, H, Sq, Sk);
+  const int64_t splits = slapo::flash_fwd_splits(B, H, Sq, Sk, D);
   Tensor scratch;
   if (splits > 1)
     scratch = at::empty({splits * B * H * Sq * (D + 2)}, q.options().dtype(at::kFloat));

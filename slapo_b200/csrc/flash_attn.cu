@@ -25,7 +25,7 @@
 // Measured (L2 flushed; P through shared memory, O folded in registers, one work item per CTA ->
 // now): 32 x 512 x 16 heads of 64, p 0.1: 126 -> 114 us; 4 x 2048 x 16 x 128 causal: 302 -> 137 us; 4 x
 // 1000 x 32 x 80 causal with key bias: 180 -> 105 us; 8 x 512 x 16 x 64 with T5's bias, key bias and p
-// 0.1: 66 -> 47 us; 1 query x 1500 keys x 8 x 16 x 128, keys split: 54 -> 33 us with the combine kernel.
+// 0.1: 66 -> 47 us; 1 query x 1500 keys x 4 x 16 x 128, keys split: 53 -> 25 us with the combine kernel.
 //
 // Biases are added from shared memory, which asynchronous copies fill a tile ahead: a warp's 32
 // queries see 159 distances in a tile of 128 keys, against 128 loads per query.  Fetched by each
@@ -623,16 +623,22 @@ static int launch_fwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
-// Work items per row tile.  One row tile per (batch, head) - generation, short queries - and
-// fewer of them than half the resident CTAs (two per SM): the keys are split so that the CTAs
-// are used, down to one key tile per item.
-int flash_fwd_splits(int B, int H, int Sq, int Sk) {
+// Work items per row tile.  One row tile per (batch, head) - generation, short queries - and at
+// most half as many of them as resident CTAs (two per SM for D = 64, one beyond): the keys are split
+// as far as one wave of CTAs takes them.  More items than that wait for one another (1 query x 1500
+// keys, D = 128, 128 heads on 148 SMs: two splits 33 us, none 27).  The combine kernel has to be
+// earned by a shorter chain: four tiles less, at 1.6 - 2 us each (1 query x 1000 keys x 12 heads: 20 ->
+// 14 us; 300 keys: 12 -> 14).
+int flash_fwd_splits(int B, int H, int Sq, int Sk, int D) {
   const int tiles = (Sk + kBlockN - 1) / kBlockN;
-  const int64_t bh = static_cast<int64_t>(B) * H, cap = 2 * sm_count();
-  if (Sq > kBlockM || bh <= 0 || 2 * bh > cap || tiles < 2) return 1;
+  const int64_t bh = static_cast<int64_t>(B) * H;
+  const int64_t cap = (D <= 64 ? FwdSmem<64>::kCtas : FwdSmem<128>::kCtas) * sm_count();
+  if (Sq > kBlockM || bh <= 0) return 1;
   int64_t s = cap / bh;
   if (s > tiles) s = tiles;
+  if (s < 2) return 1;
   const int per = static_cast<int>((tiles + s - 1) / s);
+  if (tiles - per < 4) return 1;
   return (tiles + per - 1) / per;     // no empty split
 }
 
@@ -658,7 +664,7 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float
   p.walk.row_tiles = (Sq + kBlockM - 1) / kBlockM;
   p.walk.bh0 = 0; p.walk.nbh = B * H; p.walk.H = H;
   p.walk.by_cost = causal ? 2 : 0;
-  p.splits = scratch != nullptr ? flash_fwd_splits(B, H, Sq, Sk) : 1;
+  p.splits = scratch != nullptr ? flash_fwd_splits(B, H, Sq, Sk, D) : 1;
   const int key_tiles = (Sk + kBlockN - 1) / kBlockN;
   p.tiles_per_split = (key_tiles + p.splits - 1) / p.splits;
   const int64_t rows = static_cast<int64_t>(B) * H * Sq;

@@ -105,6 +105,22 @@ def test_flash_attention_paths(b, sq, sk, h, d, dtype, how, p):
         assert err < TOL[dtype], f"{name}: {err:.2e}"
 
 
+@pytest.mark.parametrize("bh,sk,d,launches", [
+    (128, 1500, 128, 1),      # one CTA per SM: a second item per head would wait for the first
+    (128, 1500, 64, 2),       # two per SM
+    (12, 1500, 128, 2),
+    (12, 300, 64, 1),         # too few tiles to shorten
+    (300, 4000, 64, 1),
+])
+def test_keys_are_split_where_that_shortens_the_chain(bh, sk, d, launches):
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the rule counts SMs")
+    q, k, v = (torch.randn(1, n, bh, d, device="cuda", dtype=BF) for n in (1, sk, sk))
+    before = native.launch_count()
+    NF.flash_attention(q, k, v)
+    assert native.launch_count() - before == launches
+
+
 def _rounded_as_the_running_maximum_says(q, k, v, scale, dtype, tile=128):
     """64-bit attention with one rounding of P, scaled by the row maximum of the keys up to and
     including its tile, and one of the result: what the order of an online softmax gives."""
