@@ -25,7 +25,7 @@
 // Measured (L2 flushed; P through shared memory, O folded in registers, one work item per CTA ->
 // now): 32 x 512 x 16 heads of 64, p 0.1: 126 -> 114 us; 4 x 2048 x 16 x 128 causal: 302 -> 137 us; 4 x
 // 1000 x 32 x 80 causal with key bias: 180 -> 105 us; 8 x 512 x 16 x 64 with T5's bias, key bias and p
-// 0.1: 66 -> 47 us; 1 query x 1500 keys x 4 x 16 x 128, keys split: 53 -> 25 us with the combine kernel.
+// 0.1: 66 -> 47 us; 1 query x 1500 keys x 4 x 12 x 128, keys split: 52 -> 21 us with the combine kernel.
 //
 // Biases are added from shared memory, which asynchronous copies fill a tile ahead: a warp's 32
 // queries see 159 distances in a tile of 128 keys, against 128 loads per query.  Fetched by each

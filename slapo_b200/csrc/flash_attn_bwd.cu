@@ -126,7 +126,10 @@ struct BwdSmem {
   static constexpr int kY = 2 * kTile;
   static constexpr int kVecs = kY + kStages * 2 * kTile;
   static constexpr int kDrel = kVecs + kStages * kVec;       // [8 warps][64] floats
-  static constexpr int kBars = kDrel + (kKeys ? 8 * 64 * 4 : 0);
+  // per softmax warp, twice: the relative bias of the 32 + 64 - 1 distances of its part of a tile
+  static constexpr int kRelFloats = 96;
+  static constexpr int kRel = kDrel + (kKeys ? 8 * 64 * 4 : 0);
+  static constexpr int kBars = kRel + 8 * 2 * kRelFloats * 4;
   static constexpr int kTotal = kBars + 24 * 8 + 1024;
 };
 
@@ -458,6 +461,27 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
       }
     };
 
+    // Relative bias of this warp's 32 rows and 64 columns in streamed tile `y` of a work item, on
+    // its way into buffer `buf`: copied a tile ahead, as in the forward.  A column further is a key
+    // further in the dQ pass, a query further (a smaller distance) in the other.
+    float* rel_buf = reinterpret_cast<float*>(smem + L::kRel) + (warp - 2) * 2 * L::kRelFloats;
+    const bool has_rel = kGeneral && p.rel != nullptr;
+    auto fetch_rel = [&](int tile, int bhl, int y, int buf) {
+      const int head = (p.walk.bh0 + bhl) % p.H;
+      const float* src = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + p.Sq - 1;
+      const int r0 = tile * 128 + quarter * 32, c0 = y * 128 + half * 64;
+      const int d0 = kKeys ? r0 - (c0 + 63) : c0 - (r0 + 31);
+#pragma unroll
+      for (int i = lane; i < L::kRelFloats; i += 32)
+        cp_async4(rel_buf + buf * L::kRelFloats + i, src + max(1 - p.Sq, min(d0 + i, p.Sk - 1)));
+    };
+    if (has_rel && static_cast<int>(blockIdx.x) < items) {
+      int tile, bhl, first;
+      p.walk.at(blockIdx.x, tile, bhl);
+      tiles_of(tile, first);
+      fetch_rel(tile, bhl, first, 0);
+    }
+
     bool ok = true;
     int t = 0, w = 0, prev_item = -1;
     float rs_a, rs_b;
@@ -476,6 +500,18 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
         const int st = t % kStages;
         const int col0 = (first + j) * 128 + half * 64;     // this thread's first column
         const uint8_t* vec = s_vec + st * L::kVec;
+        if (has_rel) {
+          cp_async_wait();
+          __syncwarp();     // (visible to the warp, and the other buffer's readers are done)
+          if (j + 1 < n) {
+            fetch_rel(tile, bhl, first + j + 1, (t + 1) & 1);
+          } else if (item + static_cast<int>(gridDim.x) < items) {
+            int next_tile, next_bhl, next_first;
+            p.walk.at(item + gridDim.x, next_tile, next_bhl);
+            tiles_of(next_tile, next_first);
+            fetch_rel(next_tile, next_bhl, next_first, (t + 1) & 1);
+          }
+        }
         // ---- dropout decisions of this row and the thread's 64 keys (dQ pass) ----
         uint32_t keep16[4][4];
         if (!kKeys && drop) {
@@ -546,18 +582,14 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
           }
         }
         if constexpr (kGeneral) {
-          if (p.rel != nullptr) {
-            const float* rel = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + p.Sq - 1;
-            if constexpr (kKeys) {
-              const int key = min(row, p.Sk - 1);
+          if (has_rel) {
+            const float* rel = rel_buf + (t & 1) * L::kRelFloats + (kKeys ? lane + 63 : 31 - lane);
+            const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
 #pragma unroll
-              for (int i = 0; i < 64; ++i)
-                pr[i] = fmaf(rel[key - min(col0 + i, p.Sq - 1)], kLog2e, pr[i]);
-            } else {
-              const int query = min(row, p.Sq - 1);
-#pragma unroll
-              for (int i = 0; i < 64; ++i)
-                pr[i] = fmaf(rel[min(col0 + i, p.Sk - 1) - query], kLog2e, pr[i]);
+            for (int i = 0; i < 64; i += 2) {
+              const uint64_t x = f2_fma(kKeys ? f2_pack(rel[-i], rel[-i - 1]) : f2_pack(rel[i], rel[i + 1]),
+                                        log2e2, f2_pack(pr[i], pr[i + 1]));
+              f2_unpack(x, pr[i], pr[i + 1]);
             }
           }
           if constexpr (kKeys) {
@@ -701,6 +733,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
     }
     if (ok && prev_item >= 0 && tc::mbar_wait_warp(acc_full, (w - 1) & 1, abort_flag))
       read_out(prev_item);
+    if (has_rel) cp_async_wait();     // (a give-up leaves copies under way)
   }
 
   tc::fence_before_sync();
