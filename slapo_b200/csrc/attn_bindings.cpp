@@ -105,11 +105,11 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> flash_attn_bwd(
     dv = at::empty({B, Sk, H, D}, q.options());
   }
   const bool has_bias = kbias.has_value() && kbias->defined();
-  const slapo::FlashBwdScratch sizes =
-      slapo::flash_bwd_scratch(B, H, Sq, Sk, has_bias, static_cast<float>(p_drop));
-  Tensor scratch = at::empty({sizes.total()}, q.options().dtype(at::kFloat));
-  Tensor drel;
   const bool has_rel = rel.has_value() && rel->defined();
+  const slapo::FlashBwdPlan plan = slapo::flash_bwd_plan(
+      B, H, Sq, Sk, D, packed_qkv, causal, has_bias, has_rel, static_cast<float>(p_drop));
+  Tensor scratch = at::empty({plan.total()}, q.options().dtype(at::kFloat));
+  Tensor drel;
   if (has_rel) drel = at::zeros_like(*rel);
   else drel = at::empty({0}, q.options().dtype(at::kFloat));
   const int64_t qs[3] = {q.stride(0), q.stride(1), q.stride(2)};
@@ -117,7 +117,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> flash_attn_bwd(
   const int64_t vs[3] = {v.stride(0), v.stride(1), v.stride(2)};
   int rc = slapo::launch_flash_bwd(
       q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), dout.data_ptr(),
-      lse.data_ptr<float>(), scratch.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(),
+      lse.data_ptr<float>(), plan, scratch.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(),
       dv.data_ptr(), row_stride, row_stride, opt_f32(kbias, "key bias"),
       opt_f32(rel, "relative bias"),
       has_rel ? drel.data_ptr<float>() : nullptr, B, H, Sq, Sk, D, qs, ks, vs,

@@ -44,19 +44,21 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float
                      const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
                      float scale, int causal, float p_drop, PhiloxArgs rng, bool bf16, int* status,
                      cudaStream_t stream);
-// Scratch of the backward pass, in floats: row statistics, padded key bias and, with dropout,
-// keep bits.  `pairs`: (batch, head) pairs per launch (the keep bits of all of them would
-// grow with B H Sq Sk).
-struct FlashBwdScratch {
-  int64_t stats, bias, keep;
-  int pairs;
-  int64_t total() const { return stats + bias + keep; }
+// How the backward runs, and its scratch in floats: row statistics, padded key bias, keep bits
+// (dropout in two launches) and shares of dQ (keys split over work items).
+struct FlashBwdPlan {
+  int pairs;         // (batch, head) pairs per launch: the keep bits of all would grow with B H Sq Sk
+  int splits;        // work items per query tile in the dQ pass
+  int q_ctas;        // both passes in one launch, this many CTAs for dQ; 0: one launch each
+  int64_t stats, bias, keep, part;
+  int64_t total() const { return stats + bias + keep + part; }
 };
-FlashBwdScratch flash_bwd_scratch(int B, int H, int Sq, int Sk, bool key_bias, float p_drop);
+FlashBwdPlan flash_bwd_plan(int B, int H, int Sq, int Sk, int D, bool packed, bool causal,
+                            bool key_bias, bool rel, float p_drop);
 // dq_row_stride / dkv_row_stride: elements between consecutive (b, s, head) rows of the outputs
 int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
-                     const float* lse, float* scratch, void* dq, void* dk, void* dv,
-                     int64_t dq_row_stride, int64_t dkv_row_stride, const float* kbias,
+                     const float* lse, const FlashBwdPlan& plan, float* scratch, void* dq, void* dk,
+                     void* dv, int64_t dq_row_stride, int64_t dkv_row_stride, const float* kbias,
                      const float* rel, float* drel, int B, int H, int Sq, int Sk, int D,
                      const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
                      float scale, int causal, float p_drop, PhiloxArgs rng, bool bf16, int* status,

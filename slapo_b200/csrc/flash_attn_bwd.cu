@@ -21,19 +21,25 @@
 //   softmax      dS (t)          P (t+1)          dS (t+1)
 // (D = 128: each pair the other way round).
 // CTAs are persistent; the loads and the first S of the next work item run under the last tile of
-// this one, and its accumulators are read out after the first P of the next.
+// this one, and its accumulators are read out after the first P of the next.  The passes run side by
+// side in one launch where that fills the GPU better (both_q_ctas); the keys of few queries are split
+// over work items.
 //
 // A single pass (5 products per tile instead of 7) has to add up dQ over the key tiles: one fp32
 // partial of dQ per key tile written and read again was most of its time (BERT-large, 32 x 512
 // tokens x 16 heads of 64: 268 MB each way).  Bound now: the chain of a tile (product, TMEM load,
 // exp2, pack, TMEM store, barrier, product); exp2 alone needs 1024 cycles per tile and pass.  Twice
 // the softmax warps on half the columns each changed nothing (181 -> 185 and 144 -> 153 us).
-// Measured (all kernels of the backward, before -> now): 32 x 512 x 16 heads of 64, p 0.1: 360 ->
-// 317 us; 4 x 2048 x 16 x 128 causal: 655 -> 395 us; 4 x 1000 x 32 x 80 causal: 345 -> 226 us.
+// Measured (all kernels of the backward, a single pass with dQ partials -> now): 32 x 512 x 16 heads
+// of 64, p 0.1: 366 -> 316 us; 4 x 2048 x 16 x 128 causal: 652 -> 398 us; 4 x 1000 x 32 x 80 causal with key
+// bias: 353 -> 237 us; 8 x 512 x 16 x 64 with T5's bias, key bias and p 0.1: 159 -> 160 us; 1 x 512 x 16 x
+// 64, p 0.1: 31 -> 25 us.  Where one key tile meets one to two query tiles of 100 - 500 heads, the single
+// pass had half the work items: 8 x 128 x 16 x 128: 24 -> 27 us, 16 x 48 x 16 x 64: 25 -> 27; also 2 x 60
+// queries x 2000 keys x 8 x 128: 33 -> 45.
 //
 // With dropout the dQ pass draws the keep decisions (16 keys of a query row per Philox call, as
 // in the forward) and leaves them as one bit each, [B H][key / 32][query] words, for the dK / dV
-// pass, whose lanes are keys.
+// pass, whose lanes are keys; side by side with the other, that pass draws them for itself.
 #include "flash_common.cuh"
 #include "kernels.h"
 
@@ -45,10 +51,14 @@ struct FlashBwdParams {
   int k_steps;            // ceil(Dr / 16)
   int Rq, Rk;             // Sq and Sk rounded up to 128
   TileWalk walk;
+  int splits;             // dQ pass: work items per row tile, each takes tiles_per_split key tiles
+  int tiles_per_split;
+  float* part;            // splits > 1: [splits][B Sq H][Dr] fp32 shares of dQ
+  int64_t part_rows;      // B Sq H
   const float* nlse;      // [B H][Rq]  -log2(e) * lse ; -inf for rows without any key (and padding)
   const float* ndelta;    // [B H][Rq]  -rowsum(dO O) * keep probability ; 0 in the padding
   const float* kb2;       // [B][Rk] log2(e) * key bias, 0 in the padding, or nullptr
-  uint32_t* keep;         // [B H of this launch][Rk / 32][Rq] keep bits (dropout), or nullptr
+  uint32_t* keep;         // [B H of this launch][Rk / 32][Rq] keep bits (dropout in two launches)
   const float* rel;       // [H, Sq + Sk - 1] or nullptr
   float* drel;            // same shape fp32 accumulator or nullptr
   void* out1;             // dQ or dK: rows (b, s, head) spaced row_stride elements apart
@@ -67,14 +77,21 @@ struct FlashBwdParams {
 //   ndelta [B H][Rq]  -keep_prob * sum_d dO[b, i, h, d] * O[b, i, h, d]
 // dO and O are contiguous [B, Sq, H, Dr].  A block takes 32 query rows of one batch entry and
 // 8 heads: lanes along d while reading (16-byte loads), then the sums pass through shared
-// memory so that the stores run along the rows.
+// memory so that the stores run along the rows.  The blocks of the first heads also write
+//   kb2    [B][Rk]    log2(e) * key bias, 0 in the padding
 template <typename T>
 __global__ void __launch_bounds__(256) flash_bwd_stats_kernel(
     const T* __restrict__ dout, const T* __restrict__ out, const float* __restrict__ lse,
-    float* __restrict__ nlse, float* __restrict__ ndelta, int H, int Sq, int Rq, int Dr, int lanes,
+    float* __restrict__ nlse, float* __restrict__ ndelta, const float* __restrict__ kbias,
+    float* __restrict__ kb2, int H, int Sq, int Rq, int Sk, int Rk, int Dr, int lanes,
     float keep_prob) {
   __shared__ float sums[8][33];
+  pdl_launch();
   const int i0 = blockIdx.x * 32, h0 = blockIdx.y * 8, b = blockIdx.z;
+  if (kbias != nullptr && blockIdx.y == 0)
+    for (int key = blockIdx.x * 256 + threadIdx.x; key < Rk; key += gridDim.x * 256)
+      kb2[static_cast<int64_t>(b) * Rk + key] =
+          key < Sk ? kbias[static_cast<int64_t>(b) * Sk + key] * kLog2e : 0.f;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rows_per_warp = 32 / lanes;        // `lanes` (8 or 16) threads share a row of Dr
   const int d = (lane % lanes) * 8;
@@ -106,16 +123,6 @@ __global__ void __launch_bounds__(256) flash_bwd_stats_kernel(
   }
 }
 
-// kb2 [B][Rk] = log2(e) * key bias, padded with zeros
-__global__ void __launch_bounds__(256) flash_bwd_bias_kernel(const float* __restrict__ kbias,
-                                                             float* __restrict__ kb2, int Sk,
-                                                             int Rk) {
-  const int key = blockIdx.x * 256 + threadIdx.x, b = blockIdx.y;
-  if (key < Rk)
-    kb2[static_cast<int64_t>(b) * Rk + key] =
-        key < Sk ? kbias[static_cast<int64_t>(b) * Sk + key] * kLog2e : 0.f;
-}
-
 template <int D, bool kKeys>
 struct BwdSmem {
   static constexpr int kTile = 128 * D * 2;
@@ -136,11 +143,12 @@ struct BwdSmem {
 // 10 warps: TMA, MMA and 8 softmax warps; warps w and w + 4 share a quarter of the TMEM lanes
 // (rows) and split the tile's columns in halves.
 // kKeys: the dK / dV pass.  kGeneral: key bias, relative bias, causal mask or ragged lengths.
-template <int D, bool kKeys, bool kGeneral, typename T>
-__global__ void __launch_bounds__(320, 1)
-flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ CUtensorMap tm_x2,
-                 const __grid_constant__ CUtensorMap tm_y1, const __grid_constant__ CUtensorMap tm_y2,
-                 const FlashBwdParams p) {
+// kDraw: with dropout the dK / dV pass draws the keep decisions itself, and the dQ pass leaves none.
+// CTA `cta` of `ctas` that run the pass.
+template <int D, bool kKeys, bool kGeneral, bool kDraw, typename T>
+__device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtensorMap& tm_x2,
+                                         const CUtensorMap& tm_y1, const CUtensorMap& tm_y2,
+                                         const FlashBwdParams& p, const int cta, const int ctas) {
   using L = BwdSmem<D, kKeys>;
   constexpr int kTileBytes = L::kTile;
   constexpr int kBlkBytes = 128 * 128;
@@ -188,12 +196,14 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
   // D = 128 the products are twice as long and two stages leave the loads less slack, and the dQ
   // pass lost (170 -> 183 us at 4 x 2048 x 16, causal).
   constexpr bool kFirst = D == 64;
-  const int items = p.walk.items();
+  const int items = p.walk.items() * (kKeys ? 1 : p.splits);
   const bool drop = p.thr7 != 0;
 
-  // first streamed tile of a row tile, and how many (at least one: a row tile that nothing
-  // reaches still has its zeros written)
-  auto tiles_of = [&](int tile, int& first) {
+  // row tile and (batch, head) of a work item, its first streamed tile and how many (at least one: a
+  // row tile or a split that nothing reaches still has its zeros written)
+  auto item_at = [&](int item, int& tile, int& bhl, int& first) {
+    const int unit = kKeys || p.splits == 1 ? item : item / p.splits;
+    p.walk.at(unit, tile, bhl);
     int n;
     if constexpr (kKeys) {
       const int q_tiles = p.Rq >> 7;
@@ -204,6 +214,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
       first = 0;
       n = p.Rk >> 7;
       if (p.causal) n = max(1, min(n, (min(p.Sk, tile * 128 + 128 + diag) + 127) / 128));
+      if (p.splits > 1) {
+        first = (item - unit * p.splits) * p.tiles_per_split;
+        n = max(1, min(p.tiles_per_split, n - first));
+      }
     }
     return n;
   };
@@ -236,6 +250,9 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  // what the kernels before this one wrote is read from here on
+  pdl_wait();
+  pdl_launch();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -243,15 +260,15 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
       tc::tma_prefetch_desc(&tm_x2);
       tc::tma_prefetch_desc(&tm_y1);
       tc::tma_prefetch_desc(&tm_y2);
-      const uint32_t vec_bytes = kKeys ? 1024u + (drop ? 2048u : 0u) : (p.kb2 != nullptr ? 512u : 0u);
+      const bool load_keep = !kDraw && drop;
+      const uint32_t vec_bytes = kKeys ? 1024u + (load_keep ? 2048u : 0u) : (p.kb2 != nullptr ? 512u : 0u);
       bool ok = true;
       int t = 0, w = 0;
-      for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++w) {
+      for (int item = cta; item < items && ok; item += ctas, ++w) {
         int tile, bhl, first;
-        p.walk.at(item, tile, bhl);
+        const int n = item_at(item, tile, bhl, first);
         const int bh = p.walk.bh0 + bhl;
         const int batch = bh / p.H, head = bh - batch * p.H;
-        const int n = tiles_of(tile, first);
         auto load_y = [&](int j) -> bool {
           const int st = t % kStages;
           const uint32_t ph = ((t / kStages) & 1) ^ 1;
@@ -271,7 +288,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
           if constexpr (kKeys) {
             tc::bulk_load(v, p.nlse + static_cast<int64_t>(bh) * p.Rq + s0, 512, &y_full[st]);
             tc::bulk_load(v + 512, p.ndelta + static_cast<int64_t>(bh) * p.Rq + s0, 512, &y_full[st]);
-            if (drop)
+            if (load_keep)
 #pragma unroll
               for (int r = 0; r < 4; ++r)
                 tc::bulk_load(v + 1024 + r * 512,
@@ -343,15 +360,14 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
       auto n_of = [&](int item) {
         if (item >= items) return 0;
         int tile, bhl, first;
-        p.walk.at(item, tile, bhl);
-        return tiles_of(tile, first);
+        return item_at(item, tile, bhl, first);
       };
       bool ok = true;
-      int t = 0, w = 0, item = blockIdx.x;
+      int t = 0, w = 0, item = cta;
       int n = n_of(item);
       if (n > 0) ok = issue_s(0, 0, true, n == 1) && issue_dp(0, 0, true, n == 1);
       while (item < items && ok) {
-        const int next_item = item + gridDim.x;
+        const int next_item = item + ctas;
         const int next_n = n_of(next_item);
         for (int j = 0; j < n; ++j, ++t) {
           const int st = t % kStages;
@@ -395,7 +411,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
     const int r_in = quarter * 32 + lane;
     const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     uint64_t seed = 0, offset = 0;
-    if (!kKeys && drop) philox_unpack(p.rng, seed, offset);
+    if ((!kKeys || kDraw) && drop) philox_unpack(p.rng, seed, offset);
     const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
     const int sk16 = (p.Sk + 15) >> 4;
     // dS is formed without the factors scale and 1 / keep_prob; they are applied once to
@@ -405,8 +421,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
 
     // accumulators of work item `item` out of tensor memory
     auto read_out = [&](int item) {
-      int tile, bhl;
-      p.walk.at(item, tile, bhl);
+      int tile, bhl, first;
+      item_at(item, tile, bhl, first);
       const int bh = p.walk.bh0 + bhl;
       const int batch = bh / p.H, head = bh - batch * p.H;
       const int row = tile * 128 + r_in;
@@ -419,13 +435,24 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
                       : static_cast<T*>(p.out1) + at * p.row_stride1;
       const int c0 = kKeys ? 0 : half * (D / 2);
       const uint32_t col = second ? kColA2 : kColA1;
+      float* share = nullptr;
+      if (!kKeys && p.splits > 1)
+        share = p.part + (static_cast<int64_t>(item % p.splits) * p.part_rows + at) * p.Dr;
       tc::fence_after_sync();
 #pragma unroll
       for (int c = 0; c < (kKeys ? D : D / 2); c += 32) {
         uint32_t r[32];
         tc::tmem_ld_x32(tmem_row + col + c0 + c, r);
         tc::tmem_ld_wait();
-        if (row < rows) {
+        if (!kKeys && share != nullptr) {
+          if (row < rows) {
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+              if (c0 + c + g * 4 < p.Dr)
+                *reinterpret_cast<uint4*>(share + c0 + c + g * 4) =
+                    make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+          }
+        } else if (row < rows) {
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
             if (c0 + c + g * 8 < p.Dr) {
@@ -449,8 +476,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
       a = 0.f;
       b = 0.f;
       if (item >= items) return;
-      int tile, bhl;
-      p.walk.at(item, tile, bhl);
+      int tile, bhl, first;
+      item_at(item, tile, bhl, first);
       const int bh = p.walk.bh0 + bhl;
       if constexpr (kKeys) {
         if (kGeneral && p.kb2 != nullptr)
@@ -475,26 +502,24 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
       for (int i = lane; i < L::kRelFloats; i += 32)
         cp_async4(rel_buf + buf * L::kRelFloats + i, src + max(1 - p.Sq, min(d0 + i, p.Sk - 1)));
     };
-    if (has_rel && static_cast<int>(blockIdx.x) < items) {
+    if (has_rel && cta < items) {
       int tile, bhl, first;
-      p.walk.at(blockIdx.x, tile, bhl);
-      tiles_of(tile, first);
+      item_at(cta, tile, bhl, first);
       fetch_rel(tile, bhl, first, 0);
     }
 
     bool ok = true;
     int t = 0, w = 0, prev_item = -1;
     float rs_a, rs_b;
-    row_scalars(blockIdx.x, rs_a, rs_b);
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++w) {
+    row_scalars(cta, rs_a, rs_b);
+    for (int item = cta; item < items && ok; item += ctas, ++w) {
       int tile, bhl, first;
-      p.walk.at(item, tile, bhl);
+      const int n = item_at(item, tile, bhl, first);
       const int bh = p.walk.bh0 + bhl;
       const int head = bh % p.H;
       const int row = tile * 128 + r_in;
-      const int n = tiles_of(tile, first);
       const float row_a = rs_a, row_b = rs_b;
-      row_scalars(item + gridDim.x, rs_a, rs_b);      // under this item's work
+      row_scalars(item + ctas, rs_a, rs_b);      // under this item's work
       const uint64_t ra2 = f2_pack(row_a, row_a), rb2 = f2_pack(row_b, row_b);
       for (int j = 0; j < n; ++j, ++t) {
         const int st = t % kStages;
@@ -505,10 +530,9 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
           __syncwarp();     // (visible to the warp, and the other buffer's readers are done)
           if (j + 1 < n) {
             fetch_rel(tile, bhl, first + j + 1, (t + 1) & 1);
-          } else if (item + static_cast<int>(gridDim.x) < items) {
+          } else if (item + ctas < items) {
             int next_tile, next_bhl, next_first;
-            p.walk.at(item + gridDim.x, next_tile, next_bhl);
-            tiles_of(next_tile, next_first);
+            item_at(item + ctas, next_tile, next_bhl, next_first);
             fetch_rel(next_tile, next_bhl, next_first, (t + 1) & 1);
           }
         }
@@ -521,16 +545,32 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
           for (int g = 0; g < 4; ++g) {
             const uint4 kw = philox_keep16(seed, offset, base + g, add4);
             keep16[g][0] = kw.x; keep16[g][1] = kw.y; keep16[g][2] = kw.z; keep16[g][3] = kw.w;
-            uint32_t m = 0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)     // bit 7 of the four bytes, gathered by one multiply
-              m |= ((((keep16[g][i] >> 7) & 0x01010101u) * 0x01020408u) >> 24) << (4 * i);
-            if (g & 1) bits[g >> 1] |= m << 16;
-            else bits[g >> 1] = m;
+            if constexpr (!kDraw) {
+              const uint32_t m = keep_bits16(kw);
+              if (g & 1) bits[g >> 1] |= m << 16;
+              else bits[g >> 1] = m;
+            }
           }
-          uint32_t* dst = p.keep + (static_cast<int64_t>(bhl) * (p.Rk >> 5) + (col0 >> 5)) * p.Rq + row;
-          dst[0] = bits[0];
-          dst[p.Rq] = bits[1];
+          if constexpr (!kDraw) {
+            uint32_t* dst = p.keep + (static_cast<int64_t>(bhl) * (p.Rk >> 5) + (col0 >> 5)) * p.Rq + row;
+            dst[0] = bits[0];
+            dst[p.Rq] = bits[1];
+          }
+        }
+        // ---- ... of the warp's 32 keys and 64 queries (dK / dV pass), two queries per lane, into the
+        // words that the other form loads ----
+        if constexpr (kKeys && kDraw) {
+          if (drop) {
+            uint32_t* words = reinterpret_cast<uint32_t*>(s_vec + st * L::kVec + 1024 + quarter * 512) + half * 64;
+#pragma unroll
+            for (int i = lane; i < 64; i += 32) {
+              const uint64_t base = (static_cast<uint64_t>(bh) * p.Sq + min(col0 + i, p.Sq - 1)) * sk16 +
+                                    ((tile * 128 + quarter * 32) >> 4);
+              words[i] = keep_bits16(philox_keep16(seed, offset, base, add4)) |
+                         keep_bits16(philox_keep16(seed, offset, base + 1, add4)) << 16;
+            }
+            __syncwarp();
+          }
         }
         // ---- P ----
         if (!tc::mbar_wait_warp(s_full, t & 1, abort_flag)) { ok = false; break; }
@@ -745,63 +785,201 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
   }
 }
 
+// One pass.
 template <int D, bool kKeys, bool kGeneral, typename T>
-static int launch_bwd_d(const CUtensorMap& x1, const CUtensorMap& x2, const CUtensorMap& y1,
-                        const CUtensorMap& y2, const FlashBwdParams& p, cudaStream_t stream) {
+__global__ void __launch_bounds__(320, 1)
+flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ CUtensorMap tm_x2,
+                 const __grid_constant__ CUtensorMap tm_y1, const __grid_constant__ CUtensorMap tm_y2,
+                 const __grid_constant__ FlashBwdParams p) {
+  bwd_pass<D, kKeys, kGeneral, false, T>(tm_x1, tm_x2, tm_y1, tm_y2, p, blockIdx.x, gridDim.x);
+}
+
+// Both passes side by side, the dQ pass on the first `q_ctas` CTAs.
+template <int D, bool kGeneral, typename T>
+__global__ void __launch_bounds__(320, 1)
+flash_bwd_both_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                      const __grid_constant__ FlashBwdParams pq,
+                      const __grid_constant__ FlashBwdParams pk, const int q_ctas) {
+  const int cta = blockIdx.x;
+  if (cta < q_ctas)
+    bwd_pass<D, false, kGeneral, true, T>(tm_q, tm_do, tm_k, tm_v, pq, cta, q_ctas);
+  else
+    bwd_pass<D, true, kGeneral, true, T>(tm_k, tm_v, tm_q, tm_do, pk, cta - q_ctas,
+                                         gridDim.x - q_ctas);
+}
+
+// dQ of rows whose keys were split over work items: the shares added in their order
+template <typename T>
+__global__ void __launch_bounds__(256) flash_dq_combine_kernel(const float* __restrict__ part,
+                                                               T* __restrict__ dq, int splits,
+                                                               int64_t n, float scale) {
+  const int64_t at = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) * 8;
+  if (at >= n) return;
+  float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int s = 0; s < splits; ++s) {
+    float x[8];
+    Vec8<float>::load(part + s * n + at, x);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] += x[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] *= scale;
+  Vec8<T>::store(dq + at, v);
+}
+
+// A kernel's shared memory, allowed once per kernel
+template <typename K>
+static bool allow_smem(K kernel, int bytes, bool& configured) {
+  if (!configured)
+    configured = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) ==
+                 cudaSuccess;
+  return configured;
+}
+
+// `early`: the kernel's prologue may run under the end of the kernel before it (it waits in
+// pdl_wait), which saves 2 - 4 us of a short backward.  CTAs that go round several times were slower
+// for it: 768 + 768 items of 3 tiles, side by side, 106 -> 125 us (128 + 128 of 1: 27 -> 23), one pass
+// after the other 2048 + 2048 of 4, causal, 226 -> 241 (384 + 384 of 3, dropout: 75 -> 74).
+template <typename... P, typename... A>
+static int launch_bwd(void (*kernel)(P...), int ctas, int smem, bool early, cudaStream_t stream,
+                      const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(320);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
+  count_launch();
+  return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? 0 : 4;
+}
+
+template <int D, bool kKeys, bool kGeneral, typename T>
+static int launch_pass(const CUtensorMap& x1, const CUtensorMap& x2, const CUtensorMap& y1,
+                       const CUtensorMap& y2, const FlashBwdParams& p, cudaStream_t stream) {
   constexpr int kSmem = BwdSmem<D, kKeys>::kTotal;
   static_assert(kSmem <= 227 * 1024, "flash backward: shared memory over the per-CTA limit");
   auto kernel = flash_bwd_kernel<D, kKeys, kGeneral, T>;
   static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
-        cudaSuccess)
-      return 3;
-    configured = true;
-  }
-  const int64_t items = static_cast<int64_t>(p.walk.row_tiles) * p.walk.nbh;
+  if (!allow_smem(kernel, kSmem, configured)) return 3;
+  const int64_t items = static_cast<int64_t>(p.walk.row_tiles) * p.walk.nbh * p.splits;
   const int64_t cap = sm_count();
-  count_launch();
-  kernel<<<static_cast<int>(items < cap ? items : cap), 320, kSmem, stream>>>(x1, x2, y1, y2, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+  return launch_bwd(kernel, static_cast<int>(items < cap ? items : cap), kSmem, items <= 3 * cap, stream,
+                    x1, x2, y1, y2, p);
 }
 
-template <bool kKeys>
-static int launch_bwd_pass(const CUtensorMap& x1, const CUtensorMap& x2, const CUtensorMap& y1,
-                           const CUtensorMap& y2, const FlashBwdParams& p, bool general, bool bf16,
-                           cudaStream_t stream) {
-#define FLASH_BWD_CASE(D_, T_)                                                            \
-  return general ? launch_bwd_d<D_, kKeys, true, T_>(x1, x2, y1, y2, p, stream)           \
-                 : launch_bwd_d<D_, kKeys, false, T_>(x1, x2, y1, y2, p, stream)
-  if (p.Dr <= 64) {
-    if (bf16) FLASH_BWD_CASE(64, __nv_bfloat16);
-    FLASH_BWD_CASE(64, __half);
+// The passes of `pq` (dQ) and `pk` (dK / dV), side by side or one after the other
+template <int D, bool kGeneral, typename T>
+static int launch_passes(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v,
+                         const CUtensorMap& dout, const FlashBwdParams& pq, const FlashBwdParams& pk,
+                         int q_ctas, cudaStream_t stream) {
+  if (q_ctas == 0) {
+    // dQ first: with dropout it leaves the keep bits that the dK / dV pass reads
+    const int rc = launch_pass<D, false, kGeneral, T>(q, dout, k, v, pq, stream);
+    return rc != 0 ? rc : launch_pass<D, true, kGeneral, T>(k, v, q, dout, pk, stream);
   }
-  if (bf16) FLASH_BWD_CASE(128, __nv_bfloat16);
-  FLASH_BWD_CASE(128, __half);
-#undef FLASH_BWD_CASE
+  constexpr int kSmemQ = BwdSmem<D, false>::kTotal, kSmemK = BwdSmem<D, true>::kTotal;
+  constexpr int kSmem = kSmemQ > kSmemK ? kSmemQ : kSmemK;
+  auto kernel = flash_bwd_both_kernel<D, kGeneral, T>;
+  static bool configured = false;
+  if (!allow_smem(kernel, kSmem, configured)) return 3;
+  const int64_t items = static_cast<int64_t>(pk.walk.row_tiles) * pk.walk.nbh;
+  const int64_t k_cap = sm_count() - q_ctas;
+  const int64_t q_items = static_cast<int64_t>(pq.walk.row_tiles) * pq.walk.nbh * pq.splits;
+  const bool early = q_items + items <= 2 * sm_count();
+  return launch_bwd(kernel, q_ctas + static_cast<int>(items < k_cap ? items : k_cap), kSmem, early, stream,
+                    q, k, v, dout, pq, pk, q_ctas);
+}
+
+template <typename T>
+static int launch_typed(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v,
+                        const CUtensorMap& dout, const FlashBwdParams& pq, const FlashBwdParams& pk,
+                        int q_ctas, bool general, cudaStream_t stream) {
+  if (pq.Dr <= 64)
+    return general ? launch_passes<64, true, T>(q, k, v, dout, pq, pk, q_ctas, stream)
+                   : launch_passes<64, false, T>(q, k, v, dout, pq, pk, q_ctas, stream);
+  return general ? launch_passes<128, true, T>(q, k, v, dout, pq, pk, q_ctas, stream)
+                 : launch_passes<128, false, T>(q, k, v, dout, pq, pk, q_ctas, stream);
 }
 
 static int round128(int n) { return (n + 127) / 128 * 128; }
 
-FlashBwdScratch flash_bwd_scratch(int B, int H, int Sq, int Sk, bool key_bias, float p_drop) {
-  FlashBwdScratch s;
+// One launch or two, and how many CTAs of one launch take the dQ pass (0: two launches).  Side by
+// side the passes fill the waves that each alone would leave partly empty and save a launch; one
+// after the other the dK / dV pass reads the keep bits that the dQ pass drew instead of drawing them
+// again, and each pass has its tensors in L2 to itself.  Weighed as rounds of work items, in tiles
+// of the dQ pass: a tile of dK / dV takes 1.2 of them (2 with the relative bias's gradient, 0.3 more
+// drawing), an item a quarter more (D = 128: 1.5, its accumulators leave tensor memory without a
+// second set to go on with), a launch 1.5; both in one came out 5 % over that.  Under a causal mask items differ and the heaviest go first, so that
+// no whole rounds are lost in two launches or one: side by side up to 5 waves of each.
+// Measured, two launches -> one (us): 1 x 512 x 16 x 64: 33 -> 22; 1 x 2048 x 12 x 64 causal: 102 -> 79;
+// 4 x 1024 x 16 x 128: 199 -> 188; 4 x 256 x 12 x 64 with dropout: 33 -> 25; but 32 x 512 x 16 x 64 with
+// dropout 367 -> 420, without 258 -> 265, causal 225 -> 236.
+static int both_q_ctas(int64_t q_items, int64_t k_items, int64_t q_item_tiles, int64_t q_tiles, int D,
+                       bool causal, bool rel, bool drop) {
+  const int64_t sms = sm_count();
+  const double item = D <= 64 ? 0.25 : 1.5;
+  const double k_tile = rel ? 2.0 : 1.2;
+  const double q_item = q_item_tiles + item, k_item = q_tiles * k_tile + item;
+  const double k_item_draws = q_tiles * (k_tile + (drop ? 0.3 : 0.0)) + item;
+  if (q_items + k_items <= sms) return static_cast<int>(q_items);
+  auto rounds = [](int64_t items, int64_t ctas) { return (items + ctas - 1) / ctas; };
+  double best = (rounds(q_items, sms) * q_item + rounds(k_items, sms) * k_item + 1.5) / 1.05;
+  if (causal && !drop) best = q_items + k_items > 10 * sms ? 0.0 : 1e30;
+  int best_n = 0;
+  for (int64_t r = rounds(q_items, sms - 1); r * q_item < best; ++r) {
+    const int64_t n = rounds(q_items, r);       // the fewest CTAs with r rounds
+    const double k_time = rounds(k_items, sms - n) * k_item_draws;
+    const double t = r * q_item > k_time ? r * q_item : k_time;
+    if (t < best) { best = t; best_n = static_cast<int>(n); }
+    if (n == 1) break;
+  }
+  return best_n;
+}
+
+FlashBwdPlan flash_bwd_plan(int B, int H, int Sq, int Sk, int D, bool packed, bool causal,
+                            bool key_bias, bool rel, float p_drop) {
+  FlashBwdPlan s;
   const int64_t rq = round128(Sq), rk = round128(Sk), bh = static_cast<int64_t>(B) * H;
+  const int64_t q_tiles = rq / 128, k_tiles = rk / 128;
+  const bool drop = dropout_thr7(p_drop) != 0;
+  // Few queries, many keys: the keys of a dQ item are split over idle SMs, down to the other pass's
+  // chain of tiles, where that takes four tiles off its own.  (2 x 60 queries x 2000 keys x 8 x 128:
+  // 72 -> 48 us for the whole backward.)
+  s.splits = 1;
+  if (!packed && bh > 0 && k_tiles > q_tiles) {
+    int64_t n = sm_count() / (q_tiles * bh);
+    const int64_t most = (k_tiles + q_tiles - 1) / q_tiles;
+    if (n > most) n = most;
+    if (n >= 2) {
+      const int64_t per = (k_tiles + n - 1) / n;
+      if (k_tiles - per >= 4) s.splits = static_cast<int>((k_tiles + per - 1) / per);
+    }
+  }
+  s.q_ctas = bh == 0 ? 0
+                     : both_q_ctas(q_tiles * bh * s.splits, k_tiles * bh,
+                                   (k_tiles + s.splits - 1) / s.splits, q_tiles, D, causal, rel, drop);
   s.stats = 2 * bh * rq;
   s.bias = key_bias ? B * rk : 0;
   // keep bits of as many (batch, head) pairs at a time as fit 1 GB (at least one)
+  const bool keep = drop && s.q_ctas == 0;
   const int64_t words = rk / 32 * rq;
-  int64_t pairs = words > 0 ? (int64_t(1) << 28) / words : bh;
+  int64_t pairs = keep && words > 0 ? (int64_t(1) << 28) / words : bh;
   if (pairs < 1) pairs = 1;
   if (pairs > bh) pairs = bh;
-  const bool drop = dropout_thr7(p_drop) != 0;
-  s.pairs = static_cast<int>(drop ? pairs : bh);
-  s.keep = drop ? s.pairs * words : 0;
+  s.pairs = static_cast<int>(pairs);
+  s.keep = keep ? s.pairs * words : 0;
+  s.part = s.splits > 1 ? s.splits * bh * Sq * D : 0;
   return s;
 }
 
 int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
-                     const float* lse, float* scratch, void* dq, void* dk, void* dv,
-                     int64_t dq_row_stride, int64_t dkv_row_stride, const float* kbias,
+                     const float* lse, const FlashBwdPlan& plan, float* scratch, void* dq, void* dk,
+                     void* dv, int64_t dq_row_stride, int64_t dkv_row_stride, const float* kbias,
                      const float* rel, float* drel, int B, int H, int Sq, int Sk, int D,
                      const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
                      float scale, int causal, float p_drop, PhiloxArgs rng, bool bf16, int* status,
@@ -814,20 +992,22 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o,
       !make_tmap_bshd(&tv, v, B, Sk, H, D, v_strides[0], v_strides[1], v_strides[2], 128, bf16) ||
       !make_tmap_bshd(&tdo, dout, B, Sq, H, D, do_strides[0], do_strides[1], do_strides[2], 128, bf16))
     return 2;
-  const FlashBwdScratch sizes = flash_bwd_scratch(B, H, Sq, Sk, kbias != nullptr, p_drop);
   FlashBwdParams p;
   p.Sq = Sq; p.Sk = Sk; p.H = H; p.Dr = D;
   p.k_steps = (D + 15) / 16;
   p.Rq = round128(Sq); p.Rk = round128(Sk);
   p.thr7 = dropout_thr7(p_drop);   // same quantisation as the forward kernel
   const float keep_prob = 1.f - p.thr7 / 128.f;
-  // scratch: nlse | ndelta | key bias | keep bits, each a multiple of 128 words
+  // scratch: nlse | ndelta | key bias | keep bits | shares of dQ, each a multiple of 4 words (the
+  // first four of 128)
   float* nlse = scratch;
-  float* ndelta = nlse + sizes.stats / 2;
-  float* kb2 = ndelta + sizes.stats / 2;
+  float* ndelta = nlse + plan.stats / 2;
+  float* kb2 = ndelta + plan.stats / 2;
   p.nlse = nlse; p.ndelta = ndelta;
   p.kb2 = kbias != nullptr ? kb2 : nullptr;
-  p.keep = p.thr7 != 0 ? reinterpret_cast<uint32_t*>(kb2 + sizes.bias) : nullptr;
+  p.keep = plan.keep != 0 ? reinterpret_cast<uint32_t*>(kb2 + plan.bias) : nullptr;
+  p.part = kb2 + plan.bias + plan.keep;
+  p.part_rows = static_cast<int64_t>(B) * Sq * H;
   p.rel = rel; p.drel = drel;
   p.scale = scale; p.scale_log2 = scale * kLog2e; p.inv_keep = 1.f / keep_prob;
   p.causal = causal; p.rng = rng; p.status = status;
@@ -840,35 +1020,48 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o,
     if (bf16)
       flash_bwd_stats_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(
           static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), lse, nlse,
-          ndelta, H, Sq, p.Rq, D, lanes, keep_prob);
+          ndelta, kbias, kb2, H, Sq, p.Rq, Sk, p.Rk, D, lanes, keep_prob);
     else
       flash_bwd_stats_kernel<__half><<<grid, 256, 0, stream>>>(
-          static_cast<const __half*>(dout), static_cast<const __half*>(o), lse, nlse, ndelta, H, Sq,
-          p.Rq, D, lanes, keep_prob);
-  }
-  if (kbias != nullptr) {
-    count_launch();
-    flash_bwd_bias_kernel<<<dim3((p.Rk + 255) / 256, B), 256, 0, stream>>>(kbias, kb2, Sk, p.Rk);
+          static_cast<const __half*>(dout), static_cast<const __half*>(o), lse, nlse, ndelta, kbias,
+          kb2, H, Sq, p.Rq, Sk, p.Rk, D, lanes, keep_prob);
   }
   const bool general = kbias != nullptr || rel != nullptr || causal || Sk % 128 != 0;
   p.walk.H = H;
   const int bh = B * H;
-  for (int at = 0; at < bh; at += sizes.pairs) {
-    p.walk.bh0 = at;
-    p.walk.nbh = bh - at < sizes.pairs ? bh - at : sizes.pairs;
-    // dQ first: with dropout it leaves the keep bits that the dK / dV pass reads
-    p.walk.row_tiles = p.Rq / 128;
-    p.walk.by_cost = causal ? 2 : 0;
-    p.out1 = dq; p.row_stride1 = dq_row_stride;
-    p.out2 = nullptr; p.row_stride2 = 0;
-    int rc = launch_bwd_pass<false>(tq, tdo, tk, tv, p, general, bf16, stream);
+  FlashBwdParams pq = p, pk = p;
+  pq.walk.row_tiles = p.Rq / 128;
+  pq.walk.by_cost = causal ? 2 : 0;
+  pq.splits = plan.splits;
+  pq.tiles_per_split = (p.Rk / 128 + plan.splits - 1) / plan.splits;
+  pq.out1 = dq; pq.row_stride1 = dq_row_stride;
+  pq.out2 = nullptr; pq.row_stride2 = 0;
+  pk.walk.row_tiles = p.Rk / 128;
+  pk.walk.by_cost = causal ? 1 : 0;
+  pk.splits = 1;
+  pk.tiles_per_split = p.Rq / 128;
+  pk.out1 = dk; pk.row_stride1 = dkv_row_stride;
+  pk.out2 = dv; pk.row_stride2 = dkv_row_stride;
+  for (int at = 0; at < bh; at += plan.pairs) {
+    pq.walk.bh0 = pk.walk.bh0 = at;
+    pq.walk.nbh = pk.walk.nbh = bh - at < plan.pairs ? bh - at : plan.pairs;
+    const int rc =
+        bf16 ? launch_typed<__nv_bfloat16>(tq, tk, tv, tdo, pq, pk, plan.q_ctas, general, stream)
+             : launch_typed<__half>(tq, tk, tv, tdo, pq, pk, plan.q_ctas, general, stream);
     if (rc != 0) return rc;
-    p.walk.row_tiles = p.Rk / 128;
-    p.walk.by_cost = causal ? 1 : 0;
-    p.out1 = dk; p.row_stride1 = dkv_row_stride;
-    p.out2 = dv; p.row_stride2 = dkv_row_stride;
-    rc = launch_bwd_pass<true>(tk, tv, tq, tdo, p, general, bf16, stream);
-    if (rc != 0) return rc;
+  }
+  if (plan.splits > 1) {
+    const int64_t n = p.part_rows * D;
+    const unsigned blocks = static_cast<unsigned>((n / 8 + 255) / 256);
+    const float f = p.scale * p.inv_keep;
+    count_launch();
+    if (bf16)
+      flash_dq_combine_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(
+          p.part, static_cast<__nv_bfloat16*>(dq), plan.splits, n, f);
+    else
+      flash_dq_combine_kernel<__half><<<blocks, 256, 0, stream>>>(p.part, static_cast<__half*>(dq),
+                                                                  plan.splits, n, f);
+    if (cudaGetLastError() != cudaSuccess) return 4;
   }
   return 0;
 }

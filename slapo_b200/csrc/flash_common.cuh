@@ -62,6 +62,22 @@ template <> __device__ __forceinline__ uint32_t pack16<__half>(float a, float b)
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// Overlap of a kernel's prologue with the kernel before it in the stream: a kernel that the next
+// one may start under says so, and one that was launched that way waits until all work before it
+// is complete and visible (at once, when it was launched the ordinary way).
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// the 16 decisions of one Philox call as bits
+__device__ __forceinline__ uint32_t keep_bits16(const uint4& kw) {
+  const uint32_t w[4] = {kw.x, kw.y, kw.z, kw.w};
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)       // bit 7 of the four bytes, gathered by one multiply
+    m |= ((((w[i] >> 7) & 0x01010101u) * 0x01020408u) >> 24) << (4 * i);
+  return m;
+}
+
 // Row tiles of 128 of all (batch, head) pairs, walked by a persistent grid.  Under a causal
 // mask the tiles differ in cost: they are ordered by cost, heaviest first, over all heads.
 // Otherwise the tiles of one head are neighbours, so that the tensors they share stay in L2.

@@ -64,6 +64,12 @@ CASES = [
     (2, 100, 1500, 8, 80, FP, "g", 0.1),
     (8, 1, 1500, 16, 128, BF, "c", 0.0),
     (1, 48, 2048, 4, 40, BF, "cr", 0.1),
+    (1, 400, 1700, 2, 64, BF, "c", 0.1),       # dQ: keys split, some splits beyond the diagonal
+    (2, 400, 1700, 2, 128, FP, "ck", 0.0),
+    (1, 1700, 100, 6, 128, BF, "", 0.1),       # passes of unequal lengths side by side
+    (9, 256, 256, 16, 64, FP, "c", 0.0),       # ... of several work items per CTA
+    (6, 256, 256, 16, 128, BF, "k", 0.1),
+    (20, 130, 130, 16, 64, BF, "", 0.1),
     (1, 1, 1, 1, 8, BF, "", 0.0),
     (2, 129, 1, 2, 64, BF, "", 0.0),
 ]
