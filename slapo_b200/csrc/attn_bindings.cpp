@@ -138,39 +138,58 @@ Tensor flash_attn_dropout_mask(int64_t B, int64_t H, int64_t Sq, int64_t Sk, dou
   return mask;
 }
 
-// the caches of one layer grown by new tokens: ([B, past + n, H, D] contiguous) k and v
-std::tuple<Tensor, Tensor> kv_append(const Tensor& past_k, const Tensor& past_v, const Tensor& k,
+// Whether one launch takes the four tensors: plain CUDA tensors outside of autograd and of functorch
+// / forward-mode transforms, one type and device, contiguous caches, 16-byte aligned heads.
+bool kv_append_takes(const Tensor* const (&past)[2], const Tensor* const (&fresh)[2]) {
+  static constexpr c10::DispatchKeySet kWrapped({c10::DispatchKey::FuncTorchBatched,
+                                                 c10::DispatchKey::FuncTorchGradWrapper,
+                                                 c10::DispatchKey::Functionalize, c10::DispatchKey::Python,
+                                                 c10::DispatchKey::ZeroTensor, c10::DispatchKey::Negative});
+  const Tensor& k = *fresh[0];
+  const auto dtype = k.scalar_type();
+  if (dtype != at::kBFloat16 && dtype != at::kHalf && dtype != at::kFloat) return false;
+  const bool grad = at::GradMode::is_enabled();
+  for (const Tensor* t : {past[0], past[1], fresh[0], fresh[1]}) {
+    if (t->key_set().has_any(kWrapped) || t->layout() != at::kStrided || !t->is_cuda() || t->dim() != 4 ||
+        t->scalar_type() != dtype || t->get_device() != k.get_device() || (grad && t->requires_grad()) ||
+        t->_fw_grad(/*level=*/0).defined() || reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0)
+      return false;
+  }
+  const int64_t e = k.element_size();
+  for (int i = 0; i < 2; ++i) {
+    const Tensor &p = *past[i], &f = *fresh[i];
+    if (f.sizes() != k.sizes() || p.sizes() != past[0]->sizes() || !p.is_contiguous() || f.stride(3) != 1)
+      return false;
+    for (int d = 0; d < 3; ++d)
+      if (f.stride(d) * e % 16 != 0) return false;
+  }
+  const Tensor& p = *past[0];
+  return k.numel() > 0 && p.size(0) == k.size(0) && p.size(2) == k.size(2) && p.size(3) == k.size(3) &&
+         k.size(3) * e % 16 == 0 && k.size(0) <= 65535;
+}
+
+// Key / value caches [B, S, H, D] followed by the new tokens [B, n, H, D] (slices of a packed
+// projection are read in place): two new tensors, by one launch where kv_append_takes says so.  The
+// checks live here because they cost a Python caller more than the launch (15 us against 9 for both).
+std::tuple<Tensor, Tensor> append_kv(const Tensor& past_k, const Tensor& past_v, const Tensor& k,
                                      const Tensor& v) {
-  const Tensor* past[2] = {&past_k, &past_v};
-  const Tensor* fresh[2] = {&k, &v};
-  Tensor out[2];
+  const Tensor* const past[2] = {&past_k, &past_v};
+  const Tensor* const fresh[2] = {&k, &v};
+  if (!kv_append_takes(past, fresh)) return {at::cat({past_k, k}, 1), at::cat({past_v, v}, 1)};
   c10::cuda::CUDAGuard guard(k.device());
   const int64_t B = k.size(0), n = k.size(1), H = k.size(2), D = k.size(3), len = past_k.size(1);
   const int64_t e = k.element_size();
-  TORCH_CHECK(D * e % 16 == 0, "kv_append: heads must be a multiple of 16 bytes");
+  Tensor out[2];
   const void* past_ptr[2];
   const void* fresh_ptr[2];
   void* out_ptr[2];
   int64_t strides[2][3];
   for (int i = 0; i < 2; ++i) {
-    const Tensor &p = *past[i], &f = *fresh[i];
-    TORCH_CHECK(p.is_cuda() && f.is_cuda() && p.dim() == 4 && f.dim() == 4 &&
-                    p.get_device() == k.get_device() && f.get_device() == k.get_device() &&
-                    p.scalar_type() == k.scalar_type() && f.scalar_type() == k.scalar_type(),
-                "kv_append: four [B, S, H, D] CUDA tensors of one type and device required");
-    TORCH_CHECK(p.size(0) == B && p.size(1) == len && p.size(2) == H && p.size(3) == D &&
-                    f.sizes() == k.sizes(), "kv_append: sizes differ");
-    TORCH_CHECK(p.is_contiguous() && f.stride(3) == 1, "kv_append: contiguous cache and heads required");
-    for (int d = 0; d < 3; ++d) {
-      strides[i][d] = f.stride(d) * e;
-      TORCH_CHECK(strides[i][d] % 16 == 0, "kv_append: strides must be multiples of 16 bytes");
-    }
+    for (int d = 0; d < 3; ++d) strides[i][d] = fresh[i]->stride(d) * e;
     out[i] = at::empty({B, len + n, H, D}, k.options());
-    past_ptr[i] = p.data_ptr();
-    fresh_ptr[i] = f.data_ptr();
+    past_ptr[i] = past[i]->data_ptr();
+    fresh_ptr[i] = fresh[i]->data_ptr();
     out_ptr[i] = out[i].data_ptr();
-    TORCH_CHECK((reinterpret_cast<uintptr_t>(past_ptr[i]) | reinterpret_cast<uintptr_t>(fresh_ptr[i])) %
-                        16 == 0, "kv_append: data must be 16-byte aligned");
   }
   slapo::launch_kv_append(past_ptr, fresh_ptr, out_ptr, B, len, n, H, D * e, strides,
                           at::cuda::getCurrentCUDAStream().stream());
@@ -228,7 +247,7 @@ void register_attn_ops(torch::Library& m) {
         &flash_attn_fwd);
   m.def("flash_attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor? kbias, Tensor? rel, bool causal, float scale, float p_drop, Tensor? rng, bool packed_qkv) -> (Tensor, Tensor, Tensor, Tensor)",
         &flash_attn_bwd);
-  m.def("kv_append(Tensor past_k, Tensor past_v, Tensor k, Tensor v) -> (Tensor, Tensor)", &kv_append);
+  m.def("append_kv(Tensor past_k, Tensor past_v, Tensor k, Tensor v) -> (Tensor, Tensor)", &append_kv);
   m.def("rel_bias_fwd(Tensor table, Tensor buckets) -> Tensor", &rel_bias_fwd);
   m.def("rel_bias_bwd(Tensor grad, Tensor buckets, Tensor table) -> Tensor", &rel_bias_bwd);
   m.def("flash_attn_dropout_mask(int B, int H, int Sq, int Sk, float p_drop, Tensor rng) -> Tensor",

@@ -235,35 +235,13 @@ def _transformed(tensors):
         torch._C._functorch.is_functorch_wrapped_tensor(t) for t in tensors)
 
 
-def _append_supported(past_k, past_v, k, v):
-    """The four tensors as one launch takes them: plain CUDA tensors outside of autograd and of
-    functorch / forward-mode transforms, one type, contiguous caches, 16-byte aligned heads."""
-    tensors = (past_k, past_v, k, v)
-    if not all(type(t) is torch.Tensor and t.is_cuda and t.dim() == 4 for t in tensors):
-        return False
-    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
-        return False
-    if _transformed(tensors):
-        return False
-    e = k.element_size()
-    if k.dtype not in (torch.bfloat16, torch.float16, torch.float32) or any(
-            t.dtype != k.dtype or t.device != k.device for t in tensors):
-        return False
-    b, n, h, d = k.shape
-    if v.shape != k.shape or past_v.shape != past_k.shape or n * b * h * d == 0 \
-            or (past_k.shape[0], past_k.shape[2], past_k.shape[3]) != (b, h, d) or d * e % 16:
-        return False
-    return (past_k.is_contiguous() and past_v.is_contiguous()
-            and all(t.stride(3) == 1 and not any(s * e % 16 for s in t.stride()[:3])
-                    for t in (k, v))
-            and not any(t.data_ptr() % 16 for t in tensors) and b <= 65535 and _native_ok(k))
-
-
 def append_kv(past_k, past_v, k, v):
     """Key / value caches ``[B, S, H, D]`` followed by the new tokens ``[B, n, H, D]``: two new
-    tensors.  ``k`` and ``v`` may be slices of a packed projection output, read in place."""
-    if _append_supported(past_k, past_v, k, v):
-        return native.ops().kv_append(past_k, past_v, k, v)
+    tensors.  ``k`` and ``v`` may be slices of a packed projection output, read in place by one
+    kernel; the operator concatenates what that does not take."""
+    if (type(k) is torch.Tensor and _native_ok(k)
+            and torch._C._functorch.peek_interpreter_stack() is None):
+        return native.ops().append_kv(past_k, past_v, k, v)
     return torch.cat((past_k, k), dim=1), torch.cat((past_v, v), dim=1)
 
 

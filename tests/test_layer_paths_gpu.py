@@ -61,7 +61,22 @@ def test_kv_append_leaves_other_inputs_to_cat():
     NF.append_kv(past.detach().transpose(1, 2).contiguous().transpose(1, 2), past.detach(), k, k)
     NF.append_kv(past.detach()[..., :4], past.detach()[..., :4], k[..., :4], k[..., :4])
     NF.append_kv(past.detach().float(), past.detach(), k, k)      # types differ
+    NF.append_kv(past.detach(), past.detach(), k.expand(2, 3, 2, 64)[:, :0], k[:, :0])
+    stacked = torch.stack([k, -k])
+    got = torch.vmap(lambda t: NF.append_kv(past.detach(), past.detach(), t, t)[0])(stacked)
+    assert torch.equal(got[1], torch.cat((past.detach(), -k), dim=1))
+    out, dot = torch.func.jvp(lambda t: NF.append_kv(past.detach(), t, k, k)[1], (past.detach(),),
+                              (past.detach(),))
+    assert torch.equal(dot[:, :9], past.detach()) and (dot[:, 9:] == 0).all()
+    with torch.no_grad(), torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(k, k)
+        out = torch.autograd.forward_ad.unpack_dual(NF.append_kv(past, past, dual, k)[0])
+        assert torch.equal(out.tangent[:, 9:], k)
     assert native.launch_count() == before
+    NF.append_kv(past.detach(), past.detach(), k, k)
+    with torch.no_grad():
+        NF.append_kv(past, past, k, k)
+    assert native.launch_count() == before + 2
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, BF, FP])
