@@ -79,10 +79,11 @@ std::tuple<Tensor, Tensor> flash_attn_fwd(const Tensor& q, const Tensor& k, cons
   return {o, lse};
 }
 
+// keep_words: see flash_bwd_plan (0: its default)
 std::tuple<Tensor, Tensor, Tensor, Tensor> flash_attn_bwd(
     const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o,
     const Tensor& lse, const optional<Tensor>& kbias, const optional<Tensor>& rel, bool causal,
-    double scale, double p_drop, const optional<Tensor>& rng, bool packed_qkv) {
+    double scale, double p_drop, const optional<Tensor>& rng, bool packed_qkv, int64_t keep_words) {
   check_bshd(q, "q"); check_bshd(k, "k"); check_bshd(v, "v");
   TORCH_CHECK(dout.is_contiguous() && o.is_contiguous(), "dout and out must be contiguous");
   c10::cuda::CUDAGuard guard(q.device());
@@ -107,7 +108,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> flash_attn_bwd(
   const bool has_bias = kbias.has_value() && kbias->defined();
   const bool has_rel = rel.has_value() && rel->defined();
   const slapo::FlashBwdPlan plan = slapo::flash_bwd_plan(
-      B, H, Sq, Sk, D, packed_qkv, causal, has_bias, has_rel, static_cast<float>(p_drop));
+      B, H, Sq, Sk, D, packed_qkv, causal, has_bias, has_rel, static_cast<float>(p_drop), keep_words);
   Tensor scratch = at::empty({plan.total()}, q.options().dtype(at::kFloat));
   Tensor drel;
   if (has_rel) drel = at::zeros_like(*rel);
@@ -245,7 +246,7 @@ Tensor rel_bias_bwd(const Tensor& grad, const Tensor& buckets, const Tensor& tab
 void register_attn_ops(torch::Library& m) {
   m.def("flash_attn_fwd(Tensor q, Tensor k, Tensor v, Tensor? kbias, Tensor? rel, bool causal, float scale, float p_drop, Tensor? rng) -> (Tensor, Tensor)",
         &flash_attn_fwd);
-  m.def("flash_attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor? kbias, Tensor? rel, bool causal, float scale, float p_drop, Tensor? rng, bool packed_qkv) -> (Tensor, Tensor, Tensor, Tensor)",
+  m.def("flash_attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor? kbias, Tensor? rel, bool causal, float scale, float p_drop, Tensor? rng, bool packed_qkv, int keep_words=0) -> (Tensor, Tensor, Tensor, Tensor)",
         &flash_attn_bwd);
   m.def("append_kv(Tensor past_k, Tensor past_v, Tensor k, Tensor v) -> (Tensor, Tensor)", &append_kv);
   m.def("rel_bias_fwd(Tensor table, Tensor buckets) -> Tensor", &rel_bias_fwd);

@@ -226,7 +226,7 @@ using FlashFwd = std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const 
 using FlashBwd = std::tuple<Tensor, Tensor, Tensor, Tensor>(
     const Tensor&, const Tensor&, const Tensor&, const Tensor&, const Tensor&, const Tensor&,
     const optional<Tensor>&, const optional<Tensor>&, bool, double, double, const optional<Tensor>&,
-    bool);
+    bool, int64_t);
 
 // Attention on separate q, k, v [B, S, H, D] (q only given: the packed [B, S, H, 3, D], read in
 // place through strided views and its gradient written into one tensor of that layout).
@@ -260,7 +260,7 @@ struct FlashFn : public Function<FlashFn> {
     static auto f = op<FlashBwd>("slapo_b200::flash_attn_bwd");
     auto [dq, dk, dv, drel] =
         f.call(grads[0].contiguous(), q, k, v, s[3], s[4], opt(s[5]), opt(s[6]),
-               ctx->saved_data["causal"].toBool(), ctx->saved_data["scale"].toDouble(), p, rng, packed);
+               ctx->saved_data["causal"].toBool(), ctx->saved_data["scale"].toDouble(), p, rng, packed, /*keep_words=*/0);
     tensor_list out(8);
     out[0] = dq;
     if (!packed) {

@@ -53,8 +53,10 @@ struct FlashBwdPlan {
   int64_t stats, bias, keep, part;
   int64_t total() const { return stats + bias + keep + part; }
 };
+// keep_words: 32-bit words of keep bits at a time (one pair's at least); 0: 1 GB of them, and whether
+// the passes run in one launch, without keep bits, is left to the plan.
 FlashBwdPlan flash_bwd_plan(int B, int H, int Sq, int Sk, int D, bool packed, bool causal,
-                            bool key_bias, bool rel, float p_drop);
+                            bool key_bias, bool rel, float p_drop, int64_t keep_words);
 // dq_row_stride / dkv_row_stride: elements between consecutive (b, s, head) rows of the outputs
 int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
                      const float* lse, const FlashBwdPlan& plan, float* scratch, void* dq, void* dk,

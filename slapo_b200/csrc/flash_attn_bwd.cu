@@ -942,7 +942,7 @@ static int both_q_ctas(int64_t q_items, int64_t k_items, int64_t q_item_tiles, i
 }
 
 FlashBwdPlan flash_bwd_plan(int B, int H, int Sq, int Sk, int D, bool packed, bool causal,
-                            bool key_bias, bool rel, float p_drop) {
+                            bool key_bias, bool rel, float p_drop, int64_t keep_words) {
   FlashBwdPlan s;
   const int64_t rq = round128(Sq), rk = round128(Sk), bh = static_cast<int64_t>(B) * H;
   const int64_t q_tiles = rq / 128, k_tiles = rk / 128;
@@ -960,15 +960,15 @@ FlashBwdPlan flash_bwd_plan(int B, int H, int Sq, int Sk, int D, bool packed, bo
       if (k_tiles - per >= 4) s.splits = static_cast<int>((k_tiles + per - 1) / per);
     }
   }
-  s.q_ctas = bh == 0 ? 0
+  s.q_ctas = bh == 0 || keep_words > 0 ? 0
                      : both_q_ctas(q_tiles * bh * s.splits, k_tiles * bh,
                                    (k_tiles + s.splits - 1) / s.splits, q_tiles, D, causal, rel, drop);
   s.stats = 2 * bh * rq;
   s.bias = key_bias ? B * rk : 0;
-  // keep bits of as many (batch, head) pairs at a time as fit 1 GB (at least one)
   const bool keep = drop && s.q_ctas == 0;
   const int64_t words = rk / 32 * rq;
-  int64_t pairs = keep && words > 0 ? (int64_t(1) << 28) / words : bh;
+  if (keep_words <= 0) keep_words = int64_t(1) << 28;
+  int64_t pairs = keep && words > 0 ? keep_words / words : bh;
   if (pairs < 1) pairs = 1;
   if (pairs > bh) pairs = bh;
   s.pairs = static_cast<int>(pairs);

@@ -111,6 +111,39 @@ def test_flash_attention_paths(b, sq, sk, h, d, dtype, how, p):
         assert err < TOL[dtype], f"{name}: {err:.2e}"
 
 
+@pytest.mark.parametrize("pairs", [1, 3])
+@pytest.mark.parametrize("sq,sk,d,how", [(300, 200, 64, ""), (200, 300, 128, "ckr"), (130, 900, 64, "c")])
+def test_backward_in_several_launches(sq, sk, d, how, pairs):
+    """Keep bits of a few (batch, head) pairs at a time, the last launch with fewer: bit for bit
+    what one launch for all of them gives (relative bias: sums of another order)."""
+    torch.manual_seed(sq + sk)
+    b, h, p = 2, 5, 0.1
+    q, k, v = (torch.randn(b, n, h, d, device="cuda", dtype=BF) for n in (sq, sk, sk))
+    bias = torch.zeros(b, sk, device="cuda").masked_fill(
+        torch.arange(sk, device="cuda") >= sk - 20, -10000.0) if "k" in how else None
+    rel = torch.randn(h, sq + sk - 1, device="cuda") if "r" in how else None
+    ops, causal = native.ops(), "c" in how
+    rng = ops.philox_reserve(b * h * sq * sk)
+    out, lse = ops.flash_attn_fwd(q, k, v, bias, rel, causal, d ** -0.5, p, rng)
+    dout = torch.randn_like(out)
+    words = (-(-sk // 128) * 4) * (-(-sq // 128) * 128)
+
+    def backward(n):
+        before = native.launch_count()
+        got = ops.flash_attn_bwd(dout, q, k, v, out, lse, bias, rel, causal, d ** -0.5, p, rng, False,
+                                 n * words)
+        return got, native.launch_count() - before
+
+    few, n_few = backward(pairs)
+    every, n_every = backward(b * h)
+    assert n_few - n_every == 2 * (-(-b * h // pairs) - 1)
+    assert all(torch.equal(x, y) for x, y in zip(few[:3], every[:3]))
+    torch.testing.assert_close(few[3], every[3], rtol=1e-4, atol=1e-4)
+    drawn, _ = backward(0)               # the passes side by side draw the same decisions
+    assert all(torch.equal(x, y) for x, y in zip(drawn[:3], every[:3]))
+    assert native.ops().device_status() == 0
+
+
 @pytest.mark.parametrize("bh,sk,d,launches", [
     (128, 1500, 128, 1),      # one CTA per SM: a second item per head would wait for the first
     (128, 1500, 64, 2),       # two per SM
