@@ -1,6 +1,6 @@
 // Differentiable front ends of the kernels: the autograd nodes of linear, bias + activation,
-// bias + dropout + residual, the normalisations, flash attention and the cross entropy of one
-// device, as C++ functions.
+// bias + dropout + residual, the normalisations, flash attention and T5's relative bias, as C++
+// functions.
 //
 // A layer of a small model is a few kernels of some microseconds each; a Python autograd function
 // costs about 30 us per direction on the host (argument packing, the interpreter, one operator

@@ -17,9 +17,7 @@ void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 int64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 // ------------------------------------------------------------------------ //
-// Four independent 16-byte loads per thread are issued before any of them is used: with
-// 2048 resident threads per SM a single load each leaves too few bytes in flight to cover the
-// HBM latency at full bandwidth.
+// An activation and its derivative by the type of the data (common.cuh).
 template <int kAct, typename T>
 __device__ __forceinline__ float act_value(float x) {
   if constexpr (sizeof(T) == 2) return act_fwd16<kAct>(x);
@@ -31,6 +29,9 @@ __device__ __forceinline__ float act_slope(float x) {
   else return act_grad(x, kAct);
 }
 
+// Four independent 16-byte loads per thread are issued before any of them is used: with
+// 2048 resident threads per SM a single load each leaves too few bytes in flight to cover the
+// HBM latency at full bandwidth.
 template <int kAct, typename T>
 __global__ void __launch_bounds__(256) bias_act_fwd_kernel(
     const T* __restrict__ x, const T* __restrict__ bias, T* __restrict__ y, int64_t n_vec,

@@ -662,7 +662,7 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float
   p.B = B; p.H = H; p.Sq = Sq; p.Sk = Sk; p.Dr = D; p.O = o; p.lse = lse; p.kbias = kbias; p.rel = rel;
   p.k_steps = (D + 15) / 16;
   p.walk.row_tiles = (Sq + kBlockM - 1) / kBlockM;
-  p.walk.bh0 = 0; p.walk.nbh = B * H; p.walk.H = H;
+  p.walk.bh0 = 0; p.walk.nbh = B * H;
   p.walk.by_cost = causal ? 2 : 0;
   p.splits = scratch != nullptr ? flash_fwd_splits(B, H, Sq, Sk, D) : 1;
   const int key_tiles = (Sk + kBlockN - 1) / kBlockN;

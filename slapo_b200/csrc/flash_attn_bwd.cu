@@ -132,10 +132,10 @@ struct BwdSmem {
   static constexpr int kVec = kKeys ? 1024 + 2048 : 1024;
   static constexpr int kY = 2 * kTile;
   static constexpr int kVecs = kY + kStages * 2 * kTile;
-  static constexpr int kDrel = kVecs + kStages * kVec;       // [8 warps][64] floats
+  static constexpr int kDrel = kVecs + kStages * kVec;       // [8 warps][32] floats
   // per softmax warp, twice: the relative bias of the 32 + 64 - 1 distances of its part of a tile
   static constexpr int kRelFloats = 96;
-  static constexpr int kRel = kDrel + (kKeys ? 8 * 64 * 4 : 0);
+  static constexpr int kRel = kDrel + (kKeys ? 8 * 32 * 4 : 0);
   static constexpr int kBars = kRel + 8 * 2 * kRelFloats * 4;
   static constexpr int kTotal = kBars + 24 * 8 + 1024;
 };
@@ -736,7 +736,7 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
               // Sums along the diagonals key - query = const: the running sum moves one lane up
               // (next key) with every column (next query), so that it stays on its diagonal;
               // what leaves at lane 31 is collected and added to the result 32 at a time.
-              float* buf = reinterpret_cast<float*>(smem + L::kDrel) + (warp - 2) * 64;
+              float* buf = reinterpret_cast<float*>(smem + L::kDrel) + (warp - 2) * 32;
               float* out = p.drel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1);
               const int key0 = tile * 128 + quarter * 32, q0 = col0 + c * 32;
               const int last = p.Sq + p.Sk - 2;
@@ -1027,7 +1027,6 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o,
           kb2, H, Sq, p.Rq, Sk, p.Rk, D, lanes, keep_prob);
   }
   const bool general = kbias != nullptr || rel != nullptr || causal || Sk % 128 != 0;
-  p.walk.H = H;
   const int bh = B * H;
   FlashBwdParams pq = p, pk = p;
   pq.walk.row_tiles = p.Rq / 128;

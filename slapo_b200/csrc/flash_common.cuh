@@ -84,7 +84,6 @@ __device__ __forceinline__ uint32_t keep_bits16(const uint4& kw) {
 struct TileWalk {
   int row_tiles;     // per (batch, head)
   int bh0, nbh;      // range of (batch, head) pairs of this launch
-  int H;
   int by_cost;       // 0 = head-major, 1 = first tile heaviest, 2 = last tile heaviest
   __device__ __forceinline__ int items() const { return row_tiles * nbh; }
   __device__ __forceinline__ void at(int item, int& tile, int& bh_local) const {
