@@ -41,6 +41,15 @@ def _native_ok(*tensors) -> bool:
         "SLAPO_B200_ALLOW_FALLBACK=1 to accept the eager PyTorch path")
 
 
+def _nodes():
+    """The extension's operators, for those with an autograd node of their own.  functorch has no
+    rule for such a node: vmap would run it slice by slice, whatever its ``randomness`` says."""
+    if torch._C._functorch.peek_interpreter_stack() is not None:
+        raise RuntimeError("slapo_b200's CUDA layers do not support functorch transforms "
+                           "(vmap, grad, jvp, ...)")
+    return native.ops()
+
+
 # ---------------------------------------------------------------------- #
 # activations
 def _act_ref(x, act):
@@ -60,7 +69,7 @@ def _act_code(act):
 def bias_act(x, bias, act: str = "gelu"):
     """``act(x + bias)``; act in gelu (erf) / gelu_new (tanh) / relu."""
     if _native_ok(x) and x.shape[-1] % 8 == 0:
-        return native.ops().bias_act(x, bias, _act_code(act))
+        return _nodes().bias_act(x, bias, _act_code(act))
     return _act_ref(x + bias if bias is not None else x, act)
 
 
@@ -98,7 +107,7 @@ def linear_t(x, weight, bias=None):
             and weight.shape[0] % 8 == 0 and weight.shape[1] % 8 == 0 and weight.stride(0) % 8 == 0
             and x.numel() > 0 and os.environ.get("SLAPO_B200_LIBRARY_GEMM", "0") != "1"
             and _native_ok(x)):
-        return native.ops().linear(x, weight, bias, -1, True)
+        return _nodes().linear(x, weight, bias, -1, True)
     out = torch.matmul(x, weight)
     return out if bias is None else out + bias
 
@@ -109,11 +118,11 @@ def linear(x, weight, bias=None, act=None):
     else PyTorch."""
     if gemm_supported(x, weight):
         if act is None or act == "relu":
-            return native.ops().linear(x, weight, bias, -1 if act is None else _RELU, False)
+            return _nodes().linear(x, weight, bias, -1 if act is None else _RELU, False)
         # GeLU is NOT fused: the epilogue warps of a tcgen05 GEMM have a fraction of the SM's
         # FP32 issue rate, and an erf per element made the GEMM 2.5 x slower than running
         # bias_act over the output afterwards
-        return bias_act(native.ops().linear(x, weight, None, -1, False), bias, act)
+        return bias_act(_nodes().linear(x, weight, None, -1, False), bias, act)
     out = F.linear(x, weight, bias)
     return out if act is None else _act_ref(out, act)
 
@@ -131,7 +140,7 @@ def effective_dropout_p(p: float) -> float:
 def bias_dropout_add(x, bias, residual, p: float, training: bool = True):
     """``dropout(x + bias, p) + residual`` (bias / residual may be None)."""
     if _native_ok(x) and training and p > 0.0 and x.shape[-1] % 8 == 0:
-        return native.ops().bias_dropout_add(x, bias, residual, p)
+        return _nodes().bias_dropout_add(x, bias, residual, p)
     out = x + bias if bias is not None else x
     out = F.dropout(out, p, training)
     return out + residual if residual is not None else out
@@ -145,14 +154,14 @@ def bias_dropout(x, bias, p: float, training: bool = True):
 # normalisation
 def layer_norm(x, weight, bias, eps: float = 1e-5):
     if _native_ok(x) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 16384:
-        return native.ops().norm(x, weight, bias, eps, False)
+        return _nodes().norm(x, weight, bias, eps, False)
     return F.layer_norm(x, (x.shape[-1],), weight, bias, eps)
 
 
 def rms_norm(x, weight, eps: float = 1e-6):
     """T5-style RMS norm: no mean subtraction, no bias, fp32 statistics."""
     if _native_ok(x) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 16384:
-        return native.ops().norm(x, weight, None, eps, True)
+        return _nodes().norm(x, weight, None, eps, True)
     var = x.float().pow(2).mean(-1, keepdim=True)
     return (x.float() * torch.rsqrt(var + eps)).to(x.dtype) * weight
 
@@ -164,8 +173,8 @@ def dropout_add_layer_norm(x, bias, residual, weight, ln_bias, p: float, eps: fl
     ``z`` is returned because a pre-LN block needs it as the next residual; a
     post-LN block (BERT) just drops it."""
     if _native_ok(x) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 16384:
-        return native.ops().dropout_add_norm(x, bias, residual, weight, ln_bias,
-                                             p if training else 0.0, eps)
+        return _nodes().dropout_add_norm(x, bias, residual, weight, ln_bias,
+                                         p if training else 0.0, eps)
     z = x + bias if bias is not None else x
     z = F.dropout(z, p, training) + residual
     return F.layer_norm(z, (z.shape[-1],), weight, ln_bias, eps), z

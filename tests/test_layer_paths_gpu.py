@@ -163,7 +163,6 @@ def test_gelu_extremes(dtype):
 def test_dropout_add_norm_outputs_without_a_consumer():
     x, r = (torch.randn(5, 64, device="cuda", dtype=BF, requires_grad=True) for _ in range(2))
     w, b = (torch.randn(64, device="cuda", dtype=BF, requires_grad=True) for _ in range(2))
-    grads = []
     for pick in ((0,), (1,), (0, 1)):
         out = NF.dropout_add_layer_norm(x, None, r, w, b, 0.0, 1e-5, True)
         xf, rf, wf, bf = (t.detach().double().requires_grad_(True) for t in (x, r, w, b))
@@ -177,5 +176,3 @@ def test_dropout_add_norm_outputs_without_a_consumer():
             t = torch.zeros_like(g, dtype=torch.float64) if t is None else t
             scale = t.norm().clamp(min=t.numel() ** 0.5)
             assert ((g.double() - t).norm() / scale).item() < 2.0 ** -6
-        grads.append(got)
-    assert len(grads) == 3
