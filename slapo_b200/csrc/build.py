@@ -100,10 +100,13 @@ def build(verbose: bool = False, force: bool = False) -> str:
             for cmd, out in log:
                 fh.write(cmd + "\n" + out + "\n")
     if jobs or force or _newer(objs, OUT):
-        # link beside the target and rename: a reader never sees a half-written library
+        # link beside the target and rename: a reader never sees a half-written library.
+        # libstdc++ is named by its file: a compiler that finds only the archive links a second copy
+        # of the C++ runtime, whose streams are never set up, and an error message with a number in
+        # it ends the process.
         tmp = OUT + ".tmp"
         link = [cxx, "-shared", "-o", tmp] + objs + [
-            "-L", torch_lib, "-L", os.path.join(_cuda_home(), "lib64"),
+            "-l:libstdc++.so.6", "-L", torch_lib, "-L", os.path.join(_cuda_home(), "lib64"),
             "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-lcudart",
             f"-Wl,-rpath,{torch_lib}"]
         _run(link, log)

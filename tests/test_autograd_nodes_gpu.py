@@ -98,3 +98,11 @@ def test_modes_without_a_rule_are_refused(name):
     with pytest.raises(RuntimeError):
         torch.vmap(lambda t: NF.bias_dropout_add(t, None, None, 0.5))(torch.randn(2, 8, 64, device="cuda"))
     assert native.ops().device_status() == 0
+
+
+def test_a_refusal_in_the_backward_thread_is_an_error():
+    """Weight gradients contract over the tokens, which the GEMM takes in eights."""
+    w = _leaf(48, 64)
+    y = NF.linear(torch.randn(12, 64, device="cuda", dtype=BF), w)
+    with pytest.raises(RuntimeError, match="gemm: launch refused"):
+        y.sum().backward()
