@@ -652,6 +652,7 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float
   // any head dimension up to 128 that is a multiple of 8 (16-byte rows for TMA): the kernels
   // work on 64- or 128-wide tiles whose columns beyond D are zero-filled by the tile loads
   if (D < 8 || D > 128 || D % 8 != 0) return 1;
+  if (B <= 0 || H <= 0 || Sq <= 0 || Sk <= 0) return 1;     // (no tensor map without an address)
   const int Dt = D <= 64 ? 64 : 128;
   CUtensorMap tq, tk, tv;
   if (!make_tmap_bshd(&tq, q, B, Sq, H, D, q_strides[0], q_strides[1], q_strides[2], 128, bf16) ||

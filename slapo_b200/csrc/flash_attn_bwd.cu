@@ -855,7 +855,9 @@ static int launch_bwd(void (*kernel)(P...), int ctas, int smem, bool early, cuda
   cfg.attrs = &attr;
   cfg.numAttrs = early ? 1 : 0;
   count_launch();
-  return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess ? 0 : 4;
+  if (cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess) return 0;
+  (void)cudaGetLastError();
+  return 4;
 }
 
 template <int D, bool kKeys, bool kGeneral, typename T>
@@ -951,7 +953,7 @@ FlashBwdPlan flash_bwd_plan(int B, int H, int Sq, int Sk, int D, bool packed, bo
   // chain of tiles, where that takes four tiles off its own.  (2 x 60 queries x 2000 keys x 8 x 128:
   // 72 -> 48 us for the whole backward.)
   s.splits = 1;
-  if (!packed && bh > 0 && k_tiles > q_tiles) {
+  if (!packed && bh > 0 && q_tiles > 0 && k_tiles > q_tiles) {
     int64_t n = sm_count() / (q_tiles * bh);
     const int64_t most = (k_tiles + q_tiles - 1) / q_tiles;
     if (n > most) n = most;
@@ -984,7 +986,8 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o,
                      const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
                      float scale, int causal, float p_drop, PhiloxArgs rng, bool bf16, int* status,
                      cudaStream_t stream) {
-  if (D < 8 || D > 128 || D % 8 != 0) return 1;
+  if (D < 8 || D > 128 || D % 8 != 0 || B > 65535) return 1;
+  if (B <= 0 || H <= 0 || Sq <= 0 || Sk <= 0) return 1;
   CUtensorMap tq, tk, tv, tdo;
   const int64_t do_strides[3] = {static_cast<int64_t>(Sq) * H * D, static_cast<int64_t>(H) * D, D};
   if (!make_tmap_bshd(&tq, q, B, Sq, H, D, q_strides[0], q_strides[1], q_strides[2], 128, bf16) ||
@@ -1025,6 +1028,7 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o,
       flash_bwd_stats_kernel<__half><<<grid, 256, 0, stream>>>(
           static_cast<const __half*>(dout), static_cast<const __half*>(o), lse, nlse, ndelta, kbias,
           kb2, H, Sq, p.Rq, Sk, p.Rk, D, lanes, keep_prob);
+    if (cudaGetLastError() != cudaSuccess) return 4;
   }
   const bool general = kbias != nullptr || rel != nullptr || causal || Sk % 128 != 0;
   const int bh = B * H;

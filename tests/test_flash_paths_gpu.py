@@ -144,6 +144,18 @@ def test_backward_in_several_launches(sq, sk, d, how, pairs):
     assert native.ops().device_status() == 0
 
 
+@pytest.mark.parametrize("b,sq,sk", [(1, 0, 700), (1, 700, 0), (0, 64, 64), (65536, 1, 1)])
+def test_empty_and_oversized_calls_are_refused(b, sq, sk):
+    q, k = (torch.zeros(b, n, 2, 64, device="cuda", dtype=BF) for n in (sq, sk))
+    lse = torch.zeros(b, 2, sq, device="cuda")
+    if q.numel() == 0 or k.numel() == 0:
+        with pytest.raises(RuntimeError, match="refused"):
+            native.ops().flash_attn_fwd(q, k, k, None, None, False, 0.125, 0.0, None)
+    with pytest.raises(RuntimeError, match="refused"):
+        native.ops().flash_attn_bwd(q, q, k, k, q, lse, None, None, False, 0.125, 0.1,
+                                    native.ops().philox_reserve(8), False)
+
+
 @pytest.mark.parametrize("bh,sk,d,launches", [
     (128, 1500, 128, 1),      # one CTA per SM: a second item per head would wait for the first
     (128, 1500, 64, 2),       # two per SM
