@@ -1,41 +1,42 @@
 // Flash attention backward on tcgen05 / TMEM (sm_100a).
 //
-// Two passes of one kernel, each with the same shape as the forward: a work item keeps a
-// 128-row tile of two tensors (X1, X2) in shared memory, streams 128-row tiles of two others
-// (Y1, Y2) and accumulates in tensor memory - nothing is added up between work items.
+// Two passes of one kernel: a work item keeps a 128-row tile of two tensors (X1, X2) in shared
+// memory, streams half tiles (64 rows) of two others (Y1, Y2) and accumulates in tensor memory -
+// nothing is added up between work items.
 //
 //   pass      rows      X1  X2   streams   Y1  Y2     accumulators
 //   dQ        queries   Q   dO   keys      K   V      dQ += dS K
 //   dK / dV   keys      K   V    queries   Q   dO     dK += dS^T Q     dV += P^T dO
 //
-// Per tile, with rows on the TMEM lanes:
+// Per half tile, with rows on the TMEM lanes:
 //   tensor core   S = X1 Y1^T ,  dP = X2 Y2^T                       (fp32 in TMEM)
-//   8 warps       p = exp2(s - lse) ;  ds = p * (dp - delta)        (a row and half the columns
-//                 per thread; dropout replayed), P and dS written back to TMEM as 16 bit
+//   4 warps       p = exp2(s - lse) ;  ds = p * (dp - delta)        (a row per thread; dropout
+//                 replayed), P and dS written back to TMEM as 16 bit
 //   tensor core   accumulators += dS Y1 , P Y2                      (A operand from TMEM)
 // P and dS never pass through shared memory, and no transpose is needed: the two passes form
 // S with its rows where they want them.
 //
-// The order of the products keeps the tensor core and the softmax warps apart:
-//   tensor   ... S (t+1)   P Y2 (t)      dP (t+1)   dS Y1 (t) ...
-//   softmax      dS (t)          P (t+1)          dS (t+1)
-// (D = 128: each pair the other way round).
-// CTAs are persistent; the loads and the first S of the next work item run under the last tile of
-// this one, and its accumulators are read out after the first P of the next.  The passes run side by
-// side in one launch where that fills the GPU better (both_q_ctas); the keys of few queries are split
-// over work items.
+// Two groups of four softmax warps take the half tiles in turn, each with its own barriers, so that one
+// group's exponentials run under the other's waits, loads and conversions.  Loads, S, dP and the
+// accumulating products have a thread each, which go through the sequence at their own pace, and four
+// more warps read finished accumulators out under the next work item.  CTAs are persistent.  The
+// passes run side by side in one launch where that fills the GPU better (both_q_ctas); the keys of few
+// queries are split over work items.
+//
+// What that is for, measured by clocks in the kernel: one thread that issued all products under
+// `lane == 0` took 400 - 700 cycles for the four to eight of each kind (under elect.sync half of
+// that, their operands in uniform registers) and was what a tile of 128 waited for, with both halves
+// of its columns in the same phase.  Bound now for D = 64: the chain of a half tile within its group, 2200 -
+// 3000 cycles, of which exp2 alone needs 512 for each of the two; for D = 128 the products (64 cycles
+// each, 20 or 24 to a half tile: those of 64 columns take as long as those of 128).
+// Measured (all kernels of the backward; whole tiles, one issuing thread -> now): 32 x 512 x 16 heads of
+// 64, p 0.1: 315 -> 261 us; 4 x 2048 x 16 x 128 causal: 400 -> 305; 4 x 1000 x 32 x 80 causal with key bias: 227 ->
+// 183; 8 x 512 x 16 x 64 with T5's bias, key bias and p 0.1: 155 -> 143; 4 x 2048 x 16 x 128: 553 -> 421; 1 x 512 x
+// 16 x 64, p 0.1: 26 -> 25.
 //
 // A single pass (5 products per tile instead of 7) has to add up dQ over the key tiles: one fp32
 // partial of dQ per key tile written and read again was most of its time (BERT-large, 32 x 512
-// tokens x 16 heads of 64: 268 MB each way).  Bound now: the chain of a tile (product, TMEM load,
-// exp2, pack, TMEM store, barrier, product); exp2 alone needs 1024 cycles per tile and pass.  Twice
-// the softmax warps on half the columns each changed nothing (181 -> 185 and 144 -> 153 us).
-// Measured (all kernels of the backward, a single pass with dQ partials -> now): 32 x 512 x 16 heads
-// of 64, p 0.1: 366 -> 316 us; 4 x 2048 x 16 x 128 causal: 652 -> 398 us; 4 x 1000 x 32 x 80 causal with key
-// bias: 353 -> 237 us; 8 x 512 x 16 x 64 with T5's bias, key bias and p 0.1: 159 -> 160 us; 1 x 512 x 16 x
-// 64, p 0.1: 31 -> 25 us.  Where one key tile meets one to two query tiles of 100 - 500 heads, the single
-// pass had half the work items: 8 x 128 x 16 x 128: 24 -> 27 us, 16 x 48 x 16 x 64: 25 -> 27; also 2 x 60
-// queries x 2000 keys x 8 x 128: 33 -> 45.
+// tokens x 16 heads of 64: 268 MB each way).
 //
 // With dropout the dQ pass draws the keep decisions (16 keys of a query row per Philox call, as
 // in the forward) and leaves them as one bit each, [B H][key / 32][query] words, for the dK / dV
@@ -123,25 +124,46 @@ __global__ void __launch_bounds__(256) flash_bwd_stats_kernel(
   }
 }
 
+// Registers per thread of the warpgroups: issuing, softmax (two), reading out; together the 128 per
+// thread that 512 threads are launched with.
+constexpr int kRegsIssue = 80, kRegsSoftmax = 168, kRegsOut = 96;
+static_assert(kRegsIssue + 2 * kRegsSoftmax + kRegsOut <= 4 * 128, "more registers than the block has");
+
 template <int D, bool kKeys>
 struct BwdSmem {
-  static constexpr int kTile = 128 * D * 2;
-  static constexpr int kStages = D == 64 ? 3 : 2;
-  // per stage: Y1, Y2 and the column vectors: nlse, ndelta (512 B each) and four rows of keep
-  // bits (2 KB) for the dK / dV pass, the key bias (512 B) for the dQ pass
-  static constexpr int kVec = kKeys ? 1024 + 2048 : 1024;
-  static constexpr int kY = 2 * kTile;
-  static constexpr int kVecs = kY + kStages * 2 * kTile;
-  static constexpr int kDrel = kVecs + kStages * kVec;       // [8 warps][32] floats
-  // per softmax warp, twice: the relative bias of the 32 + 64 - 1 distances of its part of a tile
+  static constexpr int kTile = 128 * D * 2;          // X1, X2
+  static constexpr int kHalfTile = 64 * D * 2;       // Y1, Y2
+  static constexpr int kX = D == 64 ? 2 : 1;         // X tiles: this item's (and the next one's)
+  // Y1 is held from S to the accumulating product a step later, Y2 is not
+  static constexpr int kY1 = D == 64 ? 6 : 5, kY2 = 4;
+  // with each Y1 its column vectors: nlse, ndelta (256 B each) and four rows of keep bits (1 KB)
+  // for the dK / dV pass, the key bias (256 B) for the dQ pass
+  static constexpr int kVec = kKeys ? 512 + 1024 : 256;
+  static constexpr int kX2 = kX * kTile;
+  static constexpr int kY1At = 2 * kX * kTile;
+  static constexpr int kY2At = kY1At + kY1 * kHalfTile;
+  static constexpr int kVecs = kY2At + kY2 * kHalfTile;
+  static constexpr int kDrel = kVecs + kY1 * kVec;           // [8 warps][32] floats
+  // per softmax warp, twice: the relative bias of the 32 + 64 - 1 distances of its half tile
   static constexpr int kRelFloats = 96;
   static constexpr int kRel = kDrel + (kKeys ? 8 * 32 * 4 : 0);
   static constexpr int kBars = kRel + 8 * 2 * kRelFloats * 4;
-  static constexpr int kTotal = kBars + 24 * 8 + 1024;
+  static constexpr int kTotal = kBars + 48 * 8 + 1024;
 };
 
-// 10 warps: TMA, MMA and 8 softmax warps; warps w and w + 4 share a quarter of the TMEM lanes
-// (rows) and split the tile's columns in halves.
+// Position in a ring of N slots
+template <int N>
+struct Ring {
+  int slot = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void step() {
+    if (++slot == N) { slot = 0; phase ^= 1; }
+  }
+};
+
+// 16 warps in four warpgroups: one thread each of warps 0 - 3 for the loads and the products; two
+// softmax groups (warps 4 - 7 and 8 - 11), one row per thread, which take the half tiles in turn; and
+// the warps that read the accumulators out (12 - 15).
 // kKeys: the dK / dV pass.  kGeneral: key bias, relative bias, causal mask or ragged lengths.
 // kDraw: with dropout the dK / dV pass draws the keep decisions itself, and the dQ pass leaves none.
 // CTA `cta` of `ctas` that run the pass.
@@ -150,95 +172,98 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
                                          const CUtensorMap& tm_y1, const CUtensorMap& tm_y2,
                                          const FlashBwdParams& p, const int cta, const int ctas) {
   using L = BwdSmem<D, kKeys>;
-  constexpr int kTileBytes = L::kTile;
-  constexpr int kBlkBytes = 128 * 128;
+  constexpr int kTileBytes = L::kTile, kHalfBytes = L::kHalfTile;
+  constexpr int kBlkX = 128 * 128, kBlkY = 64 * 128;     // [rows x 64 columns], swizzled
   constexpr int kDBlocks = D / 64;
-  constexpr int kStages = L::kStages;
+  constexpr int kX = L::kX, kY1 = L::kY1, kY2 = L::kY2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* s_x1 = smem;
-  uint8_t* s_x2 = smem + kTileBytes;
-  uint8_t* s_y = smem + L::kY;            // [stage][Y1 | Y2]
-  uint8_t* s_vec = smem + L::kVecs;       // [stage][kVec]
+  uint8_t* s_vec = smem + L::kVecs;       // [Y1 slot][kVec]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
-  uint64_t* x1_full = bars;
-  uint64_t* x1_empty = bars + 1;
-  uint64_t* x2_full = bars + 2;
-  uint64_t* x2_empty = bars + 3;
-  uint64_t* y_full = bars + 4;      // kStages (<= 3)
-  uint64_t* y_empty = bars + 7;     // kStages
-  uint64_t* s_full = bars + 10;
-  uint64_t* p_ready = bars + 11;    // 8 warps: S has been read (and P written over it)
-  uint64_t* dp_full = bars + 12;
-  uint64_t* ds_ready = bars + 13;   // 8 warps: dS written over dP
-  uint64_t* acc_full = bars + 14;
-  uint64_t* acc_free = bars + 15;   // 8 warps
-  uint64_t* a1_done = bars + 16;    // the tensor core has read dS / P of a tile
-  uint64_t* a2_done = bars + 17;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+  uint64_t* x1_full = bars;           // kX each (<= 2)
+  uint64_t* x1_empty = bars + 2;
+  uint64_t* x2_full = bars + 4;
+  uint64_t* x2_empty = bars + 6;
+  uint64_t* y1_full = bars + 8;       // kY1 (<= 6)
+  uint64_t* y1_empty = bars + 14;
+  uint64_t* y2_full = bars + 20;      // kY2 (4)
+  uint64_t* y2_empty = bars + 24;
+  uint64_t* s_full = bars + 28;       // one per softmax group from here on
+  uint64_t* p_ready = bars + 30;      // 4 warps: S has been read (and P written)
+  uint64_t* dp_full = bars + 32;
+  uint64_t* ds_ready = bars + 34;     // 4 warps: dS written
+  uint64_t* a1_done = bars + 36;      // the tensor core has read dS / P of a half tile
+  uint64_t* a2_done = bars + 38;
+  uint64_t* acc_full = bars + 40;     // kAcc (<= 2)
+  uint64_t* acc_free = bars + 42;     // 4 warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 44);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int diag = p.Sk - p.Sq;
   constexpr uint32_t kTmemCols = 512;
-  constexpr uint32_t kColS = 0, kColDP = 128, kColA1 = 256, kColA2 = 256 + D;
-  // P and dS get columns of their own where 512 suffice; for D = 128 the dK / dV pass writes them
-  // over S and dP (each warp over the half it has read: halves start 64 columns apart).
-  // Products of one thread run in order for ONE accumulator only: a product that overwrites the
-  // A operand of the one before it has to wait for that one's completion.
+  // S and dP of the two groups' half tiles, 64 columns each.  dS is written over dP, whose next product
+  // waits for the one that uses dS up.  P has columns of its own where they suffice (a group needs
+  // its next S right after this dS: 122 -> 119 us for dK / dV of 32 x 512 x 16 heads of 64), for D = 128 it is
+  // written over S likewise.  Accumulators: two sets where they fit, so that an item's are read out
+  // under the next one's products.
   constexpr bool kOver = kKeys && D == 128;
-  constexpr uint32_t kColP = kOver ? kColS : 384, kColDS = kOver ? kColDP : (kKeys ? 448 : 256 + D);
-  constexpr uint32_t kHalf = kOver ? 64 : 32;    // columns from one half of P / dS to the other
-  // With columns of their own, the next tile's S and dP need only that the softmax warps have read
-  // this tile's, and those warps wait for them: they go before the accumulating products.  That
-  // took the passes at D = 64 from 181 + 144 to 165 + 138 us (32 x 512 x 16 heads, p 0.1); at
-  // D = 128 the products are twice as long and two stages leave the loads less slack, and the dQ
-  // pass lost (170 -> 183 us at 4 x 2048 x 16, causal).
-  constexpr bool kFirst = D == 64;
+  constexpr uint32_t kColS = 0, kColDP = 128, kColA1 = 256, kColA2 = 256 + D;
+  constexpr uint32_t kColP = kOver ? kColS : 384, kPGroup = kOver ? 64 : 32;
+  constexpr uint32_t kAccCols = D;        // from one set to the next
+  constexpr int kAcc = kKeys ? 1 : 2;
   const int items = p.walk.items() * (kKeys ? 1 : p.splits);
   const bool drop = p.thr7 != 0;
 
-  // row tile and (batch, head) of a work item, its first streamed tile and how many (at least one: a
-  // row tile or a split that nothing reaches still has its zeros written)
+  // row tile and (batch, head) of a work item, its first streamed half tile and how many (at least
+  // one: a row tile or a split that nothing reaches still has its zeros written)
   auto item_at = [&](int item, int& tile, int& bhl, int& first) {
     const int unit = kKeys || p.splits == 1 ? item : item / p.splits;
     p.walk.at(unit, tile, bhl);
     int n;
+    first = 0;
     if constexpr (kKeys) {
-      const int q_tiles = p.Rq >> 7;
-      first = 0;
-      if (p.causal) first = min(max(0, (tile * 128 - diag) / 128), q_tiles - 1);
-      n = q_tiles - first;
+      n = (p.Sq + 63) >> 6;
+      if (p.causal) first = min(max(0, tile * 128 - diag) >> 6, n - 1);
+      n -= first;
     } else {
-      first = 0;
-      n = p.Rk >> 7;
-      if (p.causal) n = max(1, min(n, (min(p.Sk, tile * 128 + 128 + diag) + 127) / 128));
+      n = (p.Sk + 63) >> 6;
+      if (p.causal) n = min(n, (min(tile * 128 + 128, p.Sq) + diag + 63) >> 6);
       if (p.splits > 1) {
-        first = (item - unit * p.splits) * p.tiles_per_split;
-        n = max(1, min(p.tiles_per_split, n - first));
+        first = (item - unit * p.splits) * p.tiles_per_split * 2;
+        n = min(p.tiles_per_split * 2, n - first);
       }
+      n = max(1, n);
     }
     return n;
   };
 
   if (threadIdx.x == 0) {
-    tc::mbar_init(x1_full, 1);
-    tc::mbar_init(x1_empty, 1);
-    tc::mbar_init(x2_full, 1);
-    tc::mbar_init(x2_empty, 1);
-    for (int s = 0; s < 3; ++s) {
-      tc::mbar_init(&y_full[s], 1);
-      tc::mbar_init(&y_empty[s], 1);
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&x1_full[i], 1);
+      tc::mbar_init(&x1_empty[i], 1);
+      tc::mbar_init(&x2_full[i], 1);
+      tc::mbar_init(&x2_empty[i], 1);
+      tc::mbar_init(&s_full[i], 1);
+      tc::mbar_init(&p_ready[i], 4);
+      tc::mbar_init(&dp_full[i], 1);
+      tc::mbar_init(&ds_ready[i], 4);
+      tc::mbar_init(&a1_done[i], 1);
+      tc::mbar_init(&a2_done[i], 1);
     }
-    tc::mbar_init(s_full, 1);
-    tc::mbar_init(p_ready, 8);
-    tc::mbar_init(dp_full, 1);
-    tc::mbar_init(ds_ready, 8);
-    tc::mbar_init(acc_full, 1);
-    tc::mbar_init(acc_free, 8);
-    tc::mbar_init(a1_done, 1);
-    tc::mbar_init(a2_done, 1);
+    for (int i = 0; i < kY1; ++i) {
+      tc::mbar_init(&y1_full[i], 1);
+      tc::mbar_init(&y1_empty[i], 1);
+    }
+    for (int i = 0; i < kY2; ++i) {
+      tc::mbar_init(&y2_full[i], 1);
+      tc::mbar_init(&y2_empty[i], kKeys ? 2 : 1);      // dP and, of two threads, dV's product
+    }
+    for (int i = 0; i < kAcc; ++i) {
+      tc::mbar_init(&acc_full[i], 1);
+      tc::mbar_init(&acc_free[i], 4);
+    }
     *abort_flag = 0;
     tc::fence_barrier_init();
   }
@@ -254,334 +279,372 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
   pdl_wait();
   pdl_launch();
 
-  if (warp == 0) {
-    if (lane == 0) {
-      tc::tma_prefetch_desc(&tm_x1);
-      tc::tma_prefetch_desc(&tm_x2);
-      tc::tma_prefetch_desc(&tm_y1);
-      tc::tma_prefetch_desc(&tm_y2);
-      const bool load_keep = !kDraw && drop;
-      const uint32_t vec_bytes = kKeys ? 1024u + (load_keep ? 2048u : 0u) : (p.kb2 != nullptr ? 512u : 0u);
-      bool ok = true;
-      int t = 0, w = 0;
-      for (int item = cta; item < items && ok; item += ctas, ++w) {
-        int tile, bhl, first;
-        const int n = item_at(item, tile, bhl, first);
-        const int bh = p.walk.bh0 + bhl;
-        const int batch = bh / p.H, head = bh - batch * p.H;
-        auto load_y = [&](int j) -> bool {
-          const int st = t % kStages;
-          const uint32_t ph = ((t / kStages) & 1) ^ 1;
-          if (!tc::mbar_wait(&y_empty[st], ph, abort_flag)) return false;
-          // (the stage's column vectors were read before ds_ready, which y_empty follows)
-          tc::mbar_arrive_expect_tx(&y_full[st], 2 * kTileBytes + vec_bytes);
-          const int s0 = (first + j) * 128;
-          uint8_t* y = s_y + st * 2 * kTileBytes;
-#pragma unroll
-          for (int d = 0; d < kDBlocks; ++d)
-            tc::tma_load_4d(y + d * kBlkBytes, &tm_y1, &y_full[st], d * 64, head, s0, batch);
-#pragma unroll
-          for (int d = 0; d < kDBlocks; ++d)
-            tc::tma_load_4d(y + kTileBytes + d * kBlkBytes, &tm_y2, &y_full[st], d * 64, head, s0,
-                            batch);
-          uint8_t* v = s_vec + st * L::kVec;
-          if constexpr (kKeys) {
-            tc::bulk_load(v, p.nlse + static_cast<int64_t>(bh) * p.Rq + s0, 512, &y_full[st]);
-            tc::bulk_load(v + 512, p.ndelta + static_cast<int64_t>(bh) * p.Rq + s0, 512, &y_full[st]);
-            if (load_keep)
-#pragma unroll
-              for (int r = 0; r < 4; ++r)
-                tc::bulk_load(v + 1024 + r * 512,
-                              p.keep + (static_cast<int64_t>(bhl) * (p.Rk >> 5) + tile * 4 + r) * p.Rq + s0,
-                              512, &y_full[st]);
-          } else {
-            if (vec_bytes != 0)
-              tc::bulk_load(v, p.kb2 + static_cast<int64_t>(batch) * p.Rk + s0, 512, &y_full[st]);
-          }
-          return true;
-        };
-        if (!tc::mbar_wait(x1_empty, (w & 1) ^ 1, abort_flag)) { ok = false; break; }
-        tc::mbar_arrive_expect_tx(x1_full, kTileBytes);
-#pragma unroll
-        for (int d = 0; d < kDBlocks; ++d)
-          tc::tma_load_4d(s_x1 + d * kBlkBytes, &tm_x1, x1_full, d * 64, head, tile * 128, batch);
-        if (!load_y(0)) { ok = false; break; }
-        ++t;
-        if (!tc::mbar_wait(x2_empty, (w & 1) ^ 1, abort_flag)) { ok = false; break; }
-        tc::mbar_arrive_expect_tx(x2_full, kTileBytes);
-#pragma unroll
-        for (int d = 0; d < kDBlocks; ++d)
-          tc::tma_load_4d(s_x2 + d * kBlkBytes, &tm_x2, x2_full, d * 64, head, tile * 128, batch);
-        for (int j = 1; j < n; ++j, ++t)
-          if (!load_y(j)) { ok = false; break; }
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t x1_addr = tc::smem_u32(s_x1), x2_addr = tc::smem_u32(s_x2);
-      // S / dP of tile t, which belongs to this CTA's w-th item
-      auto scores = [&](uint32_t col, uint32_t a_addr, uint32_t b_addr) {
+  if (warp < 4) {
+    tc::regs_dec<kRegsIssue>();
+    if (tc::elect_one()) {
+      // Four threads, each of which goes through the half tiles at its own pace: loads, S, dP and the
+      // accumulating products.  One thread for all products was what a half tile waited for: issuing
+      // takes it 40 - 50 cycles a product or commit and 80 a wait.
+      constexpr uint32_t kDescHi = tc::smem_desc_hi(1024);
+      constexpr uint32_t kXStep = kTileBytes >> 4, kYStep = kHalfBytes >> 4;
+      // S / dP of a half tile (64 streamed rows); x, y: low descriptor words
+      auto scores = [&](uint32_t col, uint32_t x, uint32_t y) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
-          if (kk < p.k_steps) {
-            const uint32_t off = (kk >> 2) * kBlkBytes + (kk & 3) * 32;
-            tc::umma_f16(tmem_base + col, tc::smem_desc(a_addr + off, 16, 1024),
-                         tc::smem_desc(b_addr + off, 16, 1024), p.idesc_s, kk != 0 ? 1u : 0u);
-          }
+          if (kk < p.k_steps)
+            tc::umma_f16(tmem_base + col,
+                         tc::smem_desc_words(x + (((kk >> 2) * kBlkX + (kk & 3) * 32) >> 4), kDescHi),
+                         tc::smem_desc_words(y + (((kk >> 2) * kBlkY + (kk & 3) * 32) >> 4), kDescHi),
+                         p.idesc_s, kk != 0 ? 1u : 0u);
         }
       };
-      // accumulator += [128 rows x 128 streamed] 16-bit tile in TMEM times Y
-      auto accumulate = [&](uint32_t col, uint32_t a_col, uint32_t y_addr, bool fresh) {
+      // accumulator += [128 rows x 64 streamed] 16-bit tile in TMEM times Y
+      auto accumulate = [&](uint32_t col, uint32_t a_col, uint32_t y, bool fresh) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          tc::umma_f16_ts(tmem_base + col, tmem_base + a_col + (kk >> 2) * kHalf + (kk & 3) * 8,
-                          tc::smem_desc(y_addr + kk * 2048, kBlkBytes, 1024), p.idesc_acc,
+        for (int kk = 0; kk < 4; ++kk)
+          tc::umma_f16_ts(tmem_base + col, tmem_base + a_col + kk * 8,
+                          tc::smem_desc_words(y + ((kk * 2048) >> 4), kDescHi), p.idesc_acc,
                           (fresh && kk == 0) ? 0u : 1u);
       };
-      auto issue_s = [&](int t, int w, bool first, bool last) -> bool {
-        const int st = t % kStages;
-        if (first && !tc::mbar_wait(x1_full, w & 1, abort_flag)) return false;
-        if (!tc::mbar_wait(&y_full[st], (t / kStages) & 1, abort_flag)) return false;
-        tc::fence_after_sync();
-        scores(kColS, x1_addr, tc::smem_u32(s_y + st * 2 * kTileBytes));
-        tc::umma_commit(s_full);
-        if (last) tc::umma_commit(x1_empty);
-        return true;
-      };
-      auto issue_dp = [&](int t, int w, bool first, bool last) -> bool {
-        const int st = t % kStages;
-        if (first && !tc::mbar_wait(x2_full, w & 1, abort_flag)) return false;
-        tc::fence_after_sync();
-        scores(kColDP, x2_addr, tc::smem_u32(s_y + st * 2 * kTileBytes + kTileBytes));
-        tc::umma_commit(dp_full);
-        if (last) tc::umma_commit(x2_empty);
-        return true;
-      };
-      auto n_of = [&](int item) {
-        if (item >= items) return 0;
-        int tile, bhl, first;
-        return item_at(item, tile, bhl, first);
-      };
       bool ok = true;
-      int t = 0, w = 0, item = cta;
-      int n = n_of(item);
-      if (n > 0) ok = issue_s(0, 0, true, n == 1) && issue_dp(0, 0, true, n == 1);
-      while (item < items && ok) {
-        const int next_item = item + ctas;
-        const int next_n = n_of(next_item);
-        for (int j = 0; j < n; ++j, ++t) {
-          const int st = t % kStages;
-          const uint32_t y_addr = tc::smem_u32(s_y + st * 2 * kTileBytes);
-          const bool same = j + 1 < n, more = same || next_n > 0;
-          const bool next_last = same ? j + 2 == n : next_n == 1;
-          if (!tc::mbar_wait(p_ready, t & 1, abort_flag)) { ok = false; break; }
-          const int next_w = same ? w : w + 1;
-          if (kFirst && more && !issue_s(t + 1, next_w, !same, next_last)) { ok = false; break; }
-          if constexpr (kKeys) {
-            // the accumulators of the item before have been read out
-            if (j == 0 && !tc::mbar_wait(acc_free, (w & 1) ^ 1, abort_flag)) { ok = false; break; }
-            tc::fence_after_sync();
-            accumulate(kColA2, kColP, y_addr + kTileBytes, j == 0);
-            tc::umma_commit(a2_done);
-            if (kOver && more && !tc::mbar_wait(a2_done, t & 1, abort_flag)) { ok = false; break; }
+      if (warp == 0) {
+        // ------------------------------ loads ------------------------------
+        tc::tma_prefetch_desc(&tm_x1);
+        tc::tma_prefetch_desc(&tm_x2);
+        tc::tma_prefetch_desc(&tm_y1);
+        tc::tma_prefetch_desc(&tm_y2);
+        const bool load_keep = kKeys && !kDraw && drop;
+        const uint32_t vec_bytes = kKeys ? 512u + (load_keep ? 1024u : 0u) : (p.kb2 != nullptr ? 256u : 0u);
+        Ring<kX> x;
+        Ring<kY1> r1;
+        Ring<kY2> r2;
+        for (int item = cta; item < items && ok; item += ctas, x.step()) {
+          int tile, bhl, first;
+          const int n = item_at(item, tile, bhl, first);
+          const int bh = p.walk.bh0 + bhl;
+          const int batch = bh / p.H, head = bh - batch * p.H;
+          auto load_x = [&](const CUtensorMap* tm, uint64_t* full, uint64_t* empty, int at) -> bool {
+            if (!tc::mbar_wait(&empty[x.slot], x.phase ^ 1, abort_flag)) return false;
+            tc::mbar_arrive_expect_tx(&full[x.slot], kTileBytes);
+#pragma unroll
+            for (int d = 0; d < kDBlocks; ++d)
+#pragma unroll
+              for (int r = 0; r < 2; ++r)
+                tc::tma_load_4d(smem + at + x.slot * kTileBytes + d * kBlkX + r * kBlkY, tm, &full[x.slot],
+                                d * 64, head, tile * 128 + r * 64, batch);
+            return true;
+          };
+          ok = false;
+          if (!load_x(&tm_x1, x1_full, x1_empty, 0)) break;
+          for (int j = 0; j < n; ++j, r1.step(), r2.step()) {
+            ok = false;
+            const int s0 = (first + j) * 64;
+            // (the slot's column vectors were read before ds_ready, which y1_empty follows)
+            if (!tc::mbar_wait(&y1_empty[r1.slot], r1.phase ^ 1, abort_flag)) break;
+            uint64_t* full = &y1_full[r1.slot];
+            tc::mbar_arrive_expect_tx(full, kHalfBytes + vec_bytes);
+#pragma unroll
+            for (int d = 0; d < kDBlocks; ++d)
+              tc::tma_load_4d(smem + L::kY1At + r1.slot * kHalfBytes + d * kBlkY, &tm_y1, full, d * 64, head,
+                              s0, batch);
+            uint8_t* v = s_vec + r1.slot * L::kVec;
+            if constexpr (kKeys) {
+              tc::bulk_load(v, p.nlse + static_cast<int64_t>(bh) * p.Rq + s0, 256, full);
+              tc::bulk_load(v + 256, p.ndelta + static_cast<int64_t>(bh) * p.Rq + s0, 256, full);
+              if (load_keep)
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                  tc::bulk_load(v + 512 + r * 256,
+                                p.keep + (static_cast<int64_t>(bhl) * (p.Rk >> 5) + tile * 4 + r) * p.Rq + s0,
+                                256, full);
+            } else {
+              if (vec_bytes != 0)
+                tc::bulk_load(v, p.kb2 + static_cast<int64_t>(batch) * p.Rk + s0, 256, full);
+            }
+            if (j == 0 && !load_x(&tm_x2, x2_full, x2_empty, L::kX2)) break;
+            if (!tc::mbar_wait(&y2_empty[r2.slot], r2.phase ^ 1, abort_flag)) break;
+            tc::mbar_arrive_expect_tx(&y2_full[r2.slot], kHalfBytes);
+#pragma unroll
+            for (int d = 0; d < kDBlocks; ++d)
+              tc::tma_load_4d(smem + L::kY2At + r2.slot * kHalfBytes + d * kBlkY, &tm_y2, &y2_full[r2.slot],
+                              d * 64, head, s0, batch);
+            ok = true;
           }
-          if (!kFirst && more && !issue_s(t + 1, next_w, !same, next_last)) { ok = false; break; }
-          if (!tc::mbar_wait(ds_ready, t & 1, abort_flag)) { ok = false; break; }
-          if (kFirst && more && !issue_dp(t + 1, next_w, !same, next_last)) { ok = false; break; }
-          if constexpr (!kKeys) {
-            if (j == 0 && !tc::mbar_wait(acc_free, (w & 1) ^ 1, abort_flag)) { ok = false; break; }
-          }
-          tc::fence_after_sync();
-          accumulate(kColA1, kColDS, y_addr, j == 0);
-          tc::umma_commit(a1_done);
-          tc::umma_commit(&y_empty[st]);
-          if (j + 1 == n) tc::umma_commit(acc_full);
-          if (kOver && more && !tc::mbar_wait(a1_done, t & 1, abort_flag)) { ok = false; break; }
-          if (!kFirst && more && !issue_dp(t + 1, next_w, !same, next_last)) { ok = false; break; }
         }
-        item = next_item;
-        n = next_n;
-        ++w;
+      } else if (warp < 3) {
+        // ------------------------------ S (warp 1) and dP (warp 2) ------------------------------
+        const bool is_s = warp == 1;
+        const uint32_t x_desc = tc::smem_desc_lo(tc::smem_u32(smem + (is_s ? 0 : L::kX2)), 16);
+        const uint32_t y_desc = tc::smem_desc_lo(tc::smem_u32(smem + (is_s ? L::kY1At : L::kY2At)), 16);
+        const uint32_t col = is_s ? kColS : kColDP;
+        uint64_t* x_full = is_s ? x1_full : x2_full;
+        uint64_t* x_empty = is_s ? x1_empty : x2_empty;
+        uint64_t* y_full = is_s ? y1_full : y2_full;
+        uint64_t* out_full = is_s ? s_full : dp_full;
+        // what stood there has been read (P, dS: used up)
+        uint64_t* out_free = is_s ? (kOver ? a2_done : p_ready) : a1_done;
+        const int slots = is_s ? kY1 : kY2;
+        Ring<kX> x;
+        int slot = 0, h = 0;
+        uint32_t phase = 0;
+        for (int item = cta; item < items && ok; item += ctas, x.step()) {
+          int tile, bhl, first;
+          const int n = item_at(item, tile, bhl, first);
+          if (!tc::mbar_wait(&x_full[x.slot], x.phase, abort_flag)) break;
+          for (int j = 0; j < n; ++j, ++h) {
+            const int g = h & 1;
+            ok = false;
+            if (!tc::mbar_wait(&y_full[slot], phase, abort_flag)) break;
+            if (h >= 2 && !tc::mbar_wait(&out_free[g], ((h >> 1) & 1) ^ 1, abort_flag)) break;
+            tc::fence_after_sync();
+            scores(col + g * 64, x_desc + x.slot * kXStep, y_desc + slot * kYStep);
+            tc::umma_commit(&out_full[g]);
+            if (!is_s) tc::umma_commit(&y2_empty[slot]);
+            if (j + 1 == n) tc::umma_commit(&x_empty[x.slot]);
+            if (++slot == slots) { slot = 0; phase ^= 1; }
+            ok = true;
+          }
+        }
+      } else {
+        // ------------------------------ accumulating products ------------------------------
+        // In the dK / dV pass dV's of half tile h go before dK's of h - 1, whose dS is ready later;
+        // over the ends of items they stay in their order.
+        const uint32_t y1_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kY1At), kBlkY);
+        const uint32_t y2_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kY2At), kBlkY);
+        Ring<kY1> r1;
+        Ring<kY2> r2;
+        Ring<kAcc> acc;
+        int h = 0;
+        for (int item = cta; item < items && ok; item += ctas, acc.step()) {
+          int tile, bhl, first;
+          const int n = item_at(item, tile, bhl, first);
+          // what these accumulators held has been read out
+          if (!tc::mbar_wait(&acc_free[acc.slot], acc.phase ^ 1, abort_flag)) break;
+          const uint32_t a1 = kColA1 + acc.slot * kAccCols, a2 = kColA2 + acc.slot * kAccCols;
+          auto add_a1 = [&](int i, bool fresh) -> bool {     // half tile i of the sequence
+            if (!tc::mbar_wait(&ds_ready[i & 1], (i >> 1) & 1, abort_flag)) return false;
+            tc::fence_after_sync();
+            accumulate(a1, kColDP + (i & 1) * 64, y1_desc + r1.slot * kYStep, fresh);
+            tc::umma_commit(&a1_done[i & 1]);
+            tc::umma_commit(&y1_empty[r1.slot]);
+            r1.step();
+            return true;
+          };
+          for (int j = 0; j < n; ++j, ++h) {
+            ok = false;
+            if constexpr (kKeys) {
+              if (!tc::mbar_wait(&p_ready[h & 1], (h >> 1) & 1, abort_flag)) break;
+              tc::fence_after_sync();
+              accumulate(a2, kColP + (h & 1) * kPGroup, y2_desc + r2.slot * kYStep, j == 0);
+              tc::umma_commit(&a2_done[h & 1]);
+              tc::umma_commit(&y2_empty[r2.slot]);
+              r2.step();
+              if (j > 0 && !add_a1(h - 1, j == 1)) break;
+              if (j + 1 == n && !add_a1(h, j == 0)) break;
+            } else {
+              if (!add_a1(h, j == 0)) break;
+            }
+            ok = true;
+          }
+          if (ok) tc::umma_commit(&acc_full[acc.slot]);
+        }
       }
     }
-  } else {
-    // ------------------------------ softmax warps ------------------------------
-    const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;   // which 64 of the tile's 128 columns
-    const int r_in = quarter * 32 + lane;
-    const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    uint64_t seed = 0, offset = 0;
-    if ((!kKeys || kDraw) && drop) philox_unpack(p.rng, seed, offset);
-    const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
-    const int sk16 = (p.Sk + 15) >> 4;
-    // dS is formed without the factors scale and 1 / keep_prob; they are applied once to
-    // dQ and dK (and 1 / keep_prob to dV) when those leave TMEM
+  } else if (warp >= 12) {
+    tc::regs_dec<kRegsOut>();
+    // ------------------------------ accumulators out of tensor memory ------------------------------
+    // dS is formed without the factors scale and 1 / keep_prob; they are applied once to dQ and dK
+    // (and 1 / keep_prob to dV) here
     const float out_scale = p.scale * p.inv_keep;
-    const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
-
-    // accumulators of work item `item` out of tensor memory
-    auto read_out = [&](int item) {
+    const int r_in = (warp & 3) * 32 + lane;
+    const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    // D columns from `col` on, times f, to `dst` (or as they are to `share`)
+    auto read_out = [&](uint32_t col, float f, T* dst, float* share, bool row_ok) {
+#pragma unroll
+      for (int c = 0; c < D; c += 32) {
+        uint32_t r[32];
+        tc::tmem_ld_x32(tmem_row + col + c, r);
+        tc::tmem_ld_wait();
+        if (!row_ok) continue;
+        if (!kKeys && share != nullptr) {
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+            if (c + g * 4 < p.Dr)
+              *reinterpret_cast<uint4*>(share + c + g * 4) =
+                  make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+        } else {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            if (c + g * 8 < p.Dr) {
+              uint32_t v[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                v[i] = pack16<T>(__uint_as_float(r[g * 8 + 2 * i]) * f,
+                                 __uint_as_float(r[g * 8 + 2 * i + 1]) * f);
+              *reinterpret_cast<uint4*>(dst + c + g * 8) = make_uint4(v[0], v[1], v[2], v[3]);
+            }
+          }
+        }
+      }
+    };
+    Ring<kAcc> acc;
+    for (int item = cta; item < items; item += ctas, acc.step()) {
       int tile, bhl, first;
       item_at(item, tile, bhl, first);
       const int bh = p.walk.bh0 + bhl;
       const int batch = bh / p.H, head = bh - batch * p.H;
       const int row = tile * 128 + r_in;
       const int rows = kKeys ? p.Sk : p.Sq;
-      // dK / dV pass: the first four warps write dV, the others dK; dQ pass: half the columns each
-      const bool second = kKeys && half == 0;
-      const float f = second ? p.inv_keep : out_scale;
       const int64_t at = (static_cast<int64_t>(batch) * rows + min(row, rows - 1)) * p.H + head;
-      T* dst = second ? static_cast<T*>(p.out2) + at * p.row_stride2
-                      : static_cast<T*>(p.out1) + at * p.row_stride1;
-      const int c0 = kKeys ? 0 : half * (D / 2);
-      const uint32_t col = second ? kColA2 : kColA1;
       float* share = nullptr;
       if (!kKeys && p.splits > 1)
         share = p.part + (static_cast<int64_t>(item % p.splits) * p.part_rows + at) * p.Dr;
+      if (!tc::mbar_wait_warp(&acc_full[acc.slot], acc.phase, abort_flag)) break;
       tc::fence_after_sync();
-#pragma unroll
-      for (int c = 0; c < (kKeys ? D : D / 2); c += 32) {
-        uint32_t r[32];
-        tc::tmem_ld_x32(tmem_row + col + c0 + c, r);
-        tc::tmem_ld_wait();
-        if (!kKeys && share != nullptr) {
-          if (row < rows) {
-#pragma unroll
-            for (int g = 0; g < 8; ++g)
-              if (c0 + c + g * 4 < p.Dr)
-                *reinterpret_cast<uint4*>(share + c0 + c + g * 4) =
-                    make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
-          }
-        } else if (row < rows) {
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            if (c0 + c + g * 8 < p.Dr) {
-              uint32_t v[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                v[i] = pack16<T>(__uint_as_float(r[g * 8 + 2 * i]) * f,
-                                 __uint_as_float(r[g * 8 + 2 * i + 1]) * f);
-              *reinterpret_cast<uint4*>(dst + c0 + c + g * 8) = make_uint4(v[0], v[1], v[2], v[3]);
-            }
-          }
-        }
-      }
+      if constexpr (kKeys)
+        read_out(kColA2 + acc.slot * kAccCols, p.inv_keep, static_cast<T*>(p.out2) + at * p.row_stride2, nullptr, row < rows);
+      read_out(kColA1 + acc.slot * kAccCols, out_scale, static_cast<T*>(p.out1) + at * p.row_stride1, share, row < rows);
       tc::fence_before_sync();
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(acc_free);
-    };
+      if (lane == 0) tc::mbar_arrive(&acc_free[acc.slot]);
+    }
+  } else {
+    tc::regs_inc<kRegsSoftmax>();
+    // ------------------------------ softmax groups ------------------------------
+    const int quarter = warp & 3;
+    const int g = (warp - 4) >> 2;      // takes half tiles g, g + 2, ... of the CTA's sequence
+    const int r_in = quarter * 32 + lane;
+    const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    PhiloxUniform rng{};
+    if ((!kKeys || kDraw) && drop) rng = philox_uniform(p.rng);
+    const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
+    const int sk16 = (p.Sk + 15) >> 4;
+    const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2);
 
+    // a half tile of the sequence: half tile j of n of a work item, u0 is the item's first
+    struct Pos {
+      int item, tile, bhl, first, n, j, u0;
+    };
+    // the group's first one from sequence number pos.u0 and work item pos.item on
+    auto enter = [&](Pos& pos) {
+      while (pos.item < items) {
+        pos.n = item_at(pos.item, pos.tile, pos.bhl, pos.first);
+        pos.j = (pos.u0 & 1) ^ g;
+        if (pos.j < pos.n) return;
+        pos.u0 += pos.n;
+        pos.item += ctas;
+      }
+    };
     // per-row scalars of a work item: the dQ pass's statistics, the dK / dV pass's key bias
-    auto row_scalars = [&](int item, float& a, float& b) {
+    auto row_scalars = [&](const Pos& pos, float& a, float& b) {
       a = 0.f;
       b = 0.f;
-      if (item >= items) return;
-      int tile, bhl, first;
-      item_at(item, tile, bhl, first);
-      const int bh = p.walk.bh0 + bhl;
+      const int bh = p.walk.bh0 + pos.bhl;
       if constexpr (kKeys) {
         if (kGeneral && p.kb2 != nullptr)
-          a = p.kb2[static_cast<int64_t>(bh / p.H) * p.Rk + tile * 128 + r_in];
+          a = p.kb2[static_cast<int64_t>(bh / p.H) * p.Rk + pos.tile * 128 + r_in];
       } else {
-        a = p.nlse[static_cast<int64_t>(bh) * p.Rq + tile * 128 + r_in];
-        b = p.ndelta[static_cast<int64_t>(bh) * p.Rq + tile * 128 + r_in];
+        a = p.nlse[static_cast<int64_t>(bh) * p.Rq + pos.tile * 128 + r_in];
+        b = p.ndelta[static_cast<int64_t>(bh) * p.Rq + pos.tile * 128 + r_in];
       }
     };
 
-    // Relative bias of this warp's 32 rows and 64 columns in streamed tile `y` of a work item, on
-    // its way into buffer `buf`: copied a tile ahead, as in the forward.  A column further is a key
-    // further in the dQ pass, a query further (a smaller distance) in the other.
-    float* rel_buf = reinterpret_cast<float*>(smem + L::kRel) + (warp - 2) * 2 * L::kRelFloats;
+    // Relative bias of this warp's 32 rows and a half tile's 64 columns, on its way into buffer `buf`:
+    // copied a half tile ahead, as in the forward.  A column further is a key further in the dQ
+    // pass, a query further (a smaller distance) in the other.
+    float* rel_buf = reinterpret_cast<float*>(smem + L::kRel) + (warp - 4) * 2 * L::kRelFloats;
     const bool has_rel = kGeneral && p.rel != nullptr;
-    auto fetch_rel = [&](int tile, int bhl, int y, int buf) {
-      const int head = (p.walk.bh0 + bhl) % p.H;
+    auto fetch_rel = [&](const Pos& pos, int buf) {
+      const int head = (p.walk.bh0 + pos.bhl) % p.H;
       const float* src = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + p.Sq - 1;
-      const int r0 = tile * 128 + quarter * 32, c0 = y * 128 + half * 64;
+      const int r0 = pos.tile * 128 + quarter * 32, c0 = (pos.first + pos.j) * 64;
       const int d0 = kKeys ? r0 - (c0 + 63) : c0 - (r0 + 31);
 #pragma unroll
       for (int i = lane; i < L::kRelFloats; i += 32)
         cp_async4(rel_buf + buf * L::kRelFloats + i, src + max(1 - p.Sq, min(d0 + i, p.Sk - 1)));
     };
-    if (has_rel && cta < items) {
-      int tile, bhl, first;
-      item_at(cta, tile, bhl, first);
-      fetch_rel(tile, bhl, first, 0);
-    }
 
+    Pos pos{};
+    pos.item = cta;
+    enter(pos);
+    float row_a = 0.f, row_b = 0.f;
+    if (pos.item < items) {
+      row_scalars(pos, row_a, row_b);
+      if (has_rel) fetch_rel(pos, 0);
+    }
     bool ok = true;
-    int t = 0, w = 0, prev_item = -1;
-    float rs_a, rs_b;
-    row_scalars(cta, rs_a, rs_b);
-    for (int item = cta; item < items && ok; item += ctas, ++w) {
-      int tile, bhl, first;
-      const int n = item_at(item, tile, bhl, first);
-      const int bh = p.walk.bh0 + bhl;
-      const int head = bh % p.H;
-      const int row = tile * 128 + r_in;
-      const float row_a = rs_a, row_b = rs_b;
-      row_scalars(item + ctas, rs_a, rs_b);      // under this item's work
+    int slot = g;                         // of the Y1 ring
+    bool first_p = true;
+    uint32_t slot_phase = 0, ph = 0;      // ph: parity of the group's count of half tiles
+    while (pos.item < items && ok) {
+      const int bh = p.walk.bh0 + pos.bhl;
+      const int row = pos.tile * 128 + r_in;
       const uint64_t ra2 = f2_pack(row_a, row_a), rb2 = f2_pack(row_b, row_b);
-      for (int j = 0; j < n; ++j, ++t) {
-        const int st = t % kStages;
-        const int col0 = (first + j) * 128 + half * 64;     // this thread's first column
-        const uint8_t* vec = s_vec + st * L::kVec;
+      const uint64_t drop_row = (static_cast<uint64_t>(bh) * p.Sq + min(row, p.Sq - 1)) * sk16;
+      Pos next = pos;
+      for (; pos.j < pos.n; pos.j += 2) {
+        const int col0 = (pos.first + pos.j) * 64;       // the half tile's first column
+        const uint8_t* vec = s_vec + slot * L::kVec;
+        if (pos.j + 2 >= pos.n) {       // the item's last: the next one's rows, under its work
+          next.u0 += pos.n;
+          next.item += ctas;
+          enter(next);
+          if (next.item < items) row_scalars(next, row_a, row_b);
+        } else {
+          next.j = pos.j + 2;
+        }
         if (has_rel) {
           cp_async_wait();
           __syncwarp();     // (visible to the warp, and the other buffer's readers are done)
-          if (j + 1 < n) {
-            fetch_rel(tile, bhl, first + j + 1, (t + 1) & 1);
-          } else if (item + ctas < items) {
-            int next_tile, next_bhl, next_first;
-            item_at(item + ctas, next_tile, next_bhl, next_first);
-            fetch_rel(next_tile, next_bhl, next_first, (t + 1) & 1);
-          }
+          if (next.item < items) fetch_rel(next, ph ^ 1);
         }
-        // ---- dropout decisions of this row and the thread's 64 keys (dQ pass) ----
+        // ---- dropout decisions of this row and the half tile's keys (dQ pass) ----
         uint32_t keep16[4][4];
         if (!kKeys && drop) {
-          const uint64_t base = (static_cast<uint64_t>(bh) * p.Sq + min(row, p.Sq - 1)) * sk16 + (col0 >> 4);
           uint32_t bits[2];
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            const uint4 kw = philox_keep16(seed, offset, base + g, add4);
-            keep16[g][0] = kw.x; keep16[g][1] = kw.y; keep16[g][2] = kw.z; keep16[g][3] = kw.w;
+          for (int q = 0; q < 4; ++q) {
+            const uint4 kw = philox_keep16(rng, drop_row + (col0 >> 4) + q, add4);
+            keep16[q][0] = kw.x; keep16[q][1] = kw.y; keep16[q][2] = kw.z; keep16[q][3] = kw.w;
             if constexpr (!kDraw) {
               const uint32_t m = keep_bits16(kw);
-              if (g & 1) bits[g >> 1] |= m << 16;
-              else bits[g >> 1] = m;
+              if (q & 1) bits[q >> 1] |= m << 16;
+              else bits[q >> 1] = m;
             }
           }
           if constexpr (!kDraw) {
-            uint32_t* dst = p.keep + (static_cast<int64_t>(bhl) * (p.Rk >> 5) + (col0 >> 5)) * p.Rq + row;
+            uint32_t* dst = p.keep + (static_cast<int64_t>(pos.bhl) * (p.Rk >> 5) + (col0 >> 5)) * p.Rq + row;
             dst[0] = bits[0];
             dst[p.Rq] = bits[1];
           }
         }
-        // ---- ... of the warp's 32 keys and 64 queries (dK / dV pass), two queries per lane, into the
-        // words that the other form loads ----
+        // ---- ... of the warp's 32 keys and the half tile's queries (dK / dV pass), two queries per lane,
+        // into the words that the other form loads ----
         if constexpr (kKeys && kDraw) {
           if (drop) {
-            uint32_t* words = reinterpret_cast<uint32_t*>(s_vec + st * L::kVec + 1024 + quarter * 512) + half * 64;
+            uint32_t* words = reinterpret_cast<uint32_t*>(s_vec + slot * L::kVec + 512 + quarter * 256);
 #pragma unroll
             for (int i = lane; i < 64; i += 32) {
-              const uint64_t base = (static_cast<uint64_t>(bh) * p.Sq + min(col0 + i, p.Sq - 1)) * sk16 +
-                                    ((tile * 128 + quarter * 32) >> 4);
-              words[i] = keep_bits16(philox_keep16(seed, offset, base, add4)) |
-                         keep_bits16(philox_keep16(seed, offset, base + 1, add4)) << 16;
+              const uint64_t at = (static_cast<uint64_t>(bh) * p.Sq + min(col0 + i, p.Sq - 1)) * sk16 +
+                                  ((pos.tile * 128 + quarter * 32) >> 4);
+              words[i] = keep_bits16(philox_keep16(rng, at, add4)) |
+                         keep_bits16(philox_keep16(rng, at + 1, add4)) << 16;
             }
             __syncwarp();
           }
         }
         // ---- P ----
-        if (!tc::mbar_wait_warp(s_full, t & 1, abort_flag)) { ok = false; break; }
+        if (!tc::mbar_wait_warp(&s_full[g], ph, abort_flag)) { ok = false; break; }
         // (complete since before s_full; waiting on it makes the column vectors visible)
-        if (!tc::mbar_wait_warp(&y_full[st], (t / kStages) & 1, abort_flag)) { ok = false; break; }
+        if (kKeys || (kGeneral && p.kb2 != nullptr)) {
+          if (!tc::mbar_wait_warp(&y1_full[slot], slot_phase, abort_flag)) { ok = false; break; }
+        }
         tc::fence_after_sync();
         float pr[64];
         {
           uint32_t s0[32], s1[32];
-          tc::tmem_ld_x32(tmem_row + kColS + half * 64, s0);
-          tc::tmem_ld_x32(tmem_row + kColS + half * 64 + 32, s1);
+          tc::tmem_ld_x32(tmem_row + kColS + g * 64, s0);
+          tc::tmem_ld_x32(tmem_row + kColS + g * 64 + 32, s1);
           tc::tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
@@ -592,38 +655,38 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
         if constexpr (!kKeys) {
           tc::fence_before_sync();
           __syncwarp();
-          if (lane == 0) tc::mbar_arrive(p_ready);
+          if (lane == 0) tc::mbar_arrive(&p_ready[g]);
         }
-        {
-          const float4* cv = reinterpret_cast<const float4*>(vec) + half * 16;
-          const bool cols = kKeys || (kGeneral && p.kb2 != nullptr);
+        const float4* cv = reinterpret_cast<const float4*>(vec);
 #pragma unroll
-          for (int i = 0; i < 64; i += 4) {
-            uint64_t x0 = f2_pack(pr[i], pr[i + 1]), x1 = f2_pack(pr[i + 2], pr[i + 3]);
-            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (cols) c = cv[i >> 2];
-            if constexpr (kKeys) {
-              x0 = f2_fma(x0, sc2, f2_pack(c.x, c.y));
-              x1 = f2_fma(x1, sc2, f2_pack(c.z, c.w));
-              if (kGeneral) {
-                x0 = f2_add(x0, ra2);
-                x1 = f2_add(x1, ra2);
-              }
-            } else {
-              x0 = f2_fma(x0, sc2, ra2);
-              x1 = f2_fma(x1, sc2, ra2);
-              if (kGeneral && cols) {
-                x0 = f2_add(x0, f2_pack(c.x, c.y));
-                x1 = f2_add(x1, f2_pack(c.z, c.w));
-              }
+        for (int i = 0; i < 64; i += 4) {
+          uint64_t x0 = f2_pack(pr[i], pr[i + 1]), x1 = f2_pack(pr[i + 2], pr[i + 3]);
+          if constexpr (kKeys) {
+            const float4 c = cv[i >> 2];
+            x0 = f2_fma(x0, sc2, f2_pack(c.x, c.y));
+            x1 = f2_fma(x1, sc2, f2_pack(c.z, c.w));
+            if (kGeneral) {
+              x0 = f2_add(x0, ra2);
+              x1 = f2_add(x1, ra2);
             }
-            f2_unpack(x0, pr[i], pr[i + 1]);
-            f2_unpack(x1, pr[i + 2], pr[i + 3]);
+          } else {
+            x0 = f2_fma(x0, sc2, ra2);
+            x1 = f2_fma(x1, sc2, ra2);
           }
+          f2_unpack(x0, pr[i], pr[i + 1]);
+          f2_unpack(x1, pr[i + 2], pr[i + 3]);
         }
         if constexpr (kGeneral) {
+          if (!kKeys && p.kb2 != nullptr) {
+#pragma unroll
+            for (int i = 0; i < 64; i += 4) {
+              const float4 c = cv[i >> 2];
+              f2_unpack(f2_add(f2_pack(pr[i], pr[i + 1]), f2_pack(c.x, c.y)), pr[i], pr[i + 1]);
+              f2_unpack(f2_add(f2_pack(pr[i + 2], pr[i + 3]), f2_pack(c.z, c.w)), pr[i + 2], pr[i + 3]);
+            }
+          }
           if (has_rel) {
-            const float* rel = rel_buf + (t & 1) * L::kRelFloats + (kKeys ? lane + 63 : 31 - lane);
+            const float* rel = rel_buf + ph * L::kRelFloats + (kKeys ? lane + 63 : 31 - lane);
             const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
 #pragma unroll
             for (int i = 0; i < 64; i += 2) {
@@ -634,111 +697,113 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
           }
           if constexpr (kKeys) {
             // key `row` is seen by queries >= row - diag (queries beyond Sq have nlse = -inf)
-            if (p.causal && col0 + diag < tile * 128 + quarter * 32 + 31) {
+            if (p.causal && col0 + diag < pos.tile * 128 + quarter * 32 + 31) {
+              const int from = row - diag - col0;
 #pragma unroll
-              for (int i = 0; i < 64; ++i)
-                if (col0 + i + diag < row) pr[i] = -INFINITY;
+              for (int c = 0; c < 2; ++c) {
+                const uint32_t hidden = low_bits(from - c * 32);
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (hidden & (1u << i)) pr[c * 32 + i] = -INFINITY;
+              }
             }
           } else {
-            const int limit = p.causal ? min(p.Sk, row + diag + 1) : p.Sk;
-            const int first_limit = p.causal ? min(p.Sk, tile * 128 + quarter * 32 + diag + 1) : p.Sk;
+            const int first_limit = p.causal ? min(p.Sk, pos.tile * 128 + quarter * 32 + diag + 1) : p.Sk;
             if (col0 + 64 > first_limit) {
+              const int limit = (p.causal ? min(p.Sk, row + diag + 1) : p.Sk) - col0;
 #pragma unroll
-              for (int i = 0; i < 64; ++i)
-                if (col0 + i >= limit) pr[i] = -INFINITY;
+              for (int c = 0; c < 2; ++c) {
+                const uint32_t seen = low_bits(limit - c * 32);
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (!(seen & (1u << i))) pr[c * 32 + i] = -INFINITY;
+              }
             }
           }
         }
+        // (kept before the waits that follow: the compiler would move it behind them)
 #pragma unroll
-        for (int i = 0; i < 64; ++i) pr[i] = exp2f(pr[i]);
-        const uint4* kw4 = reinterpret_cast<const uint4*>(vec + 1024 + quarter * 512) + half * 16;
-        const uint32_t lane_bit = 1u << lane;
+        for (int i = 0; i < 64; ++i) pr[i] = exp2_here(pr[i]);
         if constexpr (kKeys) {
-          if (!kOver && t > 0 && !tc::mbar_wait_warp(a2_done, (t - 1) & 1, abort_flag)) {
-            ok = false;
-            break;
-          }
+          if (!kOver && !first_p && !tc::mbar_wait_warp(&a2_done[g], ph ^ 1, abort_flag)) { ok = false; break; }
           tc::fence_after_sync();
+          first_p = false;
+          if (drop) {
+            // a dropped probability is kept as its negative: it still counts in dS's row term
+            const uint4* kw4 = reinterpret_cast<const uint4*>(vec + 512 + quarter * 256);
+            const uint32_t lane_bit = 1u << lane;
+#pragma unroll
+            for (int i = 0; i < 64; i += 4) {
+              const uint4 kw = kw4[i >> 2];
+              pr[i] = kw.x & lane_bit ? pr[i] : -pr[i];
+              pr[i + 1] = kw.y & lane_bit ? pr[i + 1] : -pr[i + 1];
+              pr[i + 2] = kw.z & lane_bit ? pr[i + 2] : -pr[i + 2];
+              pr[i + 3] = kw.w & lane_bit ? pr[i + 3] : -pr[i + 3];
+            }
+          }
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             uint32_t pk[16];
-            if (drop) {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                const uint4 k = kw4[c * 8 + i];
-                const float* v = pr + c * 32 + i * 4;
-                pk[2 * i] = pack16<T>((k.x & lane_bit) ? v[0] : 0.f, (k.y & lane_bit) ? v[1] : 0.f);
-                pk[2 * i + 1] = pack16<T>((k.z & lane_bit) ? v[2] : 0.f, (k.w & lane_bit) ? v[3] : 0.f);
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 16; ++i) pk[i] = pack16<T>(pr[c * 32 + 2 * i], pr[c * 32 + 2 * i + 1]);
-            }
-            tc::tmem_st_x16(tmem_row + kColP + half * kHalf + c * 16, pk);
+            for (int i = 0; i < 16; ++i) pk[i] = pack16_relu<T>(pr[c * 32 + 2 * i], pr[c * 32 + 2 * i + 1]);
+            tc::tmem_st_x16(tmem_row + kColP + g * kPGroup + c * 16, pk);
           }
           tc::tmem_st_wait();
           tc::fence_before_sync();
           __syncwarp();
-          if (lane == 0) tc::mbar_arrive(p_ready);
-        }
-        // ---- the item before this one leaves tensor memory ----
-        if (j == 0 && prev_item >= 0) {
-          if (!tc::mbar_wait_warp(acc_full, (w - 1) & 1, abort_flag)) { ok = false; break; }
-          read_out(prev_item);
+          if (lane == 0) tc::mbar_arrive(&p_ready[g]);
         }
         // ---- dS ----
-        if (!tc::mbar_wait_warp(dp_full, t & 1, abort_flag)) { ok = false; break; }
-        if (!kOver && t > 0 && !tc::mbar_wait_warp(a1_done, (t - 1) & 1, abort_flag)) { ok = false; break; }
+        if (!tc::mbar_wait_warp(&dp_full[g], ph, abort_flag)) { ok = false; break; }
         tc::fence_after_sync();
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t d[32];
-          tc::tmem_ld_x32(tmem_row + kColDP + half * 64 + c * 32, d);
+          tc::tmem_ld_x32(tmem_row + kColDP + g * 64 + c * 32, d);
           tc::tmem_ld_wait();
-          if (drop) {
-            if constexpr (kKeys) {
+          if (!kKeys && drop) {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                const uint4 k = kw4[c * 8 + i];
-                d[4 * i] = (k.x & lane_bit) ? d[4 * i] : 0u;
-                d[4 * i + 1] = (k.y & lane_bit) ? d[4 * i + 1] : 0u;
-                d[4 * i + 2] = (k.z & lane_bit) ? d[4 * i + 2] : 0u;
-                d[4 * i + 3] = (k.w & lane_bit) ? d[4 * i + 3] : 0u;
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                d[i] &= keep_mask_full(keep16[c * 2 + (i >> 4)][(i >> 2) & 3], i & 3);
-            }
+            for (int i = 0; i < 32; ++i)
+              d[i] &= keep_mask_full(keep16[c * 2 + (i >> 4)][(i >> 2) & 3], i & 3);
           }
-          const float4* nd = reinterpret_cast<const float4*>(vec + 512) + half * 16 + c * 8;
+          const float4* nd = reinterpret_cast<const float4*>(vec + 256) + c * 8;
+          const float* v = pr + c * 32;
           float ds[32];
+          if (kKeys && drop) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            uint64_t x0 = f2_pack(__uint_as_float(d[i]), __uint_as_float(d[i + 1]));
-            uint64_t x1 = f2_pack(__uint_as_float(d[i + 2]), __uint_as_float(d[i + 3]));
-            if constexpr (kKeys) {
+            for (int i = 0; i < 32; i += 4) {
               const float4 dl = nd[i >> 2];
-              x0 = f2_add(x0, f2_pack(dl.x, dl.y));
-              x1 = f2_add(x1, f2_pack(dl.z, dl.w));
-            } else {
-              x0 = f2_add(x0, rb2);
-              x1 = f2_add(x1, rb2);
+              const float n4[4] = {dl.x, dl.y, dl.z, dl.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                ds[i + e] = fmaf(fmaxf(v[i + e], 0.f), __uint_as_float(d[i + e]), fabsf(v[i + e]) * n4[e]);
             }
-            const float* v = pr + c * 32 + i;
-            x0 = f2_mul(x0, f2_pack(v[0], v[1]));
-            x1 = f2_mul(x1, f2_pack(v[2], v[3]));
-            f2_unpack(x0, ds[i], ds[i + 1]);
-            f2_unpack(x1, ds[i + 2], ds[i + 3]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              uint64_t x0 = f2_load(d + i), x1 = f2_load(d + i + 2);
+              if constexpr (kKeys) {
+                const float4 dl = nd[i >> 2];
+                x0 = f2_add(x0, f2_pack(dl.x, dl.y));
+                x1 = f2_add(x1, f2_pack(dl.z, dl.w));
+              } else {
+                x0 = f2_add(x0, rb2);
+                x1 = f2_add(x1, rb2);
+              }
+              x0 = f2_mul(x0, f2_pack(v[i], v[i + 1]));
+              x1 = f2_mul(x1, f2_pack(v[i + 2], v[i + 3]));
+              f2_unpack(x0, ds[i], ds[i + 1]);
+              f2_unpack(x1, ds[i + 2], ds[i + 3]);
+            }
           }
           if constexpr (kKeys && kGeneral) {
             if (p.drel != nullptr) {
               // Sums along the diagonals key - query = const: the running sum moves one lane up
               // (next key) with every column (next query), so that it stays on its diagonal;
               // what leaves at lane 31 is collected and added to the result 32 at a time.
-              float* buf = reinterpret_cast<float*>(smem + L::kDrel) + (warp - 2) * 32;
-              float* out = p.drel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1);
-              const int key0 = tile * 128 + quarter * 32, q0 = col0 + c * 32;
+              float* buf = reinterpret_cast<float*>(smem + L::kDrel) + (warp - 4) * 32;
+              float* out = p.drel + static_cast<int64_t>(bh % p.H) * (p.Sq + p.Sk - 1);
+              const int key0 = pos.tile * 128 + quarter * 32, q0 = col0 + c * 32;
               const int last = p.Sq + p.Sk - 2;
               float acc = 0.f;
 #pragma unroll
@@ -762,17 +827,18 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) pk[i] = pack16<T>(ds[2 * i], ds[2 * i + 1]);
-          tc::tmem_st_x16(tmem_row + kColDS + half * kHalf + c * 16, pk);
+          tc::tmem_st_x16(tmem_row + kColDP + g * 64 + c * 16, pk);
         }
         tc::tmem_st_wait();
         tc::fence_before_sync();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(ds_ready);
+        if (lane == 0) tc::mbar_arrive(&ds_ready[g]);
+        ph ^= 1;
+        slot += 2;
+        if (slot >= kY1) { slot -= kY1; slot_phase ^= 1; }
       }
-      prev_item = item;
+      pos = next;
     }
-    if (ok && prev_item >= 0 && tc::mbar_wait_warp(acc_full, (w - 1) & 1, abort_flag))
-      read_out(prev_item);
     if (has_rel) cp_async_wait();     // (a give-up leaves copies under way)
   }
 
@@ -787,7 +853,7 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
 
 // One pass.
 template <int D, bool kKeys, bool kGeneral, typename T>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(512, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ CUtensorMap tm_x2,
                  const __grid_constant__ CUtensorMap tm_y1, const __grid_constant__ CUtensorMap tm_y2,
                  const __grid_constant__ FlashBwdParams p) {
@@ -796,7 +862,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
 
 // Both passes side by side, the dQ pass on the first `q_ctas` CTAs.
 template <int D, bool kGeneral, typename T>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(512, 1)
 flash_bwd_both_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                       const __grid_constant__ FlashBwdParams pq,
@@ -846,7 +912,7 @@ static int launch_bwd(void (*kernel)(P...), int ctas, int smem, bool early, cuda
                       const A&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(320);
+  cfg.blockDim = dim3(512);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr{};
@@ -990,10 +1056,10 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o,
   if (B <= 0 || H <= 0 || Sq <= 0 || Sk <= 0) return 1;
   CUtensorMap tq, tk, tv, tdo;
   const int64_t do_strides[3] = {static_cast<int64_t>(Sq) * H * D, static_cast<int64_t>(H) * D, D};
-  if (!make_tmap_bshd(&tq, q, B, Sq, H, D, q_strides[0], q_strides[1], q_strides[2], 128, bf16) ||
-      !make_tmap_bshd(&tk, k, B, Sk, H, D, k_strides[0], k_strides[1], k_strides[2], 128, bf16) ||
-      !make_tmap_bshd(&tv, v, B, Sk, H, D, v_strides[0], v_strides[1], v_strides[2], 128, bf16) ||
-      !make_tmap_bshd(&tdo, dout, B, Sq, H, D, do_strides[0], do_strides[1], do_strides[2], 128, bf16))
+  if (!make_tmap_bshd(&tq, q, B, Sq, H, D, q_strides[0], q_strides[1], q_strides[2], 64, bf16) ||
+      !make_tmap_bshd(&tk, k, B, Sk, H, D, k_strides[0], k_strides[1], k_strides[2], 64, bf16) ||
+      !make_tmap_bshd(&tv, v, B, Sk, H, D, v_strides[0], v_strides[1], v_strides[2], 64, bf16) ||
+      !make_tmap_bshd(&tdo, dout, B, Sq, H, D, do_strides[0], do_strides[1], do_strides[2], 64, bf16))
     return 2;
   FlashBwdParams p;
   p.Sq = Sq; p.Sk = Sk; p.H = H; p.Dr = D;
@@ -1014,7 +1080,7 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o,
   p.rel = rel; p.drel = drel;
   p.scale = scale; p.scale_log2 = scale * kLog2e; p.inv_keep = 1.f / keep_prob;
   p.causal = causal; p.rng = rng; p.status = status;
-  p.idesc_s = tc::instr_desc_f16(128, 128, bf16 ? 1 : 0, false, false);
+  p.idesc_s = tc::instr_desc_f16(128, 64, bf16 ? 1 : 0, false, false);
   p.idesc_acc = tc::instr_desc_f16(128, p.k_steps * 16, bf16 ? 1 : 0, false, true);
   {
     const int lanes = D <= 64 ? 8 : 16;

@@ -33,6 +33,14 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
   return d;
 }
 
+// 2^x on the special-function unit (what exp2f compiles to here), where it is written: not moved
+// behind the waits that follow it
+__device__ __forceinline__ float exp2_here(float x) {
+  float r;
+  asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // two neighbouring words of a row of scores as one such pair
 __device__ __forceinline__ uint64_t f2_load(const uint32_t* r) {
   return f2_pack(__uint_as_float(r[0]), __uint_as_float(r[1]));
@@ -62,6 +70,19 @@ template <> __device__ __forceinline__ uint32_t pack16<__half>(float a, float b)
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// ... of values that count as 0 where they are negative
+template <typename T> __device__ __forceinline__ uint32_t pack16_relu(float a, float b);
+template <> __device__ __forceinline__ uint32_t pack16_relu<__nv_bfloat16>(float a, float b) {
+  uint32_t d;
+  asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(b), "f"(a));
+  return d;
+}
+template <> __device__ __forceinline__ uint32_t pack16_relu<__half>(float a, float b) {
+  uint32_t d;
+  asm("cvt.rn.relu.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(b), "f"(a));
+  return d;
+}
+
 // Overlap of a kernel's prologue with the kernel before it in the stream: a kernel that the next
 // one may start under says so, and one that was launched that way waits until all work before it
 // is complete and visible (at once, when it was launched the ordinary way).
@@ -76,6 +97,44 @@ __device__ __forceinline__ uint32_t keep_bits16(const uint4& kw) {
   for (int i = 0; i < 4; ++i)       // bit 7 of the four bytes, gathered by one multiply
     m |= ((((w[i] >> 7) & 0x01010101u) * 0x01020408u) >> 24) << (4 * i);
   return m;
+}
+
+// bits 0 .. n - 1 (none for n <= 0, all for n >= 32)
+__device__ __forceinline__ uint32_t low_bits(int n) {
+  return n >= 32 ? 0xffffffffu : (1u << max(n, 0)) - 1u;
+}
+
+// A generator's state in uniform registers: a reduction over the warp tells the compiler that all
+// lanes have the same, and the round keys of a call then cost no per-lane instruction.
+struct PhiloxUniform {
+  uint32_t seed_lo, seed_hi, offset_lo, offset_hi;
+};
+__device__ __forceinline__ PhiloxUniform philox_uniform(const PhiloxArgs& a) {
+  uint64_t seed, offset;
+  philox_unpack(a, seed, offset);
+  return {__reduce_or_sync(0xffffffffu, static_cast<uint32_t>(seed)),
+          __reduce_or_sync(0xffffffffu, static_cast<uint32_t>(seed >> 32)),
+          __reduce_or_sync(0xffffffffu, static_cast<uint32_t>(offset)),
+          __reduce_or_sync(0xffffffffu, static_cast<uint32_t>(offset >> 32))};
+}
+// philox_keep16 (common.cuh) of such a state
+__device__ __forceinline__ uint4 philox_keep16(const PhiloxUniform& s, uint64_t index, uint32_t add4) {
+  uint4 c = make_uint4(s.offset_lo, s.offset_hi, static_cast<uint32_t>(index),
+                       static_cast<uint32_t>(index >> 32));
+  uint32_t kx = s.seed_lo, ky = s.seed_hi;
+#pragma unroll
+  for (int r = 0; r < 7; ++r) {
+    const uint2 m0 = mulhilo32(0xD2511F53u, c.x);
+    const uint2 m1 = mulhilo32(0xCD9E8D57u, c.z);
+    c = make_uint4(m1.y ^ c.y ^ kx, m1.x, m0.y ^ c.w ^ ky, m0.x);
+    kx += 0x9E3779B9u;
+    ky += 0xBB67AE85u;
+  }
+  c.x = (c.x & 0x7f7f7f7fu) + add4;
+  c.y = (c.y & 0x7f7f7f7fu) + add4;
+  c.z = (c.z & 0x7f7f7f7fu) + add4;
+  c.w = (c.w & 0x7f7f7f7fu) + add4;
+  return c;
 }
 
 // Row tiles of 128 of all (batch, head) pairs, walked by a persistent grid.  Under a causal

@@ -18,6 +18,21 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// One lane of a converged warp.  Code under this condition (and not under `lane == 0`) is known to
+// run in one thread, so that addresses and descriptors stay in uniform registers, which
+// tcgen05.mma takes its operands from.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(one));
+  return one != 0;
+}
+
 // ---- mbarrier ------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
@@ -291,6 +306,18 @@ __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// ---- registers of a warpgroup ------------------------------------------------------
+// Whole-warpgroup calls (four aligned warps).  What the warpgroups of a block ask for together may
+// not exceed what the block was launched with: `inc` waits for registers that others give up.
+template <int N>
+__device__ __forceinline__ void regs_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void regs_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+
 // ---- descriptors ---------------------------------------------------------------
 // Shared-memory matrix descriptor, 128-byte swizzle, sm_100 version field.
 //   K-major tile  : rows of 128 B (64 x 16-bit along K); SBO = 1024 B between
@@ -306,6 +333,20 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t smem_addr, uint32_t lbo_b
   d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32;
   d |= static_cast<uint64_t>(1) << 46;  // descriptor version (Blackwell)
   d |= static_cast<uint64_t>(2) << 61;  // SWIZZLE_128B
+  return d;
+}
+
+// The same in two words: the low one holds the address in units of 16 bytes, so that stepping
+// through shared memory is a 32-bit addition; the high one is a constant.
+__host__ __device__ constexpr uint32_t smem_desc_hi(uint32_t sbo_bytes) {
+  return (sbo_bytes >> 4) | (1u << 14) | (2u << 29);
+}
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
+  return (smem_addr >> 4) | (lbo_bytes >> 4) << 16;
+}
+__device__ __forceinline__ uint64_t smem_desc_words(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
   return d;
 }
 
