@@ -159,7 +159,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tc::tma_prefetch_desc(&tmap_a);
       tc::tma_prefetch_desc(&tmap_b);
       int stage = 0;
@@ -193,7 +193,10 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
+      constexpr uint32_t kDescHi = tc::smem_desc_hi(1024);
+      const uint32_t a_first = tc::smem_desc_lo(tc::smem_u32(smem_a), A_MN ? BK * 128 : 16);
+      const uint32_t b_first = tc::smem_desc_lo(tc::smem_u32(smem_b), B_MN ? BK * 128 : 16);
       int stage = 0;
       uint32_t phase = 0;
       int iter = 0;
@@ -207,15 +210,13 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!tc::mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           tc::fence_after_sync();
-          const uint32_t a_addr = tc::smem_u32(smem_a + stage * S::kABytes);
-          const uint32_t b_addr = tc::smem_u32(smem_b + stage * S::kBBytes);
+          const uint32_t a_desc = a_first + stage * (S::kABytes >> 4);
+          const uint32_t b_desc = b_first + stage * (S::kBBytes >> 4);
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t a_desc = A_MN ? tc::smem_desc(a_addr + k * 2048, BK * 128, 1024)
-                                         : tc::smem_desc(a_addr + k * 32, 16, 1024);
-            const uint64_t b_desc = B_MN ? tc::smem_desc(b_addr + k * 2048, BK * 128, 1024)
-                                         : tc::smem_desc(b_addr + k * 32, 16, 1024);
-            tc::umma_f16(d_tmem, a_desc, b_desc, p.idesc, (kb | k) != 0 ? 1u : 0u);
+            tc::umma_f16(d_tmem, tc::smem_desc_words(a_desc + k * ((A_MN ? 2048 : 32) >> 4), kDescHi),
+                         tc::smem_desc_words(b_desc + k * ((B_MN ? 2048 : 32) >> 4), kDescHi), p.idesc,
+                         (kb | k) != 0 ? 1u : 0u);
           }
           tc::umma_commit(&empty_bar[stage]);  // stage reusable once these MMAs retire
           if (++stage == STAGES) { stage = 0; phase ^= 1; }

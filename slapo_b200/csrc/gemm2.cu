@@ -198,7 +198,7 @@ gemm2_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tc::tma_prefetch_desc(&tmap_a);
       tc::tma_prefetch_desc(&tmap_b);
       int stage = 0;
@@ -241,7 +241,10 @@ gemm2_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader only) -----------------------------
-    if (lane == 0 && cta == 0) {
+    if (cta == 0 && tc::elect_one()) {
+      constexpr uint32_t kDescHi = tc::smem_desc_hi(1024);
+      const uint32_t a_first = tc::smem_desc_lo(tc::smem_u32(smem_a), A_MN ? PBK * 128 : 16);
+      const uint32_t b_first = tc::smem_desc_lo(tc::smem_u32(smem_b), B_MN ? PBK * 128 : 16);
       int stage = 0;
       uint32_t phase = 0;
       int iter = 0;
@@ -260,16 +263,14 @@ gemm2_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
           tc::fence_after_sync();
 #pragma unroll
           for (int s = 0; s < KSUB; ++s) {
-            const uint32_t a_addr = tc::smem_u32(smem_a + stage * S::kABytes + s * S::kASub);
-            const uint32_t b_addr = tc::smem_u32(smem_b + stage * S::kBBytes + s * S::kBSub);
+            const uint32_t a_desc = a_first + ((stage * S::kABytes + s * S::kASub) >> 4);
+            const uint32_t b_desc = b_first + ((stage * S::kBBytes + s * S::kBSub) >> 4);
 #pragma unroll
             for (int k = 0; k < PBK / 16; ++k) {
-              const uint64_t a_desc = A_MN ? tc::smem_desc(a_addr + k * 2048, PBK * 128, 1024)
-                                           : tc::smem_desc(a_addr + k * 32, 16, 1024);
-              const uint64_t b_desc = B_MN ? tc::smem_desc(b_addr + k * 2048, PBK * 128, 1024)
-                                           : tc::smem_desc(b_addr + k * 32, 16, 1024);
-              tc::umma_f16_pair(d_tmem, a_desc, b_desc, p.idesc,
-                                (kb > kb0 || s != 0 || k != 0) ? 1u : 0u);
+              tc::umma_f16_pair(d_tmem,
+                                tc::smem_desc_words(a_desc + k * ((A_MN ? 2048 : 32) >> 4), kDescHi),
+                                tc::smem_desc_words(b_desc + k * ((B_MN ? 2048 : 32) >> 4), kDescHi),
+                                p.idesc, (kb > kb0 || s != 0 || k != 0) ? 1u : 0u);
             }
           }
           // the stage is reusable in both CTAs once these MMAs retire
