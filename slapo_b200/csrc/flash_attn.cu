@@ -192,7 +192,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tc::tma_prefetch_desc(&tm_q);
       tc::tma_prefetch_desc(&tm_k);
       tc::tma_prefetch_desc(&tm_v);
@@ -226,21 +226,24 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t q_addr = tc::smem_u32(s_q);
+    if (tc::elect_one()) {
+      constexpr uint32_t kDescHi = tc::smem_desc_hi(1024);
+      const uint32_t q_desc = tc::smem_desc_lo(tc::smem_u32(s_q), 16);
+      const uint32_t k_desc = tc::smem_desc_lo(tc::smem_u32(s_k), 16);
+      const uint32_t v_desc = tc::smem_desc_lo(tc::smem_u32(s_v), kBlkBytes);
       // S of tile t (the w-th item's; `last`: its last one)
       auto issue_qk = [&](int t, int w, bool first, bool last) -> bool {
         const int st = t % kStages;
         if (first && !tc::mbar_wait(q_full, w & 1, abort_flag)) return false;
         if (!tc::mbar_wait(&k_full[st], (t / kStages) & 1, abort_flag)) return false;
         tc::fence_after_sync();
-        const uint32_t k_addr = tc::smem_u32(s_k + st * kTileBytes);
+        const uint32_t k_at = k_desc + st * (kTileBytes >> 4);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           if (kk < p.k_steps) {
-            const uint32_t off = (kk >> 2) * kBlkBytes + (kk & 3) * 32;
-            tc::umma_f16(tmem_base, tc::smem_desc(q_addr + off, 16, 1024),
-                         tc::smem_desc(k_addr + off, 16, 1024), p.idesc_qk, kk != 0 ? 1u : 0u);
+            const uint32_t off = ((kk >> 2) * kBlkBytes + (kk & 3) * 32) >> 4;
+            tc::umma_f16(tmem_base, tc::smem_desc_words(q_desc + off, kDescHi),
+                         tc::smem_desc_words(k_at + off, kDescHi), p.idesc_qk, kk != 0 ? 1u : 0u);
           }
         }
         tc::umma_commit(s_full);
@@ -276,11 +279,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           if (!tc::mbar_wait(&v_full[st], (t / kStages) & 1, abort_flag) ||
               !tc::mbar_wait(p_full, t & 1, abort_flag)) { ok = false; break; }
           tc::fence_after_sync();
-          const uint32_t v_addr = tc::smem_u32(s_v + st * kTileBytes);
+          const uint32_t v_at = v_desc + st * (kTileBytes >> 4);
 #pragma unroll
           for (int kk = 0; kk < kBlockN / 16; ++kk)
             tc::umma_f16_ts(tmem_base + kColO, tmem_base + kColP + kk * 8,
-                            tc::smem_desc(v_addr + kk * 2048, kBlkBytes, 1024), p.idesc_pv,
+                            tc::smem_desc_words(v_at + ((kk * 2048) >> 4), kDescHi), p.idesc_pv,
                             (j | kk) != 0 ? 1u : 0u);
           tc::umma_commit(pv_done);
           tc::umma_commit(&v_empty[st]);
@@ -542,6 +545,553 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   }
 }
 
+// Registers per thread of the warpgroups: issuing, softmax (two), O; together the 128 per thread that
+// 512 threads are launched with.
+constexpr int kFwdRegsIssue = 56, kFwdRegsSoftmax = 184, kFwdRegsO = 88;
+static_assert(kFwdRegsIssue + 2 * kFwdRegsSoftmax + kFwdRegsO <= 4 * 128, "more registers than the block has");
+
+// D in 65 .. 128
+struct GroupsSmem {
+  static constexpr int kTile = 128 * 128 * 2;        // one [128 x 128] 16-bit tile
+  static constexpr int kQ = 2;                       // Q tiles: this item's and the next one's
+  static constexpr int kStages = 2;                  // K and V rings
+  static constexpr int kK = kQ * kTile;
+  static constexpr int kV = kK + kStages * kTile;
+  // per softmax warp, twice (this tile's and the next one's): the tile's 128 key biases and the
+  // relative bias of the 32 + 128 - 1 distances between its queries and the tile's keys
+  static constexpr int kBiasFloats = 128 + 160;
+  static constexpr int kBias = kV + kStages * kTile;
+  static constexpr int kAlpha = kBias + 8 * 2 * kBiasFloats * 4;     // [group][tile parity][128] floats
+  static constexpr int kMl = kAlpha + 2 * 2 * 128 * 4;               // [group][item parity][128] float2
+  static constexpr int kBars = kMl + 2 * 2 * 128 * 8;
+  static constexpr int kTotal = kBars + 48 * 8 + 1024;
+};
+
+// The forward for D > 64 and more than one row tile: two softmax groups in one CTA that take the key tiles
+// of a work item in turn, each with an online softmax and an accumulator of its own, which a third group
+// of warps scales when maxima grow and merges at the end.  Loads, S and P V have a thread each.  One CTA of
+// flash_fwd_kernel has one softmax warp per scheduler at this width and keeps all of that on the chain of
+// a tile.  Bound now: S of a group waits for its P V (512 columns hold two S and two O, P lies over S),
+// 1900 of the 4700 cycles between two tiles of a group.
+// Measured, flash_fwd_kernel -> this (us): 4 x 2048 x 16 x 128 causal: 137 -> 116; 4 x 1000 x 32 x 80 causal with
+// key bias: 104 -> 76; 4 x 2048 x 16 x 128: 197 -> 158; 4 x 1024 x 16 x 128, p 0.1: 86 -> 62.  With a single row tile there are
+// too few tiles to share out: 2 x 60 x 60 x 8 x 128: 6.5 -> 8.0; 8 x 1 x 1500 keys x 16 x 128: 27 -> 29.
+template <bool kGeneral, typename T>
+__global__ void __launch_bounds__(512, 1)
+flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ FlashFwdParams p) {
+  using L = GroupsSmem;
+  constexpr int D = 128;
+  constexpr int kTileBytes = L::kTile;
+  constexpr int kStages = L::kStages, kQ = L::kQ;
+  constexpr int kBlkBytes = 128 * 128;      // one [128 rows x 64 cols] swizzled block
+  constexpr int kDBlocks = D / 64;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
+  uint64_t* q_full = bars;            // kQ (2)
+  uint64_t* q_empty = bars + 2;
+  uint64_t* k_full = bars + 4;        // kStages (<= 4)
+  uint64_t* k_empty = bars + 8;
+  uint64_t* v_full = bars + 12;
+  uint64_t* v_empty = bars + 16;
+  uint64_t* s_full = bars + 20;       // one per softmax group from here on: S of a tile is complete
+  uint64_t* p_full = bars + 22;       // [group][half of the keys]: P is in tensor memory (4 warps)
+  uint64_t* pv_done = bars + 26;      // O includes a tile
+  uint64_t* o_ready = bars + 28;      // O is scaled (or free) for a tile (4 warps)
+  uint64_t* alpha_ready = bars + 30;  // [group][tile parity]: a tile's factors (4 warps)
+  uint64_t* ml_ready = bars + 34;     // [group][item parity]: an item's maxima and sums (4 warps)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 38);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* s_alpha = reinterpret_cast<float*>(smem + L::kAlpha);
+  float2* s_ml = reinterpret_cast<float2*>(smem + L::kMl);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int diag = p.Sk - p.Sq;  // key j visible to query i iff j <= i + diag (causal)
+  constexpr uint32_t kTmemCols = 512;
+  // S and O of the two groups; P is written over S, whose next product then waits for the one that
+  // uses P up
+  constexpr uint32_t kColS = 0, kColO = 256;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&q_full[i], 1);
+      tc::mbar_init(&q_empty[i], 1);
+      tc::mbar_init(&s_full[i], 1);
+      tc::mbar_init(&pv_done[i], 1);
+      tc::mbar_init(&o_ready[i], 4);
+    }
+    for (int i = 0; i < kStages; ++i) {
+      tc::mbar_init(&k_full[i], 1);
+      tc::mbar_init(&k_empty[i], 1);
+      tc::mbar_init(&v_full[i], 1);
+      tc::mbar_init(&v_empty[i], 1);
+    }
+    for (int i = 0; i < 4; ++i) {
+      tc::mbar_init(&p_full[i], 4);
+      tc::mbar_init(&alpha_ready[i], 4);
+      tc::mbar_init(&ml_ready[i], 4);
+    }
+    *abort_flag = 0;
+    tc::fence_barrier_init();
+  }
+  if (warp == 1) {
+    tc::tmem_alloc(tmem_slot, kTmemCols);
+    tc::tmem_relinquish();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  const int items = p.walk.items() * p.splits;
+  // row tile, (batch, head) and key tiles [j0, j0 + n) of a work item
+  auto item_at = [&](int item, int& tile, int& bh, int& j0) {
+    const int unit = p.splits == 1 ? item : item / p.splits;
+    p.walk.at(unit, tile, bh);
+    int n = (p.Sk + kBlockN - 1) / kBlockN;
+    if (p.causal) {
+      const int last_key = min(p.Sk, min(tile * kBlockM + kBlockM, p.Sq) + diag);
+      n = max(1, min(n, (last_key + kBlockN - 1) / kBlockN));
+    }
+    j0 = 0;
+    if (p.splits > 1) {     // (one row tile per head: every split has at least one key tile)
+      j0 = (item - unit * p.splits) * p.tiles_per_split;
+      n = max(1, min(p.tiles_per_split, n - j0));
+    }
+    return n;
+  };
+
+  if (warp < 4) {
+    tc::regs_dec<kFwdRegsIssue>();
+    if (tc::elect_one()) {
+      constexpr uint32_t kDescHi = tc::smem_desc_hi(1024);
+      constexpr uint32_t kStep = kTileBytes >> 4;
+      bool ok = true;
+      if (warp == 0) {
+        // ------------------------------ loads ------------------------------
+        tc::tma_prefetch_desc(&tm_q);
+        tc::tma_prefetch_desc(&tm_k);
+        tc::tma_prefetch_desc(&tm_v);
+        Ring<kQ> q;
+        Ring<kStages> r;
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x, q.step()) {
+          int tile, bh, j0;
+          const int n = item_at(item, tile, bh, j0);
+          const int batch = bh / p.H, head = bh - batch * p.H;
+          ok = false;
+          if (!tc::mbar_wait(&q_empty[q.slot], q.phase ^ 1, abort_flag)) break;
+          tc::mbar_arrive_expect_tx(&q_full[q.slot], kTileBytes);
+#pragma unroll
+          for (int d = 0; d < kDBlocks; ++d)
+            tc::tma_load_4d(smem + q.slot * kTileBytes + d * kBlkBytes, &tm_q, &q_full[q.slot], d * 64, head,
+                            tile * kBlockM, batch);
+          for (int j = 0; j < n; ++j, r.step()) {
+            ok = false;
+            const int k0 = (j0 + j) * kBlockN;
+            if (!tc::mbar_wait(&k_empty[r.slot], r.phase ^ 1, abort_flag)) break;
+            tc::mbar_arrive_expect_tx(&k_full[r.slot], kTileBytes);
+#pragma unroll
+            for (int d = 0; d < kDBlocks; ++d)
+              tc::tma_load_4d(smem + L::kK + r.slot * kTileBytes + d * kBlkBytes, &tm_k, &k_full[r.slot], d * 64,
+                              head, k0, batch);
+            if (!tc::mbar_wait(&v_empty[r.slot], r.phase ^ 1, abort_flag)) break;
+            tc::mbar_arrive_expect_tx(&v_full[r.slot], kTileBytes);
+#pragma unroll
+            for (int d = 0; d < kDBlocks; ++d)
+              tc::tma_load_4d(smem + L::kV + r.slot * kTileBytes + d * kBlkBytes, &tm_v, &v_full[r.slot], d * 64,
+                              head, k0, batch);
+            ok = true;
+          }
+        }
+      } else if (warp == 1) {
+        // ------------------------------ S = Q K^T ------------------------------
+        const uint32_t q_desc = tc::smem_desc_lo(tc::smem_u32(smem), 16);
+        const uint32_t k_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kK), 16);
+        Ring<kQ> q;
+        Ring<kStages> r;
+        int u = 0;
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x, q.step()) {
+          int tile, bh, j0;
+          const int n = item_at(item, tile, bh, j0);
+          if (!tc::mbar_wait(&q_full[q.slot], q.phase, abort_flag)) break;
+          for (int j = 0; j < n; ++j, ++u, r.step()) {
+            const int g = u & 1;
+            ok = false;
+            if (!tc::mbar_wait(&k_full[r.slot], r.phase, abort_flag)) break;
+            if (u >= 2 && !tc::mbar_wait(&pv_done[g], ((u >> 1) & 1) ^ 1, abort_flag)) break;
+            tc::fence_after_sync();
+#pragma unroll
+            for (int kk = 0; kk < D / 16; ++kk) {
+              if (kk < p.k_steps) {
+                const uint32_t off = ((kk >> 2) * kBlkBytes + (kk & 3) * 32) >> 4;
+                tc::umma_f16(tmem_base + kColS + g * 128,
+                             tc::smem_desc_words(q_desc + q.slot * kStep + off, kDescHi),
+                             tc::smem_desc_words(k_desc + r.slot * kStep + off, kDescHi), p.idesc_qk,
+                             kk != 0 ? 1u : 0u);
+              }
+            }
+            tc::umma_commit(&s_full[g]);
+            tc::umma_commit(&k_empty[r.slot]);
+            if (j + 1 == n) tc::umma_commit(&q_empty[q.slot]);
+            ok = true;
+          }
+        }
+      } else if (warp == 2) {
+        // ------------------------------ O += P V ------------------------------
+        const uint32_t v_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kV), kBlkBytes);
+        Ring<kStages> r;
+        int u = 0;
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+          int tile, bh, j0;
+          const int n = item_at(item, tile, bh, j0);
+          for (int j = 0; j < n; ++j, ++u, r.step()) {
+            const int g = u & 1;
+            const uint32_t ph = (u >> 1) & 1;
+            ok = false;
+            if (!tc::mbar_wait(&v_full[r.slot], r.phase, abort_flag) ||
+                !tc::mbar_wait(&o_ready[g], ph, abort_flag))
+              break;
+            // the first half of the keys' products run under the other half's softmax
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              if (!tc::mbar_wait(&p_full[g * 2 + half], ph, abort_flag)) break;
+              tc::fence_after_sync();
+#pragma unroll
+              for (int kk = half * 4; kk < half * 4 + 4; ++kk)
+                tc::umma_f16_ts(tmem_base + kColO + g * D, tmem_base + kColS + g * 128 + kk * 8,
+                                tc::smem_desc_words(v_desc + r.slot * kStep + ((kk * 2048) >> 4), kDescHi),
+                                p.idesc_pv, (j >= 2 || kk != 0) ? 1u : 0u);
+            }
+            if (*abort_flag != 0) break;
+            tc::umma_commit(&pv_done[g]);
+            tc::umma_commit(&v_empty[r.slot]);
+            ok = true;
+          }
+        }
+      }
+    }
+  } else if (warp >= 12) {
+    tc::regs_dec<kFwdRegsO>();
+    // ------------------------------ O: scaled when maxima grow, read out at the end ------------------
+    const int quarter = warp & 3;
+    const int row_in_tile = quarter * 32 + lane;
+    const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    bool ok = true;
+    int u = 0;
+    int parts[2] = {0, 0};        // items that each group has had a part in
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+      int tile, bh, j0;
+      const int n = item_at(item, tile, bh, j0);
+      const int first = u;
+      for (int j = 0; j < n; ++j, ++u) {
+        const int g = u & 1, k = u >> 1;
+        if (j >= 2) {
+          if (!tc::mbar_wait_warp(&alpha_ready[g * 2 + (k & 1)], (k >> 1) & 1, abort_flag)) { ok = false; break; }
+          const float alpha = s_alpha[(g * 2 + (k & 1)) * 128 + row_in_tile];
+          if (__any_sync(0xffffffffu, alpha != 1.f)) {
+            if (!tc::mbar_wait_warp(&pv_done[g], (k & 1) ^ 1, abort_flag)) { ok = false; break; }
+            tc::fence_after_sync();
+            const uint64_t alpha2 = f2_pack(alpha, alpha);
+#pragma unroll 1
+            for (int c = 0; c < D / 32; ++c) {
+              uint32_t o[32];
+              tc::tmem_ld_x32(tmem_row + kColO + g * D + c * 32, o);
+              tc::tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; i += 2) f2_store(o + i, f2_mul(f2_load(o + i), alpha2));
+              tc::tmem_st_x32(tmem_row + kColO + g * D + c * 32, o);
+            }
+            tc::tmem_st_wait();
+            tc::fence_before_sync();
+          }
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&o_ready[g]);
+      }
+      if (!ok) break;
+      // both groups' maxima and sums, and their last products
+      float m_g[2], l_g[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        m_g[i] = -INFINITY;
+        l_g[i] = 0.f;
+        const int last = u - 1 - ((u - 1 - i) & 1);      // the group's last tile so far
+        if (last >= first) {
+          const int c = parts[i]++;
+          if (!tc::mbar_wait_warp(&ml_ready[i * 2 + (c & 1)], (c >> 1) & 1, abort_flag) ||
+              !tc::mbar_wait_warp(&pv_done[i], (last >> 1) & 1, abort_flag)) { ok = false; break; }
+          const float2 ml = s_ml[(i * 2 + (c & 1)) * 128 + row_in_tile];
+          m_g[i] = ml.x;
+          l_g[i] = ml.y;
+        }
+      }
+      if (!ok) break;
+      tc::fence_after_sync();
+      const float m = fmaxf(m_g[0], m_g[1]);
+      float f[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) f[i] = m_g[i] == -INFINITY ? 0.f : exp2f(m_g[i] - m);
+      const float l = f[0] * l_g[0] + f[1] * l_g[1];
+      const bool two = n > 1;
+      const int a = first & 1;                  // the group of the item's first tile
+      float fa = f[a], fb = f[a ^ 1];
+      const int row = tile * kBlockM + row_in_tile;
+      const int batch = bh / p.H, head = bh - batch * p.H;
+      // O of the item, columns c .. c + 15
+      auto columns = [&](int c, float (&v)[16]) {
+        uint32_t x[16], y[16];
+        tc::tmem_ld_x16(tmem_row + kColO + a * D + c, x);
+        if (two) tc::tmem_ld_x16(tmem_row + kColO + (a ^ 1) * D + c, y);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          v[i] = __uint_as_float(x[i]) * fa;
+          if (two) v[i] = fmaf(__uint_as_float(y[i]), fb, v[i]);
+        }
+      };
+      if (p.splits > 1) {
+        // this split's share: unnormalised output, maximum and sum
+        const int split = item - item / p.splits * p.splits;
+        const int64_t at = (static_cast<int64_t>(split) * p.B * p.H + bh) * p.Sq + min(row, p.Sq - 1);
+#pragma unroll 1
+        for (int c = 0; c < D; c += 16) {
+          float v[16];
+          columns(c, v);
+          if (row < p.Sq) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 8)
+              if (c + i < p.Dr) Vec8<float>::store(p.part_o + at * p.Dr + c + i, v + i);
+          }
+        }
+        if (row < p.Sq) p.part_ml[at] = make_float2(m, l);
+      } else {
+        const float inv = l > 0.f ? 1.f / (l * (1.f - p.p_drop)) : 0.f;
+        fa *= inv;
+        fb *= inv;
+        T* dst = static_cast<T*>(p.O) +
+                 ((static_cast<int64_t>(batch) * p.Sq + min(row, p.Sq - 1)) * p.H + head) * p.Dr;
+#pragma unroll 1
+        for (int c = 0; c < D; c += 16) {
+          float v[16];
+          columns(c, v);
+          if (row < p.Sq) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 8)      // padded columns are not part of the output
+              if (c + i < p.Dr) Vec8<T>::store(dst + c + i, v + i);
+          }
+        }
+        if (row < p.Sq)
+          p.lse[static_cast<int64_t>(bh) * p.Sq + row] =
+              l > 0.f ? (m == -INFINITY ? 0.f : m) * 0.6931471805599453f + logf(l) : -INFINITY;
+      }
+      tc::fence_before_sync();
+    }
+  } else {
+    tc::regs_inc<kFwdRegsSoftmax>();
+    // ------------------------------ softmax groups ------------------------------
+    const int quarter = warp & 3;
+    const int g = (warp - 4) >> 2;        // takes tiles g, g + 2, ... of the CTA's sequence
+    const int row_in_tile = quarter * 32 + lane;
+    const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    float* bias_buf = reinterpret_cast<float*>(smem + L::kBias) + (warp - 4) * 2 * L::kBiasFloats;
+    PhiloxUniform rng{};
+    if (p.p_drop > 0.f) rng = philox_uniform(p.rng);
+    const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
+    const int sk16 = (p.Sk + 15) >> 4;
+    // scores are brought to the log2 domain before the maximum only where something is added
+    // to them (or the scale would turn the maximum around)
+    const bool biased = kGeneral && (p.kbias != nullptr || p.rel != nullptr || !(p.scale_log2 > 0.f));
+    const float sc = biased ? 1.f : p.scale_log2;
+    // Biases of key tile `jt` of a work item on their way into buffer `buf`: copied a tile ahead,
+    // element by element (rows start anywhere).  What lies outside of the tensors is masked later.
+    auto fetch_bias = [&](int tile, int bh, int jt, int buf) {
+      float* dst = bias_buf + buf * L::kBiasFloats;
+      const int batch = bh / p.H, head = bh - batch * p.H, k0 = jt * kBlockN;
+      if (p.kbias != nullptr) {
+        const float* src = p.kbias + static_cast<int64_t>(batch) * p.Sk;
+#pragma unroll
+        for (int i = lane; i < 128; i += 32) cp_async4(dst + i, src + min(k0 + i, p.Sk - 1));
+      }
+      if (p.rel != nullptr) {
+        // key - query from that of the warp's last row and the first key on
+        const float* src = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + p.Sq - 1;
+        const int d0 = k0 - (tile * kBlockM + quarter * 32 + 31);
+#pragma unroll
+        for (int i = lane; i < 160; i += 32)
+          cp_async4(dst + 128 + i, src + max(1 - p.Sq, min(d0 + i, p.Sk - 1)));
+      }
+    };
+    // a tile of the sequence: key tile j0 + j of a work item (j < n), u0 is the item's first
+    struct Pos {
+      int item, tile, bh, j0, n, j, u0;
+    };
+    // the group's first one from sequence number pos.u0 and work item pos.item on
+    auto enter = [&](Pos& pos) {
+      while (pos.item < items) {
+        pos.n = item_at(pos.item, pos.tile, pos.bh, pos.j0);
+        pos.j = (pos.u0 & 1) ^ g;
+        if (pos.j < pos.n) return;
+        pos.u0 += pos.n;
+        pos.item += gridDim.x;
+      }
+    };
+    Pos pos{};
+    pos.item = blockIdx.x;
+    enter(pos);
+    if (biased && pos.item < items) fetch_bias(pos.tile, pos.bh, pos.j0 + pos.j, 0);
+    bool ok = true;
+    uint32_t k = 0, part = 0;       // tiles and items of the group so far
+    while (pos.item < items && ok) {
+      const int row = pos.tile * kBlockM + row_in_tile;
+      const uint64_t drop_row = (static_cast<uint64_t>(pos.bh) * p.Sq + min(row, p.Sq - 1)) * sk16;
+      float m_ref = -INFINITY;
+      uint64_t l2 = 0;      // two fp32 partial row sums
+      Pos next = pos;
+      for (; pos.j < pos.n; pos.j += 2, ++k) {
+        const uint32_t ph = k & 1;
+        const int k0 = (pos.j0 + pos.j) * kBlockN;
+        const float* bias = bias_buf + ph * L::kBiasFloats;
+        if (pos.j + 2 >= pos.n) {
+          next.u0 += pos.n;
+          next.item += gridDim.x;
+          enter(next);
+        } else {
+          next.j = pos.j + 2;
+        }
+        if (kGeneral && biased) {
+          cp_async_wait();
+          if (p.kbias != nullptr) {
+#pragma unroll
+            for (int i = lane; i < 128; i += 32)      // (the elements that this lane copied)
+              bias_buf[ph * L::kBiasFloats + i] *= kLog2e;
+          }
+          // this tile's biases are visible to the warp, and the other buffer's readers are done
+          __syncwarp();
+          if (next.item < items) fetch_bias(next.tile, next.bh, next.j0 + next.j, ph ^ 1);
+        }
+        if (!tc::mbar_wait_warp(&s_full[g], ph, abort_flag)) { ok = false; break; }
+        tc::fence_after_sync();
+        uint32_t raw[4][32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tc::tmem_ld_x32(tmem_row + kColS + g * 128 + c * 32, raw[c]);
+        tc::tmem_ld_wait();
+        if constexpr (kGeneral) {
+          if (biased) {
+            const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2);
+            const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
+            if (p.kbias != nullptr) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {
+                  const float4 b = *reinterpret_cast<const float4*>(bias + c * 32 + i);
+                  f2_store(raw[c] + i, f2_fma(f2_load(raw[c] + i), scale2, f2_pack(b.x, b.y)));
+                  f2_store(raw[c] + i + 2, f2_fma(f2_load(raw[c] + i + 2), scale2, f2_pack(b.z, b.w)));
+                }
+            } else {
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) f2_store(raw[c] + i, f2_mul(f2_load(raw[c] + i), scale2));
+            }
+            if (p.rel != nullptr) {
+              // neighbouring lanes (queries) read neighbouring words
+              const float* rel = bias + 128 + 31 - lane;
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int i = 0; i < 32; i += 2)
+                  f2_store(raw[c] + i, f2_fma(f2_pack(rel[c * 32 + i], rel[c * 32 + i + 1]), log2e2,
+                                              f2_load(raw[c] + i)));
+            }
+          }
+          const int first_limit = p.causal ? min(p.Sk, pos.tile * kBlockM + quarter * 32 + diag + 1) : p.Sk;
+          if (k0 + kBlockN > first_limit) {     // some lane of the warp masks something
+            const int limit = (p.causal ? min(p.Sk, row + diag + 1) : p.Sk) - k0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const uint32_t seen = low_bits(limit - c * 32);
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (!(seen & (1u << i))) raw[c][i] = 0xff800000u;   // -inf
+            }
+          }
+        }
+        float mm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // 4 chains for ILP
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; i += 2)
+            mm[c] = fmaxf(mm[c], fmaxf(__uint_as_float(raw[c][i]), __uint_as_float(raw[c][i + 1])));
+        const float m_new = fmaxf(m_ref, fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3])) * sc);
+        const float alpha = m_new == m_ref ? 1.f : exp2f(m_ref - m_new);
+        s_alpha[(g * 2 + ph) * 128 + row_in_tile] = alpha;
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&alpha_ready[g * 2 + ph]);
+        l2 = f2_mul(l2, f2_pack(alpha, alpha));
+        m_ref = m_new;
+        const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+        const uint64_t sc2 = f2_pack(sc, sc), nm2 = f2_pack(-m_use, -m_use);
+        uint64_t la = l2, lb = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const uint64_t x = f2_fma(f2_load(raw[c] + 2 * i), sc2, nm2);
+            float a, b;
+            f2_unpack(x, a, b);
+            a = exp2f(a);
+            b = exp2f(b);
+            if (i & 1) lb = f2_add(lb, f2_pack(a, b));
+            else la = f2_add(la, f2_pack(a, b));
+            pk[i] = pack16<T>(a, b);
+          }
+          if (p.p_drop > 0.f) {
+            // dropped probabilities are cleared in the packed 16-bit pairs
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const uint4 kw = philox_keep16(rng, drop_row + ((k0 + c * 32 + h * 16) >> 4), add4);
+              const uint32_t wd[4] = {kw.x, kw.y, kw.z, kw.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                pk[h * 8 + i * 2 + 0] &= keep_mask_pair(wd[i], 0);
+                pk[h * 8 + i * 2 + 1] &= keep_mask_pair(wd[i], 1);
+              }
+            }
+          }
+          tc::tmem_st_x16(tmem_row + kColS + g * 128 + c * 16, pk);
+          if (c & 1) {
+            tc::tmem_st_wait();
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&p_full[g * 2 + (c >> 1)]);
+          }
+        }
+        l2 = f2_add(la, lb);
+      }
+      if (!ok) break;
+      float l_run, l_hi;
+      f2_unpack(l2, l_run, l_hi);
+      s_ml[(g * 2 + (part & 1)) * 128 + row_in_tile] = make_float2(m_ref, l_run + l_hi);
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&ml_ready[g * 2 + (part & 1)]);
+      ++part;
+      pos = next;
+    }
+    if (kGeneral) cp_async_wait();      // (a give-up leaves copies under way)
+  }
+
+  tc::fence_before_sync();
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag != 0 && p.status != nullptr) atomicExch(p.status, 2);
+  if (warp == 1) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
 // Output and log-sum-exp of rows whose keys were split over work items: one warp per row, lanes
 // along d (8 per thread for the 16 lanes that D = 128 needs, the other half idle).
 template <typename T>
@@ -603,6 +1153,24 @@ void launch_flash_dropout_mask(uint8_t* mask, int B, int H, int Sq, int Sk, floa
   flash_dropout_mask_kernel<<<sm_count() * 4, 256, 0, stream>>>(mask, B, H, Sq, Sk, p_drop, rng);
 }
 
+template <bool kGeneral, typename T>
+static int launch_fwd_groups(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+                             const FlashFwdParams& p, int64_t items, cudaStream_t stream) {
+  constexpr int kSmem = GroupsSmem::kTotal;
+  static_assert(kSmem <= 227 * 1024, "flash forward: shared memory over the per-CTA limit");
+  auto kernel = flash_fwd_groups_kernel<kGeneral, T>;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
+        cudaSuccess)
+      return 3;
+    configured = true;
+  }
+  count_launch();
+  kernel<<<static_cast<int>(items < sm_count() ? items : sm_count()), 512, kSmem, stream>>>(tq, tk, tv, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
 template <int D, bool kGeneral, typename T>
 static int launch_fwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                         const FlashFwdParams& p, cudaStream_t stream) {
@@ -617,6 +1185,7 @@ static int launch_fwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
     configured = true;
   }
   const int64_t items = static_cast<int64_t>(p.walk.row_tiles) * p.walk.nbh * p.splits;
+  if (D == 128 && p.walk.row_tiles > 1) return launch_fwd_groups<kGeneral, T>(tq, tk, tv, p, items, stream);
   const int64_t cap = FwdSmem<D>::kCtas * sm_count();
   count_launch();
   kernel<<<static_cast<int>(items < cap ? items : cap), 192, kSmem, stream>>>(tq, tk, tv, p);

@@ -151,16 +151,6 @@ struct BwdSmem {
   static constexpr int kTotal = kBars + 48 * 8 + 1024;
 };
 
-// Position in a ring of N slots
-template <int N>
-struct Ring {
-  int slot = 0;
-  uint32_t phase = 0;
-  __device__ __forceinline__ void step() {
-    if (++slot == N) { slot = 0; phase ^= 1; }
-  }
-};
-
 // 16 warps in four warpgroups: one thread each of warps 0 - 3 for the loads and the products; two
 // softmax groups (warps 4 - 7 and 8 - 11), one row per thread, which take the half tiles in turn; and
 // the warps that read the accumulators out (12 - 15).

@@ -137,6 +137,16 @@ __device__ __forceinline__ uint4 philox_keep16(const PhiloxUniform& s, uint64_t 
   return c;
 }
 
+// Position in a ring of N slots
+template <int N>
+struct Ring {
+  int slot = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void step() {
+    if (++slot == N) { slot = 0; phase ^= 1; }
+  }
+};
+
 // Row tiles of 128 of all (batch, head) pairs, walked by a persistent grid.  Under a causal
 // mask the tiles differ in cost: they are ordered by cost, heaviest first, over all heads.
 // Otherwise the tiles of one head are neighbours, so that the tensors they share stay in L2.
