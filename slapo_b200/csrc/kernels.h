@@ -65,9 +65,10 @@ void launch_rel_bias_bwd(const float* grad, const int64_t* buckets, void* dtable
                          int n_buckets, int dtype, cudaStream_t stream);
 
 // Cross entropy in two steps (per-row statistics, then gradient); see loss.cu.
-void launch_ce_stats(const void* logits, const int64_t* labels, float* stats, int rows, int cols,
-                     int64_t row_stride, int vocab_start, int64_t ignore_index, int dtype,
-                     cudaStream_t stream);
+// stats [rows, 3], or null and loss, lse [rows]
+void launch_ce_stats(const void* logits, const int64_t* labels, float* stats, float* loss, float* lse,
+                     int rows, int cols, int64_t row_stride, int vocab_start, int64_t ignore_index,
+                     int dtype, cudaStream_t stream);
 void launch_ce_grad(const void* logits, const int64_t* labels, const float* lse,
                     const float* coef, void* grad, int rows, int cols, int64_t row_stride,
                     int vocab_start, int64_t ignore_index, int dtype, cudaStream_t stream);

@@ -8,42 +8,94 @@
 //              stats[row] = (max, sum exp(x - max), logit of the target if it
 //              lies in this slice else 0).  Rows whose label is the ignore
 //              index are not read at all.
+//              On one GPU it writes the row's loss and log-sum-exp instead.
 //   (group)    the caller combines the three numbers over the group
 //              (MAX / rescaled SUM / SUM) - nothing to do on one GPU.
 //   ce_grad    grad[row, :] = (exp(x - lse) - onehot(target)) * coef[row],
 //              written in the logits' dtype; ignored rows get zeros.
-#include "common.cuh"
+#include "flash_common.cuh"
 #include "kernels.h"
 
 namespace slapo {
 
+// 16-byte vectors that a thread has in flight.  Bound by reading the logits (8192 x 50304 bf16: 824 MB, 126 us) and
+// close to it by the exponentials (92 us of the special-function unit): with one vector at a time, its own
+// rescaling and scalar arithmetic 161 us, so 141; loss and log-sum-exp from here instead of eight small kernels
+// and the gradient from the last row on, 460 -> 396 us for the loss and its gradient.
+constexpr int kCeUnroll = 4;
+
+// Maximum and sum of exp(x - maximum) of kCeUnroll vectors of 8, added to a thread's running pair: one
+// rescaling for all of them, products and sums on pairs of values.
+__device__ __forceinline__ void ce_add(const float (&v)[kCeUnroll][8], float& m, float& s) {
+  float cm = v[0][0];
+#pragma unroll
+  for (int u = 0; u < kCeUnroll; ++u)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) cm = fmaxf(cm, v[u][k]);
+  const float nm = fmaxf(m, cm);
+  const float shift = nm == -INFINITY ? 0.f : -nm * kLog2e;
+  const uint64_t scale2 = f2_pack(kLog2e, kLog2e), shift2 = f2_pack(shift, shift);
+  uint64_t acc[2] = {0, 0};
+#pragma unroll
+  for (int u = 0; u < kCeUnroll; ++u)
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      float a, b;
+      f2_unpack(f2_fma(f2_pack(v[u][k], v[u][k + 1]), scale2, shift2), a, b);
+      acc[(k >> 1) & 1] = f2_add(acc[(k >> 1) & 1], f2_pack(exp2f(a), exp2f(b)));
+    }
+  float a, b;
+  f2_unpack(f2_add(acc[0], acc[1]), a, b);
+  s = s * exp2f(fmaf(m, kLog2e, shift)) + (a + b);
+  m = nm;
+}
+
+// stats: (max, sum, target logit) per row, or null: then loss and lse of each row instead.
 template <typename T>
 __global__ void __launch_bounds__(256) ce_stats_kernel(
     const T* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ stats,
-    int rows, int cols, int64_t row_stride, int vocab_start, int64_t ignore_index) {
+    float* __restrict__ loss, float* __restrict__ lse, int rows, int cols, int64_t row_stride,
+    int vocab_start, int64_t ignore_index) {
   __shared__ float red_m[8], red_s[8];
   const int row = blockIdx.x;
   if (row >= rows) return;
   const int64_t label = labels[row];
   float* out = stats + static_cast<int64_t>(row) * 3;
   if (label == ignore_index) {
-    if (threadIdx.x == 0) { out[0] = -INFINITY; out[1] = 0.f; out[2] = 0.f; }
+    if (threadIdx.x == 0) {
+      if (stats != nullptr) {
+        out[0] = -INFINITY;
+        out[1] = 0.f;
+        out[2] = 0.f;
+      } else {
+        loss[row] = 0.f;
+        lse[row] = 0.f;
+      }
+    }
     return;
   }
   const T* x = logits + static_cast<int64_t>(row) * row_stride;
   float m = -INFINITY, s = 0.f;
-  for (int c = threadIdx.x * 8; c < cols; c += blockDim.x * 8) {
-    float v[8];
-    Vec8<T>::load(x + c, v);
-    float cm = v[0];
+  const int step = blockDim.x * 8;
+  int c = threadIdx.x * 8;
+  for (; c + (kCeUnroll - 1) * step < cols; c += kCeUnroll * step) {
+    float v[kCeUnroll][8];
 #pragma unroll
-    for (int k = 1; k < 8; ++k) cm = fmaxf(cm, v[k]);
-    const float nm = fmaxf(m, cm);
-    float acc = 0.f;
+    for (int u = 0; u < kCeUnroll; ++u) Vec8<T>::load(x + c + u * step, v[u]);
+    ce_add(v, m, s);
+  }
+  if (c < cols) {
+    float v[kCeUnroll][8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) acc += __expf(v[k] - nm);
-    s = s * __expf(m - nm) + acc;
-    m = nm;
+    for (int u = 0; u < kCeUnroll; ++u) {
+      if (c + u * step < cols) {
+        Vec8<T>::load(x + c + u * step, v[u]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[u][k] = -INFINITY;
+      }
+    }
+    ce_add(v, m, s);
   }
   // combine (m, s) over the CTA
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -68,7 +120,15 @@ __global__ void __launch_bounds__(256) ce_stats_kernel(
     const int64_t local = label - vocab_start;
     float picked = 0.f;
     if (local >= 0 && local < cols) picked = static_cast<float>(x[local]);
-    out[0] = fm; out[1] = fs; out[2] = picked;
+    if (stats != nullptr) {
+      out[0] = fm;
+      out[1] = fs;
+      out[2] = picked;
+    } else {
+      const float l = fm + static_cast<float>(log(static_cast<double>(fs)));
+      lse[row] = l;
+      loss[row] = l - picked;
+    }
   }
 }
 
@@ -77,8 +137,8 @@ __global__ void __launch_bounds__(256) ce_grad_kernel(
     const T* __restrict__ logits, const int64_t* __restrict__ labels,
     const float* __restrict__ lse, const float* __restrict__ coef, T* __restrict__ grad, int rows,
     int cols, int64_t row_stride, int vocab_start, int64_t ignore_index) {
-  const int row = blockIdx.x;
-  if (row >= rows) return;
+  // last rows first: those are what the statistics have left in L2
+  const int row = rows - 1 - static_cast<int>(blockIdx.x);
   const int64_t label = labels[row];
   T* g = grad + static_cast<int64_t>(row) * row_stride;
   if (label == ignore_index) {
@@ -148,13 +208,13 @@ __global__ void __launch_bounds__(256) sq_norm_kernel(const T* __restrict__ x,
     default: { using T = float; __VA_ARGS__; break; }                \
   }
 
-void launch_ce_stats(const void* logits, const int64_t* labels, float* stats, int rows, int cols,
-                     int64_t row_stride, int vocab_start, int64_t ignore_index, int dtype,
-                     cudaStream_t stream) {
+void launch_ce_stats(const void* logits, const int64_t* labels, float* stats, float* loss, float* lse,
+                     int rows, int cols, int64_t row_stride, int vocab_start, int64_t ignore_index,
+                     int dtype, cudaStream_t stream) {
   if (rows == 0) return;
   count_launch();
   DISPATCH_DTYPE(dtype, (ce_stats_kernel<T><<<rows, 256, 0, stream>>>(
-      static_cast<const T*>(logits), labels, stats, rows, cols, row_stride, vocab_start,
+      static_cast<const T*>(logits), labels, stats, loss, lse, rows, cols, row_stride, vocab_start,
       ignore_index)));
 }
 

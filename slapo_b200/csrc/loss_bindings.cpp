@@ -36,10 +36,23 @@ Tensor ce_stats(const Tensor& logits, const Tensor& labels, int64_t vocab_start,
   c10::cuda::CUDAGuard guard(logits.device());
   Tensor stats = at::empty({logits.size(0), 3}, logits.options().dtype(at::kFloat));
   slapo::launch_ce_stats(logits.data_ptr(), labels.data_ptr<int64_t>(), stats.data_ptr<float>(),
-                         static_cast<int>(logits.size(0)), static_cast<int>(logits.size(1)),
+                         nullptr, nullptr, static_cast<int>(logits.size(0)), static_cast<int>(logits.size(1)),
                          logits.stride(0), static_cast<int>(vocab_start), ignore_index,
                          dtype_code(logits), at::cuda::getCurrentCUDAStream().stream());
   return stats;
+}
+
+// (loss, log-sum-exp) per row of logits that are not sharded; zeros for ignored rows
+std::tuple<Tensor, Tensor> ce_loss(const Tensor& logits, const Tensor& labels, int64_t ignore_index) {
+  check_logits(logits, labels);
+  c10::cuda::CUDAGuard guard(logits.device());
+  Tensor loss = at::empty({logits.size(0)}, logits.options().dtype(at::kFloat));
+  Tensor lse = at::empty_like(loss);
+  slapo::launch_ce_stats(logits.data_ptr(), labels.data_ptr<int64_t>(), nullptr, loss.data_ptr<float>(),
+                         lse.data_ptr<float>(), static_cast<int>(logits.size(0)),
+                         static_cast<int>(logits.size(1)), logits.stride(0), 0, ignore_index,
+                         dtype_code(logits), at::cuda::getCurrentCUDAStream().stream());
+  return {loss, lse};
 }
 
 Tensor ce_grad(const Tensor& logits, const Tensor& labels, const Tensor& lse, const Tensor& coef,
@@ -77,6 +90,7 @@ Tensor sq_norm(const Tensor& x, const c10::optional<Tensor>& mask) {
 void register_loss_ops(torch::Library& m) {
   m.def("ce_stats(Tensor logits, Tensor labels, int vocab_start, int ignore_index) -> Tensor",
         &ce_stats);
+  m.def("ce_loss(Tensor logits, Tensor labels, int ignore_index) -> (Tensor, Tensor)", &ce_loss);
   m.def("ce_grad(Tensor logits, Tensor labels, Tensor lse, Tensor coef, int vocab_start, int ignore_index) -> Tensor",
         &ce_grad);
   m.def("sq_norm(Tensor x, Tensor? mask) -> Tensor", &sq_norm);

@@ -91,21 +91,24 @@ class _FusedCrossEntropy(torch.autograd.Function):
         logits2 = logits.reshape(-1, logits.shape[-1])
         target1 = target.reshape(-1).contiguous()
         lo = rank * logits2.shape[-1]
+        ctx.lo, ctx.ignore_index, ctx.logits_shape = lo, ignore_index, logits.shape
+        if world == 1:
+            loss, lse = native.ops().ce_loss(logits2, target1, ignore_index)
+            ctx.save_for_backward(logits2, target1, lse)
+            return loss.view(shape)
         stats = native.ops().ce_stats(logits2, target1, lo, ignore_index)
         row_max, sum_exp, picked = stats[:, 0], stats[:, 1], stats[:, 2]
-        if world > 1:
-            gmax = row_max.clone()
-            dist.all_reduce(gmax, op=dist.ReduceOp.MAX, group=group)
-            scale = torch.where(row_max == float("-inf"), torch.zeros_like(row_max),
-                                (row_max - gmax).exp())
-            packed = torch.stack([sum_exp * scale, picked], dim=0)
-            dist.all_reduce(packed, group=group)
-            sum_exp, picked, row_max = packed[0], packed[1], gmax
+        gmax = row_max.clone()
+        dist.all_reduce(gmax, op=dist.ReduceOp.MAX, group=group)
+        scale = torch.where(row_max == float("-inf"), torch.zeros_like(row_max),
+                            (row_max - gmax).exp())
+        packed = torch.stack([sum_exp * scale, picked], dim=0)
+        dist.all_reduce(packed, group=group)
+        sum_exp, picked, row_max = packed[0], packed[1], gmax
         valid = target1 != ignore_index
         lse = torch.where(valid, row_max + sum_exp.log(), torch.zeros_like(row_max))
         loss = torch.where(valid, lse - picked, torch.zeros_like(lse))
         ctx.save_for_backward(logits2, target1, lse)
-        ctx.lo, ctx.ignore_index, ctx.logits_shape = lo, ignore_index, logits.shape
         return loss.view(shape)
 
     @staticmethod

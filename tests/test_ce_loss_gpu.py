@@ -1,0 +1,33 @@
+"""Loss and log-sum-exp of unsharded logits from one kernel: columns around its unrolled step (four times
+256 threads of 8), ignored rows, labels outside of the vocabulary and hidden logits."""
+import pytest
+import torch
+
+from slapo_b200.ops import cross_entropy as ce
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (5, 2040), (3, 2056), (4, 8192), (7, 8200), (2, 50304)])
+def test_loss_and_gradient(rows, cols, dtype):
+    torch.manual_seed(rows + cols)
+    x = (torch.randn(rows, cols, device="cuda") * 3).to(dtype)
+    if cols > 64:
+        x[0, 8:cols // 2] = float("-inf")        # whole vectors of a thread among them
+    labels = torch.randint(0, 8, (rows,), device="cuda")
+    if rows > 2:
+        labels[1] = -100
+    x.requires_grad_()
+    loss = ce.cross_entropy(x, labels)
+    coef = torch.rand(rows, device="cuda")
+    loss.backward(coef)
+    want = torch.nn.functional.cross_entropy(x.detach().double(), labels, reduction="none",
+                                             ignore_index=-100)
+    # fp32: one rounding of sums of up to 50304 terms, which exp2's own 2e-7 relative dominates
+    torch.testing.assert_close(loss.double(), want, rtol=2e-6, atol=2e-6)
+    p = torch.softmax(x.detach().double(), -1)
+    p[torch.arange(rows, device="cuda"), labels.clamp(min=0)] -= 1
+    p = p * (coef.double() * (labels != -100))[:, None]
+    err = ((x.grad.double() - p).norm() / p.norm()).item()
+    assert err < {torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10, torch.float32: 5e-6}[dtype]
