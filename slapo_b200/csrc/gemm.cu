@@ -17,6 +17,7 @@
 // (bias, activation) and store 16-byte vectors.  All hand-offs are mbarriers;
 // every wait is bounded and reports through a device status word.
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
 #include "kernels.h"
 #include "tc05.cuh"
 
@@ -85,6 +86,9 @@ struct GemmParams {
   int out_bf16;       // 1 bf16, 0 fp16
   uint32_t idesc;
   int* status;        // device error word (0 = ok)
+  void* C2;           // kEpi forward: acc + bias, or nullptr
+  const void* Z;      // kEpi backward: input (ReLU: output) of the activation, as C in memory
+  float* col_part;    // kEpi backward: column sums over 32 rows each, or nullptr
 };
 
 constexpr int BM = 128;
@@ -112,7 +116,8 @@ __device__ __forceinline__ float load_bias(const void* bias, int col, int out_bf
   return __half2float(static_cast<const __half*>(bias)[col]);
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN>
+// kEpi: what rides in the epilogue (gemm_epilogue.cuh); kEpiPlain: bias and ReLU
+template <int BN, int STAGES, bool A_MN, bool B_MN, int kEpi>
 __global__ void __launch_bounds__(192, 1)
 gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                  const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
@@ -240,10 +245,25 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
+        const int col0 = n0 + c * 32;
+        if constexpr (kEpi != kEpiPlain) {
+          uint32_t aux[16];
+          if constexpr (epi_backward(kEpi))
+            load_row32(p.Z, static_cast<int64_t>(row) * p.ldc + col0, col0, p.N, row < p.M, aux);
+          else
+            load_row32(p.bias, col0, col0, p.N, p.bias != nullptr, aux);
+          uint32_t r[32];
+          tc::tmem_ld_x32(t_row + c * 32, r);
+          tc::tmem_ld_wait();
+          float v[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+          if (col0 < p.N) epi_finish<kEpi>(p, v, aux, m0 + quarter * 32, lane, col0, false);
+          continue;
+        }
         uint32_t r[32];
         tc::tmem_ld_x32(t_row + c * 32, r);
         tc::tmem_ld_wait();
-        const int col0 = n0 + c * 32;
         if (row < p.M && col0 < p.N) {
           uint32_t packed[16];
 #pragma unroll
@@ -318,11 +338,11 @@ bool cached_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t
   return true;
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN>
+template <int BN, int STAGES, bool A_MN, bool B_MN, int kEpi = kEpiPlain>
 static int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
                           cudaStream_t stream) {
   using S = GemmSmem<BN, STAGES>;
-  auto kernel = gemm_tc05_kernel<BN, STAGES, A_MN, B_MN>;
+  auto kernel = gemm_tc05_kernel<BN, STAGES, A_MN, B_MN, kEpi>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal) !=
@@ -340,7 +360,7 @@ static int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const Ge
 // Returns 0 on success; >0 = host-side refusal (bad shape / alignment / driver).
 int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
                 int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act, int bn,
-                int* status, cudaStream_t stream) {
+                int* status, cudaStream_t stream, const GemmEpi* epi) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (N % 8 || K % 8 || lda % 8 || ldb % 8 || ldc % 8) return 1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) |
@@ -360,6 +380,28 @@ int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, 
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.bias = bias; p.act = act;
   p.out_bf16 = bf16 ? 1 : 0; p.status = status;
   p.idesc = tc::instr_desc_f16(BM, BN, bf16 ? 1 : 0, a_mn, b_mn);
+  p.C2 = epi != nullptr ? epi->c2 : nullptr;
+  p.Z = epi != nullptr ? epi->z : nullptr;
+  p.col_part = epi != nullptr ? epi->col_part : nullptr;
+  if (epi != nullptr && epi->kind != kEpiPlain) {
+    if (a_mn) return 1;
+    if ((reinterpret_cast<uintptr_t>(p.Z) | reinterpret_cast<uintptr_t>(p.C2) |
+         reinterpret_cast<uintptr_t>(p.bias)) & 15)
+      return 1;
+#define GEMM_EPI(BN_, ST_, KIND_)                                                       \
+  if (BN == BN_ && epi->kind == KIND_)                                                  \
+    return b_mn ? launch_variant<BN_, ST_, false, true, KIND_>(ta, tb, p, stream)       \
+                : launch_variant<BN_, ST_, false, false, KIND_>(ta, tb, p, stream);
+#define GEMM_EPIS(BN_, ST_)                                                      \
+  GEMM_EPI(BN_, ST_, kEpiGelu) GEMM_EPI(BN_, ST_, kEpiGeluTanh)                  \
+  GEMM_EPI(BN_, ST_, kEpiGeluBwd) GEMM_EPI(BN_, ST_, kEpiGeluTanhBwd) GEMM_EPI(BN_, ST_, kEpiReluBwd)
+    GEMM_EPIS(256, 4)
+    GEMM_EPIS(128, 6)
+    GEMM_EPIS(64, 8)
+#undef GEMM_EPIS
+#undef GEMM_EPI
+    return 1;
+  }
 
 #define GEMM_CASE(BN_, ST_)                                                              \
   if (BN == BN_) {                                                                       \

@@ -21,6 +21,7 @@
 // a tile, each stores its partial accumulator into its own fp32 slice of a workspace; a
 // second, memory-bound kernel adds the slices, applies bias / activation and writes C.
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
 #include "kernels.h"
 #include "tc05.cuh"
 
@@ -39,6 +40,8 @@ struct Gemm2Params {
   int kb_per_split;
   float* workspace;   // [splits, M, N] fp32 scratch (splits > 1), any contents
   int* status;
+  const void* Z;      // kEpi backward: input (ReLU: output) of the activation, as C in memory
+  float* col_part;    // kEpi backward: column sums over 32 rows each, or nullptr
   int wide_store;     // rows of C are 32-byte aligned: the epilogue stores whole sectors
 };
 
@@ -146,7 +149,8 @@ __device__ __forceinline__ void g2_finish_store(const Gemm2Params& p, const floa
   }
 }
 
-template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN>
+// kEpi: what rides in the epilogue (gemm_epilogue.cuh); kEpiPlain: bias and ReLU
+template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN, int kEpi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * kEpiWarps, 1)
 gemm2_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                   const __grid_constant__ CUtensorMap tmap_b, const Gemm2Params p) {
@@ -305,7 +309,28 @@ gemm2_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
       tc::fence_after_sync();
       const int row = m0 + quarter * 32 + lane;
       const uint32_t t_row = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
-      if (p.splits == 1) {
+      if constexpr (kEpi != kEpiPlain) {
+        const int row0 = m0 + quarter * 32;
+#pragma unroll 1
+        for (int c = c_begin; c < c_end; ++c) {
+          const int col0 = n0 + c * 32;
+          uint32_t aux[16];
+          if constexpr (epi_backward(kEpi))
+            load_row32(p.Z, static_cast<int64_t>(row) * p.ldc + col0, col0, p.N, row < p.M, aux);
+          else
+            g2_load_bias(p, col0, aux);
+          uint32_t r[32];
+          tc::tmem_ld_x32(t_row + c * 32, r);
+          tc::tmem_ld_wait();
+          float v[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+          if (col0 < p.N) epi_finish<kEpi>(p, v, aux, row0, lane, col0, p.wide_store != 0);
+        }
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive_cluster(tc::map_to_cta(tc::smem_u32(&tmem_empty[acc]), 0));
+      } else if (p.splits == 1) {
         // One tensor-memory load at a time on purpose: reading ahead (two register sets, or
         // 64 columns per load) measured 20 - 30 % slower on whole GEMMs - the epilogue's
         // reads compete with the accumulator traffic of the MMAs that run under it.  Only the
@@ -414,11 +439,11 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const Gemm2Params p)
 bool cached_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer,
                     uint64_t stride, uint32_t box_outer, bool bf16);
 
-template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN>
+template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN, int kEpi = kEpiPlain>
 static int launch_pair_variant(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm2Params& p,
                                cudaStream_t stream) {
   using S = Gemm2Smem<BN, STAGES, KSUB>;
-  auto kernel = gemm2_tc05_kernel<BN, STAGES, KSUB, A_MN, B_MN>;
+  auto kernel = gemm2_tc05_kernel<BN, STAGES, KSUB, A_MN, B_MN, kEpi>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal) !=
@@ -459,19 +484,19 @@ int gemm2_splits(int M, int N, int K, int bn) {
 // Small products are one wave of few tiles, whatever the tile: the launch, the first loads and
 // the epilogue of ONE tile are what they take, and narrow tiles have less of all three and put
 // more SMs on the weights.  Measured per call (us, B in L2; wide = the tile that large products
-// use, 256 x 256 per pair or, up to 128 rows, 128 x 256):
+// use, 256 x 256 per pair or, up to 128 rows, 128 x 256; - not measured with products issued as now):
 //     M x N x K             128 x 64   256 x 128 pair   wide
-//     8 x 2048 x 2048         12.9           -          14.5
-//     200 x 3072 x 768         8.0          9.4         12.0
-//     512 x 1024 x 1024        8.6         10.4         13.3
-//     768 x 768 x 64           4.4          7.1          9.2
-//     384 x 4096 x 1024       14.4         10.8         13.7
-//     2048 x 1024 x 4096      43.0         23.1         27.5
-//     1024 x 3072 x 1024      20.1         14.9         13.9
-// So: tiles of 64 columns while they fit one wave of CTAs and the contraction is short (a narrow
-// tile pays more per step of it: 18.3 against 17.6 us at 200 x 768 x 3072), pairs of 128 columns
-// while those fit one wave of pairs, wide tiles beyond.  Up to 128 rows there is no pair tile: the
-// narrowest of 64 / 128 / 256 columns that fits one wave.
+//     8 x 2048 x 2048          9.3           -           -
+//     200 x 3072 x 768         5.7           -           -
+//     200 x 768 x 3072         9.7         13.3          -
+//     512 x 1024 x 1024        5.7           -           -
+//     768 x 768 x 64           4.2           -           -
+//     1024 x 1024 x 3072      10.5         14.4          -
+//     2048 x 1024 x 4096        -          18.5          -
+//     1024 x 3072 x 1024        -            -          13.7
+// So: tiles of 64 columns while they fit one wave of CTAs, pairs of 128 columns while those fit one
+// wave of pairs, wide tiles beyond.  Up to 128 rows there is no pair tile: the narrowest of 64 / 128 /
+// 256 columns that fits one wave.
 GemmTile gemm_tile(int M, int N, int K) {
   const int sms = sm_count();
   const int64_t rows = (M + PBM - 1) / PBM, pair_rows = (M + 2 * PBM - 1) / (2 * PBM);
@@ -480,7 +505,7 @@ GemmTile gemm_tile(int M, int N, int K) {
     if (rows * ((N + 127) / 128) <= sms) return {false, 128};
     return {false, 0};
   }
-  if (K <= 2048 && rows * ((N + 63) / 64) <= sms) return {false, 64};
+  if (rows * ((N + 63) / 64) <= sms) return {false, 64};
   if (pair_rows * ((N + 127) / 128) <= sms / 2) return {true, 128};
   return {true, 0};
 }
@@ -491,7 +516,7 @@ GemmTile gemm_tile(int M, int N, int K) {
 // for a pair tile (use launch_gemm).
 int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bias, int M, int N,
                  int K, int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act,
-                 int bn, float* workspace, int* status, cudaStream_t stream) {
+                 int bn, float* workspace, int* status, cudaStream_t stream, const GemmEpi* epi) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (N % 8 || K % 8 || lda % 8 || ldb % 8 || ldc % 8) return 1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) |
@@ -510,7 +535,9 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
   Gemm2Params p;
   p.M = M; p.N = N; p.K = K; p.C = C; p.C2 = C2; p.ldc = ldc; p.bias = bias; p.act = act;
   p.out_bf16 = bf16 ? 1 : 0; p.status = status;
-  p.wide_store = (ldc % 16 == 0 && (reinterpret_cast<uintptr_t>(C) & 31) == 0) ? 1 : 0;
+  p.wide_store = (ldc % 16 == 0 && ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(C2)) & 31) == 0) ? 1 : 0;
+  p.Z = epi != nullptr ? epi->z : nullptr;
+  p.col_part = epi != nullptr ? epi->col_part : nullptr;
   p.idesc = tc::instr_desc_f16(2 * PBM, BN, bf16 ? 1 : 0, a_mn, b_mn);
   p.splits = workspace != nullptr ? gemm2_splits(M, N, K, BN) : 1;
 
@@ -520,6 +547,22 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
   p.splits = (num_kb + p.kb_per_split - 1) / p.kb_per_split;
   p.workspace = workspace;
 
+  if (epi != nullptr && epi->kind != kEpiPlain) {
+    if (a_mn || p.splits != 1) return 1;
+    if (epi_backward(epi->kind) && (reinterpret_cast<uintptr_t>(p.Z) & 15)) return 1;
+#define GEMM2_EPI(BN_, ST_, KIND_)                                                              \
+  if (BN == BN_ && epi->kind == KIND_)                                                          \
+    return b_mn ? launch_pair_variant<BN_, ST_, kKSub, false, true, KIND_>(ta, tb, p, stream)   \
+                : launch_pair_variant<BN_, ST_, kKSub, false, false, KIND_>(ta, tb, p, stream);
+#define GEMM2_EPIS(BN_, ST_)                                                      \
+  GEMM2_EPI(BN_, ST_, kEpiGelu) GEMM2_EPI(BN_, ST_, kEpiGeluTanh)                 \
+  GEMM2_EPI(BN_, ST_, kEpiGeluBwd) GEMM2_EPI(BN_, ST_, kEpiGeluTanhBwd) GEMM2_EPI(BN_, ST_, kEpiReluBwd)
+    GEMM2_EPIS(256, 6 / kKSub)
+    GEMM2_EPIS(128, 8 / kKSub)
+#undef GEMM2_EPIS
+#undef GEMM2_EPI
+    return 1;
+  }
 #define GEMM2_CASE(BN_, ST_)                                                                  \
   if (BN == BN_) {                                                                            \
     if (!a_mn && !b_mn)                                                                       \

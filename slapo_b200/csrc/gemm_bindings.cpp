@@ -110,9 +110,81 @@ Tensor gemm_out(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& b
   return c;
 }
 
+// Operands of a product with an activation in its epilogue, a [M, K] K-major
+struct GemmCall {
+  const Tensor &a, &w;
+  bool b_mn, bf16;
+  int M, N, K;
+  GemmCall(const Tensor& a_, const Tensor& w_, bool b_mn_) : a(a_), w(w_), b_mn(b_mn_) {
+    TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 2, "gemm: 2-D CUDA operands required");
+    TORCH_CHECK(a.scalar_type() == w.scalar_type() &&
+                    (a.scalar_type() == at::kBFloat16 || a.scalar_type() == at::kHalf),
+                "gemm: bf16 or fp16 operands of the same type required");
+    TORCH_CHECK(a.stride(1) == 1 && w.stride(1) == 1, "gemm: innermost dimension must be contiguous");
+    bf16 = a.scalar_type() == at::kBFloat16;
+    M = static_cast<int>(a.size(0));
+    K = static_cast<int>(a.size(1));
+    N = static_cast<int>(b_mn ? w.size(1) : w.size(0));
+    TORCH_CHECK(K == (b_mn ? w.size(0) : w.size(1)), "gemm: contraction sizes differ");
+  }
+  void run(const Tensor& c, const void* bias, const slapo::GemmEpi& epi) const {
+    const int dev = a.get_device();
+    auto stream = at::cuda::getCurrentCUDAStream().stream();
+    int* status = status_word(dev).data_ptr<int>();
+    const int lda = static_cast<int>(a.stride(0)), ldb = static_cast<int>(w.stride(0));
+    const slapo::GemmTile tile = slapo::gemm_tile(M, N, K);
+    int rc = 5;
+    if (tile.pair)
+      rc = slapo::launch_gemm2(a.data_ptr(), w.data_ptr(), c.data_ptr(), epi.c2, bias, M, N, K, lda, ldb, N,
+                               false, b_mn, bf16, -1, tile.bn, nullptr, status, stream, &epi);
+    if (rc == 5)
+      rc = slapo::launch_gemm(a.data_ptr(), w.data_ptr(), c.data_ptr(), bias, M, N, K, lda, ldb, N, false, b_mn,
+                              bf16, -1, tile.pair ? 0 : tile.bn, status, stream, &epi);
+    TORCH_CHECK(rc == 0, "gemm: launch refused (code ", rc,
+                "): sizes must be multiples of 8 and pointers 16-byte aligned");
+  }
+};
+
 Tensor gemm(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& bias, int64_t act,
             bool a_mn, bool b_mn) {
   return gemm_out(a, b, bias, act, a_mn, b_mn, c10::nullopt, c10::nullopt, 0, false);
+}
+
+// act(a w^T + bias) with the activation (0 GeLU, 1 GeLU tanh) in the epilogue, and the value before it
+// (empty unless `keep`).  `transposed`: w is [K, N].
+std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const Tensor& bias, int64_t act,
+                                        bool transposed, bool keep) {
+  TORCH_CHECK(act == 0 || act == 1, "gemm_act_fwd: GeLU only");
+  GemmCall g(a, w, transposed);
+  TORCH_CHECK(bias.scalar_type() == a.scalar_type() && bias.numel() == g.N && bias.is_contiguous(),
+              "gemm_act_fwd: bias must be a contiguous [N] tensor of the operand dtype");
+  c10::cuda::CUDAGuard guard(a.device());
+  Tensor y = at::empty({g.M, g.N}, a.options());
+  Tensor z = keep ? at::empty({g.M, g.N}, a.options()) : at::empty({0}, a.options());
+  slapo::GemmEpi epi{act == 0 ? 1 : 2, keep ? z.data_ptr() : nullptr, nullptr, nullptr};
+  g.run(y, bias.data_ptr(), epi);
+  return {y, z};
+}
+
+// dz = (dy w) * act'(z) and its column sums: the input gradient of the layer that follows an
+// activation, on to that activation's input.  z: for ReLU (act 2) the activation's output.  w is the
+// following layer's weight [K, N] (`transposed`: [N, K]).
+std::tuple<Tensor, Tensor> gemm_act_bwd(const Tensor& dy, const Tensor& w, const Tensor& z, int64_t act,
+                                        bool transposed) {
+  TORCH_CHECK(act >= 0 && act <= 2, "gemm_act_bwd: unknown activation");
+  GemmCall g(dy, w, !transposed);
+  TORCH_CHECK(z.is_cuda() && z.is_contiguous() && z.scalar_type() == dy.scalar_type() && z.dim() == 2 &&
+                  z.size(0) == g.M && z.size(1) == g.N,
+              "gemm_act_bwd: z must be a contiguous [M, N] tensor of the operand dtype");
+  c10::cuda::CUDAGuard guard(dy.device());
+  Tensor dz = at::empty({g.M, g.N}, dy.options()), db = at::empty({g.N}, dy.options());
+  const int parts = (g.M + 31) / 32;
+  Tensor part = at::empty({parts, g.N}, dy.options().dtype(at::kFloat));
+  slapo::GemmEpi epi{3 + static_cast<int>(act), nullptr, z.data_ptr(), part.data_ptr<float>()};
+  g.run(dz, nullptr, epi);
+  slapo::launch_colsum_finalize(part.data_ptr<float>(), db.data_ptr(), parts, g.N, g.bf16 ? 0 : 1,
+                                at::cuda::getCurrentCUDAStream().stream());
+  return {dz, db};
 }
 
 }  // namespace
@@ -123,6 +195,10 @@ void register_gemm_ops(torch::Library& m) {
   m.def("gemm(Tensor a, Tensor b, Tensor? bias, int act, bool a_mn, bool b_mn) -> Tensor", &gemm);
   m.def("gemm_out(Tensor a, Tensor b, Tensor? bias, int act, bool a_mn, bool b_mn, Tensor? out, "
         "Tensor? pre_act, int impl, bool split_k) -> Tensor", &gemm_out);
+  m.def("gemm_act_fwd(Tensor a, Tensor w, Tensor bias, int act, bool transposed, bool keep) -> (Tensor, Tensor)",
+        &gemm_act_fwd);
+  m.def("gemm_act_bwd(Tensor dy, Tensor w, Tensor z, int act, bool transposed) -> (Tensor, Tensor)",
+        &gemm_act_bwd);
   m.def("gemm2_splits(int M, int N, int K) -> int", [](int64_t M, int64_t N, int64_t K) -> int64_t {
     return slapo::gemm2_splits(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K),
                                N > 128 ? 256 : 128);

@@ -34,9 +34,12 @@ void launch_fused_adamw(void* param, const void* grad, float* master, float* exp
 
 // C[M,N] = act(A B^T + bias); a_mn / b_mn select M/N-major operands (see gemm.cu).
 // Returns 0 on success, >0 when the launch was refused on the host.
+// `epi`: an activation or its derivative in the epilogue (gemm_epilogue.cuh), A K-major; `act` is not
+// looked at then.  c2, z: [M, N] with C's row stride.
+struct GemmEpi { int kind; void* c2; const void* z; float* col_part; };
 int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
                 int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act, int bn,
-                int* status, cudaStream_t stream);
+                int* status, cudaStream_t stream, const GemmEpi* epi = nullptr);
 
 // The same product on CTA pairs (gemm2.cu): 256 x 256 tiles shared by two SMs, optional second
 // output `C2` (the value before the activation), optional split-K through `workspace`
@@ -49,7 +52,8 @@ struct GemmTile { bool pair; int bn; };
 GemmTile gemm_tile(int M, int N, int K);
 int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bias, int M, int N,
                  int K, int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act,
-                 int bn, float* workspace, int* status, cudaStream_t stream);
+                 int bn, float* workspace, int* status, cudaStream_t stream,
+                 const GemmEpi* epi = nullptr);   // (its second output is C2)
 
 // out[i] = cache past[i] ([B, past_len, H, head_bytes] contiguous) followed along the tokens by
 // fresh[i] ([B, new_len, H, head_bytes], strides of B / token / head in bytes), i = k, v.

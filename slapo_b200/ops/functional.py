@@ -119,12 +119,29 @@ def linear(x, weight, bias=None, act=None):
     if gemm_supported(x, weight):
         if act is None or act == "relu":
             return _nodes().linear(x, weight, bias, -1 if act is None else _RELU, False)
-        # GeLU is NOT fused: the epilogue warps of a tcgen05 GEMM have a fraction of the SM's
-        # FP32 issue rate, and an erf per element made the GEMM 2.5 x slower than running
-        # bias_act over the output afterwards
+        if _epilogue_bias(bias, x):
+            return _nodes().linear(x, weight, bias, _act_code(act), False)
         return bias_act(_nodes().linear(x, weight, None, -1, False), bias, act)
     out = F.linear(x, weight, bias)
     return out if act is None else _act_ref(out, act)
+
+
+def _epilogue_bias(bias, x):
+    """Whether a GEMM's epilogue can add ``bias`` in 16-byte words."""
+    return (bias is not None and bias.dtype == x.dtype and bias.is_contiguous()
+            and bias.data_ptr() % 16 == 0)
+
+
+def mlp_supported(x, w1, b1, w2, b2) -> bool:
+    """Whether :func:`mlp` takes a feed-forward block: what its two GEMMs take."""
+    return (gemm_supported(x, w1) and w2.dtype == x.dtype and w2.dim() == 2 and w2.stride(1) == 1
+            and w2.shape[0] % 8 == 0 and w2.stride(0) % 8 == 0 and w1.shape[1] == x.shape[-1]
+            and w2.shape[1] == w1.shape[0] and _epilogue_bias(b1, x) and _epilogue_bias(b2, x))
+
+
+def mlp(x, w1, b1, w2, b2, act: str, p: float):
+    """``dropout(act(x @ w1.T + b1) @ w2.T + b2, p)`` as one autograd node."""
+    return _nodes().mlp(x, w1, b1, w2, b2, _act_code(act), p)
 
 
 # ---------------------------------------------------------------------- #
