@@ -1250,10 +1250,15 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float
   p.idesc_pv = tc::instr_desc_f16(128, p.k_steps * 16, bf16 ? 1 : 0, false, true);
   const bool general = kbias != nullptr || rel != nullptr || causal || Sk % kBlockN != 0 || !(scale > 0.f);
   int rc;
+  // a single query sees all keys, causal or not
+  const bool decode = Sq == 1 && p.thr7 == 0 && rel == nullptr;
 #define FLASH_FWD_CASE(D_, T_)                                            \
   rc = general ? launch_fwd_d<D_, true, T_>(tq, tk, tv, p, stream)        \
                : launch_fwd_d<D_, false, T_>(tq, tk, tv, p, stream)
-  if (Dt == 64) {
+  if (decode) {
+    rc = launch_flash_decode(q, k, v, o, lse, p.part_o, p.part_ml, kbias, B, H, Sk, D, q_strides, k_strides,
+                             v_strides, scale, p.splits, p.tiles_per_split * kBlockN, bf16, stream);
+  } else if (Dt == 64) {
     if (bf16) FLASH_FWD_CASE(64, __nv_bfloat16);
     else FLASH_FWD_CASE(64, __half);
   } else {

@@ -87,7 +87,17 @@ Tensor gemm_out(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& b
   const int splits = split_k && impl != 1 ? slapo::gemm2_splits(M, N, K, N > 128 ? 256 : 128) : 1;
   // a second output and several pairs per tile exist on the pair kernel's default tile only
   slapo::GemmTile tile{impl != 1, 0};
-  if (impl == 0 && splits == 1 && c2 == nullptr) tile = slapo::gemm_tile(M, N, K);
+  if (impl == 0 && splits == 1 && c2 == nullptr) {
+    if (!a_mn && !b_mn && slapo::gemm_rows_takes(M, N, K)) {
+      rc = slapo::launch_gemm_rows(a.data_ptr(), b.data_ptr(), c.data_ptr(), bias_ptr, M, N, K,
+                                   static_cast<int>(a.stride(0)), static_cast<int>(b.stride(0)),
+                                   static_cast<int>(c.stride(0)), bf16, static_cast<int>(act), stream);
+      TORCH_CHECK(rc == 0, "gemm: launch refused (code ", rc,
+                  "): sizes must be multiples of 8 and pointers 16-byte aligned");
+      return c;
+    }
+    tile = slapo::gemm_tile(M, N, K);
+  }
   if (tile.pair) {
     float* ws = nullptr;
     if (splits > 1) ws = split_scratch(dev, static_cast<int64_t>(splits) * M * N).data_ptr<float>();

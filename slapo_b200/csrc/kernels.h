@@ -55,6 +55,18 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
                  int bn, float* workspace, int* status, cudaStream_t stream,
                  const GemmEpi* epi = nullptr);   // (its second output is C2)
 
+// The same for at most 16 rows, both operands K-major (gemm_rows.cu), and whether that takes a product.
+int launch_gemm_rows(const void* A, const void* W, void* C, const void* bias, int M, int N, int K, int lda,
+                     int ldw, int ldc, bool bf16, int act, cudaStream_t stream);
+bool gemm_rows_takes(int M, int N, int K);
+
+// Attention of one query per (batch, head), no dropout, no relative bias (flash_decode.cu); strides of
+// batch, token and head in elements; part_o / part_ml with splits > 1 (see flash_fwd_splits)
+int launch_flash_decode(const void* q, const void* k, const void* v, void* o, float* lse, float* part_o,
+                        float2* part_ml, const float* kbias, int B, int H, int Sk, int D,
+                        const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides,
+                        float scale, int splits, int keys_per_split, bool bf16, cudaStream_t stream);
+
 // out[i] = cache past[i] ([B, past_len, H, head_bytes] contiguous) followed along the tokens by
 // fresh[i] ([B, new_len, H, head_bytes], strides of B / token / head in bytes), i = k, v.
 // Everything 16-byte aligned.
