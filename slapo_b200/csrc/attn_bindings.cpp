@@ -214,6 +214,21 @@ void check_rel(const Tensor& table, const Tensor& buckets) {
               "rel_bias: table or distances too large");
 }
 
+// int64 [sq + sk - 1]: the buckets of the distances -(sk - 1) .. sq - 1, on the device of `table`
+Tensor rel_buckets(const Tensor& table, int64_t sq, int64_t sk, bool bidirectional, double inv_exact,
+                   double inv_log) {
+  TORCH_CHECK(table.is_cuda() && table.dim() == 2 && sq > 0 && sk > 0 && sq + sk <= INT_MAX - 256 &&
+                  table.size(0) >= (bidirectional ? 4 : 2) && table.size(0) <= INT_MAX,
+              "rel_buckets: a [buckets, H] CUDA table and positive lengths required");
+  c10::cuda::CUDAGuard guard(table.device());
+  const int n = static_cast<int>(sq + sk - 1);
+  Tensor out = at::empty({n}, table.options().dtype(at::kLong));
+  slapo::launch_rel_buckets(out.data_ptr<int64_t>(), n, static_cast<int>(sk - 1), static_cast<int>(table.size(0)),
+                            bidirectional ? 1 : 0, static_cast<float>(inv_exact), static_cast<float>(inv_log),
+                            at::cuda::getCurrentCUDAStream().stream());
+  return out;
+}
+
 Tensor rel_bias_fwd(const Tensor& table, const Tensor& buckets) {
   check_rel(table, buckets);
   c10::cuda::CUDAGuard guard(table.device());
@@ -249,6 +264,8 @@ void register_attn_ops(torch::Library& m) {
   m.def("flash_attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor? kbias, Tensor? rel, bool causal, float scale, float p_drop, Tensor? rng, bool packed_qkv, int keep_words=0) -> (Tensor, Tensor, Tensor, Tensor)",
         &flash_attn_bwd);
   m.def("append_kv(Tensor past_k, Tensor past_v, Tensor k, Tensor v) -> (Tensor, Tensor)", &append_kv);
+  m.def("rel_buckets(Tensor table, int sq, int sk, bool bidirectional, float inv_exact, float inv_log) -> Tensor",
+        &rel_buckets);
   m.def("rel_bias_fwd(Tensor table, Tensor buckets) -> Tensor", &rel_bias_fwd);
   m.def("rel_bias_bwd(Tensor grad, Tensor buckets, Tensor table) -> Tensor", &rel_bias_bwd);
   m.def("flash_attn_dropout_mask(int B, int H, int Sq, int Sk, float p_drop, Tensor rng) -> Tensor",

@@ -52,10 +52,16 @@ def _table_supported(table) -> bool:
 
 def relative_bias_by_distance(table, sq, sk, bidirectional, max_distance):
     """``[num_buckets, H]`` table -> ``[H, sq + sk - 1]`` bias per (key - query)."""
-    buckets = _distance_buckets(table.device, sq, sk, table.shape[0], bidirectional, max_distance)
     # (parameters that order the buckets otherwise can index outside of the table: torch's to report)
-    if _table_supported(table) and max_distance > table.shape[0] // (4 if bidirectional else 2):
+    exact = table.shape[0] // (4 if bidirectional else 2)
+    if _table_supported(table) and max_distance > exact:
+        if exact >= 1:
+            buckets = native.ops().rel_buckets(table, sq, sk, bidirectional, 1.0 / exact,
+                                               1.0 / math.log(max_distance / exact))
+        else:
+            buckets = _distance_buckets(table.device, sq, sk, table.shape[0], bidirectional, max_distance)
         return native.ops().rel_bias(table, buckets)
+    buckets = _distance_buckets(table.device, sq, sk, table.shape[0], bidirectional, max_distance)
     return table.float()[buckets].t().contiguous()
 
 
