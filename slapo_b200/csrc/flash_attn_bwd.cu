@@ -974,7 +974,7 @@ static int round128(int n) { return (n + 127) / 128 * 128; }
 // drawing), an item a quarter more (D = 128: 1.5, its accumulators leave tensor memory without a
 // second set to go on with), a launch 1.5; both in one came out 5 % over that.  Under a causal mask items differ and the heaviest go first, so that
 // no whole rounds are lost in two launches or one: side by side up to 5 waves of each.
-// Measured, two launches -> one (us): 1 x 512 x 16 x 64: 33 -> 22; 1 x 2048 x 12 x 64 causal: 102 -> 79;
+// Measured with passes over whole tiles, two launches -> one (us): 1 x 512 x 16 x 64: 33 -> 22; 1 x 2048 x 12 x 64 causal: 102 -> 79;
 // 4 x 1024 x 16 x 128: 199 -> 188; 4 x 256 x 12 x 64 with dropout: 33 -> 25; but 32 x 512 x 16 x 64 with
 // dropout 367 -> 420, without 258 -> 265, causal 225 -> 236.
 static int both_q_ctas(int64_t q_items, int64_t k_items, int64_t q_item_tiles, int64_t q_tiles, int D,
