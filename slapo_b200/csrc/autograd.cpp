@@ -49,12 +49,18 @@ Tensor colsum(const Tensor& x) {
 }
 
 std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const Tensor& bias, int64_t act,
-                                        bool transposed, bool keep) {
-  static auto f = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, int64_t, bool, bool)>(
-      "slapo_b200::gemm_act_fwd");
-  return f.call(a, w, bias, act, transposed, keep);
+                                        bool transposed, bool keep, bool sum) {
+  static auto f = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, int64_t, bool, bool,
+                                                bool)>("slapo_b200::gemm_act_fwd");
+  return f.call(a, w, bias, act, transposed, keep, sum);
 }
 constexpr int64_t kRelu = 2;
+std::tuple<Tensor, Tensor> bias_act_bwd(const Tensor& dy, const Tensor& x, const optional<Tensor>& bias,
+                                        int64_t act) {
+  static auto f = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const optional<Tensor>&,
+                                                int64_t)>("slapo_b200::bias_act_bwd");
+  return f.call(dy, x, bias, act);
+}
 
 // `t` as a 2-D matrix with contiguous rows whose stride TMA accepts
 Tensor rows_of(const Tensor& t) {
@@ -73,15 +79,17 @@ std::vector<int64_t> with_last(at::IntArrayRef shape, int64_t last) {
 // ------------------------------------------------------------------------ //
 // y = act(x W^T + b) (act < 0: no activation): three GEMMs, none of them transposing an operand in
 // memory.  Bias and activation ride in the forward GEMM's epilogue; the backward reads ReLU's derivative
-// off the output (y > 0) and GeLU's off the value before it, which the same epilogue leaves where a
-// backward will follow (`keep`).  `transposed`: W is stored [in, out] (x W + b).
+// off the output (y > 0) and GeLU's off the product, which the same epilogue leaves where a backward
+// will follow (`keep`).  GeLU's values and gradients are to the bit those of the plain layer followed
+// by BiasActFn.  `transposed`: W is stored [in, out] (x W + b).
 struct LinearFn : public Function<LinearFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight,
                         const optional<Tensor>& bias, int64_t act, bool transposed, bool keep) {
     Tensor x2 = rows_of(x);
     Tensor y, at;         // at: where the activation's derivative is read off
-    if (act >= 0 && act != kRelu) {
-      std::tie(y, at) = gemm_act_fwd(x2, weight, *bias, act, transposed, keep);
+    const bool gelu = act >= 0 && act != kRelu;
+    if (gelu) {
+      std::tie(y, at) = gemm_act_fwd(x2, weight, *bias, act, transposed, keep, false);
     } else {
       y = gemm(x2, weight, bias, act, false, transposed, false);
       if (act >= 0) at = y;
@@ -90,7 +98,7 @@ struct LinearFn : public Function<LinearFn> {
     ctx->saved_data["transposed"] = transposed;
     ctx->saved_data["bias"] = bias.has_value();
     ctx->saved_data["shape"] = x.sizes().vec();
-    ctx->save_for_backward({x2, weight, at});
+    ctx->save_for_backward({x2, weight, at, gelu ? *bias : Tensor()});
     return y.view(with_last(x.sizes(), weight.size(transposed ? 1 : 0)));
   }
   static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
@@ -101,10 +109,12 @@ struct LinearFn : public Function<LinearFn> {
     const bool has_bias = ctx->saved_data["bias"].toBool();
     Tensor dy = rows_of(grads[0]);
     Tensor dx, dw, db;
-    if (act >= 0) {
+    if (act == kRelu) {
       static auto f = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, int64_t)>(
           "slapo_b200::act_bwd_colsum");
       std::tie(dy, db) = f.call(dy.contiguous(), at, act);
+    } else if (act >= 0) {
+      std::tie(dy, db) = bias_act_bwd(dy.contiguous(), at, opt(saved[3]), act);
     } else if (has_bias && ctx->needs_input_grad(2)) {
       db = colsum(dy);
     }
@@ -129,7 +139,7 @@ struct MlpFn : public Function<MlpFn> {
     Tensor x2 = rows_of(x);
     Tensor h, at, y;
     if (act != kRelu) {
-      std::tie(h, at) = gemm_act_fwd(x2, w1, b1, act, false, keep);
+      std::tie(h, at) = gemm_act_fwd(x2, w1, b1, act, false, keep, true);
     } else {
       h = gemm(x2, w1, b1, act, false, false, false);
       at = h;
@@ -191,10 +201,8 @@ struct BiasActFn : public Function<BiasActFn> {
   }
   static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
     const variable_list saved = ctx->get_saved_variables();
-    static auto f = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const optional<Tensor>&,
-                                                  int64_t)>("slapo_b200::bias_act_bwd");
-    auto [dx, db] = f.call(grads[0].contiguous(), saved[0].contiguous(), opt(saved[1]),
-                           ctx->saved_data["act"].toInt());
+    auto [dx, db] = bias_act_bwd(grads[0].contiguous(), saved[0].contiguous(), opt(saved[1]),
+                                 ctx->saved_data["act"].toInt());
     return {dx, saved[1].defined() ? db : Tensor(), Tensor()};
   }
 };

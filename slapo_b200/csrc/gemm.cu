@@ -86,9 +86,10 @@ struct GemmParams {
   int out_bf16;       // 1 bf16, 0 fp16
   uint32_t idesc;
   int* status;        // device error word (0 = ok)
-  void* C2;           // kEpi forward: acc + bias, or nullptr
+  void* C2;           // kEpi forward: the product, or nullptr
   const void* Z;      // kEpi backward: input (ReLU: output) of the activation, as C in memory
   float* col_part;    // kEpi backward: column sums over 32 rows each, or nullptr
+  int c2_sum;         // kEpi forward: C2 includes the bias
 };
 
 constexpr int BM = 128;
@@ -383,6 +384,7 @@ int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, 
   p.C2 = epi != nullptr ? epi->c2 : nullptr;
   p.Z = epi != nullptr ? epi->z : nullptr;
   p.col_part = epi != nullptr ? epi->col_part : nullptr;
+  p.c2_sum = epi != nullptr && epi->c2_sum ? 1 : 0;
   if (epi != nullptr && epi->kind != kEpiPlain) {
     if (a_mn) return 1;
     if ((reinterpret_cast<uintptr_t>(p.Z) | reinterpret_cast<uintptr_t>(p.C2) |

@@ -42,6 +42,7 @@ struct Gemm2Params {
   int* status;
   const void* Z;      // kEpi backward: input (ReLU: output) of the activation, as C in memory
   float* col_part;    // kEpi backward: column sums over 32 rows each, or nullptr
+  int c2_sum;         // kEpi forward: C2 includes the bias
   int wide_store;     // rows of C are 32-byte aligned: the epilogue stores whole sectors
 };
 
@@ -563,6 +564,7 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
   p.wide_store = (ldc % 16 == 0 && ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(C2)) & 31) == 0) ? 1 : 0;
   p.Z = epi != nullptr ? epi->z : nullptr;
   p.col_part = epi != nullptr ? epi->col_part : nullptr;
+  p.c2_sum = epi != nullptr && epi->c2_sum ? 1 : 0;
   p.idesc = tc::instr_desc_f16(2 * PBM, BN, bf16 ? 1 : 0, a_mn, b_mn);
   p.splits = workspace != nullptr ? gemm2_splits(M, N, K, BN) : 1;
 

@@ -161,9 +161,9 @@ Tensor gemm(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& bias,
 }
 
 // act(a w^T + bias) with the activation (0 GeLU, 1 GeLU tanh) in the epilogue, and the value before it
-// (empty unless `keep`).  `transposed`: w is [K, N].
+// (empty unless `keep`): the product, or with `sum` product + bias.  `transposed`: w is [K, N].
 std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const Tensor& bias, int64_t act,
-                                        bool transposed, bool keep) {
+                                        bool transposed, bool keep, bool sum) {
   TORCH_CHECK(act == 0 || act == 1, "gemm_act_fwd: GeLU only");
   GemmCall g(a, w, transposed);
   TORCH_CHECK(bias.scalar_type() == a.scalar_type() && bias.numel() == g.N && bias.is_contiguous(),
@@ -171,7 +171,7 @@ std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const 
   c10::cuda::CUDAGuard guard(a.device());
   Tensor y = at::empty({g.M, g.N}, a.options());
   Tensor z = keep ? at::empty({g.M, g.N}, a.options()) : at::empty({0}, a.options());
-  slapo::GemmEpi epi{act == 0 ? 1 : 2, keep ? z.data_ptr() : nullptr, nullptr, nullptr};
+  slapo::GemmEpi epi{act == 0 ? 1 : 2, sum, keep ? z.data_ptr() : nullptr, nullptr, nullptr};
   g.run(y, bias.data_ptr(), epi);
   return {y, z};
 }
@@ -190,7 +190,7 @@ std::tuple<Tensor, Tensor> gemm_act_bwd(const Tensor& dy, const Tensor& w, const
   Tensor dz = at::empty({g.M, g.N}, dy.options()), db = at::empty({g.N}, dy.options());
   const int parts = (g.M + 31) / 32;
   Tensor part = at::empty({parts, g.N}, dy.options().dtype(at::kFloat));
-  slapo::GemmEpi epi{3 + static_cast<int>(act), nullptr, z.data_ptr(), part.data_ptr<float>()};
+  slapo::GemmEpi epi{3 + static_cast<int>(act), false, nullptr, z.data_ptr(), part.data_ptr<float>()};
   g.run(dz, nullptr, epi);
   slapo::launch_colsum_finalize(part.data_ptr<float>(), db.data_ptr(), parts, g.N, g.bf16 ? 0 : 1,
                                 at::cuda::getCurrentCUDAStream().stream());
@@ -205,7 +205,7 @@ void register_gemm_ops(torch::Library& m) {
   m.def("gemm(Tensor a, Tensor b, Tensor? bias, int act, bool a_mn, bool b_mn) -> Tensor", &gemm);
   m.def("gemm_out(Tensor a, Tensor b, Tensor? bias, int act, bool a_mn, bool b_mn, Tensor? out, "
         "Tensor? pre_act, int impl, bool split_k) -> Tensor", &gemm_out);
-  m.def("gemm_act_fwd(Tensor a, Tensor w, Tensor bias, int act, bool transposed, bool keep) -> (Tensor, Tensor)",
+  m.def("gemm_act_fwd(Tensor a, Tensor w, Tensor bias, int act, bool transposed, bool keep, bool sum=True) -> (Tensor, Tensor)",
         &gemm_act_fwd);
   m.def("gemm_act_bwd(Tensor dy, Tensor w, Tensor z, int act, bool transposed) -> (Tensor, Tensor)",
         &gemm_act_bwd);

@@ -1,8 +1,11 @@
 // What the GEMM kernels do with 32 columns of a row of the fp32 accumulator when an activation or its
 // derivative rides in the epilogue (kEpi below); kind 0 is the kernels' own bias / ReLU path.
 //
-// GeLU's forward: C = act(acc + bias), and C2 = acc + bias in 16 bits for the backward when that is
-// wanted.  Backward: C = acc * act'(Z), with column sums of C (the bias gradient) over each 32 rows
+// GeLU's forward: the product is rounded to 16 bits, then C = act(product + bias): to the bit what a linear
+// layer followed by a kernel for bias + activation gives.  (Adding the bias to the accumulator rounds once
+// less and saves 5 of 122 us at 16384 x 4096, K = 1024, but moves every value that follows: after four BERT
+// layers logits and gradients by 0.9 % of their norm.)  What the backward wants goes to C2: the product, or with
+// `c2_sum` product + bias, rounded.  Backward: C = acc * act'(Z), with column sums of C (the bias gradient) over each 32 rows
 // to `col_part` [ceil(M / 32)][N], which a second kernel adds up in a fixed order.
 // An element is about 20 instructions and two of the special-function unit; eight warps have them done
 // well within the products of a 256 x 256 tile with K = 1024 (8192 cycles), under which they run.  What
@@ -114,14 +117,17 @@ __device__ __forceinline__ void epi_finish(const P& p, float (&v)[32], const uin
   } else {
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      const float2 b = unpack_pair(aux[j], p.out_bf16);
-      v[2 * j] += b.x;
-      v[2 * j + 1] += b.y;
+      w[j] = pack_pair(v[2 * j], v[2 * j + 1], p.out_bf16);
+      const float2 a = unpack_pair(w[j], p.out_bf16), b = unpack_pair(aux[j], p.out_bf16);
+      v[2 * j] = a.x + b.x;
+      v[2 * j + 1] = a.y + b.y;
     }
     if (row >= p.M) return;
     if (p.C2 != nullptr) {
+      if (p.c2_sum) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) w[j] = pack_pair(v[2 * j], v[2 * j + 1], p.out_bf16);
+        for (int j = 0; j < 16; ++j) w[j] = pack_pair(v[2 * j], v[2 * j + 1], p.out_bf16);
+      }
       store_row32(p.C2, off, col0, p.N, sectors, w);
     }
 #pragma unroll
