@@ -132,8 +132,9 @@ __global__ void __launch_bounds__(32 * kDecodeWarps, 1) flash_decode_kernel(cons
     if (d == 0) p.part_ml[row] = make_float2(top, sum);
     return;
   }
+  // (no visible key: 0; a NaN among the scores or values stays one, as in the other kernels)
   if (d < p.D)
-    static_cast<T*>(p.o)[static_cast<int64_t>(bh) * p.D + d] = static_cast<T>(sum > 0.f ? x / sum : 0.f);
+    static_cast<T*>(p.o)[static_cast<int64_t>(bh) * p.D + d] = static_cast<T>(x * (sum > 0.f ? 1.f / sum : 0.f));
   if (d == 0) p.lse[bh] = sum > 0.f ? use * 0.6931471805599453f + logf(sum) : -INFINITY;
 }
 

@@ -45,6 +45,25 @@ def test_keys_that_all_are_hidden():
     assert (NF.flash_attention(q, k, v, key_padding_bias=bias) == 0).all()
 
 
+@pytest.mark.parametrize("sk", [40, 2000])        # one work item per head, and keys split
+@pytest.mark.parametrize("what", ["q", "k", "v"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+def test_nans_and_infinities_stay(sk, what, value):
+    """An overflowed cache shows: what plain softmax attention makes a NaN or an infinity is one here, in its
+    head, and the other heads are as they were."""
+    torch.manual_seed(sk)
+    q, k, v = (torch.randn(1, n, 3, 64, device="cuda", dtype=FP) for n in (1, sk, sk))
+    clean = NF.flash_attention(q, k, v)
+    {"q": q, "k": k, "v": v}[what][0, -1, 1, 5] = value
+    out = NF.flash_attention(q, k, v)
+    scores = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) * 64 ** -0.5
+    want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(scores, -1), v.double())
+    assert torch.equal(out[:, :, [0, 2]], clean[:, :, [0, 2]])
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isinf(), want.isinf())
+    if what == "v" or value != value:
+        assert not out[:, :, 1].isfinite().all()
+
+
 @pytest.mark.parametrize("m", [1, 7, 8, 9, 16])
 @pytest.mark.parametrize("k,n,dtype,act", [(64, 64, BF, None), (72, 200, FP, "relu"), (2048, 6144, BF, None),
                                            (2560, 72, FP, None), (4104, 1024, BF, "relu")])
