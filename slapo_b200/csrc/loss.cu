@@ -25,7 +25,9 @@ namespace slapo {
 constexpr int kCeUnroll = 4;
 
 // Maximum and sum of exp(x - maximum) of kCeUnroll vectors of 8, added to a thread's running pair: one
-// rescaling for all of them, products and sums on pairs of values.
+// rescaling for all of them, differences, products and sums on pairs of values.  The maximum is subtracted
+// before the scaling: exact near it, where the terms that count are, and finite for any two numbers (the
+// lowest of the type times log2(e) is not).
 __device__ __forceinline__ void ce_add(const float (&v)[kCeUnroll][8], float& m, float& s) {
   float cm = v[0][0];
 #pragma unroll
@@ -33,20 +35,20 @@ __device__ __forceinline__ void ce_add(const float (&v)[kCeUnroll][8], float& m,
 #pragma unroll
     for (int k = 0; k < 8; ++k) cm = fmaxf(cm, v[u][k]);
   const float nm = fmaxf(m, cm);
-  const float shift = nm == -INFINITY ? 0.f : -nm * kLog2e;
-  const uint64_t scale2 = f2_pack(kLog2e, kLog2e), shift2 = f2_pack(shift, shift);
+  const float use = nm == -INFINITY ? 0.f : nm;
+  const uint64_t scale2 = f2_pack(kLog2e, kLog2e), minus2 = f2_pack(-use, -use);
   uint64_t acc[2] = {0, 0};
 #pragma unroll
   for (int u = 0; u < kCeUnroll; ++u)
 #pragma unroll
     for (int k = 0; k < 8; k += 2) {
       float a, b;
-      f2_unpack(f2_fma(f2_pack(v[u][k], v[u][k + 1]), scale2, shift2), a, b);
+      f2_unpack(f2_mul(f2_add(f2_pack(v[u][k], v[u][k + 1]), minus2), scale2), a, b);
       acc[(k >> 1) & 1] = f2_add(acc[(k >> 1) & 1], f2_pack(exp2f(a), exp2f(b)));
     }
   float a, b;
   f2_unpack(f2_add(acc[0], acc[1]), a, b);
-  s = s * exp2f(fmaf(m, kLog2e, shift)) + (a + b);
+  s = s * exp2f((m - use) * kLog2e) + (a + b);
   m = nm;
 }
 

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from slapo_b200.ops import cross_entropy as ce
+from slapo_b200.ops import native
 
 pytestmark = pytest.mark.gpu
 
@@ -31,3 +32,36 @@ def test_loss_and_gradient(rows, cols, dtype):
     p = p * (coef.double() * (labels != -100))[:, None]
     err = ((x.grad.double() - p).norm() / p.norm()).item()
     assert err < {torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10, torch.float32: 5e-6}[dtype]
+
+
+def test_error_of_peaked_rows():
+    """A trained model's rows: logits spread over 40, a handful of terms make the sum."""
+    torch.manual_seed(5)
+    x = (torch.randn(512, 49152, device="cuda") * 5).bfloat16()
+    labels = torch.randint(0, x.shape[1], (x.shape[0],), device="cuda")
+    _, lse = native.ops().ce_loss(x, labels, -100)
+    want = torch.logsumexp(x.double(), -1)
+    # the result's own rounding to 32 bits, and 2^-20 for the terms (exp2: 2^-22) and their sum
+    ulp = 2.0 ** (want.abs().log2().floor() - 23)
+    assert ((lse.double() - want).abs() <= ulp / 2 + 2.0 ** -20).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("cols", [520, 8192, 50304])
+def test_columns_masked_with_the_lowest_value(cols, dtype):
+    torch.manual_seed(cols)
+    low = torch.finfo(dtype).min
+    x = torch.randn(4, cols, device="cuda").to(dtype)
+    x[0, :cols - 8] = low               # all that most threads see
+    x[1, :cols // 2] = low
+    x[2, cols // 2:] = low
+    x[3, 0] = -low
+    labels = torch.tensor([cols - 3, cols - 1, 1, 0], device="cuda")
+    x.requires_grad_()
+    loss = ce.cross_entropy(x, labels)
+    want = torch.nn.functional.cross_entropy(x.detach().double(), labels, reduction="none")
+    torch.testing.assert_close(loss.double(), want, rtol=2e-6, atol=2e-6)
+    (grad,) = torch.autograd.grad(loss.sum(), [x])
+    p = torch.softmax(x.detach().double(), -1)
+    p[torch.arange(4, device="cuda"), labels] -= 1
+    torch.testing.assert_close(grad.double(), p, rtol=2.0 ** -7, atol=1e-6)
