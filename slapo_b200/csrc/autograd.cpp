@@ -48,10 +48,10 @@ Tensor colsum(const Tensor& x) {
   return f.call(x);
 }
 
-std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const Tensor& bias, int64_t act,
-                                        bool transposed, bool keep, bool sum) {
-  static auto f = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, int64_t, bool, bool,
-                                                bool)>("slapo_b200::gemm_act_fwd");
+std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const optional<Tensor>& bias,
+                                        int64_t act, bool transposed, bool keep, bool sum) {
+  static auto f = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const optional<Tensor>&, int64_t, bool,
+                                                bool, bool)>("slapo_b200::gemm_act_fwd");
   return f.call(a, w, bias, act, transposed, keep, sum);
 }
 constexpr int64_t kRelu = 2;
@@ -89,7 +89,7 @@ struct LinearFn : public Function<LinearFn> {
     Tensor y, at;         // at: where the activation's derivative is read off
     const bool gelu = act >= 0 && act != kRelu;
     if (gelu) {
-      std::tie(y, at) = gemm_act_fwd(x2, weight, *bias, act, transposed, keep, false);
+      std::tie(y, at) = gemm_act_fwd(x2, weight, bias, act, transposed, keep, false);
     } else {
       y = gemm(x2, weight, bias, act, false, transposed, false);
       if (act >= 0) at = y;
@@ -98,7 +98,7 @@ struct LinearFn : public Function<LinearFn> {
     ctx->saved_data["transposed"] = transposed;
     ctx->saved_data["bias"] = bias.has_value();
     ctx->saved_data["shape"] = x.sizes().vec();
-    ctx->save_for_backward({x2, weight, at, gelu ? *bias : Tensor()});
+    ctx->save_for_backward({x2, weight, at, gelu ? or_undefined(bias) : Tensor()});
     return y.view(with_last(x.sizes(), weight.size(transposed ? 1 : 0)));
   }
   static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
@@ -384,24 +384,39 @@ tensor_list RelBiasFn::backward(AutogradContext* ctx, tensor_list grads) {
 }
 
 // ------------------------------------------------------------------------ //
-Tensor linear(const Tensor& x, const Tensor& weight, const optional<Tensor>& bias, int64_t act,
+// A bias that starts anywhere, as the kernels read it: 16 bytes at a time.  (A copy that is differentiated.)
+Tensor aligned(const Tensor& bias) {
+  return bias.is_cuda() && reinterpret_cast<uintptr_t>(bias.data_ptr()) % 16 != 0 ? bias.clone() : bias;
+}
+optional<Tensor> aligned(const optional<Tensor>& bias) {
+  return bias.has_value() && bias->defined() ? optional<Tensor>(aligned(*bias)) : c10::nullopt;
+}
+
+Tensor linear(const Tensor& x, const Tensor& weight, const optional<Tensor>& bias_in, int64_t act,
               bool transposed) {
+  const optional<Tensor> bias = aligned(bias_in);
   const bool keep = at::GradMode::is_enabled() &&
                     (x.requires_grad() || weight.requires_grad() || (bias.has_value() && bias->requires_grad()));
   return LinearFn::apply(x, weight, bias, act, transposed, keep);
 }
 Tensor mlp(const Tensor& x, const Tensor& w1, const Tensor& b1, const Tensor& w2, const Tensor& b2,
            int64_t act, double p) {
+  TORCH_CHECK(w1.dim() == 2 && w2.dim() == 2 && x.dim() >= 1 && x.size(-1) == w1.size(1) &&
+                  w2.size(1) == w1.size(0) && b1.numel() == w1.size(0) && b2.numel() == w2.size(0),
+              "mlp: x [.., in], w1 [inner, in], b1 [inner], w2 [out, inner] and b2 [out] required");
+  for (const Tensor* t : {&w1, &b1, &w2, &b2})
+    TORCH_CHECK(t->device() == x.device() && t->scalar_type() == x.scalar_type() && t->stride(-1) == 1,
+                "mlp: contiguous parameters of x's type and device required");
   const bool keep = at::GradMode::is_enabled() && (x.requires_grad() || w1.requires_grad() || b1.requires_grad() ||
                                                    w2.requires_grad() || b2.requires_grad());
-  return MlpFn::apply(x, w1, b1, w2, b2, act, p, keep);
+  return MlpFn::apply(x, w1, aligned(b1), w2, aligned(b2), act, p, keep);
 }
 Tensor bias_act(const Tensor& x, const optional<Tensor>& bias, int64_t act) {
-  return BiasActFn::apply(x, bias, act);
+  return BiasActFn::apply(x, aligned(bias), act);
 }
 Tensor bias_dropout_add(const Tensor& x, const optional<Tensor>& bias, const optional<Tensor>& residual,
                         double p) {
-  return BiasDropoutAddFn::apply(x, bias, residual, p);
+  return BiasDropoutAddFn::apply(x, aligned(bias), residual, p);
 }
 Tensor norm(const Tensor& x, const Tensor& weight, const optional<Tensor>& bias, double eps, bool rms) {
   return LayerNormFn::apply(x, weight, bias, eps, rms);
@@ -409,7 +424,7 @@ Tensor norm(const Tensor& x, const Tensor& weight, const optional<Tensor>& bias,
 std::tuple<Tensor, Tensor> dropout_add_norm(const Tensor& x, const optional<Tensor>& bias,
                                             const Tensor& residual, const Tensor& weight,
                                             const optional<Tensor>& ln_bias, double p, double eps) {
-  variable_list r = DropoutAddNormFn::apply(x, bias, residual, weight, ln_bias, p, eps);
+  variable_list r = DropoutAddNormFn::apply(x, aligned(bias), residual, weight, ln_bias, p, eps);
   return {r[0], r[1]};
 }
 Tensor flash(const Tensor& q, const optional<Tensor>& k, const optional<Tensor>& v,

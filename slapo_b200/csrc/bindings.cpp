@@ -21,8 +21,12 @@ int dtype_code(const Tensor& t) {
   }
 }
 
+// (the kernels read it 16 bytes at a time)
 const void* opt_ptr(const optional<Tensor>& t) {
-  return (t.has_value() && t->defined()) ? t->data_ptr() : nullptr;
+  if (!t.has_value() || !t->defined()) return nullptr;
+  TORCH_CHECK(t->is_cuda() && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0,
+              "slapo_b200: bias, residual and the like must be 16-byte aligned CUDA tensors");
+  return t->data_ptr();
 }
 
 void check_cuda_contig(const Tensor& t, const char* name) {

@@ -546,7 +546,8 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (N % 8 || K % 8 || lda % 8 || ldb % 8 || ldc % 8) return 1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) |
-       reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(C2)) & 15)
+       reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(C2) |
+       reinterpret_cast<uintptr_t>(bias)) & 15)
     return 1;
   if (a_mn && M % 8) return 1;
   if (M <= PBM || N <= 64) return 5;

@@ -43,10 +43,19 @@ Tensor& split_scratch(int device, int64_t floats) {
 // the word itself (device tensor), for callers that copy it out asynchronously
 Tensor device_status_tensor() { return status_word(at::cuda::current_device()); }
 
+// A bias [N] as the kernels read it, 16 bytes at a time, or null
+const void* bias_words(const c10::optional<Tensor>& bias, const Tensor& a, int N) {
+  if (!bias.has_value() || !bias->defined()) return nullptr;
+  TORCH_CHECK(bias->device() == a.device() && bias->scalar_type() == a.scalar_type() && bias->numel() == N &&
+                  bias->is_contiguous(),
+              "gemm: bias must be a contiguous [N] tensor of the operands' type and device");
+  return bias->data_ptr();
+}
+
 Tensor gemm_out(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& bias, int64_t act,
                 bool a_mn, bool b_mn, const c10::optional<Tensor>& out,
                 const c10::optional<Tensor>& pre_act, int64_t impl, bool split_k) {
-  TORCH_CHECK(a.is_cuda() && b.is_cuda(), "gemm: CUDA tensors required");
+  TORCH_CHECK(a.is_cuda() && b.device() == a.device(), "gemm: tensors on one CUDA device required");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2, "gemm: 2-D operands required");
   TORCH_CHECK(a.scalar_type() == b.scalar_type() &&
                   (a.scalar_type() == at::kBFloat16 || a.scalar_type() == at::kHalf),
@@ -62,7 +71,7 @@ Tensor gemm_out(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& b
   if (out.has_value() && out->defined()) {
     c = *out;
     TORCH_CHECK(c.dim() == 2 && c.size(0) == M && c.size(1) == N && c.stride(1) == 1 &&
-                    c.scalar_type() == a.scalar_type(),
+                    c.scalar_type() == a.scalar_type() && c.device() == a.device(),
                 "gemm: `out` must be an [M, N] tensor of the operand dtype with contiguous rows");
   } else {
     c = at::empty({M, N}, a.options());
@@ -70,16 +79,11 @@ Tensor gemm_out(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& b
   void* c2 = nullptr;
   if (pre_act.has_value() && pre_act->defined()) {
     TORCH_CHECK(pre_act->sizes() == c.sizes() && pre_act->strides() == c.strides() &&
-                    pre_act->scalar_type() == c.scalar_type(),
+                    pre_act->scalar_type() == c.scalar_type() && pre_act->device() == c.device(),
                 "gemm: `pre_act` must match the output's shape, strides and dtype");
     c2 = pre_act->data_ptr();
   }
-  const void* bias_ptr = nullptr;
-  if (bias.has_value() && bias->defined()) {
-    TORCH_CHECK(bias->scalar_type() == a.scalar_type() && bias->numel() == N && bias->is_contiguous(),
-                "gemm: bias must be a contiguous [N] tensor of the operand dtype");
-    bias_ptr = bias->data_ptr();
-  }
+  const void* bias_ptr = bias_words(bias, a, N);
   const int dev = a.get_device();
   const bool bf16 = a.scalar_type() == at::kBFloat16;
   auto stream = at::cuda::getCurrentCUDAStream().stream();
@@ -126,7 +130,8 @@ struct GemmCall {
   bool b_mn, bf16;
   int M, N, K;
   GemmCall(const Tensor& a_, const Tensor& w_, bool b_mn_) : a(a_), w(w_), b_mn(b_mn_) {
-    TORCH_CHECK(a.is_cuda() && w.is_cuda() && a.dim() == 2 && w.dim() == 2, "gemm: 2-D CUDA operands required");
+    TORCH_CHECK(a.is_cuda() && w.device() == a.device() && a.dim() == 2 && w.dim() == 2,
+                "gemm: 2-D operands on one CUDA device required");
     TORCH_CHECK(a.scalar_type() == w.scalar_type() &&
                     (a.scalar_type() == at::kBFloat16 || a.scalar_type() == at::kHalf),
                 "gemm: bf16 or fp16 operands of the same type required");
@@ -162,17 +167,16 @@ Tensor gemm(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& bias,
 
 // act(a w^T + bias) with the activation (0 GeLU, 1 GeLU tanh) in the epilogue, and the value before it
 // (empty unless `keep`): the product, or with `sum` product + bias.  `transposed`: w is [K, N].
-std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const Tensor& bias, int64_t act,
-                                        bool transposed, bool keep, bool sum) {
+std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias,
+                                        int64_t act, bool transposed, bool keep, bool sum) {
   TORCH_CHECK(act == 0 || act == 1, "gemm_act_fwd: GeLU only");
   GemmCall g(a, w, transposed);
-  TORCH_CHECK(bias.scalar_type() == a.scalar_type() && bias.numel() == g.N && bias.is_contiguous(),
-              "gemm_act_fwd: bias must be a contiguous [N] tensor of the operand dtype");
+  const void* bias_ptr = bias_words(bias, a, g.N);
   c10::cuda::CUDAGuard guard(a.device());
   Tensor y = at::empty({g.M, g.N}, a.options());
   Tensor z = keep ? at::empty({g.M, g.N}, a.options()) : at::empty({0}, a.options());
   slapo::GemmEpi epi{act == 0 ? 1 : 2, sum, keep ? z.data_ptr() : nullptr, nullptr, nullptr};
-  g.run(y, bias.data_ptr(), epi);
+  g.run(y, bias_ptr, epi);
   return {y, z};
 }
 
@@ -183,7 +187,7 @@ std::tuple<Tensor, Tensor> gemm_act_bwd(const Tensor& dy, const Tensor& w, const
                                         bool transposed) {
   TORCH_CHECK(act >= 0 && act <= 2, "gemm_act_bwd: unknown activation");
   GemmCall g(dy, w, !transposed);
-  TORCH_CHECK(z.is_cuda() && z.is_contiguous() && z.scalar_type() == dy.scalar_type() && z.dim() == 2 &&
+  TORCH_CHECK(z.device() == dy.device() && z.is_contiguous() && z.scalar_type() == dy.scalar_type() && z.dim() == 2 &&
                   z.size(0) == g.M && z.size(1) == g.N,
               "gemm_act_bwd: z must be a contiguous [M, N] tensor of the operand dtype");
   c10::cuda::CUDAGuard guard(dy.device());
@@ -205,7 +209,7 @@ void register_gemm_ops(torch::Library& m) {
   m.def("gemm(Tensor a, Tensor b, Tensor? bias, int act, bool a_mn, bool b_mn) -> Tensor", &gemm);
   m.def("gemm_out(Tensor a, Tensor b, Tensor? bias, int act, bool a_mn, bool b_mn, Tensor? out, "
         "Tensor? pre_act, int impl, bool split_k) -> Tensor", &gemm_out);
-  m.def("gemm_act_fwd(Tensor a, Tensor w, Tensor bias, int act, bool transposed, bool keep, bool sum=True) -> (Tensor, Tensor)",
+  m.def("gemm_act_fwd(Tensor a, Tensor w, Tensor? bias, int act, bool transposed, bool keep, bool sum=True) -> (Tensor, Tensor)",
         &gemm_act_fwd);
   m.def("gemm_act_bwd(Tensor dy, Tensor w, Tensor z, int act, bool transposed) -> (Tensor, Tensor)",
         &gemm_act_bwd);
