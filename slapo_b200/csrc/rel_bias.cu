@@ -44,9 +44,11 @@ __global__ void __launch_bounds__(256) rel_bias_bwd_kernel(const float* __restri
   }
 }
 
-// T5's bucket of every distance key - query, as the reference implementation's operators round it: fp32
-// throughout, divisions by a number as products with its reciprocal, each rounded.  One launch where
-// those operators were fourteen (40 us of kernels and 150 us of the host's time at 1023 distances).
+// T5's bucket of every distance key - query, as the operators of t5_relative_position_bucket round it: fp32
+// throughout, divisions by a number as products with its reciprocal, each rounded, and the logarithm that
+// the operators call (this file is built without --use_fast_math).  Where a distance lies on a border between
+// buckets the last bit of any of these decides.  One launch where those operators were fourteen (40 us of
+// kernels and 150 us of the host's time at 1023 distances).
 __global__ void __launch_bounds__(256) rel_buckets_kernel(int64_t* __restrict__ out, int n, int last_key,
                                                           int buckets, int bidirectional, float inv_exact,
                                                           float inv_log) {
@@ -63,9 +65,8 @@ __global__ void __launch_bounds__(256) rel_buckets_kernel(int64_t* __restrict__ 
   int b = far;
   if (far >= exact) {
     const float x = __fmul_rn(static_cast<float>(max(far, 1)), inv_exact);
-    // (the float nearest to the logarithm: the build's logf is the fast one)
-    const float l = static_cast<float>(log(static_cast<double>(x)));
-    b = min(exact + static_cast<int>(__fmul_rn(__fmul_rn(l, inv_log), static_cast<float>(buckets - exact))),
+    const float l = __fmul_rn(logf(x), inv_log);
+    b = min(exact + static_cast<int>(__fmul_rn(l, static_cast<float>(buckets - exact))),
             buckets - 1);
   }
   out[i] = base + b;

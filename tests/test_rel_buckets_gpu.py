@@ -23,3 +23,18 @@ def test_buckets(buckets, max_distance, bidirectional):
                                        1.0 / math.log(max_distance / exact))
         want = _distance_buckets("cuda", sq, sk, buckets, bidirectional, max_distance)
         assert torch.equal(got, want), (sq, sk)
+
+
+@pytest.mark.parametrize("bidirectional", [True, False])
+@pytest.mark.parametrize("buckets", list(range(6, 90, 3)) + [160, 200, 256])
+def test_distances_on_borders(buckets, bidirectional):
+    """Largest distances that are a square, cube or other power of a ratio times the exact buckets: distances fall
+    on borders between buckets, where the last bit of the logarithm decides."""
+    exact = buckets // (4 if bidirectional else 2)
+    table = torch.zeros(buckets, 2, device="cuda")
+    for far in sorted({exact * r ** e for r in (2, 3, 5, 6, 7, 10) for e in (1, 2, 3, 4)}
+                      | {exact * a * a // 4 for a in range(3, 16)} | set(range(exact + 1, exact + 40))):
+        if exact < far < 20000:
+            got = native.ops().rel_buckets(table, 1500, 1500, bidirectional, 1.0 / exact,
+                                           1.0 / math.log(far / exact))
+            assert torch.equal(got, _distance_buckets("cuda", 1500, 1500, buckets, bidirectional, far)), far
