@@ -22,16 +22,21 @@ namespace slapo {
 // close to it by the exponentials (92 us of the special-function unit): with one vector at a time, its own
 // rescaling and scalar arithmetic 161 us, so 141; loss and log-sum-exp from here instead of eight small kernels
 // and the gradient from the last row on, 460 -> 396 us for the loss and its gradient.
-constexpr int kCeUnroll = 4;
+//
+// Rows of fewer than two such steps are taken a vector at a time by a kernel a half as large, whose CTAs come and
+// go faster (us, 4096 rows, a vector at a time / four): 128 columns 6.7 / 9.6, 3816: 10.7 / 14.1, 12288: 23.4 /
+// 25.8, 16384: 31.0 / 27.4, 24576: 42.8 / 36.6.
+constexpr int kCeUnroll = 4, kCeLongRow = 2 * kCeUnroll * 256 * 8;
 
-// Maximum and sum of exp(x - maximum) of kCeUnroll vectors of 8, added to a thread's running pair: one
+// Maximum and sum of exp(x - maximum) of U vectors of 8, added to a thread's running pair: one
 // rescaling for all of them, differences, products and sums on pairs of values.  The maximum is subtracted
 // before the scaling: exact near it, where the terms that count are, and finite for any two numbers (the
 // lowest of the type times log2(e) is not).
-__device__ __forceinline__ void ce_add(const float (&v)[kCeUnroll][8], float& m, float& s) {
+template <int U>
+__device__ __forceinline__ void ce_add(const float (&v)[U][8], float& m, float& s) {
   float cm = v[0][0];
 #pragma unroll
-  for (int u = 0; u < kCeUnroll; ++u)
+  for (int u = 0; u < U; ++u)
 #pragma unroll
     for (int k = 0; k < 8; ++k) cm = fmaxf(cm, v[u][k]);
   const float nm = fmaxf(m, cm);
@@ -39,7 +44,7 @@ __device__ __forceinline__ void ce_add(const float (&v)[kCeUnroll][8], float& m,
   const uint64_t scale2 = f2_pack(kLog2e, kLog2e), minus2 = f2_pack(-use, -use);
   uint64_t acc[2] = {0, 0};
 #pragma unroll
-  for (int u = 0; u < kCeUnroll; ++u)
+  for (int u = 0; u < U; ++u)
 #pragma unroll
     for (int k = 0; k < 8; k += 2) {
       float a, b;
@@ -52,8 +57,8 @@ __device__ __forceinline__ void ce_add(const float (&v)[kCeUnroll][8], float& m,
   m = nm;
 }
 
-// stats: (max, sum, target logit) per row, or null: then loss and lse of each row instead.
-template <typename T>
+// kLoss: loss and lse of each row, otherwise stats (max, sum, target logit).  U vectors of a thread at a time.
+template <typename T, int U, bool kLoss>
 __global__ void __launch_bounds__(256) ce_stats_kernel(
     const T* __restrict__ logits, const int64_t* __restrict__ labels, float* __restrict__ stats,
     float* __restrict__ loss, float* __restrict__ lse, int rows, int cols, int64_t row_stride,
@@ -65,13 +70,13 @@ __global__ void __launch_bounds__(256) ce_stats_kernel(
   float* out = stats + static_cast<int64_t>(row) * 3;
   if (label == ignore_index) {
     if (threadIdx.x == 0) {
-      if (stats != nullptr) {
+      if constexpr (kLoss) {
+        loss[row] = 0.f;
+        lse[row] = 0.f;
+      } else {
         out[0] = -INFINITY;
         out[1] = 0.f;
         out[2] = 0.f;
-      } else {
-        loss[row] = 0.f;
-        lse[row] = 0.f;
       }
     }
     return;
@@ -80,16 +85,17 @@ __global__ void __launch_bounds__(256) ce_stats_kernel(
   float m = -INFINITY, s = 0.f;
   const int step = blockDim.x * 8;
   int c = threadIdx.x * 8;
-  for (; c + (kCeUnroll - 1) * step < cols; c += kCeUnroll * step) {
-    float v[kCeUnroll][8];
+#pragma unroll 1
+  for (; c + (U - 1) * step < cols; c += U * step) {
+    float v[U][8];
 #pragma unroll
-    for (int u = 0; u < kCeUnroll; ++u) Vec8<T>::load(x + c + u * step, v[u]);
+    for (int u = 0; u < U; ++u) Vec8<T>::load(x + c + u * step, v[u]);
     ce_add(v, m, s);
   }
-  if (c < cols) {
-    float v[kCeUnroll][8];
+  if (U > 1 && c < cols) {
+    float v[U][8];
 #pragma unroll
-    for (int u = 0; u < kCeUnroll; ++u) {
+    for (int u = 0; u < U; ++u) {
       if (c + u * step < cols) {
         Vec8<T>::load(x + c + u * step, v[u]);
       } else {
@@ -122,14 +128,14 @@ __global__ void __launch_bounds__(256) ce_stats_kernel(
     const int64_t local = label - vocab_start;
     float picked = 0.f;
     if (local >= 0 && local < cols) picked = static_cast<float>(x[local]);
-    if (stats != nullptr) {
-      out[0] = fm;
-      out[1] = fs;
-      out[2] = picked;
-    } else {
+    if constexpr (kLoss) {
       const float l = fm + static_cast<float>(log(static_cast<double>(fs)));
       lse[row] = l;
       loss[row] = l - picked;
+    } else {
+      out[0] = fm;
+      out[1] = fs;
+      out[2] = picked;
     }
   }
 }
@@ -210,14 +216,23 @@ __global__ void __launch_bounds__(256) sq_norm_kernel(const T* __restrict__ x,
     default: { using T = float; __VA_ARGS__; break; }                \
   }
 
+template <int U, bool kLoss>
+static void launch_stats(const void* logits, const int64_t* labels, float* stats, float* loss, float* lse,
+                         int rows, int cols, int64_t row_stride, int vocab_start, int64_t ignore_index,
+                         int dtype, cudaStream_t stream) {
+  DISPATCH_DTYPE(dtype, (ce_stats_kernel<T, U, kLoss><<<rows, 256, 0, stream>>>(
+      static_cast<const T*>(logits), labels, stats, loss, lse, rows, cols, row_stride, vocab_start,
+      ignore_index)));
+}
+
 void launch_ce_stats(const void* logits, const int64_t* labels, float* stats, float* loss, float* lse,
                      int rows, int cols, int64_t row_stride, int vocab_start, int64_t ignore_index,
                      int dtype, cudaStream_t stream) {
   if (rows == 0) return;
   count_launch();
-  DISPATCH_DTYPE(dtype, (ce_stats_kernel<T><<<rows, 256, 0, stream>>>(
-      static_cast<const T*>(logits), labels, stats, loss, lse, rows, cols, row_stride, vocab_start,
-      ignore_index)));
+  auto launch = cols < kCeLongRow ? (stats == nullptr ? launch_stats<1, true> : launch_stats<1, false>)
+                                  : (stats == nullptr ? launch_stats<kCeUnroll, true> : launch_stats<kCeUnroll, false>);
+  launch(logits, labels, stats, loss, lse, rows, cols, row_stride, vocab_start, ignore_index, dtype, stream);
 }
 
 void launch_ce_grad(const void* logits, const int64_t* labels, const float* lse,

@@ -34,6 +34,23 @@ def test_loss_and_gradient(rows, cols, dtype):
     assert err < {torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10, torch.float32: 5e-6}[dtype]
 
 
+@pytest.mark.parametrize("cols", [16376, 16384, 16392])      # a vector at a time, and four
+def test_border_of_long_rows(cols):
+    torch.manual_seed(cols)
+    x = torch.randn(9, cols, device="cuda").bfloat16()
+    labels = torch.randint(0, cols, (9,), device="cuda")
+    labels[4] = -100
+    loss, lse = native.ops().ce_loss(x, labels, -100)
+    stats = native.ops().ce_stats(x, labels, 0, -100).double()
+    want = torch.logsumexp(x.double(), -1) * (labels != -100)
+    picked = x.double()[torch.arange(9, device="cuda"), labels.clamp(min=0)] * (labels != -100)
+    torch.testing.assert_close(lse.double(), want, rtol=2e-6, atol=2e-6)
+    torch.testing.assert_close(loss.double(), want - picked, rtol=2e-6, atol=2e-6)
+    ok = labels != -100
+    torch.testing.assert_close((stats[:, 0] + stats[:, 1].log())[ok], want[ok], rtol=2e-6, atol=2e-6)
+    assert torch.equal(stats[:, 2], picked) and stats[4].tolist() == [float("-inf"), 0.0, 0.0]
+
+
 def test_error_of_peaked_rows():
     """A trained model's rows: logits spread over 40, a handful of terms make the sum."""
     torch.manual_seed(5)
