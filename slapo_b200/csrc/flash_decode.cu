@@ -6,7 +6,7 @@
 // the four before.  L lanes share a key
 // row, so that a warp's load is 32 / L whole rows; each such group of lanes keeps a running maximum, sum and
 // output of its own, merged over the lanes and warps at the end.  Probabilities stay in fp32.
-// A CTA takes the keys of one work item: all of a head's, or a share of them that flash_combine_kernel
+// A CTA of sixteen or four warps takes the keys of one work item: all of a head's, or a share of them that flash_combine_kernel
 // adds up (the rule is flash_fwd_splits).
 // Measured (us), tensor-core tiles -> this: 8 x 1500 keys x 16 heads of 128: 24.4 -> 19.5 after a cache was grown
 // (32 -> 20 alone; without the rows fetched ahead 38); 16 x 2000 x 20 x 64: 90 -> 41; 1 x 300 x 12 x 64: 10.7 -> 4.6; 1 x 2000 x 16 x 128,
@@ -29,13 +29,13 @@ struct FlashDecodeParams {
   int rows;             // B H
 };
 
-constexpr int kDecodeWarps = 16, kDecodeUnroll = 4;
+constexpr int kDecodeUnroll = 4;
 
-template <int L, typename T>
-__global__ void __launch_bounds__(32 * kDecodeWarps, 1) flash_decode_kernel(const FlashDecodeParams p) {
+template <int L, int kWarps, typename T>
+__global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) flash_decode_kernel(const FlashDecodeParams p) {
   constexpr int kRows = 32 / L;                 // key rows of a warp's load
-  __shared__ float s_o[kDecodeWarps][L * 8];
-  __shared__ float2 s_ml[kDecodeWarps];
+  __shared__ float s_o[kWarps][L * 8];
+  __shared__ float2 s_ml[kWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bh = blockIdx.x / p.splits, split = blockIdx.x - bh * p.splits;
   const int b = bh / p.H, h = bh - b * p.H;
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(32 * kDecodeWarps, 1) flash_decode_kernel(cons
 
   // a step's rows as they are in memory, the next step's on their way under this one's arithmetic
   struct Rows { uint4 k[kDecodeUnroll], v[kDecodeUnroll]; };
-  constexpr int kStep = kDecodeWarps * kRows * kDecodeUnroll;
+  constexpr int kStep = kWarps * kRows * kDecodeUnroll;
   auto load = [&](int at, Rows& r) {
 #pragma unroll
     for (int u = 0; u < kDecodeUnroll; ++u) {
@@ -116,12 +116,12 @@ __global__ void __launch_bounds__(32 * kDecodeWarps, 1) flash_decode_kernel(cons
   __syncthreads();
   float top = -INFINITY;
 #pragma unroll
-  for (int w = 0; w < kDecodeWarps; ++w) top = fmaxf(top, s_ml[w].x);
+  for (int w = 0; w < kWarps; ++w) top = fmaxf(top, s_ml[w].x);
   const float use = top == -INFINITY ? 0.f : top;
   float sum = 0.f, x = 0.f;
   const int d = threadIdx.x;
 #pragma unroll
-  for (int w = 0; w < kDecodeWarps; ++w) {
+  for (int w = 0; w < kWarps; ++w) {
     const float f = exp2f(s_ml[w].x - use);
     sum += s_ml[w].y * f;
     if (d < p.D) x += s_o[w][d] * f;
@@ -156,13 +156,26 @@ int launch_flash_decode(const void* q, const void* k, const void* v, void* o, fl
   if (ctas > 0x7fffffff) return 1;
   const unsigned grid = static_cast<unsigned>(ctas);
   count_launch();
+  // Sixteen warps where a work item has many keys and the items leave SMs idle, four (and four CTAs per SM)
+  // where most of sixteen would have nothing to load or the items fill the SMs by themselves.  Measured (us;
+  // 128-row tensor-core tiles / sixteen / four), bf16, items x keys x D: 96 x 16 x 64: 6.8 / 3.4 / 2.9; 96 x 256 x 64: 8.0 / 4.2 /
+  // 4.6; 384 x 128 x 64: 10.5 / 8.8 / 4.6; 640 x 2000 x 64: 96 / 67 / 75; 2048 x 128 x 64: 28 / 48 / 19; 4096 x 512 x
+  // 64: 147 / 144 / 93; 144 x 384 x 128: 11.8 / 8.1 / 13.1; 384 x 256 x 128: 19.8 / 17.5 / 12.9; 2048 x 512 x 128:
+  // 110 / 111 / 89.
+  const int step = D <= 64 ? 256 : 128;         // keys that sixteen warps take at a time
+  const bool few = 2 * keys_per_split <= step || (2 * ctas >= 3 * sm_count() && keys_per_split <= 2 * step) ||
+                   ctas >= 6 * sm_count();
+#define FLASH_DECODE_CASE(L_, W_)                                                                     \
+  if (bf16) flash_decode_kernel<L_, W_, __nv_bfloat16><<<grid, 32 * W_, 0, stream>>>(p);              \
+  else flash_decode_kernel<L_, W_, __half><<<grid, 32 * W_, 0, stream>>>(p)
   if (D <= 64) {
-    if (bf16) flash_decode_kernel<8, __nv_bfloat16><<<grid, 32 * kDecodeWarps, 0, stream>>>(p);
-    else flash_decode_kernel<8, __half><<<grid, 32 * kDecodeWarps, 0, stream>>>(p);
+    if (few) { FLASH_DECODE_CASE(8, 4); }
+    else { FLASH_DECODE_CASE(8, 16); }
   } else {
-    if (bf16) flash_decode_kernel<16, __nv_bfloat16><<<grid, 32 * kDecodeWarps, 0, stream>>>(p);
-    else flash_decode_kernel<16, __half><<<grid, 32 * kDecodeWarps, 0, stream>>>(p);
+    if (few) { FLASH_DECODE_CASE(16, 4); }
+    else { FLASH_DECODE_CASE(16, 16); }
   }
+#undef FLASH_DECODE_CASE
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 

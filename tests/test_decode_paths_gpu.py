@@ -39,6 +39,14 @@ def test_single_query(sk, b, h, d, dtype, how):
     assert native.ops().device_status() == 0
 
 
+# four warps per work item or sixteen: half a step of keys, two steps with 222 items, any number with 888
+@pytest.mark.parametrize("h,sk,d", [(4, 128, 64), (4, 129, 64), (4, 64, 128), (4, 65, 80), (221, 512, 64),
+                                    (222, 512, 64), (222, 513, 64), (222, 256, 128), (222, 257, 128), (887, 520, 64),
+                                    (888, 520, 64), (888, 300, 128), (888, 7, 128)])
+def test_warps_of_a_work_item(h, sk, d):
+    test_single_query(sk, 1, h, d, BF, "k")
+
+
 def test_keys_that_all_are_hidden():
     q, k, v = (torch.randn(1, n, 2, 64, device="cuda", dtype=BF) for n in (1, 200, 200))
     bias = torch.full((1, 200), float("-inf"), device="cuda")
