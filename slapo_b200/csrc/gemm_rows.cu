@@ -41,7 +41,8 @@ __device__ __forceinline__ void mma_16x8x16<__half>(float (&d)[4], const uint32_
 
 constexpr int kRowsWarps = 8, kRowsUnroll = 8;
 
-template <typename T>
+// kRuns: a warp takes eight steps of K in a row (512 bytes of each row of W), otherwise every eighth one
+template <typename T, bool kRuns>
 __global__ void __launch_bounds__(32 * kRowsWarps) gemm_rows_kernel(const GemmRowsParams p) {
   __shared__ float s_sum[kRowsWarps][16][9];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -55,18 +56,19 @@ __global__ void __launch_bounds__(32 * kRowsWarps) gemm_rows_kernel(const GemmRo
   const bool two = p.M > 8;
   float d[4] = {0.f, 0.f, 0.f, 0.f};
   const int steps = (p.K + 31) / 32;
-  for (int s0 = warp * kRowsUnroll; s0 < steps; s0 += kRowsWarps * kRowsUnroll) {
+  constexpr int kNext = kRuns ? 1 : kRowsWarps;
+  for (int s0 = kRuns ? warp * kRowsUnroll : warp; s0 < steps; s0 += kRowsWarps * kRowsUnroll) {
     uint4 ww[kRowsUnroll], x[kRowsUnroll];
 #pragma unroll
     for (int u = 0; u < kRowsUnroll; ++u) {
-      const int k = (s0 + u) * 32;
+      const int k = (s0 + u * kNext) * 32;
       const bool ok = k + k_lane < p.K;       // K % 8 == 0: all eight or none
       ww[u] = ok ? __ldcs(reinterpret_cast<const uint4*>(w + k)) : zero;
       x[u] = ok ? __ldg(reinterpret_cast<const uint4*>(a0 + k)) : zero;
     }
 #pragma unroll
     for (int u = 0; u < kRowsUnroll; ++u) {
-      const int k = (s0 + u) * 32;
+      const int k = (s0 + u * kNext) * 32;
       uint4 y = zero;
       if (two && k + k_lane < p.K) y = __ldg(reinterpret_cast<const uint4*>(a1 + k));
       const uint32_t f0[4] = {x[u].x, y.x, x[u].y, y.y}, f1[4] = {x[u].z, y.z, x[u].w, y.w};
@@ -93,6 +95,8 @@ __global__ void __launch_bounds__(32 * kRowsWarps) gemm_rows_kernel(const GemmRo
   }
 }
 
+// All products on so few rows that fill a block of 64 columns and two steps of K: from 64 x 64 (5.2 -> 2.4 us
+// with 8 rows) to a vocabulary's width (the table below).
 bool gemm_rows_takes(int M, int N, int K) { return M <= 16 && K >= 64 && N >= 64; }
 
 // Returns 0 on success; >0 = refused on the host, as launch_gemm does.
@@ -103,9 +107,16 @@ int launch_gemm_rows(const void* A, const void* W, void* C, const void* bias, in
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(C)) & 15)
     return 1;
   const GemmRowsParams p{A, W, bias, C, M, N, K, lda, ldw, ldc, act};
+  // Runs where every warp has whole ones (K a multiple of 2048), otherwise steps one by one: at K = 768 runs
+  // would be three of eight warps' work.  Measured (us, 8 rows; 64-column tcgen05 tiles / runs / one by one), W
+  // not in L2: 2048 x 2048: 15.2 / 6.2 / 7.0; 2560 x 10240: 51.6 / 20.4 / 25.5; 2560 x 2560: 17.8 / 9.8 / 8.7; 3072 x
+  // 768: 8.5 / 5.5 / 4.3; 30528 x 768: 21.9 / 24.7 / 20.5; 32000 x 512: 19.3 / 24.1 / 17.7; 50304 x 1024: 37.8 / 37.3 /
+  // 35.8; 50304 x 2048: 54.0 / 44.5 / 52.4.
+  const bool runs = K % (32 * kRowsWarps * kRowsUnroll) == 0;
+  auto kernel = bf16 ? (runs ? gemm_rows_kernel<__nv_bfloat16, true> : gemm_rows_kernel<__nv_bfloat16, false>)
+                     : (runs ? gemm_rows_kernel<__half, true> : gemm_rows_kernel<__half, false>);
   count_launch();
-  if (bf16) gemm_rows_kernel<__nv_bfloat16><<<N / 8, 32 * kRowsWarps, 0, stream>>>(p);
-  else gemm_rows_kernel<__half><<<N / 8, 32 * kRowsWarps, 0, stream>>>(p);
+  kernel<<<N / 8, 32 * kRowsWarps, 0, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 

@@ -72,6 +72,11 @@ def test_nans_and_infinities_stay(sk, what, value):
         assert not out[:, :, 1].isfinite().all()
 
 
+@pytest.mark.parametrize("k", [2040, 2048, 2056, 4096, 4128, 768, 512])       # steps of K in runs and one by one
+def test_few_rows_contractions(k):
+    test_few_rows(16, k, 1032, BF, None)
+
+
 @pytest.mark.parametrize("m", [1, 7, 8, 9, 16])
 @pytest.mark.parametrize("k,n,dtype,act", [(64, 64, BF, None), (72, 200, FP, "relu"), (2048, 6144, BF, None),
                                            (2560, 72, FP, None), (4104, 1024, BF, "relu")])
