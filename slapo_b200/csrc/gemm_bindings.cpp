@@ -149,7 +149,10 @@ struct GemmCall {
     const int lda = static_cast<int>(a.stride(0)), ldb = static_cast<int>(w.stride(0));
     const slapo::GemmTile tile = slapo::gemm_tile(M, N, K);
     int rc = 5;
-    if (tile.pair)
+    if (epi.z == nullptr && !b_mn && slapo::gemm_rows_takes(M, N, K))
+      rc = slapo::launch_gemm_rows(a.data_ptr(), w.data_ptr(), c.data_ptr(), bias, M, N, K, lda, ldb, N, bf16, -1,
+                                   stream, &epi);
+    else if (tile.pair)
       rc = slapo::launch_gemm2(a.data_ptr(), w.data_ptr(), c.data_ptr(), epi.c2, bias, M, N, K, lda, ldb, N,
                                false, b_mn, bf16, -1, tile.bn, nullptr, status, stream, &epi);
     if (rc == 5)

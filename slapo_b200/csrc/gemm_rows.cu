@@ -1,5 +1,5 @@
 // C[M, N] = act(A[M, K] W[N, K]^T + bias) for at most 16 rows: a linear layer on the tokens of one step of
-// generation.  bf16 / fp16, fp32 accumulation.
+// generation, GeLU and what its backward wants included (gemm_epilogue.cuh).  bf16 / fp16, fp32 accumulation.
 //
 // Bound by reading W once.  A 128-row tcgen05 tile has few CTAs for it (2048 columns: 32) and each
 // waits for its ring; here a CTA takes 8 columns and its eight warps a part of K each, lanes load W straight
@@ -8,14 +8,16 @@
 // values of k) are the operands of two products, with A's values picked alike.
 // Measured, 64-column tcgen05 tiles -> this: 8 x 6144 x 2048 and 8 x 2048 x 2048 together 30.3 -> 19.0 us (weights not in L2).
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
 #include "kernels.h"
 
 namespace slapo {
 
 struct GemmRowsParams {
   const void *a, *w, *bias;
-  void* c;
+  void *c, *c2;         // c2: GeLU's (GemmEpi), or nullptr
   int M, N, K, lda, ldw, ldc, act;
+  int gelu, c2_sum;     // kind of GemmEpi and what goes to c2; 0: bias and `act`
 };
 
 template <typename T>
@@ -88,9 +90,18 @@ __global__ void __launch_bounds__(32 * kRowsWarps) gemm_rows_kernel(const GemmRo
       float v = 0.f;
 #pragma unroll
       for (int i = 0; i < kRowsWarps; ++i) v += s_sum[i][r][c];
-      if (p.bias != nullptr) v += static_cast<float>(static_cast<const T*>(p.bias)[n0 + c]);
-      if (p.act >= 0) v = act_fwd(v, p.act);
-      static_cast<T*>(p.c)[static_cast<int64_t>(r) * p.ldc + n0 + c] = static_cast<T>(v);
+      const float bias = p.bias != nullptr ? static_cast<float>(static_cast<const T*>(p.bias)[n0 + c]) : 0.f;
+      const int64_t at = static_cast<int64_t>(r) * p.ldc + n0 + c;
+      if (p.gelu != kEpiPlain) {        // as epi_finish has it
+        const T product = static_cast<T>(v);
+        v = static_cast<float>(product) + bias;
+        if (p.c2 != nullptr) static_cast<T*>(p.c2)[at] = p.c2_sum ? static_cast<T>(v) : product;
+        v = p.gelu == kEpiGelu ? epi_value<kEpiGelu>(v) : epi_value<kEpiGeluTanh>(v);
+      } else {
+        v += bias;
+        if (p.act >= 0) v = act_fwd(v, p.act);
+      }
+      static_cast<T*>(p.c)[at] = static_cast<T>(v);
     }
   }
 }
@@ -101,12 +112,14 @@ bool gemm_rows_takes(int M, int N, int K) { return M <= 16 && K >= 64 && N >= 64
 
 // Returns 0 on success; >0 = refused on the host, as launch_gemm does.
 int launch_gemm_rows(const void* A, const void* W, void* C, const void* bias, int M, int N, int K, int lda,
-                     int ldw, int ldc, bool bf16, int act, cudaStream_t stream) {
+                     int ldw, int ldc, bool bf16, int act, cudaStream_t stream, const GemmEpi* epi) {
+  if (epi != nullptr && epi_backward(epi->kind)) return 1;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (M > 16 || N % 8 || K % 8 || lda % 8 || ldw % 8 || ldc % 8) return 1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(C)) & 15)
     return 1;
-  const GemmRowsParams p{A, W, bias, C, M, N, K, lda, ldw, ldc, act};
+  const GemmRowsParams p{A, W, bias, C, epi != nullptr ? epi->c2 : nullptr, M, N, K, lda, ldw, ldc, act,
+                         epi != nullptr ? epi->kind : kEpiPlain, epi != nullptr && epi->c2_sum ? 1 : 0};
   // Runs where every warp has whole ones (K a multiple of 2048), otherwise steps one by one: at K = 768 runs
   // would be three of eight warps' work.  Measured (us, 8 rows; 64-column tcgen05 tiles / runs / one by one), W
   // not in L2: 2048 x 2048: 15.2 / 6.2 / 7.0; 2560 x 10240: 51.6 / 20.4 / 25.5; 2560 x 2560: 17.8 / 9.8 / 8.7; 3072 x

@@ -57,7 +57,8 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
 
 // The same for at most 16 rows, both operands K-major (gemm_rows.cu), and whether that takes a product.
 int launch_gemm_rows(const void* A, const void* W, void* C, const void* bias, int M, int N, int K, int lda,
-                     int ldw, int ldc, bool bf16, int act, cudaStream_t stream);
+                     int ldw, int ldc, bool bf16, int act, cudaStream_t stream,
+                     const GemmEpi* epi = nullptr);    // (forward kinds only)
 bool gemm_rows_takes(int M, int N, int K);
 
 // Attention of one query per (batch, head), no dropout, no relative bias (flash_decode.cu); strides of

@@ -15,9 +15,9 @@ pytestmark = pytest.mark.gpu
 BF, FP = torch.bfloat16, torch.float16
 
 
-# every tile: one CTA of 64 / 128 / 256 columns, pairs of 128 / 256; ragged rows and columns
+# few rows, steps of K in runs and one by one; every tile: one CTA of 64 / 128 / 256 columns, pairs of 128 / 256; ragged rows and columns
 @pytest.mark.parametrize("act,dtype", [("gelu", BF), ("gelu_new", FP)])
-@pytest.mark.parametrize("m,k,n", [(40, 72, 200), (200, 768, 3072), (128, 64, 64 * 148 + 8), (120, 64, 19200),
+@pytest.mark.parametrize("m,k,n", [(8, 64, 64), (16, 2048, 200), (8, 776, 3072), (40, 72, 200), (200, 768, 3072), (128, 64, 64 * 148 + 8), (120, 64, 19200),
                                    (392, 64, 4104), (2056, 64, 2056)])
 def test_equals_layer_then_activation(m, k, n, act, dtype):
     torch.manual_seed(m + n)
@@ -35,6 +35,9 @@ def test_equals_layer_then_activation(m, k, n, act, dtype):
         assert torch.equal(p, q), name
     with torch.no_grad():
         assert torch.equal(NF.linear(x, w, b, act), one[0])
+        summed = native.ops().gemm_act_fwd(x, w, b, NF._act_code(act), False, True, True)
+        assert torch.equal(summed[0], one[0])
+        assert torch.equal(summed[1], (NF.linear(x, w).float() + b.float()).to(dtype))
     assert native.ops().device_status() == 0
 
 
