@@ -117,11 +117,12 @@ def linear(x, weight, bias=None, act=None):
     16-bit tensors run this library's GEMM (bias and activation in its epilogue), anything
     else PyTorch."""
     if gemm_supported(x, weight):
+        nodes = _nodes()
         if act is None or act == "relu":
-            return _nodes().linear(x, weight, bias, -1 if act is None else _RELU, False)
+            return nodes.linear(x, weight, bias, -1 if act is None else _RELU, False)
         if _epilogue_bias(bias, x):
-            return _nodes().linear(x, weight, bias, _act_code(act), False)
-        return bias_act(_nodes().linear(x, weight, None, -1, False), bias, act)
+            return nodes.linear(x, weight, bias, _act_code(act), False)
+        return bias_act(nodes.linear(x, weight, None, -1, False), bias, act)
     out = F.linear(x, weight, bias)
     return out if act is None else _act_ref(out, act)
 
@@ -134,7 +135,10 @@ def _epilogue_bias(bias, x):
 
 def mlp_supported(x, w1, b1, w2, b2) -> bool:
     """Whether :func:`mlp` takes a feed-forward block: what its two GEMMs take."""
-    return (gemm_supported(x, w1) and w2.dtype == x.dtype and w2.dim() == 2 and w2.stride(1) == 1
+    if not gemm_supported(x, w1):
+        return False
+    _nodes()        # (a transform is refused before the biases' addresses are looked at)
+    return (w2.dtype == x.dtype and w2.dim() == 2 and w2.stride(1) == 1
             and w2.shape[0] % 8 == 0 and w2.stride(0) % 8 == 0 and w1.shape[1] == x.shape[-1]
             and w2.shape[1] == w1.shape[0] and _epilogue_bias(b1, x) and _epilogue_bias(b2, x))
 

@@ -1,0 +1,60 @@
+"""The feed-forward block's autograd node under what its layers had to bear: saved-tensor hooks, inputs that are
+differentiated alone, and transforms, which are refused with the reason whatever they batch."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwd
+
+from slapo_b200.op import FusedMLP
+from slapo_b200.ops import functional as NF
+
+pytestmark = pytest.mark.gpu
+
+BF = torch.bfloat16
+
+
+def _block(act, p):
+    torch.manual_seed(2)
+    block = FusedMLP(64, 256, act, p, device="cuda", dtype=BF)
+    x = torch.randn(40, 64, device="cuda", dtype=BF, requires_grad=True)
+    return block, x, [x, *block.parameters()]
+
+
+def _run(block, x):
+    torch.cuda.manual_seed(7)
+    return block(x)
+
+
+@pytest.mark.parametrize("act,p", [("gelu", 0.1), ("relu", 0.0)])
+def test_hooks_and_single_inputs(act, p):
+    block, x, leaves = _block(act, p)
+    y = _run(block, x)
+    dy = torch.randn_like(y)
+    want = torch.autograd.grad(y, leaves, dy)
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(1), t.cpu())[1], lambda t: t.cuda()):
+        y = _run(block, x)
+    assert seen and all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y, leaves, dy), want))
+    for i, leaf in enumerate(leaves):
+        for other in leaves:
+            other.requires_grad_(other is leaf)
+        (got,) = torch.autograd.grad(_run(block, x), [leaf], dy)
+        assert torch.equal(got, want[i]), i
+
+
+def test_transforms_are_refused():
+    block, x, leaves = _block("gelu", 0.0)
+    x = x.detach()
+    names = [n for n, _ in block.named_parameters()]
+    plain = [p.detach() for p in block.parameters()]
+    with fwd.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
+        block(fwd.make_dual(x, torch.ones_like(x)))
+    with pytest.raises(RuntimeError, match="functorch"):
+        torch.vmap(block)(torch.stack([x, x]))
+    for i, name in enumerate(names):        # each parameter batched, the biases among them
+        def call(t):
+            return torch.func.functional_call(block, {**dict(zip(names, plain)), name: t}, (x,))
+        with pytest.raises(RuntimeError, match="functorch"):
+            torch.vmap(call)(torch.stack([plain[i], plain[i]]))
+    w, b = plain[:2]
+    with pytest.raises(RuntimeError, match="functorch"):
+        torch.vmap(lambda t: NF.linear(x, w, t, "gelu"))(torch.stack([b, b]))
