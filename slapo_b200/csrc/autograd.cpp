@@ -49,12 +49,16 @@ Tensor colsum(const Tensor& x) {
 }
 
 std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const optional<Tensor>& bias,
-                                        int64_t act, bool transposed, bool keep, bool sum) {
+                                        int64_t act, bool keep, bool sum) {
   static auto f = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const optional<Tensor>&, int64_t, bool,
-                                                bool, bool)>("slapo_b200::gemm_act_fwd");
-  return f.call(a, w, bias, act, transposed, keep, sum);
+                                                bool)>("slapo_b200::gemm_act_fwd");
+  return f.call(a, w, bias, act, keep, sum);
 }
 constexpr int64_t kRelu = 2;
+Tensor bias_act_fwd(const Tensor& x, const optional<Tensor>& bias, int64_t act) {
+  static auto f = op<Tensor(const Tensor&, const optional<Tensor>&, int64_t)>("slapo_b200::bias_act_fwd");
+  return f.call(x, bias, act);
+}
 std::tuple<Tensor, Tensor> bias_act_bwd(const Tensor& dy, const Tensor& x, const optional<Tensor>& bias,
                                         int64_t act) {
   static auto f = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const optional<Tensor>&,
@@ -88,8 +92,11 @@ struct LinearFn : public Function<LinearFn> {
     Tensor x2 = rows_of(x);
     Tensor y, at;         // at: where the activation's derivative is read off
     const bool gelu = act >= 0 && act != kRelu;
-    if (gelu) {
-      std::tie(y, at) = gemm_act_fwd(x2, weight, bias, act, transposed, keep, false);
+    if (gelu && transposed) {       // (the epilogue forms take W as [out, in])
+      at = gemm(x2, weight, c10::nullopt, -1, false, true, false);
+      y = bias_act_fwd(at, bias, act);
+    } else if (gelu) {
+      std::tie(y, at) = gemm_act_fwd(x2, weight, bias, act, keep, false);
     } else {
       y = gemm(x2, weight, bias, act, false, transposed, false);
       if (act >= 0) at = y;
@@ -139,7 +146,7 @@ struct MlpFn : public Function<MlpFn> {
     Tensor x2 = rows_of(x);
     Tensor h, at, y;
     if (act != kRelu) {
-      std::tie(h, at) = gemm_act_fwd(x2, w1, b1, act, false, keep, true);
+      std::tie(h, at) = gemm_act_fwd(x2, w1, b1, act, keep, true);
     } else {
       h = gemm(x2, w1, b1, act, false, false, false);
       at = h;
@@ -179,9 +186,9 @@ struct MlpFn : public Function<MlpFn> {
     }
     if (ctx->needs_input_grad(3)) out[3] = gemm(dy, h, c10::nullopt, -1, true, true, true);
     if (ctx->needs_input_grad(0) || ctx->needs_input_grad(1) || ctx->needs_input_grad(2)) {
-      static auto f = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, int64_t, bool)>(
+      static auto f = op<std::tuple<Tensor, Tensor>(const Tensor&, const Tensor&, const Tensor&, int64_t)>(
           "slapo_b200::gemm_act_bwd");
-      auto [dz, db1] = f.call(dy, w2, at, ctx->saved_data["act"].toInt(), false);
+      auto [dz, db1] = f.call(dy, w2, at, ctx->saved_data["act"].toInt());
       out[2] = db1;
       if (ctx->needs_input_grad(0))
         out[0] = gemm(dz, w1, c10::nullopt, -1, false, true, false).view(ctx->saved_data["shape"].toIntVector());
@@ -196,8 +203,7 @@ struct BiasActFn : public Function<BiasActFn> {
                         int64_t act) {
     ctx->saved_data["act"] = act;
     ctx->save_for_backward({x, or_undefined(bias)});
-    static auto f = op<Tensor(const Tensor&, const optional<Tensor>&, int64_t)>("slapo_b200::bias_act_fwd");
-    return f.call(x.contiguous(), bias, act);
+    return bias_act_fwd(x.contiguous(), bias, act);
   }
   static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
     const variable_list saved = ctx->get_saved_variables();

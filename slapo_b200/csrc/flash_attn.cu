@@ -644,20 +644,14 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  const int items = p.walk.items() * p.splits;
-  // row tile, (batch, head) and key tiles [j0, j0 + n) of a work item
-  auto item_at = [&](int item, int& tile, int& bh, int& j0) {
-    const int unit = p.splits == 1 ? item : item / p.splits;
-    p.walk.at(unit, tile, bh);
+  const int items = p.walk.items();       // (several row tiles: keys are not split)
+  // row tile, (batch, head) and number of key tiles of a work item
+  auto item_at = [&](int item, int& tile, int& bh) {
+    p.walk.at(item, tile, bh);
     int n = (p.Sk + kBlockN - 1) / kBlockN;
     if (p.causal) {
       const int last_key = min(p.Sk, min(tile * kBlockM + kBlockM, p.Sq) + diag);
       n = max(1, min(n, (last_key + kBlockN - 1) / kBlockN));
-    }
-    j0 = 0;
-    if (p.splits > 1) {     // (one row tile per head: every split has at least one key tile)
-      j0 = (item - unit * p.splits) * p.tiles_per_split;
-      n = max(1, min(p.tiles_per_split, n - j0));
     }
     return n;
   };
@@ -676,8 +670,8 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         Ring<kQ> q;
         Ring<kStages> r;
         for (int item = blockIdx.x; item < items && ok; item += gridDim.x, q.step()) {
-          int tile, bh, j0;
-          const int n = item_at(item, tile, bh, j0);
+          int tile, bh;
+          const int n = item_at(item, tile, bh);
           const int batch = bh / p.H, head = bh - batch * p.H;
           ok = false;
           if (!tc::mbar_wait(&q_empty[q.slot], q.phase ^ 1, abort_flag)) break;
@@ -688,7 +682,7 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                             tile * kBlockM, batch);
           for (int j = 0; j < n; ++j, r.step()) {
             ok = false;
-            const int k0 = (j0 + j) * kBlockN;
+            const int k0 = j * kBlockN;
             if (!tc::mbar_wait(&k_empty[r.slot], r.phase ^ 1, abort_flag)) break;
             tc::mbar_arrive_expect_tx(&k_full[r.slot], kTileBytes);
 #pragma unroll
@@ -712,8 +706,8 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         Ring<kStages> r;
         int u = 0;
         for (int item = blockIdx.x; item < items && ok; item += gridDim.x, q.step()) {
-          int tile, bh, j0;
-          const int n = item_at(item, tile, bh, j0);
+          int tile, bh;
+          const int n = item_at(item, tile, bh);
           if (!tc::mbar_wait(&q_full[q.slot], q.phase, abort_flag)) break;
           for (int j = 0; j < n; ++j, ++u, r.step()) {
             const int g = u & 1;
@@ -743,8 +737,8 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         Ring<kStages> r;
         int u = 0;
         for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-          int tile, bh, j0;
-          const int n = item_at(item, tile, bh, j0);
+          int tile, bh;
+          const int n = item_at(item, tile, bh);
           for (int j = 0; j < n; ++j, ++u, r.step()) {
             const int g = u & 1;
             const uint32_t ph = (u >> 1) & 1;
@@ -781,8 +775,8 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     int u = 0;
     int parts[2] = {0, 0};        // items that each group has had a part in
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-      int tile, bh, j0;
-      const int n = item_at(item, tile, bh, j0);
+      int tile, bh;
+      const int n = item_at(item, tile, bh);
       const int first = u;
       for (int j = 0; j < n; ++j, ++u) {
         const int g = u & 1, k = u >> 1;
@@ -850,41 +844,24 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
           if (two) v[i] = fmaf(__uint_as_float(y[i]), fb, v[i]);
         }
       };
-      if (p.splits > 1) {
-        // this split's share: unnormalised output, maximum and sum
-        const int split = item - item / p.splits * p.splits;
-        const int64_t at = (static_cast<int64_t>(split) * p.B * p.H + bh) * p.Sq + min(row, p.Sq - 1);
+      const float inv = l > 0.f ? 1.f / (l * (1.f - p.p_drop)) : 0.f;
+      fa *= inv;
+      fb *= inv;
+      T* dst = static_cast<T*>(p.O) +
+               ((static_cast<int64_t>(batch) * p.Sq + min(row, p.Sq - 1)) * p.H + head) * p.Dr;
 #pragma unroll 1
-        for (int c = 0; c < D; c += 16) {
-          float v[16];
-          columns(c, v);
-          if (row < p.Sq) {
+      for (int c = 0; c < D; c += 16) {
+        float v[16];
+        columns(c, v);
+        if (row < p.Sq) {
 #pragma unroll
-            for (int i = 0; i < 16; i += 8)
-              if (c + i < p.Dr) Vec8<float>::store(p.part_o + at * p.Dr + c + i, v + i);
-          }
+          for (int i = 0; i < 16; i += 8)      // padded columns are not part of the output
+            if (c + i < p.Dr) Vec8<T>::store(dst + c + i, v + i);
         }
-        if (row < p.Sq) p.part_ml[at] = make_float2(m, l);
-      } else {
-        const float inv = l > 0.f ? 1.f / (l * (1.f - p.p_drop)) : 0.f;
-        fa *= inv;
-        fb *= inv;
-        T* dst = static_cast<T*>(p.O) +
-                 ((static_cast<int64_t>(batch) * p.Sq + min(row, p.Sq - 1)) * p.H + head) * p.Dr;
-#pragma unroll 1
-        for (int c = 0; c < D; c += 16) {
-          float v[16];
-          columns(c, v);
-          if (row < p.Sq) {
-#pragma unroll
-            for (int i = 0; i < 16; i += 8)      // padded columns are not part of the output
-              if (c + i < p.Dr) Vec8<T>::store(dst + c + i, v + i);
-          }
-        }
-        if (row < p.Sq)
-          p.lse[static_cast<int64_t>(bh) * p.Sq + row] =
-              l > 0.f ? (m == -INFINITY ? 0.f : m) * 0.6931471805599453f + logf(l) : -INFINITY;
       }
+      if (row < p.Sq)
+        p.lse[static_cast<int64_t>(bh) * p.Sq + row] =
+            l > 0.f ? (m == -INFINITY ? 0.f : m) * 0.6931471805599453f + logf(l) : -INFINITY;
       tc::fence_before_sync();
     }
   } else {
@@ -922,14 +899,14 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
           cp_async4(dst + 128 + i, src + max(1 - p.Sq, min(d0 + i, p.Sk - 1)));
       }
     };
-    // a tile of the sequence: key tile j0 + j of a work item (j < n), u0 is the item's first
+    // a tile of the sequence: key tile j of a work item (j < n), u0 is the item's first
     struct Pos {
-      int item, tile, bh, j0, n, j, u0;
+      int item, tile, bh, n, j, u0;
     };
     // the group's first one from sequence number pos.u0 and work item pos.item on
     auto enter = [&](Pos& pos) {
       while (pos.item < items) {
-        pos.n = item_at(pos.item, pos.tile, pos.bh, pos.j0);
+        pos.n = item_at(pos.item, pos.tile, pos.bh);
         pos.j = (pos.u0 & 1) ^ g;
         if (pos.j < pos.n) return;
         pos.u0 += pos.n;
@@ -939,7 +916,7 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     Pos pos{};
     pos.item = blockIdx.x;
     enter(pos);
-    if (biased && pos.item < items) fetch_bias(pos.tile, pos.bh, pos.j0 + pos.j, 0);
+    if (biased && pos.item < items) fetch_bias(pos.tile, pos.bh, pos.j, 0);
     bool ok = true;
     uint32_t k = 0, part = 0;       // tiles and items of the group so far
     while (pos.item < items && ok) {
@@ -950,7 +927,7 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       Pos next = pos;
       for (; pos.j < pos.n; pos.j += 2, ++k) {
         const uint32_t ph = k & 1;
-        const int k0 = (pos.j0 + pos.j) * kBlockN;
+        const int k0 = pos.j * kBlockN;
         const float* bias = bias_buf + ph * L::kBiasFloats;
         if (pos.j + 2 >= pos.n) {
           next.u0 += pos.n;
@@ -968,7 +945,7 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
           }
           // this tile's biases are visible to the warp, and the other buffer's readers are done
           __syncwarp();
-          if (next.item < items) fetch_bias(next.tile, next.bh, next.j0 + next.j, ph ^ 1);
+          if (next.item < items) fetch_bias(next.tile, next.bh, next.j, ph ^ 1);
         }
         if (!tc::mbar_wait_warp(&s_full[g], ph, abort_flag)) { ok = false; break; }
         tc::fence_after_sync();

@@ -386,14 +386,13 @@ int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, 
   p.col_part = epi != nullptr ? epi->col_part : nullptr;
   p.c2_sum = epi != nullptr && epi->c2_sum ? 1 : 0;
   if (epi != nullptr && epi->kind != kEpiPlain) {
-    if (a_mn) return 1;
+    if (a_mn || b_mn != epi_backward(epi->kind)) return 1;
     if ((reinterpret_cast<uintptr_t>(p.Z) | reinterpret_cast<uintptr_t>(p.C2) |
          reinterpret_cast<uintptr_t>(p.bias)) & 15)
       return 1;
 #define GEMM_EPI(BN_, ST_, KIND_)                                                       \
   if (BN == BN_ && epi->kind == KIND_)                                                  \
-    return b_mn ? launch_variant<BN_, ST_, false, true, KIND_>(ta, tb, p, stream)       \
-                : launch_variant<BN_, ST_, false, false, KIND_>(ta, tb, p, stream);
+    return launch_variant<BN_, ST_, false, epi_backward(KIND_), KIND_>(ta, tb, p, stream);
 #define GEMM_EPIS(BN_, ST_)                                                      \
   GEMM_EPI(BN_, ST_, kEpiGelu) GEMM_EPI(BN_, ST_, kEpiGeluTanh)                  \
   GEMM_EPI(BN_, ST_, kEpiGeluBwd) GEMM_EPI(BN_, ST_, kEpiGeluTanhBwd) GEMM_EPI(BN_, ST_, kEpiReluBwd)

@@ -576,12 +576,11 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
   p.workspace = workspace;
 
   if (epi != nullptr && epi->kind != kEpiPlain) {
-    if (a_mn || p.splits != 1) return 1;
+    if (a_mn || b_mn != epi_backward(epi->kind) || p.splits != 1) return 1;
     if (epi_backward(epi->kind) && (reinterpret_cast<uintptr_t>(p.Z) & 15)) return 1;
 #define GEMM2_EPI(BN_, ST_, KIND_)                                                              \
   if (BN == BN_ && epi->kind == KIND_)                                                          \
-    return b_mn ? launch_pair_variant<BN_, ST_, kKSub, false, true, KIND_>(ta, tb, p, stream)   \
-                : launch_pair_variant<BN_, ST_, kKSub, false, false, KIND_>(ta, tb, p, stream);
+    return launch_pair_variant<BN_, ST_, kKSub, false, epi_backward(KIND_), KIND_>(ta, tb, p, stream);
 #define GEMM2_EPIS(BN_, ST_)                                                      \
   GEMM2_EPI(BN_, ST_, kEpiGelu) GEMM2_EPI(BN_, ST_, kEpiGeluTanh)                 \
   GEMM2_EPI(BN_, ST_, kEpiGeluBwd) GEMM2_EPI(BN_, ST_, kEpiGeluTanhBwd) GEMM2_EPI(BN_, ST_, kEpiReluBwd)

@@ -169,11 +169,11 @@ Tensor gemm(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& bias,
 }
 
 // act(a w^T + bias) with the activation (0 GeLU, 1 GeLU tanh) in the epilogue, and the value before it
-// (empty unless `keep`): the product, or with `sum` product + bias.  `transposed`: w is [K, N].
+// (empty unless `keep`): the product, or with `sum` product + bias.
 std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias,
-                                        int64_t act, bool transposed, bool keep, bool sum) {
+                                        int64_t act, bool keep, bool sum) {
   TORCH_CHECK(act == 0 || act == 1, "gemm_act_fwd: GeLU only");
-  GemmCall g(a, w, transposed);
+  GemmCall g(a, w, false);
   const void* bias_ptr = bias_words(bias, a, g.N);
   c10::cuda::CUDAGuard guard(a.device());
   Tensor y = at::empty({g.M, g.N}, a.options());
@@ -185,11 +185,10 @@ std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const 
 
 // dz = (dy w) * act'(z) and its column sums: the input gradient of the layer that follows an
 // activation, on to that activation's input.  z: for ReLU (act 2) the activation's output.  w is the
-// following layer's weight [K, N] (`transposed`: [N, K]).
-std::tuple<Tensor, Tensor> gemm_act_bwd(const Tensor& dy, const Tensor& w, const Tensor& z, int64_t act,
-                                        bool transposed) {
+// following layer's weight [K, N].
+std::tuple<Tensor, Tensor> gemm_act_bwd(const Tensor& dy, const Tensor& w, const Tensor& z, int64_t act) {
   TORCH_CHECK(act >= 0 && act <= 2, "gemm_act_bwd: unknown activation");
-  GemmCall g(dy, w, !transposed);
+  GemmCall g(dy, w, true);
   TORCH_CHECK(z.device() == dy.device() && z.is_contiguous() && z.scalar_type() == dy.scalar_type() && z.dim() == 2 &&
                   z.size(0) == g.M && z.size(1) == g.N,
               "gemm_act_bwd: z must be a contiguous [M, N] tensor of the operand dtype");
@@ -212,9 +211,9 @@ void register_gemm_ops(torch::Library& m) {
   m.def("gemm(Tensor a, Tensor b, Tensor? bias, int act, bool a_mn, bool b_mn) -> Tensor", &gemm);
   m.def("gemm_out(Tensor a, Tensor b, Tensor? bias, int act, bool a_mn, bool b_mn, Tensor? out, "
         "Tensor? pre_act, int impl, bool split_k) -> Tensor", &gemm_out);
-  m.def("gemm_act_fwd(Tensor a, Tensor w, Tensor? bias, int act, bool transposed, bool keep, bool sum=True) -> (Tensor, Tensor)",
+  m.def("gemm_act_fwd(Tensor a, Tensor w, Tensor? bias, int act, bool keep, bool sum=True) -> (Tensor, Tensor)",
         &gemm_act_fwd);
-  m.def("gemm_act_bwd(Tensor dy, Tensor w, Tensor z, int act, bool transposed) -> (Tensor, Tensor)",
+  m.def("gemm_act_bwd(Tensor dy, Tensor w, Tensor z, int act) -> (Tensor, Tensor)",
         &gemm_act_bwd);
   m.def("gemm2_splits(int M, int N, int K) -> int", [](int64_t M, int64_t N, int64_t K) -> int64_t {
     return slapo::gemm2_splits(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K),

@@ -42,11 +42,11 @@ def test_epilogue(m, k, n, act, dtype):
     code = NF._act_code(act)
     ops = native.ops()
     if act != "relu":
-        y, kept = ops.gemm_act_fwd(x, w, b, code, False, True)
+        y, kept = ops.gemm_act_fwd(x, w, b, code, True)
         assert _close(y, _act(z, act), TOL[dtype]) and _close(kept, z, TOL[dtype])
-        alone, none = ops.gemm_act_fwd(x, w, b, code, False, False)
+        alone, none = ops.gemm_act_fwd(x, w, b, code, False)
         assert torch.equal(alone, y) and none.numel() == 0
-        other, _ = ops.gemm_act_fwd(x, w.t().contiguous(), b, code, True, False)
+        other = ops.linear(x, w.t().contiguous(), b, code, True)       # W as [in, out]
         assert _close(other, _act(z, act), TOL[dtype])
     # the derivative behind the following layer's input gradient: dy [m, k2] w2 [k2, n]
     dy = torch.randn(m, k, device="cuda", dtype=dtype)
@@ -54,10 +54,9 @@ def test_epilogue(m, k, n, act, dtype):
     at = _act(z, act).to(dtype) if act == "relu" else z.to(dtype)
     zz = at.double().requires_grad_()
     (want,) = torch.autograd.grad(_act(zz, act), zz, dy.double() @ w2.double())
-    for weight, transposed in ((w2, False), (w2.t().contiguous(), True)):
-        dz, db = ops.gemm_act_bwd(dy, weight, at, code, transposed)
-        assert _close(dz, want, TOL[dtype])
-        assert _close(db, want.sum(0), TOL[dtype])
+    dz, db = ops.gemm_act_bwd(dy, w2, at, code)
+    assert _close(dz, want, TOL[dtype])
+    assert _close(db, want.sum(0), TOL[dtype])
     assert ops.device_status() == 0
 
 
@@ -66,7 +65,7 @@ def test_epilogue_keeps_infinities_and_nans():
     x[0, 0], x[1, 0], x[2, 0] = float("inf"), float("-inf"), float("nan")
     w = torch.ones(64, 64, device="cuda", dtype=BF)
     b = torch.zeros(64, device="cuda", dtype=BF)
-    y, z = native.ops().gemm_act_fwd(x, w, b, 0, False, True)
+    y, z = native.ops().gemm_act_fwd(x, w, b, 0, True)
     want = NF.bias_act(F.linear(x, w), b, "gelu")
     assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.isinf(y[0]).all()
     assert torch.isinf(z[:2]).all() and torch.isnan(z[2]).all() and (y[3:] == 0).all()

@@ -35,9 +35,16 @@ def test_equals_layer_then_activation(m, k, n, act, dtype):
         assert torch.equal(p, q), name
     with torch.no_grad():
         assert torch.equal(NF.linear(x, w, b, act), one[0])
-        summed = native.ops().gemm_act_fwd(x, w, b, NF._act_code(act), False, True, True)
+        summed = native.ops().gemm_act_fwd(x, w, b, NF._act_code(act), True, True)
         assert torch.equal(summed[0], one[0])
         assert torch.equal(summed[1], (NF.linear(x, w).float() + b.float()).to(dtype))
+    # W as [in, out]: product and activation apart
+    wt = w.detach().t().contiguous().requires_grad_()
+    y = native.ops().linear(x, wt, b, NF._act_code(act), True)
+    z = NF.linear_t(x, wt)
+    assert torch.equal(y, NF.bias_act(z, b, act))
+    for p, q in zip(torch.autograd.grad(y, [x, wt, b], dy), torch.autograd.grad(NF.bias_act(z, b, act), [x, wt, b], dy)):
+        assert torch.equal(p, q)
     assert native.ops().device_status() == 0
 
 

@@ -55,12 +55,12 @@ def test_refusals():
     ops = native.ops()
     x, w, b = _inputs(392, 64, 4104)
     for bias in (b[:4104].cpu(), b[:4096], b[:4104].float()):
-        for call in (lambda: ops.gemm_act_fwd(x, w, bias, 0, False, False),
+        for call in (lambda: ops.gemm_act_fwd(x, w, bias, 0, False),
                      lambda: ops.gemm(x, w, bias, -1, False, False), lambda: ops.linear(x, w, bias, 0, False)):
             with pytest.raises(RuntimeError):
                 call()
     with pytest.raises(RuntimeError):
-        ops.gemm_act_fwd(x, w, b[1:4105], 0, False, False)
+        ops.gemm_act_fwd(x, w, b[1:4105], 0, False)
     with pytest.raises(RuntimeError):
         ops.gemm(x, w.detach().cpu(), None, -1, False, False)
     w2 = torch.zeros(64, 4104, device="cuda", dtype=BF)
