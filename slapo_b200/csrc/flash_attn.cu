@@ -1199,12 +1199,6 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float
   // work on 64- or 128-wide tiles whose columns beyond D are zero-filled by the tile loads
   if (D < 8 || D > 128 || D % 8 != 0) return 1;
   if (B <= 0 || H <= 0 || Sq <= 0 || Sk <= 0) return 1;     // (no tensor map without an address)
-  const int Dt = D <= 64 ? 64 : 128;
-  CUtensorMap tq, tk, tv;
-  if (!make_tmap_bshd(&tq, q, B, Sq, H, D, q_strides[0], q_strides[1], q_strides[2], 128, bf16) ||
-      !make_tmap_bshd(&tk, k, B, Sk, H, D, k_strides[0], k_strides[1], k_strides[2], 128, bf16) ||
-      !make_tmap_bshd(&tv, v, B, Sk, H, D, v_strides[0], v_strides[1], v_strides[2], 128, bf16))
-    return 2;
   FlashFwdParams p;
   p.B = B; p.H = H; p.Sq = Sq; p.Sk = Sk; p.Dr = D; p.O = o; p.lse = lse; p.kbias = kbias; p.rel = rel;
   p.k_steps = (D + 15) / 16;
@@ -1227,22 +1221,28 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float
   p.idesc_pv = tc::instr_desc_f16(128, p.k_steps * 16, bf16 ? 1 : 0, false, true);
   const bool general = kbias != nullptr || rel != nullptr || causal || Sk % kBlockN != 0 || !(scale > 0.f);
   int rc;
-  // a single query sees all keys, causal or not
-  const bool decode = Sq == 1 && p.thr7 == 0 && rel == nullptr;
+  if (Sq == 1 && p.thr7 == 0 && rel == nullptr) {
+    // a single query sees all keys, causal or not; its kernel needs no tensor maps
+    rc = launch_flash_decode(q, k, v, o, lse, p.part_o, p.part_ml, kbias, B, H, Sk, D, q_strides, k_strides,
+                             v_strides, scale, p.splits, p.tiles_per_split * kBlockN, bf16, stream);
+  } else {
+    CUtensorMap tq, tk, tv;
+    if (!make_tmap_bshd(&tq, q, B, Sq, H, D, q_strides[0], q_strides[1], q_strides[2], 128, bf16) ||
+        !make_tmap_bshd(&tk, k, B, Sk, H, D, k_strides[0], k_strides[1], k_strides[2], 128, bf16) ||
+        !make_tmap_bshd(&tv, v, B, Sk, H, D, v_strides[0], v_strides[1], v_strides[2], 128, bf16))
+      return 2;
 #define FLASH_FWD_CASE(D_, T_)                                            \
   rc = general ? launch_fwd_d<D_, true, T_>(tq, tk, tv, p, stream)        \
                : launch_fwd_d<D_, false, T_>(tq, tk, tv, p, stream)
-  if (decode) {
-    rc = launch_flash_decode(q, k, v, o, lse, p.part_o, p.part_ml, kbias, B, H, Sk, D, q_strides, k_strides,
-                             v_strides, scale, p.splits, p.tiles_per_split * kBlockN, bf16, stream);
-  } else if (Dt == 64) {
-    if (bf16) FLASH_FWD_CASE(64, __nv_bfloat16);
-    else FLASH_FWD_CASE(64, __half);
-  } else {
-    if (bf16) FLASH_FWD_CASE(128, __nv_bfloat16);
-    else FLASH_FWD_CASE(128, __half);
-  }
+    if (D <= 64) {
+      if (bf16) FLASH_FWD_CASE(64, __nv_bfloat16);
+      else FLASH_FWD_CASE(64, __half);
+    } else {
+      if (bf16) FLASH_FWD_CASE(128, __nv_bfloat16);
+      else FLASH_FWD_CASE(128, __half);
+    }
 #undef FLASH_FWD_CASE
+  }
   if (rc != 0 || p.splits == 1) return rc;
   count_launch();
   const unsigned blocks = static_cast<unsigned>((rows + 3) / 4);

@@ -145,6 +145,8 @@ int launch_flash_decode(const void* q, const void* k, const void* v, void* o, fl
                         float scale, int splits, int keys_per_split, bool bf16, cudaStream_t stream) {
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15)
     return 1;
+  for (int i = 0; i < 3; ++i)
+    if ((i != 1 && q_strides[i] % 8) || k_strides[i] % 8 || v_strides[i] % 8) return 1;
   FlashDecodeParams p;
   p.q = q; p.k = k; p.v = v; p.o = o; p.lse = lse; p.part_o = part_o; p.part_ml = part_ml;
   p.qb = q_strides[0]; p.qh = q_strides[2];
