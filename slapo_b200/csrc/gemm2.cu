@@ -509,21 +509,27 @@ int gemm2_splits(int M, int N, int K, int bn) {
 
 // Small products are one wave of few tiles, whatever the tile: the launch, the first loads and
 // the epilogue of ONE tile are what they take, and narrow tiles have less of all three and put
-// more SMs on the weights.  Measured per call (us, B in L2; wide = the tile that large products
-// use, 256 x 256 per pair or, up to 128 rows, 128 x 256; - not measured with products issued as now):
-//     M x N x K             128 x 64   256 x 128 pair   wide
-//     8 x 2048 x 2048          9.3           -           -
-//     200 x 3072 x 768         5.7           -           -
-//     200 x 768 x 3072         9.7         13.3          -
-//     512 x 1024 x 1024        5.7           -           -
-//     768 x 768 x 64           4.2           -           -
-//     1024 x 1024 x 3072      10.5         14.4          -
-//     2048 x 1024 x 4096        -          18.5          -
-//     1024 x 3072 x 1024        -            -          13.7
+// more SMs on the weights.  Measured per call (us, operands in L2; - does not fit one wave; wide = the tile
+// that large products use, 256 x 256 per pair or, up to 128 rows, 128 x 256):
+//     M x N x K              64    128 (rows > 128: pair)   wide
+//     40 x 2048 x 2048       7.8         9.3                14.7
+//     128 x 768 x 3072      10.5        12.7                21.0
+//     128 x 9480 x 1024       -          7.9                11.1
+//     128 x 19200 x 1024      -           -                 12.8
+//     200 x 3072 x 768       6.4         8.9                12.6
+//     200 x 768 x 3072      10.4        13.8                22.5
+//     512 x 1024 x 1024      6.2         9.4                13.7
+//     768 x 768 x 64         4.8         7.5                 9.5
+//     1024 x 1024 x 3072    11.1        14.7                23.4
+//     640 x 1792 x 8192     21.4        26.4                45.3
+//     1024 x 1024 x 16384   36.8        47.9                81.4
+//     1000 x 2056 x 1024      -         10.4                14.4
+//     2048 x 1024 x 4096      -         18.5                28.3
+//     1024 x 3072 x 1024      -           -                 14.4
 // So: tiles of 64 columns while they fit one wave of CTAs, pairs of 128 columns while those fit one
 // wave of pairs, wide tiles beyond.  Up to 128 rows there is no pair tile: the narrowest of 64 / 128 /
 // 256 columns that fits one wave.
-GemmTile gemm_tile(int M, int N, int K) {
+GemmTile gemm_tile(int M, int N) {
   const int sms = sm_count();
   const int64_t rows = (M + PBM - 1) / PBM, pair_rows = (M + 2 * PBM - 1) / (2 * PBM);
   if (M <= PBM) {

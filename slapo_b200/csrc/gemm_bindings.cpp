@@ -100,7 +100,7 @@ Tensor gemm_out(const Tensor& a, const Tensor& b, const c10::optional<Tensor>& b
                   "): sizes must be multiples of 8 and pointers 16-byte aligned");
       return c;
     }
-    tile = slapo::gemm_tile(M, N, K);
+    tile = slapo::gemm_tile(M, N);
   }
   if (tile.pair) {
     float* ws = nullptr;
@@ -147,7 +147,7 @@ struct GemmCall {
     auto stream = at::cuda::getCurrentCUDAStream().stream();
     int* status = status_word(dev).data_ptr<int>();
     const int lda = static_cast<int>(a.stride(0)), ldb = static_cast<int>(w.stride(0));
-    const slapo::GemmTile tile = slapo::gemm_tile(M, N, K);
+    const slapo::GemmTile tile = slapo::gemm_tile(M, N);
     int rc = 5;
     if (epi.z == nullptr && !b_mn && slapo::gemm_rows_takes(M, N, K))
       rc = slapo::launch_gemm_rows(a.data_ptr(), w.data_ptr(), c.data_ptr(), bias, M, N, K, lda, ldb, N, bf16, -1,
@@ -215,6 +215,11 @@ void register_gemm_ops(torch::Library& m) {
         &gemm_act_fwd);
   m.def("gemm_act_bwd(Tensor dy, Tensor w, Tensor z, int act) -> (Tensor, Tensor)",
         &gemm_act_bwd);
+  // which tile a product without split K gets: a CTA pair's or one CTA's, and its columns (0: the widest)
+  m.def("gemm_tile(int M, int N) -> (bool, int)", [](int64_t M, int64_t N) -> std::tuple<bool, int64_t> {
+    const slapo::GemmTile t = slapo::gemm_tile(static_cast<int>(M), static_cast<int>(N));
+    return {t.pair, t.bn};
+  });
   m.def("gemm2_splits(int M, int N, int K) -> int", [](int64_t M, int64_t N, int64_t K) -> int64_t {
     return slapo::gemm2_splits(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K),
                                N > 128 ? 256 : 128);

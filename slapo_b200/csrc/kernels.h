@@ -49,7 +49,7 @@ int gemm2_splits(int M, int N, int K, int bn);
 // Tile for a product: CTA pairs or single CTAs, and the tile's columns (`bn` of the launchers;
 // there 0 = the widest that N fills).
 struct GemmTile { bool pair; int bn; };
-GemmTile gemm_tile(int M, int N, int K);
+GemmTile gemm_tile(int M, int N);
 int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bias, int M, int N,
                  int K, int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act,
                  int bn, float* workspace, int* status, cudaStream_t stream,

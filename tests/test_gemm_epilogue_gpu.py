@@ -25,15 +25,19 @@ def _close(got, want, tol):
     return ((got.double() - want).norm() / want.norm().clamp(min=1e-30)).item() < tol
 
 
-# rows, inner, columns: one narrow tile; a ragged one of each kind (single CTA of 64 / 128 / 256 columns,
-# pairs of 128 / 256); several row blocks and work items
-SHAPES = [(8, 64, 8), (40, 72, 200), (128, 64, 4096), (120, 64, 19200), (136, 264, 136), (264, 64, 72),
-          (200, 3072, 768), (1000, 2560, 1096), (2056, 64, 2056), (33 * 8, 8, 24)]
+# rows, inner, columns, and the tile (of a CTA pair, its columns; 0: 256): narrow ones, a ragged one of each other
+# kind, several row blocks and work items, more than one band of row tiles and a ragged last one
+ONE64, ONE128, ONE256, PAIR128, PAIR256 = (False, 64), (False, 128), (False, 0), (True, 128), (True, 0)
+SHAPES = [(8, 64, 8, ONE64), (40, 72, 200, ONE64), (128, 64, 4096, ONE64), (120, 64, 19200, ONE256),
+          (136, 264, 136, ONE64), (264, 64, 72, ONE64), (200, 3072, 768, ONE64), (1000, 2560, 1096, ONE64),
+          (2056, 64, 2056, PAIR256), (33 * 8, 8, 24, ONE64), (128, 64, 64 * 148 + 8, ONE128),
+          (392, 64, 4104, PAIR128), (1000, 72, 2056, PAIR128), (2312, 72, 4360, PAIR256)]
 
 
 @pytest.mark.parametrize("act,dtype", [("gelu", BF), ("gelu_new", FP), ("relu", BF)])
-@pytest.mark.parametrize("m,k,n", SHAPES)
-def test_epilogue(m, k, n, act, dtype):
+@pytest.mark.parametrize("m,k,n,tile", SHAPES)
+def test_epilogue(m, k, n, tile, act, dtype):
+    assert tuple(native.ops().gemm_tile(m, n)) == tile
     torch.manual_seed(m + k + n)
     x = torch.randn(m, k, device="cuda", dtype=dtype)
     w = (torch.randn(n, k, device="cuda") * k ** -0.5).to(dtype)
@@ -57,6 +61,28 @@ def test_epilogue(m, k, n, act, dtype):
     dz, db = ops.gemm_act_bwd(dy, w2, at, code)
     assert _close(dz, want, TOL[dtype])
     assert _close(db, want.sum(0), TOL[dtype])
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("m,k,n,split", [
+    (2312, 72, 4360, False),        # a band of eight row tiles and one of two, 18 column tiles
+    (4104, 64, 4104, False),        # two whole bands and one of a ragged tile
+    (264, 2048, 4360, True)])       # a band of two, two pairs per tile
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, True)])
+def test_bands_of_row_tiles(m, k, n, split, a_mn, b_mn):
+    torch.manual_seed(n)
+    ops = native.ops()
+    a = torch.randn((k, m) if a_mn else (m, k), device="cuda", dtype=BF)
+    w = torch.randn((k, n) if b_mn else (n, k), device="cuda", dtype=BF)
+    b = torch.randn(n, device="cuda", dtype=BF)
+    assert (ops.gemm2_splits(m, n, k) > 1) == split
+    c = ops.gemm_out(a, w, b, -1, a_mn, b_mn, None, None, 0, split)
+    want = (a.double().t() if a_mn else a.double()) @ (w.double() if b_mn else w.double().t()) + b.double()
+    # each 128 x 128 block of its own: fp32 sums and one rounding
+    err = (c.double() - want).square()
+    for s, t in zip(err.split(128), want.square().split(128)):
+        for p, q in zip(s.split(128, 1), t.split(128, 1)):
+            assert (p.sum() / q.sum()).sqrt().item() < 2.0 ** -8
     assert ops.device_status() == 0
 
 

@@ -17,7 +17,7 @@ BF, FP = torch.bfloat16, torch.float16
     (128, 64 * 148 + 8, 64, False, True),
     (128, 128 * 148 + 8, 64, False, False),
     (129, 64, 72, False, True),
-    (200, 768, 2048, False, False),        # the longest contraction on narrow tiles
+    (200, 768, 2048, False, False),        # narrow tiles, whatever the contraction
     (200, 768, 2056, False, True),
     (384, 4096, 1024, False, False),       # 128-column pairs
     (520, 9216, 136, False, False),        # beyond one wave of them
