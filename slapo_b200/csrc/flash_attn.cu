@@ -19,13 +19,15 @@
 // P has columns of its own: S of the next tile is computed while the softmax warps work on this
 // one.
 //
+// Two other kernels take what this one is not best at: heads wider than 64 with several row tiles
+// (flash_fwd_groups_kernel below) and a single query (flash_decode.cu).
+//
 // What bounds it: the special-function unit (one exp2 per score, 1024 cycles per 128 x 128 tile
 // and SM) next to the issue slots of the softmax warps.  One thread per whole row needs no
 // exchange between warps; for D = 64 two independent CTAs fill each other's waits.
 // Measured (L2 flushed; P through shared memory, O folded in registers, one work item per CTA ->
-// now): 32 x 512 x 16 heads of 64, p 0.1: 126 -> 114 us; 4 x 2048 x 16 x 128 causal: 302 -> 137 us; 4 x
-// 1000 x 32 x 80 causal with key bias: 180 -> 105 us; 8 x 512 x 16 x 64 with T5's bias, key bias and p
-// 0.1: 66 -> 47 us; 1 query x 1500 keys x 4 x 12 x 128, keys split: 52 -> 21 us with the combine kernel.
+// now): 32 x 512 x 16 heads of 64, p 0.1: 126 -> 106 us; 8 x 512 x 16 x 64 with T5's bias, key bias and p
+// 0.1: 66 -> 45 us; 60 queries x 2000 keys x 2 x 8 x 128, keys split: 15 us with the combine kernel.
 //
 // Biases are added from shared memory, which asynchronous copies fill a tile ahead: a warp's 32
 // queries see 159 distances in a tile of 128 keys, against 128 loads per query.  Fetched by each
@@ -1170,11 +1172,14 @@ static int launch_fwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
 }
 
 // Work items per row tile.  One row tile per (batch, head) - generation, short queries - and at
-// most half as many of them as resident CTAs (two per SM for D = 64, one beyond): the keys are split
-// as far as one wave of CTAs takes them.  More items than that wait for one another (1 query x 1500
-// keys, D = 128, 128 heads on 148 SMs: two splits 33 us, none 27).  The combine kernel has to be
-// earned by a shorter chain: four tiles less, at 1.6 - 2 us each (1 query x 1000 keys x 12 heads: 20 ->
-// 14 us; 300 keys: 12 -> 14).
+// most half as many of them as resident CTAs of flash_fwd_kernel (two per SM for D <= 64, one beyond): the
+// keys are split as far as one wave of CTAs takes them.  The combine kernel, 3 us, has to be earned by a
+// chain of four tiles less.  Several queries (1.4 - 1.7 us a tile), none -> split: 60 queries x 8 heads of 64: 600 keys 13.0 ->
+// 10.3 us, 2000 keys 31 -> 14; 5 queries x 300 keys: 9.6 -> 9.9.  One query (flash_decode_kernel, 0.6 us for 128 keys
+// with D <= 64 and 1.1 beyond), heads x keys x D: 12 x 2000 x 64: 13.0 -> 10.2, 12 x 8000 x 64: 40 -> 15, 12 x 1000 x 128:
+// 12.7 -> 8.9, 48 x 2000 x 128: 21.9 -> 14.3, 74 x 4000 x 128: 42 -> 30, 48 x 450 x 128: 8.0 -> 8.3.  For one query with
+// D <= 64 the line lies too low: seven tiles and one item per SM would be right (12 x 600 x 64: 6.5 -> 7.6, 48 x
+// 1000 x 64: 8.5 -> 11.0, 96 x 2000 x 64: 13.0 -> 16.4).
 int flash_fwd_splits(int B, int H, int Sq, int Sk, int D) {
   const int tiles = (Sk + kBlockN - 1) / kBlockN;
   const int64_t bh = static_cast<int64_t>(B) * H;

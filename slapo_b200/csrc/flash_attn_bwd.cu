@@ -894,9 +894,11 @@ static bool allow_smem(K kernel, int bytes, bool& configured) {
 }
 
 // `early`: the kernel's prologue may run under the end of the kernel before it (it waits in
-// pdl_wait), which saves 2 - 4 us of a short backward.  CTAs that go round several times were slower
-// for it: 768 + 768 items of 3 tiles, side by side, 106 -> 125 us (128 + 128 of 1: 27 -> 23), one pass
-// after the other 2048 + 2048 of 4, causal, 226 -> 241 (384 + 384 of 3, dropout: 75 -> 74).
+// pdl_wait), which saves up to 2 us of a short backward (late -> early: 1 x 512 x 16 x 64: 18.2 -> 17.5 us, 1 x 1024 x 12 x
+// 64: 30.7 -> 28.7, 4 x 512 x 16 x 64 in two launches: 40.4 -> 38.8).  CTAs that go round several times are
+// slower for it where their items differ or both passes are at work: 4 x 1024 x 12 x 64 causal, side by
+// side: 63.9 -> 75.4; 64 x 128 x 12 x 64, p 0.1, side by side: 53.3 -> 66.7; 32 x 512 x 16 x 64 causal, one after the
+// other: 172.8 -> 178.1 (without a mask 203.3 -> 200.7).
 template <typename... P, typename... A>
 static int launch_bwd(void (*kernel)(P...), int ctas, int smem, bool early, cudaStream_t stream,
                       const A&... args) {
@@ -970,18 +972,22 @@ static int round128(int n) { return (n + 127) / 128 * 128; }
 // side the passes fill the waves that each alone would leave partly empty and save a launch; one
 // after the other the dK / dV pass reads the keep bits that the dQ pass drew instead of drawing them
 // again, and each pass has its tensors in L2 to itself.  Weighed as rounds of work items, in tiles
-// of the dQ pass: a tile of dK / dV takes 1.2 of them (2 with the relative bias's gradient, 0.3 more
-// drawing), an item a quarter more (D = 128: 1.5, its accumulators leave tensor memory without a
-// second set to go on with), a launch 1.5; both in one came out 5 % over that.  Under a causal mask items differ and the heaviest go first, so that
-// no whole rounds are lost in two launches or one: side by side up to 5 waves of each.
-// Measured with passes over whole tiles, two launches -> one (us): 1 x 512 x 16 x 64: 33 -> 22; 1 x 2048 x 12 x 64 causal: 102 -> 79;
-// 4 x 1024 x 16 x 128: 199 -> 188; 4 x 256 x 12 x 64 with dropout: 33 -> 25; but 32 x 512 x 16 x 64 with
-// dropout 367 -> 420, without 258 -> 265, causal 225 -> 236.
+// of the dQ pass: a tile of dK / dV takes 1.2 of them (D = 128: 1.45; 2 with the relative bias's gradient, 0.3
+// more drawing), an item a quarter more (D = 128: 1.5, its accumulators leave tensor memory without a
+// second set to go on with), a launch 1.5; both in one came out 5 % over that.  Under a causal mask items
+// differ and the heaviest go first, so that no whole rounds are lost in two launches or one: side by side
+// up to 5 waves of each.
+// Measured, two launches -> one (us).  Taken side by side: 1 x 512 x 16 x 64: 23.5 -> 17.5; 1 x 2048 x 12 x 64 causal: 83 -> 66; 4 x
+// 256 x 12 x 64, p 0.1: 23.5 -> 16.8; 1 x 512 x 16 x 128: 31 -> 23; 4 x 1024 x 16 x 128: 143 -> 135, causal 113 -> 110;
+// 1 x 2048 x 16 x 128 causal: 110 -> 94.  Not: 4 x 512 x 16 x 64: 38.7 -> 41.8; 32 x 512 x 16 x 64, p 0.1: 253 -> 298,
+// without 203 -> 244, causal 173 -> 236; 4 x 2048 x 16 x 128: 409 -> 436; 32 x 256 x 16 x 128: 113 -> 127.  Of 37 shapes the
+// rule misses the better one by 4 - 6 % in two (2 x 1024 x 16 x 128, p 0.1: 93.4, not 88.5) and by at most 2.5 % in
+// the others.
 static int both_q_ctas(int64_t q_items, int64_t k_items, int64_t q_item_tiles, int64_t q_tiles, int D,
                        bool causal, bool rel, bool drop) {
   const int64_t sms = sm_count();
   const double item = D <= 64 ? 0.25 : 1.5;
-  const double k_tile = rel ? 2.0 : 1.2;
+  const double k_tile = rel ? 2.0 : (D <= 64 ? 1.2 : 1.45);
   const double q_item = q_item_tiles + item, k_item = q_tiles * k_tile + item;
   const double k_item_draws = q_tiles * (k_tile + (drop ? 0.3 : 0.0)) + item;
   if (q_items + k_items <= sms) return static_cast<int>(q_items);
