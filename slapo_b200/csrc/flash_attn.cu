@@ -99,6 +99,100 @@ struct FlashFwdParams {
   int* status;
 };
 
+// ---- what a softmax warp of either kernel does with the scores of its 32 query rows and 128 keys ----
+// Biases in shared memory: the tile's 128 key biases, then the relative bias of the 32 + 128 - 1 distances
+// between the warp's queries and the tile's keys.
+constexpr int kBiasFloats = 128 + 160;
+
+// Biases of key tile `jt` of a work item on their way to `dst`: copied a tile ahead, element by
+// element (rows start anywhere).  What lies outside of the tensors is masked later.
+__device__ __forceinline__ void fwd_fetch_bias(const FlashFwdParams& p, float* dst, int tile, int quarter, int lane,
+                                               int bh, int jt) {
+  const int batch = bh / p.H, head = bh - batch * p.H, k0 = jt * kBlockN;
+  if (p.kbias != nullptr) {
+    const float* src = p.kbias + static_cast<int64_t>(batch) * p.Sk;
+#pragma unroll
+    for (int i = lane; i < 128; i += 32) cp_async4(dst + i, src + min(k0 + i, p.Sk - 1));
+  }
+  if (p.rel != nullptr) {
+    // key - query from that of the warp's last row and the first key on
+    const float* src = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + p.Sq - 1;
+    const int d0 = k0 - (tile * kBlockM + quarter * 32 + 31);
+#pragma unroll
+    for (int i = lane; i < 160; i += 32)
+      cp_async4(dst + 128 + i, src + max(1 - p.Sq, min(d0 + i, p.Sk - 1)));
+  }
+}
+
+// They have arrived, are visible to the warp, and the readers of its other buffer are done.
+__device__ __forceinline__ void fwd_land_bias(const FlashFwdParams& p, float* bias, int lane) {
+  cp_async_wait();
+  if (p.kbias != nullptr) {
+#pragma unroll
+    for (int i = lane; i < 128; i += 32) bias[i] *= kLog2e;      // (the elements that this lane copied)
+  }
+  __syncwarp();
+}
+
+// A row's scores, scaled to the log2 domain, plus its biases
+__device__ __forceinline__ void fwd_add_bias(const FlashFwdParams& p, uint32_t (&raw)[4][32], const float* bias,
+                                             int lane) {
+  const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2);
+  const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
+  if (p.kbias != nullptr) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int i = 0; i < 32; i += 4) {
+        const float4 b = *reinterpret_cast<const float4*>(bias + c * 32 + i);
+        f2_store(raw[c] + i, f2_fma(f2_load(raw[c] + i), scale2, f2_pack(b.x, b.y)));
+        f2_store(raw[c] + i + 2, f2_fma(f2_load(raw[c] + i + 2), scale2, f2_pack(b.z, b.w)));
+      }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int i = 0; i < 32; i += 2) f2_store(raw[c] + i, f2_mul(f2_load(raw[c] + i), scale2));
+  }
+  if (p.rel != nullptr) {
+    // neighbouring lanes (queries) read neighbouring words
+    const float* rel = bias + 128 + 31 - lane;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int i = 0; i < 32; i += 2)
+        f2_store(raw[c] + i,
+                 f2_fma(f2_pack(rel[c * 32 + i], rel[c * 32 + i + 1]), log2e2, f2_load(raw[c] + i)));
+  }
+}
+
+// -inf for keys that a row does not see, of the tile from k0 on; row0: the warp's first row
+__device__ __forceinline__ void fwd_mask(const FlashFwdParams& p, uint32_t (&raw)[4][32], int k0, int row0,
+                                         int lane) {
+  const int diag = p.Sk - p.Sq;         // key j visible to query i iff j <= i + diag (causal)
+  const int first_limit = p.causal ? min(p.Sk, row0 + diag + 1) : p.Sk;
+  if (k0 + kBlockN > first_limit) {     // some lane of the warp masks something
+    const int limit = (p.causal ? min(p.Sk, row0 + lane + diag + 1) : p.Sk) - k0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint32_t seen = low_bits(limit - c * 32);
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (!(seen & (1u << i))) raw[c][i] = 0xff800000u;   // -inf
+    }
+  }
+}
+
+__device__ __forceinline__ float fwd_max(const uint32_t (&raw)[4][32]) {
+  float mm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // 4 chains for ILP
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int i = 0; i < 32; i += 2)
+      mm[c] = fmaxf(mm[c], fmaxf(__uint_as_float(raw[c][i]), __uint_as_float(raw[c][i + 1])));
+  return fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3]));
+}
+
 template <int D>
 struct FwdSmem {
   static constexpr int kTile = 128 * D * 2;          // one [128 x D] 16-bit tile
@@ -106,9 +200,7 @@ struct FwdSmem {
   static constexpr int kCtas = D == 64 ? 2 : 1;      // per SM: shared memory and TMEM columns
   static constexpr int kK = kTile;
   static constexpr int kV = kK + kStages * kTile;
-  // per softmax warp, twice (this tile's and the next one's): the tile's 128 key biases and the
-  // relative bias of the 32 + 128 - 1 distances between its queries and the tile's keys
-  static constexpr int kBiasFloats = 128 + 160;
+  // (per softmax warp, twice: this tile's biases and the next one's)
   static constexpr int kBias = kV + kStages * kTile;
   static constexpr int kBars = kBias + 4 * 2 * kBiasFloats * 4;
   static constexpr int kTotal = kBars + 20 * 8 + 1024;
@@ -300,7 +392,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const int quarter = warp & 3;
     const int row_in_tile = quarter * 32 + lane;
     const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    float* bias_buf = reinterpret_cast<float*>(smem + L::kBias) + (warp - 2) * 2 * L::kBiasFloats;
+    float* bias_buf = reinterpret_cast<float*>(smem + L::kBias) + (warp - 2) * 2 * kBiasFloats;
     uint64_t seed = 0, offset = 0;
     if (p.p_drop > 0.f) philox_unpack(p.rng, seed, offset);
     const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
@@ -309,24 +401,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // to them (or the scale would turn the maximum around)
     const bool biased = kGeneral && (p.kbias != nullptr || p.rel != nullptr || !(p.scale_log2 > 0.f));
     const float sc = biased ? 1.f : p.scale_log2;
-    // Biases of key tile `jt` of a work item on their way into buffer `buf`: copied a tile ahead,
-    // element by element (rows start anywhere).  What lies outside of the tensors is masked later.
     auto fetch_bias = [&](int tile, int bh, int jt, int buf) {
-      float* dst = bias_buf + buf * L::kBiasFloats;
-      const int batch = bh / p.H, head = bh - batch * p.H, k0 = jt * kBlockN;
-      if (p.kbias != nullptr) {
-        const float* src = p.kbias + static_cast<int64_t>(batch) * p.Sk;
-#pragma unroll
-        for (int i = lane; i < 128; i += 32) cp_async4(dst + i, src + min(k0 + i, p.Sk - 1));
-      }
-      if (p.rel != nullptr) {
-        // key - query from that of the warp's last row and the first key on
-        const float* src = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + p.Sq - 1;
-        const int d0 = k0 - (tile * kBlockM + quarter * 32 + 31);
-#pragma unroll
-        for (int i = lane; i < 160; i += 32)
-          cp_async4(dst + 128 + i, src + max(1 - p.Sq, min(d0 + i, p.Sk - 1)));
-      }
+      fwd_fetch_bias(p, bias_buf + buf * kBiasFloats, tile, quarter, lane, bh, jt);
     };
     bool ok = true;
     int t = 0;
@@ -342,22 +418,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int row = tile * kBlockM + row_in_tile;
       const uint64_t drop_row_base =
           (static_cast<uint64_t>(bh) * p.Sq + min(row, p.Sq - 1)) * sk16;
-      int key_limit = p.Sk;
-      if (p.causal) key_limit = min(key_limit, row + diag + 1);
       float m_ref = -INFINITY;
       uint64_t l2 = 0;      // two fp32 partial row sums
       for (int j = 0; j < n; ++j, ++t) {
         const int k0 = (j0 + j) * kBlockN;
-        const float* bias = bias_buf + (t & 1) * L::kBiasFloats;
+        const float* bias = bias_buf + (t & 1) * kBiasFloats;
         if (kGeneral && biased) {
-          cp_async_wait();
-          if (p.kbias != nullptr) {
-#pragma unroll
-            for (int i = lane; i < 128; i += 32)      // (the elements that this lane copied)
-              bias_buf[(t & 1) * L::kBiasFloats + i] *= kLog2e;
-          }
-          // this tile's biases are visible to the warp, and the other buffer's readers are done
-          __syncwarp();
+          fwd_land_bias(p, bias_buf + (t & 1) * kBiasFloats, lane);
           if (j + 1 < n) {
             fetch_bias(tile, bh, j0 + j + 1, (t + 1) & 1);
           } else if (item + static_cast<int>(gridDim.x) < items) {
@@ -376,46 +443,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(s_free);
         if constexpr (kGeneral) {
-          if (biased) {
-            const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2);
-            const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
-            const bool key_bias = p.kbias != nullptr;
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-              for (int i = 0; i < 32; i += 4) {
-                float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (key_bias) b = *reinterpret_cast<const float4*>(bias + c * 32 + i);
-                f2_store(raw[c] + i, f2_fma(f2_load(raw[c] + i), scale2, f2_pack(b.x, b.y)));
-                f2_store(raw[c] + i + 2, f2_fma(f2_load(raw[c] + i + 2), scale2, f2_pack(b.z, b.w)));
-              }
-            if (p.rel != nullptr) {
-              // neighbouring lanes (queries) read neighbouring words
-              const float* rel = bias + 128 + 31 - lane;
-#pragma unroll
-              for (int c = 0; c < 4; ++c)
-#pragma unroll
-                for (int i = 0; i < 32; i += 2)
-                  f2_store(raw[c] + i, f2_fma(f2_pack(rel[c * 32 + i], rel[c * 32 + i + 1]), log2e2,
-                                              f2_load(raw[c] + i)));
-            }
-          }
-          const int first_limit = p.causal ? min(p.Sk, tile * kBlockM + quarter * 32 + diag + 1) : p.Sk;
-          if (k0 + kBlockN > first_limit) {     // some lane of the warp masks something
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (k0 + c * 32 + i >= key_limit) raw[c][i] = 0xff800000u;   // -inf
-          }
+          if (biased) fwd_add_bias(p, raw, bias, lane);
+          fwd_mask(p, raw, k0, tile * kBlockM + quarter * 32, lane);
         }
-        float mm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // 4 chains for ILP
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; i += 2)
-            mm[c] = fmaxf(mm[c], fmaxf(__uint_as_float(raw[c][i]), __uint_as_float(raw[c][i + 1])));
-        const float m_tile = fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3])) * sc;
+        const float m_tile = fwd_max(raw) * sc;
         // P of the tile before has been read (and O includes it)
         if (t > 0 && !tc::mbar_wait_warp(pv_done, (t - 1) & 1, abort_flag)) { ok = false; break; }
         tc::fence_after_sync();
@@ -559,9 +590,7 @@ struct GroupsSmem {
   static constexpr int kStages = 2;                  // K and V rings
   static constexpr int kK = kQ * kTile;
   static constexpr int kV = kK + kStages * kTile;
-  // per softmax warp, twice (this tile's and the next one's): the tile's 128 key biases and the
-  // relative bias of the 32 + 128 - 1 distances between its queries and the tile's keys
-  static constexpr int kBiasFloats = 128 + 160;
+  // (per softmax warp, twice: this tile's biases and the next one's)
   static constexpr int kBias = kV + kStages * kTile;
   static constexpr int kAlpha = kBias + 8 * 2 * kBiasFloats * 4;     // [group][tile parity][128] floats
   static constexpr int kMl = kAlpha + 2 * 2 * 128 * 4;               // [group][item parity][128] float2
@@ -873,7 +902,7 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     const int g = (warp - 4) >> 2;        // takes tiles g, g + 2, ... of the CTA's sequence
     const int row_in_tile = quarter * 32 + lane;
     const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    float* bias_buf = reinterpret_cast<float*>(smem + L::kBias) + (warp - 4) * 2 * L::kBiasFloats;
+    float* bias_buf = reinterpret_cast<float*>(smem + L::kBias) + (warp - 4) * 2 * kBiasFloats;
     PhiloxUniform rng{};
     if (p.p_drop > 0.f) rng = philox_uniform(p.rng);
     const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
@@ -882,24 +911,8 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     // to them (or the scale would turn the maximum around)
     const bool biased = kGeneral && (p.kbias != nullptr || p.rel != nullptr || !(p.scale_log2 > 0.f));
     const float sc = biased ? 1.f : p.scale_log2;
-    // Biases of key tile `jt` of a work item on their way into buffer `buf`: copied a tile ahead,
-    // element by element (rows start anywhere).  What lies outside of the tensors is masked later.
     auto fetch_bias = [&](int tile, int bh, int jt, int buf) {
-      float* dst = bias_buf + buf * L::kBiasFloats;
-      const int batch = bh / p.H, head = bh - batch * p.H, k0 = jt * kBlockN;
-      if (p.kbias != nullptr) {
-        const float* src = p.kbias + static_cast<int64_t>(batch) * p.Sk;
-#pragma unroll
-        for (int i = lane; i < 128; i += 32) cp_async4(dst + i, src + min(k0 + i, p.Sk - 1));
-      }
-      if (p.rel != nullptr) {
-        // key - query from that of the warp's last row and the first key on
-        const float* src = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + p.Sq - 1;
-        const int d0 = k0 - (tile * kBlockM + quarter * 32 + 31);
-#pragma unroll
-        for (int i = lane; i < 160; i += 32)
-          cp_async4(dst + 128 + i, src + max(1 - p.Sq, min(d0 + i, p.Sk - 1)));
-      }
+      fwd_fetch_bias(p, bias_buf + buf * kBiasFloats, tile, quarter, lane, bh, jt);
     };
     // a tile of the sequence: key tile j of a work item (j < n), u0 is the item's first
     struct Pos {
@@ -930,7 +943,7 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       for (; pos.j < pos.n; pos.j += 2, ++k) {
         const uint32_t ph = k & 1;
         const int k0 = pos.j * kBlockN;
-        const float* bias = bias_buf + ph * L::kBiasFloats;
+        const float* bias = bias_buf + ph * kBiasFloats;
         if (pos.j + 2 >= pos.n) {
           next.u0 += pos.n;
           next.item += gridDim.x;
@@ -939,14 +952,7 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
           next.j = pos.j + 2;
         }
         if (kGeneral && biased) {
-          cp_async_wait();
-          if (p.kbias != nullptr) {
-#pragma unroll
-            for (int i = lane; i < 128; i += 32)      // (the elements that this lane copied)
-              bias_buf[ph * L::kBiasFloats + i] *= kLog2e;
-          }
-          // this tile's biases are visible to the warp, and the other buffer's readers are done
-          __syncwarp();
+          fwd_land_bias(p, bias_buf + ph * kBiasFloats, lane);
           if (next.item < items) fetch_bias(next.tile, next.bh, next.j, ph ^ 1);
         }
         if (!tc::mbar_wait_warp(&s_full[g], ph, abort_flag)) { ok = false; break; }
@@ -956,54 +962,10 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         for (int c = 0; c < 4; ++c) tc::tmem_ld_x32(tmem_row + kColS + g * 128 + c * 32, raw[c]);
         tc::tmem_ld_wait();
         if constexpr (kGeneral) {
-          if (biased) {
-            const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2);
-            const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
-            if (p.kbias != nullptr) {
-#pragma unroll
-              for (int c = 0; c < 4; ++c)
-#pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                  const float4 b = *reinterpret_cast<const float4*>(bias + c * 32 + i);
-                  f2_store(raw[c] + i, f2_fma(f2_load(raw[c] + i), scale2, f2_pack(b.x, b.y)));
-                  f2_store(raw[c] + i + 2, f2_fma(f2_load(raw[c] + i + 2), scale2, f2_pack(b.z, b.w)));
-                }
-            } else {
-#pragma unroll
-              for (int c = 0; c < 4; ++c)
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) f2_store(raw[c] + i, f2_mul(f2_load(raw[c] + i), scale2));
-            }
-            if (p.rel != nullptr) {
-              // neighbouring lanes (queries) read neighbouring words
-              const float* rel = bias + 128 + 31 - lane;
-#pragma unroll
-              for (int c = 0; c < 4; ++c)
-#pragma unroll
-                for (int i = 0; i < 32; i += 2)
-                  f2_store(raw[c] + i, f2_fma(f2_pack(rel[c * 32 + i], rel[c * 32 + i + 1]), log2e2,
-                                              f2_load(raw[c] + i)));
-            }
-          }
-          const int first_limit = p.causal ? min(p.Sk, pos.tile * kBlockM + quarter * 32 + diag + 1) : p.Sk;
-          if (k0 + kBlockN > first_limit) {     // some lane of the warp masks something
-            const int limit = (p.causal ? min(p.Sk, row + diag + 1) : p.Sk) - k0;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const uint32_t seen = low_bits(limit - c * 32);
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (!(seen & (1u << i))) raw[c][i] = 0xff800000u;   // -inf
-            }
-          }
+          if (biased) fwd_add_bias(p, raw, bias, lane);
+          fwd_mask(p, raw, k0, pos.tile * kBlockM + quarter * 32, lane);
         }
-        float mm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // 4 chains for ILP
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; i += 2)
-            mm[c] = fmaxf(mm[c], fmaxf(__uint_as_float(raw[c][i]), __uint_as_float(raw[c][i + 1])));
-        const float m_new = fmaxf(m_ref, fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3])) * sc);
+        const float m_new = fmaxf(m_ref, fwd_max(raw) * sc);
         const float alpha = m_new == m_ref ? 1.f : exp2f(m_ref - m_new);
         s_alpha[(g * 2 + ph) * 128 + row_in_tile] = alpha;
         __syncwarp();
