@@ -604,8 +604,8 @@ struct GroupsSmem {
 // flash_fwd_kernel has one softmax warp per scheduler at this width and keeps all of that on the chain of
 // a tile.  Bound now: S of a group waits for its P V (512 columns hold two S and two O, P lies over S),
 // 1900 of the 4700 cycles between two tiles of a group.
-// Measured, flash_fwd_kernel -> this (us): 4 x 2048 x 16 x 128 causal: 137 -> 116; 4 x 1000 x 32 x 80 causal with
-// key bias: 104 -> 76; 4 x 2048 x 16 x 128: 197 -> 158; 4 x 1024 x 16 x 128, p 0.1: 86 -> 62.  With a single row tile there are
+// Measured, flash_fwd_kernel -> this (us): 4 x 2048 x 16 x 128 causal: 137 -> 110; 4 x 1000 x 32 x 80 causal with
+// key bias: 104 -> 70; 4 x 2048 x 16 x 128: 197 -> 156; 4 x 1024 x 16 x 128, p 0.1: 86 -> 62.  With a single row tile there are
 // too few tiles to share out: 2 x 60 x 60 x 8 x 128: 6.5 -> 8.0; 8 x 1 x 1500 keys x 16 x 128: 27 -> 29.
 template <bool kGeneral, typename T>
 __global__ void __launch_bounds__(512, 1)

@@ -30,8 +30,8 @@
 // 3000 cycles, of which exp2 alone needs 512 for each of the two; for D = 128 the products (64 cycles
 // each, 20 or 24 to a half tile: those of 64 columns take as long as those of 128).
 // Measured (all kernels of the backward; whole tiles, one issuing thread -> now): 32 x 512 x 16 heads of
-// 64, p 0.1: 315 -> 261 us; 4 x 2048 x 16 x 128 causal: 400 -> 305; 4 x 1000 x 32 x 80 causal with key bias: 227 ->
-// 183; 8 x 512 x 16 x 64 with T5's bias, key bias and p 0.1: 155 -> 143; 4 x 2048 x 16 x 128: 553 -> 421; 1 x 512 x
+// 64, p 0.1: 315 -> 262 us; 4 x 2048 x 16 x 128 causal: 400 -> 310; 4 x 1000 x 32 x 80 causal with key bias: 227 ->
+// 183; 8 x 512 x 16 x 64 with T5's bias, key bias and p 0.1: 155 -> 142; 4 x 2048 x 16 x 128: 553 -> 421; 1 x 512 x
 // 16 x 64, p 0.1: 26 -> 25.
 //
 // A single pass (5 products per tile instead of 7) has to add up dQ over the key tiles: one fp32

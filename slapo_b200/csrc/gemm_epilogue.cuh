@@ -7,9 +7,15 @@
 // layers logits and gradients by 0.9 % of their norm.)  What the backward wants goes to C2: the product, or with
 // `c2_sum` product + bias, rounded.  Backward: C = acc * act'(Z), with column sums of C (the bias gradient) over each 32 rows
 // to `col_part` [ceil(M / 32)][N], which a second kernel adds up in a fixed order.
-// An element is about 20 instructions and two of the special-function unit; eight warps have them done
-// well within the products of a 256 x 256 tile with K = 1024 (8192 cycles), under which they run.  What
-// that saves is a pass over memory each: 16384 x 4096 in bf16: 59 us in the forward, 89 us in the backward.
+// An element is about 20 instructions and two of the special-function unit, which run under the next
+// tile's products as far as those last.  Measured, L2 flushed (us; plain product / with the epilogue / the pass over
+// memory that it replaces):                            16384 x 4096, K = 1024     4096 x 10240, K = 2560
+//   GeLU                                               105 / 108 / 62             136 / 137 / 42
+//   GeLU, the product kept                             105 / 117 / 62             136 / 142 / 42
+//   GeLU's derivative and column sums                   95 / 148 / 79             138 / 157 / 66
+//   ReLU's                                              95 / 130 / -              138 / 161 / -
+// So the forward is all but hidden, while the derivative's epilogue is what bounds a product with K = 1024:
+// of the pass of 79 us it saves 26, at K = 2560 48 of 66.
 #pragma once
 #include "common.cuh"
 

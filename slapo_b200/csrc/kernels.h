@@ -75,11 +75,11 @@ void launch_kv_append(const void* const past[2], const void* const fresh[2], voi
                       int64_t B, int64_t past_len, int64_t new_len, int64_t H, int64_t head_bytes,
                       const int64_t (&fresh_strides)[2][3], cudaStream_t stream);
 
-// out[h, d] = table[buckets[d], h] (fp32) and dtable[b, h] = sum of grad[h, d] over buckets[d] == b
 // out[i] = bucket of distance i - last_key (rel_bias.cu); inv_exact = 1 / exact buckets, inv_log = 1 / log(max
 // distance / exact buckets)
 void launch_rel_buckets(int64_t* out, int n, int last_key, int buckets, int bidirectional, float inv_exact,
                         float inv_log, cudaStream_t stream);
+// out[h, d] = table[buckets[d], h] (fp32) and dtable[b, h] = sum of grad[h, d] over buckets[d] == b
 void launch_rel_bias_fwd(const void* table, const int64_t* buckets, float* out, int n, int H,
                          int n_buckets, int dtype, cudaStream_t stream);
 void launch_rel_bias_bwd(const float* grad, const int64_t* buckets, void* dtable, int n, int H,

@@ -19,9 +19,9 @@
 namespace slapo {
 
 // 16-byte vectors that a thread has in flight.  Bound by reading the logits (8192 x 50304 bf16: 824 MB, 126 us) and
-// close to it by the exponentials (92 us of the special-function unit): with one vector at a time, its own
-// rescaling and scalar arithmetic 161 us, so 141; loss and log-sum-exp from here instead of eight small kernels
-// and the gradient from the last row on, 460 -> 396 us for the loss and its gradient.
+// close to it by the exponentials (92 us of the special-function unit): with one vector at a time 153 us, so
+// 134; with loss and log-sum-exp from here instead of eight small kernels and the gradient from the last row on, the
+// loss and its gradient took 453 us a pass and take 423.
 //
 // Rows of fewer than two such steps are taken a vector at a time by a kernel a half as large, whose CTAs come and
 // go faster (us, 4096 rows, a vector at a time / four): 128 columns 6.7 / 9.6, 3816: 10.7 / 14.1, 12288: 23.4 /
