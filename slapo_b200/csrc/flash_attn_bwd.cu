@@ -423,7 +423,11 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
           for (int j = 0; j < n; ++j, ++h) {
             ok = false;
             if constexpr (kKeys) {
-              if (!tc::mbar_wait(&p_ready[h & 1], (h >> 1) & 1, abort_flag)) break;
+              // (P comes of S and says nothing about Y2, which is loaded after Y1; Y1 is there, S was
+              // formed from it before dS)
+              if (!tc::mbar_wait(&y2_full[r2.slot], r2.phase, abort_flag) ||
+                  !tc::mbar_wait(&p_ready[h & 1], (h >> 1) & 1, abort_flag))
+                break;
               tc::fence_after_sync();
               accumulate(a2, kColP + (h & 1) * kPGroup, y2_desc + r2.slot * kYStep, j == 0);
               tc::umma_commit(&a2_done[h & 1]);

@@ -58,3 +58,32 @@ def test_table_gradient_of_a_crowded_bucket(d, causal, sk):
 @pytest.mark.parametrize("sq,sk", [(60, 60), (150, 150)])
 def test_turns_over_items(sq, sk, d):
     _check(40, sq, sk, 8, d, torch.bfloat16, "", 0.1)
+
+
+# Every CTA's first item, all loads of the launch at once: products must not run ahead of the tiles that they read.
+@pytest.mark.parametrize("b,sq,sk,h,d,causal", [(36, 256, 15, 16, 128, False), (32, 672, 12, 16, 128, False),
+                                                (39, 642, 288, 8, 128, True), (14, 1039, 186, 16, 96, True),
+                                                (39, 256, 256, 16, 128, False), (60, 256, 40, 16, 64, False)])
+def test_first_items_of_a_launch(b, sq, sk, h, d, causal):
+    torch.manual_seed(sq + sk)
+    q, k, v, g = (torch.randn(b, n, h, d, device="cuda", dtype=torch.bfloat16) for n in (sq, sk, sk, sq))
+    ops = native.ops()
+    out, lse = ops.flash_attn_fwd(q, k, v, None, None, causal, d ** -0.5, 0.0, None)
+    once = ops.flash_attn_bwd(g, q, k, v, out, lse, None, None, causal, d ** -0.5, 0.0, None, False)[:3]
+    for _ in range(6):
+        again = ops.flash_attn_bwd(g, q, k, v, out, lse, None, None, causal, d ** -0.5, 0.0, None, False)
+        assert all(torch.equal(x, y) for x, y in zip(again, once))      # (sums have one order)
+    s = torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) * d ** -0.5
+    if causal:
+        s = s.masked_fill(torch.ones(sq, sk, dtype=torch.bool, device="cuda").triu(sk - sq + 1), float("-inf"))
+    p = torch.softmax(s, -1).nan_to_num(0.0)
+    dv = torch.einsum("bhqk,bqhd->bkhd", p, g.float())
+    ds = p * (torch.einsum("bqhd,bkhd->bhqk", g.float(), v.float())
+              - (g.float() * out.float()).sum(-1).transpose(1, 2)[..., None])
+    dk = torch.einsum("bhqk,bqhd->bkhd", ds, q.float()) * d ** -0.5
+    dq = torch.einsum("bhqk,bkhd->bqhd", ds, k.float()) * d ** -0.5
+    for got, want in zip(once, (dq, dk, dv)):
+        # each head of its own: a single wrong half tile shows
+        err = (got.float() - want).square().sum((1, 3)).sqrt() / want.square().sum((1, 3)).sqrt()
+        assert err.max().item() < 2 * TOL[torch.bfloat16]
+    assert ops.device_status() == 0

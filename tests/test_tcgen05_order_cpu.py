@@ -43,6 +43,43 @@ def unfenced(source):
     return found
 
 
+ROLE = re.compile(r"// -{8,} *(?P<name>[^-\n]+?) *-{8,}")
+RELEASE = re.compile(r"umma_commit\(&(?P<ring>\w+)_empty\[")
+# ring slots that a thread releases without having waited for them, and why they are full
+IMPLIED = {("flash_attn_bwd.cu", "accumulating products", "y1"): "dS follows S, which was formed from the slot"}
+
+
+def unwaited(name, source):
+    """(role, ring) where the thread whose products release a ring's slots never waits for them to be full.  Roles
+    are the stretches between dashed comments; a ring chosen at run time (``y_full``) goes by its first letter."""
+    source = source.replace("\\\n", " ")
+    heads = list(ROLE.finditer(source))
+    found = []
+    for head, after in zip(heads, heads[1:] + [None]):
+        body = source[head.end():after.start() if after else len(source)]
+        for ring in sorted(set(m["ring"] for m in RELEASE.finditer(body))):
+            waits = (f"mbar_wait(&{ring}_full[", f"mbar_wait(&{ring[0]}_full[", f"mbar_wait({ring}_full")
+            if not any(w in body for w in waits) and (name, head["name"], ring) not in IMPLIED:
+                found.append((head["name"], ring))
+    return found
+
+
+def test_the_reader_of_roles_sees_what_it_should():
+    role = "// ---------- one ----------\n%s\n// ---------- two ----------\nmbar_wait(&y2_full[0]);"
+    assert unwaited("x", role % "umma_commit(&y2_empty[s]);") == [("one", "y2")]
+    assert unwaited("x", role % "mbar_wait(&y2_full[s]); umma_commit(&y2_empty[s]);") == []
+    assert unwaited("x", role % "mbar_wait(&y_full[s]); umma_commit(&y2_empty[s]);") == []
+
+
+@pytest.mark.parametrize("name", ["flash_attn.cu", "flash_attn_bwd.cu"])
+def test_a_thread_waits_for_what_its_products_read(name):
+    with open(os.path.join(CSRC, name)) as f:
+        source = f.read()
+    assert len(RELEASE.findall(source)) >= 3
+    missing = unwaited(name, source)
+    assert not missing, f"{name}: slots released without a wait for their loads: {missing}"
+
+
 def test_the_reader_sees_what_it_should():
     assert unfenced("{ mbar_wait(a); tmem_ld_x32(r); }") == [1]
     assert unfenced("{ mbar_wait(a); fence_after_sync(); tmem_ld_x32(r); }") == []
