@@ -2,15 +2,15 @@
 //
 // Bound by reading K and V (8 x 1500 keys x 16 heads of 128: 98 MB, 15 us from HBM, less where a cache
 // grown just before is still in L2).  A 128-row tensor-core tile would be one row of work in 128, and
-// its loads wait for its softmax; here every lane has 16 bytes of four rows of K and V on their way under the arithmetic of
-// the four before.  L lanes share a key
-// row, so that a warp's load is 32 / L whole rows; each such group of lanes keeps a running maximum, sum and
-// output of its own, merged over the lanes and warps at the end.  Probabilities stay in fp32.
-// A CTA of sixteen or four warps takes the keys of one work item: all of a head's, or a share of them that flash_combine_kernel
-// adds up (the rule is flash_fwd_splits).
-// Measured (us), tensor-core tiles -> this: 8 x 1500 keys x 16 heads of 128: 24.4 -> 19.5 after a cache was grown
-// (32 -> 20 alone; without the rows fetched ahead 38); 16 x 2000 x 20 x 64: 90 -> 41; 1 x 300 x 12 x 64: 10.7 -> 4.6; 1 x 2000 x 16 x 128,
-// keys split: 14.5 -> 9.4 with the combine kernel.
+// its loads wait for its softmax; here every lane has 16 bytes of four rows of K and V on their way under
+// the arithmetic of the four before.  L lanes share a key row, so that a warp's load is 32 / L whole rows;
+// each such group of lanes keeps a running maximum, sum and output of its own, merged over the lanes and
+// warps at the end.  Probabilities stay in fp32.
+// A CTA of sixteen or four warps takes the keys of one work item: all of a head's, or a share of them that
+// flash_combine_kernel adds up (the rule is flash_fwd_splits).
+// Measured (us), tensor-core tiles -> this: 8 x 1500 keys x 16 heads of 128: 24.4 -> 19.5 after a cache was
+// grown (32 -> 20 alone; without the rows fetched ahead 38); 16 x 2000 x 20 x 64: 90 -> 41; 1 x 300 x 12 x 64:
+// 10.7 -> 4.6; 1 x 2000 x 16 x 128, keys split: 14.5 -> 9.4 with the combine kernel.
 #include "flash_common.cuh"
 #include "kernels.h"
 
@@ -160,10 +160,10 @@ int launch_flash_decode(const void* q, const void* k, const void* v, void* o, fl
   count_launch();
   // Sixteen warps where a work item has many keys and the items leave SMs idle, four (and four CTAs per SM)
   // where most of sixteen would have nothing to load or the items fill the SMs by themselves.  Measured (us;
-  // 128-row tensor-core tiles / sixteen / four), bf16, items x keys x D: 96 x 16 x 64: 6.8 / 3.4 / 2.9; 96 x 256 x 64: 8.0 / 4.2 /
-  // 4.6; 384 x 128 x 64: 10.5 / 8.8 / 4.6; 640 x 2000 x 64: 96 / 67 / 75; 2048 x 128 x 64: 28 / 48 / 19; 4096 x 512 x
-  // 64: 147 / 144 / 93; 144 x 384 x 128: 11.8 / 8.1 / 13.1; 384 x 256 x 128: 19.8 / 17.5 / 12.9; 2048 x 512 x 128:
-  // 110 / 111 / 89.
+  // 128-row tensor-core tiles / sixteen / four), bf16, items x keys x D: 96 x 16 x 64: 6.8 / 3.4 / 2.9; 96 x 256 x
+  // 64: 8.0 / 4.2 / 4.6; 384 x 128 x 64: 10.5 / 8.8 / 4.6; 640 x 2000 x 64: 96 / 67 / 75; 2048 x 128 x 64: 28 / 48 /
+  // 19; 4096 x 512 x 64: 147 / 144 / 93; 144 x 384 x 128: 11.8 / 8.1 / 13.1; 384 x 256 x 128: 19.8 / 17.5 / 12.9;
+  // 2048 x 512 x 128: 110 / 111 / 89.
   const int step = D <= 64 ? 256 : 128;         // keys that sixteen warps take at a time
   const bool few = 2 * keys_per_split <= step || (2 * ctas >= 3 * sm_count() && keys_per_split <= 2 * step) ||
                    ctas >= 6 * sm_count();

@@ -41,7 +41,8 @@ def test_single_query(sk, b, h, d, dtype, how):
 
 # four warps per work item or sixteen: half a step of keys, two steps with 222 items, any number with 888
 @pytest.mark.parametrize("h,sk,d", [(4, 128, 64), (4, 129, 64), (4, 64, 128), (4, 65, 80), (221, 512, 64),
-                                    (222, 512, 64), (222, 513, 64), (222, 256, 128), (222, 257, 128), (887, 520, 64),
+                                    (222, 512, 64), (222, 513, 64), (222, 256, 128), (222, 257, 128),
+                                     (887, 520, 64),
                                     (888, 520, 64), (888, 300, 128), (888, 7, 128)])
 def test_warps_of_a_work_item(h, sk, d):
     test_single_query(sk, 1, h, d, BF, "k")
@@ -72,7 +73,8 @@ def test_nans_and_infinities_stay(sk, what, value):
         assert not out[:, :, 1].isfinite().all()
 
 
-@pytest.mark.parametrize("k", [2040, 2048, 2056, 4096, 4128, 768, 512])       # steps of K in runs and one by one
+# steps of K in runs and one by one
+@pytest.mark.parametrize("k", [2040, 2048, 2056, 4096, 4128, 768, 512])
 def test_few_rows_contractions(k):
     test_few_rows(16, k, 1032, BF, None)
 

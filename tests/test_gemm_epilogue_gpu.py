@@ -25,8 +25,8 @@ def _close(got, want, tol):
     return ((got.double() - want).norm() / want.norm().clamp(min=1e-30)).item() < tol
 
 
-# rows, inner, columns, and the tile (of a CTA pair, its columns; 0: 256): narrow ones, a ragged one of each other
-# kind, several row blocks and work items, more than one band of row tiles and a ragged last one
+# rows, inner, columns, and the tile (of a CTA pair, its columns; 0: 256): narrow ones, a ragged one of each
+# other kind, several row blocks and work items, more than one band of row tiles and a ragged last one
 ONE64, ONE128, ONE256, PAIR128, PAIR256 = (False, 64), (False, 128), (False, 0), (True, 128), (True, 0)
 SHAPES = [(8, 64, 8, ONE64), (40, 72, 200, ONE64), (128, 64, 4096, ONE64), (120, 64, 19200, ONE256),
           (136, 264, 136, ONE64), (264, 64, 72, ONE64), (200, 3072, 768, ONE64), (1000, 2560, 1096, ONE64),

@@ -15,9 +15,11 @@ pytestmark = pytest.mark.gpu
 BF, FP = torch.bfloat16, torch.float16
 
 
-# few rows, steps of K in runs and one by one; every tile: one CTA of 64 / 128 / 256 columns, pairs of 128 / 256; ragged rows and columns
+# few rows, steps of K in runs and one by one; every tile: one CTA of 64 / 128 / 256 columns, pairs of
+# 128 / 256; ragged rows and columns
 @pytest.mark.parametrize("act,dtype", [("gelu", BF), ("gelu_new", FP)])
-@pytest.mark.parametrize("m,k,n", [(8, 64, 64), (16, 2048, 200), (8, 776, 3072), (40, 72, 200), (200, 768, 3072), (128, 64, 64 * 148 + 8), (120, 64, 19200),
+@pytest.mark.parametrize("m,k,n", [(8, 64, 64), (16, 2048, 200), (8, 776, 3072), (40, 72, 200),
+                                   (200, 768, 3072), (128, 64, 64 * 148 + 8), (120, 64, 19200),
                                    (392, 64, 4104), (2056, 64, 2056)])
 def test_equals_layer_then_activation(m, k, n, act, dtype):
     torch.manual_seed(m + n)
@@ -43,7 +45,8 @@ def test_equals_layer_then_activation(m, k, n, act, dtype):
     y = native.ops().linear(x, wt, b, NF._act_code(act), True)
     z = NF.linear_t(x, wt)
     assert torch.equal(y, NF.bias_act(z, b, act))
-    for p, q in zip(torch.autograd.grad(y, [x, wt, b], dy), torch.autograd.grad(NF.bias_act(z, b, act), [x, wt, b], dy)):
+    two = torch.autograd.grad(NF.bias_act(z, b, act), [x, wt, b], dy)
+    for p, q in zip(torch.autograd.grad(y, [x, wt, b], dy), two):
         assert torch.equal(p, q)
     assert native.ops().device_status() == 0
 

@@ -1,5 +1,5 @@
-"""The feed-forward block's autograd node under what its layers had to bear: saved-tensor hooks, inputs that are
-differentiated alone, and transforms, which are refused with the reason whatever they batch."""
+"""The feed-forward block's autograd node under what its layers had to bear: saved-tensor hooks, inputs that
+are differentiated alone, and transforms, which are refused with the reason whatever they batch."""
 import pytest
 import torch
 import torch.autograd.forward_ad as fwd

@@ -1,5 +1,5 @@
-"""What the GEMM's epilogue operators take and refuse: biases that are missing, start off a 16-byte boundary, lie
-elsewhere or have another length.  (None of these may reach a kernel that would read out of range.)"""
+"""What the GEMM's epilogue operators take and refuse: biases that are missing, start off a 16-byte boundary,
+lie elsewhere or have another length.  (None of these may reach a kernel that would read out of range.)"""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -56,7 +56,8 @@ def test_refusals():
     x, w, b = _inputs(392, 64, 4104)
     for bias in (b[:4104].cpu(), b[:4096], b[:4104].float()):
         for call in (lambda: ops.gemm_act_fwd(x, w, bias, 0, False),
-                     lambda: ops.gemm(x, w, bias, -1, False, False), lambda: ops.linear(x, w, bias, 0, False)):
+                     lambda: ops.gemm(x, w, bias, -1, False, False),
+                     lambda: ops.linear(x, w, bias, 0, False)):
             with pytest.raises(RuntimeError):
                 call()
     with pytest.raises(RuntimeError):
@@ -66,8 +67,8 @@ def test_refusals():
     w2 = torch.zeros(64, 4104, device="cuda", dtype=BF)
     good = (x, w, b[:4104], w2, b[:64])
     ops.mlp(*good, 0, 0.0)
-    for i, t in ((1, w[:, :56]), (2, b[:4096]), (2, b[:4104].cpu()), (3, w2[:, :4096]), (3, w2.cpu()), (4, b[:56]),
-                 (4, b[:64].cpu()), (4, b[:64].float())):
+    for i, t in ((1, w[:, :56]), (2, b[:4096]), (2, b[:4104].cpu()), (3, w2[:, :4096]), (3, w2.cpu()),
+                 (4, b[:56]), (4, b[:64].cpu()), (4, b[:64].float())):
         bad = list(good)
         bad[i] = t
         for p in (0.0, 0.5):

@@ -28,8 +28,8 @@ def test_buckets(buckets, max_distance, bidirectional):
 @pytest.mark.parametrize("bidirectional", [True, False])
 @pytest.mark.parametrize("buckets", list(range(6, 90, 3)) + [160, 200, 256])
 def test_distances_on_borders(buckets, bidirectional):
-    """Largest distances that are a square, cube or other power of a ratio times the exact buckets: distances fall
-    on borders between buckets, where the last bit of the logarithm decides."""
+    """Largest distances that are a square, cube or other power of a ratio times the exact buckets: distances
+    fall on borders between buckets, where the last bit of the logarithm decides."""
     exact = buckets // (4 if bidirectional else 2)
     table = torch.zeros(buckets, 2, device="cuda")
     for far in sorted({exact * r ** e for r in (2, 3, 5, 6, 7, 10) for e in (1, 2, 3, 4)}

@@ -46,12 +46,14 @@ def unfenced(source):
 ROLE = re.compile(r"// -{8,} *(?P<name>[^-\n]+?) *-{8,}")
 RELEASE = re.compile(r"umma_commit\(&(?P<ring>\w+)_empty\[")
 # ring slots that a thread releases without having waited for them, and why they are full
-IMPLIED = {("flash_attn_bwd.cu", "accumulating products", "y1"): "dS follows S, which was formed from the slot"}
+IMPLIED = {("flash_attn_bwd.cu", "accumulating products", "y1"):
+           "dS follows S, which was formed from the slot"}
 
 
 def unwaited(name, source):
-    """(role, ring) where the thread whose products release a ring's slots never waits for them to be full.  Roles
-    are the stretches between dashed comments; a ring chosen at run time (``y_full``) goes by its first letter."""
+    """(role, ring) where the thread whose products release a ring's slots never waits for them to be full.
+    Roles are the stretches between dashed comments; a ring chosen at run time (``y_full``) goes by its
+    first letter."""
     source = source.replace("\\\n", " ")
     heads = list(ROLE.finditer(source))
     found = []
