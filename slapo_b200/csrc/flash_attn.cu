@@ -4,30 +4,27 @@
 // (so q/k/v slices of a fused QKV projection are read in place through 4-D
 // TMA maps - no .contiguous() copies).  D is 64 or 128.
 //
-// Persistent CTAs (D = 64: two per SM with 256 of the 512 TMEM columns each; D = 128: one) walk
-// over work items of 128 query rows of one (batch, head); for each they stream the keys in tiles of 128:
-//   warp 0    TMA: Q, K ring, V ring (runs ahead over tiles and over work items)
-//   warp 1    tcgen05.mma:  S = Q K^T       (fp32, 128 TMEM columns)
-//                           O += P V        (P read from TMEM, fp32 accumulator in TMEM)
-//   warps 2-5 one query row per thread: the row's 128 scores in registers, online softmax in
-//             the exp2 domain, P back to TMEM as bf16 / fp16.
+// Two kernels.  flash_fwd_groups_kernel takes calls with more than one tile of 128 query rows: persistent
+// CTAs, one per SM, with two softmax groups that take the key tiles of a work item in turn.  Persistent CTAs of
+// flash_fwd_kernel (D = 64: two per SM with 256 of the 512 TMEM columns each; D = 128: one) take those with a
+// single row tile, where the keys may be split over work items.  Both walk over work items of 128 query rows
+// of one (batch, head), for each of which they stream the keys in tiles of 128:
+//   a thread     TMA: Q, K ring, V ring (runs ahead over tiles and over work items)
+//   a thread     tcgen05.mma:  S = Q K^T       (fp32, 128 TMEM columns)
+//                              O += P V        (P read from TMEM, fp32 accumulator in TMEM)
+//   four warps   one query row per thread: online softmax in the exp2 domain, P back to TMEM as bf16 / fp16
 // P and O are scaled by the running row maximum: when that of any of a warp's rows has grown, the
-// warp scales its O rows in TMEM.  (Raising it only after a growth of 2^8 saves 2 - 9 % of the
-// forward - 32 x 512 x 16 x 64, p 0.1: 113 against 117 us, 4 x 2048 x 16 x 128: 186 against 205 - but
-// then the probabilities that count lie anywhere in their binade instead of at or just below 1,
+// warp's O rows are scaled in TMEM.  (Raising it only after a growth of 2^8 saves 2 - 9 % of the
+// forward, but then the probabilities that count lie anywhere in their binade instead of at or just below 1,
 // and the result's rounding error grows by up to 5 %: 0.00230 against 0.00220 at 512 keys, bf16.)
-// P has columns of its own: S of the next tile is computed while the softmax warps work on this
-// one.
+// A single query goes to flash_decode.cu.
 //
-// Two other kernels take what this one is not best at: heads wider than 64 with several row tiles
-// (flash_fwd_groups_kernel below) and a single query (flash_decode.cu).
-//
-// What bounds it: the special-function unit (one exp2 per score, 1024 cycles per 128 x 128 tile
-// and SM) next to the issue slots of the softmax warps.  One thread per whole row needs no
-// exchange between warps; for D = 64 two independent CTAs fill each other's waits.
-// Measured (L2 flushed; P through shared memory, O folded in registers, one work item per CTA ->
-// now): 32 x 512 x 16 heads of 64, p 0.1: 126 -> 106 us; 8 x 512 x 16 x 64 with T5's bias, key bias and p
-// 0.1: 66 -> 45 us; 60 queries x 2000 keys x 2 x 8 x 128, keys split: 15 us with the combine kernel.
+// What bounds it: the special-function unit (one exp2 per score, 1024 cycles per 128 x 128 tile and SM) next to
+// the issue slots of the softmax warps, and what a tile's chain has between them: waits of 50 - 250 cycles, reads of
+// tensor memory, issuing (40 cycles a product).  Dropout is a template parameter: skipped at run time its draws are
+// branches over code that has to be fetched, and taken at run time they do not mix with the exponentials
+// (us, run time -> template: 32 x 512 x 16 heads of 64, p 0.1: 105.5 -> 99.3, without 76.9 -> 75.3; 4 x 2048
+// causal: 83.5 -> 77.5).
 //
 // Biases are added from shared memory, which asynchronous copies fill a tile ahead: a warp's 32
 // queries see 159 distances in a tile of 128 keys, against 128 loads per query.  Fetched by each
@@ -135,13 +132,14 @@ __device__ __forceinline__ void fwd_land_bias(const FlashFwdParams& p, float* bi
 }
 
 // A row's scores, scaled to the log2 domain, plus its biases
-__device__ __forceinline__ void fwd_add_bias(const FlashFwdParams& p, uint32_t (&raw)[4][32], const float* bias,
+template <int kSets>
+__device__ __forceinline__ void fwd_add_bias(const FlashFwdParams& p, uint32_t (&raw)[kSets][32], const float* bias,
                                              int lane) {
   const uint64_t scale2 = f2_pack(p.scale_log2, p.scale_log2);
   const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
   if (p.kbias != nullptr) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
+    for (int c = 0; c < kSets; ++c)
 #pragma unroll
       for (int i = 0; i < 32; i += 4) {
         const float4 b = *reinterpret_cast<const float4*>(bias + c * 32 + i);
@@ -150,7 +148,7 @@ __device__ __forceinline__ void fwd_add_bias(const FlashFwdParams& p, uint32_t (
       }
   } else {
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
+    for (int c = 0; c < kSets; ++c)
 #pragma unroll
       for (int i = 0; i < 32; i += 2) f2_store(raw[c] + i, f2_mul(f2_load(raw[c] + i), scale2));
   }
@@ -158,7 +156,7 @@ __device__ __forceinline__ void fwd_add_bias(const FlashFwdParams& p, uint32_t (
     // neighbouring lanes (queries) read neighbouring words
     const float* rel = bias + 128 + 31 - lane;
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
+    for (int c = 0; c < kSets; ++c)
 #pragma unroll
       for (int i = 0; i < 32; i += 2)
         f2_store(raw[c] + i,
@@ -167,14 +165,15 @@ __device__ __forceinline__ void fwd_add_bias(const FlashFwdParams& p, uint32_t (
 }
 
 // -inf for keys that a row does not see, of the tile from k0 on; row0: the warp's first row
-__device__ __forceinline__ void fwd_mask(const FlashFwdParams& p, uint32_t (&raw)[4][32], int k0, int row0,
+template <int kSets>
+__device__ __forceinline__ void fwd_mask(const FlashFwdParams& p, uint32_t (&raw)[kSets][32], int k0, int row0,
                                          int lane) {
   const int diag = p.Sk - p.Sq;         // key j visible to query i iff j <= i + diag (causal)
   const int first_limit = p.causal ? min(p.Sk, row0 + diag + 1) : p.Sk;
-  if (k0 + kBlockN > first_limit) {     // some lane of the warp masks something
+  if (k0 + kSets * 32 > first_limit) {     // some lane of the warp masks something
     const int limit = (p.causal ? min(p.Sk, row0 + lane + diag + 1) : p.Sk) - k0;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < kSets; ++c) {
       const uint32_t seen = low_bits(limit - c * 32);
 #pragma unroll
       for (int i = 0; i < 32; ++i)
@@ -183,14 +182,33 @@ __device__ __forceinline__ void fwd_mask(const FlashFwdParams& p, uint32_t (&raw
   }
 }
 
-__device__ __forceinline__ float fwd_max(const uint32_t (&raw)[4][32]) {
+template <int kSets>
+__device__ __forceinline__ float fwd_max(const uint32_t (&raw)[kSets][32]) {
   float mm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // 4 chains for ILP
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
+  for (int c = 0; c < kSets; ++c)
 #pragma unroll
-    for (int i = 0; i < 32; i += 2)
-      mm[c] = fmaxf(mm[c], fmaxf(__uint_as_float(raw[c][i]), __uint_as_float(raw[c][i + 1])));
+    for (int i = 0; i < 32; i += 2) {
+      float& m = mm[(i >> 1) & 3];
+      m = fmaxf(m, fmaxf(__uint_as_float(raw[c][i]), __uint_as_float(raw[c][i + 1])));
+    }
   return fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3]));
+}
+
+// Columns col .. col + 15 of a row of `cols` 16-bit values (a multiple of 8; padded columns are not part of
+// it).  Neighbouring rows lie whole lines apart, so that a store takes a cycle per row: one of 32 bytes
+// where rows keep to 32 bytes.
+__device__ __forceinline__ void store_cols16(void* row, int col, int cols, const uint32_t (&v)[8]) {
+  uint8_t* dst = static_cast<uint8_t*>(row) + col * 2;
+  if ((cols & 15) == 0) {
+    if (col < cols)
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]),
+                   "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                   : "memory");
+  } else {
+    if (col < cols) *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+    if (col + 8 < cols) *reinterpret_cast<uint4*>(dst + 16) = make_uint4(v[4], v[5], v[6], v[7]);
+  }
 }
 
 template <int D>
@@ -209,7 +227,7 @@ struct FwdSmem {
 // kGeneral: key bias, relative bias, causal mask, a ragged last key tile or a scale <= 0;
 // without any of them the kernel takes row maxima on the raw scores and every probability is
 // one fused multiply-add plus one exp2.
-template <int D, bool kGeneral, typename T>
+template <int D, bool kGeneral, bool kDrop, typename T>
 __global__ void __launch_bounds__(192, D == 64 ? 2 : 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const FlashFwdParams p) {
@@ -393,8 +411,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const int row_in_tile = quarter * 32 + lane;
     const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     float* bias_buf = reinterpret_cast<float*>(smem + L::kBias) + (warp - 2) * 2 * kBiasFloats;
-    uint64_t seed = 0, offset = 0;
-    if (p.p_drop > 0.f) philox_unpack(p.rng, seed, offset);
+    PhiloxUniform rng{};
+    if constexpr (kDrop) rng = philox_uniform(p.rng);
     const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
     const int sk16 = (p.Sk + 15) >> 4;
     // scores are brought to the log2 domain before the maximum only where something is added
@@ -488,12 +506,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             else la = f2_add(la, f2_pack(a, b));
             pk[i] = pack16<T>(a, b);
           }
-          if (p.p_drop > 0.f) {
+          if constexpr (kDrop) {
             // dropped probabilities are cleared in the packed 16-bit pairs
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              const uint4 kw = philox_keep16(seed, offset,
-                                             drop_row_base + ((k0 + c * 32 + h * 16) >> 4), add4);
+              const uint4 kw = philox_keep16(rng, drop_row_base + ((k0 + c * 32 + h * 16) >> 4), add4);
               const uint32_t wd[4] = {kw.x, kw.y, kw.z, kw.w};
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
@@ -580,14 +597,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
 // Registers per thread of the warpgroups: issuing, softmax (two), O; together the 128 per thread that
 // 512 threads are launched with.
-constexpr int kFwdRegsIssue = 56, kFwdRegsSoftmax = 184, kFwdRegsO = 88;
+constexpr int kFwdRegsIssue = 72, kFwdRegsSoftmax = 176, kFwdRegsO = 88;
 static_assert(kFwdRegsIssue + 2 * kFwdRegsSoftmax + kFwdRegsO <= 4 * 128, "more registers than the block has");
 
-// D in 65 .. 128
+template <int D>
 struct GroupsSmem {
-  static constexpr int kTile = 128 * 128 * 2;        // one [128 x 128] 16-bit tile
+  static constexpr int kTile = 128 * D * 2;          // one [128 x D] 16-bit tile
   static constexpr int kQ = 2;                       // Q tiles: this item's and the next one's
-  static constexpr int kStages = 2;                  // K and V rings
+  static constexpr int kStages = D == 64 ? 4 : 2;    // K and V rings
   static constexpr int kK = kQ * kTile;
   static constexpr int kV = kK + kStages * kTile;
   // (per softmax warp, twice: this tile's biases and the next one's)
@@ -598,21 +615,29 @@ struct GroupsSmem {
   static constexpr int kTotal = kBars + 48 * 8 + 1024;
 };
 
-// The forward for D > 64 and more than one row tile: two softmax groups in one CTA that take the key tiles
-// of a work item in turn, each with an online softmax and an accumulator of its own, which a third group
-// of warps scales when maxima grow and merges at the end.  Loads, S and P V have a thread each.  One CTA of
-// flash_fwd_kernel has one softmax warp per scheduler at this width and keeps all of that on the chain of
-// a tile.  Bound now: S of a group waits for its P V (512 columns hold two S and two O, P lies over S),
-// 1900 of the 4700 cycles between two tiles of a group.
-// Measured, flash_fwd_kernel -> this (us): 4 x 2048 x 16 x 128 causal: 137 -> 110; 4 x 1000 x 32 x 80 causal with
-// key bias: 104 -> 70; 4 x 2048 x 16 x 128: 197 -> 156; 4 x 1024 x 16 x 128, p 0.1: 86 -> 62.  With a single row tile there are
-// too few tiles to share out: 2 x 60 x 60 x 8 x 128: 6.5 -> 8.0; 8 x 1 x 1500 keys x 16 x 128: 27 -> 29.
-template <bool kGeneral, typename T>
+// The forward for more than one row tile: two softmax groups in one CTA that take the key tiles of a work
+// item in turn, each with an online softmax and an accumulator of its own, which a third group of warps
+// scales when maxima grow and merges at the end.
+// One thread issues all products: two products' queue is served in the order it is filled in, so that
+// a group's P V and next S do not wait behind each other's halves (a thread per group: 128 -> 153 us for 4 x 2048
+// x 16 x 128).  Between two tiles of a group (some 4000 cycles) lie 2000 - 2500 of exponentials that the groups
+// take together, the products and 300 - 500 each of reading S, its maximum, handing the factors for O over and
+// waiting; D = 128 waits 1300 for P V and S, whose columns P lies in.  (The groups held apart, so that one has
+// the special-function unit to itself: no difference.)
+// The scores stay in tensor memory and come out of it twice, in pieces.  Held in registers from the maximum to
+// the exponentials, 128 a row, they left too few for dropout's draws and biases, which spilled:
+// 32 x 512 x 16 x 64, p 0.1: 87 -> 79 us; 4 x 1000 x 32 x 80 causal with key bias: 66 -> 60.
+// Measured, all of that together (us; one softmax group in each of two CTAs per SM for D = 64, two issuing threads
+// for D = 128 -> this): 32 x 512 x 16 x 64, p 0.1: 105.5 -> 78.7, without 76.9 -> 60.9; 4 x 2048 x 16 x 64 causal:
+// 83.5 -> 74.9; 8 x 512 x 16 x 64 with T5's bias, key bias and p 0.1: 43.7 -> 41.2; 1 x 512 x 16 x 64, p 0.1: 12.9 ->
+// 9.4; 4 x 2048 x 16 x 128 causal: 111 -> 91, all keys 154 -> 128; 4 x 1000 x 32 x 80 causal with key bias: 70 -> 60;
+// 4 x 1024 x 16 x 128, p 0.1: 61 -> 49.  With a single row tile there are too few tiles to share out: 2 x 60 x 60 x
+// 8 x 128: 6.5 -> 8.0.
+template <int D, bool kGeneral, bool kDrop, typename T>
 __global__ void __launch_bounds__(512, 1)
 flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ FlashFwdParams p) {
-  using L = GroupsSmem;
-  constexpr int D = 128;
+  using L = GroupsSmem<D>;
   constexpr int kTileBytes = L::kTile;
   constexpr int kStages = L::kStages, kQ = L::kQ;
   constexpr int kBlkBytes = 128 * 128;      // one [128 rows x 64 cols] swizzled block
@@ -633,7 +658,8 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   uint64_t* o_ready = bars + 28;      // O is scaled (or free) for a tile (4 warps)
   uint64_t* alpha_ready = bars + 30;  // [group][tile parity]: a tile's factors (4 warps)
   uint64_t* ml_ready = bars + 34;     // [group][item parity]: an item's maxima and sums (4 warps)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 38);
+  uint64_t* s_free = bars + 38;       // S of a tile has been read (4 warps; D = 64)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 40);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* s_alpha = reinterpret_cast<float*>(smem + L::kAlpha);
   float2* s_ml = reinterpret_cast<float2*>(smem + L::kMl);
@@ -641,9 +667,11 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int diag = p.Sk - p.Sq;  // key j visible to query i iff j <= i + diag (causal)
   constexpr uint32_t kTmemCols = 512;
-  // S and O of the two groups; P is written over S, whose next product then waits for the one that
-  // uses P up
-  constexpr uint32_t kColS = 0, kColO = 256;
+  // S, O and P of the two groups.  For D = 128 P is written over S: the next S of a group goes into the
+  // tensor core's queue behind the product that uses P up.  For D = 64 P has columns of its own and the next
+  // S is formed as soon as this one has been read.
+  constexpr bool kOver = D == 128;
+  constexpr uint32_t kColS = 0, kColO = 256, kColP = kOver ? kColS : 384, kPGroup = kOver ? 128 : 64;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -652,6 +680,7 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       tc::mbar_init(&s_full[i], 1);
       tc::mbar_init(&pv_done[i], 1);
       tc::mbar_init(&o_ready[i], 4);
+      tc::mbar_init(&s_free[i], 4);
     }
     for (int i = 0; i < kStages; ++i) {
       tc::mbar_init(&k_full[i], 1);
@@ -730,51 +759,53 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
           }
         }
       } else if (warp == 1) {
-        // ------------------------------ S = Q K^T ------------------------------
+        // ------------------------------ products ------------------------------
+        // In the order S(0), S(1), then for every tile u of the CTA's sequence P V(u) and S(u + 2), for D = 64
+        // the other way round: S as soon as the one before it in its columns has been read.
         const uint32_t q_desc = tc::smem_desc_lo(tc::smem_u32(smem), 16);
         const uint32_t k_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kK), 16);
-        Ring<kQ> q;
-        Ring<kStages> r;
-        int u = 0;
-        for (int item = blockIdx.x; item < items && ok; item += gridDim.x, q.step()) {
-          int tile, bh;
-          const int n = item_at(item, tile, bh);
-          if (!tc::mbar_wait(&q_full[q.slot], q.phase, abort_flag)) break;
-          for (int j = 0; j < n; ++j, ++u, r.step()) {
-            const int g = u & 1;
-            ok = false;
-            if (!tc::mbar_wait(&k_full[r.slot], r.phase, abort_flag)) break;
-            if (u >= 2 && !tc::mbar_wait(&pv_done[g], ((u >> 1) & 1) ^ 1, abort_flag)) break;
-            tc::fence_after_sync();
-#pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
-              if (kk < p.k_steps) {
-                const uint32_t off = ((kk >> 2) * kBlkBytes + (kk & 3) * 32) >> 4;
-                tc::umma_f16(tmem_base + kColS + g * 128,
-                             tc::smem_desc_words(q_desc + q.slot * kStep + off, kDescHi),
-                             tc::smem_desc_words(k_desc + r.slot * kStep + off, kDescHi), p.idesc_qk,
-                             kk != 0 ? 1u : 0u);
-              }
-            }
-            tc::umma_commit(&s_full[g]);
-            tc::umma_commit(&k_empty[r.slot]);
-            if (j + 1 == n) tc::umma_commit(&q_empty[q.slot]);
-            ok = true;
-          }
-        }
-      } else if (warp == 2) {
-        // ------------------------------ O += P V ------------------------------
         const uint32_t v_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kV), kBlkBytes);
-        Ring<kStages> r;
+        Ring<kQ> q;
+        Ring<kStages> rk, rv;
+        int s_item = blockIdx.x, s_n = 0, s_j = 0;      // the next S
+        int tile, bh;
+        if (s_item < items) s_n = item_at(s_item, tile, bh);
+        auto form_s = [&](int g) -> bool {
+          if (s_item >= items) return true;
+          if (s_j == 0 && !tc::mbar_wait(&q_full[q.slot], q.phase, abort_flag)) return false;
+          if (!tc::mbar_wait(&k_full[rk.slot], rk.phase, abort_flag)) return false;
+          tc::fence_after_sync();
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk) {
+            if (kk < p.k_steps) {
+              const uint32_t off = ((kk >> 2) * kBlkBytes + (kk & 3) * 32) >> 4;
+              tc::umma_f16(tmem_base + kColS + g * 128, tc::smem_desc_words(q_desc + q.slot * kStep + off, kDescHi),
+                           tc::smem_desc_words(k_desc + rk.slot * kStep + off, kDescHi), p.idesc_qk,
+                           kk != 0 ? 1u : 0u);
+            }
+          }
+          tc::umma_commit(&s_full[g]);
+          tc::umma_commit(&k_empty[rk.slot]);
+          rk.step();
+          if (++s_j == s_n) {
+            tc::umma_commit(&q_empty[q.slot]);
+            q.step();
+            s_j = 0;
+            s_item += gridDim.x;
+            if (s_item < items) s_n = item_at(s_item, tile, bh);
+          }
+          return true;
+        };
+        ok = form_s(0) && form_s(1);
         int u = 0;
         for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-          int tile, bh;
           const int n = item_at(item, tile, bh);
-          for (int j = 0; j < n; ++j, ++u, r.step()) {
+          for (int j = 0; j < n; ++j, ++u, rv.step()) {
             const int g = u & 1;
             const uint32_t ph = (u >> 1) & 1;
             ok = false;
-            if (!tc::mbar_wait(&v_full[r.slot], r.phase, abort_flag) ||
+            if (!kOver && (!tc::mbar_wait(&s_free[g], ph, abort_flag) || !form_s(g))) break;
+            if (!tc::mbar_wait(&v_full[rv.slot], rv.phase, abort_flag) ||
                 !tc::mbar_wait(&o_ready[g], ph, abort_flag))
               break;
             // the first half of the keys' products run under the other half's softmax
@@ -784,13 +815,15 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
               tc::fence_after_sync();
 #pragma unroll
               for (int kk = half * 4; kk < half * 4 + 4; ++kk)
-                tc::umma_f16_ts(tmem_base + kColO + g * D, tmem_base + kColS + g * 128 + kk * 8,
-                                tc::smem_desc_words(v_desc + r.slot * kStep + ((kk * 2048) >> 4), kDescHi),
+                tc::umma_f16_ts(tmem_base + kColO + g * D, tmem_base + kColP + g * kPGroup + kk * 8,
+                                tc::smem_desc_words(v_desc + rv.slot * kStep + ((kk * 2048) >> 4), kDescHi),
                                 p.idesc_pv, (j >= 2 || kk != 0) ? 1u : 0u);
             }
             if (*abort_flag != 0) break;
             tc::umma_commit(&pv_done[g]);
-            tc::umma_commit(&v_empty[r.slot]);
+            tc::umma_commit(&v_empty[rv.slot]);
+            // (products of one thread run in order: S goes over a P that has been used up)
+            if (kOver && !form_s(g)) break;
             ok = true;
           }
         }
@@ -805,34 +838,50 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     bool ok = true;
     int u = 0;
     int parts[2] = {0, 0};        // items that each group has had a part in
+    // D = 64: the item before, its row of O packed, is stored once its columns have been given up
+    constexpr bool kHold = D == 64;
+    uint32_t done[kHold ? D / 16 : 1][8];
+    T* done_at = nullptr;
+    auto flush = [&]() {
+      if (!kHold || done_at == nullptr) return;
+#pragma unroll
+      for (int c = 0; c < D / 16; ++c) store_cols16(done_at, c * 16, p.Dr, done[kHold ? c : 0]);
+    };
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
       int tile, bh;
       const int n = item_at(item, tile, bh);
       const int first = u;
-      for (int j = 0; j < n; ++j, ++u) {
-        const int g = u & 1, k = u >> 1;
-        if (j >= 2) {
-          if (!tc::mbar_wait_warp(&alpha_ready[g * 2 + (k & 1)], (k >> 1) & 1, abort_flag)) { ok = false; break; }
-          const float alpha = s_alpha[(g * 2 + (k & 1)) * 128 + row_in_tile];
-          if (__any_sync(0xffffffffu, alpha != 1.f)) {
-            if (!tc::mbar_wait_warp(&pv_done[g], (k & 1) ^ 1, abort_flag)) { ok = false; break; }
-            tc::fence_after_sync();
-            const uint64_t alpha2 = f2_pack(alpha, alpha);
+      // (O of the item before is in registers)
+      __syncwarp();
+      if (lane == 0) {
+        tc::mbar_arrive(&o_ready[first & 1]);
+        if (n > 1) tc::mbar_arrive(&o_ready[(first & 1) ^ 1]);
+      }
+      flush();
+      u += n;
+      for (int t = first + 2; t < u; ++t) {
+        const int g = t & 1, k = t >> 1;
+        if (!tc::mbar_wait_warp(&alpha_ready[g * 2 + (k & 1)], (k >> 1) & 1, abort_flag)) { ok = false; break; }
+        const float alpha = s_alpha[(g * 2 + (k & 1)) * 128 + row_in_tile];
+        // (also where nothing grows: a warp's arrivals for two tiles of a group must not meet in one phase)
+        if (!tc::mbar_wait_warp(&pv_done[g], (k & 1) ^ 1, abort_flag)) { ok = false; break; }
+        if (__any_sync(0xffffffffu, alpha != 1.f)) {
+          tc::fence_after_sync();
+          const uint64_t alpha2 = f2_pack(alpha, alpha);
 #pragma unroll 1
-            for (int c = 0; c < D / 32; ++c) {
-              uint32_t o[32];
-              tc::tmem_ld_x32(tmem_row + kColO + g * D + c * 32, o);
-              tc::tmem_ld_wait();
+          for (int c = 0; c < D; c += 32) {
+            uint32_t o[32];
+            tc::tmem_ld_x32(tmem_row + kColO + g * D + c, o);
+            tc::tmem_ld_wait();
 #pragma unroll
-              for (int i = 0; i < 32; i += 2) f2_store(o + i, f2_mul(f2_load(o + i), alpha2));
-              tc::tmem_st_x32(tmem_row + kColO + g * D + c * 32, o);
-            }
-            tc::tmem_st_wait();
-            tc::fence_before_sync();
+            for (int i = 0; i < 32; i += 2) f2_store(o + i, f2_mul(f2_load(o + i), alpha2));
+            tc::tmem_st_x32(tmem_row + kColO + g * D + c, o);
           }
+          tc::tmem_st_wait();
+          tc::fence_before_sync();
         }
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&o_ready[g]);
+        tc::mbar_arrive_if(&o_ready[g], lane == 0);
       }
       if (!ok) break;
       // both groups' maxima and sums, and their last products
@@ -863,38 +912,37 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       float fa = f[a], fb = f[a ^ 1];
       const int row = tile * kBlockM + row_in_tile;
       const int batch = bh / p.H, head = bh - batch * p.H;
-      // O of the item, columns c .. c + 15
-      auto columns = [&](int c, float (&v)[16]) {
-        uint32_t x[16], y[16];
-        tc::tmem_ld_x16(tmem_row + kColO + a * D + c, x);
-        if (two) tc::tmem_ld_x16(tmem_row + kColO + (a ^ 1) * D + c, y);
-        tc::tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          v[i] = __uint_as_float(x[i]) * fa;
-          if (two) v[i] = fmaf(__uint_as_float(y[i]), fb, v[i]);
-        }
-      };
       const float inv = l > 0.f ? 1.f / (l * (1.f - p.p_drop)) : 0.f;
       fa *= inv;
       fb *= inv;
-      T* dst = static_cast<T*>(p.O) +
-               ((static_cast<int64_t>(batch) * p.Sq + min(row, p.Sq - 1)) * p.H + head) * p.Dr;
-#pragma unroll 1
-      for (int c = 0; c < D; c += 16) {
-        float v[16];
-        columns(c, v);
-        if (row < p.Sq) {
-#pragma unroll
-          for (int i = 0; i < 16; i += 8)      // padded columns are not part of the output
-            if (c + i < p.Dr) Vec8<T>::store(dst + c + i, v + i);
-        }
-      }
-      if (row < p.Sq)
+      done_at = nullptr;
+      if (row < p.Sq) {
+        done_at = static_cast<T*>(p.O) + ((static_cast<int64_t>(batch) * p.Sq + row) * p.H + head) * p.Dr;
         p.lse[static_cast<int64_t>(bh) * p.Sq + row] =
             l > 0.f ? (m == -INFINITY ? 0.f : m) * 0.6931471805599453f + logf(l) : -INFINITY;
+      }
+#pragma unroll
+      for (int c = 0; c < D / 16; ++c) {
+        uint32_t x[16], y[16];
+        tc::tmem_ld_x16(tmem_row + kColO + a * D + c * 16, x);
+        if (two) tc::tmem_ld_x16(tmem_row + kColO + (a ^ 1) * D + c * 16, y);
+        tc::tmem_ld_wait();
+        uint32_t(&w)[8] = done[kHold ? c : 0];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          float v[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            v[e] = __uint_as_float(x[2 * i + e]) * fa;
+            if (two) v[e] = fmaf(__uint_as_float(y[2 * i + e]), fb, v[e]);
+          }
+          w[i] = pack16<T>(v[0], v[1]);
+        }
+        if (!kHold && row < p.Sq) store_cols16(done_at, c * 16, p.Dr, w);
+      }
       tc::fence_before_sync();
     }
+    if (ok) flush();
   } else {
     tc::regs_inc<kFwdRegsSoftmax>();
     // ------------------------------ softmax groups ------------------------------
@@ -904,13 +952,14 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     float* bias_buf = reinterpret_cast<float*>(smem + L::kBias) + (warp - 4) * 2 * kBiasFloats;
     PhiloxUniform rng{};
-    if (p.p_drop > 0.f) rng = philox_uniform(p.rng);
+    if constexpr (kDrop) rng = philox_uniform(p.rng);
     const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
     const int sk16 = (p.Sk + 15) >> 4;
     // scores are brought to the log2 domain before the maximum only where something is added
     // to them (or the scale would turn the maximum around)
     const bool biased = kGeneral && (p.kbias != nullptr || p.rel != nullptr || !(p.scale_log2 > 0.f));
     const float sc = biased ? 1.f : p.scale_log2;
+    const uint64_t sc2 = f2_pack(sc, sc);
     auto fetch_bias = [&](int tile, int bh, int jt, int buf) {
       fwd_fetch_bias(p, bias_buf + buf * kBiasFloats, tile, quarter, lane, bh, jt);
     };
@@ -957,39 +1006,56 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         }
         if (!tc::mbar_wait_warp(&s_full[g], ph, abort_flag)) { ok = false; break; }
         tc::fence_after_sync();
-        uint32_t raw[4][32];
+        // The tile's scores stay in tensor memory and come out of it twice, 64 for the maximum and 32 for the
+        // exponentials at a time.
+        const uint32_t tmem_s = tmem_row + kColS + g * 128;
+        float m_tile = -INFINITY;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tc::tmem_ld_x32(tmem_row + kColS + g * 128 + c * 32, raw[c]);
-        tc::tmem_ld_wait();
-        if constexpr (kGeneral) {
-          if (biased) fwd_add_bias(p, raw, bias, lane);
-          fwd_mask(p, raw, k0, pos.tile * kBlockM + quarter * 32, lane);
+        for (int c = 0; c < 128; c += 64) {
+          uint32_t raw[2][32];
+#pragma unroll
+          for (int b = 0; b < 2; ++b) tc::tmem_ld_x32(tmem_s + c + b * 32, raw[b]);
+          tc::tmem_ld_wait();
+          if constexpr (kGeneral) {
+            if (biased) fwd_add_bias(p, raw, bias + c, lane);
+            fwd_mask(p, raw, k0 + c, pos.tile * kBlockM + quarter * 32, lane);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) tc::tmem_st_x32(tmem_s + c + b * 32, raw[b]);
+          }
+          m_tile = fmaxf(m_tile, fwd_max(raw));
         }
-        const float m_new = fmaxf(m_ref, fwd_max(raw) * sc);
+        uint32_t raw[2][32];
+        if (kGeneral) tc::tmem_st_wait();
+        tc::tmem_ld_x32(tmem_s, raw[0]);
+        const float m_new = fmaxf(m_ref, m_tile * sc);
+        const float m_use = m_new == -INFINITY ? 0.f : m_new;
+        const uint64_t nm2 = f2_pack(-m_use, -m_use);
         const float alpha = m_new == m_ref ? 1.f : exp2f(m_ref - m_new);
+        m_ref = m_new;
         s_alpha[(g * 2 + ph) * 128 + row_in_tile] = alpha;
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&alpha_ready[g * 2 + ph]);
-        l2 = f2_mul(l2, f2_pack(alpha, alpha));
-        m_ref = m_new;
-        const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
-        const uint64_t sc2 = f2_pack(sc, sc), nm2 = f2_pack(-m_use, -m_use);
-        uint64_t la = l2, lb = 0;
+        tc::mbar_arrive_if(&alpha_ready[g * 2 + ph], lane == 0);
+        uint64_t la = f2_mul(l2, f2_pack(alpha, alpha)), lb = 0;
+        // P of the tile before has been used up
+        if (!kOver && k > 0 && !tc::mbar_wait_warp(&pv_done[g], ph ^ 1, abort_flag)) { ok = false; break; }
+        if (!kOver) tc::fence_after_sync();
+        tc::tmem_ld_wait();
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
+          uint32_t(&r)[32] = raw[c & 1];
+          if (c < 3) tc::tmem_ld_x32(tmem_s + (c + 1) * 32, raw[(c + 1) & 1]);
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const uint64_t x = f2_fma(f2_load(raw[c] + 2 * i), sc2, nm2);
             float a, b;
-            f2_unpack(x, a, b);
+            f2_unpack(f2_fma(f2_load(r + 2 * i), sc2, nm2), a, b);
             a = exp2f(a);
             b = exp2f(b);
             if (i & 1) lb = f2_add(lb, f2_pack(a, b));
             else la = f2_add(la, f2_pack(a, b));
             pk[i] = pack16<T>(a, b);
           }
-          if (p.p_drop > 0.f) {
+          if constexpr (kDrop) {
             // dropped probabilities are cleared in the packed 16-bit pairs
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -1002,12 +1068,18 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
               }
             }
           }
-          tc::tmem_st_x16(tmem_row + kColS + g * 128 + c * 16, pk);
+          if (c < 3) tc::tmem_ld_wait();
+          tc::tmem_st_x16(tmem_row + kColP + g * kPGroup + c * 16, pk);
+          if (!kOver && c == 2) {      // (the last scores are in registers)
+            tc::fence_before_sync();
+            __syncwarp();
+            tc::mbar_arrive_if(&s_free[g], lane == 0);
+          }
           if (c & 1) {
             tc::tmem_st_wait();
             tc::fence_before_sync();
             __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&p_full[g * 2 + (c >> 1)]);
+            tc::mbar_arrive_if(&p_full[g * 2 + (c >> 1)], lane == 0);
           }
         }
         l2 = f2_add(la, lb);
@@ -1017,7 +1089,7 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       f2_unpack(l2, l_run, l_hi);
       s_ml[(g * 2 + (part & 1)) * 128 + row_in_tile] = make_float2(m_ref, l_run + l_hi);
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&ml_ready[g * 2 + (part & 1)]);
+      tc::mbar_arrive_if(&ml_ready[g * 2 + (part & 1)], lane == 0);
       ++part;
       pos = next;
     }
@@ -1094,12 +1166,12 @@ void launch_flash_dropout_mask(uint8_t* mask, int B, int H, int Sq, int Sk, floa
   flash_dropout_mask_kernel<<<sm_count() * 4, 256, 0, stream>>>(mask, B, H, Sq, Sk, p_drop, rng);
 }
 
-template <bool kGeneral, typename T>
+template <int D, bool kGeneral, bool kDrop, typename T>
 static int launch_fwd_groups(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                              const FlashFwdParams& p, int64_t items, cudaStream_t stream) {
-  constexpr int kSmem = GroupsSmem::kTotal;
+  constexpr int kSmem = GroupsSmem<D>::kTotal;
   static_assert(kSmem <= 227 * 1024, "flash forward: shared memory over the per-CTA limit");
-  auto kernel = flash_fwd_groups_kernel<kGeneral, T>;
+  auto kernel = flash_fwd_groups_kernel<D, kGeneral, kDrop, T>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
@@ -1112,12 +1184,12 @@ static int launch_fwd_groups(const CUtensorMap& tq, const CUtensorMap& tk, const
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
-template <int D, bool kGeneral, typename T>
+template <int D, bool kGeneral, bool kDrop, typename T>
 static int launch_fwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                         const FlashFwdParams& p, cudaStream_t stream) {
   constexpr int kSmem = FwdSmem<D>::kTotal;
   static_assert(FwdSmem<D>::kCtas * (kSmem + 1024) <= 228 * 1024, "flash forward: shared memory");
-  auto kernel = flash_fwd_kernel<D, kGeneral, T>;
+  auto kernel = flash_fwd_kernel<D, kGeneral, kDrop, T>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) !=
@@ -1126,7 +1198,7 @@ static int launch_fwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
     configured = true;
   }
   const int64_t items = static_cast<int64_t>(p.walk.row_tiles) * p.walk.nbh * p.splits;
-  if (D == 128 && p.walk.row_tiles > 1) return launch_fwd_groups<kGeneral, T>(tq, tk, tv, p, items, stream);
+  if (p.walk.row_tiles > 1) return launch_fwd_groups<D, kGeneral, kDrop, T>(tq, tk, tv, p, items, stream);
   const int64_t cap = FwdSmem<D>::kCtas * sm_count();
   count_launch();
   kernel<<<static_cast<int>(items < cap ? items : cap), 192, kSmem, stream>>>(tq, tk, tv, p);
@@ -1169,9 +1241,7 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float
   FlashFwdParams p;
   p.B = B; p.H = H; p.Sq = Sq; p.Sk = Sk; p.Dr = D; p.O = o; p.lse = lse; p.kbias = kbias; p.rel = rel;
   p.k_steps = (D + 15) / 16;
-  p.walk.row_tiles = (Sq + kBlockM - 1) / kBlockM;
-  p.walk.bh0 = 0; p.walk.nbh = B * H;
-  p.walk.by_cost = causal ? 2 : 0;
+  p.walk.set((Sq + kBlockM - 1) / kBlockM, 0, B * H, causal ? 2 : 0);
   p.splits = scratch != nullptr ? flash_fwd_splits(B, H, Sq, Sk, D) : 1;
   const int key_tiles = (Sk + kBlockN - 1) / kBlockN;
   p.tiles_per_split = (key_tiles + p.splits - 1) / p.splits;
@@ -1199,8 +1269,10 @@ int launch_flash_fwd(const void* q, const void* k, const void* v, void* o, float
         !make_tmap_bshd(&tv, v, B, Sk, H, D, v_strides[0], v_strides[1], v_strides[2], 128, bf16))
       return 2;
 #define FLASH_FWD_CASE(D_, T_)                                            \
-  rc = general ? launch_fwd_d<D_, true, T_>(tq, tk, tv, p, stream)        \
-               : launch_fwd_d<D_, false, T_>(tq, tk, tv, p, stream)
+  rc = p.thr7 != 0 ? (general ? launch_fwd_d<D_, true, true, T_>(tq, tk, tv, p, stream)          \
+                              : launch_fwd_d<D_, false, true, T_>(tq, tk, tv, p, stream))        \
+                   : (general ? launch_fwd_d<D_, true, false, T_>(tq, tk, tv, p, stream)         \
+                              : launch_fwd_d<D_, false, false, T_>(tq, tk, tv, p, stream))
     if (D <= 64) {
       if (bf16) FLASH_FWD_CASE(64, __nv_bfloat16);
       else FLASH_FWD_CASE(64, __half);

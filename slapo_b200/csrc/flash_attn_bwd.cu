@@ -1099,21 +1099,18 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o,
   const bool general = kbias != nullptr || rel != nullptr || causal || Sk % 128 != 0;
   const int bh = B * H;
   FlashBwdParams pq = p, pk = p;
-  pq.walk.row_tiles = p.Rq / 128;
-  pq.walk.by_cost = causal ? 2 : 0;
   pq.splits = plan.splits;
   pq.tiles_per_split = (p.Rk / 128 + plan.splits - 1) / plan.splits;
   pq.out1 = dq; pq.row_stride1 = dq_row_stride;
   pq.out2 = nullptr; pq.row_stride2 = 0;
-  pk.walk.row_tiles = p.Rk / 128;
-  pk.walk.by_cost = causal ? 1 : 0;
   pk.splits = 1;
   pk.tiles_per_split = p.Rq / 128;
   pk.out1 = dk; pk.row_stride1 = dkv_row_stride;
   pk.out2 = dv; pk.row_stride2 = dkv_row_stride;
   for (int at = 0; at < bh; at += plan.pairs) {
-    pq.walk.bh0 = pk.walk.bh0 = at;
-    pq.walk.nbh = pk.walk.nbh = bh - at < plan.pairs ? bh - at : plan.pairs;
+    const int pairs = bh - at < plan.pairs ? bh - at : plan.pairs;
+    pq.walk.set(p.Rq / 128, at, pairs, causal ? 2 : 0);
+    pk.walk.set(p.Rk / 128, at, pairs, causal ? 1 : 0);
     const int rc =
         bf16 ? launch_typed<__nv_bfloat16>(tq, tk, tv, tdo, pq, pk, plan.q_ctas, general, stream)
              : launch_typed<__half>(tq, tk, tv, tdo, pq, pk, plan.q_ctas, general, stream);

@@ -147,6 +147,24 @@ struct Ring {
   }
 };
 
+// Division of 0 .. 2^31 - 1 by a number that is fixed for a launch: a product and a shift, for d <= 2^s with
+// mul = ceil(2^(31 + s) / d) = (2^(31 + s) + e) / d, e < d: n mul / 2^(31 + s) exceeds n / d by n e / (d 2^(31 + s)) < 1 / d.
+// (A division by a run-time number is some 40 dependent instructions.)
+struct FastDiv {
+  uint32_t mul = 0, shift = 0;
+  __host__ void set(int d) {
+    shift = 0;
+    while ((1 << shift) < d && shift < 30) ++shift;
+    if ((1 << shift) < d) ++shift;
+    const uint64_t top = uint64_t(1) << (31 + shift);
+    mul = static_cast<uint32_t>((top + d - 1) / d);
+    shift += 31;
+  }
+  __device__ __forceinline__ int operator()(int n) const {
+    return static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(n)) * mul) >> shift);
+  }
+};
+
 // Row tiles of 128 of all (batch, head) pairs, walked by a persistent grid.  Under a causal
 // mask the tiles differ in cost: they are ordered by cost, heaviest first, over all heads.
 // Otherwise the tiles of one head are neighbours, so that the tensors they share stay in L2.
@@ -154,13 +172,21 @@ struct TileWalk {
   int row_tiles;     // per (batch, head)
   int bh0, nbh;      // range of (batch, head) pairs of this launch
   int by_cost;       // 0 = head-major, 1 = first tile heaviest, 2 = last tile heaviest
+  FastDiv div;       // by row_tiles, or by nbh when ordered by cost
+  __host__ void set(int tiles, int first_bh, int bhs, int cost) {
+    row_tiles = tiles;
+    bh0 = first_bh;
+    nbh = bhs;
+    by_cost = cost;
+    div.set(cost == 0 ? tiles : bhs);
+  }
   __device__ __forceinline__ int items() const { return row_tiles * nbh; }
   __device__ __forceinline__ void at(int item, int& tile, int& bh_local) const {
     if (by_cost == 0) {
-      bh_local = item / row_tiles;
+      bh_local = div(item);
       tile = item - bh_local * row_tiles;
     } else {
-      tile = item / nbh;
+      tile = div(item);
       bh_local = item - tile * nbh;
       if (by_cost == 2) tile = row_tiles - 1 - tile;
     }
