@@ -195,22 +195,6 @@ __device__ __forceinline__ float fwd_max(const uint32_t (&raw)[kSets][32]) {
   return fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3]));
 }
 
-// Columns col .. col + 15 of a row of `cols` 16-bit values (a multiple of 8; padded columns are not part of
-// it).  Neighbouring rows lie whole lines apart, so that a store takes a cycle per row: one of 32 bytes
-// where rows keep to 32 bytes.
-__device__ __forceinline__ void store_cols16(void* row, int col, int cols, const uint32_t (&v)[8]) {
-  uint8_t* dst = static_cast<uint8_t*>(row) + col * 2;
-  if ((cols & 15) == 0) {
-    if (col < cols)
-      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]),
-                   "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-                   : "memory");
-  } else {
-    if (col < cols) *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
-    if (col + 8 < cols) *reinterpret_cast<uint4*>(dst + 16) = make_uint4(v[4], v[5], v[6], v[7]);
-  }
-}
-
 template <int D>
 struct FwdSmem {
   static constexpr int kTile = 128 * D * 2;          // one [128 x D] 16-bit tile

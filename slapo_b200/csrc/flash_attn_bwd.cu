@@ -38,6 +38,12 @@
 // partial of dQ per key tile written and read again was most of its time (BERT-large, 32 x 512
 // tokens x 16 heads of 64: 268 MB each way).
 //
+// Later, on top of that (us): dropout as a template parameter (its draws were branches over code that has to be
+// fetched): dQ 117 -> 112, dK / dV 130 -> 123 for 32 x 512 x 16 x 64, p 0.1, dQ 82 -> 72 without; two sets of dK / dV
+// accumulators at D = 64 and dV's read out a step before dK's, rows stored 32 bytes at a time (a store takes a
+// cycle per row, and reads of shared memory queue behind it): dK / dV 123 -> 113 and, without dropout, 118 -> 101;
+// 4 x 2048 x 16 x 128 causal 161 -> 140; 16 x 200 x 16 x 128, both passes: 85 -> 64.
+//
 // With dropout the dQ pass draws the keep decisions (16 keys of a query row per Philox call, as
 // in the forward) and leaves them as one bit each, [B H][key / 32][query] words, for the dK / dV
 // pass, whose lanes are keys; side by side with the other, that pass draws them for itself.
@@ -126,7 +132,7 @@ __global__ void __launch_bounds__(256) flash_bwd_stats_kernel(
 
 // Registers per thread of the warpgroups: issuing, softmax (two), reading out; together the 128 per
 // thread that 512 threads are launched with.
-constexpr int kRegsIssue = 80, kRegsSoftmax = 168, kRegsOut = 96;
+constexpr int kRegsIssue = 80, kRegsSoftmax = 176, kRegsOut = 80;
 static_assert(kRegsIssue + 2 * kRegsSoftmax + kRegsOut <= 4 * 128, "more registers than the block has");
 
 template <int D, bool kKeys>
@@ -148,16 +154,16 @@ struct BwdSmem {
   static constexpr int kRelFloats = 96;
   static constexpr int kRel = kDrel + (kKeys ? 8 * 32 * 4 : 0);
   static constexpr int kBars = kRel + 8 * 2 * kRelFloats * 4;
-  static constexpr int kTotal = kBars + 48 * 8 + 1024;
+  static constexpr int kTotal = kBars + 52 * 8 + 1024;
 };
 
 // 16 warps in four warpgroups: one thread each of warps 0 - 3 for the loads and the products; two
 // softmax groups (warps 4 - 7 and 8 - 11), one row per thread, which take the half tiles in turn; and
 // the warps that read the accumulators out (12 - 15).
 // kKeys: the dK / dV pass.  kGeneral: key bias, relative bias, causal mask or ragged lengths.
-// kDraw: with dropout the dK / dV pass draws the keep decisions itself, and the dQ pass leaves none.
+// kDrop: with dropout.  kDraw: the dK / dV pass then draws the keep decisions itself, and the dQ pass leaves none.
 // CTA `cta` of `ctas` that run the pass.
-template <int D, bool kKeys, bool kGeneral, bool kDraw, typename T>
+template <int D, bool kKeys, bool kGeneral, bool kDrop, bool kDraw, typename T>
 __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtensorMap& tm_x2,
                                          const CUtensorMap& tm_y1, const CUtensorMap& tm_y2,
                                          const FlashBwdParams& p, const int cta, const int ctas) {
@@ -185,26 +191,25 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
   uint64_t* ds_ready = bars + 34;     // 4 warps: dS written
   uint64_t* a1_done = bars + 36;      // the tensor core has read dS / P of a half tile
   uint64_t* a2_done = bars + 38;
-  uint64_t* acc_full = bars + 40;     // kAcc (<= 2)
-  uint64_t* acc_free = bars + 42;     // 4 warps
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 44);
+  uint64_t* acc1_full = bars + 40;    // kAcc (<= 2) each
+  uint64_t* acc1_free = bars + 42;    // 4 warps
+  uint64_t* acc2_full = bars + 44;
+  uint64_t* acc2_free = bars + 46;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 48);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int diag = p.Sk - p.Sq;
   constexpr uint32_t kTmemCols = 512;
-  // S and dP of the two groups' half tiles, 64 columns each.  dS is written over dP, whose next product
-  // waits for the one that uses dS up.  P has columns of its own where they suffice (a group needs
-  // its next S right after this dS: 122 -> 119 us for dK / dV of 32 x 512 x 16 heads of 64), for D = 128 it is
-  // written over S likewise.  Accumulators: two sets where they fit, so that an item's are read out
-  // under the next one's products.
-  constexpr bool kOver = kKeys && D == 128;
-  constexpr uint32_t kColS = 0, kColDP = 128, kColA1 = 256, kColA2 = 256 + D;
-  constexpr uint32_t kColP = kOver ? kColS : 384, kPGroup = kOver ? 64 : 32;
-  constexpr uint32_t kAccCols = D;        // from one set to the next
-  constexpr int kAcc = kKeys ? 1 : 2;
+  // S and dP of the two groups' half tiles, 64 columns each.  P is written over S, dS over dP, whose next
+  // products wait for the ones that use them up.  Accumulators: two sets where they fit, so that an item's are
+  // read out under the next one's products.  (dK / dV at D = 64 had one set and P in columns of its own, so that the next
+  // S did not wait: a third of an item of eight half tiles went by between two items.)
+  constexpr uint32_t kColS = 0, kColDP = 128, kColA1 = 256, kColA2 = 256 + D, kColP = kColS;
+  constexpr uint32_t kAccCols = kKeys ? 2 * D : D;        // from one set to the next
+  constexpr int kAcc = kKeys && D == 128 ? 1 : 2;
   const int items = p.walk.items() * (kKeys ? 1 : p.splits);
-  const bool drop = p.thr7 != 0;
+  constexpr bool drop = kDrop;
 
   // row tile and (batch, head) of a work item, its first streamed half tile and how many (at least
   // one: a row tile or a split that nothing reaches still has its zeros written)
@@ -251,8 +256,10 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
       tc::mbar_init(&y2_empty[i], kKeys ? 2 : 1);      // dP and, of two threads, dV's product
     }
     for (int i = 0; i < kAcc; ++i) {
-      tc::mbar_init(&acc_full[i], 1);
-      tc::mbar_init(&acc_free[i], 4);
+      tc::mbar_init(&acc1_full[i], 1);
+      tc::mbar_init(&acc1_free[i], 4);
+      tc::mbar_init(&acc2_full[i], 1);
+      tc::mbar_init(&acc2_free[i], 4);
     }
     *abort_flag = 0;
     tc::fence_barrier_init();
@@ -372,7 +379,7 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
         uint64_t* y_full = is_s ? y1_full : y2_full;
         uint64_t* out_full = is_s ? s_full : dp_full;
         // what stood there has been read (P, dS: used up)
-        uint64_t* out_free = is_s ? (kOver ? a2_done : p_ready) : a1_done;
+        uint64_t* out_free = is_s ? (kKeys ? a2_done : p_ready) : a1_done;
         const int slots = is_s ? kY1 : kY2;
         Ring<kX> x;
         int slot = 0, h = 0;
@@ -408,10 +415,10 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
         for (int item = cta; item < items && ok; item += ctas, acc.step()) {
           int tile, bhl, first;
           const int n = item_at(item, tile, bhl, first);
-          // what these accumulators held has been read out
-          if (!tc::mbar_wait(&acc_free[acc.slot], acc.phase ^ 1, abort_flag)) break;
           const uint32_t a1 = kColA1 + acc.slot * kAccCols, a2 = kColA2 + acc.slot * kAccCols;
           auto add_a1 = [&](int i, bool fresh) -> bool {     // half tile i of the sequence
+            // (what these accumulators held has been read out)
+            if (fresh && !tc::mbar_wait(&acc1_free[acc.slot], acc.phase ^ 1, abort_flag)) return false;
             if (!tc::mbar_wait(&ds_ready[i & 1], (i >> 1) & 1, abort_flag)) return false;
             tc::fence_after_sync();
             accumulate(a1, kColDP + (i & 1) * 64, y1_desc + r1.slot * kYStep, fresh);
@@ -425,13 +432,15 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
             if constexpr (kKeys) {
               // (P comes of S and says nothing about Y2, which is loaded after Y1; Y1 is there, S was
               // formed from it before dS)
+              if (j == 0 && !tc::mbar_wait(&acc2_free[acc.slot], acc.phase ^ 1, abort_flag)) break;
               if (!tc::mbar_wait(&y2_full[r2.slot], r2.phase, abort_flag) ||
                   !tc::mbar_wait(&p_ready[h & 1], (h >> 1) & 1, abort_flag))
                 break;
               tc::fence_after_sync();
-              accumulate(a2, kColP + (h & 1) * kPGroup, y2_desc + r2.slot * kYStep, j == 0);
+              accumulate(a2, kColP + (h & 1) * 64, y2_desc + r2.slot * kYStep, j == 0);
               tc::umma_commit(&a2_done[h & 1]);
               tc::umma_commit(&y2_empty[r2.slot]);
+              if (j + 1 == n) tc::umma_commit(&acc2_full[acc.slot]);
               r2.step();
               if (j > 0 && !add_a1(h - 1, j == 1)) break;
               if (j + 1 == n && !add_a1(h, j == 0)) break;
@@ -440,7 +449,7 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
             }
             ok = true;
           }
-          if (ok) tc::umma_commit(&acc_full[acc.slot]);
+          if (ok) tc::umma_commit(&acc1_full[acc.slot]);
         }
       }
     }
@@ -468,15 +477,12 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
                   make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
         } else {
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            if (c + g * 8 < p.Dr) {
-              uint32_t v[4];
+          for (int g = 0; g < 32; g += 16) {
+            uint32_t v[8];
 #pragma unroll
-              for (int i = 0; i < 4; ++i)
-                v[i] = pack16<T>(__uint_as_float(r[g * 8 + 2 * i]) * f,
-                                 __uint_as_float(r[g * 8 + 2 * i + 1]) * f);
-              *reinterpret_cast<uint4*>(dst + c + g * 8) = make_uint4(v[0], v[1], v[2], v[3]);
-            }
+            for (int i = 0; i < 8; ++i)
+              v[i] = pack16<T>(__uint_as_float(r[g + 2 * i]) * f, __uint_as_float(r[g + 2 * i + 1]) * f);
+            store_cols16(dst, c + g, p.Dr, v);
           }
         }
       }
@@ -493,14 +499,22 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
       float* share = nullptr;
       if (!kKeys && p.splits > 1)
         share = p.part + (static_cast<int64_t>(item % p.splits) * p.part_rows + at) * p.Dr;
-      if (!tc::mbar_wait_warp(&acc_full[acc.slot], acc.phase, abort_flag)) break;
+      if constexpr (kKeys) {      // (dV's last product is a step before dK's)
+        if (!tc::mbar_wait_warp(&acc2_full[acc.slot], acc.phase, abort_flag)) break;
+        tc::fence_after_sync();
+        read_out(kColA2 + acc.slot * kAccCols, p.inv_keep, static_cast<T*>(p.out2) + at * p.row_stride2, nullptr,
+                 row < rows);
+        tc::fence_before_sync();
+        __syncwarp();
+        tc::mbar_arrive_if(&acc2_free[acc.slot], lane == 0);
+      }
+      if (!tc::mbar_wait_warp(&acc1_full[acc.slot], acc.phase, abort_flag)) break;
       tc::fence_after_sync();
-      if constexpr (kKeys)
-        read_out(kColA2 + acc.slot * kAccCols, p.inv_keep, static_cast<T*>(p.out2) + at * p.row_stride2, nullptr, row < rows);
-      read_out(kColA1 + acc.slot * kAccCols, out_scale, static_cast<T*>(p.out1) + at * p.row_stride1, share, row < rows);
+      read_out(kColA1 + acc.slot * kAccCols, out_scale, static_cast<T*>(p.out1) + at * p.row_stride1, share,
+               row < rows);
       tc::fence_before_sync();
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&acc_free[acc.slot]);
+      tc::mbar_arrive_if(&acc1_free[acc.slot], lane == 0);
     }
   } else {
     tc::regs_inc<kRegsSoftmax>();
@@ -568,7 +582,6 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
     }
     bool ok = true;
     int slot = g;                         // of the Y1 ring
-    bool first_p = true;
     uint32_t slot_phase = 0, ph = 0;      // ph: parity of the group's count of half tiles
     while (pos.item < items && ok) {
       const int bh = p.walk.bh0 + pos.bhl;
@@ -649,7 +662,7 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
         if constexpr (!kKeys) {
           tc::fence_before_sync();
           __syncwarp();
-          if (lane == 0) tc::mbar_arrive(&p_ready[g]);
+          tc::mbar_arrive_if(&p_ready[g], lane == 0);
         }
         const float4* cv = reinterpret_cast<const float4*>(vec);
 #pragma unroll
@@ -719,9 +732,6 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
 #pragma unroll
         for (int i = 0; i < 64; ++i) pr[i] = exp2_here(pr[i]);
         if constexpr (kKeys) {
-          if (!kOver && !first_p && !tc::mbar_wait_warp(&a2_done[g], ph ^ 1, abort_flag)) { ok = false; break; }
-          tc::fence_after_sync();
-          first_p = false;
           if (drop) {
             // a dropped probability is kept as its negative: it still counts in dS's row term
             const uint4* kw4 = reinterpret_cast<const uint4*>(vec + 512 + quarter * 256);
@@ -740,12 +750,12 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
             uint32_t pk[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) pk[i] = pack16_relu<T>(pr[c * 32 + 2 * i], pr[c * 32 + 2 * i + 1]);
-            tc::tmem_st_x16(tmem_row + kColP + g * kPGroup + c * 16, pk);
+            tc::tmem_st_x16(tmem_row + kColP + g * 64 + c * 16, pk);
           }
           tc::tmem_st_wait();
           tc::fence_before_sync();
           __syncwarp();
-          if (lane == 0) tc::mbar_arrive(&p_ready[g]);
+          tc::mbar_arrive_if(&p_ready[g], lane == 0);
         }
         // ---- dS ----
         if (!tc::mbar_wait_warp(&dp_full[g], ph, abort_flag)) { ok = false; break; }
@@ -826,7 +836,7 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
         tc::tmem_st_wait();
         tc::fence_before_sync();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&ds_ready[g]);
+        tc::mbar_arrive_if(&ds_ready[g], lane == 0);
         ph ^= 1;
         slot += 2;
         if (slot >= kY1) { slot -= kY1; slot_phase ^= 1; }
@@ -846,16 +856,16 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
 }
 
 // One pass.
-template <int D, bool kKeys, bool kGeneral, typename T>
+template <int D, bool kKeys, bool kGeneral, bool kDrop, typename T>
 __global__ void __launch_bounds__(512, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ CUtensorMap tm_x2,
                  const __grid_constant__ CUtensorMap tm_y1, const __grid_constant__ CUtensorMap tm_y2,
                  const __grid_constant__ FlashBwdParams p) {
-  bwd_pass<D, kKeys, kGeneral, false, T>(tm_x1, tm_x2, tm_y1, tm_y2, p, blockIdx.x, gridDim.x);
+  bwd_pass<D, kKeys, kGeneral, kDrop, false, T>(tm_x1, tm_x2, tm_y1, tm_y2, p, blockIdx.x, gridDim.x);
 }
 
 // Both passes side by side, the dQ pass on the first `q_ctas` CTAs.
-template <int D, bool kGeneral, typename T>
+template <int D, bool kGeneral, bool kDrop, typename T>
 __global__ void __launch_bounds__(512, 1)
 flash_bwd_both_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -863,9 +873,9 @@ flash_bwd_both_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                       const __grid_constant__ FlashBwdParams pk, const int q_ctas) {
   const int cta = blockIdx.x;
   if (cta < q_ctas)
-    bwd_pass<D, false, kGeneral, true, T>(tm_q, tm_do, tm_k, tm_v, pq, cta, q_ctas);
+    bwd_pass<D, false, kGeneral, kDrop, true, T>(tm_q, tm_do, tm_k, tm_v, pq, cta, q_ctas);
   else
-    bwd_pass<D, true, kGeneral, true, T>(tm_k, tm_v, tm_q, tm_do, pk, cta - q_ctas,
+    bwd_pass<D, true, kGeneral, kDrop, true, T>(tm_k, tm_v, tm_q, tm_do, pk, cta - q_ctas,
                                          gridDim.x - q_ctas);
 }
 
@@ -922,12 +932,12 @@ static int launch_bwd(void (*kernel)(P...), int ctas, int smem, bool early, cuda
   return 4;
 }
 
-template <int D, bool kKeys, bool kGeneral, typename T>
+template <int D, bool kKeys, bool kGeneral, bool kDrop, typename T>
 static int launch_pass(const CUtensorMap& x1, const CUtensorMap& x2, const CUtensorMap& y1,
                        const CUtensorMap& y2, const FlashBwdParams& p, cudaStream_t stream) {
   constexpr int kSmem = BwdSmem<D, kKeys>::kTotal;
   static_assert(kSmem <= 227 * 1024, "flash backward: shared memory over the per-CTA limit");
-  auto kernel = flash_bwd_kernel<D, kKeys, kGeneral, T>;
+  auto kernel = flash_bwd_kernel<D, kKeys, kGeneral, kDrop, T>;
   static bool configured = false;
   if (!allow_smem(kernel, kSmem, configured)) return 3;
   const int64_t items = static_cast<int64_t>(p.walk.row_tiles) * p.walk.nbh * p.splits;
@@ -937,18 +947,18 @@ static int launch_pass(const CUtensorMap& x1, const CUtensorMap& x2, const CUten
 }
 
 // The passes of `pq` (dQ) and `pk` (dK / dV), side by side or one after the other
-template <int D, bool kGeneral, typename T>
+template <int D, bool kGeneral, bool kDrop, typename T>
 static int launch_passes(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v,
                          const CUtensorMap& dout, const FlashBwdParams& pq, const FlashBwdParams& pk,
                          int q_ctas, cudaStream_t stream) {
   if (q_ctas == 0) {
     // dQ first: with dropout it leaves the keep bits that the dK / dV pass reads
-    const int rc = launch_pass<D, false, kGeneral, T>(q, dout, k, v, pq, stream);
-    return rc != 0 ? rc : launch_pass<D, true, kGeneral, T>(k, v, q, dout, pk, stream);
+    const int rc = launch_pass<D, false, kGeneral, kDrop, T>(q, dout, k, v, pq, stream);
+    return rc != 0 ? rc : launch_pass<D, true, kGeneral, kDrop, T>(k, v, q, dout, pk, stream);
   }
   constexpr int kSmemQ = BwdSmem<D, false>::kTotal, kSmemK = BwdSmem<D, true>::kTotal;
   constexpr int kSmem = kSmemQ > kSmemK ? kSmemQ : kSmemK;
-  auto kernel = flash_bwd_both_kernel<D, kGeneral, T>;
+  auto kernel = flash_bwd_both_kernel<D, kGeneral, kDrop, T>;
   static bool configured = false;
   if (!allow_smem(kernel, kSmem, configured)) return 3;
   const int64_t items = static_cast<int64_t>(pk.walk.row_tiles) * pk.walk.nbh;
@@ -959,15 +969,15 @@ static int launch_passes(const CUtensorMap& q, const CUtensorMap& k, const CUten
                     q, k, v, dout, pq, pk, q_ctas);
 }
 
-template <typename T>
+template <bool kDrop, typename T>
 static int launch_typed(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v,
                         const CUtensorMap& dout, const FlashBwdParams& pq, const FlashBwdParams& pk,
                         int q_ctas, bool general, cudaStream_t stream) {
   if (pq.Dr <= 64)
-    return general ? launch_passes<64, true, T>(q, k, v, dout, pq, pk, q_ctas, stream)
-                   : launch_passes<64, false, T>(q, k, v, dout, pq, pk, q_ctas, stream);
-  return general ? launch_passes<128, true, T>(q, k, v, dout, pq, pk, q_ctas, stream)
-                 : launch_passes<128, false, T>(q, k, v, dout, pq, pk, q_ctas, stream);
+    return general ? launch_passes<64, true, kDrop, T>(q, k, v, dout, pq, pk, q_ctas, stream)
+                   : launch_passes<64, false, kDrop, T>(q, k, v, dout, pq, pk, q_ctas, stream);
+  return general ? launch_passes<128, true, kDrop, T>(q, k, v, dout, pq, pk, q_ctas, stream)
+                 : launch_passes<128, false, kDrop, T>(q, k, v, dout, pq, pk, q_ctas, stream);
 }
 
 static int round128(int n) { return (n + 127) / 128 * 128; }
@@ -1111,9 +1121,11 @@ int launch_flash_bwd(const void* q, const void* k, const void* v, const void* o,
     const int pairs = bh - at < plan.pairs ? bh - at : plan.pairs;
     pq.walk.set(p.Rq / 128, at, pairs, causal ? 2 : 0);
     pk.walk.set(p.Rk / 128, at, pairs, causal ? 1 : 0);
-    const int rc =
-        bf16 ? launch_typed<__nv_bfloat16>(tq, tk, tv, tdo, pq, pk, plan.q_ctas, general, stream)
-             : launch_typed<__half>(tq, tk, tv, tdo, pq, pk, plan.q_ctas, general, stream);
+#define FLASH_BWD_CASE(T_)                                                                          \
+  p.thr7 != 0 ? launch_typed<true, T_>(tq, tk, tv, tdo, pq, pk, plan.q_ctas, general, stream)       \
+              : launch_typed<false, T_>(tq, tk, tv, tdo, pq, pk, plan.q_ctas, general, stream)
+    const int rc = bf16 ? (FLASH_BWD_CASE(__nv_bfloat16)) : (FLASH_BWD_CASE(__half));
+#undef FLASH_BWD_CASE
     if (rc != 0) return rc;
   }
   if (plan.splits > 1) {

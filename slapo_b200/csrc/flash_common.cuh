@@ -83,6 +83,22 @@ template <> __device__ __forceinline__ uint32_t pack16_relu<__half>(float a, flo
   return d;
 }
 
+// Columns col .. col + 15 of a row of `cols` 16-bit values (a multiple of 8; padded columns are not part of
+// it).  Neighbouring rows lie whole lines apart, so that a store takes a cycle per row: one of 32 bytes
+// where rows keep to 32 bytes.
+__device__ __forceinline__ void store_cols16(void* row, int col, int cols, const uint32_t (&v)[8]) {
+  uint8_t* dst = static_cast<uint8_t*>(row) + col * 2;
+  if ((cols & 15) == 0) {
+    if (col < cols)
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]),
+                   "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                   : "memory");
+  } else {
+    if (col < cols) *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+    if (col + 8 < cols) *reinterpret_cast<uint4*>(dst + 16) = make_uint4(v[4], v[5], v[6], v[7]);
+  }
+}
+
 // Overlap of a kernel's prologue with the kernel before it in the stream: a kernel that the next
 // one may start under says so, and one that was launched that way waits until all work before it
 // is complete and visible (at once, when it was launched the ordinary way).
