@@ -10,39 +10,48 @@
 //
 // Per half tile, with rows on the TMEM lanes:
 //   tensor core   S = X1 Y1^T ,  dP = X2 Y2^T                       (fp32 in TMEM)
-//   4 warps       p = exp2(s - lse) ;  ds = p * (dp - delta)        (a row per thread; dropout
+//   8 warps       p = exp2(s - lse) ;  ds = p * (dp - delta)        (half a row per thread; dropout
 //                 replayed), P and dS written back to TMEM as 16 bit
 //   tensor core   accumulators += dS Y1 , P Y2                      (A operand from TMEM)
 // P and dS never pass through shared memory, and no transpose is needed: the two passes form
 // S with its rows where they want them.
 //
-// Two groups of four softmax warps take the half tiles in turn, each with its own barriers, so that one
-// group's exponentials run under the other's waits, loads and conversions.  Loads, S, dP and the
-// accumulating products have a thread each, which go through the sequence at their own pace, and four
-// more warps read finished accumulators out under the next work item.  CTAs are persistent.  The
+// Two groups of eight softmax warps take the half tiles in turn, each with its own barriers, so that one
+// group's exponentials run under the other's waits, loads and conversions; two threads share a row, which
+// needs no exchange here and halves what stands between two products.  Loads and products have threads of
+// their own, which go through the sequence at their own pace, and four more warps read finished
+// accumulators out under the next work item.  CTAs are persistent.  The
 // passes run side by side in one launch where that fills the GPU better (both_q_ctas); the keys of few
 // queries are split over work items.
 //
 // What that is for, measured by clocks in the kernel: one thread that issued all products under
 // `lane == 0` took 400 - 700 cycles for the four to eight of each kind (under elect.sync half of
 // that, their operands in uniform registers) and was what a tile of 128 waited for, with both halves
-// of its columns in the same phase.  Bound now for D = 64: the chain of a half tile within its group, 2200 -
-// 3000 cycles, of which exp2 alone needs 512 for each of the two; for D = 128 the products (64 cycles
-// each, 20 or 24 to a half tile: those of 64 columns take as long as those of 128).
-// Measured (all kernels of the backward; whole tiles, one issuing thread -> now): 32 x 512 x 16 heads of
-// 64, p 0.1: 315 -> 262 us; 4 x 2048 x 16 x 128 causal: 400 -> 310; 4 x 1000 x 32 x 80 causal with key bias: 227 ->
-// 183; 8 x 512 x 16 x 64 with T5's bias, key bias and p 0.1: 155 -> 142; 4 x 2048 x 16 x 128: 553 -> 421; 1 x 512 x
-// 16 x 64, p 0.1: 26 -> 25.
+// of its columns in the same phase.  Bound now for D = 64: the chain of a half tile within its group, 2000 -
+// 2700 cycles (waits, reads of tensor memory and hand-overs of 100 - 400 each next to 512 of exp2); for D = 128
+// the products (48 - 64 cycles each, 20 or 24 to a half tile: the first operand's 4 KB from shared memory are as
+// many for 64 columns as for 128).
+// Measured (all kernels of the backward; whole tiles, one issuing thread -> half tiles, a thread for each kind of
+// product): 32 x 512 x 16 heads of 64, p 0.1: 315 -> 262 us; 4 x 2048 x 16 x 128 causal: 400 -> 310; 4 x 1000 x 32 x 80
+// causal with key bias: 227 -> 183; 8 x 512 x 16 x 64 with T5's bias, key bias and p 0.1: 155 -> 142; 4 x 2048 x 16 x 128:
+// 553 -> 421.
 //
 // A single pass (5 products per tile instead of 7) has to add up dQ over the key tiles: one fp32
 // partial of dQ per key tile written and read again was most of its time (BERT-large, 32 x 512
 // tokens x 16 heads of 64: 268 MB each way).
 //
-// Later, on top of that (us): dropout as a template parameter (its draws were branches over code that has to be
+// On top of that (us): dropout as a template parameter (its draws were branches over code that has to be
 // fetched): dQ 117 -> 112, dK / dV 130 -> 123 for 32 x 512 x 16 x 64, p 0.1, dQ 82 -> 72 without; two sets of dK / dV
 // accumulators at D = 64 and dV's read out a step before dK's, rows stored 32 bytes at a time (a store takes a
 // cycle per row, and reads of shared memory queue behind it): dK / dV 123 -> 113 and, without dropout, 118 -> 101;
 // 4 x 2048 x 16 x 128 causal 161 -> 140; 16 x 200 x 16 x 128, both passes: 85 -> 64.
+//
+// Two threads a row instead of one, and the next S / dP of the dK / dV pass queued by the thread that issues the
+// product which uses up what stands in its place (us, dQ and dK / dV): 32 x 512 x 16 x 64, p 0.1: 110 -> 101 and 113 ->
+// 106, without dropout 71 -> 63 and 101 -> 89; 8 x 512 x 16 x 64 with T5's bias and p 0.1: 52 -> 47 and 80 -> 65; 4 x 2048 x
+// 16 x 64 causal: 98 -> 88 and 113 -> 110; 4 x 2048 x 16 x 128: 161 -> 156 and 230 -> 214.  (Two threads a row without the
+// queue, causal: dK / dV 113 -> 117; the queue in the dQ pass too: dQ 63 -> 66; S and dP by one text with the operands in
+// variables: dK / dV 89 -> 93.)
 //
 // With dropout the dQ pass draws the keep decisions (16 keys of a query row per Philox call, as
 // in the forward) and leaves them as one bit each, [B H][key / 32][query] words, for the dK / dV
@@ -130,10 +139,14 @@ __global__ void __launch_bounds__(256) flash_bwd_stats_kernel(
   }
 }
 
-// Registers per thread of the warpgroups: issuing, softmax (two), reading out; together the 128 per
-// thread that 512 threads are launched with.
-constexpr int kRegsIssue = 80, kRegsSoftmax = 176, kRegsOut = 80;
-static_assert(kRegsIssue + 2 * kRegsSoftmax + kRegsOut <= 4 * 128, "more registers than the block has");
+// Registers per thread of the warpgroups: issuing, softmax (four), reading out; together the 80 per thread
+// that 768 threads are launched with.
+constexpr int kBwdThreads = 768, kRegsLaunch = 80, kRegsSoftmax = 96;
+template <bool kDrop>
+struct BwdRegs {
+  static constexpr int kIssue = kDrop ? 48 : 56, kOut = kDrop ? 48 : 40;
+  static_assert(kIssue + 4 * kRegsSoftmax + kOut <= 6 * kRegsLaunch, "more registers than the block has");
+};
 
 template <int D, bool kKeys>
 struct BwdSmem {
@@ -149,17 +162,17 @@ struct BwdSmem {
   static constexpr int kY1At = 2 * kX * kTile;
   static constexpr int kY2At = kY1At + kY1 * kHalfTile;
   static constexpr int kVecs = kY2At + kY2 * kHalfTile;
-  static constexpr int kDrel = kVecs + kY1 * kVec;           // [8 warps][32] floats
-  // per softmax warp, twice: the relative bias of the 32 + 64 - 1 distances of its half tile
-  static constexpr int kRelFloats = 96;
-  static constexpr int kRel = kDrel + (kKeys ? 8 * 32 * 4 : 0);
-  static constexpr int kBars = kRel + 8 * 2 * kRelFloats * 4;
+  static constexpr int kDrel = kVecs + kY1 * kVec;           // [16 warps][32] floats
+  // per softmax warp, twice: the relative bias of the 32 + 32 - 1 distances of its rows and columns
+  static constexpr int kRelFloats = 64;
+  static constexpr int kRel = kDrel + (kKeys ? 16 * 32 * 4 : 0);
+  static constexpr int kBars = kRel + 16 * 2 * kRelFloats * 4;
   static constexpr int kTotal = kBars + 52 * 8 + 1024;
 };
 
-// 16 warps in four warpgroups: one thread each of warps 0 - 3 for the loads and the products; two
-// softmax groups (warps 4 - 7 and 8 - 11), one row per thread, which take the half tiles in turn; and
-// the warps that read the accumulators out (12 - 15).
+// 24 warps in six warpgroups: a thread each of warps 0 - 3 for the loads and the products; two softmax
+// groups (warps 4 - 11 and 12 - 19), a row and half of a half tile's columns per thread, which take the half
+// tiles in turn; and the warps that read the accumulators out (20 - 23).
 // kKeys: the dK / dV pass.  kGeneral: key bias, relative bias, causal mask or ragged lengths.
 // kDrop: with dropout.  kDraw: the dK / dV pass then draws the keep decisions itself, and the dQ pass leaves none.
 // CTA `cta` of `ctas` that run the pass.
@@ -188,9 +201,8 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
   uint64_t* s_full = bars + 28;       // one per softmax group from here on
   uint64_t* p_ready = bars + 30;      // 4 warps: S has been read (and P written)
   uint64_t* dp_full = bars + 32;
+  uint64_t* a1_done = bars + 36;      // dQ pass: dS of a half tile has been used up
   uint64_t* ds_ready = bars + 34;     // 4 warps: dS written
-  uint64_t* a1_done = bars + 36;      // the tensor core has read dS / P of a half tile
-  uint64_t* a2_done = bars + 38;
   uint64_t* acc1_full = bars + 40;    // kAcc (<= 2) each
   uint64_t* acc1_free = bars + 42;    // 4 warps
   uint64_t* acc2_full = bars + 44;
@@ -241,11 +253,10 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
       tc::mbar_init(&x2_full[i], 1);
       tc::mbar_init(&x2_empty[i], 1);
       tc::mbar_init(&s_full[i], 1);
-      tc::mbar_init(&p_ready[i], 4);
+      tc::mbar_init(&p_ready[i], 8);
       tc::mbar_init(&dp_full[i], 1);
-      tc::mbar_init(&ds_ready[i], 4);
       tc::mbar_init(&a1_done[i], 1);
-      tc::mbar_init(&a2_done[i], 1);
+      tc::mbar_init(&ds_ready[i], 8);
     }
     for (int i = 0; i < kY1; ++i) {
       tc::mbar_init(&y1_full[i], 1);
@@ -277,11 +288,11 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
   pdl_launch();
 
   if (warp < 4) {
-    tc::regs_dec<kRegsIssue>();
+    tc::regs_dec<BwdRegs<kDrop>::kIssue>();
     if (tc::elect_one()) {
-      // Four threads, each of which goes through the half tiles at its own pace: loads, S, dP and the
-      // accumulating products.  One thread for all products was what a half tile waited for: issuing
-      // takes it 40 - 50 cycles a product or commit and 80 a wait.
+      // Threads that go through the half tiles at their own pace: loads, S, dP and the accumulating products.
+      // One thread for all products was what a half tile waited for: issuing takes it 40 - 50 cycles a product or
+      // commit and 80 a wait.
       constexpr uint32_t kDescHi = tc::smem_desc_hi(1024);
       constexpr uint32_t kXStep = kTileBytes >> 4, kYStep = kHalfBytes >> 4;
       // S / dP of a half tile (64 streamed rows); x, y: low descriptor words
@@ -299,9 +310,18 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
       auto accumulate = [&](uint32_t col, uint32_t a_col, uint32_t y, bool fresh) {
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          tc::umma_f16_ts(tmem_base + col, tmem_base + a_col + kk * 8,
+          tc::umma_f16_ts(tmem_base + col, tmem_base + a_col + (kk >> 1) * 32 + (kk & 1) * 8,
                           tc::smem_desc_words(y + ((kk * 2048) >> 4), kDescHi), p.idesc_acc,
                           (fresh && kk == 0) ? 0u : 1u);
+      };
+      // where a thread of the dK / dV pass is with S / dP: half tile j of n of a work item
+      struct Lead {
+        int item, n, j;
+      };
+      auto lead_enter = [&](Lead& l) {
+        int tile, bhl, first;
+        l.j = 0;
+        if (l.item < items) l.n = item_at(l.item, tile, bhl, first);
       };
       bool ok = true;
       if (warp == 0) {
@@ -368,8 +388,8 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
             ok = true;
           }
         }
-      } else if (warp < 3) {
-        // ------------------------------ S (warp 1) and dP (warp 2) ------------------------------
+      } else if (!kKeys && warp < 3) {
+        // ------------------------------ dQ pass: S (warp 1) and dP (warp 2) ------------------------------
         const bool is_s = warp == 1;
         const uint32_t x_desc = tc::smem_desc_lo(tc::smem_u32(smem + (is_s ? 0 : L::kX2)), 16);
         const uint32_t y_desc = tc::smem_desc_lo(tc::smem_u32(smem + (is_s ? L::kY1At : L::kY2At)), 16);
@@ -378,8 +398,7 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
         uint64_t* x_empty = is_s ? x1_empty : x2_empty;
         uint64_t* y_full = is_s ? y1_full : y2_full;
         uint64_t* out_full = is_s ? s_full : dp_full;
-        // what stood there has been read (P, dS: used up)
-        uint64_t* out_free = is_s ? (kKeys ? a2_done : p_ready) : a1_done;
+        uint64_t* out_free = is_s ? p_ready : a1_done;      // what stood there has been read (dS: used up)
         const int slots = is_s ? kY1 : kY2;
         Ring<kX> x;
         int slot = 0, h = 0;
@@ -402,59 +421,129 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
             ok = true;
           }
         }
-      } else {
+      } else if (!kKeys) {
         // ------------------------------ accumulating products ------------------------------
-        // In the dK / dV pass dV's of half tile h go before dK's of h - 1, whose dS is ready later;
-        // over the ends of items they stay in their order.
         const uint32_t y1_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kY1At), kBlkY);
-        const uint32_t y2_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kY2At), kBlkY);
         Ring<kY1> r1;
-        Ring<kY2> r2;
         Ring<kAcc> acc;
         int h = 0;
         for (int item = cta; item < items && ok; item += ctas, acc.step()) {
           int tile, bhl, first;
           const int n = item_at(item, tile, bhl, first);
-          const uint32_t a1 = kColA1 + acc.slot * kAccCols, a2 = kColA2 + acc.slot * kAccCols;
-          auto add_a1 = [&](int i, bool fresh) -> bool {     // half tile i of the sequence
-            // (what these accumulators held has been read out)
-            if (fresh && !tc::mbar_wait(&acc1_free[acc.slot], acc.phase ^ 1, abort_flag)) return false;
-            if (!tc::mbar_wait(&ds_ready[i & 1], (i >> 1) & 1, abort_flag)) return false;
+          // (what these accumulators held has been read out)
+          ok = tc::mbar_wait(&acc1_free[acc.slot], acc.phase ^ 1, abort_flag);
+          for (int j = 0; j < n && ok; ++j, ++h, r1.step()) {
+            // (Y1 is there: S was formed from it before dS)
+            ok = tc::mbar_wait(&ds_ready[h & 1], (h >> 1) & 1, abort_flag);
+            if (!ok) break;
             tc::fence_after_sync();
-            accumulate(a1, kColDP + (i & 1) * 64, y1_desc + r1.slot * kYStep, fresh);
-            tc::umma_commit(&a1_done[i & 1]);
+            accumulate(kColA1 + acc.slot * kAccCols, kColDP + (h & 1) * 64, y1_desc + r1.slot * kYStep, j == 0);
+            tc::umma_commit(&a1_done[h & 1]);
             tc::umma_commit(&y1_empty[r1.slot]);
-            r1.step();
-            return true;
-          };
-          for (int j = 0; j < n; ++j, ++h) {
-            ok = false;
-            if constexpr (kKeys) {
-              // (P comes of S and says nothing about Y2, which is loaded after Y1; Y1 is there, S was
-              // formed from it before dS)
-              if (j == 0 && !tc::mbar_wait(&acc2_free[acc.slot], acc.phase ^ 1, abort_flag)) break;
-              if (!tc::mbar_wait(&y2_full[r2.slot], r2.phase, abort_flag) ||
-                  !tc::mbar_wait(&p_ready[h & 1], (h >> 1) & 1, abort_flag))
-                break;
-              tc::fence_after_sync();
-              accumulate(a2, kColP + (h & 1) * 64, y2_desc + r2.slot * kYStep, j == 0);
-              tc::umma_commit(&a2_done[h & 1]);
-              tc::umma_commit(&y2_empty[r2.slot]);
-              if (j + 1 == n) tc::umma_commit(&acc2_full[acc.slot]);
-              r2.step();
-              if (j > 0 && !add_a1(h - 1, j == 1)) break;
-              if (j + 1 == n && !add_a1(h, j == 0)) break;
-            } else {
-              if (!add_a1(h, j == 0)) break;
-            }
-            ok = true;
           }
           if (ok) tc::umma_commit(&acc1_full[acc.slot]);
         }
+      } else if (warp == 1) {
+        // ------------------------------ dK / dV pass: S and dV ------------------------------
+        // The next S of a group goes into the tensor core's queue behind the product that uses up the P in its
+        // place, two half tiles ahead.
+        const uint32_t x_desc = tc::smem_desc_lo(tc::smem_u32(smem), 16);
+        const uint32_t y_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kY1At), 16);
+        const uint32_t y2_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kY2At), kBlkY);
+        Ring<kX> x;
+        Ring<kY1> r1;
+        Ring<kY2> r2;
+        Ring<kAcc> acc;
+        Lead lead{cta, 0, 0};
+        lead_enter(lead);
+        auto next_s = [&](int g) -> bool {
+          if (lead.item >= items) return true;
+          if (lead.j == 0 && !tc::mbar_wait(&x1_full[x.slot], x.phase, abort_flag)) return false;
+          if (!tc::mbar_wait(&y1_full[r1.slot], r1.phase, abort_flag)) return false;
+          tc::fence_after_sync();
+          scores(kColS + g * 64, x_desc + x.slot * kXStep, y_desc + r1.slot * kYStep);
+          tc::umma_commit(&s_full[g]);
+          r1.step();
+          if (++lead.j == lead.n) {
+            tc::umma_commit(&x1_empty[x.slot]);
+            x.step();
+            lead.item += ctas;
+            lead_enter(lead);
+          }
+          return true;
+        };
+        ok = next_s(0) && next_s(1);
+        int h = 0;
+        for (int item = cta; item < items && ok; item += ctas, acc.step()) {
+          int tile, bhl, first;
+          const int n = item_at(item, tile, bhl, first);
+          // (what these accumulators held has been read out)
+          ok = tc::mbar_wait(&acc2_free[acc.slot], acc.phase ^ 1, abort_flag);
+          for (int j = 0; j < n && ok; ++j, ++h) {
+            ok = false;
+            // (P comes of S and says nothing about Y2, which is loaded after Y1)
+            if (!tc::mbar_wait(&y2_full[r2.slot], r2.phase, abort_flag) ||
+                !tc::mbar_wait(&p_ready[h & 1], (h >> 1) & 1, abort_flag))
+              break;
+            tc::fence_after_sync();
+            accumulate(kColA2 + acc.slot * kAccCols, kColP + (h & 1) * 64, y2_desc + r2.slot * kYStep, j == 0);
+            tc::umma_commit(&y2_empty[r2.slot]);
+            if (j + 1 == n) tc::umma_commit(&acc2_full[acc.slot]);
+            r2.step();
+            ok = next_s(h & 1);
+          }
+        }
+      } else if (warp == 2) {
+        // ------------------------------ accumulating products ------------------------------
+        // (dK / dV pass: dP and dK, likewise)
+        const uint32_t x_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kX2), 16);
+        const uint32_t y_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kY2At), 16);
+        const uint32_t y1_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kY1At), kBlkY);
+        Ring<kX> x;
+        Ring<kY1> r1;
+        Ring<kY2> r2;
+        Ring<kAcc> acc;
+        Lead lead{cta, 0, 0};
+        lead_enter(lead);
+        auto next_dp = [&](int g) -> bool {
+          if (lead.item >= items) return true;
+          if (lead.j == 0 && !tc::mbar_wait(&x2_full[x.slot], x.phase, abort_flag)) return false;
+          if (!tc::mbar_wait(&y2_full[r2.slot], r2.phase, abort_flag)) return false;
+          tc::fence_after_sync();
+          scores(kColDP + g * 64, x_desc + x.slot * kXStep, y_desc + r2.slot * kYStep);
+          tc::umma_commit(&dp_full[g]);
+          tc::umma_commit(&y2_empty[r2.slot]);
+          r2.step();
+          if (++lead.j == lead.n) {
+            tc::umma_commit(&x2_empty[x.slot]);
+            x.step();
+            lead.item += ctas;
+            lead_enter(lead);
+          }
+          return true;
+        };
+        ok = next_dp(0) && next_dp(1);
+        int h = 0;
+        for (int item = cta; item < items && ok; item += ctas, acc.step()) {
+          int tile, bhl, first;
+          const int n = item_at(item, tile, bhl, first);
+          ok = tc::mbar_wait(&acc1_free[acc.slot], acc.phase ^ 1, abort_flag);
+          for (int j = 0; j < n && ok; ++j, ++h) {
+            // (Y1 is there: S was formed from it before dS)
+            ok = tc::mbar_wait(&ds_ready[h & 1], (h >> 1) & 1, abort_flag);
+            if (!ok) break;
+            tc::fence_after_sync();
+            accumulate(kColA1 + acc.slot * kAccCols, kColDP + (h & 1) * 64, y1_desc + r1.slot * kYStep, j == 0);
+            tc::umma_commit(&y1_empty[r1.slot]);
+            if (j + 1 == n) tc::umma_commit(&acc1_full[acc.slot]);
+            r1.step();
+            ok = next_dp(h & 1);
+          }
+        }
       }
     }
-  } else if (warp >= 12) {
-    tc::regs_dec<kRegsOut>();
+  } else if (warp >= 20) {
+    tc::regs_dec<BwdRegs<kDrop>::kOut>();
     // ------------------------------ accumulators out of tensor memory ------------------------------
     // dS is formed without the factors scale and 1 / keep_prob; they are applied once to dQ and dK
     // (and 1 / keep_prob to dV) here
@@ -464,26 +553,22 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
     // D columns from `col` on, times f, to `dst` (or as they are to `share`)
     auto read_out = [&](uint32_t col, float f, T* dst, float* share, bool row_ok) {
 #pragma unroll
-      for (int c = 0; c < D; c += 32) {
-        uint32_t r[32];
-        tc::tmem_ld_x32(tmem_row + col + c, r);
+      for (int c = 0; c < D; c += 16) {
+        uint32_t r[16];
+        tc::tmem_ld_x16(tmem_row + col + c, r);
         tc::tmem_ld_wait();
         if (!row_ok) continue;
         if (!kKeys && share != nullptr) {
 #pragma unroll
-          for (int g = 0; g < 8; ++g)
-            if (c + g * 4 < p.Dr)
-              *reinterpret_cast<uint4*>(share + c + g * 4) =
-                  make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+          for (int g = 0; g < 16; g += 4)
+            if (c + g < p.Dr)
+              *reinterpret_cast<uint4*>(share + c + g) = make_uint4(r[g], r[g + 1], r[g + 2], r[g + 3]);
         } else {
+          uint32_t v[8];
 #pragma unroll
-          for (int g = 0; g < 32; g += 16) {
-            uint32_t v[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              v[i] = pack16<T>(__uint_as_float(r[g + 2 * i]) * f, __uint_as_float(r[g + 2 * i + 1]) * f);
-            store_cols16(dst, c + g, p.Dr, v);
-          }
+          for (int i = 0; i < 8; ++i)
+            v[i] = pack16<T>(__uint_as_float(r[2 * i]) * f, __uint_as_float(r[2 * i + 1]) * f);
+          store_cols16(dst, c, p.Dr, v);
         }
       }
     };
@@ -520,9 +605,10 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
     tc::regs_inc<kRegsSoftmax>();
     // ------------------------------ softmax groups ------------------------------
     const int quarter = warp & 3;
-    const int g = (warp - 4) >> 2;      // takes half tiles g, g + 2, ... of the CTA's sequence
+    const int g = (warp - 4) >> 3;      // takes half tiles g, g + 2, ... of the CTA's sequence
+    const int half = ((warp - 4) >> 2) & 1;      // ... and of each 32 columns
     const int r_in = quarter * 32 + lane;
-    const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + g * 64 + half * 32;
     PhiloxUniform rng{};
     if ((!kKeys || kDraw) && drop) rng = philox_uniform(p.rng);
     const uint32_t add4 = (128u - p.thr7) * 0x01010101u;
@@ -565,8 +651,8 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
     auto fetch_rel = [&](const Pos& pos, int buf) {
       const int head = (p.walk.bh0 + pos.bhl) % p.H;
       const float* src = p.rel + static_cast<int64_t>(head) * (p.Sq + p.Sk - 1) + p.Sq - 1;
-      const int r0 = pos.tile * 128 + quarter * 32, c0 = (pos.first + pos.j) * 64;
-      const int d0 = kKeys ? r0 - (c0 + 63) : c0 - (r0 + 31);
+      const int r0 = pos.tile * 128 + quarter * 32, c0 = (pos.first + pos.j) * 64 + half * 32;
+      const int d0 = kKeys ? r0 - (c0 + 31) : c0 - (r0 + 31);
 #pragma unroll
       for (int i = lane; i < L::kRelFloats; i += 32)
         cp_async4(rel_buf + buf * L::kRelFloats + i, src + max(1 - p.Sq, min(d0 + i, p.Sk - 1)));
@@ -590,7 +676,7 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
       const uint64_t drop_row = (static_cast<uint64_t>(bh) * p.Sq + min(row, p.Sq - 1)) * sk16;
       Pos next = pos;
       for (; pos.j < pos.n; pos.j += 2) {
-        const int col0 = (pos.first + pos.j) * 64;       // the half tile's first column
+        const int col0 = (pos.first + pos.j) * 64 + half * 32;       // this warp's first column
         const uint8_t* vec = s_vec + slot * L::kVec;
         if (pos.j + 2 >= pos.n) {       // the item's last: the next one's rows, under its work
           next.u0 += pos.n;
@@ -606,37 +692,27 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
           if (next.item < items) fetch_rel(next, ph ^ 1);
         }
         // ---- dropout decisions of this row and the half tile's keys (dQ pass) ----
-        uint32_t keep16[4][4];
+        uint32_t keep16[2][4];
         if (!kKeys && drop) {
-          uint32_t bits[2];
+          uint32_t bits = 0;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
+          for (int q = 0; q < 2; ++q) {
             const uint4 kw = philox_keep16(rng, drop_row + (col0 >> 4) + q, add4);
             keep16[q][0] = kw.x; keep16[q][1] = kw.y; keep16[q][2] = kw.z; keep16[q][3] = kw.w;
-            if constexpr (!kDraw) {
-              const uint32_t m = keep_bits16(kw);
-              if (q & 1) bits[q >> 1] |= m << 16;
-              else bits[q >> 1] = m;
-            }
+            if constexpr (!kDraw) bits |= keep_bits16(kw) << (q * 16);
           }
-          if constexpr (!kDraw) {
-            uint32_t* dst = p.keep + (static_cast<int64_t>(pos.bhl) * (p.Rk >> 5) + (col0 >> 5)) * p.Rq + row;
-            dst[0] = bits[0];
-            dst[p.Rq] = bits[1];
-          }
+          if constexpr (!kDraw)
+            p.keep[(static_cast<int64_t>(pos.bhl) * (p.Rk >> 5) + (col0 >> 5)) * p.Rq + row] = bits;
         }
-        // ---- ... of the warp's 32 keys and the half tile's queries (dK / dV pass), two queries per lane,
-        // into the words that the other form loads ----
+        // ---- ... of the warp's 32 keys and 32 queries (dK / dV pass), a query per lane, into the words that
+        // the other form loads ----
         if constexpr (kKeys && kDraw) {
           if (drop) {
-            uint32_t* words = reinterpret_cast<uint32_t*>(s_vec + slot * L::kVec + 512 + quarter * 256);
-#pragma unroll
-            for (int i = lane; i < 64; i += 32) {
-              const uint64_t at = (static_cast<uint64_t>(bh) * p.Sq + min(col0 + i, p.Sq - 1)) * sk16 +
-                                  ((pos.tile * 128 + quarter * 32) >> 4);
-              words[i] = keep_bits16(philox_keep16(rng, at, add4)) |
-                         keep_bits16(philox_keep16(rng, at + 1, add4)) << 16;
-            }
+            uint32_t* words = reinterpret_cast<uint32_t*>(s_vec + slot * L::kVec + 512 + quarter * 256) + half * 32;
+            const uint64_t at = (static_cast<uint64_t>(bh) * p.Sq + min(col0 + lane, p.Sq - 1)) * sk16 +
+                                ((pos.tile * 128 + quarter * 32) >> 4);
+            words[lane] = keep_bits16(philox_keep16(rng, at, add4)) |
+                          keep_bits16(philox_keep16(rng, at + 1, add4)) << 16;
             __syncwarp();
           }
         }
@@ -647,26 +723,22 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
           if (!tc::mbar_wait_warp(&y1_full[slot], slot_phase, abort_flag)) { ok = false; break; }
         }
         tc::fence_after_sync();
-        float pr[64];
+        float pr[32];
         {
-          uint32_t s0[32], s1[32];
-          tc::tmem_ld_x32(tmem_row + kColS + g * 64, s0);
-          tc::tmem_ld_x32(tmem_row + kColS + g * 64 + 32, s1);
+          uint32_t s0[32];
+          tc::tmem_ld_x32(tmem_row + kColS, s0);
           tc::tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            pr[i] = __uint_as_float(s0[i]);
-            pr[32 + i] = __uint_as_float(s1[i]);
-          }
+          for (int i = 0; i < 32; ++i) pr[i] = __uint_as_float(s0[i]);
         }
         if constexpr (!kKeys) {
           tc::fence_before_sync();
           __syncwarp();
           tc::mbar_arrive_if(&p_ready[g], lane == 0);
         }
-        const float4* cv = reinterpret_cast<const float4*>(vec);
+        const float4* cv = reinterpret_cast<const float4*>(vec) + half * 8;
 #pragma unroll
-        for (int i = 0; i < 64; i += 4) {
+        for (int i = 0; i < 32; i += 4) {
           uint64_t x0 = f2_pack(pr[i], pr[i + 1]), x1 = f2_pack(pr[i + 2], pr[i + 3]);
           if constexpr (kKeys) {
             const float4 c = cv[i >> 2];
@@ -686,17 +758,17 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
         if constexpr (kGeneral) {
           if (!kKeys && p.kb2 != nullptr) {
 #pragma unroll
-            for (int i = 0; i < 64; i += 4) {
+            for (int i = 0; i < 32; i += 4) {
               const float4 c = cv[i >> 2];
               f2_unpack(f2_add(f2_pack(pr[i], pr[i + 1]), f2_pack(c.x, c.y)), pr[i], pr[i + 1]);
               f2_unpack(f2_add(f2_pack(pr[i + 2], pr[i + 3]), f2_pack(c.z, c.w)), pr[i + 2], pr[i + 3]);
             }
           }
           if (has_rel) {
-            const float* rel = rel_buf + ph * L::kRelFloats + (kKeys ? lane + 63 : 31 - lane);
+            const float* rel = rel_buf + ph * L::kRelFloats + (kKeys ? lane + 31 : 31 - lane);
             const uint64_t log2e2 = f2_pack(kLog2e, kLog2e);
 #pragma unroll
-            for (int i = 0; i < 64; i += 2) {
+            for (int i = 0; i < 32; i += 2) {
               const uint64_t x = f2_fma(kKeys ? f2_pack(rel[-i], rel[-i - 1]) : f2_pack(rel[i], rel[i + 1]),
                                         log2e2, f2_pack(pr[i], pr[i + 1]));
               f2_unpack(x, pr[i], pr[i + 1]);
@@ -705,39 +777,31 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
           if constexpr (kKeys) {
             // key `row` is seen by queries >= row - diag (queries beyond Sq have nlse = -inf)
             if (p.causal && col0 + diag < pos.tile * 128 + quarter * 32 + 31) {
-              const int from = row - diag - col0;
+              const uint32_t hidden = low_bits(row - diag - col0);
 #pragma unroll
-              for (int c = 0; c < 2; ++c) {
-                const uint32_t hidden = low_bits(from - c * 32);
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                  if (hidden & (1u << i)) pr[c * 32 + i] = -INFINITY;
-              }
+              for (int i = 0; i < 32; ++i)
+                if (hidden & (1u << i)) pr[i] = -INFINITY;
             }
           } else {
             const int first_limit = p.causal ? min(p.Sk, pos.tile * 128 + quarter * 32 + diag + 1) : p.Sk;
-            if (col0 + 64 > first_limit) {
-              const int limit = (p.causal ? min(p.Sk, row + diag + 1) : p.Sk) - col0;
+            if (col0 + 32 > first_limit) {
+              const uint32_t seen = low_bits((p.causal ? min(p.Sk, row + diag + 1) : p.Sk) - col0);
 #pragma unroll
-              for (int c = 0; c < 2; ++c) {
-                const uint32_t seen = low_bits(limit - c * 32);
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                  if (!(seen & (1u << i))) pr[c * 32 + i] = -INFINITY;
-              }
+              for (int i = 0; i < 32; ++i)
+                if (!(seen & (1u << i))) pr[i] = -INFINITY;
             }
           }
         }
         // (kept before the waits that follow: the compiler would move it behind them)
 #pragma unroll
-        for (int i = 0; i < 64; ++i) pr[i] = exp2_here(pr[i]);
+        for (int i = 0; i < 32; ++i) pr[i] = exp2_here(pr[i]);
         if constexpr (kKeys) {
           if (drop) {
             // a dropped probability is kept as its negative: it still counts in dS's row term
-            const uint4* kw4 = reinterpret_cast<const uint4*>(vec + 512 + quarter * 256);
+            const uint4* kw4 = reinterpret_cast<const uint4*>(vec + 512 + quarter * 256) + half * 8;
             const uint32_t lane_bit = 1u << lane;
 #pragma unroll
-            for (int i = 0; i < 64; i += 4) {
+            for (int i = 0; i < 32; i += 4) {
               const uint4 kw = kw4[i >> 2];
               pr[i] = kw.x & lane_bit ? pr[i] : -pr[i];
               pr[i + 1] = kw.y & lane_bit ? pr[i + 1] : -pr[i + 1];
@@ -745,13 +809,10 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
               pr[i + 3] = kw.w & lane_bit ? pr[i + 3] : -pr[i + 3];
             }
           }
+          uint32_t pk[16];
 #pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            uint32_t pk[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) pk[i] = pack16_relu<T>(pr[c * 32 + 2 * i], pr[c * 32 + 2 * i + 1]);
-            tc::tmem_st_x16(tmem_row + kColP + g * 64 + c * 16, pk);
-          }
+          for (int i = 0; i < 16; ++i) pk[i] = pack16_relu<T>(pr[2 * i], pr[2 * i + 1]);
+          tc::tmem_st_x16(tmem_row + kColP, pk);
           tc::tmem_st_wait();
           tc::fence_before_sync();
           __syncwarp();
@@ -760,22 +821,26 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
         // ---- dS ----
         if (!tc::mbar_wait_warp(&dp_full[g], ph, abort_flag)) { ok = false; break; }
         tc::fence_after_sync();
+        // Sums along the diagonals key - query = const, for the gradient of T5's table: the running sum moves
+        // one lane up (next key) with every column (next query), so that it stays on its diagonal;
+        // what leaves at lane 31 is collected and added to the result 32 at a time.
+        float diagonal = 0.f;
+        float* buf = reinterpret_cast<float*>(smem + L::kDrel) + (warp - 4) * 32;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t d[32];
-          tc::tmem_ld_x32(tmem_row + kColDP + g * 64 + c * 32, d);
+        for (int c = 0; c < 32; c += 16) {
+          uint32_t d[16];
+          tc::tmem_ld_x16(tmem_row + kColDP + c, d);
           tc::tmem_ld_wait();
           if (!kKeys && drop) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              d[i] &= keep_mask_full(keep16[c * 2 + (i >> 4)][(i >> 2) & 3], i & 3);
+            for (int i = 0; i < 16; ++i) d[i] &= keep_mask_full(keep16[c >> 4][i >> 2], i & 3);
           }
-          const float4* nd = reinterpret_cast<const float4*>(vec + 256) + c * 8;
-          const float* v = pr + c * 32;
-          float ds[32];
+          const float4* nd = reinterpret_cast<const float4*>(vec + 256) + half * 8 + (c >> 2);
+          const float* v = pr + c;
+          float ds[16];
           if (kKeys && drop) {
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
+            for (int i = 0; i < 16; i += 4) {
               const float4 dl = nd[i >> 2];
               const float n4[4] = {dl.x, dl.y, dl.z, dl.w};
 #pragma unroll
@@ -784,7 +849,7 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
             }
           } else {
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
+            for (int i = 0; i < 16; i += 4) {
               uint64_t x0 = f2_load(d + i), x1 = f2_load(d + i + 2);
               if constexpr (kKeys) {
                 const float4 dl = nd[i >> 2];
@@ -802,36 +867,34 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
           }
           if constexpr (kKeys && kGeneral) {
             if (p.drel != nullptr) {
-              // Sums along the diagonals key - query = const: the running sum moves one lane up
-              // (next key) with every column (next query), so that it stays on its diagonal;
-              // what leaves at lane 31 is collected and added to the result 32 at a time.
-              float* buf = reinterpret_cast<float*>(smem + L::kDrel) + (warp - 4) * 32;
-              float* out = p.drel + static_cast<int64_t>(bh % p.H) * (p.Sq + p.Sk - 1);
-              const int key0 = pos.tile * 128 + quarter * 32, q0 = col0 + c * 32;
-              const int last = p.Sq + p.Sk - 2;
-              float acc = 0.f;
 #pragma unroll
-              for (int i = 0; i < 32; ++i) {
+              for (int i = 0; i < 16; ++i) {
                 // padding: keys beyond Sk have a P (their rows go nowhere else), queries have none
-                if (row < p.Sk) acc += ds[i];
-                acc = __shfl_sync(0xffffffffu, acc, (lane + 31) & 31);
+                if (row < p.Sk) diagonal += ds[i];
+                diagonal = __shfl_sync(0xffffffffu, diagonal, (lane + 31) & 31);
                 if (lane == 0) {
-                  buf[i] = acc;               // diagonal key0 + 31 - (q0 + i)
-                  acc = 0.f;
+                  buf[c + i] = diagonal;      // diagonal key0 + 31 - (col0 + c + i)
+                  diagonal = 0.f;
                 }
               }
-              __syncwarp();
-              const int at = key0 + 31 - (q0 + lane) + p.Sq - 1;
-              if (at >= 0 && at <= last) atomicAdd(out + at, buf[lane] * p.inv_keep);
-              const int rest = key0 + lane - (q0 + 32) + p.Sq - 1;     // still under way in the lanes
-              if (lane > 0 && rest >= 0 && rest <= last) atomicAdd(out + rest, acc * p.inv_keep);
-              __syncwarp();
             }
           }
-          uint32_t pk[16];
+          uint32_t pk[8];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) pk[i] = pack16<T>(ds[2 * i], ds[2 * i + 1]);
-          tc::tmem_st_x16(tmem_row + kColDP + g * 64 + c * 16, pk);
+          for (int i = 0; i < 8; ++i) pk[i] = pack16<T>(ds[2 * i], ds[2 * i + 1]);
+          tc::tmem_st_x8(tmem_row + kColDP + (c >> 1), pk);
+        }
+        if constexpr (kKeys && kGeneral) {
+          if (p.drel != nullptr) {
+            float* out = p.drel + static_cast<int64_t>(bh % p.H) * (p.Sq + p.Sk - 1);
+            const int key0 = pos.tile * 128 + quarter * 32, last = p.Sq + p.Sk - 2;
+            __syncwarp();
+            const int at = key0 + 31 - (col0 + lane) + p.Sq - 1;
+            if (at >= 0 && at <= last) atomicAdd(out + at, buf[lane] * p.inv_keep);
+            const int rest = key0 + lane - (col0 + 32) + p.Sq - 1;     // still under way in the lanes
+            if (lane > 0 && rest >= 0 && rest <= last) atomicAdd(out + rest, diagonal * p.inv_keep);
+            __syncwarp();
+          }
         }
         tc::tmem_st_wait();
         tc::fence_before_sync();
@@ -857,7 +920,7 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
 
 // One pass.
 template <int D, bool kKeys, bool kGeneral, bool kDrop, typename T>
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(kBwdThreads, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ CUtensorMap tm_x2,
                  const __grid_constant__ CUtensorMap tm_y1, const __grid_constant__ CUtensorMap tm_y2,
                  const __grid_constant__ FlashBwdParams p) {
@@ -866,7 +929,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constan
 
 // Both passes side by side, the dQ pass on the first `q_ctas` CTAs.
 template <int D, bool kGeneral, bool kDrop, typename T>
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(kBwdThreads, 1)
 flash_bwd_both_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                       const __grid_constant__ FlashBwdParams pq,
@@ -918,7 +981,7 @@ static int launch_bwd(void (*kernel)(P...), int ctas, int smem, bool early, cuda
                       const A&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(512);
+  cfg.blockDim = dim3(kBwdThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr{};
