@@ -88,6 +88,18 @@ struct FlashBwdParams {
   int* status;
 };
 
+// s + a.x b.x + a.y b.y of two 16-bit pairs
+template <typename T> __device__ __forceinline__ float dot_pair(uint32_t a, uint32_t b, float s);
+template <> __device__ __forceinline__ float dot_pair<__nv_bfloat16>(uint32_t a, uint32_t b, float s) {
+  s = fmaf(__uint_as_float(a << 16), __uint_as_float(b << 16), s);
+  return fmaf(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u), s);
+}
+template <> __device__ __forceinline__ float dot_pair<__half>(uint32_t a, uint32_t b, float s) {
+  const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&a));
+  const float2 y = __half22float2(*reinterpret_cast<const __half2*>(&b));
+  return fmaf(x.y, y.y, fmaf(x.x, y.x, s));
+}
+
 // Row statistics in the layout the kernels read, one launch:
 //   nlse   [B H][Rq]  -log2(e) * lse
 //   ndelta [B H][Rq]  -keep_prob * sum_d dO[b, i, h, d] * O[b, i, h, d]
@@ -109,21 +121,33 @@ __global__ void __launch_bounds__(256) flash_bwd_stats_kernel(
       kb2[static_cast<int64_t>(b) * Rk + key] =
           key < Sk ? kbias[static_cast<int64_t>(b) * Sk + key] * kLog2e : 0.f;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int rows_per_warp = 32 / lanes;        // `lanes` (8 or 16) threads share a row of Dr
+  // `lanes` (8 or 16) threads share a row of Dr; a warp's rows four at a time, all of their loads first (one at
+  // a time the kernel ran at half of the memory's rate: 4 x 2048 x 16 x 128: 18.5 -> 13.3 us, 4 x 1000 x 32 x 80: 17 -> 12)
+  const int rows_per_warp = 32 / lanes;
   const int d = (lane % lanes) * 8;
-  for (int r = warp * rows_per_warp + lane / lanes; r < 256; r += 8 * rows_per_warp) {
-    const int i = i0 + (r >> 3), h = h0 + (r & 7);    // neighbouring heads are contiguous
-    float s = 0.f;
-    if (i < Sq && h < H && d < Dr) {
-      const int64_t at = ((static_cast<int64_t>(b) * Sq + i) * H + h) * Dr + d;
-      float x[8], y[8];
-      Vec8<T>::load(dout + at, x);
-      Vec8<T>::load(out + at, y);
+  constexpr int kAhead = 4;                    // (256 rows are 8 or 16 rounds)
+  for (int r0 = warp * rows_per_warp + lane / lanes; r0 < 256; r0 += kAhead * 8 * rows_per_warp) {
+    uint4 x[kAhead], y[kAhead];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) s += x[k] * y[k];
+    for (int u = 0; u < kAhead; ++u) {
+      const int r = r0 + u * 8 * rows_per_warp, i = i0 + (r >> 3), h = h0 + (r & 7);    // neighbouring heads are contiguous
+      x[u] = y[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (i < Sq && h < H && d < Dr) {
+        const int64_t at = ((static_cast<int64_t>(b) * Sq + i) * H + h) * Dr + d;
+        x[u] = __ldg(reinterpret_cast<const uint4*>(dout + at));
+        y[u] = __ldg(reinterpret_cast<const uint4*>(out + at));
+      }
     }
-    for (int o = lanes >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane % lanes == 0) sums[r & 7][r >> 3] = s;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      float s = dot_pair<T>(x[u].x, y[u].x, 0.f);
+      s = dot_pair<T>(x[u].y, y[u].y, s);
+      s = dot_pair<T>(x[u].z, y[u].z, s);
+      s = dot_pair<T>(x[u].w, y[u].w, s);
+      for (int o = lanes >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const int r = r0 + u * 8 * rows_per_warp;
+      if (lane % lanes == 0) sums[r & 7][r >> 3] = s;
+    }
   }
   __syncthreads();
   const int h = h0 + warp, i = i0 + lane;
