@@ -46,8 +46,16 @@ struct Gemm2Params {
   int wide_store;     // rows of C are 32-byte aligned: the epilogue stores whole sectors
 };
 
-constexpr int kEpiWarps = 8;   // epilogue warps per CTA: two per quarter of the tensor-memory lanes,
-                               // each taking half of the tile's columns
+// Epilogue warps per CTA: two per quarter of the tensor-memory lanes, each taking half of the tile's columns, or
+// four with a quarter of them each.  Sixteen warps drain a tile faster (their reads of tensor memory and stores
+// wait side by side), which counts where the epilogue is what a tile takes: a GeLU in it, or a short contraction.
+// With a long one their registers and polls cost a little.  Measured, 8 -> 16 (us, L2 flushed):
+//   16384 x 4096, K = 1024: plain 94.0 -> 89.3, GeLU 97.6 -> 89.7, product kept too 107.6 -> 102.0, GeLU's derivative
+//     133.6 -> 126.4, tanh form's 132.6 -> 129.6, ReLU's 113.3 -> 119.6
+//   8192 x 4096, K = 1024: 52.0 -> 50.5, 52.7 -> 49.4, 57.7 -> 54.7, 71.2 -> 70.1, 69.9 -> 70.8, 62.2 -> 65.1
+//   2048 x 3072, K = 768: plain 19.8 -> 19.3;  16384 x 1024, K = 4096: plain 93.1 -> 94.7;  4096 x 10240, K = 2560: 128.4 -> 129.5
+constexpr int kManyEpiWarpsK = 1536;      // plain products up to this K have sixteen
+constexpr int epi_warps(int kind) { return kind == kEpiGeluTanhBwd || kind == kEpiReluBwd ? 8 : 16; }
 constexpr int PBM = 128;   // rows of A per CTA (the pair's tile has 256)
 constexpr int PBK = 64;
 #ifndef SLAPO_GEMM2_KSUB
@@ -163,7 +171,7 @@ __device__ __forceinline__ void tile_at(int tile, int tiles_m, int tiles_n, int&
 }
 
 // kEpi: what rides in the epilogue (gemm_epilogue.cuh); kEpiPlain: bias and ReLU
-template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN, int kEpi>
+template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN, int kEpi, int kEpiWarps>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * kEpiWarps, 1)
 gemm2_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
                   const __grid_constant__ CUtensorMap tmap_b, const Gemm2Params p) {
@@ -308,7 +316,7 @@ gemm2_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
   } else {
     // ------------------------------ epilogue (both CTAs) ----------------------------------
     const int quarter = warp & 3;  // TMEM lane quarter this warp may read
-    // with eight warps, warps w and w + 4 share a quarter and split the columns
+    // warps w, w + 4, .. share a quarter and split the columns
     const int col_part = (warp - 2) >> 2, col_parts = kEpiWarps / 4;
     constexpr int kChunks = BN / 32;
     const int c_begin = col_part * (kChunks / col_parts), c_end = c_begin + kChunks / col_parts;
@@ -465,11 +473,11 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const Gemm2Params p)
 bool cached_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer,
                     uint64_t stride, uint32_t box_outer, bool bf16);
 
-template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN, int kEpi = kEpiPlain>
-static int launch_pair_variant(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm2Params& p,
+template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN, int kEpi, int kEpiWarps>
+static int launch_pair_warps(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm2Params& p,
                                cudaStream_t stream) {
   using S = Gemm2Smem<BN, STAGES, KSUB>;
-  auto kernel = gemm2_tc05_kernel<BN, STAGES, KSUB, A_MN, B_MN, kEpi>;
+  auto kernel = gemm2_tc05_kernel<BN, STAGES, KSUB, A_MN, B_MN, kEpi, kEpiWarps>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal) !=
@@ -490,6 +498,20 @@ static int launch_pair_variant(const CUtensorMap& ta, const CUtensorMap& tb, con
     splitk_reduce_kernel<<<static_cast<int>(blocks < cap ? blocks : cap), 256, 0, stream>>>(p);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN, int kEpi = kEpiPlain>
+static int launch_pair_variant(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm2Params& p,
+                               cudaStream_t stream) {
+  if constexpr (kEpi != kEpiPlain) {
+    return launch_pair_warps<BN, STAGES, KSUB, A_MN, B_MN, kEpi, epi_warps(kEpi)>(ta, tb, p, stream);
+  } else {
+    // (a weight gradient's contraction is over the tokens; narrow tiles are short calls)
+    if constexpr (!A_MN && BN == 256)
+      if (p.K <= kManyEpiWarpsK && p.splits == 1)
+        return launch_pair_warps<BN, STAGES, KSUB, A_MN, B_MN, kEpi, 16>(ta, tb, p, stream);
+    return launch_pair_warps<BN, STAGES, KSUB, A_MN, B_MN, kEpi, 8>(ta, tb, p, stream);
+  }
 }
 
 // Number of CTA pairs that share one output tile: 1 unless the tiles alone leave most of the
