@@ -7,29 +7,12 @@
 #include "kernels.h"
 
 int* slapo_status_ptr(int device);
+slapo::PhiloxArgs unpack_rng(const c10::optional<at::Tensor>& rng);      // bindings.cpp
 
 namespace {
 
 using at::Tensor;
 using c10::optional;
-
-slapo::PhiloxArgs unpack_rng(const optional<Tensor>& rng) {
-  slapo::PhiloxArgs a{};
-  if (!rng.has_value() || !rng->defined()) return a;
-  TORCH_CHECK(rng->device().is_cpu() && rng->scalar_type() == at::kLong && rng->numel() == 4,
-              "rng must be the CPU int64[4] tensor returned by philox_reserve");
-  const int64_t* r = rng->data_ptr<int64_t>();
-  a.captured = static_cast<int>(r[3]);
-  a.offset_intragraph = static_cast<uint32_t>(r[2]);
-  if (a.captured) {
-    a.seed_ptr = reinterpret_cast<const int64_t*>(r[0]);
-    a.offset_ptr = reinterpret_cast<const int64_t*>(r[1]);
-  } else {
-    a.seed = static_cast<uint64_t>(r[0]);
-    a.offset = static_cast<uint64_t>(r[1]);
-  }
-  return a;
-}
 
 void check_bshd(const Tensor& t, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.dim() == 4, name, " must be a CUDA tensor [B, S, H, D]");

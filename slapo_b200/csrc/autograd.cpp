@@ -152,11 +152,16 @@ struct MlpFn : public Function<MlpFn> {
       at = h;
     }
     if (p > 0.0) {
-      Tensor t = gemm(h, w2, c10::nullopt, -1, false, false, false);
-      Tensor rng = philox_reserve(t.numel());
-      static auto f = op<Tensor(const Tensor&, const optional<Tensor>&, const optional<Tensor>&, double,
-                                const Tensor&)>("slapo_b200::bias_dropout_add_fwd");
-      y = f.call(t, b2, c10::nullopt, p, rng);
+      Tensor rng = philox_reserve(h.size(0) * w2.size(0));
+      if (h.size(0) > 16 && w2.size(0) % 16 == 0) {      // dropout in the product's epilogue
+        static auto f = op<Tensor(const Tensor&, const Tensor&, const optional<Tensor>&, double, const Tensor&)>(
+            "slapo_b200::gemm_dropout_fwd");
+        y = f.call(h, w2, b2, p, rng);
+      } else {
+        static auto f = op<Tensor(const Tensor&, const optional<Tensor>&, const optional<Tensor>&, double,
+                                  const Tensor&)>("slapo_b200::bias_dropout_add_fwd");
+        y = f.call(gemm(h, w2, c10::nullopt, -1, false, false, false), b2, c10::nullopt, p, rng);
+      }
       ctx->saved_data["rng"] = rng;
     } else {
       y = gemm(h, w2, b2, -1, false, false, false);

@@ -7,6 +7,25 @@
 
 #include "kernels.h"
 
+// a generator state of philox_reserve as the kernels take it (all zero without one)
+slapo::PhiloxArgs unpack_rng(const c10::optional<at::Tensor>& rng) {
+  slapo::PhiloxArgs a{};
+  if (!rng.has_value() || !rng->defined()) return a;
+  TORCH_CHECK(rng->device().is_cpu() && rng->scalar_type() == at::kLong && rng->numel() == 4,
+              "rng must be the CPU int64[4] tensor returned by philox_reserve");
+  const int64_t* r = rng->data_ptr<int64_t>();
+  a.captured = static_cast<int>(r[3]);
+  a.offset_intragraph = static_cast<uint32_t>(r[2]);
+  if (a.captured) {
+    a.seed_ptr = reinterpret_cast<const int64_t*>(r[0]);
+    a.offset_ptr = reinterpret_cast<const int64_t*>(r[1]);
+  } else {
+    a.seed = static_cast<uint64_t>(r[0]);
+    a.offset = static_cast<uint64_t>(r[1]);
+  }
+  return a;
+}
+
 namespace {
 
 using at::Tensor;
@@ -61,24 +80,6 @@ Tensor philox_reserve(int64_t increment) {
   o[2] = static_cast<int64_t>(st.offset_intragraph_);
   o[3] = st.captured_ ? 1 : 0;
   return out;
-}
-
-slapo::PhiloxArgs unpack_rng(const optional<Tensor>& rng) {
-  slapo::PhiloxArgs a{};
-  if (!rng.has_value() || !rng->defined()) return a;
-  TORCH_CHECK(rng->device().is_cpu() && rng->scalar_type() == at::kLong && rng->numel() == 4,
-              "rng must be the CPU int64[4] tensor returned by philox_reserve");
-  const int64_t* r = rng->data_ptr<int64_t>();
-  a.captured = static_cast<int>(r[3]);
-  a.offset_intragraph = static_cast<uint32_t>(r[2]);
-  if (a.captured) {
-    a.seed_ptr = reinterpret_cast<const int64_t*>(r[0]);
-    a.offset_ptr = reinterpret_cast<const int64_t*>(r[1]);
-  } else {
-    a.seed = static_cast<uint64_t>(r[0]);
-    a.offset = static_cast<uint64_t>(r[1]);
-  }
-  return a;
 }
 
 // ------------------------------------------------------------------------ //

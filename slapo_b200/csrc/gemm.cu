@@ -90,6 +90,9 @@ struct GemmParams {
   const void* Z;      // kEpi backward: input (ReLU: output) of the activation, as C in memory
   float* col_part;    // kEpi backward: column sums over 32 rows each, or nullptr
   int c2_sum;         // kEpi forward: C2 includes the bias
+  PhiloxArgs rng;     // kEpiDropout: generator state, what a draw is compared by, factor of kept values
+  uint32_t drop_add4;
+  float drop_scale;
 };
 
 constexpr int BM = 128;
@@ -385,8 +388,14 @@ int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, 
   p.Z = epi != nullptr ? epi->z : nullptr;
   p.col_part = epi != nullptr ? epi->col_part : nullptr;
   p.c2_sum = epi != nullptr && epi->c2_sum ? 1 : 0;
+  if (epi != nullptr && epi->rng != nullptr) {
+    p.rng = *epi->rng;
+    p.drop_add4 = (128u - dropout_thr7(epi->p)) * 0x01010101u;
+    p.drop_scale = dropout_scale(epi->p);
+  }
   if (epi != nullptr && epi->kind != kEpiPlain) {
     if (a_mn || b_mn != epi_backward(epi->kind)) return 1;
+    if (epi->kind == kEpiDropout && (epi->rng == nullptr || N % 16 || ldc != N)) return 1;
     if ((reinterpret_cast<uintptr_t>(p.Z) | reinterpret_cast<uintptr_t>(p.C2) |
          reinterpret_cast<uintptr_t>(p.bias)) & 15)
       return 1;
@@ -394,7 +403,7 @@ int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, 
   if (BN == BN_ && epi->kind == KIND_)                                                  \
     return launch_variant<BN_, ST_, false, epi_backward(KIND_), KIND_>(ta, tb, p, stream);
 #define GEMM_EPIS(BN_, ST_)                                                      \
-  GEMM_EPI(BN_, ST_, kEpiGelu) GEMM_EPI(BN_, ST_, kEpiGeluTanh)                  \
+  GEMM_EPI(BN_, ST_, kEpiGelu) GEMM_EPI(BN_, ST_, kEpiGeluTanh) GEMM_EPI(BN_, ST_, kEpiDropout) \
   GEMM_EPI(BN_, ST_, kEpiGeluBwd) GEMM_EPI(BN_, ST_, kEpiGeluTanhBwd) GEMM_EPI(BN_, ST_, kEpiReluBwd)
     GEMM_EPIS(256, 4)
     GEMM_EPIS(128, 6)

@@ -43,6 +43,9 @@ struct Gemm2Params {
   const void* Z;      // kEpi backward: input (ReLU: output) of the activation, as C in memory
   float* col_part;    // kEpi backward: column sums over 32 rows each, or nullptr
   int c2_sum;         // kEpi forward: C2 includes the bias
+  PhiloxArgs rng;     // kEpiDropout: generator state, what a draw is compared by, factor of kept values
+  uint32_t drop_add4;
+  float drop_scale;
   int wide_store;     // rows of C are 32-byte aligned: the epilogue stores whole sectors
 };
 
@@ -594,6 +597,11 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
   p.Z = epi != nullptr ? epi->z : nullptr;
   p.col_part = epi != nullptr ? epi->col_part : nullptr;
   p.c2_sum = epi != nullptr && epi->c2_sum ? 1 : 0;
+  if (epi != nullptr && epi->rng != nullptr) {
+    p.rng = *epi->rng;
+    p.drop_add4 = (128u - dropout_thr7(epi->p)) * 0x01010101u;
+    p.drop_scale = dropout_scale(epi->p);
+  }
   p.idesc = tc::instr_desc_f16(2 * PBM, BN, bf16 ? 1 : 0, a_mn, b_mn);
   p.splits = workspace != nullptr ? gemm2_splits(M, N, K, BN) : 1;
 
@@ -606,11 +614,12 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
   if (epi != nullptr && epi->kind != kEpiPlain) {
     if (a_mn || b_mn != epi_backward(epi->kind) || p.splits != 1) return 1;
     if (epi_backward(epi->kind) && (reinterpret_cast<uintptr_t>(p.Z) & 15)) return 1;
+    if (epi->kind == kEpiDropout && (epi->rng == nullptr || N % 16 || ldc != N)) return 1;
 #define GEMM2_EPI(BN_, ST_, KIND_)                                                              \
   if (BN == BN_ && epi->kind == KIND_)                                                          \
     return launch_pair_variant<BN_, ST_, kKSub, false, epi_backward(KIND_), KIND_>(ta, tb, p, stream);
 #define GEMM2_EPIS(BN_, ST_)                                                      \
-  GEMM2_EPI(BN_, ST_, kEpiGelu) GEMM2_EPI(BN_, ST_, kEpiGeluTanh)                 \
+  GEMM2_EPI(BN_, ST_, kEpiGelu) GEMM2_EPI(BN_, ST_, kEpiGeluTanh) GEMM2_EPI(BN_, ST_, kEpiDropout) \
   GEMM2_EPI(BN_, ST_, kEpiGeluBwd) GEMM2_EPI(BN_, ST_, kEpiGeluTanhBwd) GEMM2_EPI(BN_, ST_, kEpiReluBwd)
     GEMM2_EPIS(256, 6 / kKSub)
     GEMM2_EPIS(128, 8 / kKSub)

@@ -6,6 +6,8 @@
 
 #include "kernels.h"
 
+slapo::PhiloxArgs unpack_rng(const c10::optional<at::Tensor>& rng);      // bindings.cpp
+
 namespace {
 
 using at::Tensor;
@@ -183,6 +185,20 @@ std::tuple<Tensor, Tensor> gemm_act_fwd(const Tensor& a, const Tensor& w, const 
   return {y, z};
 }
 
+// dropout(a w^T + bias) with the decisions of bias_dropout_add_fwd, more than 16 rows and N % 16 == 0
+Tensor gemm_dropout_fwd(const Tensor& a, const Tensor& w, const c10::optional<Tensor>& bias, double p,
+                        const Tensor& rng) {
+  GemmCall g(a, w, false);
+  TORCH_CHECK(g.N % 16 == 0 && !slapo::gemm_rows_takes(g.M, g.N, g.K), "gemm_dropout_fwd: N % 16 == 0 and more rows");
+  const void* bias_ptr = bias_words(bias, a, g.N);
+  c10::cuda::CUDAGuard guard(a.device());
+  const slapo::PhiloxArgs state = unpack_rng(rng);
+  Tensor y = at::empty({g.M, g.N}, a.options());
+  slapo::GemmEpi epi{6, false, nullptr, nullptr, nullptr, &state, static_cast<float>(p)};
+  g.run(y, bias_ptr, epi);
+  return y;
+}
+
 // dz = (dy w) * act'(z) and its column sums: the input gradient of the layer that follows an
 // activation, on to that activation's input.  z: for ReLU (act 2) the activation's output.  w is the
 // following layer's weight [K, N].
@@ -213,6 +229,7 @@ void register_gemm_ops(torch::Library& m) {
         "Tensor? pre_act, int impl, bool split_k) -> Tensor", &gemm_out);
   m.def("gemm_act_fwd(Tensor a, Tensor w, Tensor? bias, int act, bool keep, bool sum=True) -> (Tensor, Tensor)",
         &gemm_act_fwd);
+  m.def("gemm_dropout_fwd(Tensor a, Tensor w, Tensor? bias, float p, Tensor rng) -> Tensor", &gemm_dropout_fwd);
   m.def("gemm_act_bwd(Tensor dy, Tensor w, Tensor z, int act) -> (Tensor, Tensor)",
         &gemm_act_bwd);
   // which tile a product without split K gets: a CTA pair's or one CTA's, and its columns (0: the widest)

@@ -113,7 +113,7 @@ bool gemm_rows_takes(int M, int N, int K) { return M <= 16 && K >= 64 && N >= 64
 // Returns 0 on success; >0 = refused on the host, as launch_gemm does.
 int launch_gemm_rows(const void* A, const void* W, void* C, const void* bias, int M, int N, int K, int lda,
                      int ldw, int ldc, bool bf16, int act, cudaStream_t stream, const GemmEpi* epi) {
-  if (epi != nullptr && epi_backward(epi->kind)) return 1;
+  if (epi != nullptr && (epi_backward(epi->kind) || epi->kind == kEpiDropout)) return 1;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (M > 16 || N % 8 || K % 8 || lda % 8 || ldw % 8 || ldc % 8) return 1;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(C)) & 15)

@@ -36,7 +36,16 @@ void launch_fused_adamw(void* param, const void* grad, float* master, float* exp
 // Returns 0 on success, >0 when the launch was refused on the host.
 // `epi`: an activation (A and B K-major) or its derivative (B N-major) in the epilogue, as a layer's forward and
 // the following layer's input gradient have them (gemm_epilogue.cuh); `act` is not looked at then.  c2, z: [M, N] with C's row stride.
-struct GemmEpi { int kind; bool c2_sum; void* c2; const void* z; float* col_part; };
+struct PhiloxArgs;
+struct GemmEpi {
+  int kind;
+  bool c2_sum;
+  void* c2;
+  const void* z;
+  float* col_part;
+  const PhiloxArgs* rng = nullptr;      // dropout: generator state and probability
+  float p = 0.f;
+};
 int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
                 int lda, int ldb, int ldc, bool a_mn, bool b_mn, bool bf16, int act, int bn,
                 int* status, cudaStream_t stream, const GemmEpi* epi = nullptr);

@@ -6,6 +6,7 @@ import torch.autograd.forward_ad as fwd
 
 from slapo_b200.op import FusedMLP
 from slapo_b200.ops import functional as NF
+from slapo_b200.ops import native
 
 pytestmark = pytest.mark.gpu
 
@@ -58,3 +59,21 @@ def test_transforms_are_refused():
     w, b = plain[:2]
     with pytest.raises(RuntimeError, match="functorch"):
         torch.vmap(lambda t: NF.linear(x, w, t, "gelu"))(torch.stack([b, b]))
+
+
+@pytest.mark.parametrize("rows,n,k", [(17, 64, 64), (24, 16, 72), (128, 272, 64), (130, 48, 512), (257, 144, 136),
+                                      (300, 1040, 128), (1000, 2064, 256), (2048, 512, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_dropout_in_the_epilogue(rows, n, k, dtype):
+    """To the bit what a product followed by bias and dropout gives, in every tile that a product can get."""
+    torch.manual_seed(rows + n)
+    ops = native.ops()
+    a = torch.randn(rows, k, device="cuda", dtype=dtype)
+    w = (torch.randn(n, k, device="cuda") * k ** -0.5).to(dtype)
+    for bias in (None, torch.randn(n, device="cuda", dtype=dtype)):
+        for p in (0.1, 0.5):
+            rng = ops.philox_reserve(rows * n)
+            got = ops.gemm_dropout_fwd(a, w, bias, p, rng)
+            want = ops.bias_dropout_add_fwd(ops.gemm(a, w, None, -1, False, False), bias, None, p, rng)
+            assert torch.equal(got, want)
+    assert ops.device_status() == 0
