@@ -1073,27 +1073,28 @@ static int round128(int n) { return (n + 127) / 128 * 128; }
 // side the passes fill the waves that each alone would leave partly empty and save a launch; one
 // after the other the dK / dV pass reads the keep bits that the dQ pass drew instead of drawing them
 // again, and each pass has its tensors in L2 to itself.  Weighed as rounds of work items, in tiles
-// of the dQ pass: a tile of dK / dV takes 1.2 of them (D = 128: 1.45; 2 with the relative bias's gradient, 0.3
-// more drawing), an item a quarter more (D = 128: 1.5, its accumulators leave tensor memory without a
-// second set to go on with), a launch 1.5; both in one came out 5 % over that.  Under a causal mask items
+// of the dQ pass: a tile of dK / dV takes 1.4 of them (1.37 for D = 128; with dropout, which costs the dQ pass more,
+// 1.05 and 1.27, and 0.5 more drawing), an item a quarter more (D = 128: one, its dK has no second set of
+// accumulators to go on with), a launch 2; both in one came out a tenth under that.  Under a causal mask items
 // differ and the heaviest go first, so that no whole rounds are lost in two launches or one: side by side
 // up to 5 waves of each.
-// Measured, two launches -> one (us).  Taken side by side: 1 x 512 x 16 x 64: 23.5 -> 17.5; 1 x 2048 x 12 x 64 causal: 83 -> 66; 4 x
-// 256 x 12 x 64, p 0.1: 23.5 -> 16.8; 1 x 512 x 16 x 128: 31 -> 23; 4 x 1024 x 16 x 128: 143 -> 135, causal 113 -> 110;
-// 1 x 2048 x 16 x 128 causal: 110 -> 94.  Not: 4 x 512 x 16 x 64: 38.7 -> 41.8; 32 x 512 x 16 x 64, p 0.1: 253 -> 298,
-// without 203 -> 244, causal 173 -> 236; 4 x 2048 x 16 x 128: 409 -> 436; 32 x 256 x 16 x 128: 113 -> 127.  Of 37 shapes the
-// rule misses the better one by 4 - 6 % in two (2 x 1024 x 16 x 128, p 0.1: 93.4, not 88.5) and by at most 2.5 % in
-// the others.
+// Measured, two launches -> one (us).  Taken side by side: 1 x 512 x 16 x 64: 23.3 -> 15.0; 1 x 2048 x 12 x 64 causal: 86
+// -> 54; 4 x 512 x 16 x 64: 38.5 -> 28.4; 2 x 1024 x 16 x 128, p 0.1: 94 -> 77; 3 x 1820 x 8 x 128 causal, p 0.1: 162 -> 113; 27
+// x 245 x 8 x 64 causal, p 0.1: 44 -> 36; 7 x 1496 x 16 x 64: 331 -> 305; 4 x 1024 x 16 x 128: 122 -> 112; 32 x 256 x 16 x
+// 128: 94 -> 87.  Not: 16 x 512 x 16 x 64, p 0.1: 113 -> 137; 20 x 172 x 32 x 64, p 0.1: 83 -> 89; 19 x 378 x 12 x 64, p 0.1: 1.18
+// times as long; 32 x 493 x 8 x 128, p 0.1: 155 -> 164.  Over 60 shapes, half of them drawn, the rule is 1.6 % over the
+// better of all that was tried (4.1 % with the weights of earlier kernels, 25 % with two launches always), at
+// worst 20 % (12 x 684 x 4 x 80, p 0.1: 80, not 67).
 static int both_q_ctas(int64_t q_items, int64_t k_items, int64_t q_item_tiles, int64_t q_tiles, int D,
                        bool causal, bool rel, bool drop) {
   const int64_t sms = sm_count();
-  const double item = D <= 64 ? 0.25 : 1.5;
-  const double k_tile = rel ? 2.0 : (D <= 64 ? 1.2 : 1.45);
+  const double item = D <= 64 ? 0.25 : 1.0;
+  const double k_tile = rel ? 1.4 : (D <= 64 ? (drop ? 1.05 : 1.4) : (drop ? 1.27 : 1.37));
   const double q_item = q_item_tiles + item, k_item = q_tiles * k_tile + item;
-  const double k_item_draws = q_tiles * (k_tile + (drop ? 0.3 : 0.0)) + item;
+  const double k_item_draws = q_tiles * (k_tile + (drop ? 0.5 : 0.0)) + item;
   if (q_items + k_items <= sms) return static_cast<int>(q_items);
   auto rounds = [](int64_t items, int64_t ctas) { return (items + ctas - 1) / ctas; };
-  double best = (rounds(q_items, sms) * q_item + rounds(k_items, sms) * k_item + 1.5) / 1.05;
+  double best = (rounds(q_items, sms) * q_item + rounds(k_items, sms) * k_item + 2.0) / 0.9;
   if (causal && !drop) best = q_items + k_items > 10 * sms ? 0.0 : 1e30;
   int best_n = 0;
   for (int64_t r = rounds(q_items, sms - 1); r * q_item < best; ++r) {
