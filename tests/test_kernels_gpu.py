@@ -162,3 +162,22 @@ def test_fused_adamw_matches_torch():
         opt.step()
         torch.testing.assert_close(master, ref.data, rtol=1e-4, atol=1e-5)
         torch.testing.assert_close(p.float(), ref.data, rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("n", [8, 2048, 100_008])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_fused_adamw_at_any_16_bytes(n, dtype):
+    """State that starts on 32 bytes and state that does not take different loads: the same bits."""
+    torch.manual_seed(n)
+    grad = torch.randn(n, device="cuda").to(dtype)
+    start = torch.randn(3, n, device="cuda").abs()
+    decay = (torch.arange(n, device="cuda") % 3 == 0).to(torch.uint8)
+    scale = torch.full((1,), 0.5, device="cuda")
+    got = []
+    for offset in (0, 4):
+        state = [torch.empty(n + 8, device="cuda")[offset:offset + n].copy_(x) for x in start]
+        assert all(x.data_ptr() % 32 == 4 * offset for x in state)
+        param = torch.empty(n, device="cuda", dtype=dtype)
+        native.ops().fused_adamw(param, grad, *state, decay, scale, 1e-2, 0.9, 0.95, 1e-8, 0.1, 0.1, 0.05)
+        got.append([param, *state])
+    assert all(torch.equal(a, b) for a, b in zip(*got))
