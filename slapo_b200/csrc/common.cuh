@@ -1,6 +1,7 @@
 // Shared device helpers: 8-wide vector access for bf16/fp16/fp32, warp
 // reductions, Philox4x32-10 with an (optionally device-resident) seed/offset.
 #pragma once
+#include <initializer_list>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -174,6 +175,61 @@ __device__ __forceinline__ void round_through(float v[8]) {
 #pragma unroll
     for (int k = 0; k < 8; ++k) v[k] = static_cast<float>(static_cast<T>(v[k]));
   }
+}
+
+// Sixteen 16-bit values of a thread, on 32 bytes: one access, and all the draws of one Philox call.
+template <typename T>
+__device__ __forceinline__ void load16_raw(const T* p, uint32_t (&w)[8]) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+               : "l"(p));
+}
+template <typename T>
+__device__ __forceinline__ void store16_raw(T* p, const uint32_t (&w)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+               "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
+__device__ __forceinline__ float2 pair_floats(uint32_t w, __nv_bfloat16) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+__device__ __forceinline__ float2 pair_floats(uint32_t w, __half) {
+  return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+__device__ __forceinline__ uint32_t pair_word(float a, float b, __nv_bfloat16) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ uint32_t pair_word(float a, float b, __half) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+template <typename T>
+__device__ __forceinline__ void unpack16(const uint32_t (&w)[8], float (&v)[16]) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float2 f = pair_floats(w[k], T());
+    v[2 * k] = f.x;
+    v[2 * k + 1] = f.y;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void pack16(const float (&v)[16], uint32_t (&w)[8]) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) w[k] = pair_word(v[2 * k], v[2 * k + 1], T());
+}
+// the decisions of one Philox call, in the order of its sixteen elements
+__device__ __forceinline__ void drop16(const uint4& c, float scale, float (&v)[16]) {
+  const uint32_t kw[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[k] = (kw[k >> 2] & (0x80u << (8 * (k & 3)))) ? v[k] * scale : 0.f;
+}
+
+inline bool on_32_bytes(std::initializer_list<const void*> operands) {
+  uintptr_t bits = 0;
+  for (const void* p : operands) bits |= reinterpret_cast<uintptr_t>(p);
+  return bits % 32 == 0;
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

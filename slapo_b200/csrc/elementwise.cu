@@ -85,7 +85,8 @@ __global__ void __launch_bounds__(256) bias_act_fwd_kernel(
 
 // Column-slab layout shared by the backward kernels: a CTA of 8 warps covers
 // 256 columns (lane -> 8 columns) and a chunk of rows (warp w takes rows
-// w, w+8, ...).  Per-thread partial column sums are combined across the 8
+// w, w+8, ...), or, where rows of 16-bit values are whole groups of 16 on 32 bytes, a lane 16 columns and a warp two
+// rows (2 w, 2 w + 1, and so on in steps of 16).  Per-thread partial column sums are combined across the 8
 // warps in shared memory and written to partial[blockIdx.y][col].
 __device__ __forceinline__ void slab_reduce_store(float acc[8], float* partial, int cols,
                                                   int col, bool col_ok) {
@@ -105,6 +106,116 @@ __device__ __forceinline__ void slab_reduce_store(float acc[8], float* partial, 
     }
     Vec8<float>::store(partial + static_cast<int64_t>(blockIdx.y) * cols + col, s);
   }
+}
+
+__device__ __forceinline__ void slab_reduce_store(const float (&acc16)[16], float* partial, int cols, int col0) {
+  __shared__ float red16[8][16 * 17];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    const float v = acc16[k] + __shfl_xor_sync(0xffffffffu, acc16[k], 16);
+    if (lane < 16) red16[warp][k * 17 + lane] = v;
+  }
+  __syncthreads();
+  const int c = threadIdx.x;
+  float t = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) t += red16[w][(c & 15) * 17 + (c >> 4)];
+  if (col0 + c < cols) partial[static_cast<int64_t>(blockIdx.y) * cols + col0 + c] = t;
+}
+
+// 32-byte accesses, and one Philox call per thread and row instead of one in each of two neighbours.  8 columns ->
+// 16 columns per lane, L2 flushed (us):
+//                       GeLU's backward      ReLU's             dropout's
+//   16384 x  4096       96.2 -> 77.4         72.1 -> 66.2       64.9 -> 48.7
+//    8192 x  4096       51.2 -> 42.9         40.0 -> 36.4       34.8 -> 26.2
+//    4096 x 10240       77.3 -> 61.8         56.1 -> 50.2       42.3 -> 36.8
+//    8192 x  1024       17.4 -> 14.8         13.8 -> 12.3       11.6 ->  8.4
+//    4096 x  1024        9.2 -> 10.1          8.7 ->  8.2        7.5 ->  5.8
+//     512 x  2048        4.3 ->  4.6          4.3 ->  4.2        3.6 ->  3.5
+// (GeLU's at 16384 x 4096: 5.2 of 6.5 TB/s).
+template <int kAct, typename T>
+__global__ void __launch_bounds__(256) bias_act_bwd_wide_kernel(
+    const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ bias,
+    T* __restrict__ dx, float* __restrict__ partial, int rows, int cols, int rows_per_chunk) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int col = blockIdx.x * 256 + (lane & 15) * 16;
+  float acc[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) acc[k] = 0.f;
+  if (col < cols) {
+    uint32_t bw[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+    if (bias != nullptr) load16_raw(bias + col, bw);
+    const int r0 = blockIdx.y * rows_per_chunk;
+    const int r1 = min(rows, r0 + rows_per_chunk);
+    constexpr int kRows = 2;  // whose loads are issued before any is used
+    for (int r = r0 + warp * 2 + (lane >> 4); r < r1; r += 16 * kRows) {
+      const int64_t e = static_cast<int64_t>(r) * cols + col;
+      uint32_t gw[kRows][8], vw[kRows][8];
+#pragma unroll
+      for (int u = 0; u < kRows; ++u)
+        if (r + 16 * u < r1) {
+          load16_raw(dy + e + static_cast<int64_t>(16 * u) * cols, gw[u]);
+          load16_raw(x + e + static_cast<int64_t>(16 * u) * cols, vw[u]);
+        }
+#pragma unroll
+      for (int u = 0; u < kRows; ++u)
+        if (r + 16 * u < r1) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            float2 g = pair_floats(gw[u][k], T());
+            const float2 v = pair_floats(vw[u][k], T()), b = pair_floats(bw[k], T());
+            g.x *= act_slope<kAct, T>(v.x + b.x);
+            g.y *= act_slope<kAct, T>(v.y + b.y);
+            acc[2 * k] += g.x;
+            acc[2 * k + 1] += g.y;
+            gw[u][k] = pair_word(g.x, g.y, T());
+          }
+          store16_raw(dx + e + static_cast<int64_t>(16 * u) * cols, gw[u]);
+        }
+    }
+  }
+  if (partial != nullptr) slab_reduce_store(acc, partial, cols, blockIdx.x * 256);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) bias_dropout_add_bwd_wide_kernel(
+    const T* __restrict__ dy, T* __restrict__ dx, float* __restrict__ partial, int rows,
+    int cols, int rows_per_chunk, float p, PhiloxArgs rng) {
+  uint64_t seed, offset;
+  philox_unpack(rng, seed, offset);
+  const float scale = dropout_scale(p);
+  const uint32_t add4 = (128u - dropout_thr7(p)) * 0x01010101u;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int col = blockIdx.x * 256 + (lane & 15) * 16;
+  float acc[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) acc[k] = 0.f;
+  if (col < cols) {
+    const int r0 = blockIdx.y * rows_per_chunk;
+    const int r1 = min(rows, r0 + rows_per_chunk);
+    constexpr int kRows = 2;
+    for (int r = r0 + warp * 2 + (lane >> 4); r < r1; r += 16 * kRows) {
+      const int64_t e0 = static_cast<int64_t>(r) * cols + col;
+      uint32_t w[kRows][8];
+#pragma unroll
+      for (int u = 0; u < kRows; ++u)
+        if (r + 16 * u < r1) load16_raw(dy + e0 + static_cast<int64_t>(16 * u) * cols, w[u]);
+#pragma unroll
+      for (int u = 0; u < kRows; ++u)
+        if (r + 16 * u < r1) {
+          const int64_t e = e0 + static_cast<int64_t>(16 * u) * cols;
+          float g[16];
+          unpack16<T>(w[u], g);
+          drop16(philox_keep16(seed, offset, static_cast<uint64_t>(e) >> 4, add4), scale, g);
+#pragma unroll
+          for (int k = 0; k < 16; ++k) acc[k] += g[k];
+          pack16<T>(g, w[u]);
+          store16_raw(dx + e, w[u]);
+        }
+    }
+  }
+  if (partial != nullptr) slab_reduce_store(acc, partial, cols, blockIdx.x * 256);
 }
 
 template <int kAct, typename T>
@@ -333,6 +444,22 @@ int colsum_chunks(int rows, int cols) {
     default: { using T = float; __VA_ARGS__; break; }                \
   }
 
+#define DISPATCH_16BIT(dtype, ...)                                   \
+  switch (dtype) {                                                   \
+    case 0: { using T = __nv_bfloat16; __VA_ARGS__; break; }         \
+    default: { using T = __half; __VA_ARGS__; break; }               \
+  }
+// The kernels with 16 columns per lane hold more registers and take longer over the sums at a CTA's end, so they run
+// with half of the CTAs and from `least` values on.  (Summing alone, without a store, gained under 6 % and is not
+// done that way.)
+static bool slab_wide(int rows, int cols, int dtype, int64_t least) {
+  return dtype < 2 && cols % 16 == 0 && static_cast<int64_t>(rows) * cols >= least;
+}
+static int slab_chunks(int rows, int cols, bool wide) {
+  const int chunks = colsum_chunks(rows, cols);
+  return wide ? (chunks + 1) / 2 : chunks;
+}
+
 #define DISPATCH_ACT(act, ...)                                       \
   switch (act) {                                                     \
     case 0: { constexpr int kAct = 0; __VA_ARGS__; break; }          \
@@ -361,14 +488,21 @@ void launch_bias_act_bwd(const void* dy, const void* x, const void* bias, void* 
                          float* partial, int rows, int cols, int act, int dtype,
                          cudaStream_t stream) {
   if (rows == 0) return;
-  const int chunks = colsum_chunks(rows, cols);
+  const bool wide = slab_wide(rows, cols, dtype, 8 << 20) && on_32_bytes({dy, x, bias, dx});
+  const int chunks = slab_chunks(rows, cols, wide);
   const int rows_per_chunk = (rows + chunks - 1) / chunks;
   dim3 grid((cols + 255) / 256, chunks);
   float* part = dbias != nullptr ? partial : nullptr;
   count_launch();
-  DISPATCH_DTYPE(dtype, DISPATCH_ACT(act, (bias_act_bwd_kernel<kAct, T><<<grid, 256, 0, stream>>>(
-      static_cast<const T*>(dy), static_cast<const T*>(x), static_cast<const T*>(bias),
-      static_cast<T*>(dx), part, rows, cols, rows_per_chunk))));
+  if (wide) {
+    DISPATCH_16BIT(dtype, DISPATCH_ACT(act, (bias_act_bwd_wide_kernel<kAct, T><<<grid, 256, 0, stream>>>(
+        static_cast<const T*>(dy), static_cast<const T*>(x), static_cast<const T*>(bias),
+        static_cast<T*>(dx), part, rows, cols, rows_per_chunk))));
+  } else {
+    DISPATCH_DTYPE(dtype, DISPATCH_ACT(act, (bias_act_bwd_kernel<kAct, T><<<grid, 256, 0, stream>>>(
+        static_cast<const T*>(dy), static_cast<const T*>(x), static_cast<const T*>(bias),
+        static_cast<T*>(dx), part, rows, cols, rows_per_chunk))));
+  }
   if (dbias != nullptr) launch_colsum_finalize(partial, dbias, chunks, cols, dtype, stream);
 }
 
@@ -399,13 +533,19 @@ void launch_bias_dropout_add_bwd(const void* dy, void* dx, void* dbias, float* p
                                  int cols, float p, PhiloxArgs rng, int dtype,
                                  cudaStream_t stream) {
   if (rows == 0) return;
-  const int chunks = colsum_chunks(rows, cols);
+  const bool wide = slab_wide(rows, cols, dtype, 2 << 20) && on_32_bytes({dy, dx});
+  const int chunks = slab_chunks(rows, cols, wide);
   const int rows_per_chunk = (rows + chunks - 1) / chunks;
   dim3 grid((cols + 255) / 256, chunks);
   float* part = dbias != nullptr ? partial : nullptr;
   count_launch();
-  DISPATCH_DTYPE(dtype, (bias_dropout_add_bwd_kernel<T><<<grid, 256, 0, stream>>>(
-      static_cast<const T*>(dy), static_cast<T*>(dx), part, rows, cols, rows_per_chunk, p, rng)));
+  if (wide) {
+    DISPATCH_16BIT(dtype, (bias_dropout_add_bwd_wide_kernel<T><<<grid, 256, 0, stream>>>(
+        static_cast<const T*>(dy), static_cast<T*>(dx), part, rows, cols, rows_per_chunk, p, rng)));
+  } else {
+    DISPATCH_DTYPE(dtype, (bias_dropout_add_bwd_kernel<T><<<grid, 256, 0, stream>>>(
+        static_cast<const T*>(dy), static_cast<T*>(dx), part, rows, cols, rows_per_chunk, p, rng)));
+  }
   if (dbias != nullptr) launch_colsum_finalize(partial, dbias, chunks, cols, dtype, stream);
 }
 

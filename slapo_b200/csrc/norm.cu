@@ -8,8 +8,6 @@
 // beta / bias gradients are accumulated in registers over all rows a CTA
 // visits, written once per CTA to an fp32 scratch [grid, 3, cols] and summed
 // by a small second kernel.
-#include <initializer_list>
-
 #include "common.cuh"
 #include "kernels.h"
 
@@ -160,54 +158,6 @@ __global__ void __launch_bounds__(32 * WPR * RG, (VPL == 1 && WPR * RG == 16) ? 
       }
     }
   }
-}
-
-template <typename T>
-__device__ __forceinline__ void load16_raw(const T* p, uint32_t (&w)[8]) {
-  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
-               : "l"(p));
-}
-template <typename T>
-__device__ __forceinline__ void store16_raw(T* p, const uint32_t (&w)[8]) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
-               "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-               : "memory");
-}
-__device__ __forceinline__ float2 pair_floats(uint32_t w, __nv_bfloat16) {
-  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-}
-__device__ __forceinline__ float2 pair_floats(uint32_t w, __half) {
-  return __half22float2(*reinterpret_cast<const __half2*>(&w));
-}
-__device__ __forceinline__ uint32_t pair_word(float a, float b, __nv_bfloat16) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-__device__ __forceinline__ uint32_t pair_word(float a, float b, __half) {
-  const __half2 h = __floats2half2_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-template <typename T>
-__device__ __forceinline__ void unpack16(const uint32_t (&w)[8], float (&v)[16]) {
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const float2 f = pair_floats(w[k], T());
-    v[2 * k] = f.x;
-    v[2 * k + 1] = f.y;
-  }
-}
-template <typename T>
-__device__ __forceinline__ void pack16(const float (&v)[16], uint32_t (&w)[8]) {
-#pragma unroll
-  for (int k = 0; k < 8; ++k) w[k] = pair_word(v[2 * k], v[2 * k + 1], T());
-}
-// the decisions of one Philox call, in the order of its sixteen elements
-__device__ __forceinline__ void drop16(const uint4& c, float scale, float (&v)[16]) {
-  const uint32_t kw[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-  for (int k = 0; k < 16; ++k) v[k] = (kw[k >> 2] & (0x80u << (8 * (k & 3)))) ? v[k] * scale : 0.f;
 }
 
 // The forward for 16-bit rows of 16 values per thread: a 32-byte access and one Philox call for all of them (the
@@ -657,11 +607,6 @@ static int ln_grid(int rows, int cols, int ctas_per_sm) {
 
 // The kernels with 16 values per thread: which rows they take (16-bit, whole groups of 16 values on 32 bytes).
 static bool rows_shape(int cols, int dtype) { return dtype < 2 && cols > 256 && cols <= 4096 && cols % 16 == 0; }
-static bool wide_rows(std::initializer_list<const void*> operands) {
-  uintptr_t bits = 0;
-  for (const void* p : operands) bits |= reinterpret_cast<uintptr_t>(p);
-  return bits % 32 == 0;
-}
 static int rows_wpr(int cols) { return cols <= 512 ? 1 : cols <= 1024 ? 2 : cols <= 2048 ? 4 : 8; }
 // (the figures are at ln_bwd_rows_kernel)
 static bool rows_bwd_pays(int rows, int cols) { return cols > 1024 || rows >= (cols > 512 ? 6000 : 4096); }
@@ -726,7 +671,7 @@ void launch_ln_fwd(const void* x, const void* bias, const void* residual, const 
                    int cols, float eps, float p, PhiloxArgs rng, int rms, int dtype,
                    cudaStream_t stream) {
   if (rows == 0) return;
-  if (rows_shape(cols, dtype) && wide_rows({x, bias, residual, gamma, beta, y, z})) {
+  if (rows_shape(cols, dtype) && on_32_bytes({x, bias, residual, gamma, beta, y, z})) {
     const int grid = rows_grid(rows, cols);
     count_launch();
     ROWS_SWITCH(dtype, cols, p, (ln_fwd_rows_kernel<T, WPR, kDrop><<<grid, 256, 0, stream>>>(
@@ -753,7 +698,7 @@ void launch_ln_bwd(const void* gy, const void* gz, const void* zin, const void* 
   const int want_dbias = dbias != nullptr;
   int grid;
   count_launch(2);
-  if (rows_shape(cols, dtype) && rows_bwd_pays(rows, cols) && wide_rows({gy, gz, zin, gamma, dx, dres})) {
+  if (rows_shape(cols, dtype) && rows_bwd_pays(rows, cols) && on_32_bytes({gy, gz, zin, gamma, dx, dres})) {
     grid = rows_grid(rows, cols);
     ROWS_SWITCH(dtype, cols, p, (ln_bwd_rows_kernel<T, WPR, kDrop><<<grid, 256, 0, stream>>>(
         static_cast<const T*>(gy), static_cast<const T*>(gz), static_cast<const T*>(zin),

@@ -181,3 +181,29 @@ def test_fused_adamw_at_any_16_bytes(n, dtype):
         native.ops().fused_adamw(param, grad, *state, decay, scale, 1e-2, 0.9, 0.95, 1e-8, 0.1, 0.1, 0.05)
         got.append([param, *state])
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("rows,cols", [(8193, 1040), (20000, 432), (530000, 16), (2048, 1024), (300, 30528)])
+@pytest.mark.parametrize("act", [0, 1, 2, None])
+def test_sixteen_columns_per_lane_backward(rows, cols, act):
+    """The kernels for large 16-bit gradients against the general ones, which take the same call with operands
+    that start on 16 bytes only: the same values to the bit, the same column sums up to their order."""
+    from slapo_b200.ops import native
+
+    ops = native.ops()
+    torch.manual_seed(rows)
+    dy, x = (torch.randn(rows, cols, device="cuda").bfloat16() for _ in range(2))
+    bias = torch.randn(cols, device="cuda").bfloat16()
+    room = torch.empty(rows * cols + 8, device="cuda", dtype=dy.dtype)
+    off = room[8:].view(rows, cols).copy_(dy)
+    rng = torch.tensor([5, 4, 0, 0], dtype=torch.int64)
+
+    def run(g):
+        return ops.bias_dropout_add_bwd(g, 0.1, rng, True) if act is None else ops.bias_act_bwd(g, x, bias, act)
+
+    wide, slim, again = run(dy), run(off), run(dy)
+    assert torch.equal(wide[0], slim[0])
+    # fp32 sums of `rows` values in two orders, rounded once to 16 bits
+    err = 2 ** -24 * rows * float(wide[0].float().abs().max())
+    torch.testing.assert_close(wide[1].float(), slim[1].float(), rtol=2 ** -7, atol=err)
+    assert torch.equal(again[1], wide[1])

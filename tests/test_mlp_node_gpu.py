@@ -61,8 +61,8 @@ def test_transforms_are_refused():
         torch.vmap(lambda t: NF.linear(x, w, t, "gelu"))(torch.stack([b, b]))
 
 
-@pytest.mark.parametrize("rows,n,k", [(17, 64, 64), (24, 16, 72), (128, 272, 64), (130, 48, 512), (257, 144, 136),
-                                      (300, 1040, 128), (1000, 2064, 256), (2048, 512, 64)])
+@pytest.mark.parametrize("rows,n,k", [(17, 64, 64), (24, 16, 72), (128, 272, 64), (130, 48, 512),
+                                      (257, 144, 136), (300, 1040, 128), (1000, 2064, 256), (2048, 512, 64)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_dropout_in_the_epilogue(rows, n, k, dtype):
     """To the bit what a product followed by bias and dropout gives, in every tile that a product can get."""

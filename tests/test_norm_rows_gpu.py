@@ -1,6 +1,7 @@
-"""Normalisation of 16-bit rows with 16 values per thread, against the general kernel (which takes the same call with a
-weight that starts on 16 bytes only) and against 64 bits: every number of warps per row, its last column group, fewer
-rows than groups, a ragged last step, and the numbers of rows from which the backward takes the new form."""
+"""Normalisation of 16-bit rows with 16 values per thread, against the general kernel (which takes the same
+call with a weight that starts on 16 bytes only) and against 64 bits: every number of warps per row, its last
+column group, fewer rows than groups, a ragged last step, and the numbers of rows from which the backward
+takes the new form."""
 import pytest
 import torch
 
