@@ -15,7 +15,7 @@
 //              the pair complete their bytes on it
 //   empty[s]   in each CTA; the leader's MMA thread commits to both after the MMAs of a stage
 //   tmem_full[a]   in each CTA; committed to both when a tile's accumulator is complete
-//   tmem_empty[a]  in the leader; the eight epilogue warps of the pair arrive on it
+//   tmem_empty[a]  in the leader; the epilogue warps of both CTAs arrive on it
 //
 // Split-K (few output tiles, long contraction - weight gradients): `splits` CTA pairs share
 // a tile, each stores its partial accumulator into its own fp32 slice of a workspace; a

@@ -199,7 +199,9 @@ def test_sixteen_columns_per_lane_backward(rows, cols, act):
     rng = torch.tensor([5, 4, 0, 0], dtype=torch.int64)
 
     def run(g):
-        return ops.bias_dropout_add_bwd(g, 0.1, rng, True) if act is None else ops.bias_act_bwd(g, x, bias, act)
+        if act is None:
+            return ops.bias_dropout_add_bwd(g, 0.1, rng, True)
+        return ops.bias_act_bwd(g, x, bias, act)
 
     wide, slim, again = run(dy), run(off), run(dy)
     assert torch.equal(wide[0], slim[0])
