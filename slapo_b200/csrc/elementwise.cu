@@ -129,7 +129,7 @@ __device__ __forceinline__ void slab_reduce_store(const float (&acc16)[16], floa
 //                       GeLU's backward      ReLU's             dropout's
 //   16384 x  4096       96.2 -> 77.4         72.1 -> 66.2       64.9 -> 48.7
 //    8192 x  4096       51.2 -> 42.9         40.0 -> 36.4       34.8 -> 26.2
-//    4096 x 10240       77.3 -> 61.8         56.1 -> 50.2       42.3 -> 36.8
+//    4096 x 10240       77.3 -> 52.5         56.1 -> 44.1       42.3 -> 30.6
 //    8192 x  1024       17.4 -> 14.8         13.8 -> 12.3       11.6 ->  8.4
 //    4096 x  1024        9.2 -> 10.1          8.7 ->  8.2        7.5 ->  5.8
 //     512 x  2048        4.3 ->  4.6          4.3 ->  4.2        3.6 ->  3.5
@@ -430,7 +430,9 @@ static inline int flat_grid(int64_t n_vec) {
 
 int colsum_chunks(int rows, int cols) {
   const int slabs = (cols + 255) / 256;
-  int chunks = (sm_count() * 8 + slabs - 1) / slabs;
+  // eight CTAs per SM at most, which is one wave of `colsum_kernel` and two of the others: one CTA more waits for
+  // a wave of its own (8192 x 30528, sums alone: 1200 CTAs 109 us, 1080 CTAs 96; 8192 x 2560 12.4 -> 11.3)
+  int chunks = sm_count() * 8 / slabs;
   const int max_chunks = (rows + 7) / 8;
   if (chunks > max_chunks) chunks = max_chunks;
   if (chunks < 1) chunks = 1;
@@ -450,14 +452,24 @@ int colsum_chunks(int rows, int cols) {
     default: { using T = __half; __VA_ARGS__; break; }               \
   }
 // The kernels with 16 columns per lane hold more registers and take longer over the sums at a CTA's end, so they run
-// with half of the CTAs and from `least` values on.  (Summing alone, without a store, gained under 6 % and is not
+// with fewer CTAs and from `least` values on.  (Summing alone, without a store, gained under 6 % and is not
 // done that way.)
 static bool slab_wide(int rows, int cols, int dtype, int64_t least) {
   return dtype < 2 && cols % 16 == 0 && static_cast<int64_t>(rows) * cols >= least;
 }
-static int slab_chunks(int rows, int cols, bool wide) {
+// Row chunks of theirs, half of the general kernels' to all of them: the number with which waves of `per_sm` CTAs times
+// the rows of a CTA, and some 16 rows' time for its sums, is least.  Against half of them: GeLU's backward 4096 x 10240
+// 62.1 -> 52.5 us, 8192 x 30528 329 -> 274, 16384 x 4096 77.2 -> 77.4; dropout's 36.7 -> 30.6, 203 -> 163, 48.4 -> 48.8.
+static int slab_chunks(int rows, int cols, int per_sm) {
   const int chunks = colsum_chunks(rows, cols);
-  return wide ? (chunks + 1) / 2 : chunks;
+  const int64_t slabs = (cols + 255) / 256, resident = static_cast<int64_t>(sm_count()) * per_sm;
+  int best = chunks;
+  int64_t least = -1;
+  for (int c = (chunks + 1) / 2; c <= chunks; ++c) {
+    const int64_t time = (c * slabs + resident - 1) / resident * ((rows + c - 1) / c + 16);
+    if (least < 0 || time < least) { least = time; best = c; }
+  }
+  return best;
 }
 
 #define DISPATCH_ACT(act, ...)                                       \
@@ -489,7 +501,7 @@ void launch_bias_act_bwd(const void* dy, const void* x, const void* bias, void* 
                          cudaStream_t stream) {
   if (rows == 0) return;
   const bool wide = slab_wide(rows, cols, dtype, 8 << 20) && on_32_bytes({dy, x, bias, dx});
-  const int chunks = slab_chunks(rows, cols, wide);
+  const int chunks = wide ? slab_chunks(rows, cols, 2) : colsum_chunks(rows, cols);
   const int rows_per_chunk = (rows + chunks - 1) / chunks;
   dim3 grid((cols + 255) / 256, chunks);
   float* part = dbias != nullptr ? partial : nullptr;
@@ -534,7 +546,7 @@ void launch_bias_dropout_add_bwd(const void* dy, void* dx, void* dbias, float* p
                                  cudaStream_t stream) {
   if (rows == 0) return;
   const bool wide = slab_wide(rows, cols, dtype, 2 << 20) && on_32_bytes({dy, dx});
-  const int chunks = slab_chunks(rows, cols, wide);
+  const int chunks = wide ? slab_chunks(rows, cols, 4) : colsum_chunks(rows, cols);
   const int rows_per_chunk = (rows + chunks - 1) / chunks;
   dim3 grid((cols + 255) / 256, chunks);
   float* part = dbias != nullptr ? partial : nullptr;

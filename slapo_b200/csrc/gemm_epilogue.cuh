@@ -12,15 +12,15 @@
 // memory that it replaces), with eight epilogue warps per CTA: 16384 x 4096, K = 1024     4096 x 10240, K = 2560
 //   GeLU                                               105 / 108 / 62             136 / 137 / 42
 //   GeLU, the product kept                             105 / 117 / 62             136 / 142 / 42
-//   GeLU's derivative and column sums                   95 / 148 / 77             138 / 157 / 62
-//   ReLU's                                              95 / 130 / 66             138 / 161 / 50
+//   GeLU's derivative and column sums                   95 / 148 / 77             138 / 157 / 53
+//   ReLU's                                              95 / 130 / 66             138 / 161 / 44
 // (with the sixteen that GeLU has now: gemm2.cu at kManyEpiWarpsK)
 // Dropout (kEpiDropout): C = dropout(product + bias), again to the bit what a product and a kernel behind it give:
 // the product is rounded first, and an element's decision is that of its index in C (16 to a Philox call, two calls
 // for 32 columns; N % 16 == 0).  16384 x 1024, K = 4096: 92.3 -> 92.0 us, and a
 // pass of 20 less; a whole feed-forward block of 8192 x 512 204 -> 187.
 // So the forward is all but hidden, while the derivative's epilogue is what bounds a product with K = 1024:
-// of the pass of 77 us it saves 24, at K = 2560 43 of 62.
+// of the pass of 77 us it saves 24, at K = 2560 34 of 53.
 #pragma once
 #include "common.cuh"
 
