@@ -428,15 +428,22 @@ static inline int flat_grid(int64_t n_vec) {
   return static_cast<int>(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
+// most row chunks that any of the kernels below uses: what their scratch holds
 int colsum_chunks(int rows, int cols) {
   const int slabs = (cols + 255) / 256;
-  // eight CTAs per SM at most, which is one wave of `colsum_kernel` and two of the others: one CTA more waits for
-  // a wave of its own (8192 x 30528, sums alone: 1200 CTAs 109 us, 1080 CTAs 96; 8192 x 2560 12.4 -> 11.3)
-  int chunks = sm_count() * 8 / slabs;
+  int chunks = (sm_count() * 8 + slabs - 1) / slabs;
   const int max_chunks = (rows + 7) / 8;
   if (chunks > max_chunks) chunks = max_chunks;
   if (chunks < 1) chunks = 1;
   return chunks;
+}
+
+// Row chunks of a launch: eight CTAs per SM at most, which is one wave of `colsum_kernel` and two of the others.  One
+// CTA more waits for a wave of its own (8192 x 30528, sums alone: 1200 CTAs 109 us, 1080 CTAs 96; 8192 x 2560
+// 12.4 -> 11.3).
+static int wave_chunks(int rows, int cols) {
+  const int most = colsum_chunks(rows, cols), fit = sm_count() * 8 / ((cols + 255) / 256);
+  return fit < 1 ? 1 : (fit < most ? fit : most);
 }
 
 #define DISPATCH_DTYPE(dtype, ...)                                   \
@@ -461,7 +468,7 @@ static bool slab_wide(int rows, int cols, int dtype, int64_t least) {
 // the rows of a CTA, and some 16 rows' time for its sums, is least.  Against half of them: GeLU's backward 4096 x 10240
 // 62.1 -> 52.5 us, 8192 x 30528 329 -> 274, 16384 x 4096 77.2 -> 77.4; dropout's 36.7 -> 30.6, 203 -> 163, 48.4 -> 48.8.
 static int slab_chunks(int rows, int cols, int per_sm) {
-  const int chunks = colsum_chunks(rows, cols);
+  const int chunks = wave_chunks(rows, cols);
   const int64_t slabs = (cols + 255) / 256, resident = static_cast<int64_t>(sm_count()) * per_sm;
   int best = chunks;
   int64_t least = -1;
@@ -501,7 +508,7 @@ void launch_bias_act_bwd(const void* dy, const void* x, const void* bias, void* 
                          cudaStream_t stream) {
   if (rows == 0) return;
   const bool wide = slab_wide(rows, cols, dtype, 8 << 20) && on_32_bytes({dy, x, bias, dx});
-  const int chunks = wide ? slab_chunks(rows, cols, 2) : colsum_chunks(rows, cols);
+  const int chunks = wide ? slab_chunks(rows, cols, 2) : wave_chunks(rows, cols);
   const int rows_per_chunk = (rows + chunks - 1) / chunks;
   dim3 grid((cols + 255) / 256, chunks);
   float* part = dbias != nullptr ? partial : nullptr;
@@ -521,7 +528,7 @@ void launch_bias_act_bwd(const void* dy, const void* x, const void* bias, void* 
 void launch_colsum(const void* x, void* out, float* partial, int rows, int cols,
                    int64_t row_stride, int dtype, cudaStream_t stream) {
   if (rows == 0 || cols == 0) return;
-  const int chunks = colsum_chunks(rows, cols);
+  const int chunks = wave_chunks(rows, cols);
   const int rows_per_chunk = (rows + chunks - 1) / chunks;
   dim3 grid((cols + 255) / 256, chunks);
   count_launch();
@@ -546,7 +553,7 @@ void launch_bias_dropout_add_bwd(const void* dy, void* dx, void* dbias, float* p
                                  cudaStream_t stream) {
   if (rows == 0) return;
   const bool wide = slab_wide(rows, cols, dtype, 2 << 20) && on_32_bytes({dy, dx});
-  const int chunks = wide ? slab_chunks(rows, cols, 4) : colsum_chunks(rows, cols);
+  const int chunks = wide ? slab_chunks(rows, cols, 4) : wave_chunks(rows, cols);
   const int rows_per_chunk = (rows + chunks - 1) / chunks;
   dim3 grid((cols + 255) / 256, chunks);
   float* part = dbias != nullptr ? partial : nullptr;
