@@ -90,9 +90,6 @@ struct GemmParams {
   const void* Z;      // kEpi backward: input (ReLU: output) of the activation, as C in memory
   float* col_part;    // kEpi backward: column sums over 32 rows each, or nullptr
   int c2_sum;         // kEpi forward: C2 includes the bias
-  PhiloxArgs rng;     // kEpiDropout: generator state, what a draw is compared by, factor of kept values
-  uint32_t drop_add4;
-  float drop_scale;
 };
 
 constexpr int BM = 128;
@@ -124,7 +121,7 @@ __device__ __forceinline__ float load_bias(const void* bias, int col, int out_bf
 template <int BN, int STAGES, bool A_MN, bool B_MN, int kEpi>
 __global__ void __launch_bounds__(192, 1)
 gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                 const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+                 const __grid_constant__ CUtensorMap tmap_b, const EpiParams<GemmParams, kEpi> p) {
   using S = GemmSmem<BN, STAGES>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
@@ -343,7 +340,7 @@ bool cached_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t
 }
 
 template <int BN, int STAGES, bool A_MN, bool B_MN, int kEpi = kEpiPlain>
-static int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
+static int launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const EpiParams<GemmParams, kEpi>& p,
                           cudaStream_t stream) {
   using S = GemmSmem<BN, STAGES>;
   auto kernel = gemm_tc05_kernel<BN, STAGES, A_MN, B_MN, kEpi>;
@@ -380,7 +377,7 @@ int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, 
   if (!ok) return 2;
   ok = b_mn ? cached_tmap_2d(&tb, B, N, K, ldb, BK, bf16) : cached_tmap_2d(&tb, B, K, N, ldb, BN, bf16);
   if (!ok) return 2;
-  GemmParams p;
+  DropParams<GemmParams> p;
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.bias = bias; p.act = act;
   p.out_bf16 = bf16 ? 1 : 0; p.status = status;
   p.idesc = tc::instr_desc_f16(BM, BN, bf16 ? 1 : 0, a_mn, b_mn);
@@ -388,11 +385,7 @@ int launch_gemm(const void* A, const void* B, void* C, const void* bias, int M, 
   p.Z = epi != nullptr ? epi->z : nullptr;
   p.col_part = epi != nullptr ? epi->col_part : nullptr;
   p.c2_sum = epi != nullptr && epi->c2_sum ? 1 : 0;
-  if (epi != nullptr && epi->rng != nullptr) {
-    p.rng = *epi->rng;
-    p.drop_add4 = (128u - dropout_thr7(epi->p)) * 0x01010101u;
-    p.drop_scale = dropout_scale(epi->p);
-  }
+  if (epi != nullptr && epi->rng != nullptr) p.set(*epi);
   if (epi != nullptr && epi->kind != kEpiPlain) {
     if (a_mn || b_mn != epi_backward(epi->kind)) return 1;
     if (epi->kind == kEpiDropout && (epi->rng == nullptr || N % 16 || ldc != N)) return 1;

@@ -43,9 +43,6 @@ struct Gemm2Params {
   const void* Z;      // kEpi backward: input (ReLU: output) of the activation, as C in memory
   float* col_part;    // kEpi backward: column sums over 32 rows each, or nullptr
   int c2_sum;         // kEpi forward: C2 includes the bias
-  PhiloxArgs rng;     // kEpiDropout: generator state, what a draw is compared by, factor of kept values
-  uint32_t drop_add4;
-  float drop_scale;
   int wide_store;     // rows of C are 32-byte aligned: the epilogue stores whole sectors
 };
 
@@ -177,7 +174,7 @@ __device__ __forceinline__ void tile_at(int tile, int tiles_m, int tiles_n, int&
 template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN, int kEpi, int kEpiWarps>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * kEpiWarps, 1)
 gemm2_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                  const __grid_constant__ CUtensorMap tmap_b, const Gemm2Params p) {
+                  const __grid_constant__ CUtensorMap tmap_b, const EpiParams<Gemm2Params, kEpi> p) {
   using S = Gemm2Smem<BN, STAGES, KSUB>;
   constexpr int HBN = BN / 2;   // rows of B per CTA
   extern __shared__ uint8_t smem_raw[];
@@ -477,7 +474,7 @@ bool cached_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t
                     uint64_t stride, uint32_t box_outer, bool bf16);
 
 template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN, int kEpi, int kEpiWarps>
-static int launch_pair_warps(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm2Params& p,
+static int launch_pair_warps(const CUtensorMap& ta, const CUtensorMap& tb, const EpiParams<Gemm2Params, kEpi>& p,
                                cudaStream_t stream) {
   using S = Gemm2Smem<BN, STAGES, KSUB>;
   auto kernel = gemm2_tc05_kernel<BN, STAGES, KSUB, A_MN, B_MN, kEpi, kEpiWarps>;
@@ -504,7 +501,7 @@ static int launch_pair_warps(const CUtensorMap& ta, const CUtensorMap& tb, const
 }
 
 template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN, int kEpi = kEpiPlain>
-static int launch_pair_variant(const CUtensorMap& ta, const CUtensorMap& tb, const Gemm2Params& p,
+static int launch_pair_variant(const CUtensorMap& ta, const CUtensorMap& tb, const EpiParams<Gemm2Params, kEpi>& p,
                                cudaStream_t stream) {
   if constexpr (kEpi != kEpiPlain) {
     return launch_pair_warps<BN, STAGES, KSUB, A_MN, B_MN, kEpi, epi_warps(kEpi)>(ta, tb, p, stream);
@@ -590,18 +587,14 @@ int launch_gemm2(const void* A, const void* B, void* C, void* C2, const void* bi
   ok = b_mn ? cached_tmap_2d(&tb, B, N, K, ldb, PBK, bf16)
             : cached_tmap_2d(&tb, B, K, N, ldb, BN / 2, bf16);
   if (!ok) return 2;
-  Gemm2Params p;
+  DropParams<Gemm2Params> p;
   p.M = M; p.N = N; p.K = K; p.C = C; p.C2 = C2; p.ldc = ldc; p.bias = bias; p.act = act;
   p.out_bf16 = bf16 ? 1 : 0; p.status = status;
   p.wide_store = (ldc % 16 == 0 && ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(C2)) & 31) == 0) ? 1 : 0;
   p.Z = epi != nullptr ? epi->z : nullptr;
   p.col_part = epi != nullptr ? epi->col_part : nullptr;
   p.c2_sum = epi != nullptr && epi->c2_sum ? 1 : 0;
-  if (epi != nullptr && epi->rng != nullptr) {
-    p.rng = *epi->rng;
-    p.drop_add4 = (128u - dropout_thr7(epi->p)) * 0x01010101u;
-    p.drop_scale = dropout_scale(epi->p);
-  }
+  if (epi != nullptr && epi->rng != nullptr) p.set(*epi);
   p.idesc = tc::instr_desc_f16(2 * PBM, BN, bf16 ? 1 : 0, a_mn, b_mn);
   p.splits = workspace != nullptr ? gemm2_splits(M, N, K, BN) : 1;
 

@@ -22,7 +22,9 @@
 // So the forward is all but hidden, while the derivative's epilogue is what bounds a product with K = 1024:
 // of the pass of 77 us it saves 24, at K = 2560 34 of 53.
 #pragma once
+#include <type_traits>
 #include "common.cuh"
+#include "kernels.h"
 
 namespace slapo {
 
@@ -30,6 +32,23 @@ enum GemmEpiKind {
   kEpiPlain = 0, kEpiGelu = 1, kEpiGeluTanh = 2, kEpiGeluBwd = 3, kEpiGeluTanhBwd = 4, kEpiReluBwd = 5, kEpiDropout = 6
 };
 constexpr bool epi_backward(int kind) { return kind >= kEpiGeluBwd && kind <= kEpiReluBwd; }
+
+// Dropout's parameters, in that kernel's alone: with them among those of all, the plain kernel of gemm.cu was compiled
+// to 64 registers instead of 80 and its tiles of 64 columns took 0.6 - 0.9 us longer (M x N x K, operands in L2:
+// 200 x 2048 x 512 6.4 -> 7.3 us, 24 x 512 x 2048 4.6 -> 5.4).
+template <typename P>
+struct DropParams : P {
+  PhiloxArgs rng;         // generator state
+  uint32_t drop_add4;     // what a draw is compared by
+  float drop_scale;       // factor of kept values
+  void set(const GemmEpi& epi) {
+    rng = *epi.rng;
+    drop_add4 = (128u - dropout_thr7(epi.p)) * 0x01010101u;
+    drop_scale = dropout_scale(epi.p);
+  }
+};
+template <typename P, int kEpi>
+using EpiParams = std::conditional_t<kEpi == kEpiDropout, DropParams<P>, P>;
 
 template <int kEpi>
 __device__ __forceinline__ float epi_value(float x) {
