@@ -48,14 +48,21 @@ struct Gemm2Params {
 
 // Epilogue warps per CTA: two per quarter of the tensor-memory lanes, each taking half of the tile's columns, or
 // four with a quarter of them each.  Sixteen warps drain a tile faster (their reads of tensor memory and stores
-// wait side by side), which counts where the epilogue is what a tile takes: a GeLU in it, or a short contraction.
-// With a long one their registers and polls cost a little.  Measured, 8 -> 16 (us, L2 flushed):
-//   16384 x 4096, K = 1024: plain 94.0 -> 89.3, GeLU 97.6 -> 89.7, product kept too 107.6 -> 102.0, GeLU's derivative
-//     133.6 -> 126.4, tanh form's 132.6 -> 129.6, ReLU's 113.3 -> 119.6
-//   8192 x 4096, K = 1024: 52.0 -> 50.5, 52.7 -> 49.4, 57.7 -> 54.7, 71.2 -> 70.1, 69.9 -> 70.8, 62.2 -> 65.1
-//   2048 x 3072, K = 768: plain 19.8 -> 19.3;  16384 x 1024, K = 4096: plain 93.1 -> 94.7;  4096 x 10240, K = 2560: 128.4 -> 129.5
-constexpr int kManyEpiWarpsK = 1536;      // plain products up to this K have sixteen
-constexpr int epi_warps(int kind) { return kind == kEpiGeluTanhBwd || kind == kEpiReluBwd ? 8 : 16; }
+// wait side by side), which counts where the epilogue is what a tile takes; there are 96 registers for a thread then, which
+// spills a little of the plain one, and a block of eighteen warps starts later.  Measured, 8 -> 16 (us):
+//   tiles of 256 columns, L2 flushed, 16384 x 4096, K = 1024: plain 94.0 -> 89.3, GeLU 97.6 -> 89.7, product kept too
+//     107.6 -> 102.0, GeLU's derivative 133.6 -> 126.4, tanh form's 132.6 -> 129.6, ReLU's 113.3 -> 119.6;
+//     8192 x 4096, K = 1024: 52.0 -> 50.5, 52.7 -> 49.4, 57.7 -> 54.7, 71.2 -> 70.1, 69.9 -> 70.8, 62.2 -> 65.1
+//   ... operands in L2, times as long, geometric means over M = 136 .. 8192 and N = 2048 .. 10240:
+//     GeLU 0.91 - 0.98 (K <= 1024: 0.93, one to four rounds of tiles alike), product kept too 0.94 - 1.00; tanh form 0.96 -
+//     0.99, product kept too 1.00 - 1.02; GeLU's derivative 0.98 - 1.00; dropout 0.99
+//     plain, K <= 1024: one round of tiles 1.03, two 1.005, three 0.98, more 0.95; K = 1152 .. 2560: 1.00 - 1.03
+//     whatever the rounds
+//     plain with B N-major (an input gradient): 1.05, 1.03, 1.01, 0.99; K = 1600 and 2560: 1.01 - 1.03
+//   tiles of 128 columns (at most one round), operands in L2: GeLU 1.04 - 1.06, product kept too 1.015, tanh form 1.04 -
+//     1.06 both, GeLU's derivative 1.003 - 1.014, dropout 1.02 - 1.04 (1000 x 2048, K = 512: GeLU 8.0 -> 8.7)
+constexpr int kManyEpiWarpsK = 1024;      // plain products up to this K have sixteen
+constexpr bool epi_sixteen(int kind) { return kind == kEpiGelu || kind == kEpiGeluBwd || kind == kEpiDropout; }
 constexpr int PBM = 128;   // rows of A per CTA (the pair's tile has 256)
 constexpr int PBK = 64;
 #ifndef SLAPO_GEMM2_KSUB
@@ -319,6 +326,7 @@ gemm2_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     // warps w, w + 4, .. share a quarter and split the columns
     const int col_part = (warp - 2) >> 2, col_parts = kEpiWarps / 4;
     constexpr int kChunks = BN / 32;
+    static_assert(kChunks % (kEpiWarps / 4) == 0, "epilogue: whole chunks of 32 columns for every warp");
     const int c_begin = col_part * (kChunks / col_parts), c_end = c_begin + kChunks / col_parts;
     int iter = 0;
     bool ok = true;
@@ -503,13 +511,18 @@ static int launch_pair_warps(const CUtensorMap& ta, const CUtensorMap& tb, const
 template <int BN, int STAGES, int KSUB, bool A_MN, bool B_MN, int kEpi = kEpiPlain>
 static int launch_pair_variant(const CUtensorMap& ta, const CUtensorMap& tb, const EpiParams<Gemm2Params, kEpi>& p,
                                cudaStream_t stream) {
-  if constexpr (kEpi != kEpiPlain) {
-    return launch_pair_warps<BN, STAGES, KSUB, A_MN, B_MN, kEpi, epi_warps(kEpi)>(ta, tb, p, stream);
+  // sixteen epilogue warps or eight (the figures are at kManyEpiWarpsK)
+  constexpr bool kWide = BN == 256 && !A_MN;
+  if constexpr (kWide && epi_sixteen(kEpi)) {
+    return launch_pair_warps<BN, STAGES, KSUB, A_MN, B_MN, kEpi, 16>(ta, tb, p, stream);
   } else {
-    // (a weight gradient's contraction is over the tokens; narrow tiles are short calls)
-    if constexpr (!A_MN && BN == 256)
-      if (p.K <= kManyEpiWarpsK && p.splits == 1)
+    if constexpr (kWide && !B_MN && kEpi == kEpiPlain) {
+      const int64_t tiles = static_cast<int64_t>((p.M + 2 * PBM - 1) / (2 * PBM)) * ((p.N + BN - 1) / BN);
+      if (p.K <= kManyEpiWarpsK && p.splits == 1 && tiles > 2 * (sm_count() / 2))
         return launch_pair_warps<BN, STAGES, KSUB, A_MN, B_MN, kEpi, 16>(ta, tb, p, stream);
+    }
+    if constexpr (kWide && kEpi == kEpiGeluTanh)
+      if (p.C2 == nullptr) return launch_pair_warps<BN, STAGES, KSUB, A_MN, B_MN, kEpi, 16>(ta, tb, p, stream);
     return launch_pair_warps<BN, STAGES, KSUB, A_MN, B_MN, kEpi, 8>(ta, tb, p, stream);
   }
 }
