@@ -130,7 +130,7 @@ __device__ __forceinline__ void slab_reduce_store(const float (&acc16)[16], floa
 //   16384 x  4096       96.2 -> 77.4         72.1 -> 66.2       64.9 -> 48.7
 //    8192 x  4096       51.2 -> 42.9         40.0 -> 36.4       34.8 -> 26.2
 //    4096 x 10240       77.3 -> 52.5         56.1 -> 44.1       42.3 -> 30.6
-//    8192 x  1024       17.4 -> 14.8         13.8 -> 12.3       11.6 ->  8.4
+//    8192 x  1024       17.4 -> 13.5         13.8 -> 11.2       11.6 ->  8.4
 //    4096 x  1024        9.2 -> 10.1          8.7 ->  8.2        7.5 ->  5.8
 //     512 x  2048        4.3 ->  4.6          4.3 ->  4.2        3.6 ->  3.5
 // (GeLU's at 16384 x 4096: 5.2 of 6.5 TB/s).
@@ -464,17 +464,27 @@ static int wave_chunks(int rows, int cols) {
 static bool slab_wide(int rows, int cols, int dtype, int64_t least) {
   return dtype < 2 && cols % 16 == 0 && static_cast<int64_t>(rows) * cols >= least;
 }
-// Row chunks of theirs, half of the general kernels' to all of them: the number with which waves of `per_sm` CTAs times
-// the rows of a CTA, and some 16 rows' time for its sums, is least.  Against half of them: GeLU's backward 4096 x 10240
-// 62.1 -> 52.5 us, 8192 x 30528 329 -> 274, 16384 x 4096 77.2 -> 77.4; dropout's 36.7 -> 30.6, 203 -> 163, 48.4 -> 48.8.
+// Row chunks of theirs: the most that fill one, two, three or four waves of `per_sm` CTAs, whichever takes least when a
+// wave takes the rows of a CTA and some 16 rows' time for its sums.  That is one wave unless the slabs of 256 columns leave
+// much of it empty (30528 columns, 120 slabs for 296 CTAs: two chunks up to some 500 rows, seven from there on).
+// Operands in L2 / L2 flushed (us), general kernel, two waves, one wave:
+//   GeLU's backward  8192 x 1024   13.0 / 17.1, 12.8 / 14.6, 11.9 / 13.5    1024 x 8192   12.7 / 17.1, 12.8 / 15.0, 11.9 / 14.1
+//                   16384 x 4096   93.9 / 94.8, 76.5 / 77.5, 75.9 / 77.4    4096 x 10240     - / 77.3,    - / 62.1, 52.2 / 52.4
+//                    8192 x 30528     -  /  - ,    -  / 329 , 277  / 275
+//   ReLU's           8192 x 2048   19.3 / 22.0, 17.6 / 20.3, 14.3 / 19.8    819 x 10240    9.4 / 13.2, 9.0 / 11.8, 8.4 / 11.5
+//   dropout's        1024 x 8192   11.1 / 11.5,  9.4 /  9.3,  8.4 /  8.3    68 x 30528     8.8 /  5.2, 8.8 /  5.7, 7.9 / 4.6
 static int slab_chunks(int rows, int cols, int per_sm) {
-  const int chunks = wave_chunks(rows, cols);
+  const int most = wave_chunks(rows, cols);
   const int64_t slabs = (cols + 255) / 256, resident = static_cast<int64_t>(sm_count()) * per_sm;
-  int best = chunks;
+  int best = most;
   int64_t least = -1;
-  for (int c = (chunks + 1) / 2; c <= chunks; ++c) {
+  for (int w = 1; w <= 4; ++w) {
+    const int64_t fill = w * resident / slabs;
+    const int c = fill < most ? static_cast<int>(fill) : most;
+    if (c < 1) continue;
     const int64_t time = (c * slabs + resident - 1) / resident * ((rows + c - 1) / c + 16);
     if (least < 0 || time < least) { least = time; best = c; }
+    if (c == most) break;
   }
   return best;
 }
