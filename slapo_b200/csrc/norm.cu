@@ -162,14 +162,16 @@ __global__ void __launch_bounds__(32 * WPR * RG, (VPL == 1 && WPR * RG == 16) ? 
 
 // The forward for 16-bit rows of 16 values per thread: a 32-byte access and one Philox call for all of them (the
 // kernel above draws each call twice, in neighbouring threads), WPR warps to a row, eight warps to a CTA, and the
-// next row fetched before this one's sums.  Same sums in the same roundings, so the outputs are the kernel's above.
+// next row fetched before this one's sums.  A row's two sums are added up in another order, so that y differs from the
+// kernel's above by single last places of 16 bits; z is the same to the bit.
 // Both are bound by the instructions and reductions of a row more than by memory; two CTAs of 128 registers per SM
-// hold 64 KB of loads in flight.  Kernel above -> this one, L2 flushed, dropout + residual / LayerNorm alone (us):
+// hold 32 KB of loads in flight (16 without a residual).  Kernel above -> this one, L2 flushed, dropout + residual /
+// LayerNorm alone (us):
 //   64 x 1024    3.7 -> 3.7 /  3.3 ->  2.9       16384 x  512    32.8 -> 16.2 / 22.4 ->  9.6
 //   2048 x 1024  7.6 -> 6.8 /  5.7 ->  4.5       16384 x 1536   100.6 -> 47.0 / 55.9 -> 29.3
 //   16384 x 1024 36.4 -> 28.6 / 24.6 -> 16.9     8192 x 2560     63.2 -> 42.6 / 48.0 -> 28.1
 //   8192 x 2048  55.6 -> 29.1 / 32.0 -> 17.6     8192 x 4096     74.9 -> 52.7 / 54.8 -> 32.8
-// (5.3 TB/s of 6.5 at 16384 x 1024 x 4 passes).  Up to 256 columns half of the lanes and more would have no values:
+// (4.7 TB/s of 6.5 at 16384 x 1024 x 4 passes).  Up to 256 columns half of the lanes and more would have no values:
 // 16384 x 256 12.7 there, 13.1 here.
 template <typename T, int WPR, bool kDrop>
 __global__ void __launch_bounds__(256, 2) ln_fwd_rows_kernel(
@@ -406,10 +408,7 @@ __global__ void __launch_bounds__(32 * WPR * RG, (VPL == 1 && WPR * RG == 16) ? 
 //   16384 x  512  37.2 -> 20.9 / 25.7 -> 17.2      16384 x 1024  41.1 -> 34.5 / 29.9 -> 27.1
 //   16384 x 1536  92.9 -> 58.2 / 66.9 -> 46.0       8192 x 2048  54.3 -> 36.3 / 39.9 -> 28.1
 //    8192 x 2560  66.4 -> 48.0 / 49.8 -> 39.5       8192 x 4096  85.5 -> 76.2 / 63.8 -> 61.2
-// Up to 1024 columns a CTA has four or eight groups whose column sums are added in turn at its end, which few rows do
-// not pay for: 1024 x 1024 7.3 -> 8.3, 4096 x 768 10.6 -> 11.5 without dropout; 6000 x 768 17.2 -> 16.2 and
-// 13.1 -> 13.3, 6000 x 1024 18.5 -> 17.8 and 14.1 -> 13.9, 3000 x 512 10.9 -> 9.8 and 8.4 -> 8.7, 4096 x 512
-// 13.3 -> 10.9 and 9.8 -> 9.3.
+// (which calls: rows_bwd_pays)
 template <typename T, int WPR, bool kDrop>
 __global__ void __launch_bounds__(256, 2) ln_bwd_rows_kernel(
     const T* __restrict__ gy, const T* __restrict__ gz, const T* __restrict__ zin,
@@ -608,8 +607,27 @@ static int ln_grid(int rows, int cols, int ctas_per_sm) {
 // The kernels with 16 values per thread: which rows they take (16-bit, whole groups of 16 values on 32 bytes).
 static bool rows_shape(int cols, int dtype) { return dtype < 2 && cols > 256 && cols <= 4096 && cols % 16 == 0; }
 static int rows_wpr(int cols) { return cols <= 512 ? 1 : cols <= 1024 ? 2 : cols <= 2048 ? 4 : 8; }
-// (the figures are at ln_bwd_rows_kernel)
-static bool rows_bwd_pays(int rows, int cols) { return cols > 1024 || rows >= (cols > 512 ? 6000 : 4096); }
+// Which backward calls they take.  Times against the general kernel's, finalising kernel included, with the operands in
+// L2 / the incoming gradients there and the rest not, as they are in a backward / L2 flushed:
+//                   LayerNorm alone         with dropout                         LayerNorm alone         with dropout
+//   512 x 3500      1.05 / 1.03 / 1.02      0.98 / 0.92 / 0.95       2048 x 296   0.94 /   -  /   -       0.91 /   -  /   -
+//   512 x 4096      0.96 / 0.95 / 0.93      0.86 / 0.83 / 0.84       2048 x 304   1.18 / 1.09 /   -       1.14 / 1.10 /   -
+//   768 x 4096      1.11 / 1.07 / 1.06      1.02 / 0.97 / 1.00       2048 x 592   1.19 / 1.10 /   -       1.14 / 1.09 /   -
+//   768 x 6000      1.14 / 1.03 / 1.01      1.00 / 0.95 / 0.95       2048 x 700   0.86 / 0.79 /   -       0.81 / 0.77 /   -
+//   768 x 8192      1.09 / 0.98 / 0.99      0.98 / 0.92 / 0.92       2048 x 4096  0.98 / 0.78 / 0.74      0.89 / 0.78 / 0.74
+//  1024 x 8192      1.09 / 0.96 / 0.97      0.98 / 0.92 / 0.89       2064 x 296   1.05 /   -  /   -       1.07 /   -  /   -
+//   768 x 16384     1.06 / 0.96 / 0.93      0.87 / 0.87 / 0.86       2064 x 1000  1.05 / 0.93 / 0.91      0.99 / 0.91 / 0.90
+//  1536 x 64        0.89 /   -  /   -       0.85 /   -  /   -        4096 x 296   1.03 /   -  /   -       1.08 /   -  /   -
+//  1536 x 2048      0.91 / 0.78 / 0.77      0.85 / 0.75 / 0.74       4096 x 1000  1.00 / 1.00 / 0.99      0.95 / 0.97 / 0.97
+// Up to 1024 columns a CTA's four or eight groups add their column sums in turn at its end, which takes many rows to pay
+// for.  Up to 2048 the general kernel has four rows to a CTA and this one two: between two and four rows an SM that one
+// has a CTA for each SM, and here some SMs have two.
+static bool rows_bwd_pays(int rows, int cols, bool drop) {
+  if (cols <= 512) return rows >= 4096;
+  if (cols <= 1024) return rows >= (drop ? 6000 : 8192);
+  if (cols <= 2048) return rows <= 2 * sm_count() || rows > 4 * sm_count();
+  return rows >= 1000;
+}
 static int rows_grid(int rows, int cols) {
   const int rg = 8 / rows_wpr(cols), want = (rows + rg - 1) / rg, cap = sm_count() * 2;
   return want < cap ? want : cap;
@@ -698,7 +716,8 @@ void launch_ln_bwd(const void* gy, const void* gz, const void* zin, const void* 
   const int want_dbias = dbias != nullptr;
   int grid;
   count_launch(2);
-  if (rows_shape(cols, dtype) && rows_bwd_pays(rows, cols) && on_32_bytes({gy, gz, zin, gamma, dx, dres})) {
+  if (rows_shape(cols, dtype) && rows_bwd_pays(rows, cols, p > 0.f) &&
+      on_32_bytes({gy, gz, zin, gamma, dx, dres})) {
     grid = rows_grid(rows, cols);
     ROWS_SWITCH(dtype, cols, p, (ln_bwd_rows_kernel<T, WPR, kDrop><<<grid, 256, 0, stream>>>(
         static_cast<const T*>(gy), static_cast<const T*>(gz), static_cast<const T*>(zin),

@@ -11,7 +11,7 @@ from slapo_b200.ops import native
 
 pytestmark = pytest.mark.gpu
 
-BF = torch.bfloat16
+BF, FP = torch.bfloat16, torch.float16
 
 
 def launched(call):
@@ -24,6 +24,10 @@ def launched(call):
     names = [e.name for e in seen.events() if e.device_type == torch.autograd.DeviceType.CUDA]
     ours = (re.search(r"slapo::(\w+(?:<[^(]*>)?)\(", n) for n in names)
     return [m.group(1) for m in ours if m]
+
+
+def sms():
+    return torch.cuda.get_device_properties(0).multi_processor_count
 
 
 def of(call, what):
@@ -84,3 +88,44 @@ def test_epilogue_warps_of_activations(m, n, k):
         assert of(call, "gemm2_tc05").endswith(f", {16 if wide else 8}>")
         plain = ops.bias_dropout_add_fwd(ops.gemm(x, w, None, -1, False, False), b, None, 0.1, rng)
         assert torch.equal(call(), plain)
+
+
+# ----------------------------------------------------------- backward of the norms
+def _norm_lines():
+    s = sms()
+    return [(4095, 512, 0.1, True, False), (4096, 512, 0.0, False, True),
+            (5999, 1024, 0.1, False, False), (6000, 1024, 0.1, False, True),
+            (8191, 528, 0.0, True, False), (8192, 528, 0.0, True, True),
+            (8191, 768, 0.0, False, False), (8192, 1024, 0.0, False, True),
+            (2 * s, 1536, 0.0, False, True), (2 * s + 1, 1536, 0.1, True, False),
+            (4 * s, 1040, 0.0, False, False), (4 * s + 1, 1040, 0.1, False, True),
+            (999, 2064, 0.1, True, False), (1000, 2064, 0.0, False, True)]
+
+
+@pytest.mark.parametrize("line", range(14))
+def test_norm_backward_lines(line):
+    rows, cols, p, two, by_rows = _norm_lines()[line]
+    ops = native.ops()
+    torch.manual_seed(rows + cols)
+    z, gy, gz = (torch.randn(rows, cols, device="cuda", dtype=FP) for _ in range(3))
+    gamma = torch.randn(cols, device="cuda", dtype=FP)
+    m = z.double().mean(-1, keepdim=True)
+    rs = torch.rsqrt((z.double() - m).square().mean(-1, keepdim=True) + 1e-5)
+    rng = torch.tensor([3, 8, 0, 0], dtype=torch.int64) if p else None
+    stats = m[:, 0].float(), rs[:, 0].float()
+    call = lambda: ops.dropout_add_ln_bwd(gy, gz if two else None, z, gamma, *stats, p, rng, True)
+    assert of(call, "ln_bwd_rows_kernel" if by_rows else "ln_bwd_kernel")
+    dx, dres, dgamma, dbeta, dbias = call()
+    xh = (z.double() - m) * rs
+    g = gy.double() * gamma.double()
+    dz = rs * (g - g.mean(-1, keepdim=True) - xh * (g * xh).mean(-1, keepdim=True))
+    if two:
+        dz = dz + gz.double()
+    close(dres, dz, FP)
+    close(dgamma, (gy.double() * xh).sum(0), FP)
+    close(dbeta, gy.double().sum(0), FP)
+    keep = dx != 0 if p else torch.ones_like(dx, dtype=torch.bool)
+    from slapo_b200.ops import functional as NF
+    want = dz * keep / (1 - (NF.effective_dropout_p(p) if p else 0.0))
+    close(dx, want, FP)
+    close(dbias, want.sum(0), FP)
