@@ -4,11 +4,11 @@
 // (so q/k/v slices of a fused QKV projection are read in place through 4-D
 // TMA maps - no .contiguous() copies).  D is 64 or 128.
 //
-// Two kernels.  flash_fwd_groups_kernel takes calls with more than one tile of 128 query rows: persistent
+// Two kernels.  flash_fwd_groups_kernel takes most calls with more than one tile of 128 query rows: persistent
 // CTAs, one per SM, with two softmax groups that take the key tiles of a work item in turn.  Persistent CTAs of
 // flash_fwd_kernel (D = 64: two per SM with 256 of the 512 TMEM columns each; D = 128: one) take those with a
-// single row tile, where the keys may be split over work items.  Both walk over work items of 128 query rows
-// of one (batch, head), for each of which they stream the keys in tiles of 128:
+// single row tile, where the keys may be split over work items, and short calls with few key tiles (fwd_in_groups).
+// Both walk over work items of 128 query rows of one (batch, head), for each of which they stream the keys in tiles of 128:
 //   a thread     TMA: Q, K ring, V ring (runs ahead over tiles and over work items)
 //   a thread     tcgen05.mma:  S = Q K^T       (fp32, 128 TMEM columns)
 //                              O += P V        (P read from TMEM, fp32 accumulator in TMEM)
@@ -616,7 +616,7 @@ struct GroupsSmem {
 // 83.5 -> 74.9; 8 x 512 x 16 x 64 with T5's bias, key bias and p 0.1: 43.7 -> 41.2; 1 x 512 x 16 x 64, p 0.1: 12.9 ->
 // 9.4; 4 x 2048 x 16 x 128 causal: 111 -> 91, all keys 154 -> 128; 4 x 1000 x 32 x 80 causal with key bias: 70 -> 60;
 // 4 x 1024 x 16 x 128, p 0.1: 61 -> 49.  With a single row tile there are too few tiles to share out: 2 x 60 x 60 x
-// 8 x 128: 6.5 -> 8.0.
+// 8 x 128: 6.5 -> 8.0 (which calls come here: fwd_in_groups).
 template <int D, bool kGeneral, bool kDrop, typename T>
 __global__ void __launch_bounds__(512, 1)
 flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -1168,6 +1168,25 @@ static int launch_fwd_groups(const CUtensorMap& tq, const CUtensorMap& tk, const
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
+// Whether a call without split keys goes to the two softmax groups.  At D = 64 they have one CTA per SM where the other
+// kernel has two, so that calls which that one takes in a single wave, and whose few key tiles leave the groups little to
+// share, stay with it.  Groups against the other kernel, times as long, by number of work items on 148 SMs
+// (heads of 64 and 32, 129 - 2048 queries, all keys / with dropout / causal; 8 x 200 x 100 keys x 16 x 64: 9.9 against 8.5 us):
+//   one key tile     up to 296: 0.98 - 1.17 / 0.95 - 1.11 / -    from 300 on: 0.79 - 1.01 / 0.79 - 0.98 / -
+//   two              up to 148: 0.92 - 1.02 / 0.83 - 0.90 / 0.94 - 1.00    160 - 296: 0.97 - 1.11 / 0.94 - 1.04 / 1.14 - 1.18
+//                    from 300 on: 0.86 - 1.00 / 0.83 - 1.02 / 0.90 - 1.05
+//   three            up to 148: 0.94 - 1.04 / 0.83 - 0.91 / 0.95 - 1.02    150 - 296: 0.95 - 1.15 / 0.93 - 1.10 / 0.95 - 1.16
+//                    from 300 on: 0.88 - 1.04 / 0.83 - 1.04 / 0.98 - 1.06
+//   four and more    150 - 296: 0.90 - 1.14 / 0.84 - 1.06 / 0.80 - 1.04
+// (dropout with nothing else, two or three key tiles, 150 - 296 items: 0.93 - 0.99)
+template <int D, bool kGeneral, bool kDrop>
+static bool fwd_in_groups(const FlashFwdParams& p, int64_t items) {
+  if (p.walk.row_tiles == 1) return false;
+  if (D != 64 || items > 2 * sm_count()) return true;
+  const int key_tiles = (p.Sk + kBlockN - 1) / kBlockN;
+  return key_tiles > 3 || (key_tiles > 1 && (items <= sm_count() || (kDrop && !kGeneral)));
+}
+
 template <int D, bool kGeneral, bool kDrop, typename T>
 static int launch_fwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                         const FlashFwdParams& p, cudaStream_t stream) {
@@ -1182,7 +1201,8 @@ static int launch_fwd_d(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
     configured = true;
   }
   const int64_t items = static_cast<int64_t>(p.walk.row_tiles) * p.walk.nbh * p.splits;
-  if (p.walk.row_tiles > 1) return launch_fwd_groups<D, kGeneral, kDrop, T>(tq, tk, tv, p, items, stream);
+  if (fwd_in_groups<D, kGeneral, kDrop>(p, items))
+    return launch_fwd_groups<D, kGeneral, kDrop, T>(tq, tk, tv, p, items, stream);
   const int64_t cap = FwdSmem<D>::kCtas * sm_count();
   count_launch();
   kernel<<<static_cast<int>(items < cap ? items : cap), 192, kSmem, stream>>>(tq, tk, tv, p);

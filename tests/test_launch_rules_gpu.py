@@ -1,5 +1,6 @@
 """Which kernel a call gets on either side of the lines that the dispatch rules draw, from a profile of the
 launch, and that both sides of a line agree with 64 bits.  The lines follow from times beside each rule."""
+import math
 import re
 
 import pytest
@@ -129,3 +130,45 @@ def test_norm_backward_lines(line):
     want = dz * keep / (1 - (NF.effective_dropout_p(p) if p else 0.0))
     close(dx, want, FP)
     close(dbias, want.sum(0), FP)
+
+
+# ----------------------------------------------------------- forward of attention, short calls
+def _attn_lines():
+    s = sms()
+    # heads, queries, keys, head dim, causal, dropout, key bias; softmax groups or not
+    # (two row tiles for 129 - 256 queries)
+    return [(s, 200, 100, 64, False, 0.0, False, False),
+            (s + 1, 200, 100, 64, False, 0.0, False, True),
+            (s, 256, 128, 32, False, 0.1, True, False),
+            (8, 130, 64, 64, False, 0.0, False, False),
+            (s // 2, 200, 256, 64, False, 0.0, False, True),
+            (s // 2 + 1, 200, 256, 64, False, 0.0, False, False),
+            (s // 2 + 1, 200, 256, 64, False, 0.1, False, True),
+            (s // 2 + 1, 200, 256, 64, False, 0.1, True, False),
+            (s // 2 + 1, 200, 200, 64, True, 0.1, False, False),
+            (s - 20, 200, 300, 64, False, 0.0, True, False),
+            (s - 20, 200, 400, 64, False, 0.0, True, True),
+            (s - 20, 200, 100, 128, False, 0.0, False, True),
+            (s - 20, 100, 100, 64, False, 0.0, False, False)]
+
+
+@pytest.mark.parametrize("line", range(13))
+def test_attention_forward_lines(line):
+    h, sq, sk, d, causal, p, biased, groups = _attn_lines()[line]
+    ops = native.ops()
+    torch.manual_seed(h + sq)
+    q, k, v = (torch.randn(1, s, h, d, device="cuda", dtype=BF) for s in (sq, sk, sk))
+    kb = torch.randn(1, sk, device="cuda") if biased else None
+    rng = torch.tensor([3, 8, 0, 0], dtype=torch.int64) if p else None
+    call = lambda: ops.flash_attn_fwd(q, k, v, kb, None, causal, d ** -0.5, p, rng)
+    assert of(call, "flash_fwd_groups_kernel" if groups else "flash_fwd_kernel")
+    out, lse = call()
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) * d ** -0.5
+    if biased:
+        s = s + kb.double()[:, None, None]
+    if causal:
+        s = s.masked_fill(torch.ones(sq, sk, dtype=torch.bool, device="cuda").triu(sk - sq + 1), -math.inf)
+    torch.testing.assert_close(lse.double(), torch.logsumexp(s, -1).view_as(lse), rtol=1e-5, atol=2e-5)
+    if not p:      # (dropped calls: tests/test_flash_paths_gpu.py)
+        close(out, torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), v.double()), BF, roundings=2)
+    assert ops.device_status() == 0
