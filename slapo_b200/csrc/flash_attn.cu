@@ -654,6 +654,10 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   // S, O and P of the two groups.  For D = 128 P is written over S: the next S of a group goes into the
   // tensor core's queue behind the product that uses P up.  For D = 64 P has columns of its own and the next
   // S is formed as soon as this one has been read.
+  // Relied on here: a later product of the same thread writes its result only after an earlier one has read its operands.
+  // PTX promises two tcgen05.mma in their order of issue for the same accumulator and shape; these differ in both, and
+  // a wait on pv_done, 400 - 650 cycles from commit to wait, would be what the documents ask for.  The order is
+  // what the hardware shows: no difference in repeated and random calls, tests/test_flash_order_gpu.py.
   constexpr bool kOver = D == 128;
   constexpr uint32_t kColS = 0, kColO = 256, kColP = kOver ? kColS : 384, kPGroup = kOver ? 128 : 64;
 
@@ -806,7 +810,7 @@ flash_fwd_groups_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
             if (*abort_flag != 0) break;
             tc::umma_commit(&pv_done[g]);
             tc::umma_commit(&v_empty[rv.slot]);
-            // (products of one thread run in order: S goes over a P that has been used up)
+            // (no wait: S goes over a P that the products just issued still read; the order is explained at kOver)
             if (kOver && !form_s(g)) break;
             ok = true;
           }

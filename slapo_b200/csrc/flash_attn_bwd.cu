@@ -223,10 +223,10 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
   uint64_t* y2_full = bars + 20;      // kY2 (4)
   uint64_t* y2_empty = bars + 24;
   uint64_t* s_full = bars + 28;       // one per softmax group from here on
-  uint64_t* p_ready = bars + 30;      // 4 warps: S has been read (and P written)
+  uint64_t* p_ready = bars + 30;      // 8 warps: S has been read (and P written)
   uint64_t* dp_full = bars + 32;
   uint64_t* a1_done = bars + 36;      // dQ pass: dS of a half tile has been used up
-  uint64_t* ds_ready = bars + 34;     // 4 warps: dS written
+  uint64_t* ds_ready = bars + 34;     // 8 warps: dS written
   uint64_t* acc1_full = bars + 40;    // kAcc (<= 2) each
   uint64_t* acc1_free = bars + 42;    // 4 warps
   uint64_t* acc2_full = bars + 44;
@@ -470,7 +470,10 @@ __device__ __forceinline__ void bwd_pass(const CUtensorMap& tm_x1, const CUtenso
       } else if (warp == 1) {
         // ------------------------------ dK / dV pass: S and dV ------------------------------
         // The next S of a group goes into the tensor core's queue behind the product that uses up the P in its
-        // place, two half tiles ahead.
+        // place, two half tiles ahead.  That S does not overtake that product's reads is the order in which the tensor core
+        // takes one thread's products; PTX promises it for the same accumulator and shape only, and here both
+        // differ (N = 64 for S, the head's columns for dV).  Same for dP over dS in the next warp.  Checked by
+        // tests/test_flash_order_gpu.py; the dQ pass waits for the product (380 - 650 cycles from commit to wait).
         const uint32_t x_desc = tc::smem_desc_lo(tc::smem_u32(smem), 16);
         const uint32_t y_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kY1At), 16);
         const uint32_t y2_desc = tc::smem_desc_lo(tc::smem_u32(smem + L::kY2At), kBlkY);
@@ -1075,9 +1078,9 @@ static int round128(int n) { return (n + 127) / 128 * 128; }
 // again, and each pass has its tensors in L2 to itself.  Weighed as rounds of work items, in tiles
 // of the dQ pass: a tile of dK / dV takes 1.4 of them (1.37 for D = 128; with dropout, which costs the dQ pass more,
 // 1.05 and 1.27, and 0.5 more drawing), an item a quarter more (D = 128: one, its dK has no second set of
-// accumulators to go on with), a launch 2; both in one came out a tenth under that.  Under a causal mask items
-// differ and the heaviest go first, so that no whole rounds are lost in two launches or one: side by side
-// up to 5 waves of each.
+// accumulators to go on with), a launch 2; both in one came out a tenth under that.  Under a causal mask without
+// dropout items differ and the heaviest go first, so that no whole rounds are lost in two launches or one: side by
+// side up to 5 waves of each.  (With dropout, where drawing counts, causal calls are weighed as the others.)
 // Measured, two launches -> one (us).  Taken side by side: 1 x 512 x 16 x 64: 23.3 -> 15.0; 1 x 2048 x 12 x 64 causal: 86
 // -> 54; 4 x 512 x 16 x 64: 38.5 -> 28.4; 2 x 1024 x 16 x 128, p 0.1: 94 -> 77; 3 x 1820 x 8 x 128 causal, p 0.1: 162 -> 113; 27
 // x 245 x 8 x 64 causal, p 0.1: 44 -> 36; 7 x 1496 x 16 x 64: 331 -> 305; 4 x 1024 x 16 x 128: 122 -> 112; 32 x 256 x 16 x
