@@ -209,3 +209,41 @@ def test_sixteen_columns_per_lane_backward(rows, cols, act):
     err = 2 ** -24 * rows * float(wide[0].float().abs().max())
     torch.testing.assert_close(wide[1].float(), slim[1].float(), rtol=2 ** -7, atol=err)
     assert torch.equal(again[1], wide[1])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols", [(8200, 1024), (275, 30528), (1000, 8448)])
+def test_sixteen_columns_per_lane_backward_forms(rows, cols, dtype):
+    """Both types, without a bias, without column sums, every activation from 8 Mi values on (where the
+    kernels with sixteen columns per lane take an activation's backward), against the general kernels and
+    64 bits."""
+    ops = native.ops()
+    assert rows * cols >= 8 << 20
+    torch.manual_seed(cols)
+    dy, x = (torch.randn(rows, cols, device="cuda").to(dtype) for _ in range(2))
+    bias = torch.randn(cols, device="cuda").to(dtype)
+    off = torch.empty(rows * cols + 8, device="cuda", dtype=dtype)[8:].view(rows, cols).copy_(dy)
+    assert dy.data_ptr() % 32 == 0 and off.data_ptr() % 32 == 16
+    rng = torch.tensor([5, 4, 0, 0], dtype=torch.int64)
+    # one rounding of a sum to 16 bits; sums of `rows` values in 32 bits whatever their order
+    eps = torch.finfo(dtype).eps
+
+    def sums(got, dx):
+        want = dx.double().sum(0)       # of values before their rounding, each up to eps / 2 of its own away
+        rounded = float((dx.double().abs() * eps).norm(dim=0).max())
+        slack = rows * 2.0 ** -24 * float(dx.double().abs().max()) + 2 * rounded
+        assert float(((got.double() - want).abs() - eps * want.abs()).max()) <= slack
+
+    for act in (0, 1, 2):
+        for call in (lambda g: ops.bias_act_bwd(g, x, bias, act), lambda g: ops.act_bwd_colsum(g, x, act)):
+            wide, slim = call(dy), call(off)
+            assert torch.equal(wide[0], slim[0])
+            sums(wide[1], wide[0])
+            sums(slim[1], slim[0])
+        alone, none = ops.bias_act_bwd(dy, x, None, act)
+        assert none.numel() == 0 and torch.equal(alone, ops.bias_act_bwd(off, x, None, act)[0])
+    wide, slim = (ops.bias_dropout_add_bwd(g, 0.1, rng, True) for g in (dy, off))
+    assert torch.equal(wide[0], slim[0])
+    sums(wide[1], wide[0])
+    alone, none = ops.bias_dropout_add_bwd(dy, 0.1, rng, False)
+    assert none.numel() == 0 and torch.equal(alone, wide[0])

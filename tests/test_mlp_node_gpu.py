@@ -77,3 +77,24 @@ def test_dropout_in_the_epilogue(rows, n, k, dtype):
             want = ops.bias_dropout_add_fwd(ops.gemm(a, w, None, -1, False, False), bias, None, p, rng)
             assert torch.equal(got, want)
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,n,k,tile", [
+    (4100, 2576, 128, (True, 0)), (16384, 1024, 64, (True, 0)), (2049, 4112, 72, (True, 0)),
+    (1000, 2064, 136, (True, 128)), (120, 148 * 64 + 16, 64, (False, 128)),
+    (100, 148 * 128 + 48, 64, (False, 0)), (40, 144, 64, (False, 64))])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_dropout_in_the_epilogue_of_each_tile(rows, n, k, tile, dtype):
+    """As above, with the tile named: CTA pairs' of 256 and 128 columns, one CTA's of 64, 128 and 256, ragged
+    last ones."""
+    ops = native.ops()
+    assert tuple(ops.gemm_tile(rows, n)) == tile
+    torch.manual_seed(rows + n)
+    a = torch.randn(rows, k, device="cuda", dtype=dtype)
+    w = (torch.randn(n, k, device="cuda") * k ** -0.5).to(dtype)
+    for bias in (None, torch.randn(n, device="cuda", dtype=dtype)):
+        rng = ops.philox_reserve(rows * n)
+        got = ops.gemm_dropout_fwd(a, w, bias, 0.1, rng)
+        want = ops.bias_dropout_add_fwd(ops.gemm(a, w, None, -1, False, False), bias, None, 0.1, rng)
+        assert torch.equal(got, want)
+    assert ops.device_status() == 0
