@@ -206,7 +206,7 @@ __device__ __forceinline__ uint32_t pair_word(float a, float b, __half) {
 }
 
 template <typename T>
-__device__ __forceinline__ void unpack16(const uint32_t (&w)[8], float (&v)[16]) {
+__device__ __forceinline__ void unpack_values(const uint32_t (&w)[8], float (&v)[16]) {
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const float2 f = pair_floats(w[k], T());
@@ -215,7 +215,7 @@ __device__ __forceinline__ void unpack16(const uint32_t (&w)[8], float (&v)[16])
   }
 }
 template <typename T>
-__device__ __forceinline__ void pack16(const float (&v)[16], uint32_t (&w)[8]) {
+__device__ __forceinline__ void pack_values(const float (&v)[16], uint32_t (&w)[8]) {
 #pragma unroll
   for (int k = 0; k < 8; ++k) w[k] = pair_word(v[2 * k], v[2 * k + 1], T());
 }

@@ -206,11 +206,11 @@ __global__ void __launch_bounds__(256) bias_dropout_add_bwd_wide_kernel(
         if (r + 16 * u < r1) {
           const int64_t e = e0 + static_cast<int64_t>(16 * u) * cols;
           float g[16];
-          unpack16<T>(w[u], g);
+          unpack_values<T>(w[u], g);
           drop16(philox_keep16(seed, offset, static_cast<uint64_t>(e) >> 4, add4), scale, g);
 #pragma unroll
           for (int k = 0; k < 16; ++k) acc[k] += g[k];
-          pack16<T>(g, w[u]);
+          pack_values<T>(g, w[u]);
           store16_raw(dx + e, w[u]);
         }
     }

@@ -60,15 +60,7 @@ __device__ __forceinline__ void cp_async4(float* smem_dst, const float* src) {
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-template <typename T> __device__ __forceinline__ uint32_t pack16(float a, float b);
-template <> __device__ __forceinline__ uint32_t pack16<__nv_bfloat16>(float a, float b) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-template <> __device__ __forceinline__ uint32_t pack16<__half>(float a, float b) {
-  __half2 v = __floats2half2_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
+template <typename T> __device__ __forceinline__ uint32_t pack16(float a, float b) { return pair_word(a, b, T()); }
 
 // ... of values that count as 0 where they are negative
 template <typename T> __device__ __forceinline__ uint32_t pack16_relu(float a, float b);

@@ -103,15 +103,6 @@ struct GemmSmem {
   static constexpr int kTotal = kBarOffset + 256 + 1024;  // + barriers + alignment slack
 };
 
-__device__ __forceinline__ uint32_t pack2(float a, float b, int out_bf16) {
-  if (out_bf16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-  __half2 v = __floats2half2_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-
 __device__ __forceinline__ float load_bias(const void* bias, int col, int out_bf16) {
   if (out_bf16) return __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[col]);
   return __half2float(static_cast<const __half*>(bias)[col]);
@@ -280,7 +271,7 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap tmap_a,
               v0 = act_fwd(v0, p.act);
               v1 = act_fwd(v1, p.act);
             }
-            packed[j] = pack2(v0, v1, p.out_bf16);
+            packed[j] = pack_pair(v0, v1, p.out_bf16);
           }
           uint8_t* dst = static_cast<uint8_t*>(p.C) +
                          (static_cast<int64_t>(row) * p.ldc + col0) * 2;

@@ -83,14 +83,6 @@ struct Gemm2Smem {
   static constexpr int kTotal = kBarOffset + 256 + 1024;
 };
 
-__device__ __forceinline__ uint32_t g2_pack2(float a, float b, int out_bf16) {
-  if (out_bf16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-  __half2 v = __floats2half2_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
 __device__ __forceinline__ float g2_bias(const void* bias, int col, int out_bf16) {
   if (out_bf16) return __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[col]);
   return __half2float(static_cast<const __half*>(bias)[col]);
@@ -126,12 +118,12 @@ __device__ __forceinline__ void g2_finish_store(const Gemm2Params& p, const floa
       v0 += b2.x;
       v1 += b2.y;
     }
-    if (p.C2 != nullptr) packed2[j] = g2_pack2(v0, v1, p.out_bf16);
+    if (p.C2 != nullptr) packed2[j] = pack_pair(v0, v1, p.out_bf16);
     if (p.act >= 0) {
       v0 = act_fwd(v0, p.act);
       v1 = act_fwd(v1, p.act);
     }
-    packed[j] = g2_pack2(v0, v1, p.out_bf16);
+    packed[j] = pack_pair(v0, v1, p.out_bf16);
   }
   const int64_t off = (static_cast<int64_t>(row) * p.ldc + col0) * 2;
   uint8_t* dst = static_cast<uint8_t*>(p.C) + off;
@@ -469,7 +461,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const Gemm2Params p)
         v0 = act_fwd(v0, p.act);
         v1 = act_fwd(v1, p.act);
       }
-      packed[j] = g2_pack2(v0, v1, p.out_bf16);
+      packed[j] = pack_pair(v0, v1, p.out_bf16);
     }
     *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.C) +
                               (static_cast<int64_t>(row) * p.ldc + col) * 2) =

@@ -64,12 +64,7 @@ __device__ __forceinline__ float2 unpack_pair(uint32_t w, int bf16) {
   return __half22float2(*reinterpret_cast<const __half2*>(&w));
 }
 __device__ __forceinline__ uint32_t pack_pair(float a, float b, int bf16) {
-  if (bf16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-  __half2 v = __floats2half2_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
+  return bf16 ? pair_word(a, b, __nv_bfloat16()) : pair_word(a, b, __half());
 }
 
 // 32 columns of a row as 16 words, from and to 16-byte aligned memory (N % 8 == 0: whole groups of

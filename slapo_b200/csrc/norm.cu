@@ -205,12 +205,12 @@ __global__ void __launch_bounds__(256, 2) ln_fwd_rows_kernel(
     float v[16];
     float s = 0.f;
     if (ok) {
-      unpack16<T>(xn, v);
+      unpack_values<T>(xn, v);
       if (bias != nullptr) {
         uint32_t w[8];
         float b[16];
         load16_raw(bias + col, w);
-        unpack16<T>(w, b);
+        unpack_values<T>(w, b);
 #pragma unroll
         for (int k = 0; k < 16; ++k) v[k] += b[k];
       }
@@ -220,16 +220,16 @@ __global__ void __launch_bounds__(256, 2) ln_fwd_rows_kernel(
       }
       if (residual != nullptr) {
         float r[16];
-        unpack16<T>(rn, r);
+        unpack_values<T>(rn, r);
 #pragma unroll
         for (int k = 0; k < 16; ++k) v[k] += r[k];
       }
       if (z != nullptr) {
         // statistics must see exactly what the backward will re-read
         uint32_t w[8];
-        pack16<T>(v, w);
+        pack_values<T>(v, w);
         store16_raw(z + e, w);
-        unpack16<T>(w, v);
+        unpack_values<T>(w, v);
       }
 #pragma unroll
       for (int k = 0; k < 16; ++k) s += v[k];
@@ -246,14 +246,14 @@ __global__ void __launch_bounds__(256, 2) ln_fwd_rows_kernel(
       uint32_t w[8];
       float g[16], b[16];
       load16_raw(gamma + col, w);
-      unpack16<T>(w, g);
+      unpack_values<T>(w, g);
       if (beta != nullptr) {
         load16_raw(beta + col, w);
-        unpack16<T>(w, b);
+        unpack_values<T>(w, b);
       }
 #pragma unroll
       for (int k = 0; k < 16; ++k) v[k] = (v[k] - mean) * rstd * g[k] + (beta != nullptr ? b[k] : 0.f);
-      pack16<T>(v, w);
+      pack_values<T>(v, w);
       store16_raw(y + e, w);
     }
     if (lane == 0 && wir == 0) {
