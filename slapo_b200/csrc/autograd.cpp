@@ -138,7 +138,7 @@ struct LinearFn : public Function<LinearFn> {
 
 // y = dropout(act(x W1^T + b1) W2^T + b2): a feed-forward block as one node.  The input gradient of the
 // second layer goes through the activation's derivative and its column sums in that product's epilogue,
-// which as separate nodes is a pass of its own over the inner width (16384 x 4096 bf16: 95 + 79 -> 148 us), and
+// which as separate nodes is a pass of its own over the inner width (16384 x 4096 bf16: 94 + 72 -> 137 us), and
 // the host enters autograd once per direction instead of three or four times.
 struct MlpFn : public Function<MlpFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w1, const Tensor& b1,

@@ -8,19 +8,22 @@
 // `c2_sum` product + bias, rounded.  Backward: C = acc * act'(Z), with column sums of C (the bias gradient) over each 32 rows
 // to `col_part` [ceil(M / 32)][N], which a second kernel adds up in a fixed order.
 // An element is about 20 instructions and two of the special-function unit, which run under the next
-// tile's products as far as those last.  Measured, L2 flushed (us; plain product / with the epilogue / the pass over
-// memory that it replaces), with eight epilogue warps per CTA: 16384 x 4096, K = 1024     4096 x 10240, K = 2560
-//   GeLU                                               105 / 108 / 62             136 / 137 / 42
-//   GeLU, the product kept                             105 / 117 / 62             136 / 142 / 42
-//   GeLU's derivative and column sums                   95 / 148 / 77             138 / 157 / 53
-//   ReLU's                                              95 / 130 / 66             138 / 161 / 44
-// (with the sixteen that GeLU has now: gemm2.cu at kManyEpiWarpsK)
+// tile's products as far as those last.  Measured, L2 flushed, one machine (us; plain product / with the epilogue / the
+// pass over memory that it replaces; eight or sixteen epilogue warps as in gemm2.cu at kManyEpiWarpsK):
+//                                              16384 x 4096, K = 1024     4096 x 10240, K = 2560
+//   GeLU                                               96 /  98 / 58             138 / 140 / 39
+//   GeLU, the product kept                             96 / 111 / 58             138 / 146 / 39
+//   tanh form                                          96 /  92 / 58             138 / 138 / 39
+//   tanh form, the product kept                        96 / 109 / 58             138 / 145 / 39
+//   GeLU's derivative and column sums                  94 / 137 / 72             138 / 156 / 50
+//   tanh form's                                        94 / 143 / 73             138 / 156 / 49
+//   ReLU's                                             94 / 126 / 54             138 / 153 / 36
+// So the forward is all but hidden, while the derivative's epilogue is what bounds a product with K = 1024:
+// of the pass of 72 us it saves 29, at K = 2560 32 of 50.
 // Dropout (kEpiDropout): C = dropout(product + bias), again to the bit what a product and a kernel behind it give:
 // the product is rounded first, and an element's decision is that of its index in C (16 to a Philox call, two calls
-// for 32 columns; N % 16 == 0).  16384 x 1024, K = 4096: 92.3 -> 92.0 us, and a
+// for 32 columns; N % 16 == 0).  16384 x 1024, K = 4096: 98.8 -> 97.9 us, and a
 // pass of 20 less; a whole feed-forward block of 8192 x 512 204 -> 187.
-// So the forward is all but hidden, while the derivative's epilogue is what bounds a product with K = 1024:
-// of the pass of 77 us it saves 24, at K = 2560 34 of 53.
 #pragma once
 #include <type_traits>
 #include "common.cuh"
